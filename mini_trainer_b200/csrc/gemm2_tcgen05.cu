@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "gather.cuh"
+#include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 
 namespace mtb {
@@ -48,14 +49,9 @@ constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;   // clears the CTA-rank bit of a sh
 
 struct Params {
   int M, N, K;
-  void* D;
-  long long ldd;
-  const void* R;
-  long long ldr;
-  const __nv_bfloat16* bias;
   int* status;
   int num_pairs;
-  float alpha;
+  EpiParams e;
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -111,6 +107,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), tiles_n = (p.N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
   const int kblocks = (p.K + BK - 1) / BK;
+  const int splits = GATHER ? 1 : p.e.splits;
+  const int num_items = num_tiles * splits;   // item = split * num_tiles + tile: neighbours share operand tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -131,6 +129,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  auto k_range = [&](int split, int& kb0, int& kb1) {
+    kb0 = static_cast<int>(static_cast<long long>(kblocks) * split / splits);
+    kb1 = static_cast<int>(static_cast<long long>(kblocks) * (split + 1) / splits);
+  };
   auto tile_coords = [&](int t, int& tm, int& tn) {
     if constexpr (GATHER) {   // bands of column-tiles: the weight is consumed front to back at an even rate
       const int band = t / (GATHER_GROUP_N * tiles_m);
@@ -154,9 +156,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     if (elect_one()) {
       uint32_t it = 0, tl = 0;
       unsigned long long waited_ns = 0;
-      for (int t = pair; t < num_tiles; t += p.num_pairs) {
-        int tm, tn;
-        tile_coords(t, tm, tn);
+      for (int w = pair; w < num_items; w += p.num_pairs) {
+        int tm, tn, kb0, kb1;
+        tile_coords(w % num_tiles, tm, tn);
+        k_range(w / num_tiles, kb0, kb1);
         const int row0 = tm * 2 * BM + rank * BM;        // this CTA's rows of A
         const int col0 = tn * BN + rank * BNH;           // this CTA's half of the B tile
         if (GATHER) {
@@ -164,7 +167,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           asm volatile("fence.proxy.async;" ::: "memory");   // peer data was written with ordinary stores, TMA reads it
           ++tl;
         }
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag)) { atomicExch(p.status, 51); goto done; }
@@ -196,13 +199,15 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       uint32_t it = 0, tl = 0;
-      for (int t = pair; t < num_tiles; t += p.num_pairs, ++tl) {
+      for (int w = pair; w < num_items; w += p.num_pairs, ++tl) {
+        int kb0, kb1;
+        k_range(w / num_tiles, kb0, kb1);
         const int acc = tl & 1;
         const uint32_t aph = (tl >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], aph ^ 1, abort_flag)) { atomicExch(p.status, 52); goto done; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&full_bar[s], ph, abort_flag)) { atomicExch(p.status, 53); goto done; }
@@ -213,7 +218,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t da = A_MN ? make_smem_desc(sa + k * 2048, 8192, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
             const uint64_t db = B_MN ? make_smem_desc(sb + k * 2048, 8192, 1024) : make_smem_desc(sb + k * 32, 16, 1024);
-            umma2_bf16(d_tmem, da, db, idesc, (kb | k) != 0);
+            umma2_bf16(d_tmem, da, db, idesc, kb != kb0 || k != 0);
           }
           umma2_commit_pair(&empty_bar[s]);
         }
@@ -247,70 +252,16 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // ------------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
     uint32_t tl = 0;
-    for (int t = pair; t < num_tiles; t += p.num_pairs, ++tl) {
+    for (int w = pair; w < num_items; w += p.num_pairs, ++tl) {
+      const int t = w % num_tiles;
       int tm, tn;
       tile_coords(t, tm, tn);
       const int acc = tl & 1;
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag)) { atomicExch(p.status, 54); goto done; }
       tc_fence_after();
-      const int row = tm * 2 * BM + rank * BM + q * 32 + lane;
-      const bool row_ok = row < p.M;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int col0 = tn * BN + c * 32;
-        if (col0 >= p.N) break;
-        uint32_t v[32];
-        tmem_ld_32x32(taddr + c * 32, v);
-        tmem_ld_wait();
-        if (row_ok) {
-          float f[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * p.alpha;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col0 + j < p.N) {
-                const uint4 b = *reinterpret_cast<const uint4*>(p.bias + col0 + j);
-                const float2 b0 = unpack_bf16(b.x), b1 = unpack_bf16(b.y), b2 = unpack_bf16(b.z), b3 = unpack_bf16(b.w);
-                f[j] += b0.x; f[j + 1] += b0.y; f[j + 2] += b1.x; f[j + 3] += b1.y;
-                f[j + 4] += b2.x; f[j + 5] += b2.y; f[j + 6] += b3.x; f[j + 7] += b3.y;
-              }
-            }
-          }
-          if (OUT_F32) {
-            float* dptr = reinterpret_cast<float*>(p.D) + static_cast<long long>(row) * p.ldd + col0;
-            const float* rptr = p.R ? reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0 : nullptr;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (col0 + j < p.N) {
-                float4 o = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
-                if (rptr) { const float4 r = *reinterpret_cast<const float4*>(rptr + j); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
-                *reinterpret_cast<float4*>(dptr + j) = o;
-              }
-            }
-          } else {
-            __nv_bfloat16* dptr = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(row) * p.ldd + col0;
-            const __nv_bfloat16* rptr = p.R ? reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0 : nullptr;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col0 + j < p.N) {
-                if (rptr) {
-                  const uint4 r = *reinterpret_cast<const uint4*>(rptr + j);
-                  const float2 r0 = unpack_bf16(r.x), r1 = unpack_bf16(r.y), r2 = unpack_bf16(r.z), r3 = unpack_bf16(r.w);
-                  f[j] += r0.x; f[j + 1] += r0.y; f[j + 2] += r1.x; f[j + 3] += r1.y;
-                  f[j + 4] += r2.x; f[j + 5] += r2.y; f[j + 6] += r3.x; f[j + 7] += r3.y;
-                }
-                uint4 o;
-                o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
-                o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
-                *reinterpret_cast<uint4*>(dptr + j) = o;
-              }
-            }
-          }
-        }
-      }
+      epilogue_quarter<OUT_F32, !GATHER>(p.e, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
+                                2 * t + static_cast<int>(rank), w / num_tiles);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cta0(&tempty_bar[acc]);
@@ -329,7 +280,8 @@ done:
 static int g_pairs[2] = {-1, -1};   // clusters of two that can be co-resident (0: unsupported), plain / gather variant
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, Params p, cudaStream_t stream, const GatherParams* gp = nullptr) {
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
+                  long long ws_bytes = 0) {
   auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER>;
   constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS;
   static bool configured = false;
@@ -354,8 +306,15 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, Params p, cudaSt
   }
   if (pairs <= 0) return -6;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
+  // The arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest.
+  if (!GATHER && p.e.ws != nullptr && tiles * 8 * 4 <= SPLIT_COUNTER_BYTES) {
+    p.e.counters = reinterpret_cast<unsigned*>(p.e.ws);
+    p.e.ws += SPLIT_COUNTER_BYTES / 4;
+    p.e.splits = choose_splits(tiles, (p.K + BK - 1) / BK, pairs, (ws_bytes - SPLIT_COUNTER_BYTES) / (2 * SPLIT_UNIT * 4));
+  }
   // the gathering variant always uses every pair: its extra warps carry the transfer
-  p.num_pairs = (GATHER || tiles >= pairs) ? pairs : tiles;
+  const int items = tiles * p.e.splits;
+  p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
   static const GatherParams none{};
   kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, p, gp ? *gp : none);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
@@ -369,7 +328,7 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, w, K, N, K, BK, BNH);
   if (rc) return rc - 10;
-  Params p{M, N, K, D, ldd, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), status, 0, 1.0f};
+  Params p{M, N, K, status, 0, EpiParams{M, N, D, ldd, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr}};
   return launch<false, false, false, true>(ta, tb, p, stream, &g);
 }
 
@@ -382,7 +341,7 @@ extern "C" {
 // clusters of two cannot be scheduled on this device; callers then use the one-CTA kernel.
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                      float alpha, int* status, cudaStream_t stream) {
+                      float alpha, float* ws, long long ws_bytes, int* status, cudaStream_t stream) {
   using namespace mtb;
   using namespace mtb::g2;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -395,17 +354,17 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BNH);
   if (rc) return rc - 10;
-  Params p{M, N, K, D, ldd, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), status, 0, alpha};
+  Params p{M, N, K, status, 0, EpiParams{M, N, D, ldd, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, nullptr}};
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
-    case 0: return launch<false, false, false>(ta, tb, p, stream);
-    case 1: return launch<false, false, true>(ta, tb, p, stream);
-    case 2: return launch<false, true, false>(ta, tb, p, stream);
-    case 3: return launch<false, true, true>(ta, tb, p, stream);
-    case 4: return launch<true, false, false>(ta, tb, p, stream);
-    case 5: return launch<true, false, true>(ta, tb, p, stream);
-    case 6: return launch<true, true, false>(ta, tb, p, stream);
-    default: return launch<true, true, true>(ta, tb, p, stream);
+    case 0: return launch<false, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 1: return launch<false, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 2: return launch<false, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 3: return launch<false, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 4: return launch<true, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 5: return launch<true, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 6: return launch<true, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    default: return launch<true, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
   }
 }
 

@@ -27,6 +27,7 @@
 #include <stdlib.h>
 
 #include "gather.cuh"
+#include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 
 namespace mtb {
@@ -43,16 +44,11 @@ constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 
 
 struct GemmParams {
   int M, N, K;
-  void* D;
-  long long ldd;
-  const void* R;          // optional residual / accumulate source, same dtype as D
-  long long ldr;
-  const __nv_bfloat16* bias;  // optional, [N]
   int* status;            // device word; set non-zero when a bounded wait expired
-  float alpha;            // the product is multiplied by alpha before bias and residual are added
   int group_m;            // row-tiles per band of the tile order
   unsigned wait_hint_ns;  // suspend-time hint of the epilogue's and the MMA thread's long waits (0: plain polling)
   unsigned wait_limit_us; // > 0: every pipeline wait is bounded by this time instead of a poll count (fused reduce + GEMM)
+  EpiParams e;            // output, epilogue operands, split-K
 };
 
 // The fused all-gather variant (GATHER = true) adds the gather warps and the flag checker of gather.cuh;
@@ -60,10 +56,12 @@ struct GemmParams {
 // REDUCE (with GATHER): the gathered operand is A, and it is the SUM over ranks of a region of their gradient
 // buffers (reduce_chunks in gather.cuh): the gradient reduce-scatter with ownership by tensor, fused into the GEMM
 // that consumes the reduced gradient (OSFT factor gradients).
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false>
+// GROUP: one launch over the expert slabs of a mixture-of-experts layer (gemm_epilogue.cuh).
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE>
 __global__ void __launch_bounds__(GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p,
-            const __grid_constant__ GatherParams g) {
+            const __grid_constant__ GatherParams g, GroupParams gr) {
+  __shared__ GroupTable gtab;   // unused (and not allocated) outside the grouped forms
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -79,6 +77,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
   const int kblocks = (p.K + BK - 1) / BK;
+  const int splits = (GATHER || GROUP) ? 1 : p.e.splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -90,11 +89,30 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tma_prefetch_desc(&tmap_b);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (GROUP && warp == 2) fill_group_table<GROUP>(gtab, gr, BM, tiles_n, num_tiles, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  // item = split * num_tiles + tile: neighbours share operand tiles
+  const int num_items = GROUP ? gtab.tile_start[gr.E] : num_tiles * splits;
+  // The grouped forms walk the experts with the items: `e` only moves forward.
+  auto group_coords = [&](int w, int& e, int& tm, int& tn) {
+    while (w >= gtab.tile_start[e + 1]) ++e;
+    const int rows_m = GROUP == GROUP_ROWS ? (gtab.rows[e] + BM - 1) / BM : tiles_m;
+    const int t = w - gtab.tile_start[e];
+    const int band = t / (p.group_m * tiles_n);
+    const int first_m = band * p.group_m;
+    const int rows = min(p.group_m, rows_m - first_m);
+    const int local = t - band * p.group_m * tiles_n;
+    tm = first_m + local % rows;
+    tn = local / rows;
+  };
+  auto k_range = [&](int split, int& kb0, int& kb1) {
+    kb0 = static_cast<int>(static_cast<long long>(kblocks) * split / splits);
+    kb1 = static_cast<int>(static_cast<long long>(kblocks) * (split + 1) / splits);
+  };
   auto tile_coords = [&](int t, int& tm, int& tn) {
     if constexpr (GATHER && !REDUCE) {
       // Bands of GROUP_N column-tiles, all row-tiles inside a band: the weight is consumed front to
@@ -121,16 +139,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     if (elect_one()) {
       uint32_t it = 0, tl = 0;
       unsigned long long waited_ns = 0;
-      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) {
-        int tm, tn;
-        tile_coords(t, tm, tn);
+      int e = 0;
+      for (int w = blockIdx.x; w < num_items; w += gridDim.x) {
+        int tm, tn, kb0, kb1;
+        if constexpr (GROUP != GROUP_NONE) {
+          group_coords(w, e, tm, tn);
+          kb0 = 0;
+          kb1 = GROUP == GROUP_REDUCE ? (gtab.rows[e] + BK - 1) / BK : kblocks;
+        } else {
+          tile_coords(w % num_tiles, tm, tn);
+          k_range(w / num_tiles, kb0, kb1);
+        }
+        const int a_row = GROUP == GROUP_ROWS ? gtab.row[e] + tm * BM : tm * BM;   // first row of the A tile
+        const int k_row = GROUP == GROUP_REDUCE ? gtab.row[e] : 0;                 // first row of the reduction
         if (GATHER) {
           // the checker warp has seen the flags of every chunk under this tile's B rows
           if (!wait_verified(verified, tl, abort_flag, waited_ns, p.wait_limit_us)) { *abort_flag = 1; atomicExch(p.status, 5); goto done; }
           asm volatile("fence.proxy.async;" ::: "memory");   // peer data was written with ordinary stores, TMA reads it
           ++tl;
         }
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag, 0, p.wait_limit_us)) { atomicExch(p.status, 1); goto done; }
@@ -139,15 +167,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
           if (A_MN) {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, &tmap_a, &full_bar[s], tm * BM + j * 64, kb * BK);
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d(sa + j * 8192, &tmap_a, &full_bar[s], a_row + j * 64, k_row + kb * BK);
           } else {
-            tma_load_2d(sa, &tmap_a, &full_bar[s], kb * BK, tm * BM);
+            tma_load_2d(sa, &tmap_a, &full_bar[s], kb * BK, a_row);
           }
           if (B_MN) {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[s], tn * BN + j * 64, kb * BK);
+            for (int j = 0; j < BN / 64; ++j) {
+              if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb + j * 8192, &tmap_b, &full_bar[s], tn * BN + j * 64, kb * BK, e);
+              else tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[s], tn * BN + j * 64, k_row + kb * BK);
+            }
           } else {
-            tma_load_2d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN);
+            if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN, e);
+            else tma_load_2d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN);
           }
         }
       }
@@ -161,13 +193,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
       uint32_t it = 0, tl = 0;
-      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tl) {
+      int e = 0;
+      for (int w = blockIdx.x; w < num_items; w += gridDim.x, ++tl) {
+        int kb0, kb1;
+        if constexpr (GROUP != GROUP_NONE) {
+          while (w >= gtab.tile_start[e + 1]) ++e;
+          kb0 = 0;
+          kb1 = GROUP == GROUP_REDUCE ? (gtab.rows[e] + BK - 1) / BK : kblocks;
+        } else {
+          k_range(w / num_tiles, kb0, kb1);
+        }
         const int acc = tl & 1;
         const uint32_t aph = (tl >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], aph ^ 1, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 2); goto done; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < kblocks; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&full_bar[s], ph, abort_flag, 0, p.wait_limit_us)) { atomicExch(p.status, 3); goto done; }
@@ -178,7 +219,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t da = A_MN ? make_smem_desc(sa + k * 2048, 8192, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
             const uint64_t db = B_MN ? make_smem_desc(sb + k * 2048, 8192, 1024) : make_smem_desc(sb + k * 32, 16, 1024);
-            umma_bf16(d_tmem, da, db, idesc, (kb | k) != 0);
+            umma_bf16(d_tmem, da, db, idesc, kb != kb0 || k != 0);
           }
           umma_commit(&empty_bar[s]);   // frees the stage when these MMAs have read it
         }
@@ -213,70 +254,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     // ------------------------------------------------------------------ epilogue (warps 2..5)
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t tl = 0;
-    for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tl) {
-      int tm, tn;
-      tile_coords(t, tm, tn);
+    int e = 0;
+    EpiParams ep = p.e;
+    for (int w = blockIdx.x; w < num_items; w += gridDim.x, ++tl) {
+      const int t = w % num_tiles;
+      int tm, tn, row0;
+      if constexpr (GROUP != GROUP_NONE) group_coords(w, e, tm, tn); else tile_coords(t, tm, tn);
+      row0 = tm * BM;
+      if constexpr (GROUP == GROUP_ROWS) row0 += gtab.row[e];   // slabs are padded to whole tiles: every row may be stored
+      if constexpr (GROUP == GROUP_REDUCE) ep.D = reinterpret_cast<unsigned char*>(p.e.D) + e * gr.d_stride * (OUT_F32 ? 4 : 2);
       const int acc = tl & 1;
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 4); goto done; }
       tc_fence_after();
-      const int row = tm * BM + q * 32 + lane;
-      const bool row_ok = row < p.M;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        const int col0 = tn * BN + c * 32;
-        if (col0 >= p.N) break;  // uniform across the warp
-        uint32_t v[32];
-        tmem_ld_32x32(taddr + c * 32, v);
-        tmem_ld_wait();
-        if (row_ok) {
-          float f[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]) * p.alpha;
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col0 + j < p.N) {
-                const uint4 b = *reinterpret_cast<const uint4*>(p.bias + col0 + j);
-                const float2 b0 = unpack_bf16(b.x), b1 = unpack_bf16(b.y), b2 = unpack_bf16(b.z), b3 = unpack_bf16(b.w);
-                f[j] += b0.x; f[j + 1] += b0.y; f[j + 2] += b1.x; f[j + 3] += b1.y;
-                f[j + 4] += b2.x; f[j + 5] += b2.y; f[j + 6] += b3.x; f[j + 7] += b3.y;
-              }
-            }
-          }
-          if (OUT_F32) {
-            float* dptr = reinterpret_cast<float*>(p.D) + static_cast<long long>(row) * p.ldd + col0;
-            const float* rptr = p.R ? reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0 : nullptr;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (col0 + j < p.N) {
-                float4 o = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
-                if (rptr) { const float4 r = *reinterpret_cast<const float4*>(rptr + j); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
-                *reinterpret_cast<float4*>(dptr + j) = o;
-              }
-            }
-          } else {
-            __nv_bfloat16* dptr = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(row) * p.ldd + col0;
-            const __nv_bfloat16* rptr = p.R ? reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0 : nullptr;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col0 + j < p.N) {
-                if (rptr) {
-                  const uint4 r = *reinterpret_cast<const uint4*>(rptr + j);
-                  const float2 r0 = unpack_bf16(r.x), r1 = unpack_bf16(r.y), r2 = unpack_bf16(r.z), r3 = unpack_bf16(r.w);
-                  f[j] += r0.x; f[j + 1] += r0.y; f[j + 2] += r1.x; f[j + 3] += r1.y;
-                  f[j + 4] += r2.x; f[j + 5] += r2.y; f[j + 6] += r3.x; f[j + 7] += r3.y;
-                }
-                uint4 o;
-                o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
-                o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
-                *reinterpret_cast<uint4*>(dptr + j) = o;
-              }
-            }
-          }
-        }
-      }
+      if (GROUP == GROUP_REDUCE && gtab.rows[e] == 0)   // nothing was multiplied: the accumulator holds an older tile
+        epilogue_zero<OUT_F32>(ep, row0, tn * BN, q, lane);
+      else
+        epilogue_quarter<OUT_F32, !GATHER && !GROUP>(ep, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
+                                                     w / num_tiles);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
@@ -344,6 +339,22 @@ int make_tmap_2d_f32(CUtensorMap* out, const void* base, uint64_t inner, uint64_
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// 3-D bf16 tensor map over `n` row-major [outer, inner] matrices, `stride` elements from one to the next.
+int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t n, uint64_t stride,
+                      uint32_t box_inner, uint32_t box_outer) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || inner % 8 || stride % 8) return -2;
+  cuuint64_t dims[3] = {inner, outer, n};
+  cuuint64_t strides[2] = {inner * 2, stride * 2};
+  cuuint32_t box[3] = {box_inner, box_outer, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 static int g_num_sms = 0;
 
 // Tuning knobs read once from the environment (experiments; the defaults are what ships).
@@ -363,11 +374,11 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
                   const void* w, int* status, const GatherParams& g, cudaStream_t stream);
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, cudaStream_t stream,
-                  const GatherParams* gp = nullptr) {
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE>
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream,
+                  const GatherParams* gp = nullptr, long long ws_bytes = 0, const GroupParams* grp = nullptr) {
   static bool configured = false;
-  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE>;
+  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess) return -4;
     configured = true;
@@ -377,11 +388,19 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  const int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  if (GROUP == GROUP_REDUCE) tiles *= grp->E;
+  // The arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest.
+  if (!GATHER && !GROUP && p.e.ws != nullptr && tiles * 4 * 4 <= SPLIT_COUNTER_BYTES) {
+    p.e.counters = reinterpret_cast<unsigned*>(p.e.ws);
+    p.e.ws += SPLIT_COUNTER_BYTES / 4;
+    p.e.splits = choose_splits(tiles, (p.K + BK - 1) / BK, g_num_sms, (ws_bytes - SPLIT_COUNTER_BYTES) / (SPLIT_UNIT * 4));
+  }
   // the gathering variant always uses every SM: its extra warps carry the transfer
-  const int grid = (GATHER || tiles >= g_num_sms) ? g_num_sms : tiles;
+  const int items = tiles * p.e.splits;
+  const int grid = (GATHER || items >= g_num_sms) ? g_num_sms : items;
   static const GatherParams none{};
-  kern<<<grid, GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, p, gp ? *gp : none);
+  kern<<<grid, GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, p, gp ? *gp : none, grp ? *grp : GroupParams{});
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -393,10 +412,12 @@ extern "C" {
 //   a_mn = 0: A is row-major [M, K] (lda >= K);  a_mn = 1: A is row-major [K, M] (lda >= M)
 //   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
 //   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
+//   ws: optional fp32 workspace of ws_bytes for split-K (null: never split); its first SPLIT_COUNTER_BYTES are zero
+//   before the first call, every launch leaves them zero again, and launches that may overlap have one each
 // Returns 0 on success, a negative code on invalid arguments or launch failure.
 int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                     float alpha, int* status, cudaStream_t stream) {
+                     float alpha, float* ws, long long ws_bytes, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || ldd % 8 || (R && ldr % 8)) return -10;
@@ -408,18 +429,46 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc - 10;
-  GemmParams p{M, N, K, D, ldd, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), status, alpha, tune_group_m(), tune_wait_hint(), 0u};
+  GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
+               EpiParams{M, N, D, ldd, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, nullptr}};
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
-    case 0: return launch<false, false, false>(ta, tb, p, stream);
-    case 1: return launch<false, false, true>(ta, tb, p, stream);
-    case 2: return launch<false, true, false>(ta, tb, p, stream);
-    case 3: return launch<false, true, true>(ta, tb, p, stream);
-    case 4: return launch<true, false, false>(ta, tb, p, stream);
-    case 5: return launch<true, false, true>(ta, tb, p, stream);
-    case 6: return launch<true, true, false>(ta, tb, p, stream);
-    default: return launch<true, true, true>(ta, tb, p, stream);
+    case 0: return launch<false, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 1: return launch<false, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 2: return launch<false, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 3: return launch<false, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 4: return launch<true, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 5: return launch<true, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 6: return launch<true, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
+    default: return launch<true, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
   }
+}
+
+// Grouped GEMM over expert slabs (see gemm_epilogue.cuh); starts [E + 1] and counts [E] are device arrays, `rows` is the
+// height of the row buffers.
+//   mode 0  D[rows, N] = A[rows, K] * W_e[N, K]^T        W: E matrices [N, K], w_stride elements apart
+//   mode 1  D[rows, N] = A[rows, K] * W_e[K, N]          W: E matrices [K, N], w_stride elements apart
+//   mode 2  W_e[M, N] = A[rows_e, M]^T * B[rows_e, N]    D is W here: E outputs, w_stride elements apart; K is ignored
+int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long ldb, void* D, long long ldd, int mode, int rows,
+                        int M, int N, int K, const int* starts, const int* counts, int E, long long w_stride, int* status,
+                        cudaStream_t stream) {
+  using namespace mtb;
+  if (E <= 0 || rows <= 0 || N <= 0 || (mode == 2 ? M : K) <= 0) return 0;
+  if (E > GROUP_MAX || N % 8 || ldd % 8 || rows % GROUP_ALIGN || w_stride % 8 || mode < 0 || mode > 2) return -10;
+  CUtensorMap ta, tb;
+  int rc = mode == 2 ? make_tmap_2d_bf16(&ta, A, M, rows, lda, 64, 64) : make_tmap_2d_bf16(&ta, A, K, rows, lda, BK, BM);
+  if (rc) return rc;
+  if (mode == 0) rc = make_tmap_3d_bf16(&tb, B, K, N, E, w_stride, BK, BN);
+  else if (mode == 1) rc = make_tmap_3d_bf16(&tb, B, N, K, E, w_stride, 64, 64);
+  else rc = make_tmap_2d_bf16(&tb, B, N, rows, ldb, 64, 64);
+  if (rc) return rc - 10;
+  const int out_rows = mode == 2 ? M : rows;
+  GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
+               EpiParams{out_rows, N, D, ldd, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr}};
+  GroupParams g{starts, counts, E, w_stride};
+  if (mode == 0) return launch<false, false, false, false, false, GROUP_ROWS>(ta, tb, p, stream, nullptr, 0, &g);
+  if (mode == 1) return launch<false, true, false, false, false, GROUP_ROWS>(ta, tb, p, stream, nullptr, 0, &g);
+  return launch<true, true, false, false, false, GROUP_REDUCE>(ta, tb, p, stream, nullptr, 0, &g);
 }
 
 // Fused all-gather + GEMM:  D[M,N] = A[M,K] * W[N,K]^T (+bias) with W living in `full`, the local
@@ -446,7 +495,8 @@ int mtb200_gemm_bf16_allgather(const void* A, long long lda, void* D, long long 
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, reinterpret_cast<const unsigned char*>(full) + w_byte_off, K, N, K, BK, BN);
   if (rc) return rc - 10;
-  GemmParams p{M, N, K, D, ldd, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), status, 1.0f, tune_group_m(), tune_wait_hint(), 0u};
+  GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
+               EpiParams{M, N, D, ldd, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr}};
   GatherParams g{};
   for (int i = 0; i < world; ++i) g.peer_base[i] = bases[i];
   g.shard_off = shard_off; g.shard_bytes = shard_bytes; g.dst = reinterpret_cast<unsigned char*>(full);
@@ -485,7 +535,8 @@ int mtb200_gemm_bf16_reduce_a(void* dst, const void* B, long long ldb, float* D,
   if (rc) return rc - 10;
   // every pipeline wait sits out the peers' skew: a little longer than the bound of the ready-flag wait itself
   const unsigned lim = limit_us ? limit_us : FLAG_SPIN_LIMIT;
-  GemmParams p{M, N, K, D, ldd, R, ldr, nullptr, status, 1.0f, tune_group_m(), tune_wait_hint(), lim + lim / 2 + 10000000u};
+  GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), lim + lim / 2 + 10000000u,
+               EpiParams{M, N, D, ldd, R, ldr, nullptr, 1.0f, 1, nullptr, nullptr}};
   GatherParams g{};
   for (int i = 0; i < world; ++i) g.peer_base[i] = bases[i];
   g.dst = reinterpret_cast<unsigned char*>(dst);

@@ -7,12 +7,12 @@ router logits in the compute dtype, softmax in fp32, top-k, weights renormalised
 experts (optional for Qwen3-MoE), each expert a SwiGLU MLP, outputs combined with the weights. No auxiliary load-balancing loss (transformers only adds one with
 ``output_router_logits``; a config that asks for it is refused at load time).
 
-Schedule: the (token, slot) pairs are sorted by expert once per block, so every expert sees one
-contiguous slab of gathered rows and its three projections are plain GEMMs on row slices of shared
-buffers (the same tcgen05 kernel as the dense model; slabs of any height, empty ones skipped).
-The slab boundaries are the one device-to-host read of a block. Contributions of a token's
-experts are put back in token order by the inverse permutation and summed in fp32, so forward and
-backward are deterministic (no atomics).
+Schedule on the kernels: the (token, slot) pairs are grouped by expert on the device into slabs of shared row
+buffers, so the experts' projections are one grouped tcgen05 GEMM per product, forward and backward, however many
+experts there are and however unevenly they are used; nothing is read back to the host. Any other backend, and
+weights that do not sit at equal distances in memory, take the loop over experts: sorted pairs, one plain GEMM per
+slab and product, the slab boundaries being the block's one device-to-host read. Either way a token's experts are
+summed in fp32 in slot order, so forward and backward are deterministic (no atomics).
 """
 from __future__ import annotations
 
@@ -28,31 +28,44 @@ class MoeState:
     probs: torch.Tensor          # [T, E] fp32 softmax of the router logits
     topi: torch.Tensor           # [T, k] experts chosen per token
     w: torch.Tensor              # [T, k] fp32 weights, renormalised over the chosen experts
-    order: torch.Tensor          # [T*k] routed row -> index of its (token, slot) pair, grouped by expert
-    tok: torch.Tensor            # [T*k] token of each routed row
-    bounds: list                 # E+1 host ints: routed rows [bounds[e], bounds[e+1]) belong to expert e
-    gu: torch.Tensor             # [T*k, 2F] gate/up pre-activations of the routed rows
+    order: Optional[torch.Tensor]   # [T*k] routed row -> index of its (token, slot) pair, grouped by expert
+    tok: Optional[torch.Tensor]  # [T*k] token of each routed row
+    bounds: Optional[list]       # E+1 host ints: routed rows [bounds[e], bounds[e+1]) belong to expert e
+    gu: torch.Tensor             # [rows, 2F] gate/up pre-activations of the routed rows
     act: Optional[torch.Tensor]  # [T*k, F] SwiGLU output (None: rebuilt in backward)
     gu_s: Optional[torch.Tensor] = None    # [T, 2Fs] gate/up pre-activations of the shared expert (Qwen2-MoE)
     act_s: Optional[torch.Tensor] = None   # [T, Fs] its SwiGLU output (None: rebuilt in backward)
+    slabs: Optional[object] = None         # grouped path: the expert slabs; order, tok and bounds are None then
 
 
 def route(cfg, router_w: torch.Tensor, n2: torch.Tensor, topi: Optional[torch.Tensor] = None):
-    """Router of one block: ``(probs, topi, w, order, tok, bounds)``. With ``topi`` given, those experts
+    """Router of one block: ``(probs, topi, w)``. With ``topi`` given, those experts
     are used instead of the top-k while the weights still follow this call's logits (comparisons
     between backends of different precision, where a near-tie may otherwise select differently)."""
-    E, k = cfg.num_local_experts, cfg.num_experts_per_tok
+    k = cfg.num_experts_per_tok
     probs = torch.softmax((n2 @ router_w.t()).float(), dim=-1)
     if topi is None:
         topv, topi = torch.topk(probs, k, dim=-1)
     else:
         topv = probs.gather(1, topi)
     w = topv / topv.sum(-1, keepdim=True) if cfg.norm_topk_prob else topv
+    return probs, topi, w
+
+
+def _sort_by_expert(topi: torch.Tensor, E: int):
+    """``(order, tok, bounds)`` of the loop over experts (see ``MoeState``)."""
     flat = topi.reshape(-1)
     order = torch.argsort(flat, stable=True)
     bounds = [0] + torch.cumsum(torch.bincount(flat, minlength=E), 0).tolist()   # the block's one host read
-    tok = torch.div(order, k, rounding_mode="floor")
-    return probs, topi, w, order, tok, bounds
+    return order, torch.div(order, topi.shape[1], rounding_mode="floor"), bounds
+
+
+def _expert_stacks(ops, cfg, p: dict, x: torch.Tensor):
+    """The stacked gate/up and down matrices when the grouped kernels can run this layer, else ``None``."""
+    if not hasattr(ops, "expert_stack") or x.dtype != torch.bfloat16 or x.shape[0] == 0:
+        return None
+    wgu, wd = ops.expert_stack(p, "wgu", cfg.num_local_experts), ops.expert_stack(p, "wd", cfg.num_local_experts)
+    return None if wgu is None or wd is None else (wgu, wd)
 
 
 def _slabs(bounds: list):
@@ -72,7 +85,11 @@ def moe_forward(ops, cfg, p: dict, n2: torch.Tensor, h1: torch.Tensor, need_out:
     (a recompute inside backward stops after the gate/up projections)."""
     T, H = n2.shape
     k, fe = cfg.num_experts_per_tok, cfg.expert_intermediate_size
-    probs, topi, w, order, tok, bounds = route(cfg, p["router"], n2)
+    probs, topi, w = route(cfg, p["router"], n2)
+    stacks = _expert_stacks(ops, cfg, p, n2)
+    if stacks is not None:
+        return _grouped_forward(ops, cfg, p, n2, h1, need_out, keep_act, probs, topi, w, *stacks)
+    order, tok, bounds = _sort_by_expert(topi, cfg.num_local_experts)
     xs = ops.embedding(n2, tok)                       # rows gathered expert by expert
     gu = torch.empty(T * k, 2 * fe, dtype=n2.dtype, device=n2.device)
     for e, a, b in _slabs(bounds):
@@ -104,15 +121,63 @@ def moe_forward(ops, cfg, p: dict, n2: torch.Tensor, h1: torch.Tensor, need_out:
     return (h1.float() + cfg.residual_multiplier * y).to(h1.dtype), st
 
 
+def _grouped_forward(ops, cfg, p: dict, n2, h1, need_out: bool, keep_act: bool, probs, topi, w, wgu, wd):
+    """``moe_forward`` on the grouped kernels. The activation is never kept: backward's gradient kernel rebuilds it in the
+    pass over gate/up that it makes anyway."""
+    sl = ops.expert_slabs(topi, cfg.num_local_experts)
+    gu = ops.grouped_linear(ops.gather_rows(n2, sl), wgu, sl)
+    st = MoeState(probs, topi, w.contiguous(), None, None, None, gu, None, slabs=sl)
+    add = None
+    if "wgus" in p:
+        st.gu_s = ops.linear(n2, p["wgus"])
+    if not need_out:
+        return None, st
+    yr = ops.grouped_linear(ops.swiglu(gu, cfg.mlp_act), wd, sl)
+    if "wgus" in p:
+        act_s = ops.swiglu(st.gu_s, cfg.mlp_act)
+        add = torch.sigmoid((n2 @ p["wsg"].t()).float()) * ops.linear(act_s, p["wds"]).float()
+        st.act_s = act_s if keep_act else None
+    return ops.combine_rows(yr, sl, h1, w=st.w, add=add, scale=cfg.residual_multiplier), st
+
+
+def _grouped_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor, dout: torch.Tensor, wgu, wd, dwgu, dwd) -> torch.Tensor:
+    sl = st.slabs
+    gr = ops.gather_rows(dout, sl, cfg.residual_multiplier)
+    du = ops.grouped_dgrad(gr, wd, sl)
+    dgu, wact, dw = ops.expert_glu_bwd(du, st.gu, st.w, sl, cfg.mlp_act)
+    ops.grouped_wgrad(gr, wact, dwd, sl)
+    del gr, du, wact
+    dxs = ops.grouped_dgrad(dgu, wgu, sl)
+    ops.grouped_wgrad(dgu, ops.gather_rows(n2, sl), dwgu, sl)
+    del dgu
+    add = None
+    if "wgus" in p:
+        add = torch.zeros(n2.shape, dtype=torch.float32, device=n2.device)
+        _shared_backward(ops, cfg, p, g, st, n2, dout, add)
+    dlogits = ops.route_bwd(st.probs, st.topi, st.w, dw, cfg.norm_topk_prob, n2.dtype)
+    g["router"].copy_(dlogits.t() @ n2)
+    return ops.combine_rows(dxs, sl, dlogits @ p["router"], add=add)
+
+
 def moe_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor, dout: torch.Tensor) -> torch.Tensor:
     """Writes the gradients of the router and of every expert into ``g`` and returns the gradient of
     ``n2`` (the normalised MLP input). ``dout`` is the gradient of the block output.
 
-    Everything between the gathered output gradient and the gathered input gradient runs slab by slab, so the
-    intermediates (activation, its gradient, the gate/up gradient) only ever exist for one expert's rows."""
+    In the loop over experts everything between the gathered output gradient and the gathered input gradient runs slab by
+    slab, so the intermediates (activation, its gradient, the gate/up gradient) only ever exist for one expert's rows."""
     T, H = n2.shape
     k = cfg.num_experts_per_tok
     rm = cfg.residual_multiplier
+    if st.slabs is not None:
+        E = cfg.num_local_experts
+        stacks = {n: (ops.expert_stack(p, n, E), ops.expert_stack(g, n, E)) for n in ("wgu", "wd")}
+        loose = {n: torch.empty(E, *p[f"{n}0"].shape, dtype=n2.dtype, device=n2.device) for n, s in stacks.items() if s[1] is None}
+        grads = {n: (loose[n][0], loose[n][0].numel()) if n in loose else s[1] for n, s in stacks.items()}
+        dn2 = _grouped_backward(ops, cfg, p, g, st, n2, dout, stacks["wgu"][0], stacks["wd"][0], grads["wgu"], grads["wd"])
+        for n, stack in loose.items():   # gradient tensors that are not stacked like the weights
+            for e in range(E):
+                g[f"{n}{e}"].copy_(stack[e])
+        return dn2
     order, tok, bounds = st.order, st.tok, st.bounds
     gr = ops.embedding(dout, tok)                     # output gradient of every routed row, before its weight
     if rm != 1.0:
@@ -141,23 +206,8 @@ def moe_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor, dou
         del dgu
     dn2 = _combine(dxs, order, T, k)
     del xs, dxs, gr
-    if "wgus" in p:   # shared expert: y_s = sigmoid(n2 wsg^T) * MLP_s(n2)
-        act_s = st.act_s if st.act_s is not None else ops.swiglu(st.gu_s, cfg.mlp_act)
-        ys = ops.linear(act_s, p["wds"]).float()          # its output again: the gate's gradient needs it
-        sg = torch.sigmoid((n2 @ p["wsg"].t()).float())   # [T, 1]
-        df = dout.float() * rm
-        dz = ((df * ys).sum(-1, keepdim=True) * sg * (1 - sg)).to(n2.dtype)
-        g["wsg"].copy_(dz.t() @ n2)
-        dn2 += (dz @ p["wsg"]).float()
-        dys = (df * sg).to(n2.dtype)
-        del ys, df
-        dact_s = ops.linear_dgrad(dys, p["wds"])
-        ops.linear_wgrad(dys, act_s, g["wds"])
-        dgu_s = ops.swiglu_bwd(dact_s, st.gu_s, cfg.mlp_act)
-        del dact_s, act_s, dys
-        dn2 += ops.linear_dgrad(dgu_s, p["wgus"]).float()
-        ops.linear_wgrad(dgu_s, n2, g["wgus"])
-        del dgu_s
+    if "wgus" in p:
+        _shared_backward(ops, cfg, p, g, st, n2, dout, dn2)
     # router: weights -> renormalisation -> top-k selection -> softmax -> logits
     dw = torch.empty(T * k, dtype=torch.float32, device=n2.device)
     dw[order] = dwr
@@ -172,3 +222,24 @@ def moe_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor, dou
     g["router"].copy_(dlogits.t() @ n2)
     dn2 += (dlogits @ p["router"]).float()
     return dn2.to(n2.dtype)
+
+
+def _shared_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor, dout: torch.Tensor, dn2: torch.Tensor) -> None:
+    """Shared expert, y_s = sigmoid(n2 wsg^T) * MLP_s(n2): its gradients into ``g``, its input gradient added to the fp32 ``dn2``."""
+    rm = cfg.residual_multiplier
+    act_s = st.act_s if st.act_s is not None else ops.swiglu(st.gu_s, cfg.mlp_act)
+    ys = ops.linear(act_s, p["wds"]).float()          # its output again: the gate's gradient needs it
+    sg = torch.sigmoid((n2 @ p["wsg"].t()).float())   # [T, 1]
+    df = dout.float() * rm
+    dz = ((df * ys).sum(-1, keepdim=True) * sg * (1 - sg)).to(n2.dtype)
+    g["wsg"].copy_(dz.t() @ n2)
+    dn2 += (dz @ p["wsg"]).float()
+    dys = (df * sg).to(n2.dtype)
+    del ys, df
+    dact_s = ops.linear_dgrad(dys, p["wds"])
+    ops.linear_wgrad(dys, act_s, g["wds"])
+    dgu_s = ops.swiglu_bwd(dact_s, st.gu_s, cfg.mlp_act)
+    del dact_s, act_s, dys
+    dn2 += ops.linear_dgrad(dgu_s, p["wgus"]).float()
+    ops.linear_wgrad(dgu_s, n2, g["wgus"])
+    del dgu_s

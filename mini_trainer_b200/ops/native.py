@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+from dataclasses import dataclass
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
@@ -43,8 +44,8 @@ P, I, L, F = c_void_p, c_int, c_longlong, c_float
 
 
 class _Sig:
-    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, P]
-    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, P]
+    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P]
+    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P]
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P]
     mtb200_rmsnorm_bwd_blocks = [I]
     mtb200_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, I, P]
@@ -70,12 +71,33 @@ class _Sig:
     mtb200_f32_to_bf16 = [P, P, L, I, P]
     mtb200_sumsq = [P, L, P, P]
     mtb200_adamw = [P, P, P, I, P, P, L, F, F, F, F, F, I, P, P]
+    mtb200_gemm_grouped = [P, L, P, L, P, L, I, I, I, I, I, P, P, I, L, P, P]
+    mtb200_moe_plan = [P, I, I, I, P, P, P, P, P, P]
+    mtb200_moe_gather = [P, P, P, I, I, I, I, F, P, P]
+    mtb200_moe_glu_bwd = [P, P, P, P, P, I, I, I, I, P, P, P]
+    mtb200_moe_combine = [P, P, P, P, P, F, I, I, I, P, P]
+    mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
     mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, F, P, P]
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
 NATIVE_HEAD_DIMS = (64, 128)   # head dimensions of the hand-written attention kernels
+
+
+_GROUP_ALIGN = 128   # GROUP_ALIGN and GROUP_MAX of csrc/gemm_epilogue.cuh
+_GROUP_MAX = 256
+
+
+@dataclass
+class ExpertSlabs:
+    """Rows of a mixture-of-experts layer grouped by expert (see csrc/moe.cu); all on the device."""
+    starts: torch.Tensor    # [E + 1] int32 first row of each expert's slab
+    counts: torch.Tensor    # [E] int32 rows of each expert
+    pair_of: torch.Tensor   # [cap] int32 (token, slot) pair of a row, -1 in padding
+    row_of: torch.Tensor    # [T * k] int32 row of a pair
+    cap: int                # height of the row buffers
+    k: int                  # experts per token
 
 
 def _ptr(t):
@@ -161,7 +183,8 @@ class NativeOps:
         code = int(self.status.item())
         if code:
             self.status.zero_()
-            what = {60: "a token id outside the embedding table", 61: "an attention work item outside the packed batch"}.get(
+            what = {60: "a token id outside the embedding table", 61: "an attention work item outside the packed batch",
+                    62: "a chosen expert outside the model's experts"}.get(
                 code, "a device-side bounded wait expired")
             raise RuntimeError(f"{what} (status code {code})")
 
@@ -174,10 +197,11 @@ class NativeOps:
         assert residual is None or residual.dtype == out.dtype
         if two_cta is None:
             two_cta = self.use_gemm2 and (-(-M // 256)) * (-(-N // 256)) >= 64
+        st = self._st()
         self._call("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
                    residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha),
-                   self.status.data_ptr(), self._st(), tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
+                   None, 0, self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
         return out
 
     # -- embedding --------------------------------------------------------------------
@@ -300,7 +324,7 @@ class NativeOps:
     # -- attention --------------------------------------------------------------------
     def _attn_plan(self, cu_host, block, most_work_last_block: bool):
         """Work table for the attention kernels: one row (seq_start, seq_len, block_start) per
-        128-row block of every sequence, most work first (forward: late query blocks see the most
+        ``block`` rows of every sequence, most work first (forward: late query blocks see the most
         keys; backward: early key blocks are seen by the most queries). Built once per minibatch
         and reused by every layer."""
         key = (id(cu_host), block, most_work_last_block)
@@ -397,6 +421,92 @@ class NativeOps:
         dgu = torch.empty_like(gate_up)
         self._call(_GLU[act] + "_bwd_act", dact.data_ptr(), gate_up.data_ptr(), dgu.data_ptr(), T, F2 // 2, self._st())
         return dgu, dact
+
+    # -- mixture of experts: grouped projections over expert slabs ----------------------------
+    @staticmethod
+    def expert_stack(p: dict, name: str, E: int):
+        """``(first matrix, elements between two experts)`` when the matrices ``name0 .. name{E-1}`` of ``p`` sit at equal
+        distances in memory, as in a block's flat buffer; ``None`` when one grouped launch cannot address them."""
+        ws = [p[f"{name}{e}"] for e in range(E)]
+        a = ws[0]
+        if E > _GROUP_MAX or any(w.dtype != torch.bfloat16 or not w.is_contiguous() or w.shape != a.shape for w in ws) \
+                or a.data_ptr() % 16 or a.shape[0] % 8 or a.shape[1] % 8:
+            return None
+        step = ws[1].data_ptr() - a.data_ptr() if E > 1 else a.numel() * 2
+        if step <= 0 or step % 16 or any(w.data_ptr() - a.data_ptr() != e * step for e, w in enumerate(ws)):
+            return None
+        return a, step // 2
+
+    def expert_slabs(self, topi, E: int) -> ExpertSlabs:
+        """Groups the (token, slot) pairs of ``topi`` [T, k] by expert. No host read: the buffers are sized for the worst case."""
+        T, k = topi.shape
+        n = T * k
+        cap = -(-(n + E * (_GROUP_ALIGN - 1)) // _GROUP_ALIGN) * _GROUP_ALIGN
+        buf = torch.empty(2 * E + 1 + cap + n, dtype=torch.int32, device=self.device)
+        starts, counts, pair_of, row_of = buf.split([E + 1, E, cap, n])
+        topi = topi.contiguous()
+        self._call("mtb200_moe_plan", topi.data_ptr(), n, E, cap, starts.data_ptr(), counts.data_ptr(), pair_of.data_ptr(),
+                   row_of.data_ptr(), self.status.data_ptr(), self._st())
+        return ExpertSlabs(starts, counts, pair_of, row_of, cap, k)
+
+    def gather_rows(self, src, sl: ExpertSlabs, scale: float = 1.0):
+        """Rows of ``src`` [T, H] in slab order, zeros between the slabs."""
+        H = src.shape[1]
+        out = torch.empty(sl.cap, H, dtype=src.dtype, device=self.device)
+        self._call("mtb200_moe_gather", src.contiguous().data_ptr(), sl.pair_of.data_ptr(), sl.starts.data_ptr(), sl.counts.shape[0], sl.k,
+                   sl.cap, H, float(scale), out.data_ptr(), self._st())
+        return out
+
+    def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride):
+        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, mode, sl.cap, M, N, K,
+                   sl.starts.data_ptr(), sl.counts.data_ptr(), sl.counts.shape[0], stride, self.status.data_ptr(), self._st(),
+                   tag="gemm_grouped_" + ("nt", "nn", "tn")[mode])
+        return out
+
+    def grouped_linear(self, x, stack, sl: ExpertSlabs):
+        """``x_e @ W_e.T`` for every slab; ``stack``: see ``expert_stack``, matrices ``[N, K]``."""
+        w, stride = stack
+        N, K = w.shape
+        out = torch.empty(sl.cap, N, dtype=x.dtype, device=self.device)
+        return self._grouped(0, x, w, K, out, N, sl, sl.cap, N, K, stride)
+
+    def grouped_dgrad(self, dy, stack, sl: ExpertSlabs):
+        """``dy_e @ W_e`` for every slab."""
+        w, stride = stack
+        N, K = w.shape
+        out = torch.empty(sl.cap, K, dtype=dy.dtype, device=self.device)
+        return self._grouped(1, dy, w, K, out, K, sl, sl.cap, K, N, stride)
+
+    def grouped_wgrad(self, dy, x, stack, sl: ExpertSlabs):
+        """``dW_e = dy_e.T @ x_e`` into the stacked gradient matrices; zeros for an expert without rows."""
+        g, stride = stack
+        N, K = g.shape
+        self._grouped(2, dy, x, x.stride(0), g, K, sl, N, K, 0, stride)
+
+    def expert_glu_bwd(self, du, gu, w, sl: ExpertSlabs, act="silu"):
+        """``(dgu, weighted activation (over du), dw)`` from ``du``, the gradient of the activation before the expert weight."""
+        F = du.shape[1]
+        dgu = torch.empty_like(gu)
+        dw = torch.zeros_like(w)
+        self._call("mtb200_moe_glu_bwd", du.data_ptr(), gu.data_ptr(), w.data_ptr(), sl.pair_of.data_ptr(), sl.starts.data_ptr(),
+                   sl.counts.shape[0], sl.cap, F, int(act != "silu"), dgu.data_ptr(), dw.data_ptr(), self._st())
+        return dgu, du, dw
+
+    def combine_rows(self, rows, sl: ExpertSlabs, base, w=None, add=None, scale=1.0):
+        """``base + scale * (sum over a token's slots of w * row + add)``, summed in fp32; ``w`` [T, k] and ``add`` [T, H] fp32."""
+        T, H = base.shape
+        out = torch.empty_like(base)
+        self._call("mtb200_moe_combine", rows.data_ptr(), sl.row_of.data_ptr(), _ptr(w), _ptr(add), base.contiguous().data_ptr(), float(scale), T,
+                   sl.k, H, out.data_ptr(), self._st())
+        return out
+
+    def route_bwd(self, probs, topi, w, dw, renorm: bool, dtype):
+        """Gradient of the router logits ``[T, E]``."""
+        T, E = probs.shape
+        out = torch.empty(T, E, dtype=dtype, device=self.device)
+        self._call("mtb200_moe_route_bwd", probs.data_ptr(), topi.data_ptr(), w.data_ptr(), dw.data_ptr(), int(renorm), T, E, topi.shape[1],
+                   out.data_ptr(), self._st())
+        return out
 
     # -- plain GELU (tanh approximation) of a not gated MLP ----------------------------------
     def gelu(self, x):

@@ -511,3 +511,68 @@ def test_out_of_range_inputs_are_reported_not_dereferenced(ops):
         ops.check_status()
     ops.check_status()     # cleared; and the device still works
     assert torch.ones(8, device="cuda").sum().item() == 8
+
+
+def _moe_layer(T, H, F, E, k, popular, seed=0, act="silu"):
+    """A routed layer in one flat buffer: ``(cfg, p, g, n2, h1, dout)``; only the first ``popular`` experts are ever chosen."""
+    from mini_trainer_b200.models import layout as L
+    from mini_trainer_b200.models.config import ModelConfig
+    torch.manual_seed(seed)
+    cfg = ModelConfig(model_type="mixtral", vocab_size=64, hidden_size=H, intermediate_size=F, num_hidden_layers=1, num_attention_heads=1,
+                      num_key_value_heads=1, head_dim=64, num_local_experts=E, num_experts_per_tok=k,
+                      hidden_act="gelu_pytorch_tanh" if act != "silu" else "silu")
+    entries = [("router", (E, H))]
+    for e in range(E):
+        entries += [(f"wgu{e}", (2 * F, H)), (f"wd{e}", (H, F))]
+    lay = L.GroupLayout("x", entries, 1)
+    p = lay.views(bf(lay.padded_numel, scale=0.05))
+    g = lay.views(torch.full((lay.padded_numel,), float("nan"), dtype=torch.bfloat16, device="cuda"))
+    n2 = bf(T, H)
+    if popular < E:   # the other experts' logits lie far below
+        d = torch.randn(H, device="cuda")
+        d /= d.norm()
+        n2 = (n2.float() + 6 * d).bfloat16()
+        p["router"][popular:] = (p["router"][popular:].float() - 10 * d).bfloat16()
+    return cfg, p, g, n2, bf(T, H), bf(T, H)
+
+
+# one token; slabs of exactly one and two row tiles; sizes off every tile edge; idle experts; a reduction shorter than one k-block;
+# more experts than a warp has lanes
+@pytest.mark.parametrize("T,H,F,E,k,popular,act", [(1, 64, 72, 4, 2, 4, "silu"), (128, 128, 64, 2, 2, 2, "silu"), (256, 264, 200, 3, 1, 1, "silu"),
+                                                   (777, 520, 328, 8, 2, 5, "silu"), (300, 256, 136, 40, 8, 40, "gelu"),
+                                                   (2051, 512, 256, 64, 4, 33, "silu")])
+def test_grouped_experts_match_loop_over_experts(ops, T, H, F, E, k, popular, act):
+    from mini_trainer_b200.models import moe as M
+    cfg, p, g, n2, h1, dout = _moe_layer(T, H, F, E, k, popular, act=act)
+    assert ops.expert_stack(p, "wgu", E) is not None
+    loose = {n: w.clone() for n, w in p.items()}           # separate tensors: the loop over experts
+    gl = {n: torch.full_like(w, float("nan")) for n, w in loose.items()}
+    res = {}
+    try:
+        for name, pp, gg in (("grouped", p, g), ("loop", loose, gl)):
+            if name == "loop":
+                ops.expert_stack = lambda *a: None
+            out, st = M.moe_forward(ops, cfg, pp, n2, h1, True, False)
+            assert (st.slabs is not None) == (name == "grouped")
+            res[name] = (out, M.moe_backward(ops, cfg, pp, gg, st, n2, dout))
+    finally:
+        del ops.expert_stack
+    ops.check_status()
+    # same products in bf16; the loop rounds the weighted rows and the scaled gradients to bf16 where the kernels do not
+    for a, b in zip(res["grouped"], res["loop"]):
+        assert rel_err(a, b) < 1e-2
+    for n in p:
+        if gl[n].float().norm() == 0:
+            assert g[n].float().norm() == 0, n
+        else:
+            assert rel_err(g[n], gl[n]) < 1.5e-2, n
+    again = M.moe_forward(ops, cfg, p, n2, h1, True, False)
+    assert torch.equal(again[0], res["grouped"][0])
+    first = {n: w.clone() for n, w in g.items()}
+    dn2 = M.moe_backward(ops, cfg, p, g, again[1], n2, dout)
+    assert torch.equal(dn2, res["grouped"][1]) and all(torch.equal(first[n], g[n]) for n in g)
+    # gradients that are not stacked like the weights come out the same
+    gs = {n: torch.full_like(w, float("nan")) for n, w in p.items()}
+    gs["wgu0"] = torch.cat([gs["wgu0"].reshape(-1), gs["wgu0"].new_zeros(8)])[: gs["wgu0"].numel()].view_as(p["wgu0"])
+    M.moe_backward(ops, cfg, p, gs, again[1], n2, dout)
+    assert all(torch.equal(first[n], gs[n]) for n in gs)

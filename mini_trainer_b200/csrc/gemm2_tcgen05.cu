@@ -30,6 +30,7 @@ namespace mtb {
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer);
+int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32);
 
 namespace g2 {
 
@@ -44,7 +45,7 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 192;
 constexpr int GROUP_M = 8;               // band of 8 pair-tiles = 2048 rows
 constexpr int GATHER_GROUP_N = 4;        // column-tiles per band in the all-gather variant
-constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+constexpr int SMEM = STAGES * STAGE_BYTES + EPI_SMEM + 1024 + 256;
 constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;   // clears the CTA-rank bit of a shared::cluster address -> CTA 0
 
 struct Params {
@@ -88,11 +89,12 @@ __device__ __forceinline__ void mbar_arrive_cta0(uint64_t* bar) {
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS, 1)
-gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, Params p,
+gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+             const __grid_constant__ CUtensorMap tmap_d, Params p,
              const __grid_constant__ GatherParams g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + EPI_SMEM);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
@@ -118,6 +120,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    tma_prefetch_desc(&tmap_d);
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
@@ -251,6 +254,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   } else {
     // ------------------------------------------------------------------ epilogue (both CTAs)
     const int q = warp & 3;
+    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + q * 2 * STORE_BOX, -1, 0};
     uint32_t tl = 0;
     for (int w = pair; w < num_items; w += p.num_pairs, ++tl) {
       const int t = w % num_tiles;
@@ -260,14 +264,15 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag)) { atomicExch(p.status, 54); goto done; }
       tc_fence_after();
-      epilogue_quarter<OUT_F32, !GATHER>(p.e, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
-                                2 * t + static_cast<int>(rank), w / num_tiles);
+      epilogue_quarter<OUT_F32, !GATHER>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
+                                2 * t + static_cast<int>(rank), w / num_tiles, false);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cta0(&tempty_bar[acc]);
     }
   }
 done:
+  if (warp >= 2 && warp < 6 && lane == 0) drain_boxes();
   tc_fence_before();
   __syncthreads();
   cluster_sync();          // nobody tears down while the partner may still signal or read
@@ -280,7 +285,7 @@ done:
 static int g_pairs[2] = {-1, -1};   // clusters of two that can be co-resident (0: unsupported), plain / gather variant
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
                   long long ws_bytes = 0) {
   auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER>;
   constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS;
@@ -316,20 +321,22 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, Params p, cudaSt
   const int items = tiles * p.e.splits;
   p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
   static const GatherParams none{};
-  kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, p, gp ? *gp : none);
+  kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, p, gp ? *gp : none);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 // Fused all-gather + GEMM on CTA pairs; called by mtb200_gemm_bf16_allgather.
 int launch_gather(const void* A, long long lda, void* D, long long ldd, const void* bias, int M, int N, int K,
                   const void* w, int* status, const GatherParams& g, cudaStream_t stream) {
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   int rc = make_tmap_2d_bf16(&ta, A, K, M, lda, BK, BM);
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, w, K, N, K, BK, BNH);
   if (rc) return rc - 10;
-  Params p{M, N, K, status, 0, EpiParams{M, N, D, ldd, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr}};
-  return launch<false, false, false, true>(ta, tb, p, stream, &g);
+  rc = make_tmap_out(&td, D, M, N, ldd, 0);
+  if (rc) return rc - 20;
+  Params p{M, N, K, status, 0, EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr}};
+  return launch<false, false, false, true>(ta, tb, td, p, stream, &g);
 }
 
 }  // namespace g2
@@ -341,12 +348,12 @@ extern "C" {
 // clusters of two cannot be scheduled on this device; callers then use the one-CTA kernel.
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                      float alpha, float* ws, long long ws_bytes, int* status, cudaStream_t stream) {
+                      float alpha, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   using namespace mtb::g2;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (N % 8 || ldd % 8 || (R && ldr % 8)) return -10;
-  CUtensorMap ta, tb;
+  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32)) return -10;
+  CUtensorMap ta, tb, td;
   int rc;
   if (a_mn) rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, 64);
   else rc = make_tmap_2d_bf16(&ta, A, K, M, lda, BK, BM);
@@ -354,17 +361,19 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BNH);
   if (rc) return rc - 10;
-  Params p{M, N, K, status, 0, EpiParams{M, N, D, ldd, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, nullptr}};
+  rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
+  if (rc) return rc - 20;
+  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, stats, nullptr}};
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
-    case 0: return launch<false, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 1: return launch<false, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 2: return launch<false, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 3: return launch<false, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 4: return launch<true, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 5: return launch<true, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 6: return launch<true, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    default: return launch<true, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 0: return launch<false, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 1: return launch<false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 2: return launch<false, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 3: return launch<false, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 4: return launch<true, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 5: return launch<true, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 6: return launch<true, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    default: return launch<true, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
   }
 }
 

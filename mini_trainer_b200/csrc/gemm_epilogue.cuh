@@ -5,7 +5,8 @@
 // with few tiles and a long reduction, the tail of a two-wave grid). Every item leaves its fp32 partial in a workspace; the
 // warp that arrives last at the counter of a (tile, 32-row quarter) adds the partials in split order and runs the ordinary
 // epilogue. Nobody waits for anybody (the items may run in any order, on any number of SMs), the sum has one fixed order
-// whoever arrives last, and the counters are back at zero when the launch ends.
+// whoever arrives last, and the counters are back at zero when the launch ends. 1536 x 1536 x 5987 (72 tiles on 148 SMs): 40 -> 33 us,
+// 3720 x 1536 x 151936 (180 tiles): 1791 -> 1231 us.
 #pragma once
 #include "ptx.cuh"
 
@@ -13,23 +14,68 @@ namespace mtb {
 
 struct EpiParams {
   int M, N;
-  void* D;
-  long long ldd;
   const void* R;          // optional residual / accumulate source, same dtype as D
   long long ldr;
   const __nv_bfloat16* bias;  // optional, [N]
   float alpha;            // the product is multiplied by alpha before bias and residual are added
   int splits;             // work items per tile
   float* ws;              // splits > 1: partials, SPLIT_UNIT floats per (128-row unit, split)
+  float2* stats;          // optional (bf16 output): per row and column tile, maximum and sum of exp(x - maximum) of the stored
+                          // values, [M, ceil(N / 256)]; saves the cross-entropy its first pass over the logits
   unsigned* counters;     // splits > 1: one arrival counter per (128-row unit, quarter); zero between launches
 };
 
 constexpr int SPLIT_COUNTER_BYTES = 16384;
 constexpr int SPLIT_UNIT = 128 * 256;   // floats of one partial: 128 rows x 256 columns
 
-// 32 accumulator columns of one row -> D. `col0` < N; columns past N are not stored.
+// Running maximum and sum of exponentials of a row.
+struct RowStats {
+  float m = -INFINITY, s = 0.f;
+};
+
+// Output staging. A row of a tile belongs to one thread, so storing it directly sends 32 half-sectors to 32 rows with every
+// instruction: a 128 x 256 tile cost about 4000 clocks of the load/store unit, more than its MMAs when the reduction is short.
+// A warp stages 128 bytes of each of its 32 rows in shared memory (128B-swizzled, conflict-free) and one TMA store writes the
+// box, clipped to the matrix, while the next columns are read (5987 x 1536 x 1536: 28.6 -> 24.6 us, 5987 x 17920 x 1536: 270 -> 250 us;
+// long reductions hide either form).
+constexpr int STORE_BOX = 32 * 128;                  // bytes of one staged box: 32 rows x 128 bytes
+constexpr int EPI_SMEM = 4 * 2 * STORE_BOX;          // four epilogue warps, two boxes each
+
+struct EpiOut {
+  const void* map;      // tensor map of D, box 32 rows x 128 bytes
+  uint8_t* stage;       // this warp's two boxes
+  int z;                // matrix of a 3-D map, or -1
+  uint32_t n;           // boxes so far
+};
+
+// Buffer for the next box: free once at most the last store (the other buffer's) is still reading.
+__device__ __forceinline__ uint8_t* next_box(EpiOut& o, int lane) {
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+  __syncwarp();
+  return o.stage + (o.n & 1) * STORE_BOX;
+}
+__device__ __forceinline__ void store_box(EpiOut& o, const uint8_t* box, int x, int y, int rows, int lane) {
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0 && y < rows) {
+    if (o.z < 0)
+      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                   ::"l"(reinterpret_cast<uint64_t>(o.map)), "r"(smem_u32(box)), "r"(x), "r"(y) : "memory");
+    else
+      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+                   ::"l"(reinterpret_cast<uint64_t>(o.map)), "r"(smem_u32(box)), "r"(x), "r"(y), "r"(o.z) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+  ++o.n;
+}
+// Before the CTA's shared memory goes away.
+__device__ __forceinline__ void drain_boxes() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// 32 accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
+// bf16 box; an fp32 box holds 32 columns). Columns past N and rows past M are computed from nothing and clipped by the store.
 template <bool OUT_F32>
-__device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32], int row, int col0) {
+__device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
+                                               RowStats& st) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) f[j] *= p.alpha;
   if (p.bias != nullptr) {
@@ -43,61 +89,74 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
       }
     }
   }
+  const bool res = p.R != nullptr && row_ok;
   if constexpr (OUT_F32) {
-    float* dptr = reinterpret_cast<float*>(p.D) + static_cast<long long>(row) * p.ldd + col0;
-    const float* rptr = p.R ? reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0 : nullptr;
+    const float* rptr = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
-      if (col0 + j < p.N) {
-        float4 o = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
-        if (rptr) { const float4 r = *reinterpret_cast<const float4*>(rptr + j); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
-        *reinterpret_cast<float4*>(dptr + j) = o;
-      }
+      float4 o = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
+      if (res && col0 + j < p.N) { const float4 r = *reinterpret_cast<const float4*>(rptr + j); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
+      *reinterpret_cast<float4*>(srow + (((j >> 2) ^ (lane & 7)) << 4)) = o;
     }
   } else {
-    __nv_bfloat16* dptr = reinterpret_cast<__nv_bfloat16*>(p.D) + static_cast<long long>(row) * p.ldd + col0;
-    const __nv_bfloat16* rptr = p.R ? reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0 : nullptr;
+    const __nv_bfloat16* rptr = reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
-      if (col0 + j < p.N) {
-        if (rptr) {
-          const uint4 r = *reinterpret_cast<const uint4*>(rptr + j);
-          const float2 r0 = unpack_bf16(r.x), r1 = unpack_bf16(r.y), r2 = unpack_bf16(r.z), r3 = unpack_bf16(r.w);
-          f[j] += r0.x; f[j + 1] += r0.y; f[j + 2] += r1.x; f[j + 3] += r1.y;
-          f[j + 4] += r2.x; f[j + 5] += r2.y; f[j + 6] += r3.x; f[j + 7] += r3.y;
-        }
-        uint4 o;
-        o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
-        o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
-        *reinterpret_cast<uint4*>(dptr + j) = o;
+      if (res && col0 + j < p.N) {
+        const uint4 r = *reinterpret_cast<const uint4*>(rptr + j);
+        const float2 r0 = unpack_bf16(r.x), r1 = unpack_bf16(r.y), r2 = unpack_bf16(r.z), r3 = unpack_bf16(r.w);
+        f[j] += r0.x; f[j + 1] += r0.y; f[j + 2] += r1.x; f[j + 3] += r1.y;
+        f[j + 4] += r2.x; f[j + 5] += r2.y; f[j + 6] += r3.x; f[j + 7] += r3.y;
+      }
+      uint4 o;
+      o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
+      o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
+      *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
+      if (p.stats != nullptr && col0 + j < p.N) {   // of the values as stored
+        const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y), r2 = unpack_bf16(o.z), r3 = unpack_bf16(o.w);
+        const float mx = fmaxf(fmax3(fmaxf(r0.x, r0.y), r1.x, r1.y), fmax3(fmaxf(r2.x, r2.y), r3.x, r3.y));
+        if (mx > st.m) { st.s *= __expf(st.m - mx); st.m = mx; }
+        st.s += __expf(r0.x - st.m) + __expf(r0.y - st.m) + __expf(r1.x - st.m) + __expf(r1.y - st.m) + __expf(r2.x - st.m) +
+                __expf(r2.y - st.m) + __expf(r3.x - st.m) + __expf(r3.y - st.m);
       }
     }
   }
 }
 
 // One warp's part of a work item: quarter `q` of the 128-row unit that starts at row `row0`, columns [tn0, tn0 + 256).
-// `taddr`: tensor-memory address of the quarter. `unit`: index of the 128-row unit among all tiles' units.
-// SPLIT = false (the gathering kernels, which never split) leaves the split-K part out.
+// `taddr`: tensor-memory address of the quarter. `unit`: index of the 128-row unit among all tiles' units. `zero`: the item
+// had nothing to multiply, the accumulator holds an older tile. SPLIT = false leaves the split-K part out.
 template <bool OUT_F32, bool SPLIT>
-__device__ __forceinline__ void epilogue_quarter(const EpiParams& p, uint32_t taddr, int row0, int tn0, int q, int lane,
-                                                 int unit, int split) {
+__device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane,
+                                                 int unit, int split, bool zero) {
+  constexpr int PARTS = OUT_F32 ? 1 : 2;      // 32-column pieces per box
   const int row = row0 + q * 32 + lane;
   const bool row_ok = row < p.M;
+  RowStats st;
+  auto finish = [&]() {
+    if (!OUT_F32 && p.stats != nullptr && row_ok && tn0 < p.N)
+      p.stats[static_cast<long long>(row) * ((p.N + 255) / 256) + tn0 / 256] = make_float2(st.m, st.s);
+  };
   if (!SPLIT || p.splits == 1) {
 #pragma unroll 1
-    for (int c = 0; c < 8; ++c) {
+    for (int c = 0; c < 8; c += PARTS) {
       const int col0 = tn0 + c * 32;
       if (col0 >= p.N) break;  // uniform across the warp
-      uint32_t v[32];
-      tmem_ld_32x32(taddr + c * 32, v);
+      uint32_t v[PARTS][32];
+#pragma unroll
+      for (int k = 0; k < PARTS; ++k) tmem_ld_32x32(taddr + (c + k) * 32, v[k]);
+      uint8_t* box = next_box(out, lane);
       tmem_ld_wait();
-      if (row_ok) {
+#pragma unroll
+      for (int k = 0; k < PARTS; ++k) {
         float f[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-        epilogue_row32<OUT_F32>(p, f, row, col0);
+        for (int j = 0; j < 32; ++j) f[j] = zero ? 0.f : __uint_as_float(v[k][j]);
+        epilogue_row32<OUT_F32>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
       }
+      store_box(out, box, col0, row0 + q * 32, p.M, lane);
     }
+    finish();
     return;
   }
   // partial to the workspace: lane-interleaved 16-byte pieces, so every store and load is one contiguous 512 bytes
@@ -122,38 +181,32 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, uint32_t ta
   __threadfence();
   const float* base = p.ws + static_cast<long long>(unit) * p.splits * SPLIT_UNIT + q * 8192 + lane * 4;
 #pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < 8; c += PARTS) {
     const int col0 = tn0 + c * 32;
     if (col0 >= p.N) break;
-    float f[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) f[j] = 0.f;
-#pragma unroll 2
-    for (int s = 0; s < p.splits; ++s) {
-      const float* src = base + static_cast<long long>(s) * SPLIT_UNIT + c * 1024;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(src + j * 128));
-        f[4 * j] += v.x; f[4 * j + 1] += v.y; f[4 * j + 2] += v.z; f[4 * j + 3] += v.w;
-      }
-    }
-    if (row_ok) epilogue_row32<OUT_F32>(p, f, row, col0);
-  }
-  if (lane == 0) p.counters[unit * 4 + q] = 0;
-}
-
-// The same part of an output tile without a product.
-template <bool OUT_F32>
-__device__ __forceinline__ void epilogue_zero(const EpiParams& p, int row0, int tn0, int q, int lane) {
-  const int row = row0 + q * 32 + lane;
-  if (row >= p.M) return;
+    uint8_t* box = next_box(out, lane);
 #pragma unroll 1
-  for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
-    float f[32];
+    for (int k = 0; k < PARTS; ++k) {
+      float f[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) f[j] = 0.f;
-    epilogue_row32<OUT_F32>(p, f, row, tn0 + c * 32);
+      for (int j = 0; j < 32; ++j) f[j] = 0.f;
+      if (col0 + k * 32 < p.N) {   // pieces past N were never written
+#pragma unroll 2
+        for (int s = 0; s < p.splits; ++s) {
+          const float* src = base + static_cast<long long>(s) * SPLIT_UNIT + (c + k) * 1024;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + j * 128));
+            f[4 * j] += v.x; f[4 * j + 1] += v.y; f[4 * j + 2] += v.z; f[4 * j + 3] += v.w;
+          }
+        }
+      }
+      epilogue_row32<OUT_F32>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
+    }
+    store_box(out, box, col0, row0 + q * 32, p.M, lane);
   }
+  finish();
+  if (lane == 0) p.counters[unit * 4 + q] = 0;
 }
 
 // Grouped GEMM: one launch over the slabs of all experts of a mixture-of-experts layer. The rows of expert e are
@@ -173,13 +226,12 @@ struct GroupParams {
   const int* starts;     // [E + 1]
   const int* counts;     // [E]
   int E;
-  long long d_stride;    // REDUCE: elements between two experts' outputs
 };
 
-// Work items of a grouped launch in shared memory: tile_start[e] is the first tile of expert e.
+// Work items of a grouped launch in shared memory: tile_start[e] is the first tile of expert e. (Slab starts and counts are read
+// from global memory where they are needed, once per tile: shared memory is full.)
 struct GroupTable {
   int tile_start[GROUP_MAX + 1];
-  int row[GROUP_MAX], rows[GROUP_MAX];
 };
 
 // Filled by one warp; the caller synchronises the block.
@@ -193,14 +245,16 @@ __device__ __forceinline__ void fill_group_table(GroupTable& tab, const GroupPar
     int incl = n;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
-    if (e < g.E) { tab.tile_start[e] = base + incl - n; tab.row[e] = g.starts[e]; tab.rows[e] = rows; }
+    if (e < g.E) tab.tile_start[e] = base + incl - n;
     base += __shfl_sync(0xffffffffu, incl, 31);
   }
   if (lane == 0) tab.tile_start[g.E] = base;
 }
 
-// Number of work items per tile (of 0.4 us k-blocks on one SM): 1 when whole tiles fill the `workers` (SMs or CTA pairs) well, else the smallest cost in
+// Number of work items per tile: 1 when whole tiles fill the `workers` (SMs or CTA pairs) well, else the smallest cost in
 // units of one k-block of a tile: full waves of items, plus what the extra partials cost (write, one counter, ordered sum).
+// A k-block is about 0.4 us on one SM; an item costs ten more (its share of a partial's write and of the pipeline fill), the
+// ordered sum three per partial: without those terms 2048 x 1536 x 5987 (96 tiles) was split in three and went from 40 to 46 us.
 // `max_items`: what the workspace holds.
 inline int choose_splits(long long tiles, int kblocks, int workers, long long max_items) {
   if (tiles <= 0 || workers <= 0) return 1;

@@ -40,7 +40,7 @@ constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
 constexpr int GEMM_THREADS = 192;
 constexpr int GROUP_M = 16;
 constexpr int GATHER_GROUP_N = 4;   // column-tiles per band in the all-gather variant
-constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
+constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + EPI_SMEM + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 struct GemmParams {
   int M, N, K;
@@ -59,12 +59,13 @@ struct GemmParams {
 // GROUP: one launch over the expert slabs of a mixture-of-experts layer (gemm_epilogue.cuh).
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE>
 __global__ void __launch_bounds__(GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p,
+gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+            const __grid_constant__ CUtensorMap tmap_d, GemmParams p,
             const __grid_constant__ GatherParams g, GroupParams gr) {
   __shared__ GroupTable gtab;   // unused (and not allocated) outside the grouped forms
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + EPI_SMEM);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;   // [2] accumulator ready for the epilogue
   uint64_t* tempty_bar = tfull_bar + 2;       // [2] accumulator drained
@@ -87,6 +88,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
+    tma_prefetch_desc(&tmap_d);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   if (GROUP && warp == 2) fill_group_table<GROUP>(gtab, gr, BM, tiles_n, num_tiles, lane);
@@ -100,7 +102,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   // The grouped forms walk the experts with the items: `e` only moves forward.
   auto group_coords = [&](int w, int& e, int& tm, int& tn) {
     while (w >= gtab.tile_start[e + 1]) ++e;
-    const int rows_m = GROUP == GROUP_ROWS ? (gtab.rows[e] + BM - 1) / BM : tiles_m;
+    const int rows_m = GROUP == GROUP_ROWS ? (gr.counts[e] + BM - 1) / BM : tiles_m;
     const int t = w - gtab.tile_start[e];
     const int band = t / (p.group_m * tiles_n);
     const int first_m = band * p.group_m;
@@ -145,13 +147,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         if constexpr (GROUP != GROUP_NONE) {
           group_coords(w, e, tm, tn);
           kb0 = 0;
-          kb1 = GROUP == GROUP_REDUCE ? (gtab.rows[e] + BK - 1) / BK : kblocks;
+          kb1 = GROUP == GROUP_REDUCE ? (gr.counts[e] + BK - 1) / BK : kblocks;
         } else {
           tile_coords(w % num_tiles, tm, tn);
           k_range(w / num_tiles, kb0, kb1);
         }
-        const int a_row = GROUP == GROUP_ROWS ? gtab.row[e] + tm * BM : tm * BM;   // first row of the A tile
-        const int k_row = GROUP == GROUP_REDUCE ? gtab.row[e] : 0;                 // first row of the reduction
+        const int a_row = GROUP == GROUP_ROWS ? gr.starts[e] + tm * BM : tm * BM;   // first row of the A tile
+        const int k_row = GROUP == GROUP_REDUCE ? gr.starts[e] : 0;                 // first row of the reduction
         if (GATHER) {
           // the checker warp has seen the flags of every chunk under this tile's B rows
           if (!wait_verified(verified, tl, abort_flag, waited_ns, p.wait_limit_us)) { *abort_flag = 1; atomicExch(p.status, 5); goto done; }
@@ -199,7 +201,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         if constexpr (GROUP != GROUP_NONE) {
           while (w >= gtab.tile_start[e + 1]) ++e;
           kb0 = 0;
-          kb1 = GROUP == GROUP_REDUCE ? (gtab.rows[e] + BK - 1) / BK : kblocks;
+          kb1 = GROUP == GROUP_REDUCE ? (gr.counts[e] + BK - 1) / BK : kblocks;
         } else {
           k_range(w / num_tiles, kb0, kb1);
         }
@@ -255,29 +257,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t tl = 0;
     int e = 0;
-    EpiParams ep = p.e;
+    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + q * 2 * STORE_BOX, -1, 0};
     for (int w = blockIdx.x; w < num_items; w += gridDim.x, ++tl) {
       const int t = w % num_tiles;
       int tm, tn, row0;
       if constexpr (GROUP != GROUP_NONE) group_coords(w, e, tm, tn); else tile_coords(t, tm, tn);
       row0 = tm * BM;
-      if constexpr (GROUP == GROUP_ROWS) row0 += gtab.row[e];   // slabs are padded to whole tiles: every row may be stored
-      if constexpr (GROUP == GROUP_REDUCE) ep.D = reinterpret_cast<unsigned char*>(p.e.D) + e * gr.d_stride * (OUT_F32 ? 4 : 2);
+      if constexpr (GROUP == GROUP_ROWS) row0 += gr.starts[e];   // slabs are padded to whole tiles: every row may be stored
+      if constexpr (GROUP == GROUP_REDUCE) out.z = e;
       const int acc = tl & 1;
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 4); goto done; }
       tc_fence_after();
-      if (GROUP == GROUP_REDUCE && gtab.rows[e] == 0)   // nothing was multiplied: the accumulator holds an older tile
-        epilogue_zero<OUT_F32>(ep, row0, tn * BN, q, lane);
-      else
-        epilogue_quarter<OUT_F32, !GATHER && !GROUP>(ep, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
-                                                     w / num_tiles);
+      epilogue_quarter<OUT_F32, !GATHER && !GROUP>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
+                                                   w / num_tiles, GROUP == GROUP_REDUCE && gr.counts[e] == 0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
     }
   }
 done:
+  if (warp >= 2 && warp < 6 && lane == 0) drain_boxes();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -355,6 +355,11 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// Tensor map the epilogue stores D through: boxes of 32 rows x 128 bytes.
+int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32) {
+  return out_f32 ? make_tmap_2d_f32(out, D, N, M, ldd, 32, 32) : make_tmap_2d_bf16(out, D, N, M, ldd, 64, 32);
+}
+
 static int g_num_sms = 0;
 
 // Tuning knobs read once from the environment (experiments; the defaults are what ships).
@@ -375,7 +380,7 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
 }
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE>
-static int launch(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream,
+static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmParams p, cudaStream_t stream,
                   const GatherParams* gp = nullptr, long long ws_bytes = 0, const GroupParams* grp = nullptr) {
   static bool configured = false;
   auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP>;
@@ -400,7 +405,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cu
   const int items = tiles * p.e.splits;
   const int grid = (GATHER || items >= g_num_sms) ? g_num_sms : items;
   static const GatherParams none{};
-  kern<<<grid, GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, p, gp ? *gp : none, grp ? *grp : GroupParams{});
+  kern<<<grid, GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, p, gp ? *gp : none, grp ? *grp : GroupParams{});
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -414,14 +419,15 @@ extern "C" {
 //   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
 //   ws: optional fp32 workspace of ws_bytes for split-K (null: never split); its first SPLIT_COUNTER_BYTES are zero
 //   before the first call, every launch leaves them zero again, and launches that may overlap have one each
+//   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
 // Returns 0 on success, a negative code on invalid arguments or launch failure.
 int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                     float alpha, float* ws, long long ws_bytes, int* status, cudaStream_t stream) {
+                     float alpha, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (N % 8 || ldd % 8 || (R && ldr % 8)) return -10;
-  CUtensorMap ta, tb;
+  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32)) return -10;
+  CUtensorMap ta, tb, td;
   int rc;
   if (a_mn) rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, 64);
   else rc = make_tmap_2d_bf16(&ta, A, K, M, lda, BK, BM);
@@ -429,18 +435,20 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc - 10;
+  rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
+  if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{M, N, D, ldd, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, nullptr}};
+               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, stats, nullptr}};
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
-    case 0: return launch<false, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 1: return launch<false, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 2: return launch<false, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 3: return launch<false, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 4: return launch<true, false, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 5: return launch<true, false, true>(ta, tb, p, stream, nullptr, ws_bytes);
-    case 6: return launch<true, true, false>(ta, tb, p, stream, nullptr, ws_bytes);
-    default: return launch<true, true, true>(ta, tb, p, stream, nullptr, ws_bytes);
+    case 0: return launch<false, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 1: return launch<false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 2: return launch<false, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 3: return launch<false, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 4: return launch<true, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 5: return launch<true, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 6: return launch<true, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    default: return launch<true, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
   }
 }
 
@@ -448,14 +456,14 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
 // height of the row buffers.
 //   mode 0  D[rows, N] = A[rows, K] * W_e[N, K]^T        W: E matrices [N, K], w_stride elements apart
 //   mode 1  D[rows, N] = A[rows, K] * W_e[K, N]          W: E matrices [K, N], w_stride elements apart
-//   mode 2  W_e[M, N] = A[rows_e, M]^T * B[rows_e, N]    D is W here: E outputs, w_stride elements apart; K is ignored
+//   mode 2  W_e[M, N] = A[rows_e, M]^T * B[rows_e, N]    D is W here: E outputs, w_stride elements apart, ldd = N; K is ignored
 int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long ldb, void* D, long long ldd, int mode, int rows,
                         int M, int N, int K, const int* starts, const int* counts, int E, long long w_stride, int* status,
                         cudaStream_t stream) {
   using namespace mtb;
   if (E <= 0 || rows <= 0 || N <= 0 || (mode == 2 ? M : K) <= 0) return 0;
   if (E > GROUP_MAX || N % 8 || ldd % 8 || rows % GROUP_ALIGN || w_stride % 8 || mode < 0 || mode > 2) return -10;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   int rc = mode == 2 ? make_tmap_2d_bf16(&ta, A, M, rows, lda, 64, 64) : make_tmap_2d_bf16(&ta, A, K, rows, lda, BK, BM);
   if (rc) return rc;
   if (mode == 0) rc = make_tmap_3d_bf16(&tb, B, K, N, E, w_stride, BK, BN);
@@ -463,12 +471,15 @@ int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long l
   else rc = make_tmap_2d_bf16(&tb, B, N, rows, ldb, 64, 64);
   if (rc) return rc - 10;
   const int out_rows = mode == 2 ? M : rows;
+  if (mode == 2) rc = ldd == N ? make_tmap_3d_bf16(&td, D, N, M, E, w_stride, 64, 32) : -10;
+  else rc = make_tmap_out(&td, D, rows, N, ldd, 0);
+  if (rc) return rc - 20;
   GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{out_rows, N, D, ldd, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr}};
-  GroupParams g{starts, counts, E, w_stride};
-  if (mode == 0) return launch<false, false, false, false, false, GROUP_ROWS>(ta, tb, p, stream, nullptr, 0, &g);
-  if (mode == 1) return launch<false, true, false, false, false, GROUP_ROWS>(ta, tb, p, stream, nullptr, 0, &g);
-  return launch<true, true, false, false, false, GROUP_REDUCE>(ta, tb, p, stream, nullptr, 0, &g);
+               EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr}};
+  GroupParams g{starts, counts, E};
+  if (mode == 0) return launch<false, false, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
+  if (mode == 1) return launch<false, true, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
+  return launch<true, true, false, false, false, GROUP_REDUCE>(ta, tb, td, p, stream, nullptr, 0, &g);
 }
 
 // Fused all-gather + GEMM:  D[M,N] = A[M,K] * W[N,K]^T (+bias) with W living in `full`, the local
@@ -490,13 +501,15 @@ int mtb200_gemm_bf16_allgather(const void* A, long long lda, void* D, long long 
   if (M <= 0 || N <= 0 || K <= 0) return -10;
   if (N % 8 || ldd % 8 || K % 8 || world < 1 || world > GATHER_MAX_RANKS || shard_bytes % 16 || w_byte_off % 16) return -10;
   if (world > 1 && shard_bytes < static_cast<unsigned long long>(GATHER_CHUNK_BYTES)) return -11;   // a chunk may straddle one shard boundary at most
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   int rc = make_tmap_2d_bf16(&ta, A, K, M, lda, BK, BM);
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, reinterpret_cast<const unsigned char*>(full) + w_byte_off, K, N, K, BK, BN);
   if (rc) return rc - 10;
+  rc = make_tmap_out(&td, D, M, N, ldd, 0);
+  if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{M, N, D, ldd, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr}};
+               EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr}};
   GatherParams g{};
   for (int i = 0; i < world; ++i) g.peer_base[i] = bases[i];
   g.shard_off = shard_off; g.shard_bytes = shard_bytes; g.dst = reinterpret_cast<unsigned char*>(full);
@@ -511,7 +524,7 @@ int mtb200_gemm_bf16_allgather(const void* A, long long lda, void* D, long long 
     rc = g2::launch_gather(A, lda, D, ldd, bias, M, N, K, reinterpret_cast<const unsigned char*>(full) + w_byte_off, status, g, stream);
     if (rc != -6) return rc;   // -6: CTA pairs cannot be scheduled here; fall through to the one-CTA kernel
   }
-  return launch<false, false, false, true>(ta, tb, p, stream, &g);
+  return launch<false, false, false, true>(ta, tb, td, p, stream, &g);
 }
 
 // Fused gradient reduce + GEMM:  D[M,N] (fp32) = (sum over ranks of G_r)[M,K] * B[N,K]^T (+ R), where G_r is the region
@@ -528,15 +541,17 @@ int mtb200_gemm_bf16_reduce_a(void* dst, const void* B, long long ldb, float* D,
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return -10;
   if (N % 8 || ldd % 8 || K % 8 || (R && ldr % 8) || world < 1 || world > 8 || src_off % 16 || ticket == nullptr || done == nullptr) return -10;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   int rc = make_tmap_2d_bf16(&ta, dst, K, M, K, BK, BM);
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc - 10;
   // every pipeline wait sits out the peers' skew: a little longer than the bound of the ready-flag wait itself
   const unsigned lim = limit_us ? limit_us : FLAG_SPIN_LIMIT;
+  rc = make_tmap_out(&td, D, M, N, ldd, 1);
+  if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), lim + lim / 2 + 10000000u,
-               EpiParams{M, N, D, ldd, R, ldr, nullptr, 1.0f, 1, nullptr, nullptr}};
+               EpiParams{M, N, R, ldr, nullptr, 1.0f, 1, nullptr, nullptr, nullptr}};
   GatherParams g{};
   for (int i = 0; i < world; ++i) g.peer_base[i] = bases[i];
   g.dst = reinterpret_cast<unsigned char*>(dst);
@@ -549,7 +564,7 @@ int mtb200_gemm_bf16_reduce_a(void* dst, const void* B, long long ldb, float* D,
   g.rs_epoch = rs_epoch; g.limit_us = limit_us ? limit_us : FLAG_SPIN_LIMIT; g.status = status;
   if (cudaMemsetAsync(ticket, 0, sizeof(unsigned int), stream) != cudaSuccess) return -5;
   if (cudaMemsetAsync(done, 0, sizeof(unsigned int), stream) != cudaSuccess) return -5;
-  return launch<false, false, true, true, true>(ta, tb, p, stream, &g);
+  return launch<false, false, true, true, true>(ta, tb, td, p, stream, &g);
 }
 
 }  // extern "C"

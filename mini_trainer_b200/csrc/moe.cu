@@ -16,7 +16,7 @@ namespace mtb {
 
 typedef __nv_bfloat16 bf16;
 constexpr int MOE_THREADS = 256;
-constexpr int PLAN_THREADS = 1024;
+constexpr int PLAN_THREADS = 1024;   // 32 warps: one lane per warp total
 
 struct Vec8 {
   uint4 u;
@@ -69,9 +69,11 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const long long*
     const unsigned m = __ballot_sync(0xffffffffu, hit);
     if (lane == 0) wsum[it & 1][warp] = __popc(m);
     __syncthreads();
-    int before = 0, total = 0;
+    const int mine = wsum[it & 1][lane];   // every warp scans the warps' totals for itself
+    int incl = mine;
 #pragma unroll
-    for (int w = 0; w < PLAN_THREADS / 32; ++w) { const int c = wsum[it & 1][w]; if (w < warp) before += c; total += c; }
+    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+    const int before = __shfl_sync(0xffffffffu, incl - mine, warp), total = __shfl_sync(0xffffffffu, incl, 31);
     if (hit) {
       const int row = next + before + __popc(m & ((1u << lane) - 1));
       pair_of[row] = i;

@@ -44,8 +44,8 @@ P, I, L, F = c_void_p, c_int, c_longlong, c_float
 
 
 class _Sig:
-    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P]
-    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P]
+    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
+    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P]
     mtb200_rmsnorm_bwd_blocks = [I]
     mtb200_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, I, P]
@@ -82,6 +82,8 @@ class _Sig:
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
+_SPLIT_COUNTERS = 4096          # 4-byte words in front of the partials (SPLIT_COUNTER_BYTES in csrc/gemm_epilogue.cuh)
+_SPLIT_FLOATS = 32 << 20        # partials: 128 MB = 1024 work items of 128 x 256
 NATIVE_HEAD_DIMS = (64, 128)   # head dimensions of the hand-written attention kernels
 
 
@@ -127,6 +129,7 @@ class NativeOps:
         self.launches = 0
         self.profile = [] if os.environ.get("MTB200_PROFILE") else None
         self._scratch = {}
+        self._gemm_ws = {}   # stream handle -> split-K workspace
         self._attn_plan_cache = {}
 
     # -- plumbing ---------------------------------------------------------------------
@@ -183,14 +186,27 @@ class NativeOps:
         code = int(self.status.item())
         if code:
             self.status.zero_()
+            for ws in self._gemm_ws.values():   # a kernel that gave up may have left arrivals behind
+                ws[: _SPLIT_COUNTERS].zero_()
             what = {60: "a token id outside the embedding table", 61: "an attention work item outside the packed batch",
                     62: "a chosen expert outside the model's experts"}.get(
                 code, "a device-side bounded wait expired")
             raise RuntimeError(f"{what} (status code {code})")
 
     # -- GEMM -------------------------------------------------------------------------
-    def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0):
+    def _split_workspace(self, stream):
+        """Split-K workspace of a stream: arrival counters (zero between launches) and fp32 partials. GEMMs of one stream run
+        one after the other, those of different streams may overlap, so each stream has its own."""
+        ws = self._gemm_ws.get(stream)
+        if ws is None:
+            ws = torch.empty(_SPLIT_COUNTERS + _SPLIT_FLOATS, dtype=torch.float32, device=self.device)
+            ws[: _SPLIT_COUNTERS].zero_()
+            self._gemm_ws[stream] = ws
+        return ws
+
+    def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
         """out[M,N] = alpha*A*B (+bias) (+residual). ``a_mn``/``b_mn``: operand stored [K, rows].
+        ``stats`` [M, ceil(N / 256), 2] fp32 receives the softmax statistics of the (bf16) output rows per 256 columns.
         ``two_cta``: force (True) or forbid (False) the cta_group::2 kernel; default by problem size."""
         out_f32 = out.dtype == torch.float32
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
@@ -198,10 +214,11 @@ class NativeOps:
         if two_cta is None:
             two_cta = self.use_gemm2 and (-(-M // 256)) * (-(-N // 256)) >= 64
         st = self._st()
+        ws = self._split_workspace(st)
         self._call("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
                    residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha),
-                   None, 0, self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
+                   ws.data_ptr(), ws.numel() * 4, _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
         return out
 
     # -- embedding --------------------------------------------------------------------
@@ -523,9 +540,9 @@ class NativeOps:
     def linear_ce(self, x, w, targets, grad_scale, dw_out, accumulate_dw=False, ignore_index=-100, logit_scale=1.0):
         """Per-token CE of ``logit_scale * x @ w.T``. Chunked over tokens (8192 rows): bf16 logits chunk
         by the tcgen05 GEMM (fp32 accumulation, one rounding: what the reference's fused linear-CE holds
-        too) -> per-row softmax statistics, loss and the bf16 gradient written over the logits -> dX
+        too), whose epilogue also leaves softmax statistics -> loss and the bf16 gradient written over the logits -> dX
         chunk and dW accumulation, again on the tcgen05 GEMM. Only ``[chunk, V]`` logits ever exist.
-        dW is accumulated in fp32 and rounded to bf16 once at the end."""
+        dW is accumulated in fp32 over the chunks and rounded to bf16 once."""
         T, H = x.shape
         V = w.shape[0]
         loss = torch.empty(T, dtype=torch.float32, device=self.device)

@@ -576,3 +576,28 @@ def test_grouped_experts_match_loop_over_experts(ops, T, H, F, E, k, popular, ac
     gs["wgu0"] = torch.cat([gs["wgu0"].reshape(-1), gs["wgu0"].new_zeros(8)])[: gs["wgu0"].numel()].view_as(p["wgu0"])
     M.moe_backward(ops, cfg, p, gs, again[1], n2, dout)
     assert all(torch.equal(first[n], gs[n]) for n in gs)
+
+
+# work items per tile > 1: few tiles and a long reduction, odd sizes, both kernels, every operand layout, bias / residual / fp32
+@pytest.mark.parametrize("M,N,K", [(128, 256, 4096), (1536, 1536, 6000), (136, 264, 1000), (2048, 520, 7777)])
+@pytest.mark.parametrize("two_cta", [False, True])
+def test_gemm_split_k(ops, M, N, K, two_cta):
+    torch.manual_seed(M + K)
+    K8 = -(-K // 8) * 8
+    a, b = bf(M, K8), bf(N, K8, scale=0.1)
+    a, b = a[:, :K], b[:, :K]
+    ref = a.float() @ b.float().t()
+    res, bias = bf(M, N), bf(N)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    ops.gemm(a, False, b, False, out, M, N, K, residual=res, bias=bias, alpha=0.5, two_cta=two_cta)
+    want = 0.5 * ref + bias.float() + res.float()
+    assert rel_err(out, want) < 4e-3
+    first = out.clone()
+    ops.gemm(a, False, b, False, out, M, N, K, residual=res, bias=bias, alpha=0.5, two_cta=two_cta)
+    assert torch.equal(first, out)     # one order of summation, whoever arrives last
+    o32 = torch.empty(M, N, dtype=torch.float32, device="cuda")
+    if M % 8 == 0:
+        at, bt = a.t().contiguous(), b.t().contiguous()
+        ops.gemm(at, True, bt, True, o32, M, N, K, two_cta=two_cta)
+        assert rel_err(o32, ref) < 1e-5    # fp32 sums of exact products of bf16 values
+    ops.check_status()

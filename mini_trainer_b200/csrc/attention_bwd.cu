@@ -3,26 +3,35 @@
 // One CTA owns one (sequence, 128-key block, kv head): K and V of that block stay in shared memory
 // and dK, dV accumulate in tensor memory over every query head of the GQA group and every query
 // block at or below the causal diagonal, so they are written once, without atomics. Per
-// (query head, query block) the CTA runs five tcgen05 GEMMs:
-//   S  = Q K^T            dP = dO V^T                      (TMEM, 128 columns each)
-//   P  = exp(S*scale - lse), dS = P * (dP - delta) * scale  (4 warps; bf16 P and dS to smem)
-//   dQ = dS K  (into S's TMEM columns)   dV += P^T dO   dK += dS^T Q
-// dQ tiles (several key blocks contribute to one query block) are staged in shared memory and added
-// into an fp32 [T, Hq*D] accumulator with TMA tensor reduces (cp.reduce.async.bulk.tensor .add, one
-// 32-column x 128-row box each, 128B-swizzled so the staging stores are free of bank conflicts); a
-// small kernel rounds the accumulator to bf16 afterwards. The first half of the D columns is staged
-// in the P tile (idle once the MMAs have read it), the second half in a buffer of its own, and a
-// separate warp issues the reduces: those of the P tile first and alone, so that the next softmax, which
-// has to overwrite P, waits for half of the read-out only, and never for the thread that issued it.
-// P and dS are stored once as [query, key] 128B-swizzled tiles and read both K-major (for dQ) and
-// MN-major (for dV / dK), so no transposes are materialised.
+// (query head, query block) the CTA runs five tcgen05 GEMMs on TRANSPOSED scores (keys on the lanes):
+//   S^T = K Q^T        dP^T = V dO^T                        (TMEM, 128 columns each)
+//   P^T = exp(S^T*scale - lse), dS^T = P^T * (dP^T - delta) * scale   (8 warps)
+//   dV += P^T dO       dK += dS^T Q       dQ = dS K
+// With keys on the lanes, P^T and dS^T are the A operands of dV and dK as they stand: they are written back over the
+// columns of tensor memory they were computed from and never become shared-memory tiles (a 128 x 128 product with both
+// operands in shared memory already reads the 128 bytes per clock that shared memory has). Only dS has a shared-memory
+// tile, for dQ, where it is read MN-major. The room that frees holds a second Q tile.
 //
-// Rows past the end of the sequence (queries or keys) are masked to zero contribution.
+// The MMAs of neighbouring iterations interleave so that the softmax of one runs under the products of another. Issue order:
+//   ... dK(i) dQ(i) | dV(i+1) dP(i+1) S(i+2) | dK(i+1) dQ(i+1) | ...
+// P(i+1) is computed while dK(i), dQ(i) run, dQ(i) is drained under dV(i+1), dS(i+1) is computed while S(i+2) and the tail
+// of dP(i+1) run. The chain that bounds an iteration is dS -> dK dQ dV dP -> dS: four products plus the dS half of the
+// softmax, where the form with everything in one chain (S dP | softmax | dK dV dQ | drain) had five products, the whole
+// softmax and the drain. 1 x 16384 tokens, 32/8 heads, D = 128: 6.49 -> 5.47 ms.
+//
+// dQ shares the columns of dP (read out before the next dP is issued). Its tiles (several key blocks contribute to one
+// query block) go through a 32 KB staging buffer, 64 columns at a time, into an fp32 [T, Hq*D] accumulator with TMA tensor
+// reduces (cp.reduce.async.bulk.tensor .add, one 32-column x 128-row box each, 128B-swizzled so the staging stores are free of
+// bank conflicts); a small kernel rounds the accumulator to bf16 afterwards. Four warps of their own drain, one more issues
+// the reduces, so the softmax warps see nothing of dQ.
+//
+// Rows past the end of the sequence contribute nothing: a query's lse is staged as +infinity, a key's scores are masked.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 
 namespace mtb {
@@ -33,31 +42,23 @@ int make_tmap_2d_f32(CUtensorMap* out, const void* base, uint64_t inner, uint64_
                      uint32_t box_inner, uint32_t box_outer);
 
 constexpr int AB_B = 128;          // block edge (queries and keys)
-constexpr int AB_THREADS = 352;     // TMA warp, MMA warp, 8 softmax warps (two threads per query row), dQ reduce warp
-
-// Phase timestamps for kernel development. They exist only in a library built with
-// -DMTB200_ATTN_BWD_TIMESTAMPS (the shipped build has neither the buffer nor the stores): per
-// iteration of CTA 0, 4 clock64 values from the MMA thread (start, S/dP issued, P/dS seen, late MMAs
-// issued) and 5 from one softmax thread (S/dP seen, P/dS computed, P tile free, dQ complete, dQ
-// staged), read back with mtb200_attn_bwd_debug_read.
-#ifdef MTB200_ATTN_BWD_TIMESTAMPS
-constexpr int DBG_ITERS = 256;
-__device__ long long g_attn_bwd_dbg[DBG_ITERS * 9];
-#define MTB_STAMP(cond, it, slot) do { if ((cond) && (it) < DBG_ITERS) g_attn_bwd_dbg[(it) * 9 + (slot)] = clock64(); } while (0)
-#else
-#define MTB_STAMP(cond, it, slot) do { } while (0)
-#endif
+// four warpgroups: {TMA, MMA, dQ reduce, row statistics}, 2 x softmax (two threads per key row), dQ drain
+constexpr int AB_THREADS = 512;
+// Registers per thread after the split; over the four warpgroups they add up to the 4 x 128 of the launch.
+constexpr int AB_REGS_IO = 104, AB_REGS_SOFTMAX = 152, AB_REGS_DRAIN = 104;
+static_assert(AB_REGS_IO + 2 * AB_REGS_SOFTMAX + AB_REGS_DRAIN == 4 * 128, "register split");
 
 template <int D>
 struct AttBwdSmem {
   static constexpr int TILE = AB_B * D * 2;         // a [128, D] bf16 tile
-  static constexpr int PT = AB_B * AB_B * 2;        // a [128, 128] bf16 tile
-  static constexpr int OFF_K = 0, OFF_V = TILE, OFF_Q = 2 * TILE, OFF_DO = 3 * TILE;
-  static constexpr int OFF_P = 4 * TILE, OFF_DS = OFF_P + PT;
-  static constexpr int OFF_ST2 = OFF_DS + PT;       // staging of the second half of a dQ tile: D/64 boxes of [128 rows x 128 B]
-  static constexpr int ST2 = (D / 64) * 16384;
-  static constexpr int OFF_BAR = OFF_ST2 + ST2;
-  static constexpr int TOTAL = OFF_BAR + 256 + 1024;
+  static constexpr int OFF_K = 0, OFF_V = TILE, OFF_DO = 2 * TILE, OFF_Q = 3 * TILE;   // Q: 2 buffers
+  static constexpr int OFF_DS = 5 * TILE;           // dS as [key, query], 128 x 128 bf16
+  static constexpr int OFF_ST = OFF_DS + AB_B * AB_B * 2;    // dQ staging: 2 boxes of 128 rows x 32 fp32 columns
+  static constexpr int OFF_STAT = OFF_ST + 2 * 16384;        // 2 buffers x {-lse * log2 e, -delta * scale} x 128 queries
+  static constexpr int OFF_BAR = OFF_STAT + 2 * 2 * 128 * 4;
+  // D = 128 fills the shared memory of an SM, so there is no slack to align with: the kernel checks that the window
+  // starts on a 1024-byte boundary (swizzle atom).
+  static constexpr int TOTAL = OFF_BAR + 256;
 };
 
 struct AttBwdParams {
@@ -68,9 +69,15 @@ struct AttBwdParams {
   float* dq_acc;        // [T, Hq*D] fp32, zero-initialised
   const int* plan;      // [n_items, 3] = seq_start, seq_len, k0
   int T, Hq, Hkv;
+  int splits;           // CTAs that share a key block's query heads
+  float* ws;            // splits > 1: fp32 partials of dK and dV
+  unsigned* counters;   // splits > 1: one arrival counter per (key block, warp); zero between launches
   float scale;
   int* status;
 };
+
+template <int R> __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
 template <int D>
 __global__ void __launch_bounds__(AB_THREADS, 1)
@@ -79,31 +86,41 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   using L = AttBwdSmem<D>;
   constexpr int KB = D / 64;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = smem_raw;
+  if (smem_u32(smem) & 1023u) {   // uniform over the CTA: nothing has been allocated or armed yet
+    if (threadIdx.x == 0) atomicExch(p.status, 20);
+    return;
+  }
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* kv_full = bars;        // K and V resident
-  uint64_t* qdo_full = bars + 1;   // [2] Q_i landed / dO_i landed (at bars + 1 and bars + 9)
-  uint64_t* sdp_full = bars + 2;   // S and dP complete
-  uint64_t* pds_ready = bars + 3;  // P and dS written (4 arrivals)
-  uint64_t* stage_full = bars + 4; // dQ tile copied from TMEM to the smem staging area (8 arrivals)
-  uint64_t* mma_done = bars + 5;   // dV, dK, dQ complete: Q, dO, P, dS reusable, dQ readable
-  uint64_t* dq_read = bars + 6;    // dQ tile drained from TMEM (8 arrivals): S columns reusable
-  uint64_t* stage_free = bars + 7; // the tensor reduces have read the dQ half staged in the P tile: P writable
-  uint64_t* q_free = bars + 8;     // dK has read Q: the next Q tile may be loaded while dV and dQ still run
-  uint64_t* do_full = bars + 9;    // dO_i landed
-  uint64_t* do_free = bars + 10;   // dV has read dO: the next dO tile may be loaded while dQ still runs
-  uint64_t* st2_free = bars + 11;  // the tensor reduces have read the second staging buffer
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* kv_full = bars;          // K and V resident
+  uint64_t* q_full = bars + 1;       // [2] Q landed
+  uint64_t* q_free = bars + 3;       // [2] dK has read Q
+  uint64_t* do_full = bars + 5;      // dO landed
+  uint64_t* do_free = bars + 6;      // dV and dP have read dO
+  uint64_t* s_full = bars + 7;       // S^T complete
+  uint64_t* dp_full = bars + 8;      // dP^T complete; every earlier MMA too, so the dS tile is writable
+  uint64_t* p_ready = bars + 9;      // P^T in tensor memory (8 arrivals)
+  uint64_t* ds_ready = bars + 10;    // dS^T in tensor memory and dS in shared memory (8 arrivals)
+  uint64_t* dq_full = bars + 11;     // dQ complete
+  uint64_t* dq_read = bars + 12;     // dQ read out of tensor memory (4 arrivals): dP columns reusable
+  uint64_t* stage_full = bars + 13;  // 64 columns of dQ staged (4 arrivals)
+  uint64_t* stage_free = bars + 14;  // the tensor reduces have read the staging buffer
+  uint64_t* stat_full = bars + 15;   // [2] lse / delta of a query block staged
+  uint64_t* stat_free = bars + 17;   // [2] consumed (8 arrivals)
+  uint64_t* all_done = bars + 19;    // dK and dV complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = blockIdx.x / p.Hkv, hk = blockIdx.x % p.Hkv;
+  const int unit = blockIdx.x / p.splits, sub = blockIdx.x - unit * p.splits;
+  const int item = unit / p.Hkv, hk = unit % p.Hkv;
   const int G = p.Hq / p.Hkv;
+  const int h_first = hk * G + G * sub / p.splits, heads = G * (sub + 1) / p.splits - G * sub / p.splits;
   const int seq_start = p.plan[item * 3 + 0], seq_len = p.plan[item * 3 + 1], k0 = p.plan[item * 3 + 2];
   const int jblk = k0 / AB_B;
   const int nq = (seq_len + AB_B - 1) / AB_B;      // query blocks of the sequence
   const int per_head = nq - jblk;                  // query blocks at or below the diagonal
-  const int n_iters = G * per_head;
+  const int n_iters = heads * per_head;
   // bounds check of the host-built work item (uniform over the CTA; nothing allocated or armed yet)
   if (seq_start < 0 || seq_len <= 0 || k0 < 0 || k0 >= seq_len || static_cast<long long>(seq_start) + seq_len > p.T) {
     if (threadIdx.x == 0) atomicExch(p.status, 61);
@@ -111,9 +128,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   }
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1); mbar_init(qdo_full, 1); mbar_init(sdp_full, 1); mbar_init(pds_ready, 8);
-    mbar_init(stage_full, 8); mbar_init(mma_done, 1); mbar_init(dq_read, 8); mbar_init(stage_free, 1);
-    mbar_init(q_free, 1); mbar_init(do_full, 1); mbar_init(do_free, 1); mbar_init(st2_free, 1);
+    mbar_init(kv_full, 1); mbar_init(do_full, 1); mbar_init(do_free, 1); mbar_init(s_full, 1); mbar_init(dp_full, 1);
+    mbar_init(p_ready, 8); mbar_init(ds_ready, 8); mbar_init(dq_full, 1); mbar_init(dq_read, 4);
+    mbar_init(stage_full, 4); mbar_init(stage_free, 1); mbar_init(all_done, 1);
+    for (int b = 0; b < 2; ++b) { mbar_init(&q_full[b], 1); mbar_init(&q_free[b], 1); mbar_init(&stat_full[b], 1); mbar_init(&stat_free[b], 8); }
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tm_qkv);
@@ -126,241 +144,326 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 256 + D;
+  const uint32_t t_dq = t_dp;
 
-  if (warp == 0) {
-    if (elect_one()) {
-      mbar_arrive_expect_tx(kv_full, 2 * L::TILE);
+  if (warp < 4) {
+    setmaxnreg_dec<AB_REGS_IO>();
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer
+      if (elect_one()) {
+        mbar_arrive_expect_tx(kv_full, 2 * L::TILE);
 #pragma unroll
-      for (int kb = 0; kb < KB; ++kb) {
-        tma_load_2d(smem + L::OFF_K + kb * 16384, &tm_qkv, kv_full, (p.Hq + hk) * D + kb * 64, seq_start + k0);
-        tma_load_2d(smem + L::OFF_V + kb * 16384, &tm_qkv, kv_full, (p.Hq + p.Hkv + hk) * D + kb * 64, seq_start + k0);
-      }
-      for (int it = 0; it < n_iters; ++it) {
-        const int h = hk * G + it / per_head, i = jblk + it % per_head;
-        // Q is released first (after dK), dO second (after dV): both loads overlap the tail of the MMAs
-        if (it > 0 && !mbar_wait(q_free, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 21); goto done; }
-        mbar_arrive_expect_tx(qdo_full, L::TILE);
-#pragma unroll
-        for (int kb = 0; kb < KB; ++kb)
-          tma_load_2d(smem + L::OFF_Q + kb * 16384, &tm_qkv, qdo_full, h * D + kb * 64, seq_start + i * AB_B);
-        if (it > 0 && !mbar_wait(do_free, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 21); goto done; }
-        mbar_arrive_expect_tx(do_full, L::TILE);
-#pragma unroll
-        for (int kb = 0; kb < KB; ++kb)
-          tma_load_2d(smem + L::OFF_DO + kb * 16384, &tm_do, do_full, h * D + kb * 64, seq_start + i * AB_B);
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t id_nt = make_idesc_bf16(AB_B, AB_B, false, false);   // S, dP
-      constexpr uint32_t id_dq = make_idesc_bf16(AB_B, D, false, true);       // dQ = dS K
-      constexpr uint32_t id_tn = make_idesc_bf16(AB_B, D, true, true);        // dV, dK
-      const uint32_t sk = smem_u32(smem + L::OFF_K), sv = smem_u32(smem + L::OFF_V), sq = smem_u32(smem + L::OFF_Q);
-      const uint32_t sdo = smem_u32(smem + L::OFF_DO), spp = smem_u32(smem + L::OFF_P), sds = smem_u32(smem + L::OFF_DS);
-      // every tile lives at a fixed shared-memory address, so the descriptors are built once; inside
-      // the loop a k-step is one 64-bit add (start-address field, in 16-byte units)
-      const uint64_t dQk = make_smem_desc(sq, 16, 1024), dKk = make_smem_desc(sk, 16, 1024);
-      const uint64_t dDOk = make_smem_desc(sdo, 16, 1024), dVk = make_smem_desc(sv, 16, 1024);
-      const uint64_t dDSk = make_smem_desc(sds, 16, 1024);
-      const uint64_t dDSm = make_smem_desc(sds, 16384, 1024), dPm = make_smem_desc(spp, 16384, 1024);
-      const uint64_t dQm = make_smem_desc(sq, 16384, 1024), dDOm = make_smem_desc(sdo, 16384, 1024);
-      const uint64_t dKm = make_smem_desc(sk, 16384, 1024);
-      auto kstep = [](int k) { return static_cast<uint64_t>((k >> 2) * 1024 + (k & 3) * 2); };   // K-major: 32 B per step, 16 KB per 64
-      auto mstep = [](int k) { return static_cast<uint64_t>(k * 128); };                           // MN-major: 2048 B per step
-      if (!mbar_wait(kv_full, 0, abort_flag)) { atomicExch(p.status, 22); goto done; }
-      for (int it = 0; it < n_iters; ++it) {
-        if (!mbar_wait(qdo_full, it & 1, abort_flag)) { atomicExch(p.status, 23); goto done; }
-        if (it > 0 && !mbar_wait(dq_read, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 24); goto done; }
-        tc_fence_after();
-        MTB_STAMP(blockIdx.x == 0, it, 0);
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          umma_bf16(t_s, dQk + kstep(k), dKk + kstep(k), id_nt, k != 0);
+        for (int kb = 0; kb < KB; ++kb) {
+          tma_load_2d(smem + L::OFF_K + kb * 16384, &tm_qkv, kv_full, (p.Hq + hk) * D + kb * 64, seq_start + k0);
+          tma_load_2d(smem + L::OFF_V + kb * 16384, &tm_qkv, kv_full, (p.Hq + p.Hkv + hk) * D + kb * 64, seq_start + k0);
         }
-        if (!mbar_wait(do_full, it & 1, abort_flag)) { atomicExch(p.status, 23); goto done; }
-        tc_fence_after();
+        int h = h_first, i = jblk;
+        for (int it = 0; it < n_iters; ++it) {
+          const int b = it & 1;
+          if (it > 1 && !mbar_wait(&q_free[b], ((it - 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 21); goto done; }
+          mbar_arrive_expect_tx(&q_full[b], L::TILE);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          umma_bf16(t_dp, dDOk + kstep(k), dVk + kstep(k), id_nt, k != 0);
+          for (int kb = 0; kb < KB; ++kb)
+            tma_load_2d(smem + L::OFF_Q + b * L::TILE + kb * 16384, &tm_qkv, &q_full[b], h * D + kb * 64, seq_start + i * AB_B);
+          if (it > 0 && !mbar_wait(do_free, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 21); goto done; }
+          mbar_arrive_expect_tx(do_full, L::TILE);
+#pragma unroll
+          for (int kb = 0; kb < KB; ++kb)
+            tma_load_2d(smem + L::OFF_DO + kb * 16384, &tm_do, do_full, h * D + kb * 64, seq_start + i * AB_B);
+          if (++i == nq) { i = jblk; ++h; }
         }
-        umma_commit(sdp_full);
-        MTB_STAMP(blockIdx.x == 0, it, 1);
-        if (!mbar_wait(pds_ready, it & 1, abort_flag)) { atomicExch(p.status, 25); goto done; }
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issuer
+      if (elect_one()) {
+        constexpr uint32_t id_nt = make_idesc_bf16(AB_B, AB_B, false, false);   // S^T, dP^T
+        constexpr uint32_t id_ts = make_idesc_bf16(AB_B, D, false, true);       // dV, dK (A in tensor memory)
+        constexpr uint32_t id_dq = make_idesc_bf16(AB_B, D, true, true);        // dQ = dS K
+        // every tile lives at a fixed shared-memory address, so the descriptors are built once; inside
+        // the loop a k-step is one add (start-address field, in 16-byte units)
+        const uint32_t sk = smem_u32(smem + L::OFF_K), sq = smem_u32(smem + L::OFF_Q), sdo = smem_u32(smem + L::OFF_DO);
+        const uint32_t dKk = smem_desc_lo(sk, 16), dVk = smem_desc_lo(smem_u32(smem + L::OFF_V), 16);
+        const uint32_t dQk = smem_desc_lo(sq, 16), dDOk = smem_desc_lo(sdo, 16);
+        const uint32_t dDSm = smem_desc_lo(smem_u32(smem + L::OFF_DS), 16384), dKm = smem_desc_lo(sk, 16384);
+        const uint32_t dQm = smem_desc_lo(sq, 16384), dDOm = smem_desc_lo(sdo, 16384);
+        auto kstep = [](int k) { return static_cast<uint32_t>((k >> 2) * 1024 + (k & 3) * 2); };   // K-major: 32 B per step, 16 KB per 64
+        auto mstep = [](int k) { return static_cast<uint32_t>(k * 128); };                           // MN-major: 2048 B per step
+        auto astep = [](int k) { return static_cast<uint32_t>(k < 4 ? k * 8 : 64 + (k - 4) * 8); };   // bf16 A operand in tensor memory
+        auto qbuf = [&](int it) { return static_cast<uint32_t>((it & 1) * (L::TILE >> 4)); };
+        auto issue_s = [&](int it) {
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) umma_bf16_lo(t_s, dKk + kstep(k), dQk + qbuf(it) + kstep(k), id_nt, k != 0);
+          umma_commit(s_full);
+        };
+        auto issue_dp = [&]() {   // dV of the same iteration has been issued: dO is free when both are done
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) umma_bf16_lo(t_dp, dVk + kstep(k), dDOk + kstep(k), id_nt, k != 0);
+          umma_commit(dp_full);
+        };
+        auto issue_dv = [&](int it) {
+#pragma unroll
+          for (int k = 0; k < AB_B / 16; ++k) umma_bf16_ts_lo(t_dv, t_s + astep(k), dDOm + mstep(k), id_ts, it != 0 || k != 0);
+        };
+        if (!mbar_wait(kv_full, 0, abort_flag)) { atomicExch(p.status, 22); goto done; }
+        if (!mbar_wait(&q_full[0], 0, abort_flag)) { atomicExch(p.status, 23); goto done; }
         tc_fence_after();
-        MTB_STAMP(blockIdx.x == 0, it, 2);
-        // dK += dS^T Q, then dV += P^T dO  (A = [query, key] tile read MN-major, B = [query, D] tile read MN-major)
-#pragma unroll
-        for (int k = 0; k < AB_B / 16; ++k)
-          umma_bf16(t_dk, dDSm + mstep(k), dQm + mstep(k), id_tn, (it | k) != 0);
-        umma_commit(q_free);
-#pragma unroll
-        for (int k = 0; k < AB_B / 16; ++k)
-          umma_bf16(t_dv, dPm + mstep(k), dDOm + mstep(k), id_tn, (it | k) != 0);
+        issue_s(0);
+        if (!mbar_wait(do_full, 0, abort_flag)) { atomicExch(p.status, 23); goto done; }
+        tc_fence_after();
+        issue_dp();
+        if (!mbar_wait(p_ready, 0, abort_flag)) { atomicExch(p.status, 25); goto done; }
+        tc_fence_after();
+        issue_dv(0);
         umma_commit(do_free);
-        // dQ = dS K  (A K-major over keys, B = K tile read MN-major), into the columns S occupied
+        if (n_iters > 1) {
+          if (!mbar_wait(&q_full[1], 0, abort_flag)) { atomicExch(p.status, 23); goto done; }
+          tc_fence_after();
+          issue_s(1);
+        }
+        for (int it = 0; it < n_iters; ++it) {
+          if (!mbar_wait(ds_ready, it & 1, abort_flag)) { atomicExch(p.status, 25); goto done; }
+          tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < AB_B / 16; ++k)
-          umma_bf16(t_s, dDSk + kstep(k), dKm + mstep(k), id_dq, k != 0);
-        umma_commit(mma_done);
-        MTB_STAMP(blockIdx.x == 0, it, 3);
+          for (int k = 0; k < AB_B / 16; ++k) umma_bf16_ts_lo(t_dk, t_dp + astep(k), dQm + qbuf(it) + mstep(k), id_ts, it != 0 || k != 0);
+          umma_commit(&q_free[it & 1]);
+#pragma unroll
+          for (int k = 0; k < AB_B / 16; ++k) umma_bf16_lo(t_dq, dDSm + mstep(k), dKm + mstep(k), id_dq, k != 0);
+          umma_commit(dq_full);
+          if (it + 1 < n_iters) {
+            if (!mbar_wait(do_full, (it + 1) & 1, abort_flag)) { atomicExch(p.status, 23); goto done; }
+            if (!mbar_wait(p_ready, (it + 1) & 1, abort_flag)) { atomicExch(p.status, 25); goto done; }
+            tc_fence_after();
+            issue_dv(it + 1);
+            if (!mbar_wait(dq_read, it & 1, abort_flag)) { atomicExch(p.status, 24); goto done; }
+            tc_fence_after();
+            issue_dp();
+            umma_commit(do_free);
+            if (it + 2 < n_iters) {
+              if (!mbar_wait(&q_full[it & 1], ((it + 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 23); goto done; }
+              tc_fence_after();
+              issue_s(it + 2);
+            }
+          }
+        }
+        umma_commit(all_done);
+      }
+    } else if (warp == 2) {
+      // ------------------------------------------------------------------ dQ reduce warp
+      if (elect_one()) {
+        const uint32_t stage = smem_u32(smem + L::OFF_ST);
+        int h = h_first, i = jblk, n = 0;
+        for (int it = 0; it < n_iters; ++it) {
+          for (int part = 0; part < KB; ++part, ++n) {
+            if (!mbar_wait(stage_full, n & 1, abort_flag)) { atomicExch(p.status, 30); goto done; }
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
+                           ::"l"(reinterpret_cast<uint64_t>(&tm_dq)), "r"(stage + c * 16384), "r"(h * D + part * 64 + c * 32),
+                             "r"(seq_start + i * AB_B) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            mbar_arrive(stage_free);
+          }
+          if (++i == nq) { i = jblk; ++h; }
+        }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // every add has been performed before the CTA exits
+      }
+    } else {
+      // ------------------------------------------------------------------ row statistics of the query blocks
+      float* stat = reinterpret_cast<float*>(smem + L::OFF_STAT);
+      int h = h_first, i = jblk;
+      for (int it = 0; it < n_iters; ++it) {
+        const int b = it & 1;
+        if (it > 1 && !mbar_wait(&stat_free[b], ((it - 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 32); goto done; }
+        const long long base = static_cast<long long>(h) * p.T + seq_start;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int x = j * 32 + lane, qpos = i * AB_B + x;
+          const bool ok = qpos < seq_len;
+          stat[b * 256 + x] = ok ? p.lse[base + qpos] * -1.4426950408889634f : -INFINITY;
+          stat[b * 256 + 128 + x] = ok ? p.delta[base + qpos] * -p.scale : 0.f;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&stat_full[b]);
+        if (++i == nq) { i = jblk; ++h; }
       }
     }
-  } else if (warp == 10) {
-    // ------------------------------------------------------------------ dQ reduce warp
-    if (elect_one()) {
-      uint8_t* stage_a = smem + L::OFF_P;     // boxes 0 .. D/64-1
-      uint8_t* stage_b = smem + L::OFF_ST2;   // boxes D/64 .. D/32-1
-      for (int it = 0; it < n_iters; ++it) {
-        const int h = hk * G + it / per_head, i = jblk + it % per_head;
-        if (!mbar_wait(stage_full, it & 1, abort_flag)) { atomicExch(p.status, 30); goto done; }
+  } else if (warp >= 12) {
+    // ------------------------------------------------------------------ dQ drain (one thread per query row)
+    setmaxnreg_dec<AB_REGS_DRAIN>();
+    const int r = (warp & 3) * 32 + lane;
+    const uint32_t src = t_dq + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    uint8_t* rowp = smem + L::OFF_ST + r * 128;
+    int n = 0;
+    for (int it = 0; it < n_iters; ++it) {
+      if (!mbar_wait(dq_full, it & 1, abort_flag)) { atomicExch(p.status, 28); goto done; }
+      tc_fence_after();
+#pragma unroll 1
+      for (int part = 0; part < KB; ++part, ++n) {
+        uint32_t v[2][32];
+        tmem_ld_32x32(src + part * 64, v[0]);
+        tmem_ld_32x32(src + part * 64 + 32, v[1]);
+        tmem_ld_wait();
+        if (part == KB - 1) {   // the last columns are in registers: the next dP may overwrite them
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(dq_read);
+        }
+        if (n > 0 && !mbar_wait(stage_free, (n - 1) & 1, abort_flag)) { atomicExch(p.status, 31); goto done; }
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c)
-          asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
-                       ::"l"(reinterpret_cast<uint64_t>(&tm_dq)), "r"(smem_u32(stage_a + c * 16384)), "r"(h * D + c * 32),
-                         "r"(seq_start + i * AB_B) : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        // The second half is only issued once the P tile has been read: boxes in flight together share
-        // the read-out bandwidth, and the next softmax is waiting for the P tile alone.
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        mbar_arrive(stage_free);
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c)
-          asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];"
-                       ::"l"(reinterpret_cast<uint64_t>(&tm_dq)), "r"(smem_u32(stage_b + c * 16384)), "r"(h * D + (D / 64 + c) * 32),
-                         "r"(seq_start + i * AB_B) : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        mbar_arrive(st2_free);
+          for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<uint4*>(rowp + c * 16384 + ((g ^ (r & 7)) << 4)) = make_uint4(v[c][g * 4], v[c][g * 4 + 1], v[c][g * 4 + 2], v[c][g * 4 + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(stage_full);
       }
-      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // every add has been performed before the CTA exits
     }
   } else {
+    // ------------------------------------------------------------------ softmax (two threads per key row)
+    setmaxnreg_inc<AB_REGS_SOFTMAX>();
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;      // which 64 key columns (softmax) / which half of the D columns (drains)
+    const int half = (warp >> 2) - 1;      // which 64 queries (softmax) / which half of the D columns (epilogue)
     const int r = q * 32 + lane;
+    const int kpos = k0 + r;               // position of this thread's key inside the sequence
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    const uint32_t ts = t_s + lane_addr + half * 64, tp = t_dp + lane_addr + half * 64;
     const float sl2 = p.scale * 1.4426950408889634f;
-    const int HqD = p.Hq * D;
+    const float2 sl2v = make_float2(sl2, sl2), scv = make_float2(p.scale, p.scale);
+    uint8_t* ds_row = smem + L::OFF_DS + half * 16384 + r * 128;
+    int i = jblk;
     for (int it = 0; it < n_iters; ++it) {
-      const int h = hk * G + it / per_head, i = jblk + it % per_head;
-      const int qpos = i * AB_B + r;
-      const bool qok = qpos < seq_len;
-      const long long tok = static_cast<long long>(seq_start) + qpos;
-      const float lse2 = qok ? p.lse[static_cast<long long>(h) * p.T + tok] * 1.4426950408889634f : 0.f;
-      const float delta = qok ? p.delta[static_cast<long long>(h) * p.T + tok] : 0.f;
-      if (!mbar_wait(sdp_full, it & 1, abort_flag)) { atomicExch(p.status, 26); goto done; }
+      const int b = it & 1;
+      const float* stat = reinterpret_cast<const float*>(smem + L::OFF_STAT) + b * 256 + half * 64;
+      if (!mbar_wait(&stat_full[b], (it >> 1) & 1, abort_flag)) { atomicExch(p.status, 26); goto done; }
+      if (!mbar_wait(s_full, it & 1, abort_flag)) { atomicExch(p.status, 26); goto done; }
       tc_fence_after();
-      MTB_STAMP(blockIdx.x == 0 && threadIdx.x == 64, it, 4);
-      const bool need_mask = (i == jblk) || (k0 + AB_B > seq_len) || (i * AB_B + AB_B > seq_len);
-      // this thread's 64 columns of S and dP are fetched with all four loads in flight
-      uint32_t sv_[2][32], dv_[2][32];
-      tmem_ld_32x32(t_s + lane_addr + (half * 2) * 32, sv_[0]);
-      tmem_ld_32x32(t_dp + lane_addr + (half * 2) * 32, dv_[0]);
-      tmem_ld_32x32(t_s + lane_addr + (half * 2 + 1) * 32, sv_[1]);
-      tmem_ld_32x32(t_dp + lane_addr + (half * 2 + 1) * 32, dv_[1]);
-      tmem_ld_wait();
-      if (need_mask) {   // diagonal block, last key block or last query block: out-of-range entries get P = 0
+      float2 pr[32];      // probabilities of this thread's 64 (key, query) pairs
+      {
+        uint32_t sv[2][32];
+        tmem_ld_32x32(ts, sv[0]);
+        tmem_ld_32x32(ts + 32, sv[1]);
+        tmem_ld_wait();
+        if (i == jblk || k0 + AB_B > seq_len) {   // diagonal block or last key block: out-of-range entries get P = 0
+          const int q0 = i * AB_B + half * 64;
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
+          for (int cc = 0; cc < 2; ++cc)
 #pragma unroll
-          for (int x = 0; x < 32; ++x) {
-            const int kpos = k0 + (half * 2 + cc) * 32 + x;
-            if (!qok || kpos > qpos || kpos >= seq_len) sv_[cc][x] = 0xff800000u;   // exp2(-inf) = 0
+            for (int x = 0; x < 32; ++x)
+              if (kpos > q0 + cc * 32 + x || kpos >= seq_len) sv[cc][x] = 0xff800000u;   // exp2(-inf) = 0
+        }
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int x = 0; x < 32; x += 4) {
+            const float4 nl = *reinterpret_cast<const float4*>(stat + cc * 32 + x);
+            // packed fp32 pairs: one FMA scales and shifts two scores
+            const float2 a0 = ffma2(make_float2(__uint_as_float(sv[cc][x]), __uint_as_float(sv[cc][x + 1])), sl2v, make_float2(nl.x, nl.y));
+            const float2 a1 = ffma2(make_float2(__uint_as_float(sv[cc][x + 2]), __uint_as_float(sv[cc][x + 3])), sl2v, make_float2(nl.z, nl.w));
+            // a quarter of the exponentials runs on the FMA pipe: the special-function unit bounds this phase
+            const float2 e0 = make_float2(ex2_mufu(a0.x), ex2_mufu(a0.y)), e1 = make_float2(ex2_mufu(a1.x), ex2_fma(a1.y));
+            pr[cc * 16 + (x >> 1)] = e0;
+            pr[cc * 16 + (x >> 1) + 1] = e1;
+            pk[x >> 1] = pack_bf16(e0.x, e0.y);
+            pk[(x >> 1) + 1] = pack_bf16(e1.x, e1.y);
           }
+          tmem_st_32x16(ts + cc * 16, pk);
+        }
       }
-      // The P tile still holds half of the previous dQ tile until its reduces have read it. The first 32
-      // columns are computed before that wait; their stores then overlap the math of the other 32.
-      uint32_t pk[2][16], dk[2][16];
-      const float2 sl2v = make_float2(sl2, sl2), nlse = make_float2(-lse2, -lse2);
-      const float2 scv = make_float2(p.scale, p.scale), nds = make_float2(-delta * p.scale, -delta * p.scale);
-      auto compute = [&](int cc) {
-#pragma unroll
-        for (int x = 0; x < 32; x += 2) {
-          // packed fp32 pairs: one FMA scales and shifts two scores, one FMA forms (dP - delta) * scale for both
-          const float2 a = ffma2(make_float2(__uint_as_float(sv_[cc][x]), __uint_as_float(sv_[cc][x + 1])), sl2v, nlse);
-          // a quarter of the exponentials runs on the FMA pipe: the special-function unit bounds this phase
-          const float2 pr = make_float2(ex2_mufu(a.x), (x & 2) ? ex2_fma(a.y) : ex2_mufu(a.y));
-          const float2 dd = ffma2(make_float2(__uint_as_float(dv_[cc][x]), __uint_as_float(dv_[cc][x + 1])), scv, nds);
-          const float2 ds = fmul2(pr, dd);
-          pk[cc][x >> 1] = pack_bf16(pr.x, pr.y);
-          dk[cc][x >> 1] = pack_bf16(ds.x, ds.y);
-        }
-      };
-      auto store = [&](int cc) {
-        const int c = half * 2 + cc;
-        const int rowoff = (c >> 1) * 16384 + r * 128;
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          const int chunk = (((c & 1) * 4 + g) ^ (r & 7)) << 4;
-          *reinterpret_cast<uint4*>(smem + L::OFF_P + rowoff + chunk) = make_uint4(pk[cc][g * 4], pk[cc][g * 4 + 1], pk[cc][g * 4 + 2], pk[cc][g * 4 + 3]);
-          *reinterpret_cast<uint4*>(smem + L::OFF_DS + rowoff + chunk) = make_uint4(dk[cc][g * 4], dk[cc][g * 4 + 1], dk[cc][g * 4 + 2], dk[cc][g * 4 + 3]);
-        }
-      };
-      compute(0);
-      MTB_STAMP(blockIdx.x == 0 && threadIdx.x == 64, it, 5);
-      if (it > 0 && !mbar_wait(stage_free, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 27); goto done; }
-      MTB_STAMP(blockIdx.x == 0 && threadIdx.x == 64, it, 6);
-      store(0);
-      compute(1);
-      store(1);
-      fence_proxy_async_smem();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_ready);
-      // drain dQ: TMEM -> fp32 staging (128B-swizzled boxes); the reduce warp adds the boxes into global memory
-      if (!mbar_wait(mma_done, it & 1, abort_flag)) { atomicExch(p.status, 28); goto done; }
-      if (half == 1 && it > 0 && !mbar_wait(st2_free, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 31); goto done; }
+      if (lane == 0) mbar_arrive(p_ready);
+      if (!mbar_wait(dp_full, it & 1, abort_flag)) { atomicExch(p.status, 27); goto done; }
       tc_fence_after();
-      MTB_STAMP(blockIdx.x == 0 && threadIdx.x == 64, it, 7);
-      uint8_t* stage = half == 0 ? smem + L::OFF_P : smem + L::OFF_ST2;
-      // both loads in flight; the S columns are released as soon as the tile is in registers, so the
-      // next S = Q K^T runs under the staging stores
-      uint32_t v[D / 64][32];
-#pragma unroll
-      for (int cc = 0; cc < D / 64; ++cc) tmem_ld_32x32(t_s + lane_addr + (half * (D / 64) + cc) * 32, v[cc]);
+      uint32_t dv[2][32];
+      tmem_ld_32x32(tp, dv[0]);
+      tmem_ld_32x32(tp + 32, dv[1]);
       tmem_ld_wait();
+#pragma unroll
+      for (int cc = 0; cc < 2; ++cc) {
+        uint32_t dk[16];
+#pragma unroll
+        for (int x = 0; x < 32; x += 4) {
+          const float4 nd = *reinterpret_cast<const float4*>(stat + 128 + cc * 32 + x);
+          // one FMA forms (dP - delta) * scale for two entries
+          const float2 d0 = ffma2(make_float2(__uint_as_float(dv[cc][x]), __uint_as_float(dv[cc][x + 1])), scv, make_float2(nd.x, nd.y));
+          const float2 d1 = ffma2(make_float2(__uint_as_float(dv[cc][x + 2]), __uint_as_float(dv[cc][x + 3])), scv, make_float2(nd.z, nd.w));
+          const float2 s0 = fmul2(pr[cc * 16 + (x >> 1)], d0), s1 = fmul2(pr[cc * 16 + (x >> 1) + 1], d1);
+          dk[x >> 1] = pack_bf16(s0.x, s0.y);
+          dk[(x >> 1) + 1] = pack_bf16(s1.x, s1.y);
+        }
+        tmem_st_32x16(tp + cc * 16, dk);
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          *reinterpret_cast<uint4*>(ds_row + (((cc * 4 + g) ^ (r & 7)) << 4)) = make_uint4(dk[g * 4], dk[g * 4 + 1], dk[g * 4 + 2], dk[g * 4 + 3]);
+      }
+      tmem_st_wait();
+      fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(dq_read);
-#pragma unroll
-      for (int cc = 0; cc < D / 64; ++cc) {
-        uint8_t* rowp = stage + cc * 16384 + r * 128;
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          *reinterpret_cast<uint4*>(rowp + ((g ^ (r & 7)) << 4)) = make_uint4(v[cc][g * 4], v[cc][g * 4 + 1], v[cc][g * 4 + 2], v[cc][g * 4 + 3]);
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(stage_full);
-      MTB_STAMP(blockIdx.x == 0 && threadIdx.x == 64, it, 8);
+      if (lane == 0) { mbar_arrive(ds_ready); mbar_arrive(&stat_free[b]); }
+      if (++i == nq) i = jblk;
     }
     // epilogue: dK, dV (rows = keys)
-    if (n_iters > 0) {
-      if (!mbar_wait(mma_done, (n_iters - 1) & 1, abort_flag)) { atomicExch(p.status, 29); goto done; }
-      tc_fence_after();
-      const int kpos = k0 + r;
-      const bool ok = kpos < seq_len;
-      __nv_bfloat16* rowp = p.dqkv + (static_cast<long long>(seq_start) + kpos) * p.ldq;
-#pragma unroll 1
-      for (int which = 0; which < 2; ++which) {
-        const uint32_t src = (which == 0 ? t_dk : t_dv) + lane_addr;
-        __nv_bfloat16* o = rowp + (which == 0 ? (p.Hq + hk) * D : (p.Hq + p.Hkv + hk) * D);
-#pragma unroll 1
-        for (int cc = 0; cc < D / 64; ++cc) {
-          const int c = half * (D / 64) + cc;
-          uint32_t v[32];
-          tmem_ld_32x32(src + c * 32, v);
-          tmem_ld_wait();
-          if (ok) {
+    if (!mbar_wait(all_done, 0, abort_flag)) { atomicExch(p.status, 29); goto done; }
+    tc_fence_after();
+    const bool ok = kpos < seq_len;
+    __nv_bfloat16* rowp = p.dqkv + (static_cast<long long>(seq_start) + kpos) * p.ldq;
+    auto store = [&](int which, int c, const float (&f)[32]) {   // 32 columns of this thread's row of dK (0) or dV (1)
+      if (!ok) return;
+      __nv_bfloat16* o = rowp + (which == 0 ? (p.Hq + hk) * D : (p.Hq + p.Hkv + hk) * D) + c * 32;
 #pragma unroll
-            for (int g = 0; g < 4; ++g)
-              *reinterpret_cast<uint4*>(o + c * 32 + g * 8) =
-                  make_uint4(pack_bf16(__uint_as_float(v[g * 8]), __uint_as_float(v[g * 8 + 1])),
-                             pack_bf16(__uint_as_float(v[g * 8 + 2]), __uint_as_float(v[g * 8 + 3])),
-                             pack_bf16(__uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5])),
-                             pack_bf16(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7])));
+      for (int g = 0; g < 4; ++g)
+        *reinterpret_cast<uint4*>(o + g * 8) = make_uint4(pack_bf16(f[g * 8], f[g * 8 + 1]), pack_bf16(f[g * 8 + 2], f[g * 8 + 3]),
+                                                          pack_bf16(f[g * 8 + 4], f[g * 8 + 5]), pack_bf16(f[g * 8 + 6], f[g * 8 + 7]));
+    };
+    constexpr int CH = D / 64;            // 32-column pieces per thread and gradient
+    constexpr int PART = 2 * CH * 1024;   // floats of a warp's partial
+    float* base = p.ws + (static_cast<long long>(unit) * p.splits * 8 + (warp - 4)) * PART + lane * 4;   // split s: + s * 8 * PART
+#pragma unroll 1
+    for (int x = 0; x < 2 * CH; ++x) {
+      const int which = x / CH, c = half * CH + x % CH;
+      uint32_t v[32];
+      tmem_ld_32x32((which == 0 ? t_dk : t_dv) + lane_addr + c * 32, v);
+      tmem_ld_wait();
+      float f[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+      if (p.splits == 1) store(which, c, f);
+      else {   // lane-interleaved 16-byte pieces: every access is one contiguous 512 bytes
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          __stcg(reinterpret_cast<float4*>(base + static_cast<long long>(sub) * 8 * PART + x * 1024 + j * 128), make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]));
+      }
+    }
+    if (p.splits > 1) {   // the warp that arrives last adds the partials, in split order whoever that is; nobody waits
+      unsigned* counter = p.counters + unit * 8 + (warp - 4);
+      __threadfence();
+      __syncwarp();
+      unsigned old = 0;
+      if (lane == 0) old = atomicAdd(counter, 1u);
+      old = __shfl_sync(0xffffffffu, old, 0);
+      if (old == static_cast<unsigned>(p.splits) - 1) {
+        __threadfence();
+#pragma unroll 1
+        for (int x = 0; x < 2 * CH; ++x) {
+          float f[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) f[j] = 0.f;
+#pragma unroll 2
+          for (int s = 0; s < p.splits; ++s) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float4 t = __ldcg(reinterpret_cast<const float4*>(base + static_cast<long long>(s) * 8 * PART + x * 1024 + j * 128));
+              f[4 * j] += t.x; f[4 * j + 1] += t.y; f[4 * j + 2] += t.z; f[4 * j + 3] += t.w;
+            }
           }
+          store(x / CH, half * CH + x % CH, f);
         }
+        if (lane == 0) *counter = 0;
       }
     }
   }
@@ -373,23 +476,29 @@ done:
   }
 }
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (t, h).
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; D / 8 lanes per (t, h), one 16-byte load of each operand per lane. Bound by
+// reading dO and O once: 16 384 tokens x 32 heads x 128 63 us (one warp per row with 4-byte loads: 97 us).
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo, const __nv_bfloat16* __restrict__ dout,
                                                         long long lddo, float* __restrict__ delta, int T, int Hq, int D) {
-  const long long w = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= static_cast<long long>(T) * Hq) return;
-  const int t = static_cast<int>(w / Hq), h = static_cast<int>(w % Hq);
-  const __nv_bfloat16* a = o + static_cast<long long>(t) * ldo + h * D;
-  const __nv_bfloat16* b = dout + static_cast<long long>(t) * lddo + h * D;
+  const int lanes = D >> 3;   // 8 or 16: a power of two that divides the warp
+  const long long x = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const long long row = x / lanes;
+  const int c = static_cast<int>(x - row * lanes) * 8;
+  const bool ok = row < static_cast<long long>(T) * Hq;
+  const int t = static_cast<int>(row / Hq), h = static_cast<int>(row - static_cast<long long>(t) * Hq);
   float s = 0.f;
-  for (int c = lane * 2; c < D; c += 64) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a + c));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(b + c));
-    s += x.x * y.x + x.y * y.y;
+  if (ok) {
+    const uint4 a = *reinterpret_cast<const uint4*>(o + static_cast<long long>(t) * ldo + h * D + c);
+    const uint4 b = *reinterpret_cast<const uint4*>(dout + static_cast<long long>(t) * lddo + h * D + c);
+    const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 u = unpack_bf16(av[i]), v = unpack_bf16(bv[i]);
+      s += u.x * v.x + u.y * v.y;
+    }
   }
-  s = warp_sum(s);
-  if (lane == 0) delta[static_cast<long long>(h) * T + t] = s;
+  for (int m = lanes >> 1; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+  if (ok && c == 0) delta[static_cast<long long>(h) * T + t] = s;
 }
 
 // dqkv[t, 0:Hq*D] = bf16(dq_acc[t, :])
@@ -412,7 +521,7 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem<D>::TOTAL) != cudaSuccess) return -4;
     configured = true;
   }
-  kern<<<n_items * p.Hkv, AB_THREADS, AttBwdSmem<D>::TOTAL, st>>>(a, b, c, p);
+  kern<<<n_items * p.Hkv * p.splits, AB_THREADS, AttBwdSmem<D>::TOTAL, st>>>(a, b, c, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -420,9 +529,10 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
 
 // plan: key-block work table [n_items, 3] = (seq_start, seq_len, k0), most work first.
 // dq_acc: zero-initialised fp32 [T, Hq*D] scratch; delta: fp32 [Hq, T] scratch.
+// ws: optional workspace of ws_bytes, as the split-K GEMM's (its first SPLIT_COUNTER_BYTES are zero before and after a launch).
 extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, long long ldo, const void* dout, long long lddo,
                                void* dqkv, long long ldq, const float* lse, float* delta, float* dq_acc, const int* plan,
-                               int n_items, int T, int Hq, int Hkv, int D, int reserved, float scale, int* status, cudaStream_t st) {
+                               int n_items, int T, int Hq, int Hkv, int D, float* ws, long long ws_bytes, float scale, int* status, cudaStream_t st) {
   using namespace mtb;
   if (n_items <= 0 || T <= 0) return 0;
   if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8 || lddo % 8 || ldq % 8) return -10;
@@ -433,21 +543,23 @@ extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, l
   if (rc) return rc - 10;
   rc = make_tmap_2d_f32(&tdq, dq_acc, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(Hq) * D, 32, 128);
   if (rc) return rc - 20;
-  const long long warps = static_cast<long long>(T) * Hq;
-  attn_delta_kernel<<<static_cast<int>((warps * 32 + 255) / 256), 256, 0, st>>>(
+  const long long delta_threads = static_cast<long long>(T) * Hq * (D / 8);
+  attn_delta_kernel<<<static_cast<int>((delta_threads + 255) / 256), 256, 0, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(out), ldo, reinterpret_cast<const __nv_bfloat16*>(dout), lddo, delta, T, Hq, D);
-  (void)reserved;
-  AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, scale, status};
+  // A key block of a kv head is one CTA's work; with few kv heads and a short batch that leaves SMs idle (2 kv heads, 6000
+  // tokens: 94 CTAs of very different length on 148 SMs), so the query heads of a block are divided until there are about two
+  // CTAs per SM (5987 tokens, 12/2 heads: 437 -> 137 us, 7001 tokens, 24/2 heads: 1141 -> 357 us, both with the reordered loop). More gain nothing: every CTA loads K and V again and adds a partial.
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long units = static_cast<long long>(n_items) * Hkv;
+  int splits = 1;
+  if (ws != nullptr && units * 8 * 4 <= SPLIT_COUNTER_BYTES)
+    while (splits < Hq / Hkv && units * splits < 2 * sms && (splits + 1) * units * 2 * AB_B * D * 4 <= ws_bytes - SPLIT_COUNTER_BYTES) ++splits;
+  AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, splits,
+                 ws == nullptr ? nullptr : ws + SPLIT_COUNTER_BYTES / 4, reinterpret_cast<unsigned*>(ws), scale, status};
   rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, p, n_items, st);
   if (rc) return rc;
   attn_dq_store_kernel<<<dim3(static_cast<unsigned>(T), (Hq * D / 8 + 255) / 256), 256, 0, st>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, T, Hq * D);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
-
-#ifdef MTB200_ATTN_BWD_TIMESTAMPS
-// Copies the phase timestamps recorded by the last launch to the host (development builds only).
-extern "C" int mtb200_attn_bwd_debug_read(long long* out, int n) {
-  if (n > mtb::DBG_ITERS * 9) n = mtb::DBG_ITERS * 9;
-  return cudaMemcpyFromSymbol(out, mtb::g_attn_bwd_dbg, sizeof(long long) * n) == cudaSuccess ? 0 : -1;
-}
-#endif

@@ -78,7 +78,7 @@ class _Sig:
     mtb200_moe_combine = [P, P, P, P, P, F, I, I, I, P, P]
     mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
-    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, F, P, P]
+    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, P, L, F, P, P]
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
@@ -382,10 +382,12 @@ class NativeOps:
         plan = self._attn_plan(cu_host, 128, False)
         delta = torch.empty(hq, T, dtype=torch.float32, device=self.device)
         dq_acc = torch.zeros(T, hq * d, dtype=torch.float32, device=self.device)
+        st = self._st()
+        ws = self._split_workspace(st)
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
-                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, 0, scale,
-                   self.status.data_ptr(), self._st(), n=3)
+                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, ws.data_ptr(), ws.numel() * 4, scale,
+                   self.status.data_ptr(), st, n=3)
         return dqkv
 
     # Library attention (flash-attn 2): selectable for A/B comparisons, and the path of head dimensions the

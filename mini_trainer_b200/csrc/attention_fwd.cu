@@ -1,24 +1,27 @@
 // Varlen causal GQA attention forward for sm_100a.
 //
-// One CTA handles one (sequence, 128-row query block, query head). Q, K and V are read straight
-// out of the fused qkv activation [T, (Hq + 2 Hkv) * D] through ONE tensor map (128B swizzle):
-//   S = Q K^T      tcgen05.mma, M=128 queries, N=128 keys, K=D      (accumulator in TMEM, 2 buffers)
-//   P = softmax    8 warps, two threads per query row, read S from TMEM, write bf16 P to smem (2 buffers)
-//   O += P V       tcgen05.mma, M=128, N=D, K=2 x 64 keys            (two accumulators in TMEM)
-// Roles: warp 0 = TMA (K/V double-buffered), warp 1 = MMA issue, warps 2-9 = softmax + epilogue
-// (two threads per query row, each owning 64 of the 128 key columns of a tile).
-// S (TMEM) and P (smem) are double-buffered: Q K^T of tile j+1 and P V of tile j-1 both run under the
-// softmax of tile j, so the softmax warps never wait for the tensor core except to rescale O.
+// A work item is a PAIR of 128-row query tiles A and B that read the same keys: two query heads of one kv head (even GQA
+// ratio), or two consecutive query blocks of one head (odd ratio). Q, K and V are read straight out of the fused qkv
+// activation [T, (Hq + 2 Hkv) * D] through ONE tensor map (128B swizzle):
+//   S = Q K^T      tcgen05.mma, M=128 queries, N=128 keys, K=D      (one accumulator per tile in TMEM)
+//   P = softmax    one warpgroup per tile, one thread per query row: S from TMEM, bf16 P written back over S
+//   O += P V       tcgen05.mma with P as the tensor-memory A operand  (one accumulator per tile)
+// Roles: warp 0 = TMA (K and V double-buffered), warp 1 = MMA issue, warps 4-7 = softmax + epilogue of A, 8-11 of B.
 //
-// The two threads of a query row never talk to each other inside the key loop: each keeps its own
-// online-softmax state (reference maximum, row sum) for its 64 key columns of every tile, and P V is
-// issued as two half-K MMAs into two O accumulators in tensor memory (O_a: key columns 0-63 of each
-// tile, O_b: 64-127). The halves are merged once, in the epilogue, like a split-K softmax:
-//   m = max(m_a, m_b), O = (O_a 2^(m_a-m) + O_b 2^(m_b-m)) / (l_a 2^(m_a-m) + l_b 2^(m_b-m)).
-// (Exchanging the half-row maxima through shared memory and a barrier on every tile cost about a
-// fifth of the softmax time.) A state only rescales its accumulator when its running maximum grew
-// by more than 2^8 (exact: the final merge uses the same references), so the TMEM round trip for the
-// rescale is rare. Only the last key tile of a query block touches the causal diagonal and is masked.
+// Why pairs: a tile's chain is S -> softmax -> P V, and with one tile per CTA the tensor core idles under the softmax and the
+// softmax under the products, or (with two S buffers of one tile) all softmax warps do the same phase at the same time and
+// queue on the special-function unit. Two independent tiles take turns: while A is in its softmax the tensor core runs
+// P V and the next S of B. K and V are loaded and multiplied once per pair. A row belongs to one thread, so nothing is
+// exchanged between threads. 1 x 16384 tokens, 32/8 heads, D = 128: 1.82 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64:
+// 64 us (one tile per CTA, two threads per row: 1.94 ms and 94 us).
+//
+// CTAs are persistent (one per SM): barriers and tensor memory are set up once, K and V of the next item are prefetched
+// under the current one's tail, and the epilogue of an item runs under the next item's first product. Items come most work
+// first and are dealt in alternating direction, so the CTAs' totals differ by about one item.
+//
+// A row's reference maximum only moves (and its accumulator is only rescaled) when the running maximum grew by more than
+// 2^8, which is exact: the same reference is used throughout. Only the last key tile of a query tile touches the causal
+// diagonal and is masked.
 //
 // Masked scores are -inf. The exponentials that run on the special-function unit turn them into exact zeros;
 // the quarter that runs on the FMA pipe (ex2_fma2) clamps its argument at -126 and returns about 1e-38 instead, so
@@ -40,23 +43,21 @@ namespace mtb {
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer);
 
-constexpr int ATT_BM = 128, ATT_BN = 128;
-constexpr int ATT_THREADS = 320;   // TMA warp, MMA warp, 8 softmax warps (two threads per query row)
+constexpr int ATT_B = 128;         // query tile and key tile edge
+constexpr int ATT_THREADS = 384;   // three warpgroups: TMA / MMA, softmax of A, softmax of B
+// Registers per thread after the split; over the three warpgroups they add up to at most the 3 x 168 of the launch.
+// A softmax thread holds the 128 scores of its row.
+constexpr int ATT_REGS_IO = 72, ATT_REGS_SOFTMAX = 216;
+static_assert(ATT_REGS_IO + 2 * ATT_REGS_SOFTMAX <= 3 * 168, "register split");
 
 template <int D>
 struct AttFwdSmem {
-  static constexpr int Q_BYTES = ATT_BM * D * 2;
-  static constexpr int KV_BYTES = ATT_BN * D * 2;
-  static constexpr int P_BYTES = ATT_BM * ATT_BN * 2;
-  static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = OFF_Q + Q_BYTES;        // 2 stages
-  static constexpr int OFF_V = OFF_K + 2 * KV_BYTES;   // 2 stages
-  static constexpr int OFF_P = OFF_V + 2 * KV_BYTES;   // 2 buffers
-  static constexpr int OFF_BAR = OFF_P + 2 * P_BYTES;
-  static constexpr int OFF_MX = OFF_BAR + 256;          // float [reference maximum, row sum][2 halves][128 rows], epilogue only
-  // No alignment slack: with D = 128 the tiles fill 224 KB of the 227 KB a CTA can have. The kernel
-  // checks that the dynamic shared memory window starts on a 1024-byte boundary (swizzle atom).
-  static constexpr int TOTAL = OFF_MX + 2 * 2 * 128 * 4;
+  static constexpr int TILE = ATT_B * D * 2;         // a [128, D] bf16 tile
+  static constexpr int OFF_Q = 0;                    // A, B
+  static constexpr int OFF_K = 2 * TILE;             // 2 stages
+  static constexpr int OFF_V = 4 * TILE;             // 2 stages
+  static constexpr int OFF_BAR = 6 * TILE;
+  static constexpr int TOTAL = OFF_BAR + 256 + 1024;
 };
 
 struct AttFwdParams {
@@ -64,58 +65,72 @@ struct AttFwdParams {
   long long ldo;
   float* lse;
   const int* plan;   // [n_items, 3] = seq_start, seq_len, q0
+  int n_items;
   int T, Hq, Hkv;
+  int row_pairs;     // 0: item x two heads of a kv head; 1: item (256 rows) x one head
   float scale;
   int* status;
 };
 
-// PT: P stays in tensor memory. The softmax threads write bf16 P over the S columns they just read
-// (tcgen05.st; keys 0-63 of a tile into columns 0-31 of its S buffer, keys 64-127 into columns 64-95, so a
-// thread only ever overwrites S columns that it owns) and P V is issued with the A operand in tensor memory.
-// No P tile in shared memory: no st.shared / proxy fence in the softmax loop, no shared-memory reads of P by
-// the tensor core. Q K^T of tile j+2 overwrites the buffer after P V of tile j in the tensor pipe's issue order.
-template <int D, int POLY, bool PT>   // every POLY-th exponential pair runs on the FMA pipe instead of the special-function unit
+// One unit of work: the two query tiles of a pair. n = key tiles (0: no such tile).
+struct AttWork {
+  int seq_start, seq_len, hk, h[2], q0[2], n[2];
+  __device__ __forceinline__ int tiles() const { return n[0] > n[1] ? n[0] : n[1]; }
+};
+
+// The `round`-th unit of this CTA; false when there is none left. A row of the table that does not lie inside the packed
+// batch yields a unit without tiles, which every role skips.
+__device__ __forceinline__ bool att_work(const AttFwdParams& p, int round, AttWork& w) {
+  const int per_item = p.row_pairs ? p.Hq : p.Hq / 2;
+  const int total = p.n_items * per_item;
+  const int u = round * static_cast<int>(gridDim.x) + ((round & 1) ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
+  if (round * static_cast<int>(gridDim.x) >= total) return false;
+  w.n[0] = w.n[1] = 0;
+  if (u >= total) return true;   // the last round may be partial in either direction
+  const int item = u / per_item, x = u - item * per_item;
+  w.seq_start = p.plan[item * 3 + 0]; w.seq_len = p.plan[item * 3 + 1];
+  const int q0 = p.plan[item * 3 + 2];
+  if (w.seq_start < 0 || w.seq_len <= 0 || q0 < 0 || q0 >= w.seq_len || static_cast<long long>(w.seq_start) + w.seq_len > p.T) {
+    atomicExch(p.status, 61);   // reported, not dereferenced
+    return true;
+  }
+  const int G = p.Hq / p.Hkv;
+  w.h[0] = p.row_pairs ? x : 2 * x;
+  w.h[1] = p.row_pairs ? x : 2 * x + 1;
+  w.hk = w.h[0] / G;
+  w.q0[0] = q0;
+  w.q0[1] = p.row_pairs ? q0 + ATT_B : q0;
+  w.n[0] = q0 / ATT_B + 1;
+  w.n[1] = w.q0[1] < w.seq_len ? w.q0[1] / ATT_B + 1 : 0;
+  return true;
+}
+
+template <int D, int POLY>   // every POLY-th exponential pair runs on the FMA pipe instead of the special-function unit
 __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, AttFwdParams p) {
   using L = AttFwdSmem<D>;
   constexpr int KB = D / 64;  // 64-element (128 B) column blocks of a D-wide row
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = smem_raw;
-  if (smem_u32(smem) & 1023u) {   // uniform over the CTA: nothing has been allocated or armed yet
-    if (threadIdx.x == 0) atomicExch(p.status, 10);
-    return;
-  }
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
-  uint64_t* q_full = bars;            // 1
-  uint64_t* k_full = bars + 1;        // 2
-  uint64_t* v_full = bars + 3;        // 2
-  uint64_t* k_empty = bars + 5;       // 2: Q K^T of the tile in this stage has completed
-  uint64_t* v_empty = bars + 7;       // 2: P V of the tile in this stage has completed
-  uint64_t* s_full = bars + 9;        // 2
-  uint64_t* p_ready = bars + 11;      // 2: P buffer written and S buffer consumed (8 arrivals)
-  uint64_t* p_empty = bars + 13;      // 2: P V of the tile in this P buffer has completed
-  uint64_t* mx_bar = bars + 15;       // 1: epilogue, the two threads of every row have published their softmax state
+  uint64_t* q_full = bars;            // both Q tiles of a unit landed
+  uint64_t* q_free = bars + 1;        // every S of the unit has completed
+  uint64_t* k_full = bars + 2;        // [2]
+  uint64_t* k_empty = bars + 4;       // [2] S of both tiles against this K has completed
+  uint64_t* v_full = bars + 6;        // [2]
+  uint64_t* v_empty = bars + 8;       // [2] P V of both tiles has completed
+  uint64_t* s_full = bars + 10;       // [A, B]
+  uint64_t* p_ready = bars + 12;      // [A, B] P in tensor memory, O rescaled (4 arrivals)
+  uint64_t* pv_done = bars + 14;      // [A, B] P V complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int item = blockIdx.x / p.Hq, h = blockIdx.x % p.Hq;
-  const int hk = h / (p.Hq / p.Hkv);
-  const int seq_start = p.plan[item * 3 + 0], seq_len = p.plan[item * 3 + 1], q0 = p.plan[item * 3 + 2];
-  const int n_tiles = q0 / ATT_BN + 1;
-  // bounds check of the host-built work item (uniform over the CTA; nothing allocated or armed yet):
-  // a row that does not lie inside the packed batch is reported, not dereferenced
-  if (seq_start < 0 || seq_len <= 0 || q0 < 0 || q0 >= seq_len || static_cast<long long>(seq_start) + seq_len > p.T) {
-    if (threadIdx.x == 0) atomicExch(p.status, 61);
-    return;
-  }
-
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
+    mbar_init(q_full, 1); mbar_init(q_free, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 8); mbar_init(&p_empty[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); mbar_init(&pv_done[i], 1);
     }
-    mbar_init(mx_bar, 8);
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap);
@@ -124,230 +139,219 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_s0 = tmem_base, tmem_oa = tmem_base + 256, tmem_ob = tmem_base + 384;
+  const uint32_t tmem_base = *tmem_slot;   // S of A and B at columns 0 and 128, O at 256 and 256 + D
 
-  if (warp == 0) {
-    if (elect_one()) {
-      mbar_arrive_expect_tx(q_full, L::Q_BYTES);
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ATT_REGS_IO));
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer
+      if (elect_one()) {
+        AttWork w;
+        uint32_t units = 0, kt = 0;   // units with tiles so far; key tiles so far
+        for (int round = 0; att_work(p, round, w); ++round) {
+          const int n = w.tiles();
+          if (n == 0) continue;
+          if (units > 0 && !mbar_wait(q_free, (units - 1) & 1, abort_flag)) { atomicExch(p.status, 11); goto done; }
+          mbar_arrive_expect_tx(q_full, w.n[1] > 0 ? 2 * L::TILE : L::TILE);
 #pragma unroll
-      for (int kb = 0; kb < KB; ++kb) tma_load_2d(smem + L::OFF_Q + kb * 16384, &tmap, q_full, h * D + kb * 64, seq_start + q0);
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&k_empty[s], ((j >> 1) & 1) ^ 1, abort_flag)) { atomicExch(p.status, 11); goto done; }
-        const int row = seq_start + j * ATT_BN;
-        mbar_arrive_expect_tx(&k_full[s], L::KV_BYTES);
+          for (int g = 0; g < 2; ++g) {
+            if (w.n[g] == 0) continue;
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb)
-          tma_load_2d(smem + L::OFF_K + s * L::KV_BYTES + kb * 16384, &tmap, &k_full[s], (p.Hq + hk) * D + kb * 64, row);
-        if (!mbar_wait(&v_empty[s], ((j >> 1) & 1) ^ 1, abort_flag)) { atomicExch(p.status, 11); goto done; }
-        mbar_arrive_expect_tx(&v_full[s], L::KV_BYTES);
-#pragma unroll
-        for (int kb = 0; kb < KB; ++kb)
-          tma_load_2d(smem + L::OFF_V + s * L::KV_BYTES + kb * 16384, &tmap, &v_full[s], (p.Hq + p.Hkv + hk) * D + kb * 64, row);
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t idesc_qk = make_idesc_bf16(ATT_BM, ATT_BN, false, false);
-      constexpr uint32_t idesc_pv = make_idesc_bf16(ATT_BM, D, false, true);
-      const uint32_t sq = smem_u32(smem + L::OFF_Q), sp = smem_u32(smem + L::OFF_P);
-      // descriptors of tiles at fixed addresses are built once; a k-step is one 64-bit add
-      const uint64_t dQ = make_smem_desc(sq, 16, 1024);
-      const uint64_t dK0 = make_smem_desc(smem_u32(smem + L::OFF_K), 16, 1024);
-      const uint64_t dV0 = make_smem_desc(smem_u32(smem + L::OFF_V), 16384, 1024);
-      const uint64_t dP0 = make_smem_desc(sp, 16, 1024);
-      auto kstep = [](int k) { return static_cast<uint64_t>((k >> 2) * 1024 + (k & 3) * 2); };
-      auto issue_qk = [&](int j) {
-        const uint64_t dK = dK0 + static_cast<uint64_t>((j & 1) * (L::KV_BYTES >> 4));
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k)
-          umma_bf16(tmem_s0 + (j & 1) * ATT_BN, dQ + kstep(k), dK + kstep(k), idesc_qk, k != 0);
-        umma_commit(&s_full[j & 1]);
-        umma_commit(&k_empty[j & 1]);
-      };
-      if (!mbar_wait(q_full, 0, abort_flag)) { atomicExch(p.status, 12); goto done; }
-      for (int j = 0; j < 2 && j < n_tiles; ++j) {
-        if (!mbar_wait(&k_full[j], 0, abort_flag)) { atomicExch(p.status, 13); goto done; }
-        tc_fence_after();
-        issue_qk(j);
-      }
-      for (int j = 0; j < n_tiles; ++j) {
-        const int b = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&p_ready[b], ph, abort_flag)) { atomicExch(p.status, 15); goto done; }
-        if (!mbar_wait(&v_full[b], ph, abort_flag)) { atomicExch(p.status, 16); goto done; }
-        tc_fence_after();
-        const uint64_t dV = dV0 + static_cast<uint64_t>(b * (L::KV_BYTES >> 4));
-        const uint64_t dP = dP0 + static_cast<uint64_t>(b * (L::P_BYTES >> 4));
-#pragma unroll
-        for (int k = 0; k < ATT_BN / 16; ++k) {   // key columns 0-63 accumulate into O_a, 64-127 into O_b
-          constexpr int KH = ATT_BN / 32;
-          if constexpr (PT) {
-            // 16 keys = 8 packed columns; the two halves of P sit at columns 0 and 64 of the S buffer
-            const uint32_t pa = tmem_s0 + b * ATT_BN + (k < KH ? k * 8 : 64 + (k - KH) * 8);
-            umma_bf16_ts(k < KH ? tmem_oa : tmem_ob, pa, dV + static_cast<uint64_t>(k * 128), idesc_pv,
-                         j != 0 || (k != 0 && k != KH));
-          } else {
-            umma_bf16(k < KH ? tmem_oa : tmem_ob, dP + kstep(k), dV + static_cast<uint64_t>(k * 128), idesc_pv,
-                      j != 0 || (k != 0 && k != KH));
+            for (int kb = 0; kb < KB; ++kb)
+              tma_load_2d(smem + L::OFF_Q + g * L::TILE + kb * 16384, &tmap, q_full, w.h[g] * D + kb * 64, w.seq_start + w.q0[g]);
           }
+          for (int j = 0; j < n; ++j, ++kt) {
+            const int s = kt & 1;
+            const uint32_t ph = ((kt >> 1) & 1) ^ 1;
+            const int row = w.seq_start + j * ATT_B;
+            if (!mbar_wait(&k_empty[s], ph, abort_flag)) { atomicExch(p.status, 11); goto done; }
+            mbar_arrive_expect_tx(&k_full[s], L::TILE);
+#pragma unroll
+            for (int kb = 0; kb < KB; ++kb)
+              tma_load_2d(smem + L::OFF_K + s * L::TILE + kb * 16384, &tmap, &k_full[s], (p.Hq + w.hk) * D + kb * 64, row);
+            if (!mbar_wait(&v_empty[s], ph, abort_flag)) { atomicExch(p.status, 11); goto done; }
+            mbar_arrive_expect_tx(&v_full[s], L::TILE);
+#pragma unroll
+            for (int kb = 0; kb < KB; ++kb)
+              tma_load_2d(smem + L::OFF_V + s * L::TILE + kb * 16384, &tmap, &v_full[s], (p.Hq + p.Hkv + w.hk) * D + kb * 64, row);
+          }
+          ++units;
         }
-        umma_commit(&v_empty[b]);
-        umma_commit(&p_empty[b]);
-        if (j + 2 < n_tiles) {   // S buffer b was consumed by the softmax of tile j: refill it with tile j+2
-          if (!mbar_wait(&k_full[b], ((j + 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 14); goto done; }
+      }
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issuer
+      if (elect_one()) {
+        constexpr uint32_t idesc_qk = make_idesc_bf16(ATT_B, ATT_B, false, false);
+        constexpr uint32_t idesc_pv = make_idesc_bf16(ATT_B, D, false, true);
+        // descriptors of tiles at fixed addresses are built once; a k-step is one add
+        const uint32_t dQ = smem_desc_lo(smem_u32(smem + L::OFF_Q), 16);
+        const uint32_t dK = smem_desc_lo(smem_u32(smem + L::OFF_K), 16);
+        const uint32_t dV = smem_desc_lo(smem_u32(smem + L::OFF_V), 16384);
+        auto kstep = [](int k) { return static_cast<uint32_t>((k >> 2) * 1024 + (k & 3) * 2); };
+        auto stage = [](uint32_t t) { return (t & 1) * static_cast<uint32_t>(L::TILE >> 4); };
+        auto issue_s = [&](int g, uint32_t t) {
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k)
+            umma_bf16_lo(tmem_base + g * ATT_B, dQ + g * (L::TILE >> 4) + kstep(k), dK + stage(t) + kstep(k), idesc_qk, k != 0);
+          umma_commit(&s_full[g]);
+        };
+        auto issue_pv = [&](int g, uint32_t t, bool first) {
+#pragma unroll
+          for (int k = 0; k < ATT_B / 16; ++k)   // 16 keys = 8 packed columns of P
+            umma_bf16_ts_lo(tmem_base + 2 * ATT_B + g * D, tmem_base + g * ATT_B + k * 8, dV + stage(t) + k * 128, idesc_pv, !first || k != 0);
+          umma_commit(&pv_done[g]);
+        };
+        AttWork w;
+        uint32_t units = 0, kt = 0;
+        uint32_t cnt[2] = {0, 0};   // tiles of each group so far
+        for (int round = 0; att_work(p, round, w); ++round) {
+          const int n = w.tiles();
+          if (n == 0) continue;
+          if (!mbar_wait(q_full, units & 1, abort_flag)) { atomicExch(p.status, 12); goto done; }
+          if (!mbar_wait(&k_full[kt & 1], (kt >> 1) & 1, abort_flag)) { atomicExch(p.status, 13); goto done; }
           tc_fence_after();
-          issue_qk(j + 2);
+          issue_s(0, kt);
+          if (w.n[1] > 0) issue_s(1, kt);
+          umma_commit(&k_empty[kt & 1]);
+          if (n == 1) umma_commit(q_free);
+          for (int j = 0; j < n; ++j) {
+            const uint32_t t = kt + j;
+            if (!mbar_wait(&v_full[t & 1], (t >> 1) & 1, abort_flag)) { atomicExch(p.status, 16); goto done; }
+            bool k_next = false;
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              if (j >= w.n[g]) continue;
+              if (!mbar_wait(&p_ready[g], cnt[g] & 1, abort_flag)) { atomicExch(p.status, 15); goto done; }
+              tc_fence_after();
+              issue_pv(g, t, j == 0);
+              ++cnt[g];
+              if (j + 1 < w.n[g]) {   // P was the last reader of these columns: the next S of this tile follows at once
+                if (!k_next && !mbar_wait(&k_full[(t + 1) & 1], ((t + 1) >> 1) & 1, abort_flag)) { atomicExch(p.status, 14); goto done; }
+                k_next = true;
+                tc_fence_after();
+                issue_s(g, t + 1);
+              }
+            }
+            umma_commit(&v_empty[t & 1]);
+            if (j + 1 < n) {
+              umma_commit(&k_empty[(t + 1) & 1]);
+              if (j + 2 == n) umma_commit(q_free);
+            }
+          }
+          kt += n;
+          ++units;
         }
       }
     }
   } else {
-    // ---------------------------------------------------------------- softmax + epilogue
-    const int q = warp & 3;                   // TMEM lane quarter
-    const int half = (warp - 2) >> 2;         // which 64 key columns / which half of the O columns
-    const int r = q * 32 + lane;              // row inside the query block
-    const int qpos = q0 + r;                  // position inside the sequence
-    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    // ---------------------------------------------------------------- softmax + epilogue, one thread per query row
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ATT_REGS_SOFTMAX));
+    const int g = (warp >> 2) - 1;            // tile A or B
+    const int r = (warp & 3) * 32 + lane;     // row inside the query tile
+    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t ts = tmem_base + g * ATT_B + lane_addr, to = tmem_base + 2 * ATT_B + g * D + lane_addr;
     const float sl2 = p.scale * 1.4426950408889634f;
-    float m_ref = -INFINITY, l = 0.f;       // state of THIS thread's 64 key columns per tile
-    uint8_t* sp = smem + L::OFF_P;
-    float* mx = reinterpret_cast<float*>(smem + L::OFF_MX);
-    const uint32_t tmem_own = (half == 0 ? tmem_oa : tmem_ob) + lane_addr;
-    for (int j = 0; j < n_tiles; ++j) {
-      if (!mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag)) { atomicExch(p.status, 17); goto done; }
-      tc_fence_after();
-      const uint32_t ts = tmem_s0 + (j & 1) * ATT_BN + lane_addr;
-      const bool diag = (j == n_tiles - 1);
-      const int kbase = j * ATT_BN;
-      // S is read from tensor memory once: this thread's 64 columns stay in registers for both the
-      // maximum and the exponentials. Only the last tile touches the causal diagonal.
-      uint32_t sv[2][32];
-      tmem_ld_32x32(ts + (half * 2) * 32, sv[0]);
-      tmem_ld_32x32(ts + (half * 2 + 1) * 32, sv[1]);
-      tmem_ld_wait();
-      if (diag) {
+    uint32_t cnt = 0;
+    AttWork w;
+    for (int round = 0; att_work(p, round, w); ++round) {
+      const int n = g == 0 ? w.n[0] : w.n[1];
+      if (n == 0) continue;
+      const int qpos = (g == 0 ? w.q0[0] : w.q0[1]) + r;
+      float m_ref = -INFINITY, l = 0.f;
+      for (int j = 0; j < n; ++j, ++cnt) {
+        if (!mbar_wait(&s_full[g], cnt & 1, abort_flag)) { atomicExch(p.status, 17); goto done; }
+        tc_fence_after();
+        // the row of S is read from tensor memory once and stays in registers for the maximum and the exponentials
+        uint32_t sv[4][32];
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
+        for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, sv[c]);
+        tmem_ld_wait();
+        if (j == n - 1) {
+          const int kb = j * ATT_B;
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (kbase + (half * 2 + cc) * 32 + i > qpos) sv[cc][i] = 0xff800000u;   // -inf
-      }
-      float mt = -INFINITY;
+          for (int c = 0; c < 4; ++c)
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc)
+            for (int i = 0; i < 32; ++i)
+              if (kb + c * 32 + i > qpos) sv[c][i] = 0xff800000u;   // -inf
+        }
+        float mc[4];   // four independent chains
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) mt = fmax3(mt, __uint_as_float(sv[cc][i]), __uint_as_float(sv[cc][i + 1]));
-      float factor = 1.f;
-      bool rescale = false;
-      if (mt > m_ref && (mt - m_ref) * sl2 > 8.f) {   // includes the first unmasked tile (m_ref = -inf)
-        factor = (m_ref == -INFINITY) ? 0.f : ex2_mufu((m_ref - mt) * sl2);
-        rescale = (j > 0) && (m_ref != -INFINITY);    // nothing but zeros was accumulated before the first maximum
-        m_ref = mt;
-        l *= factor;
-      }
-      if (!PT && j >= 2) {   // the shared-memory P buffer of this tile must have been read by P V of tile j-2
-        if (!mbar_wait(&p_empty[j & 1], ((j - 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 18); goto done; }
-      }
-      if (j > 0) {
-        if (__any_sync(0xffffffffu, rescale)) {   // this half's O must be complete through tile j-1 before it is rescaled
-          if (!mbar_wait(&p_empty[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { atomicExch(p.status, 18); goto done; }
+        for (int c = 0; c < 4; ++c) {
+          mc[c] = fmaxf(__uint_as_float(sv[c][0]), __uint_as_float(sv[c][1]));
+#pragma unroll
+          for (int i = 2; i < 32; i += 2) mc[c] = fmax3(mc[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
+        }
+        const float mt = fmax3(fmaxf(mc[0], mc[1]), mc[2], mc[3]);
+        float factor = 1.f;
+        bool rescale = false;
+        if (mt > m_ref && (mt - m_ref) * sl2 > 8.f) {   // includes the first tile (m_ref = -inf)
+          factor = (m_ref == -INFINITY) ? 0.f : ex2_mufu((m_ref - mt) * sl2);
+          rescale = j > 0;
+          m_ref = mt;
+          l *= factor;
+        }
+        if (j > 0 && __any_sync(0xffffffffu, rescale)) {   // O must be complete through tile j-1 before it is rescaled
+          if (!mbar_wait(&pv_done[g], (cnt - 1) & 1, abort_flag)) { atomicExch(p.status, 18); goto done; }
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_own + c * 32, v);
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t v[16];
+            tmem_ld_32x16(to + c * 16, v);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
-            tmem_st_32x32(tmem_own + c * 32, v);
+            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * factor);
+            tmem_st_32x16(to + c * 16, v);
           }
-          tmem_st_wait();
         }
-      }
-      // probabilities -> bf16 P in shared memory (K-major, 128B swizzle), row sums; exp2(-inf) = 0 masks.
-      // A state that has seen only masked entries so far (m_ref = -inf) writes zeros.
-      const float mo = (m_ref == -INFINITY) ? 0.f : m_ref * sl2;
-      const float2 sl2v = make_float2(sl2, sl2), nmo = make_float2(-mo, -mo);
-      float2 l2 = make_float2(0.f, 0.f);   // this tile's row sum, two lanes of packed adds
+        // probabilities -> bf16 P over the columns of S, row sum; exp2(-inf) = 0 masks
+        const float mo = (m_ref == -INFINITY) ? 0.f : m_ref * sl2;
+        const float2 sl2v = make_float2(sl2, sl2), nmo = make_float2(-mo, -mo);
+        float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = half * 2 + cc;
-        uint8_t* rowp = sp + (j & 1) * L::P_BYTES + (c >> 1) * 16384 + r * 128;
-        uint32_t pk[16];   // PT: the 32 probabilities of this chunk as 16 packed bf16 pairs
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          float2 e[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < 16; ++i) {
             // scale and shift two scores with one packed FMA; of every POLY pairs one runs its exponentials on the FMA pipe
-            const float2 x = ffma2(make_float2(__uint_as_float(sv[cc][g * 8 + 2 * i]), __uint_as_float(sv[cc][g * 8 + 2 * i + 1])), sl2v, nmo);
-            e[i] = (i % POLY == POLY - 1) ? ex2_fma2(x) : make_float2(ex2_mufu(x.x), ex2_mufu(x.y));
-            l2 = fadd2(l2, e[i]);
+            const float2 x = ffma2(make_float2(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])), sl2v, nmo);
+            const float2 e = (i % POLY == POLY - 1) ? ex2_fma2(x) : make_float2(ex2_mufu(x.x), ex2_mufu(x.y));
+            l2[i & 1] = fadd2(l2[i & 1], e);
+            pk[i] = pack_bf16(e.x, e.y);
           }
-          if constexpr (PT) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) pk[g * 4 + i] = pack_bf16(e[i].x, e[i].y);
-          } else {
-            const int chunk = (c & 1) * 4 + g;
-            uint4 o;
-            o.x = pack_bf16(e[0].x, e[0].y); o.y = pack_bf16(e[1].x, e[1].y); o.z = pack_bf16(e[2].x, e[2].y); o.w = pack_bf16(e[3].x, e[3].y);
-            *reinterpret_cast<uint4*>(rowp + ((chunk ^ (r & 7)) << 4)) = o;
-          }
+          tmem_st_32x16(ts + c * 16, pk);
         }
-        if constexpr (PT) tmem_st_32x16(ts + half * 64 + cc * 16, pk);   // keys (half*64 + cc*32 ..+32) -> 16 packed columns
+        tmem_st_wait();
+        l += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[g]);
       }
-      if constexpr (PT) tmem_st_wait();
-      l += l2.x + l2.y;
-      if constexpr (!PT) fence_proxy_async_smem();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[j & 1]);
-    }
-    // epilogue: merge the two half-row states, O -> out, lse
-    if (!mbar_wait(&p_empty[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, abort_flag)) { atomicExch(p.status, 19); goto done; }
-    tc_fence_after();
-    mx[half * 128 + r] = m_ref;
-    mx[256 + half * 128 + r] = l;
-    __syncwarp();
-    if (lane == 0) mbar_arrive(mx_bar);
-    if (!mbar_wait(mx_bar, 0, abort_flag)) { atomicExch(p.status, 20); goto done; }   // bounded, unlike bar.sync
-    const float m_a = mx[r], m_b = mx[128 + r], l_a = mx[256 + r], l_b = mx[384 + r];
-    const float m_all = fmaxf(m_a, m_b);   // finite: the diagonal entry of every row is unmasked
-    const float f_a = (m_a == -INFINITY) ? 0.f : ex2_mufu((m_a - m_all) * sl2);
-    const float f_b = (m_b == -INFINITY) ? 0.f : ex2_mufu((m_b - m_all) * sl2);
-    const float l_all = l_a * f_a + l_b * f_b;
-    const bool ok = qpos < seq_len;
-    const float inv = 1.f / l_all;
-    const float w_a = f_a * inv, w_b = f_b * inv;
-    const long long tok = static_cast<long long>(seq_start) + qpos;
-    __nv_bfloat16* orow = p.out + tok * p.ldo + h * D;
+      // epilogue: O / l -> out, lse. The next unit's first P V overwrites O only after this thread has handed over its P.
+      if (!mbar_wait(&pv_done[g], (cnt - 1) & 1, abort_flag)) { atomicExch(p.status, 19); goto done; }
+      tc_fence_after();
+      const bool ok = qpos < w.seq_len;
+      const float inv = 1.f / l;
+      const int h = g == 0 ? w.h[0] : w.h[1];
+      const long long tok = static_cast<long long>(w.seq_start) + qpos;
+      __nv_bfloat16* orow = p.out + tok * p.ldo + h * D;
 #pragma unroll 1
-    for (int cc = 0; cc < D / 64; ++cc) {
-      const int c = half * (D / 64) + cc;     // this thread writes half of the D columns of its row
-      uint32_t va[32], vb[32];
-      tmem_ld_32x32(tmem_oa + lane_addr + c * 32, va);
-      tmem_ld_32x32(tmem_ob + lane_addr + c * 32, vb);
-      tmem_ld_wait();
-      if (ok) {
-        float f[32];
+      for (int c = 0; c < D / 32; c += 2) {
+        uint32_t v[2][32];
+        tmem_ld_32x32(to + c * 32, v[0]);
+        tmem_ld_32x32(to + c * 32 + 32, v[1]);
+        tmem_ld_wait();
+        if (ok) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          // an accumulator whose half never saw an unmasked entry holds zeros; w = 0 also covers its garbage-free case
-          f[i] = __uint_as_float(va[i]) * w_a + __uint_as_float(vb[i]) * w_b;
-        }
+          for (int k = 0; k < 8; ++k) {
+            float f[8];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint4 o;
-          o.x = pack_bf16(f[g * 8 + 0], f[g * 8 + 1]);
-          o.y = pack_bf16(f[g * 8 + 2], f[g * 8 + 3]);
-          o.z = pack_bf16(f[g * 8 + 4], f[g * 8 + 5]);
-          o.w = pack_bf16(f[g * 8 + 6], f[g * 8 + 7]);
-          *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) = o;
+            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[k >> 2][(k & 3) * 8 + i]) * inv;
+            *reinterpret_cast<uint4*>(orow + c * 32 + k * 8) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+          }
         }
       }
+      if (ok) p.lse[static_cast<long long>(h) * p.T + tok] = m_ref * p.scale + logf(l);
     }
-    if (ok && half == 0) p.lse[static_cast<long long>(h) * p.T + tok] = m_all * p.scale + logf(l_all);
   }
 done:
   tc_fence_before();
@@ -358,32 +362,37 @@ done:
   }
 }
 
-template <int D, int POLY, bool PT>
-static int launch_fwd(const CUtensorMap& tm, const AttFwdParams& p, int n_items, cudaStream_t st) {
+template <int D, int POLY>
+static int launch_fwd(const CUtensorMap& tm, const AttFwdParams& p, cudaStream_t st) {
   static bool configured = false;
-  auto kern = attn_fwd_kernel<D, POLY, PT>;
+  static int sms = 0;
+  auto kern = attn_fwd_kernel<D, POLY>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttFwdSmem<D>::TOTAL) != cudaSuccess) return -4;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     configured = true;
   }
-  kern<<<n_items * p.Hq, ATT_THREADS, AttFwdSmem<D>::TOTAL, st>>>(tm, p);
+  const long long units = static_cast<long long>(p.n_items) * (p.row_pairs ? p.Hq : p.Hq / 2);
+  if (units > (1 << 30)) return -10;
+  kern<<<static_cast<int>(units < sms ? units : sms), ATT_THREADS, AttFwdSmem<D>::TOTAL, st>>>(tm, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace mtb
 
+// plan: query-block work table [n_items, 3] = (seq_start, seq_len, q0), most work first: blocks of 128 rows when Hq / Hkv is
+// even, of 256 rows (row_pairs) when it is odd.
 extern "C" int mtb200_attn_fwd(const void* qkv, long long ld, void* out, long long ldo, float* lse, const int* plan, int n_items,
-                               int T, int Hq, int Hkv, int D, int reserved, float scale, int* status, cudaStream_t st) {
+                               int T, int Hq, int Hkv, int D, int row_pairs, float scale, int* status, cudaStream_t st) {
   using namespace mtb;
   if (n_items <= 0 || T <= 0) return 0;
-  if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8) return -10;
+  if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || ld % 8 || ldo % 8 || (!row_pairs && (Hq / Hkv) % 2)) return -10;
   CUtensorMap tm;
   const int rc = make_tmap_2d_bf16(&tm, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
   if (rc) return rc;
-  AttFwdParams p{reinterpret_cast<__nv_bfloat16*>(out), ldo, lse, plan, T, Hq, Hkv, scale, status};
-  // a quarter of the exponentials on the FMA pipe: 1011 vs 972 TFLOP/s (2 x 16384 tokens); half of them: no gain
-  // reserved bit 0: P through a shared-memory tile (the earlier form, kept for A/B timing) instead of tensor memory
-  if (reserved & 1) return D == 128 ? launch_fwd<128, 4, false>(tm, p, n_items, st) : launch_fwd<64, 4, false>(tm, p, n_items, st);
+  AttFwdParams p{reinterpret_cast<__nv_bfloat16*>(out), ldo, lse, plan, n_items, T, Hq, Hkv, row_pairs, scale, status};
   // one exponential pair in four on the FMA pipe; one in two and one in eight measured the same within the spread
-  return D == 128 ? launch_fwd<128, 4, true>(tm, p, n_items, st) : launch_fwd<64, 4, true>(tm, p, n_items, st);
+  return D == 128 ? launch_fwd<128, 4>(tm, p, st) : launch_fwd<64, 4>(tm, p, st);
 }

@@ -601,3 +601,24 @@ def test_gemm_split_k(ops, M, N, K, two_cta):
         ops.gemm(at, True, bt, True, o32, M, N, K, two_cta=two_cta)
         assert rel_err(o32, ref) < 1e-5    # fp32 sums of exact products of bf16 values
     ops.check_status()
+
+
+# work tables longer than one round of persistent CTAs; key blocks whose heads one CTA keeps (many units) or several share (few);
+# query tiles that pair up by head (even GQA ratio) or by row block (odd), with a last row block that has no partner
+@pytest.mark.parametrize("D,hq,hkv,lens", [(64, 4, 2, [130] * 100), (128, 6, 2, [257, 1, 128, 255, 256, 300] * 12), (64, 3, 1, [700, 384, 90]),
+                                           (128, 2, 2, [129] * 80)])
+def test_attention_work_distribution(ops, D, hq, hkv, lens):
+    torch.manual_seed(sum(lens))
+    T = sum(lens)
+    qkv, dout = bf(T, (hq + 2 * hkv) * D), bf(T, hq * D)
+    cu_host, cu = _cu(lens)
+    out, lse = ops.attention(qkv, cu, cu_host, max(lens), hq, hkv, D)
+    dqkv = ops.attention_bwd(dout, qkv, out, lse, cu, cu_host, max(lens), hq, hkv, D)
+    ops.check_status()
+    ro, rl = REF.attention(qkv.float(), cu, cu_host, max(lens), hq, hkv, D)
+    rd = REF.attention_bwd(dout.float(), qkv.float(), ro, rl, cu, cu_host, max(lens), hq, hkv, D)
+    assert rel_err(lse, rl) < 2e-3 and rel_err(out, ro) < 1e-2 and max_err(out, ro) < 0.1
+    assert rel_err(dqkv, rd) < 1.5e-2
+    again = ops.attention_bwd(dout, qkv, out, lse, cu, cu_host, max(lens), hq, hkv, D)
+    kv = hq * D
+    assert torch.equal(again[:, kv:], dqkv[:, kv:])     # dK and dV: one order of summation (dQ is accumulated in any order)

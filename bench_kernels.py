@@ -211,7 +211,7 @@ def main():
         tg = torch.randint(0, V, (R,), device="cuda")
         loss = torch.empty(R, device="cuda")
         dlog = torch.empty(R, V, dtype=torch.bfloat16, device="cuda")
-        fn = lambda: ops._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, tg.data_ptr(), loss.data_ptr(), dlog.data_ptr(), V, R, V,
+        fn = lambda: ops._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, None, tg.data_ptr(), loss.data_ptr(), dlog.data_ptr(), V, R, V,
                                1.0, -100, ops._st())
         # two passes over the bf16 logits (online max/sum, then gradient) + the bf16 gradient write
         report(f"ce_fwd_bwd_{R}x{V}", timeit(fn, a.iters, a.warmup, flush), bytes_=R * V * (2.0 + 2.0 + 2.0))

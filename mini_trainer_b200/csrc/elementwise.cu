@@ -52,259 +52,275 @@ __device__ __forceinline__ float block_max(float v, float* red) {
   return red[0];
 }
 
-// ------------------------------------------------------------------------------ RMSNorm fwd
-// y = bf16(x * rstd) * w ; rstd saved. A row is read ONCE: a group of LANES threads (one to eight
-// warps) holds it in registers, VPT 8-wide vectors per thread with all loads issued before the first
-// use, and a 256-thread block works on 256 / LANES rows at a time. One block-wide barrier per row set
-// (none when a row fits one warp).
-template <int VPT>
-__global__ void __launch_bounds__(EW_THREADS) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                                                __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out,
-                                                                float eps, int T, int H, int lanes) {
-  __shared__ float red[EW_THREADS / 32];
+// ------------------------------------------------------------------------------ RMSNorm / LayerNorm fwd
+// RMSNorm    y = bf16(x * rstd) * w ; rstd saved
+// LayerNorm  y = ((x - mean) * rstd) * w + b ; statistics in two passes over the row in registers (the mean first, then the
+//            centred sum of squares), mean and rstd saved
+// A group of LANES threads (one to eight warps) holds a row in registers, VPT 8-wide vectors per thread, and a 256-thread block
+// works on 256 / LANES consecutive rows at a time. Bound by reading x and writing y. Blocks are persistent and rows arrive in
+// shared memory by bulk copies NORM_STAGES row sets ahead: the bytes in flight cost no registers and do not stop for a
+// row's barriers and stores, which is what held the register form back (RMSNorm, 16384 x 4096:
+// 58 -> 53 us; 7001 x 3072: 26 -> 22 us).
+constexpr int NORM_STAGES = 3;
+
+__device__ __forceinline__ float group_sum(float v, float (&red)[EW_THREADS / 32], int lanes, int sub) {
+  v = warp_sum(v);
+  if (lanes > 32) {   // uniform over the block
+    const int wpr = lanes >> 5;
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.f;
+    for (int k = 0; k < wpr; ++k) v += red[sub * wpr + k];
+  }
+  return v;
+}
+
+template <bool LN, int VPT>
+__global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                             const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
+                                                             float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, int T,
+                                                             int H, int lanes, int* status) {
+  extern __shared__ __align__(128) uint8_t norm_smem[];
+  __shared__ uint64_t full[NORM_STAGES];
+  __shared__ float red[2][2][EW_THREADS / 32];   // [parity of the row set][mean, square]
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
   const int rows_per_block = EW_THREADS / lanes;
   const int sub = threadIdx.x / lanes, l = threadIdx.x % lanes;
-  const long long row = static_cast<long long>(blockIdx.x) * rows_per_block + sub;
-  const bool row_ok = row < T;
-  const __nv_bfloat16* xr = x + row * H;
-  bf16x8 v[VPT];
-  float ss = 0.f;
+  const uint32_t set_bytes = static_cast<uint32_t>(rows_per_block) * H * 2;
+  const long long step = static_cast<long long>(gridDim.x) * rows_per_block;
+  const long long first0 = static_cast<long long>(blockIdx.x) * rows_per_block;
+  auto request = [&](long long first, int s) {   // one thread
+    if (first >= T) return;
+    const uint32_t bytes = static_cast<uint32_t>(T - first < rows_per_block ? T - first : rows_per_block) * H * 2;
+    mbar_arrive_expect_tx(&full[s], bytes);
+    bulk_load(norm_smem + s * set_bytes, x + first * H, bytes, &full[s]);
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NORM_STAGES; ++s) mbar_init(&full[s], 1);
+    abort_word = 0;
+    fence_mbar_init();
+    for (int s = 0; s < NORM_STAGES; ++s) request(first0 + s * step, s);
+  }
+  bf16x8 wv[VPT], bv[LN ? VPT : 1];
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
     const int c = (l + k * lanes) * 8;
-    if (row_ok && c < H) v[k].load(xr + c); else v[k].u = make_uint4(0u, 0u, 0u, 0u);
+    wv[k].u = make_uint4(0u, 0u, 0u, 0u);
+    if (LN) bv[k].u = wv[k].u;
+    if (c < H) { wv[k].load(w + c); if (LN) bv[k].load(b + c); }
   }
+  __syncthreads();
+  int it = 0;
+  for (long long first = first0; first < T; first += step, ++it) {
+    const int s = it % NORM_STAGES, par = it & 1;
+    const long long row = first + sub;
+    const bool row_ok = row < T;
+    if (!mbar_wait(&full[s], (it / NORM_STAGES) & 1, abort_flag)) { atomicExch(status, 70); break; }
+    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(norm_smem + s * set_bytes) + sub * H;
+    float f[VPT][8];
+    float acc = 0.f;
 #pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    float f[8]; v[k].to_float(f);
+    for (int k = 0; k < VPT; ++k) {
+      const int c = (l + k * lanes) * 8;
+      bf16x8 v; v.u = make_uint4(0u, 0u, 0u, 0u);
+      if (row_ok && c < H) v.load(src + c);
+      v.to_float(f[k]);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
+      for (int i = 0; i < 8; ++i) acc += LN ? f[k][i] : f[k][i] * f[k][i];
+    }
+    float mean = 0.f;
+    if (LN) {
+      mean = group_sum(acc, red[par][0], lanes, sub) / H;
+      acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        if ((l + k * lanes) * 8 < H) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { f[k][i] -= mean; acc += f[k][i] * f[k][i]; }
+        }
+      }
+    }
+    const float ss = group_sum(acc, red[par][1], lanes, sub);
+    if (lanes <= 32) __syncthreads();
+    // every thread has its part of the rows in registers: the stage may be refilled
+    if (threadIdx.x == 0) request(first + NORM_STAGES * step, s);
+    if (!row_ok) continue;
+    const float rstd = rsqrtf(ss / H + eps);
+    if (l == 0) { rstd_out[row] = rstd; if (LN) mean_out[row] = mean; }
+    __nv_bfloat16* yr = y + row * H;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int c = (l + k * lanes) * 8;
+      if (c < H) {
+        float g[8], h[8]; wv[k].to_float(g);
+        if (LN) bv[k].to_float(h);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[k][i] = LN ? f[k][i] * rstd * g[i] + h[i] : __bfloat162float(__float2bfloat16(f[k][i] * rstd)) * g[i];
+        bf16x8 o; o.from_float(f[k]); o.store(yr + c);
+      }
+    }
   }
-  ss = warp_sum(ss);
-  if (lanes > 32) {   // uniform over the block
-    const int wid = threadIdx.x >> 5, wpr = lanes >> 5;
-    if ((threadIdx.x & 31) == 0) red[wid] = ss;
+}
+
+// ------------------------------------------------------------------------------ RMSNorm / LayerNorm bwd
+// RMSNorm    dx = rstd * (g - xhat * mean(g * xhat)) (+ add_to), g = dy * w, xhat = x * rstd;
+//            dw partial per block in fp32: dwp[block, H] += dy * bf16(xhat)
+// LayerNorm  dx = rstd * (g - mean(g) - xhat * mean(g * xhat)) (+ add_to), xhat = (x - mean) * rstd;
+//            partials dwp[block, 0, :] += dy * xhat, dwp[block, 1, :] += dy (the bias gradient)
+// Partials are summed over blocks by reduce_rows_kernel: no atomics. Bound by reading dy, x (and add_to) and writing dx.
+// Persistent blocks loop over rows, one row per block, VPT 8-wide vectors per thread. Rows arrive in shared memory by bulk
+// copies, `stages` ahead, and the row's statistics one row ahead; the reduction takes one barrier (every thread adds the
+// warps' sums itself, two buffers). Before, a row was load, three barriers, store, and little was in flight meanwhile
+// (RMSNorm with add_to, 16384 x 4096: 149 -> 98 us, 5987 x 1536: 58 -> 31 us; LayerNorm, 16384 x 4096: 222 -> 145 us, 7001 x 3072:
+// 106 -> 52 us; all with the sum over blocks).
+template <bool LN, int VPT>
+__global__ void __launch_bounds__(512) norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                                                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
+                                                      const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ add_to,
+                                                      __nv_bfloat16* __restrict__ dx, float* __restrict__ dwp, int T, int H, int stages,
+                                                      int* status) {
+  constexpr bool KEEP = VPT <= 2;   // wider rows form xhat and g again after the reduction instead of holding them
+  extern __shared__ __align__(128) uint8_t norm_smem[];
+  __shared__ uint64_t full[8];
+  __shared__ float2 red[2][16];
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
+  const int nt = blockDim.x, wid = threadIdx.x >> 5;
+  const uint32_t row_bytes = static_cast<uint32_t>(H) * 2;
+  const uint32_t stage_bytes = row_bytes * (add_to != nullptr ? 3 : 2);
+  auto request = [&](long long row, int s) {   // one thread
+    if (row >= T) return;
+    mbar_arrive_expect_tx(&full[s], stage_bytes);
+    uint8_t* d = norm_smem + s * stage_bytes;
+    bulk_load(d, dy + row * H, row_bytes, &full[s]);
+    bulk_load(d + row_bytes, x + row * H, row_bytes, &full[s]);
+    if (add_to != nullptr) bulk_load(d + 2 * row_bytes, add_to + row * H, row_bytes, &full[s]);
+  };
+  if (threadIdx.x < 32) red[threadIdx.x >> 4][threadIdx.x & 15] = make_float2(0.f, 0.f);   // warps that do not exist add zeros
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) mbar_init(&full[s], 1);
+    abort_word = 0;
+    fence_mbar_init();
+    for (int s = 0; s < stages; ++s) request(blockIdx.x + static_cast<long long>(s) * gridDim.x, s);
+  }
+  float2 dwacc[VPT][4], dbacc[LN ? VPT : 1][4];
+  bf16x8 wv[VPT];
+#pragma unroll
+  for (int v = 0; v < VPT; ++v) {
+    const int c = (threadIdx.x + v * nt) * 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { dwacc[v][i] = make_float2(0.f, 0.f); if (LN) dbacc[v][i] = make_float2(0.f, 0.f); }
+    wv[v].u = make_uint4(0u, 0u, 0u, 0u);
+    if (c < H) wv[v].load(w + c);
+  }
+  float mean = 0.f, rstd = 0.f;
+  if (blockIdx.x < T) { rstd = rstd_in[blockIdx.x]; if (LN) mean = mean_in[blockIdx.x]; }
+  __syncthreads();
+  int it = 0, s = 0;
+  uint32_t ph = 0;
+  for (long long row = blockIdx.x; row < T; row += gridDim.x, ++it) {
+    const long long next = row + gridDim.x;
+    float nmean = 0.f, nrstd = 0.f;
+    if (next < T) { nrstd = rstd_in[next]; if (LN) nmean = mean_in[next]; }
+    if (!mbar_wait(&full[s], ph, abort_flag)) { atomicExch(status, 71); break; }
+    const __nv_bfloat16* sdy = reinterpret_cast<const __nv_bfloat16*>(norm_smem + s * stage_bytes);
+    const float2 rs2 = make_float2(rstd, rstd), mm2 = make_float2(-mean, -mean);
+    auto load2 = [&](const __nv_bfloat16* p, int c, float2 (&f)[4]) {
+      uint4 u = make_uint4(0u, 0u, 0u, 0u);
+      if (c < H) u = *reinterpret_cast<const uint4*>(p + c);
+      f[0] = unpack_bf16(u.x); f[1] = unpack_bf16(u.y); f[2] = unpack_bf16(u.z); f[3] = unpack_bf16(u.w);
+    };
+    auto w2 = [&](int v, int i) { return unpack_bf16(i == 0 ? wv[v].u.x : i == 1 ? wv[v].u.y : i == 2 ? wv[v].u.z : wv[v].u.w); };
+    auto xhat = [&](float2 b) { return LN ? fmul2(fadd2(b, mm2), rs2) : fmul2(b, rs2); };
+    float2 g[KEEP ? VPT : 1][4], xh[KEEP ? VPT : 1][4];
+    float2 d1 = make_float2(0.f, 0.f), d2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) {
+      const int c = (threadIdx.x + v * nt) * 8;
+      float2 a[4], b[4];
+      load2(sdy, c, a); load2(sdy + H, c, b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 xv = xhat(b[i]), gv = fmul2(a[i], w2(v, i));
+        if (LN) d1 = fadd2(d1, gv);
+        d2 = ffma2(gv, xv, d2);
+        dwacc[v][i] = ffma2(a[i], LN ? xv : unpack_bf16(pack_bf16(xv.x, xv.y)), dwacc[v][i]);
+        if (LN) dbacc[v][i] = fadd2(dbacc[v][i], a[i]);
+        if (KEEP) { g[v][i] = gv; xh[v][i] = xv; }
+      }
+    }
+    float2 (&rd)[16] = red[it & 1];
+    const float s1 = LN ? warp_sum(d1.x + d1.y) : 0.f, s2 = warp_sum(d2.x + d2.y);
+    if ((threadIdx.x & 31) == 0) rd[wid] = make_float2(s1, s2);
     __syncthreads();
-    ss = 0.f;
-    for (int k = 0; k < wpr; ++k) ss += red[sub * wpr + k];
+    // all threads are past the previous row's last reads: its stage may be refilled
+    if (threadIdx.x == 0 && it > 0) request(row + static_cast<long long>(stages - 1) * gridDim.x, s == 0 ? stages - 1 : s - 1);
+    d1 = d2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 16; k += 2) {
+      const float2 t = rd[k], u = rd[k + 1];
+      if (LN) d1 = fadd2(d1, make_float2(t.x, u.x));
+      d2 = fadd2(d2, make_float2(t.y, u.y));
+    }
+    const float m1 = LN ? (d1.x + d1.y) / H : 0.f, m2 = (d2.x + d2.y) / H;
+    const float2 nm1 = make_float2(-m1, -m1), nm2 = make_float2(-m2, -m2);
+#pragma unroll
+    for (int v = 0; v < VPT; ++v) {
+      const int c = (threadIdx.x + v * nt) * 8;
+      if (c < H) {
+        float2 a[4], b[4], r[4], o[4];
+        if (!KEEP) { load2(sdy, c, a); load2(sdy + H, c, b); }
+        if (add_to != nullptr) load2(sdy + 2 * H, c, r);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float2 gv, xv;
+          if constexpr (KEEP) { gv = g[v][i]; xv = xh[v][i]; } else { gv = fmul2(a[i], w2(v, i)); xv = xhat(b[i]); }
+          if (LN) gv = fadd2(gv, nm1);
+          o[i] = fmul2(ffma2(xv, nm2, gv), rs2);
+          if (add_to != nullptr) o[i] = fadd2(o[i], r[i]);
+        }
+        *reinterpret_cast<uint4*>(dx + row * H + c) = make_uint4(pack_bf16(o[0].x, o[0].y), pack_bf16(o[1].x, o[1].y),
+                                                                 pack_bf16(o[2].x, o[2].y), pack_bf16(o[3].x, o[3].y));
+      }
+    }
+    mean = nmean; rstd = nrstd;
+    if (++s == stages) { s = 0; ph ^= 1; }
   }
-  if (!row_ok) return;
-  const float rstd = rsqrtf(ss / H + eps);
-  if (l == 0) rstd_out[row] = rstd;
-  __nv_bfloat16* yr = y + row * H;
 #pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int c = (l + k * lanes) * 8;
+  for (int v = 0; v < VPT; ++v) {
+    const int c = (threadIdx.x + v * nt) * 8;
     if (c < H) {
-      bf16x8 wv; wv.load(w + c);
-      float f[8], g[8]; v[k].to_float(f); wv.to_float(g);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(__float2bfloat16(f[i] * rstd)) * g[i];
-      bf16x8 o; o.from_float(f); o.store(yr + c);
+      float* dst = dwp + static_cast<long long>(blockIdx.x) * (LN ? 2 : 1) * H + c;
+      *reinterpret_cast<float4*>(dst) = make_float4(dwacc[v][0].x, dwacc[v][0].y, dwacc[v][1].x, dwacc[v][1].y);
+      *reinterpret_cast<float4*>(dst + 4) = make_float4(dwacc[v][2].x, dwacc[v][2].y, dwacc[v][3].x, dwacc[v][3].y);
+      if (LN) {
+        *reinterpret_cast<float4*>(dst + H) = make_float4(dbacc[v][0].x, dbacc[v][0].y, dbacc[v][1].x, dbacc[v][1].y);
+        *reinterpret_cast<float4*>(dst + H + 4) = make_float4(dbacc[v][2].x, dbacc[v][2].y, dbacc[v][3].x, dbacc[v][3].y);
+      }
     }
   }
 }
 
-// ------------------------------------------------------------------------------ RMSNorm bwd
-// dx = rstd * (g - xhat * mean(g * xhat)) (+ add_to), g = dy * w, xhat = x * rstd
-// dw partial per block in fp32: dwp[block, H] += dy * bf16(xhat). Persistent blocks loop over rows.
-// Wide rows use 512 threads with one or two vectors each: half the registers per thread of the 256-thread
-// form, so twice the warps stay resident and more loads are in flight around the per-row reduction.
-template <int VPT, int THREADS>  // 8-wide vectors per thread; H <= VPT * 8 * THREADS
-__global__ void __launch_bounds__(THREADS) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                                const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ w,
-                                                                const __nv_bfloat16* __restrict__ add_to, __nv_bfloat16* __restrict__ dx,
-                                                                float* __restrict__ dwp, int T, int H) {
-  __shared__ float red[32];
-  float dwacc[VPT][8];
-  float wreg[VPT][8];
-#pragma unroll
-  for (int v = 0; v < VPT; ++v) {
-    const int c = (threadIdx.x + v * THREADS) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { dwacc[v][i] = 0.f; wreg[v][i] = 0.f; }
-    if (c < H) { bf16x8 wv; wv.load(w + c); wv.to_float(wreg[v]); }
-  }
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
-    const float rstd = rstd_in[row];
-    float g[VPT][8], xh[VPT][8];
-    float dot = 0.f;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int c = (threadIdx.x + v * THREADS) * 8;
-      if (c < H) {
-        bf16x8 a, b; a.load(dy + row * H + c); b.load(x + row * H + c);
-        float fa[8], fb[8]; a.to_float(fa); b.to_float(fb);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          xh[v][i] = fb[i] * rstd;
-          g[v][i] = fa[i] * wreg[v][i];
-          dot += g[v][i] * xh[v][i];
-          dwacc[v][i] += fa[i] * __bfloat162float(__float2bfloat16(xh[v][i]));
-        }
-      }
-    }
-    dot = block_sum(dot, red) / H;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int c = (threadIdx.x + v * THREADS) * 8;
-      if (c < H) {
-        float o[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = rstd * (g[v][i] - xh[v][i] * dot);
-        if (add_to != nullptr) {
-          bf16x8 r; r.load(add_to + row * H + c);
-          float fr[8]; r.to_float(fr);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] += fr[i];
-        }
-        bf16x8 ov; ov.from_float(o); ov.store(dx + row * H + c);
-      }
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < VPT; ++v) {
-    const int c = (threadIdx.x + v * THREADS) * 8;
-    if (c < H) {
-      float* dst = dwp + static_cast<long long>(blockIdx.x) * H + c;
-      *reinterpret_cast<float4*>(dst) = make_float4(dwacc[v][0], dwacc[v][1], dwacc[v][2], dwacc[v][3]);
-      *reinterpret_cast<float4*>(dst + 4) = make_float4(dwacc[v][4], dwacc[v][5], dwacc[v][6], dwacc[v][7]);
-    }
-  }
-}
-
-// out[c] = bf16(sum_r part[r, c]); one thread per column, coalesced across threads.
-__global__ void reduce_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int R, int C) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
+// Sums of R partial rows of C columns; columns [0, D) go to out_a, the rest to out_b (a row may hold the partials of two
+// vectors; D = C when it holds one). 32 columns per block, 16 warps share the rows: a chain of R / 16 loads instead of R
+// (296 rows of 4096: 15 -> 5 us).
+__global__ void __launch_bounds__(512) reduce_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
+                                                         int R, int C, int D) {
+  __shared__ float sm[16][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r = 0; r < R; ++r) s += part[static_cast<long long>(r) * C + c];
-  out[c] = __float2bfloat16(s);
-}
-
-// Same for rows that hold two vectors of D columns each, delivered to two outputs.
-__global__ void reduce_rows_pair_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
-                                        int R, int D) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= 2 * D) return;
-  float s = 0.f;
-  for (int r = 0; r < R; ++r) s += part[static_cast<long long>(r) * 2 * D + c];
-  if (c < D) out_a[c] = __float2bfloat16(s); else out_b[c - D] = __float2bfloat16(s);
-}
-
-// ------------------------------------------------------------------------------ LayerNorm (Starcoder2)
-// y = ((x - mean) * rstd) * w + b, statistics in fp32 over the row held in registers (two-pass: the mean first, then
-// the centred sum of squares), mean and rstd saved. One 256-thread block per row, VPT 8-wide vectors per thread.
-template <int VPT>
-__global__ void __launch_bounds__(EW_THREADS) layernorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                                                                  const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
-                                                                  float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, int H) {
-  __shared__ float red[32];
-  const long long row = blockIdx.x;
-  const __nv_bfloat16* xr = x + row * H;
-  float f[VPT][8];
-  float s = 0.f;
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int c = (threadIdx.x + k * EW_THREADS) * 8;
-    if (c < H) {
-      bf16x8 v; v.load(xr + c); v.to_float(f[k]);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s += f[k][i];
-    }
+  if (c < C) {
+#pragma unroll 8
+    for (int r = wid; r < R; r += 16) s += part[static_cast<long long>(r) * C + c];
   }
-  const float mean = block_sum(s, red) / H;
-  float ss = 0.f;
+  sm[wid][lane] = s;
+  __syncthreads();
+  if (wid == 0 && c < C) {
 #pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int c = (threadIdx.x + k * EW_THREADS) * 8;
-    if (c < H) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { f[k][i] -= mean; ss += f[k][i] * f[k][i]; }
-    }
-  }
-  const float rstd = rsqrtf(block_sum(ss, red) / H + eps);
-  if (threadIdx.x == 0) { mean_out[row] = mean; rstd_out[row] = rstd; }
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int c = (threadIdx.x + k * EW_THREADS) * 8;
-    if (c < H) {
-      bf16x8 wv, bv; wv.load(w + c); bv.load(b + c);
-      float fw[8], fb[8], o[8]; wv.to_float(fw); bv.to_float(fb);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = f[k][i] * rstd * fw[i] + fb[i];
-      bf16x8 ov; ov.from_float(o); ov.store(y + row * H + c);
-    }
-  }
-}
-
-// dx = rstd * (g - mean(g) - xhat * mean(g * xhat)) (+ add_to), g = dy * w, xhat = (x - mean) * rstd.
-// Partials per block in fp32: dwp[block, 0, :] += dy * xhat, dwp[block, 1, :] += dy (the bias gradient); summed over
-// blocks by reduce_rows_pair_kernel. Persistent blocks loop over rows.
-template <int VPT>
-__global__ void __launch_bounds__(EW_THREADS) layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                                  const float* __restrict__ mean_in, const float* __restrict__ rstd_in,
-                                                                  const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ add_to,
-                                                                  __nv_bfloat16* __restrict__ dx, float* __restrict__ dwp, int T, int H) {
-  __shared__ float red[32];
-  float dwacc[VPT][8], dbacc[VPT][8], wreg[VPT][8];
-#pragma unroll
-  for (int v = 0; v < VPT; ++v) {
-    const int c = (threadIdx.x + v * EW_THREADS) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { dwacc[v][i] = 0.f; dbacc[v][i] = 0.f; wreg[v][i] = 0.f; }
-    if (c < H) { bf16x8 wv; wv.load(w + c); wv.to_float(wreg[v]); }
-  }
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
-    const float mean = mean_in[row], rstd = rstd_in[row];
-    float g[VPT][8], xh[VPT][8];
-    float d1 = 0.f, d2 = 0.f;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int c = (threadIdx.x + v * EW_THREADS) * 8;
-      if (c < H) {
-        bf16x8 a, b; a.load(dy + row * H + c); b.load(x + row * H + c);
-        float fa[8], fb[8]; a.to_float(fa); b.to_float(fb);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          xh[v][i] = (fb[i] - mean) * rstd;
-          g[v][i] = fa[i] * wreg[v][i];
-          d1 += g[v][i];
-          d2 += g[v][i] * xh[v][i];
-          dwacc[v][i] += fa[i] * xh[v][i];
-          dbacc[v][i] += fa[i];
-        }
-      }
-    }
-    d1 = block_sum(d1, red) / H;
-    d2 = block_sum(d2, red) / H;
-#pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int c = (threadIdx.x + v * EW_THREADS) * 8;
-      if (c < H) {
-        float o[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = rstd * (g[v][i] - d1 - xh[v][i] * d2);
-        if (add_to != nullptr) {
-          bf16x8 r; r.load(add_to + row * H + c);
-          float fr[8]; r.to_float(fr);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] += fr[i];
-        }
-        bf16x8 ov; ov.from_float(o); ov.store(dx + row * H + c);
-      }
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < VPT; ++v) {
-    const int c = (threadIdx.x + v * EW_THREADS) * 8;
-    if (c < H) {
-      float* dst = dwp + static_cast<long long>(blockIdx.x) * 2 * H + c;
-      *reinterpret_cast<float4*>(dst) = make_float4(dwacc[v][0], dwacc[v][1], dwacc[v][2], dwacc[v][3]);
-      *reinterpret_cast<float4*>(dst + 4) = make_float4(dwacc[v][4], dwacc[v][5], dwacc[v][6], dwacc[v][7]);
-      *reinterpret_cast<float4*>(dst + H) = make_float4(dbacc[v][0], dbacc[v][1], dbacc[v][2], dbacc[v][3]);
-      *reinterpret_cast<float4*>(dst + H + 4) = make_float4(dbacc[v][4], dbacc[v][5], dbacc[v][6], dbacc[v][7]);
-    }
+    for (int k = 1; k < 16; ++k) s += sm[k][lane];
+    if (c < D) out_a[c] = __float2bfloat16(s); else out_b[c - D] = __float2bfloat16(s);
   }
 }
 
@@ -469,13 +485,14 @@ __global__ void __launch_bounds__(EW_THREADS) head_rmsnorm_bwd_kernel(__nv_bfloa
 // ------------------------------------------------------------------------------ gated MLP activations
 // act(gate) * up over gu = [gate | up]. ACT 0: SiLU (SwiGLU: Llama, Qwen, Mistral, Granite, Mixtral, Phi-3);
 // ACT 1: tanh-approximated GELU (GeGLU: Gemma's gelu_pytorch_tanh).
+// gelu_gate is in ptx.cuh: 0.5 * (1 + tanh(u)) = sigmoid(2 u), which costs what SiLU costs (with tanhf the GELU kernels were bound
+// by instructions: 7001 x 12288 forward 92 -> 69 us).
 template <int ACT>
 __device__ __forceinline__ float glu_act(float g) {
   if constexpr (ACT == 0) {
     return __fdividef(g, 1.f + __expf(-g));
   } else {
-    const float th = tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g));
-    return 0.5f * g * (1.f + th);
+    return g * gelu_gate(g);
   }
 }
 // d act(g) / d g
@@ -485,8 +502,8 @@ __device__ __forceinline__ float glu_act_grad(float g) {
     const float sig = __fdividef(1.f, 1.f + __expf(-g));
     return sig * (1.f + g * (1.f - sig));
   } else {
-    const float th = tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g));
-    return 0.5f * (1.f + th) + 0.5f * g * (1.f - th * th) * 0.7978845608028654f * (1.f + 0.134145f * g * g);
+    const float s = gelu_gate(g);
+    return s + g * s * (1.f - s) * 1.5957691216057308f * (1.f + 0.134145f * g * g);
   }
 }
 
@@ -538,6 +555,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(__nv_bfloat16* d
 }
 
 // Plain (not gated) activation over n elements, forward and backward: Starcoder2's MLP is c_proj(gelu(c_fc(x))).
+// WITH_ACT: the forward output is also produced, written over dy, for a backward that did not keep it.
 template <int ACT>
 __global__ void __launch_bounds__(EW_THREADS) act_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
   const long long i0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
@@ -548,9 +566,8 @@ __global__ void __launch_bounds__(EW_THREADS) act_fwd_kernel(const __nv_bfloat16
   for (int i = 0; i < 8; ++i) f[i] = glu_act<ACT>(f[i]);
   v.from_float(f); v.store(y + i0);
 }
-template <int ACT>
-__global__ void __launch_bounds__(EW_THREADS) act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                                            __nv_bfloat16* __restrict__ dx, long long n) {
+template <bool WITH_ACT, int ACT>
+__global__ void __launch_bounds__(EW_THREADS) act_bwd_kernel(__nv_bfloat16* dy, const __nv_bfloat16* __restrict__ x, __nv_bfloat16* dx, long long n) {
   const long long i0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i0 >= n) return;
   bf16x8 v, d; v.load(x + i0); d.load(dy + i0);
@@ -558,6 +575,11 @@ __global__ void __launch_bounds__(EW_THREADS) act_bwd_kernel(const __nv_bfloat16
 #pragma unroll
   for (int i = 0; i < 8; ++i) g[i] *= glu_act_grad<ACT>(f[i]);
   d.from_float(g); d.store(dx + i0);
+  if (WITH_ACT) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = glu_act<ACT>(f[i]);   // same expression as the forward kernel
+    v.from_float(f); v.store(dy + i0);
+  }
 }
 
 // ------------------------------------------------------------------------------ embedding
@@ -611,10 +633,12 @@ __global__ void __launch_bounds__(128) embedding_bwd_kernel(__nv_bfloat16* __res
 
 // ------------------------------------------------------------------------------ cross-entropy
 // One block per row of a logits chunk ([R, V] fp32 or bf16, leading dimension ld). Pass 1: online
-// max / sum-exp. Pass 2: dlogits = (softmax - onehot) * scale in bf16. Rows whose target is
+// max / sum-exp; or, when the GEMM that made the logits left the statistics of every 256 columns (`stats`,
+// [R, ceil(V / 256)]), only their combination. Pass 2: dlogits = (softmax - onehot) * scale in bf16. Rows whose target is
 // ignore_index get zero loss and zero gradient. With bf16 logits the gradient may be written over
 // the logits (dlogits == logits): a thread reads a vector of the row before it overwrites the same
-// vector, and pass 2 starts after the block-wide reductions that end pass 1.
+// vector, and pass 2 starts after the block-wide reductions that end pass 1. Bound by the row's traffic: a row of a large
+// vocabulary (300 KB) does not stay on the SM between the passes, so pass 1 costs a third read (3720 x 151936: 578 -> 375 us with statistics).
 template <typename LogitT>
 __device__ __forceinline__ void load8(const LogitT* p, float (&f)[8]) {
   if constexpr (sizeof(LogitT) == 2) { bf16x8 v; v.load(reinterpret_cast<const __nv_bfloat16*>(p)); v.to_float(f); }
@@ -624,10 +648,11 @@ __device__ __forceinline__ void load8(const LogitT* p, float (&f)[8]) {
   }
 }
 
-template <typename LogitT>
-__global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, long long ld, const long long* __restrict__ targets,
-                                                         float* __restrict__ loss, __nv_bfloat16* dlogits, long long ldd,
-                                                         int V, float grad_scale, long long ignore_index) {
+template <typename LogitT, bool STATS>
+__global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, long long ld, const float2* __restrict__ stats,
+                                                         const long long* __restrict__ targets, float* __restrict__ loss,
+                                                         __nv_bfloat16* dlogits, long long ldd, int V, float grad_scale,
+                                                         long long ignore_index) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const LogitT* lr = logits + row * ld;
@@ -639,7 +664,15 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
     return;
   }
   float m = -INFINITY, s = 0.f;
-  for (int c = threadIdx.x * 8; c < V; c += blockDim.x * 8) {
+  if constexpr (STATS) {
+    const int tiles = (V + 255) / 256;
+    for (int c = threadIdx.x; c < tiles; c += blockDim.x) {
+      const float2 t = stats[row * tiles + c];
+      if (t.x > m) { s *= __expf(m - t.x); m = t.x; }
+      s += t.y * __expf(t.x - m);
+    }
+  }
+  else for (int c = threadIdx.x * 8; c < V; c += blockDim.x * 8) {
     float v[8];
     load8(lr + c, v);
     float mx = v[0];
@@ -660,39 +693,66 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
   }
   __syncthreads();   // the target logit has been read before any thread overwrites the row
   const float inv = grad_scale / gs;
-  for (int c = threadIdx.x * 8; c < V; c += blockDim.x * 8) {
-    float o[8];
-    load8(lr + c, o);
+  // two vectors per thread are loaded before the first is overwritten (the buffers may be the same, so the compiler cannot)
+  const int step = blockDim.x * 8;
+  for (int c0 = threadIdx.x * 8; c0 < V; c0 += 2 * step) {
+    float o[2][8];
+    load8(lr + c0, o[0]);
+    const bool two = c0 + step < V;
+    if (two) load8(lr + c0 + step, o[1]);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = __expf(o[i] - gm) * inv;
-    if (tgt >= c && tgt < c + 8) o[tgt - c] -= grad_scale;
-    bf16x8 ov; ov.from_float(o); ov.store(dr + c);
+    for (int k = 0; k < 2; ++k) {
+      if (k == 1 && !two) break;
+      const int c = c0 + k * step;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[k][i] = __expf(o[k][i] - gm) * inv;
+      if (tgt >= c && tgt < c + 8) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) if (tgt - c == i) o[k][i] -= grad_scale;   // no dynamic index: the array stays in registers
+      }
+      bf16x8 ov; ov.from_float(o[k]); ov.store(dr + c);
+    }
   }
 }
 
 // ------------------------------------------------------------------------------ column sums (bias grad)
-// part[split, c] = sum over this split's rows of x[r, c]; then reduce_rows_kernel.
+// part[split, c] = sum over this split's rows of x[r, c]; then reduce_rows_kernel. A lane adds V neighbouring columns of every
+// eighth row: V = 8 (16-byte loads) where rows are 16-byte aligned, V = 2 for any even width. Bound by reading x
+// (7001 rows of 3072 to 12288 columns, four calls: 96 -> 73 us).
+template <int V>
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restrict__ part,
                                                             int T, int N) {
-  __shared__ float sm[8][64];
+  __shared__ float sm[8][32 * V];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-  const int c = blockIdx.x * 64 + lane * 2;
+  const int c = (blockIdx.x * 32 + lane) * V;
   const int rows_per = (T + gridDim.y - 1) / gridDim.y;
   const int r0 = blockIdx.y * rows_per, r1 = min(T, r0 + rows_per);
-  float a = 0.f, b = 0.f;
+  float a[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) a[i] = 0.f;
   if (c < N) {
+#pragma unroll 4
     for (int r = r0 + wy; r < r1; r += 8) {
-      const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(x + static_cast<long long>(r) * ld + c));
-      a += v.x; b += v.y;
+      const __nv_bfloat16* p = x + static_cast<long long>(r) * ld + c;
+      if constexpr (V == 8) {
+        bf16x8 v; v.load(p);
+        float f[8]; v.to_float(f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] += f[i];
+      } else {
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+        a[0] += v.x; a[1] += v.y;
+      }
     }
   }
-  sm[wy][lane * 2] = a; sm[wy][lane * 2 + 1] = b;
+#pragma unroll
+  for (int i = 0; i < V; ++i) sm[wy][lane * V + i] = a[i];
   __syncthreads();
-  if (threadIdx.x < 64) {
+  if (threadIdx.x < 32 * V) {
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) s += sm[i][threadIdx.x];
-    const int cc = blockIdx.x * 64 + threadIdx.x;
+    const int cc = blockIdx.x * 32 * V + threadIdx.x;
     if (cc < N) part[static_cast<long long>(blockIdx.y) * N + cc] = s;
   }
 }
@@ -800,65 +860,122 @@ static int num_sms() {
 using namespace mtb;
 typedef __nv_bfloat16 bf16;
 
-extern "C" {
+template <bool LN, int VPT>
+static int launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float eps, int T, int H, int lanes,
+                           int* status, cudaStream_t st) {
+  auto kern = norm_fwd_kernel<LN, VPT>;
+  const int rows = EW_THREADS / lanes;
+  const int smem = NORM_STAGES * rows * H * 2;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM_STAGES * 8 * 8 * EW_THREADS * 2) != cudaSuccess) return -4;
+    configured = true;
+  }
+  static thread_local int for_smem = -1, resident = 0;   // the occupancy of the last shape this thread launched
+  if (for_smem != smem) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, EW_THREADS, smem) != cudaSuccess || resident < 1) return -4;
+    for_smem = smem;
+  }
+  const int want = cdiv(T, rows), most = num_sms() * resident;
+  kern<<<want < most ? want : most, EW_THREADS, smem, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, T, H, lanes, status);
+  return launch_ok();
+}
 
-int mtb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, float eps, int T, int H, cudaStream_t st) {
+template <bool LN>
+static int norm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float eps, int T, int H, int* status, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (H % 8 || H > 8 * 8 * EW_THREADS) return -10;
+  if (H <= 0 || H % 8 || H > (LN ? 4 : 8) * 8 * EW_THREADS) return -10;
+  if ((reinterpret_cast<uintptr_t>(x) & 15)) return -11;
   // about four vectors per thread; a row is held by 32 .. 256 threads (a power of two)
   const int vecs = H / 8;
   int lanes = 32;
   while (lanes < EW_THREADS && lanes * 4 < vecs) lanes *= 2;
   const int vpt = cdiv(vecs, lanes);
-  const int blocks = cdiv(T, EW_THREADS / lanes);
-#define RF(V) rmsnorm_fwd_kernel<V><<<blocks, EW_THREADS, 0, st>>>((const bf16*)x, (const bf16*)w, (bf16*)y, rstd, eps, T, H, lanes)
-  if (vpt <= 1) RF(1); else if (vpt <= 2) RF(2); else if (vpt <= 4) RF(4); else RF(8);
-#undef RF
+#define NF(V) return launch_norm_fwd<LN, V>(x, w, b, y, mean, rstd, eps, T, H, lanes, status, st)
+  if (vpt <= 1) NF(1);
+  if (vpt <= 2) NF(2);
+  if (vpt <= 3) NF(3);
+  if (vpt <= 4) NF(4);
+  if constexpr (!LN) NF(8);
+#undef NF
+  return -10;
+}
+
+// Threads of a norm backward block: the row's vectors over as few vectors per thread as 512 threads allow.
+static int norm_bwd_vpt(int H) { return cdiv(H, 8 * 512); }
+static int norm_bwd_threads(int H) { return cdiv(cdiv(H / 8, norm_bwd_vpt(H)), 32) * 32; }
+
+// Number of row-partials the backward of either norm writes (rows of the dw_partial scratch, fp32: [blocks, H], LayerNorm [blocks, 2, H]).
+// Two blocks per SM at 512 threads, more of the smaller ones: every row in flight hides another's reduction.
+extern "C" int mtb200_norm_bwd_blocks(int T, int H) {
+  const int per_sm = 1024 / norm_bwd_threads(H);
+  const int b = num_sms() * (per_sm < 2 ? 2 : (per_sm > 6 ? 6 : per_sm));
+  return T < b ? (T > 0 ? T : 1) : b;
+}
+
+template <bool LN, int VPT>
+static int launch_norm_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const void* w, const void* add_to, void* dx,
+                           float* dwp, int T, int H, int blocks, int threads, int* status, cudaStream_t st) {
+  auto kern = norm_bwd_kernel<LN, VPT>;
+  constexpr int most = 200 * 1024;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return -4;
+    configured = true;
+  }
+  // up to four rows ahead in the block's share of the SM (blocks / SMs of them are resident), two at least
+  const int stage = H * 2 * (add_to != nullptr ? 3 : 2), per_sm = cdiv(blocks, num_sms());
+  int stages = most / (per_sm * stage);
+  stages = stages > 4 ? 4 : (stages < 2 ? 2 : stages);
+  kern<<<blocks, threads, stages * stage, st>>>((const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)w, (const bf16*)add_to, (bf16*)dx, dwp, T, H,
+                                                stages, status);
   return launch_ok();
 }
 
-// Number of row-partials the backward writes (rows of the dw_partial scratch, [blocks, H] fp32).
-int mtb200_rmsnorm_bwd_blocks(int T) { const int b = num_sms() * 2; return T < b ? (T > 0 ? T : 1) : b; }
+static bool aligned16(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
 
-int mtb200_rmsnorm_bwd(const void* dy, const void* x, const float* rstd, const void* w, const void* add_to, void* dx,
-                       float* dw_partial, void* dw_out, int T, int H, cudaStream_t st) {
-  if (T <= 0) return 0;
-  if (H % 8 || H > 4 * 8 * 512) return -10;
-  const int blocks = mtb200_rmsnorm_bwd_blocks(T);
-#define RB(V, TH) rmsnorm_bwd_kernel<V, TH><<<blocks, TH, 0, st>>>((const bf16*)dy, (const bf16*)x, rstd, (const bf16*)w, (const bf16*)add_to, (bf16*)dx, dw_partial, T, H)
-  if (H <= 8 * EW_THREADS) RB(1, EW_THREADS);
-  else {
-    const int vpt = cdiv(H, 8 * 512);
-    if (vpt <= 1) RB(1, 512); else if (vpt == 2) RB(2, 512); else if (vpt == 3) RB(3, 512); else RB(4, 512);
-  }
-#undef RB
-  reduce_rows_kernel<<<cdiv(H, 256), 256, 0, st>>>(dw_partial, (bf16*)dw_out, blocks, H);
-  return launch_ok();
+extern "C" {
+
+int mtb200_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, float eps, int T, int H, int* status, cudaStream_t st) {
+  return norm_fwd<false>(x, w, nullptr, y, nullptr, rstd, eps, T, H, status, st);
 }
 
 // LayerNorm with bias over rows of H <= 8192 elements; mean / rstd: [T] fp32 each.
-int mtb200_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float eps, int T, int H,
+int mtb200_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float eps, int T, int H, int* status,
                          cudaStream_t st) {
+  return norm_fwd<true>(x, w, b, y, mean, rstd, eps, T, H, status, st);
+}
+
+int mtb200_rmsnorm_bwd(const void* dy, const void* x, const float* rstd, const void* w, const void* add_to, void* dx,
+                       float* dw_partial, void* dw_out, int T, int H, int* status, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (H % 8 || H > 4 * 8 * EW_THREADS) return -10;
-  const int vpt = cdiv(H, 8 * EW_THREADS);
-#define LF(V) layernorm_fwd_kernel<V><<<T, EW_THREADS, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, H)
-  if (vpt <= 1) LF(1); else if (vpt == 2) LF(2); else if (vpt == 3) LF(3); else LF(4);
-#undef LF
+  if (H <= 0 || H % 8 || H > 4 * 8 * 512) return -10;
+  if (!aligned16(dy, x, add_to)) return -11;
+  const int blocks = mtb200_norm_bwd_blocks(T, H), vpt = norm_bwd_vpt(H), threads = norm_bwd_threads(H);
+  int rc;
+#define RB(V) launch_norm_bwd<false, V>(dy, x, nullptr, rstd, w, add_to, dx, dw_partial, T, H, blocks, threads, status, st)
+  if (vpt <= 1) rc = RB(1); else if (vpt == 2) rc = RB(2); else if (vpt == 3) rc = RB(3); else rc = RB(4);
+#undef RB
+  if (rc) return rc;
+  reduce_rows_kernel<<<cdiv(H, 32), 512, 0, st>>>(dw_partial, (bf16*)dw_out, nullptr, blocks, H, H);
   return launch_ok();
 }
 
-// dw_partial: [mtb200_rmsnorm_bwd_blocks(T), 2, H] fp32 scratch; dw_out / db_out: [H] bf16 each.
+// dw_partial: [mtb200_norm_bwd_blocks(T, H), 2, H] fp32 scratch; dw_out / db_out: [H] bf16 each.
 int mtb200_layernorm_bwd(const void* dy, const void* x, const float* mean, const float* rstd, const void* w, const void* add_to, void* dx,
-                         float* dw_partial, void* dw_out, void* db_out, int T, int H, cudaStream_t st) {
+                         float* dw_partial, void* dw_out, void* db_out, int T, int H, int* status, cudaStream_t st) {
   if (T <= 0) return 0;
-  if (H % 8 || H > 4 * 8 * EW_THREADS) return -10;
-  const int blocks = mtb200_rmsnorm_bwd_blocks(T);
-  const int vpt = cdiv(H, 8 * EW_THREADS);
-#define LB(V) layernorm_bwd_kernel<V><<<blocks, EW_THREADS, 0, st>>>((const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)w, (const bf16*)add_to, (bf16*)dx, dw_partial, T, H)
-  if (vpt <= 1) LB(1); else if (vpt == 2) LB(2); else if (vpt == 3) LB(3); else LB(4);
+  if (H <= 0 || H % 8 || H > 4 * 8 * EW_THREADS) return -10;
+  if (!aligned16(dy, x, add_to)) return -11;
+  const int blocks = mtb200_norm_bwd_blocks(T, H), threads = norm_bwd_threads(H);
+  int rc;
+#define LB(V) launch_norm_bwd<true, V>(dy, x, mean, rstd, w, add_to, dx, dw_partial, T, H, blocks, threads, status, st)
+  if (norm_bwd_vpt(H) <= 1) rc = LB(1); else rc = LB(2);
 #undef LB
-  reduce_rows_pair_kernel<<<cdiv(2 * H, 256), 256, 0, st>>>(dw_partial, (bf16*)dw_out, (bf16*)db_out, blocks, H);
+  if (rc) return rc;
+  reduce_rows_kernel<<<cdiv(2 * H, 32), 512, 0, st>>>(dw_partial, (bf16*)dw_out, (bf16*)db_out, blocks, 2 * H, H);
   return launch_ok();
 }
 
@@ -904,7 +1021,7 @@ int mtb200_head_rmsnorm_bwd(void* dqkv, const void* pre, const float* rstd, cons
   if (D == 64) HB(2); else if (D == 128) HB(4); else HB(8);
 #undef HB
   // partial rows are [2, D]: columns 0..D-1 belong to the q weight, D..2D-1 to the k weight
-  reduce_rows_pair_kernel<<<cdiv(2 * D, 256), 256, 0, st>>>(dw_partial, (bf16*)dwq_out, (bf16*)dwk_out, blocks, D);
+  reduce_rows_kernel<<<cdiv(2 * D, 32), 512, 0, st>>>(dw_partial, (bf16*)dwq_out, (bf16*)dwk_out, blocks, 2 * D, D);
   return launch_ok();
 }
 
@@ -960,7 +1077,14 @@ int mtb200_gelu_fwd(const void* x, void* y, long long n, cudaStream_t st) {
 int mtb200_gelu_bwd(const void* dy, const void* x, void* dx, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -10;
-  act_bwd_kernel<1><<<static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st>>>((const bf16*)dy, (const bf16*)x, (bf16*)dx, n);
+  act_bwd_kernel<false, 1><<<static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)const_cast<void*>(dy), (const bf16*)x, (bf16*)dx, n);
+  return launch_ok();
+}
+// Same, and dy_inout is overwritten with gelu_tanh(x); dx is another buffer.
+int mtb200_gelu_bwd_act(void* dy_inout, const void* x, void* dx, long long n, cudaStream_t st) {
+  if (n <= 0) return 0;
+  if (n % 8 || dx == dy_inout) return -10;
+  act_bwd_kernel<true, 1><<<static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)dy_inout, (const bf16*)x, (bf16*)dx, n);
   return launch_ok();
 }
 
@@ -979,23 +1103,30 @@ int mtb200_embedding_bwd(void* dw, const long long* sorted_ids, const long long*
   return launch_ok();
 }
 
-// logits: [R, V] fp32, or bf16 when logits_bf16 (dlogits may then be the same buffer).
-int mtb200_ce_fwd_bwd(const void* logits, long long ld, int logits_bf16, const long long* targets, float* loss, void* dlogits,
-                      long long ldd, int R, int V, float grad_scale, long long ignore_index, cudaStream_t st) {
+// logits: [R, V] fp32, or bf16 when logits_bf16 (dlogits may then be the same buffer). stats: optional, bf16 logits only.
+int mtb200_ce_fwd_bwd(const void* logits, long long ld, int logits_bf16, const float2* stats, const long long* targets, float* loss,
+                      void* dlogits, long long ldd, int R, int V, float grad_scale, long long ignore_index, cudaStream_t st) {
   if (R <= 0) return 0;
-  if (V % 8 || ld % 8 || ldd % 8) return -10;
-  if (logits_bf16) ce_fwd_bwd_kernel<bf16><<<R, 1024, 0, st>>>((const bf16*)logits, ld, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index);
-  else ce_fwd_bwd_kernel<float><<<R, 1024, 0, st>>>((const float*)logits, ld, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index);
+  if (V % 8 || ld % 8 || ldd % 8 || (stats && !logits_bf16)) return -10;
+#define CE(T, S) ce_fwd_bwd_kernel<T, S><<<R, 1024, 0, st>>>((const T*)logits, ld, stats, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index)
+  if (stats) CE(bf16, true); else if (logits_bf16) CE(bf16, false); else CE(float, false);
+#undef CE
   return launch_ok();
+}
+
+static void launch_colsum(const void* x, long long ld, void* out, float* scratch, int T, int N, cudaStream_t st) {
+  const int splits = T < 32 ? 1 : 32;
+  const bool wide = N % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  if (wide) colsum_partial_kernel<8><<<dim3(cdiv(N, 256), splits), 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
+  else colsum_partial_kernel<2><<<dim3(cdiv(N, 64), splits), 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
+  reduce_rows_kernel<<<cdiv(N, 32), 512, 0, st>>>(scratch, (bf16*)out, nullptr, splits, N, N);
 }
 
 // out[N] (bf16) = column sums of x[T, N]. scratch: fp32 [32, N].
 int mtb200_colsum(const void* x, long long ld, void* out, float* scratch, int T, int N, cudaStream_t st) {
   if (T <= 0 || N <= 0) return 0;
   if (N % 2) return -10;
-  const int splits = T < 32 ? 1 : 32;
-  colsum_partial_kernel<<<dim3(cdiv(N, 64), splits), 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
-  reduce_rows_kernel<<<cdiv(N, 256), 256, 0, st>>>(scratch, (bf16*)out, splits, N);
+  launch_colsum(x, ld, out, scratch, T, N, st);
   return launch_ok();
 }
 
@@ -1075,9 +1206,7 @@ extern "C" int mtb200_colsum_noalloc(const void* x, long long ld, void* out, int
   if (ws == nullptr) return -12;
   // Every element of ws[0 : splits * N] that the second kernel reads is written by the first one,
   // so nothing left over from an earlier call can reach the result and no clearing pass is needed.
-  const int splits = T < 32 ? 1 : 32;
-  colsum_partial_kernel<<<dim3(cdiv(N, 64), splits), 256, 0, st>>>((const bf16*)x, ld, ws, T, N);
-  reduce_rows_kernel<<<cdiv(N, 256), 256, 0, st>>>(ws, (bf16*)out, splits, N);
+  launch_colsum(x, ld, out, ws, T, N, st);
   return launch_ok();
 }
 

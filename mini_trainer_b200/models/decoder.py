@@ -206,7 +206,7 @@ def block_backward(ops, cfg: ModelConfig, p: dict, g: dict, acts: BlockActs, dou
         ops.linear_wgrad(dout, a.act, g["wd"], g.get("bd"), alpha=rm)
         dgu = ops.swiglu_bwd(dact, a.gu, cfg.mlp_act) if cfg.mlp_gated else ops.gelu_bwd(dact, a.gu)
     elif not cfg.mlp_gated:
-        act, dgu = ops.gelu(a.gu), ops.gelu_bwd(dact, a.gu)
+        dgu, act = ops.gelu_bwd_act(dact, a.gu)
         ops.linear_wgrad(dout, act, g["wd"], g.get("bd"), alpha=rm)
         del act
     else:   # one pass over gate/up gives its gradient and the SwiGLU output (written over dact)

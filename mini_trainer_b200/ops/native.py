@@ -46,11 +46,11 @@ P, I, L, F = c_void_p, c_int, c_longlong, c_float
 class _Sig:
     mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
     mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
-    mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P]
-    mtb200_rmsnorm_bwd_blocks = [I]
-    mtb200_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, I, P]
-    mtb200_layernorm_fwd = [P, P, P, P, P, P, F, I, I, P]
-    mtb200_layernorm_bwd = [P, P, P, P, P, P, P, P, P, P, I, I, P]
+    mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
+    mtb200_norm_bwd_blocks = [I, I]
+    mtb200_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, I, P, P]
+    mtb200_layernorm_fwd = [P, P, P, P, P, P, F, I, I, P, P]
+    mtb200_layernorm_bwd = [P, P, P, P, P, P, P, P, P, P, I, I, P, P]
     mtb200_rope = [P, P, P, I, L, I, I, I, P]
     mtb200_head_rmsnorm_fwd = [P, P, P, P, F, I, L, I, I, I, P]
     mtb200_head_rmsnorm_bwd_blocks = [I, I]
@@ -63,9 +63,10 @@ class _Sig:
     mtb200_geglu_bwd_act = [P, P, P, L, I, P]
     mtb200_gelu_fwd = [P, P, L, P]
     mtb200_gelu_bwd = [P, P, P, L, P]
+    mtb200_gelu_bwd_act = [P, P, P, L, P]
     mtb200_embedding_fwd = [P, P, P, I, I, I, P, P]
     mtb200_embedding_bwd = [P, P, P, P, I, I, I, P, P]
-    mtb200_ce_fwd_bwd = [P, L, I, P, P, P, L, I, I, F, L, P]
+    mtb200_ce_fwd_bwd = [P, L, I, P, P, P, P, L, I, I, F, L, P]
     mtb200_colsum = [P, L, P, P, I, I, P]
     mtb200_accumulate = [P, P, L, I, I, P]
     mtb200_f32_to_bf16 = [P, P, L, I, P]
@@ -238,16 +239,17 @@ class NativeOps:
         T, H = x.shape
         y = torch.empty_like(x)
         rstd = torch.empty(T, dtype=torch.float32, device=self.device)
-        self._call("mtb200_rmsnorm_fwd", x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), eps, T, H, self._st())
+        self._call("mtb200_rmsnorm_fwd", x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr(), eps, T, H,
+                   self.status.data_ptr(), self._st())
         return y, rstd
 
     def rmsnorm_bwd(self, dy, x, rstd, w, dw_out, add_to=None):
         T, H = x.shape
         dx = torch.empty_like(x)
-        blocks = self.lib.mtb200_rmsnorm_bwd_blocks(T)
+        blocks = self.lib.mtb200_norm_bwd_blocks(T, H)
         part = self._buf("rms_part", blocks * H, torch.float32)
         self._call("mtb200_rmsnorm_bwd", dy.data_ptr(), x.data_ptr(), rstd.data_ptr(), w.data_ptr(), _ptr(add_to),
-                   dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(), T, H, self._st(), n=2)
+                   dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(), T, H, self.status.data_ptr(), self._st(), n=2)
         return dx
 
     # -- layernorm (Starcoder2) -----------------------------------------------------------
@@ -258,16 +260,17 @@ class NativeOps:
         mean = torch.empty(T, dtype=torch.float32, device=self.device)
         rstd = torch.empty(T, dtype=torch.float32, device=self.device)
         self._call("mtb200_layernorm_fwd", x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean.data_ptr(),
-                   rstd.data_ptr(), eps, T, H, self._st())
+                   rstd.data_ptr(), eps, T, H, self.status.data_ptr(), self._st())
         return y, (mean, rstd)
 
     def layernorm_bwd(self, dy, x, stats, w, dw_out, db_out, add_to=None):
         T, H = x.shape
         dx = torch.empty_like(x)
-        blocks = self.lib.mtb200_rmsnorm_bwd_blocks(T)
+        blocks = self.lib.mtb200_norm_bwd_blocks(T, H)
         part = self._buf("layernorm_dw", blocks * 2 * H, torch.float32)
         self._call("mtb200_layernorm_bwd", dy.data_ptr(), x.data_ptr(), stats[0].data_ptr(), stats[1].data_ptr(), w.data_ptr(),
-                   _ptr(add_to), dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(), db_out.data_ptr(), T, H, self._st(), n=2)
+                   _ptr(add_to), dx.data_ptr(), part.data_ptr(), dw_out.data_ptr(), db_out.data_ptr(), T, H, self.status.data_ptr(),
+                   self._st(), n=2)
         return dx
 
     # -- linear -----------------------------------------------------------------------
@@ -537,6 +540,12 @@ class NativeOps:
         self._call("mtb200_gelu_bwd", dy.data_ptr(), x.data_ptr(), dx.data_ptr(), x.numel(), self._st())
         return dx
 
+    def gelu_bwd_act(self, dy, x):
+        """Returns ``(dx, act)``; ``act`` (the forward output) is written over ``dy``."""
+        dx = torch.empty_like(x)
+        self._call("mtb200_gelu_bwd_act", dy.data_ptr(), x.data_ptr(), dx.data_ptr(), x.numel(), self._st())
+        return dx, dy
+
     # -- fused linear + cross-entropy ---------------------------------------------------
     def linear_ce(self, x, w, targets, grad_scale, dw_out, accumulate_dw=False, ignore_index=-100, logit_scale=1.0):
         """Per-token CE of ``logit_scale * x @ w.T``. Chunked over tokens (8192 rows): bf16 logits chunk
@@ -555,7 +564,7 @@ class NativeOps:
         for a in range(0, T, ck):
             n = min(ck, T - a)
             self.gemm(x[a:a + n], False, w, False, logits, n, V, H, alpha=logit_scale)
-            self._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, targets[a:a + n].data_ptr(), loss[a:a + n].data_ptr(),
+            self._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, None, targets[a:a + n].data_ptr(), loss[a:a + n].data_ptr(),
                        logits.data_ptr(), V, n, V, float(grad_scale), ignore_index, self._st())
             self.gemm(logits, False, w, True, dx[a:a + n], n, H, V, alpha=logit_scale)
             self.gemm(logits, True, x[a:a + n], True, dw32, V, H, n, residual=None if first else dw32, alpha=logit_scale)

@@ -234,6 +234,10 @@ class TorchOps:
     def gelu_bwd(self, dy, x):
         return (dy.float() * self._gelu_tanh_grad(x.float())).to(x.dtype)
 
+    def gelu_bwd_act(self, dy, x):
+        """``(dx, act)``: the gradient and the forward output a backward that did not keep it needs."""
+        return self.gelu_bwd(dy, x), self.gelu(x)
+
     # -- fused linear + cross-entropy ---------------------------------------------------
     def linear_ce(self, x, w, targets, grad_scale, dw_out, accumulate_dw=False, ignore_index=-100, logit_scale=1.0):
         """Per-token CE of ``logit_scale * x @ w.T`` against ``targets`` without materialising all logits.

@@ -622,3 +622,32 @@ def test_attention_work_distribution(ops, D, hq, hkv, lens):
     again = ops.attention_bwd(dout, qkv, out, lse, cu, cu_host, max(lens), hq, hkv, D)
     kv = hq * D
     assert torch.equal(again[:, kv:], dqkv[:, kv:])     # dK and dV: one order of summation (dQ is accumulated in any order)
+
+
+# more rows than resident blocks, row widths of one to eight vectors per thread
+@pytest.mark.parametrize("T,H", [(5000, 512), (3001, 2056), (700, 12296), (1300, 5000)])
+def test_norms_many_rows(ops, T, H):
+    torch.manual_seed(T)
+    x, w, b, dy, add = bf(T, H), bf(H), bf(H), bf(T, H), bf(T, H)
+    y, rstd = ops.rmsnorm(x, w, 1e-5)
+    ry, rr = REF.rmsnorm(x.float(), w.float(), 1e-5)
+    assert rel_err(y, ry) < 5e-3 and rel_err(rstd, rr.reshape(-1)) < 1e-5
+    dw, rdw = torch.empty_like(w), torch.empty(H, device="cuda")
+    dx = ops.rmsnorm_bwd(dy, x, rstd, w, dw, add_to=add)
+    assert rel_err(dx, REF.rmsnorm_bwd(dy.float(), x.float(), rr, w.float(), rdw, add_to=add.float())) < 5e-3 and rel_err(dw, rdw) < 5e-3
+    if H <= 8192:
+        y, st = ops.layernorm(x, w, b, 1e-5)
+        ry, rst = REF.layernorm(x.float(), w.float(), b.float(), 1e-5)
+        assert rel_err(y, ry) < 5e-3
+        db, rdb = torch.empty_like(b), torch.empty(H, device="cuda")
+        dx = ops.layernorm_bwd(dy, x, st, w, dw, db, add_to=None)
+        assert rel_err(dx, REF.layernorm_bwd(dy.float(), x.float(), rst, w.float(), rdw, rdb)) < 5e-3
+        assert rel_err(dw, rdw) < 5e-3 and rel_err(db, rdb) < 5e-3
+
+
+def test_gelu_backward_with_activation(ops):
+    x, dy = bf(333, 72, scale=3.0), bf(333, 72)
+    want_dx, want_act = ops.gelu_bwd(dy, x), ops.gelu(x)
+    d = dy.clone()
+    dx, act = ops.gelu_bwd_act(d, x)
+    assert act is d and torch.equal(dx, want_dx) and torch.equal(act, want_act)

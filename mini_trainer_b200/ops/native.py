@@ -559,17 +559,24 @@ class NativeOps:
         dx = torch.empty_like(x)
         ck = min(self.ce_chunk, T)
         logits = self._buf("ce_logits", ck * V, torch.bfloat16).view(ck, V)
-        dw32 = self._buf("ce_dw", V * H, torch.float32).view(V, H)
+        stats = self._buf("ce_stats", ck * -(-V // 256) * 2, torch.float32)
+        # one chunk: its weight gradient is the whole sum, rounded (or added to what is there) in the GEMM's epilogue
+        whole = T <= ck and dw_out.is_contiguous()
+        dw32 = None if whole else self._buf("ce_dw", V * H, torch.float32).view(V, H)
         first = True
         for a in range(0, T, ck):
             n = min(ck, T - a)
-            self.gemm(x[a:a + n], False, w, False, logits, n, V, H, alpha=logit_scale)
-            self._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, None, targets[a:a + n].data_ptr(), loss[a:a + n].data_ptr(),
-                       logits.data_ptr(), V, n, V, float(grad_scale), ignore_index, self._st())
+            self.gemm(x[a:a + n], False, w, False, logits, n, V, H, alpha=logit_scale, stats=stats)
+            self._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, stats.data_ptr(), targets[a:a + n].data_ptr(),
+                       loss[a:a + n].data_ptr(), logits.data_ptr(), V, n, V, float(grad_scale), ignore_index, self._st())
             self.gemm(logits, False, w, True, dx[a:a + n], n, H, V, alpha=logit_scale)
-            self.gemm(logits, True, x[a:a + n], True, dw32, V, H, n, residual=None if first else dw32, alpha=logit_scale)
+            if whole:
+                self.gemm(logits, True, x, True, dw_out, V, H, n, residual=dw_out if accumulate_dw else None, alpha=logit_scale)
+            else:
+                self.gemm(logits, True, x[a:a + n], True, dw32, V, H, n, residual=None if first else dw32, alpha=logit_scale)
             first = False
-        self._call("mtb200_f32_to_bf16", dw_out.data_ptr(), dw32.data_ptr(), V * H, int(accumulate_dw), self._st())
+        if not whole:
+            self._call("mtb200_f32_to_bf16", dw_out.data_ptr(), dw32.data_ptr(), V * H, int(accumulate_dw), self._st())
         return loss, dx
 
     # -- optimizer --------------------------------------------------------------------

@@ -651,3 +651,29 @@ def test_gelu_backward_with_activation(ops):
     d = dy.clone()
     dx, act = ops.gelu_bwd_act(d, x)
     assert act is d and torch.equal(dx, want_dx) and torch.equal(act, want_act)
+
+
+# one chunk (dW straight to bf16, with and without what is already there) against several (fp32 sums)
+@pytest.mark.parametrize("V", [4104, 520])
+def test_linear_ce_chunks(ops, V):
+    torch.manual_seed(V)
+    T, H = 300, 256
+    x, w = bf(T, H), bf(V, H, scale=0.05)
+    tg = torch.randint(0, V, (T,), device="cuda")
+    tg[::7] = -100
+    keep = ops.ce_chunk
+    res = []
+    try:
+        for chunk in (8192, 128):
+            ops.ce_chunk = chunk
+            dw = torch.full_like(w, 0.25)
+            loss, dx = ops.linear_ce(x, w, tg, 0.01, dw, accumulate_dw=True)
+            dw2 = torch.full_like(w, float("nan"))
+            ops.linear_ce(x, w, tg, 0.01, dw2)
+            res.append((loss, dx, dw, dw2))
+    finally:
+        ops.ce_chunk = keep
+    ref = torch.nn.functional.cross_entropy((x.float() @ w.float().t()).bfloat16().float(), tg, reduction="none", ignore_index=-100)
+    assert (res[0][0] - ref).abs().max() < 2e-3     # bf16 logits on both sides, fp32 sums of up to V exponentials
+    for a, b in zip(*res):
+        assert rel_err(a, b) < 4e-3

@@ -13,12 +13,15 @@ import os
 from dataclasses import dataclass
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
+import numpy as np
 import torch
 
 from .. import build as _build
 from ..utils import nvtx
 
 _LIB = None
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else \
+    (lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def load_library():
@@ -115,6 +118,8 @@ class NativeOps:
         if self.device.type != "cuda":
             raise RuntimeError("NativeOps needs a CUDA device")
         self.lib = load_library()
+        self._fn = {name: getattr(self.lib, name) for name in dir(_Sig) if name.startswith("mtb200_") and hasattr(self.lib, name)}
+        self._index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self.ce_chunk = ce_chunk
         self.attention_impl = attention or os.environ.get("MTB200_ATTENTION", "native")
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
@@ -133,15 +138,21 @@ class NativeOps:
 
     # -- plumbing ---------------------------------------------------------------------
     def _st(self):
-        return torch.cuda.current_stream(self.device).cuda_stream
+        return _raw_stream(self._index)   # handle of the device's current torch stream, without a Stream object around it
 
     def _call(self, name, *args, n=1, tag=None):
+        if self.profile is None and not nvtx.ENABLED:
+            rc = self._fn[name](*args)
+            if rc != 0:
+                raise RuntimeError(f"{name} failed with code {rc}")
+            self.launches += n
+            return
         if self.profile is not None:
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
         if nvtx.ENABLED:
             nvtx.push(tag or name)
-        rc = getattr(self.lib, name)(*args)
+        rc = self._fn[name](*args)
         if nvtx.ENABLED:
             nvtx.pop()
         if rc != 0:
@@ -349,14 +360,16 @@ class NativeOps:
         hit = self._attn_plan_cache.get(key)
         if hit is not None and hit[0] is cu_host:
             return hit[1]
-        items = []
-        for a, b in zip(cu_host[:-1], cu_host[1:]):
-            n = b - a
-            for s0 in range(0, n, block):
-                work = s0 if most_work_last_block else n - s0
-                items.append((work, a, n, s0))
-        items.sort(key=lambda it: -it[0])
-        table = torch.tensor([it[1:] for it in items], dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
+        cu = np.asarray(cu_host, dtype=np.int64)
+        lens = cu[1:] - cu[:-1]
+        per = -(-lens // block)                                    # blocks of every sequence
+        seq = np.repeat(np.arange(lens.shape[0]), per)
+        s0 = (np.arange(seq.shape[0]) - np.repeat(np.cumsum(per) - per, per)) * block
+        work = s0 if most_work_last_block else lens[seq] - s0
+        order = np.argsort(-work, kind="stable")
+        host = torch.empty(seq.shape[0], 3, dtype=torch.int32, pin_memory=True)
+        host.numpy()[:] = np.stack([cu[:-1][seq], lens[seq], s0], axis=1)[order]
+        table = host.to(self.device, non_blocking=True)
         if len(self._attn_plan_cache) > 8:
             self._attn_plan_cache.clear()
         self._attn_plan_cache[key] = (cu_host, table)
@@ -584,6 +597,10 @@ class NativeOps:
         out = torch.zeros(1, dtype=torch.float32, device=self.device)
         self._call("mtb200_sumsq", g.data_ptr(), g.numel(), out.data_ptr(), self._st())
         return out
+
+    def add_sumsq(self, g, out):
+        """``out += sum(g ** 2)`` (``out``: one fp32 element on the device)."""
+        self._call("mtb200_sumsq", g.data_ptr(), g.numel(), out.data_ptr(), self._st())
 
     def accumulate(self, acc, src, accumulate: bool):
         """acc(fp32) = (acc if accumulate else 0) + src (bf16 or fp32)."""

@@ -61,8 +61,15 @@ class ShardedGroup:
         self.m = torch.zeros(s, dtype=state_dtype, device=device)
         self.v = torch.zeros(s, dtype=state_dtype, device=device)
         self.gacc = torch.zeros(s, dtype=torch.float32, device=device)
+        self._views = None
         self.has_grad = False
         self.sq_done = False   # sum of squares of gacc already added to the engine's norm scalar
+
+    def shard_views(self) -> dict:
+        """Named tensors of a group that is not sharded (one rank): views of the working copy, made once."""
+        if self._views is None or self._views[0] is not self.shard:
+            self._views = (self.shard, self.layout.views(self.shard))
+        return self._views[1]
 
     def state_bytes(self) -> int:
         return sum(t.numel() * t.element_size() for t in (self.shard, self.master, self.m, self.v, self.gacc))
@@ -165,6 +172,8 @@ class ShardedEngine:
         self._gbufs = [salloc(blk) for _ in range(nbuf)]
         self._eg_full = salloc(self.embed.layout.padded_numel)   # embedding gradient (full, reduced once per microbatch)
         self._hg_full = salloc(self.head.layout.padded_numel)    # final norm / lm_head gradient
+        # named views of the gradient buffers, made once (every block has the same layout)
+        self._gviews = [layouts[1].views(b) for b in self._gbufs]
         self._root_free = {"embed": None, "head": None}
         self._sq = torch.zeros(1, dtype=torch.float32, device=self.device)
         self._pbuf_free = [None] * nbuf   # event after which the buffer may be overwritten
@@ -176,6 +185,7 @@ class ShardedEngine:
         # None = derive from free device memory; 0 = recompute every block like the reference
         self.activation_budget_bytes = activation_budget_bytes
         self._oom_retries = 0
+        self._state_bytes = None   # of the groups, which never change size
         # Reduce a block's gradients tensor region by tensor region while its backward still runs
         # (MTB200_REGION_OVERLAP=0: one reduction per block, after its backward).
         # A mixture-of-experts block is reduced once: its experts' gradients complete in no fixed layout order.
@@ -297,7 +307,7 @@ class ShardedEngine:
         the block's QKV and gate/up GEMMs pull the parameters from the peers while they run."""
         grp = self.blocks[i]
         if self.world == 1:
-            return grp.layout.views(grp.shard), None, -1
+            return grp.shard_views(), None, -1
         slot = i % len(self._pbufs)
         buf = self._pbufs[slot]
         if fused and self.fused_gather:
@@ -330,7 +340,7 @@ class ShardedEngine:
         previous owner is still being read) and the caller waits on ``event`` before the first use.
         Otherwise it runs on the compute stream inside an exposed-communication bracket."""
         if self.world == 1:
-            return grp.layout.views(grp.shard), grp.shard, None
+            return grp.shard_views(), grp.shard, None
         full = torch.empty(grp.layout.padded_numel, dtype=self.param_dtype, device=self.device)
         if self.poison:
             full.fill_(float("nan"))
@@ -348,6 +358,11 @@ class ShardedEngine:
     # named tensor to the start of the previous region; the last region is what is left at the front.
     REGION_STARTS = ("wd", "wgu", "wo")
 
+    # One rank: a group of at most this many elements is accumulated in one piece on the compute stream. The accumulation moves
+    # 10 bytes per element (16 M elements: 25 us alone); the side stream hides that under the next GEMMs, but its event
+    # hand-offs cost the host about 25 us per region, four regions per block.
+    INLINE_REDUCE = 16 << 20
+
     def _reduce(self, grp: ShardedGroup, gfull: torch.Tensor, slot: int = -1, last: bool = False,
                 region: int = 0, elem_lo: int = 0, elem_hi: Optional[int] = None, final: bool = True):
         """Reduce-scatter ``gfull`` (or elements [elem_lo, elem_hi) of it, one tensor region) into the
@@ -358,6 +373,13 @@ class ShardedEngine:
         the last microbatch of a step that kernel also adds the sum of squares of the finished
         accumulator to the step's norm scalar, so the optimizer does not have to read the accumulator
         again. ``final`` marks the last region of the buffer (bookkeeping of the group and the slot)."""
+        if self.world == 1 and hasattr(self.ops, "accumulate") and grp.gacc.numel() <= self.INLINE_REDUCE:
+            hi = grp.gacc.numel() if elem_hi is None else min(elem_hi, grp.gacc.numel())
+            if hi > elem_lo:
+                self.ops.accumulate(grp.gacc[elem_lo:hi], gfull[elem_lo:hi], grp.has_grad)
+            if final:
+                grp.has_grad = True
+            return None
         if self.symmetric:
             self.comm.grad_ready(gfull, region)
         with self.side.run(wait_current=True):
@@ -388,7 +410,8 @@ class ShardedEngine:
         if osft is not None and osft.owner_reduce:
             return osft.reducer(i, gbuf, gslot, last)
         grp = self.blocks[i]
-        per_region = self.region_overlap and (self.symmetric or (self.world == 1 and hasattr(self.ops, "accumulate")))
+        per_region = self.region_overlap and (self.symmetric or (self.world == 1 and hasattr(self.ops, "accumulate")
+                                                                 and grp.gacc.numel() > self.INLINE_REDUCE))
         state = {"hi": grp.layout.padded_numel, "k": 0}
 
         def notify(name):
@@ -449,9 +472,10 @@ class ShardedEngine:
         """
         cfg, nL = self.cfg, len(self.blocks)
         levels = [2] * nL
+        lvl1, lvl0 = self._kept_bytes(tokens)
         budget = self.activation_budget_bytes
         if budget is None:
-            budget = self._auto_activation_budget(tokens)
+            budget = self._auto_activation_budget(tokens, nL * lvl0)
         force = int(os.environ.get("MTB200_OFFLOAD_BLOCKS", "0"))
         if (budget < 0 or force) and self.device.type == "cuda":
             # Not even the block inputs fit next to the optimizer state (a 70B model with a sample far longer
@@ -464,16 +488,6 @@ class ShardedEngine:
                 levels[i] = 3
         if budget <= 0:
             return levels
-        es = 2 if self.param_dtype != torch.float32 else 4
-        h, f = cfg.hidden_size, (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
-        lvl1 = tokens * (cfg.q_size * es + cfg.num_attention_heads * 4)
-        # level 0 keeps qkv, the attention output, h1 and gate/up (the normalised inputs and the SwiGLU
-        # output are rebuilt in backward by elementwise kernels)
-        lvl0 = lvl1 + tokens * ((h + cfg.qkv_size + 2 * f) * es + 8)
-        if cfg.post_norm:   # both branch outputs before their norms and the q|k projections before theirs
-            lvl0 += tokens * (2 * h + cfg.q_size + cfg.kv_size) * es
-        if cfg.qk_norm:   # the q|k heads before their norm and one reciprocal RMS per head
-            lvl0 += tokens * ((cfg.q_size + cfg.kv_size) * es + (cfg.num_attention_heads + cfg.num_key_value_heads) * 4)
         for i in range(nL - 1, -1, -1):      # cheapest upgrade first: keep attention everywhere it fits
             if budget >= lvl1:
                 levels[i] = 1
@@ -484,7 +498,27 @@ class ShardedEngine:
                 budget -= lvl0 - lvl1
         return levels
 
-    def _auto_activation_budget(self, tokens: int) -> int:
+    def _kept_bytes(self, tokens: int) -> tuple:
+        """Bytes a block keeps beyond its input at checkpoint levels 1 and 0."""
+        cfg = self.cfg
+        es = 2 if self.param_dtype != torch.float32 else 4
+        h, f = cfg.hidden_size, (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
+        lvl1 = tokens * (cfg.q_size * es + cfg.num_attention_heads * 4)
+        # level 0 keeps qkv, the attention output, h1 and gate/up (the normalised inputs and the SwiGLU
+        # output are rebuilt in backward by elementwise kernels)
+        lvl0 = lvl1 + tokens * ((h + cfg.qkv_size + 2 * f) * es + 8)
+        if cfg.post_norm:   # both branch outputs before their norms and the q|k projections before theirs
+            lvl0 += tokens * (2 * h + cfg.q_size + cfg.kv_size) * es
+        if cfg.qk_norm:   # the q|k heads before their norm and one reciprocal RMS per head
+            lvl0 += tokens * ((cfg.q_size + cfg.kv_size) * es + (cfg.num_attention_heads + cfg.num_key_value_heads) * 4)
+        return lvl1, lvl0
+
+    # A minibatch whose kept activations and working set stay below this (a hundredth of the device) is planned without asking
+    # the driver and the allocator what is free, which costs the host a few hundred microseconds. Should it not fit after
+    # all, the forward pass is run again with every block at the cheapest level, as after any out-of-memory error.
+    ASSUMED_FREE = 2 << 30
+
+    def _auto_activation_budget(self, tokens: int, wanted: int) -> int:
         """Memory that can hold extra saved activations. Two bounds, the smaller wins:
 
         * a static plan: 93 % of the device minus optimizer/parameter state, the per-block inputs,
@@ -507,7 +541,11 @@ class ShardedEngine:
         root = 4 * v * h * 2
         bufs = sum(b.numel() * b.element_size() for b in self._pbufs + self._gbufs)
         transient = base + work + ce + root
-        static = int(0.93 * total - (self.state_bytes() + transient + bufs + (4 << 30)))
+        if self._state_bytes is None:
+            self._state_bytes = self.state_bytes()
+        static = int(0.93 * total - (self._state_bytes + transient + bufs + (4 << 30)))
+        if wanted + transient <= self.ASSUMED_FREE and wanted <= static and not self._oom_retries and (self.world == 1 or self.symmetric):
+            return static
         free, _ = torch.cuda.mem_get_info(self.device)
         cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
         live = int(0.97 * (free + cached) - transient - (3 << 30))
@@ -574,7 +612,7 @@ class ShardedEngine:
             # were all kept has no forward GEMM left, so its parameters are prefetched on the side stream
             cur = self._gather_block(i - 1, fused=saved[i - 1][1] is None) if i > 0 else None
             gbuf, gslot = self._grad_buffer(i)
-            g = self.blocks[i].layout.views(gbuf)
+            g = self._gviews[gslot]
             xin, acts, attn_state = saved.pop()
             if isinstance(xin, _HostInput):
                 xin = self._fetch_input(i, xin)
@@ -729,7 +767,10 @@ class ShardedEngine:
         sq = self._sq
         for g in live:
             if not g.sq_done:
-                sq += self.ops.sumsq(g.gacc)
+                if hasattr(self.ops, "add_sumsq"):
+                    self.ops.add_sumsq(g.gacc, sq)
+                else:
+                    sq += self.ops.sumsq(g.gacc)
         self.comm.all_reduce_sum(sq)
         norm = sq.sqrt().squeeze(0)
         if o.max_grad_norm and o.max_grad_norm > 0:

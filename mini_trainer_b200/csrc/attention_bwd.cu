@@ -13,17 +13,19 @@
 // tile, for dQ, where it is read MN-major. The room that frees holds a second Q tile.
 //
 // The MMAs of neighbouring iterations interleave so that the softmax of one runs under the products of another. Issue order:
-//   ... dK(i) dQ(i) | dV(i+1) dP(i+1) S(i+2) | dK(i+1) dQ(i+1) | ...
-// P(i+1) is computed while dK(i), dQ(i) run, dQ(i) is drained under dV(i+1), dS(i+1) is computed while S(i+2) and the tail
-// of dP(i+1) run. The chain that bounds an iteration is dS -> dK dQ dV dP -> dS: four products plus the dS half of the
-// softmax, where the form with everything in one chain (S dP | softmax | dK dV dQ | drain) had five products, the whole
-// softmax and the drain. 1 x 16384 tokens, 32/8 heads, D = 128: 6.49 -> 5.47 ms.
+//   ... dK(i) dQ(i) | dP(i+1) dV(i+1) S(i+2) | dK(i+1) dQ(i+1) | ...            (D = 64: dQ in front of dK)
+// P(i+1) is computed while dK(i), dQ(i) run and dQ(i) is drained, dS(i+1) while dV(i+1) and S(i+2) run. The chain that bounds
+// an iteration is dS -> dK dQ -> drain -> dP -> dS, where the form with everything in one chain (S dP | softmax | dK dV dQ |
+// drain) had five products, the whole softmax and the drain. At D = 128 the chain and the shared-memory port (three products
+// with both operands there, loads, the dS tile, dQ's staging and its read-out: about 3800 clocks) are of one length.
+// 1 x 16384 tokens, 32/8 heads: 6.49 -> 5.5 ms at D = 128 (either order of dK, dQ and of dP, dV measured the same there),
+// 5.28 -> 3.15 ms at D = 64 (3.57 with dV in front of dP and the shared columns).
 //
-// dQ shares the columns of dP (read out before the next dP is issued). Its tiles (several key blocks contribute to one
-// query block) go through a 32 KB staging buffer, 64 columns at a time, into an fp32 [T, Hq*D] accumulator with TMA tensor
-// reduces (cp.reduce.async.bulk.tensor .add, one 32-column x 128-row box each, 128B-swizzled so the staging stores are free of
-// bank conflicts); a small kernel rounds the accumulator to bf16 afterwards. Four warps of their own drain, one more issues
-// the reduces, so the softmax warps see nothing of dQ.
+// dQ shares the columns of dP at D = 128 (it is read out before the next dP is issued) and has its own at D = 64. Its tiles
+// (several key blocks contribute to one query block) go through a 32 KB staging buffer, 64 columns at a time, into an fp32
+// [T, Hq*D] accumulator with TMA tensor reduces (cp.reduce.async.bulk.tensor .add, one 32-column x 128-row box each,
+// 128B-swizzled so the staging stores are free of bank conflicts); a small kernel rounds the accumulator to bf16 afterwards.
+// Four warps of their own drain, one more issues the reduces, so the softmax warps see nothing of dQ.
 //
 // Rows past the end of the sequence contribute nothing: a query's lse is staged as +infinity, a key's scores are masked.
 #include <cuda.h>
@@ -144,7 +146,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 256 + D;
-  const uint32_t t_dq = t_dp;
+  // dQ has columns of its own where they are left over (D = 64); at D = 128 it shares those of dP
+  constexpr bool DQ_OWN = 2 * 128 + 3 * D <= 512;
+  const uint32_t t_dq = DQ_OWN ? tmem_base + 256 + 2 * D : t_dp;
 
   if (warp < 4) {
     setmaxnreg_dec<AB_REGS_IO>();
@@ -195,14 +199,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
           for (int k = 0; k < D / 16; ++k) umma_bf16_lo(t_s, dKk + kstep(k), dQk + qbuf(it) + kstep(k), id_nt, k != 0);
           umma_commit(s_full);
         };
-        auto issue_dp = [&]() {   // dV of the same iteration has been issued: dO is free when both are done
+        auto issue_dp = [&]() {
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) umma_bf16_lo(t_dp, dVk + kstep(k), dDOk + kstep(k), id_nt, k != 0);
           umma_commit(dp_full);
         };
-        auto issue_dv = [&](int it) {
+        auto issue_dv = [&](int it) {   // dP of the same iteration has been issued: dO is free when both are done
 #pragma unroll
           for (int k = 0; k < AB_B / 16; ++k) umma_bf16_ts_lo(t_dv, t_s + astep(k), dDOm + mstep(k), id_ts, it != 0 || k != 0);
+          umma_commit(do_free);
         };
         if (!mbar_wait(kv_full, 0, abort_flag)) { atomicExch(p.status, 22); goto done; }
         if (!mbar_wait(&q_full[0], 0, abort_flag)) { atomicExch(p.status, 23); goto done; }
@@ -214,30 +219,35 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         if (!mbar_wait(p_ready, 0, abort_flag)) { atomicExch(p.status, 25); goto done; }
         tc_fence_after();
         issue_dv(0);
-        umma_commit(do_free);
         if (n_iters > 1) {
           if (!mbar_wait(&q_full[1], 0, abort_flag)) { atomicExch(p.status, 23); goto done; }
           tc_fence_after();
           issue_s(1);
         }
-        for (int it = 0; it < n_iters; ++it) {
-          if (!mbar_wait(ds_ready, it & 1, abort_flag)) { atomicExch(p.status, 25); goto done; }
-          tc_fence_after();
+        auto issue_dk = [&](int it) {
 #pragma unroll
           for (int k = 0; k < AB_B / 16; ++k) umma_bf16_ts_lo(t_dk, t_dp + astep(k), dQm + qbuf(it) + mstep(k), id_ts, it != 0 || k != 0);
           umma_commit(&q_free[it & 1]);
+        };
+        auto issue_dq = [&]() {
 #pragma unroll
           for (int k = 0; k < AB_B / 16; ++k) umma_bf16_lo(t_dq, dDSm + mstep(k), dKm + mstep(k), id_dq, k != 0);
           umma_commit(dq_full);
+        };
+        for (int it = 0; it < n_iters; ++it) {
+          if (!mbar_wait(ds_ready, it & 1, abort_flag)) { atomicExch(p.status, 25); goto done; }
+          if (DQ_OWN && it > 0 && !mbar_wait(dq_read, (it - 1) & 1, abort_flag)) { atomicExch(p.status, 24); goto done; }
+          tc_fence_after();
+          if (DQ_OWN) { issue_dq(); issue_dk(it); }
+          else { issue_dk(it); issue_dq(); }     // dK reads dS^T from the columns that dQ overwrites
           if (it + 1 < n_iters) {
             if (!mbar_wait(do_full, (it + 1) & 1, abort_flag)) { atomicExch(p.status, 23); goto done; }
+            if (!DQ_OWN && !mbar_wait(dq_read, it & 1, abort_flag)) { atomicExch(p.status, 24); goto done; }
+            tc_fence_after();
+            issue_dp();
             if (!mbar_wait(p_ready, (it + 1) & 1, abort_flag)) { atomicExch(p.status, 25); goto done; }
             tc_fence_after();
             issue_dv(it + 1);
-            if (!mbar_wait(dq_read, it & 1, abort_flag)) { atomicExch(p.status, 24); goto done; }
-            tc_fence_after();
-            issue_dp();
-            umma_commit(do_free);
             if (it + 2 < n_iters) {
               if (!mbar_wait(&q_full[it & 1], ((it + 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 23); goto done; }
               tc_fence_after();

@@ -11,9 +11,12 @@
 // Why pairs: a tile's chain is S -> softmax -> P V, and with one tile per CTA the tensor core idles under the softmax and the
 // softmax under the products, or (with two S buffers of one tile) all softmax warps do the same phase at the same time and
 // queue on the special-function unit. Two independent tiles take turns: while A is in its softmax the tensor core runs
-// P V and the next S of B. K and V are loaded and multiplied once per pair. A row belongs to one thread, so nothing is
-// exchanged between threads. 1 x 16384 tokens, 32/8 heads, D = 128: 1.82 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64:
+// P V and the next S of B. K and V are loaded once per pair. A row belongs to one thread, so nothing is exchanged between
+// threads (two threads per row with their maxima exchanged through shared memory measured 1.92 ms below). P is handed over in
+// two halves of 64 keys, so the first half's products run under the second half's exponentials. 1 x 16384 tokens, 32/8 heads, D = 128: 1.65 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64:
 // 64 us (one tile per CTA, two threads per row: 1.94 ms and 94 us).
+// One long sequence at D = 64, where the products are short and the exponentials bound both forms, is the exception: 1.65 -> 1.81 ms
+// for 16384 tokens.
 //
 // CTAs are persistent (one per SM): barriers and tensor memory are set up once, K and V of the next item are prefetched
 // under the current one's tail, and the epilogue of an item runs under the next item's first product. Items come most work
@@ -119,9 +122,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
   uint64_t* v_full = bars + 6;        // [2]
   uint64_t* v_empty = bars + 8;       // [2] P V of both tiles has completed
   uint64_t* s_full = bars + 10;       // [A, B]
-  uint64_t* p_ready = bars + 12;      // [A, B] P in tensor memory, O rescaled (4 arrivals)
-  uint64_t* pv_done = bars + 14;      // [A, B] P V complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* p_ready = bars + 12;      // [A, B][keys 0-63, keys 64-127] P in tensor memory, O rescaled (4 arrivals)
+  uint64_t* pv_done = bars + 16;      // [A, B] P V complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -129,7 +132,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     mbar_init(q_full, 1); mbar_init(q_free, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); mbar_init(&pv_done[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&p_ready[2 * i], 4); mbar_init(&p_ready[2 * i + 1], 4); mbar_init(&pv_done[i], 1);
     }
     *abort_flag = 0;
     fence_mbar_init();
@@ -195,11 +198,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
             umma_bf16_lo(tmem_base + g * ATT_B, dQ + g * (L::TILE >> 4) + kstep(k), dK + stage(t) + kstep(k), idesc_qk, k != 0);
           umma_commit(&s_full[g]);
         };
-        auto issue_pv = [&](int g, uint32_t t, bool first) {
+        auto issue_pv = [&](int g, uint32_t t, bool first, int half) {   // the products with 64 keys; both halves make a P V
 #pragma unroll
-          for (int k = 0; k < ATT_B / 16; ++k)   // 16 keys = 8 packed columns of P
-            umma_bf16_ts_lo(tmem_base + 2 * ATT_B + g * D, tmem_base + g * ATT_B + k * 8, dV + stage(t) + k * 128, idesc_pv, !first || k != 0);
-          umma_commit(&pv_done[g]);
+          for (int k = 0; k < ATT_B / 32; ++k) {   // 16 keys = 8 packed columns of P
+            const int kk = half * (ATT_B / 32) + k;
+            umma_bf16_ts_lo(tmem_base + 2 * ATT_B + g * D, tmem_base + g * ATT_B + kk * 8, dV + stage(t) + kk * 128, idesc_pv, !first || kk != 0);
+          }
         };
         AttWork w;
         uint32_t units = 0, kt = 0;
@@ -221,9 +225,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
               if (j >= w.n[g]) continue;
-              if (!mbar_wait(&p_ready[g], cnt[g] & 1, abort_flag)) { atomicExch(p.status, 15); goto done; }
-              tc_fence_after();
-              issue_pv(g, t, j == 0);
+#pragma unroll
+              for (int half = 0; half < 2; ++half) {
+                if (!mbar_wait(&p_ready[2 * g + half], cnt[g] & 1, abort_flag)) { atomicExch(p.status, 15); goto done; }
+                tc_fence_after();
+                issue_pv(g, t, j == 0, half);
+              }
+              umma_commit(&pv_done[g]);
               ++cnt[g];
               if (j + 1 < w.n[g]) {   // P was the last reader of these columns: the next S of this tile follows at once
                 if (!k_next && !mbar_wait(&k_full[(t + 1) & 1], ((t + 1) >> 1) & 1, abort_flag)) { atomicExch(p.status, 14); goto done; }
@@ -319,12 +327,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
             pk[i] = pack_bf16(e.x, e.y);
           }
           tmem_st_32x16(ts + c * 16, pk);
+          if (c & 1) {   // half of the keys: their products start under the other half's exponentials
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_ready[2 * g + (c >> 1)]);
+          }
         }
-        tmem_st_wait();
         l += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[g]);
       }
       // epilogue: O / l -> out, lse. The next unit's first P V overwrites O only after this thread has handed over its P.
       if (!mbar_wait(&pv_done[g], (cnt - 1) & 1, abort_flag)) { atomicExch(p.status, 19); goto done; }

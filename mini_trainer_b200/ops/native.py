@@ -123,13 +123,15 @@ class NativeOps:
         self.ce_chunk = ce_chunk
         self.attention_impl = attention or os.environ.get("MTB200_ATTENTION", "native")
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-        # MTB200_GEMM2=1: two-CTA (cta_group::2, 256x256 tiles) GEMM for problems with about a full wave of such
-        # tiles or more. It is the faster kernel in isolation (0.92-0.95 of the cuBLAS burst figure against
-        # 0.74-0.90), but a training step runs at the 1000 W power cap, where the clock settles at what the GEMMs
-        # draw: with the CTA-pair kernel the SM clock drops by 12-16 % for EVERY kernel of the step, and the
-        # latency-bound ones (attention, normalisation) lose more than the GEMMs gain: measured end to end on
-        # one GPU 25.2 s against 23.9 s per step. So the one-CTA kernel is the default.
-        self.use_gemm2 = os.environ.get("MTB200_GEMM2", "0") == "1"
+        # GEMM kernel for problems with about a full wave of 256x256 tiles or more. The CTA-pair kernel (cta_group::2) loads half
+        # of what the one-CTA kernel loads per product and is the faster one in itself, but it draws more power: in a step
+        # made of long GEMMs, which runs at the 1000 W cap, it lowers the clock of EVERY kernel by 12-16 % and the step gets
+        # slower (8B model, 64 000-token minibatches: 9.77 s per step with one CTA, 10.36 with pairs). Where GEMMs are short
+        # the cap does not bind (1.5B model, 8000-token minibatches: 729 and 700 ms, clocks 1530 and 1515 MHz; forward +
+        # backward of one of its blocks at 6000 tokens: 1.99 and 1.91 ms). The line is drawn at a GEMM of about 0.8 ms.
+        # MTB200_GEMM2=0 / 1 forces one kernel for all of them (1: also for the fused gathers).
+        self.use_gemm2 = os.environ.get("MTB200_GEMM2") == "1"
+        self.pair_max_flops = 0.0 if os.environ.get("MTB200_GEMM2") == "0" else 1e12
         self.launches = 0
         self.profile = [] if os.environ.get("MTB200_PROFILE") else None
         self._scratch = {}
@@ -222,7 +224,7 @@ class NativeOps:
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
         assert residual is None or residual.dtype == out.dtype
         if two_cta is None:
-            two_cta = self.use_gemm2 and (-(-M // 256)) * (-(-N // 256)) >= 64
+            two_cta = (self.use_gemm2 or 2.0 * M * N * K <= self.pair_max_flops) and (-(-M // 256)) * (-(-N // 256)) >= 64
         st = self._st()
         ws = self._split_workspace(st)
         self._call("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),

@@ -155,11 +155,16 @@ def block_forward(ops, cfg: ModelConfig, p: dict, x: torch.Tensor, batch: Packed
     n1, rstd1 = _norm(ops, cfg, x, p, "ln1", "bln1")
     qkv = ops.linear(n1, p["wqkv"], p.get("bqkv"), gather=None if plan is None else (plan, 0))
     qk_pre = rstd_qk = None
-    if cfg.qk_norm:   # the backward of the norm needs its input; the qkv tensor itself goes on normalised and rotated
+    # the norm and the rotation of q and k in one kernel, where the backend has it (it rotates whole heads)
+    fused_qk = cfg.qk_norm and hasattr(ops, "qk_norm_rope_") and cfg.rotary_dim == cfg.head_dim
+    if fused_qk:
+        qk_pre, rstd_qk = ops.qk_norm_rope_(qkv, p["qn"], p["kn"], cfg.rms_norm_eps, cfg.num_attention_heads, cfg.num_key_value_heads,
+                                            cfg.head_dim, batch.position_ids, inv_freq, keep=bool(keep))
+    elif cfg.qk_norm:   # the backward of the norm needs its input; the qkv tensor itself goes on normalised and rotated
         qk_pre = qkv[:, : cfg.q_size + cfg.kv_size].clone()
         rstd_qk = ops.head_rmsnorm_(qkv, p["qn"], p["kn"], cfg.rms_norm_eps, cfg.num_attention_heads,
                                     cfg.num_key_value_heads, cfg.head_dim)
-    if inv_freq is not None:   # None: a layer without positional rotation (SmolLM3's NoPE layers)
+    if inv_freq is not None and not fused_qk:   # None: a layer without positional rotation (SmolLM3's NoPE layers)
         ops.rope_(qkv, batch.position_ids, inv_freq, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
                   rot_dim=cfg.rotary_dim)
     rm = cfg.residual_multiplier   # Granite scales every branch output before the residual add (1.0 elsewhere)
@@ -257,12 +262,16 @@ def _attention_backward(ops, cfg: ModelConfig, p: dict, g: dict, a: BlockActs, d
                              batch.max_seqlen, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
                              scale=cfg.attention_scale)
     del dattn
-    if inv_freq is not None:
-        ops.rope_(dqkv, batch.position_ids, inv_freq, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
-                  inverse=True, rot_dim=cfg.rotary_dim)
-    if cfg.qk_norm:
-        ops.head_rmsnorm_bwd_(dqkv, a.qk_pre, a.rstd_qk, p["qn"], p["kn"], g["qn"], g["kn"], cfg.num_attention_heads,
-                              cfg.num_key_value_heads, cfg.head_dim)
+    if cfg.qk_norm and hasattr(ops, "qk_norm_rope_bwd_") and cfg.rotary_dim == cfg.head_dim:
+        ops.qk_norm_rope_bwd_(dqkv, a.qk_pre, a.rstd_qk, p["qn"], p["kn"], g["qn"], g["kn"], cfg.num_attention_heads,
+                              cfg.num_key_value_heads, cfg.head_dim, batch.position_ids, inv_freq)
+    else:
+        if inv_freq is not None:
+            ops.rope_(dqkv, batch.position_ids, inv_freq, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,
+                      inverse=True, rot_dim=cfg.rotary_dim)
+        if cfg.qk_norm:
+            ops.head_rmsnorm_bwd_(dqkv, a.qk_pre, a.rstd_qk, p["qn"], p["kn"], g["qn"], g["kn"], cfg.num_attention_heads,
+                                  cfg.num_key_value_heads, cfg.head_dim)
     dn1 = ops.linear_dgrad(dqkv, p["wqkv"])
     n1 = a.n1 if a.n1 is not None else _norm(ops, cfg, a.x, p, "ln1", "bln1")[0]
     ops.linear_wgrad(dqkv, n1, g["wqkv"], g.get("bqkv"))

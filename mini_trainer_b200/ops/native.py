@@ -55,9 +55,9 @@ class _Sig:
     mtb200_layernorm_fwd = [P, P, P, P, P, P, F, I, I, P, P]
     mtb200_layernorm_bwd = [P, P, P, P, P, P, P, P, P, P, I, I, P, P]
     mtb200_rope = [P, P, P, I, L, I, I, I, P]
-    mtb200_head_rmsnorm_fwd = [P, P, P, P, F, I, L, I, I, I, P]
+    mtb200_head_rmsnorm_fwd = [P, P, P, P, P, P, P, F, I, L, I, I, I, P]
     mtb200_head_rmsnorm_bwd_blocks = [I, I]
-    mtb200_head_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, L, L, I, I, I, P]
+    mtb200_head_rmsnorm_bwd = [P, P, P, P, P, P, P, P, P, P, I, L, L, I, I, I, P]
     mtb200_swiglu_fwd = [P, P, L, I, P]
     mtb200_swiglu_bwd = [P, P, P, L, I, P]
     mtb200_swiglu_bwd_act = [P, P, P, L, I, P]
@@ -335,21 +335,34 @@ class NativeOps:
     def head_rmsnorm_(self, qkv, wq, wk, eps, n_q_heads, n_kv_heads, head_dim):
         """Normalises every q head (weight ``wq``) and k head (``wk``) of ``qkv`` over ``head_dim``, in place;
         returns the reciprocal RMS per (token, head), ``[T * (n_q + n_kv)]`` fp32."""
+        return self.qk_norm_rope_(qkv, wq, wk, eps, n_q_heads, n_kv_heads, head_dim, None, None, keep=False)[1]
+
+    def qk_norm_rope_(self, qkv, wq, wk, eps, n_q_heads, n_kv_heads, head_dim, position_ids, inv_freq, keep=True):
+        """``head_rmsnorm_`` and then ``rope_`` (unless ``inv_freq`` is ``None``) in one pass. Returns ``(pre, rstd)``; ``pre``, the
+        q|k heads as they came, is only made when ``keep``."""
         T, nh = qkv.shape[0], n_q_heads + n_kv_heads
+        assert inv_freq is None or position_ids.dtype == torch.int32
         rstd = torch.empty(T * nh, dtype=torch.float32, device=self.device)
-        self._call("mtb200_head_rmsnorm_fwd", qkv.data_ptr(), wq.data_ptr(), wk.data_ptr(), rstd.data_ptr(), eps, T,
-                   qkv.stride(0), n_q_heads, nh, head_dim, self._st())
-        return rstd
+        pre = torch.empty(T, nh * head_dim, dtype=qkv.dtype, device=self.device) if keep else None
+        self._call("mtb200_head_rmsnorm_fwd", qkv.data_ptr(), wq.data_ptr(), wk.data_ptr(), _ptr(pre), rstd.data_ptr(),
+                   None if inv_freq is None else position_ids.data_ptr(), _ptr(inv_freq), eps, T, qkv.stride(0), n_q_heads, nh,
+                   head_dim, self._st())
+        return pre, rstd
 
     def head_rmsnorm_bwd_(self, dqkv, pre, rstd, wq, wk, dwq_out, dwk_out, n_q_heads, n_kv_heads, head_dim):
         """In place on the q and k columns of ``dqkv``: gradient of the normalised heads in, gradient of the projection
         output out. ``pre``: the q|k heads before the norm, ``[T, (n_q + n_kv) * head_dim]``."""
+        return self.qk_norm_rope_bwd_(dqkv, pre, rstd, wq, wk, dwq_out, dwk_out, n_q_heads, n_kv_heads, head_dim, None, None)
+
+    def qk_norm_rope_bwd_(self, dqkv, pre, rstd, wq, wk, dwq_out, dwk_out, n_q_heads, n_kv_heads, head_dim, position_ids, inv_freq):
+        """The inverse rotation (unless ``inv_freq`` is ``None``) and then ``head_rmsnorm_bwd_`` in one pass."""
         T, nh = dqkv.shape[0], n_q_heads + n_kv_heads
+        assert inv_freq is None or position_ids.dtype == torch.int32
         blocks = self.lib.mtb200_head_rmsnorm_bwd_blocks(T, nh)
         part = self._buf("head_rmsnorm_dw", blocks * 2 * head_dim, torch.float32)
         self._call("mtb200_head_rmsnorm_bwd", dqkv.data_ptr(), pre.data_ptr(), rstd.data_ptr(), wq.data_ptr(), wk.data_ptr(),
-                   part.data_ptr(), dwq_out.data_ptr(), dwk_out.data_ptr(), T, dqkv.stride(0), pre.stride(0), n_q_heads, nh,
-                   head_dim, self._st(), n=2)
+                   part.data_ptr(), dwq_out.data_ptr(), dwk_out.data_ptr(), None if inv_freq is None else position_ids.data_ptr(),
+                   _ptr(inv_freq), T, dqkv.stride(0), pre.stride(0), n_q_heads, nh, head_dim, self._st(), n=2)
         return dqkv
 
     # -- attention --------------------------------------------------------------------

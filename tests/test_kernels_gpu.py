@@ -677,3 +677,28 @@ def test_linear_ce_chunks(ops, V):
     assert (res[0][0] - ref).abs().max() < 2e-3     # bf16 logits on both sides, fp32 sums of up to V exponentials
     for a, b in zip(*res):
         assert rel_err(a, b) < 4e-3
+
+
+# heads that do not fill a warp's group of four; the pass with the rotation against the norm and the rotation as passes of their own
+@pytest.mark.parametrize("D,hq,hkv,T", [(128, 4, 1, 257), (64, 4, 2, 33), (256, 2, 1, 100), (128, 16, 8, 1031)])
+def test_qk_norm_with_rotation(ops, D, hq, hkv, T):
+    torch.manual_seed(T)
+    nh = hq + hkv
+    qkv, dqkv = bf(T, (hq + 2 * hkv) * D), bf(T, (hq + 2 * hkv) * D)
+    wq, wk = (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16(), (1 + 0.1 * torch.randn(D, device="cuda")).bfloat16()
+    pos = (torch.arange(T, device="cuda") * 7 % 5000).to(torch.int32)
+    inv = (1e4 ** (-torch.arange(0, D, 2, device="cuda").float() / D))
+    a, b = qkv.clone(), qkv.clone()
+    pre, rstd = ops.qk_norm_rope_(a, wq, wk, 1e-6, hq, hkv, D, pos, inv)
+    r2 = ops.head_rmsnorm_(b, wq, wk, 1e-6, hq, hkv, D)
+    ops.rope_(b, pos, inv, hq, hkv, D)
+    assert torch.equal(pre, qkv[:, : nh * D]) and torch.equal(rstd, r2) and torch.equal(a[:, nh * D:], qkv[:, nh * D:])
+    # same roundings in between; the compiler may contract the rotation's products differently, one bf16 step
+    assert (a.float() - b.float()).abs().max() <= 2 ** -7 * b.float().abs().max() and rel_err(a, b) < 1e-3
+    g = [torch.empty_like(wq) for _ in range(4)]
+    c, d = dqkv.clone(), dqkv.clone()
+    ops.qk_norm_rope_bwd_(c, pre, rstd, wq, wk, g[0], g[1], hq, hkv, D, pos, inv)
+    ops.rope_(d, pos, inv, hq, hkv, D, inverse=True)
+    ops.head_rmsnorm_bwd_(d, pre, rstd, wq, wk, g[2], g[3], hq, hkv, D)
+    assert rel_err(c, d) < 1e-3 and rel_err(g[0], g[2]) < 5e-3 and rel_err(g[1], g[3]) < 5e-3
+    assert torch.equal(c[:, nh * D:], dqkv[:, nh * D:])

@@ -65,36 +65,20 @@ def make_packed_batch(mb: dict, device, non_blocking: bool = True) -> PackedBatc
         cu = torch.cat([starts, torch.tensor([pos.numel()], dtype=torch.int32)])
     cu_host = cu.tolist()
     max_seqlen = int(mb.get("max_seqlen", max(b - a for a, b in zip(cu_host[:-1], cu_host[1:]))))
-    counted = (targets != -100).nonzero().flatten()
+    moved = [0]
+
+    def mv(t):
+        moved[0] += t.numel() * t.element_size()
+        return t.to(device, non_blocking=non_blocking)
+
     rows = sel = None
+    counted = (targets != -100).nonzero().flatten()
     # MTB200_HEAD_ALL_ROWS=1 runs the head on every row, as the reference does (for A/B timing)
     if counted.numel() < targets.numel() and os.environ.get("MTB200_HEAD_ALL_ROWS", "0") != "1":
-        rows, sel = counted, targets[counted]
-    host = [ids, targets, pos.to(torch.int32), cu, rows, sel]
-    dev, moved = _to_device(host, device, non_blocking)
-    batch = PackedBatch(dev[0], dev[1], dev[2], dev[3], cu_host, max_seqlen, dev[4], dev[5])
-    batch.h2d_bytes = moved
+        rows, sel = mv(counted), mv(targets[counted])
+    batch = PackedBatch(mv(ids), mv(targets), mv(pos.to(torch.int32)), mv(cu), cu_host, max_seqlen, rows, sel)
+    batch.h2d_bytes = moved[0]
     return batch
-
-
-def _to_device(tensors: list, device, non_blocking: bool):
-    """Copies host tensors (``None`` stays ``None``) to ``device``: ``(copies, bytes)``. To a GPU they travel in one pinned buffer
-    and one copy, each starting on an 8-byte boundary of it."""
-    moved = sum(t.numel() * t.element_size() for t in tensors if t is not None)
-    if torch.device(device).type != "cuda" or any(t is not None and t.device.type != "cpu" for t in tensors):
-        return [None if t is None else t.to(device, non_blocking=non_blocking) for t in tensors], moved
-    words = [0 if t is None else -(-t.numel() * t.element_size() // 8) for t in tensors]
-    stage = torch.empty(sum(words), dtype=torch.int64, pin_memory=True)
-    out, at = [], 0
-    for t, n in zip(tensors, words):
-        if t is not None:
-            stage[at:at + n].view(t.dtype)[: t.numel()].copy_(t)
-        at += n
-    flat, at = stage.to(device, non_blocking=non_blocking), 0
-    for t, n in zip(tensors, words):
-        out.append(None if t is None else flat[at:at + n].view(t.dtype)[: t.numel()])
-        at += n
-    return out, moved
 
 
 def _nw(cfg: ModelConfig, w: torch.Tensor) -> torch.Tensor:

@@ -13,7 +13,6 @@ import os
 from dataclasses import dataclass
 from ctypes import c_float, c_int, c_longlong, c_void_p
 
-import numpy as np
 import torch
 
 from .. import build as _build
@@ -208,9 +207,15 @@ class NativeOps:
     # -- GEMM -------------------------------------------------------------------------
     def _split_workspace(self, stream):
         """Split-K workspace of a stream: arrival counters (zero between launches) and fp32 partials. GEMMs of one stream run
-        one after the other, those of different streams may overlap, so each stream has its own."""
+        one after the other, those of different streams may overlap, so each stream has its own (the last eight streams do;
+        a dropped one goes back to its stream's pool, behind the launches that use it). ``None`` under capture: a graph may be
+        replayed beside anything, so its launches never split."""
+        if torch.cuda.is_current_stream_capturing():
+            return None
         ws = self._gemm_ws.get(stream)
         if ws is None:
+            if len(self._gemm_ws) >= 8:
+                self._gemm_ws.pop(next(iter(self._gemm_ws), None), None)
             ws = torch.empty(_SPLIT_COUNTERS + _SPLIT_FLOATS, dtype=torch.float32, device=self.device)
             ws[: _SPLIT_COUNTERS].zero_()
             self._gemm_ws[stream] = ws
@@ -230,7 +235,7 @@ class NativeOps:
         self._call("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
                    residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha),
-                   ws.data_ptr(), ws.numel() * 4, _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
+                   _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
         return out
 
     # -- embedding --------------------------------------------------------------------
@@ -375,16 +380,14 @@ class NativeOps:
         hit = self._attn_plan_cache.get(key)
         if hit is not None and hit[0] is cu_host:
             return hit[1]
-        cu = np.asarray(cu_host, dtype=np.int64)
-        lens = cu[1:] - cu[:-1]
-        per = -(-lens // block)                                    # blocks of every sequence
-        seq = np.repeat(np.arange(lens.shape[0]), per)
-        s0 = (np.arange(seq.shape[0]) - np.repeat(np.cumsum(per) - per, per)) * block
-        work = s0 if most_work_last_block else lens[seq] - s0
-        order = np.argsort(-work, kind="stable")
-        host = torch.empty(seq.shape[0], 3, dtype=torch.int32, pin_memory=True)
-        host.numpy()[:] = np.stack([cu[:-1][seq], lens[seq], s0], axis=1)[order]
-        table = host.to(self.device, non_blocking=True)
+        items = []
+        for a, b in zip(cu_host[:-1], cu_host[1:]):
+            n = b - a
+            for s0 in range(0, n, block):
+                work = s0 if most_work_last_block else n - s0
+                items.append((work, a, n, s0))
+        items.sort(key=lambda it: -it[0])
+        table = torch.tensor([it[1:] for it in items], dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
         if len(self._attn_plan_cache) > 8:
             self._attn_plan_cache.clear()
         self._attn_plan_cache[key] = (cu_host, table)
@@ -416,7 +419,7 @@ class NativeOps:
         ws = self._split_workspace(st)
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
-                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, ws.data_ptr(), ws.numel() * 4, scale,
+                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), scale,
                    self.status.data_ptr(), st, n=3)
         return dqkv
 

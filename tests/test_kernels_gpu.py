@@ -702,3 +702,31 @@ def test_qk_norm_with_rotation(ops, D, hq, hkv, T):
     ops.head_rmsnorm_bwd_(d, pre, rstd, wq, wk, g[2], g[3], hq, hkv, D)
     assert rel_err(c, d) < 1e-3 and rel_err(g[0], g[2]) < 5e-3 and rel_err(g[1], g[3]) < 5e-3
     assert torch.equal(c[:, nh * D:], dqkv[:, nh * D:])
+
+
+def test_split_workspaces_are_per_stream_and_bounded(ops):
+    """Split GEMMs on several streams at once, more streams than workspaces are kept, and a captured one."""
+    torch.manual_seed(3)
+    M, N, K = 256, 256, 8192
+    a, b = bf(M, K), bf(N, K, scale=0.1)
+    ref = a.float() @ b.float().t()
+    streams = [torch.cuda.Stream() for _ in range(11)]
+    outs = [torch.empty(M, N, dtype=torch.bfloat16, device="cuda") for _ in streams]
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for s, o in zip(streams, outs):
+            with torch.cuda.stream(s):
+                ops.gemm(a, False, b, False, o, M, N, K)
+    torch.cuda.synchronize()
+    assert len(ops._gemm_ws) <= 8
+    assert all(torch.equal(o, outs[0]) for o in outs) and rel_err(outs[0], ref) < 4e-3
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    kept = set(ops._gemm_ws)
+    with torch.cuda.graph(g):
+        ops.gemm(a, False, b, False, out, M, N, K)
+    assert set(ops._gemm_ws) == kept
+    g.replay()
+    torch.cuda.synchronize()
+    assert rel_err(out, ref) < 4e-3
+    ops.check_status()

@@ -16,8 +16,8 @@
 //   ... dK(i) dQ(i) | dP(i+1) dV(i+1) S(i+2) | dK(i+1) dQ(i+1) | ...            (D = 64: dQ in front of dK)
 // P(i+1) is computed while dK(i), dQ(i) run and dQ(i) is drained, dS(i+1) while dV(i+1) and S(i+2) run. The chain that bounds
 // an iteration is dS -> dK dQ -> drain -> dP -> dS, where the form with everything in one chain (S dP | softmax | dK dV dQ |
-// drain) had five products, the whole softmax and the drain. At D = 128 the chain and the shared-memory port (three products
-// with both operands there, loads, the dS tile, dQ's staging and its read-out: about 3800 clocks) are of one length.
+// drain) had five products, the whole softmax and the drain. At D = 128 an iteration takes about 4950 clocks whichever way the
+// products are ordered: what paces it is dQ, 64 KB of tensor reduces per iteration (32 KB at D = 64: about 2900 clocks).
 // 1 x 16384 tokens, 32/8 heads: 6.49 -> 5.5 ms at D = 128 (either order of dK, dQ and of dP, dV measured the same there),
 // 5.28 -> 3.15 ms at D = 64 (3.57 with dV in front of dP and the shared columns).
 //

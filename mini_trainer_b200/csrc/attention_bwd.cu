@@ -16,10 +16,11 @@
 //   ... dK(i) dQ(i) | dP(i+1) dV(i+1) S(i+2) | dK(i+1) dQ(i+1) | ...            (D = 64: dQ in front of dK)
 // P(i+1) is computed while dK(i), dQ(i) run and dQ(i) is drained, dS(i+1) while dV(i+1) and S(i+2) run. The chain that bounds
 // an iteration is dS -> dK dQ -> drain -> dP -> dS, where the form with everything in one chain (S dP | softmax | dK dV dQ |
-// drain) had five products, the whole softmax and the drain. At D = 128 an iteration takes about 4950 clocks whichever way the
-// products are ordered: what paces it is dQ, 64 KB of tensor reduces per iteration (32 KB at D = 64: about 2900 clocks).
-// 1 x 16384 tokens, 32/8 heads: 6.49 -> 5.5 ms at D = 128 (either order of dK, dQ and of dP, dV measured the same there),
-// 5.28 -> 3.15 ms at D = 64 (3.57 with dV in front of dP and the shared columns).
+// drain) had five products, the whole softmax and the drain. At D = 128 an iteration takes about 4950 clocks for 2560 of MMA,
+// the same for every order of the products tried. A fifth of it is dQ's tensor reduces, 64 KB per iteration (without them, results
+// apart, 16384 tokens take 4.6 instead of 5.7 ms); the rest is the hand-offs and latencies of the chain.
+// 1 x 16384 tokens, 32/8 heads: 6.5 -> 5.5 ms at D = 128 (main kernel),
+// 5.3 -> 3.2 ms at D = 64 (all passes; 3.6 with dV in front of dP and the shared columns).
 //
 // dQ shares the columns of dP at D = 128 (it is read out before the next dP is issued) and has its own at D = 64. Its tiles
 // (several key blocks contribute to one query block) go through a 32 KB staging buffer, 64 columns at a time, into an fp32

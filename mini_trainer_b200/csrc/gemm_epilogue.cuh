@@ -48,28 +48,25 @@ struct EpiOut {
   uint32_t n;           // boxes so far
 };
 
-// Buffer for the next box: free once at most the last store (the other buffer's) is still reading.
+// Buffer for the next box: free once at most the last store (the other buffer's) is still reading. Every box that is taken here is
+// stored and committed, or the count of pending groups would no longer name the buffer.
 __device__ __forceinline__ uint8_t* next_box(EpiOut& o, int lane) {
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+  if (lane == 0) bulk_wait_read<1>();
   __syncwarp();
   return o.stage + (o.n & 1) * STORE_BOX;
 }
-__device__ __forceinline__ void store_box(EpiOut& o, const uint8_t* box, int x, int y, int rows, int lane) {
+__device__ __forceinline__ void store_box(EpiOut& o, const uint8_t* box, int x, int y, int lane) {
   fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0 && y < rows) {
-    if (o.z < 0)
-      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                   ::"l"(reinterpret_cast<uint64_t>(o.map)), "r"(smem_u32(box)), "r"(x), "r"(y) : "memory");
-    else
-      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-                   ::"l"(reinterpret_cast<uint64_t>(o.map)), "r"(smem_u32(box)), "r"(x), "r"(y), "r"(o.z) : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  if (lane == 0) {
+    if (o.z < 0) tma_store_2d(o.map, box, x, y);
+    else tma_store_3d(o.map, box, x, y, o.z);
+    bulk_commit();
   }
   ++o.n;
 }
 // Before the CTA's shared memory goes away.
-__device__ __forceinline__ void drain_boxes() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void drain_boxes() { bulk_wait_read<0>(); }
 
 // 32 accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
 // bf16 box; an fp32 box holds 32 columns). Columns past N and rows past M are computed from nothing and clipped by the store.
@@ -130,6 +127,7 @@ template <bool OUT_F32, bool SPLIT>
 __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane,
                                                  int unit, int split, bool zero) {
   constexpr int PARTS = OUT_F32 ? 1 : 2;      // 32-column pieces per box
+  if (row0 + q * 32 >= p.M) return;           // none of this warp's rows exist: nothing to stage, store or count
   const int row = row0 + q * 32 + lane;
   const bool row_ok = row < p.M;
   RowStats st;
@@ -154,7 +152,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
         for (int j = 0; j < 32; ++j) f[j] = zero ? 0.f : __uint_as_float(v[k][j]);
         epilogue_row32<OUT_F32>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
       }
-      store_box(out, box, col0, row0 + q * 32, p.M, lane);
+      store_box(out, box, col0, row0 + q * 32, lane);
     }
     finish();
     return;
@@ -203,7 +201,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
       }
       epilogue_row32<OUT_F32>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
     }
-    store_box(out, box, col0, row0 + q * 32, p.M, lane);
+    store_box(out, box, col0, row0 + q * 32, lane);
   }
   finish();
   if (lane == 0) p.counters[unit * 4 + q] = 0;

@@ -730,3 +730,43 @@ def test_split_workspaces_are_per_stream_and_bounded(ops):
     torch.cuda.synchronize()
     assert rel_err(out, ref) < 4e-3
     ops.check_status()
+
+
+def _ints(*shape):
+    return torch.randint(-1, 2, shape, device="cuda").to(torch.bfloat16)
+
+
+# last row tiles of which only one to three of the four 32-row quarters exist, many tiles per worker and reductions so short that the
+# next accumulator is ready while the last box of a tile is still being stored; operands of -1, 0, 1: every sum is exact
+@pytest.mark.parametrize("rows", [1, 33, 65, 129, 193])
+@pytest.mark.parametrize("two_cta", [False, True])
+@pytest.mark.parametrize("f32", [False, True])
+def test_gemm_ragged_last_tile_is_exact(ops, rows, two_cta, f32):
+    M, N = 256 * 37 + rows, 2056 if f32 else 2120
+    dt = torch.float32 if f32 else torch.bfloat16
+    for K in (64, 200):
+        a, b = _ints(M, K), _ints(N, K)
+        want = (a.float() @ b.float().t()).to(dt)
+        for _ in range(4):
+            out = torch.full((M, N), float("nan"), dtype=dt, device="cuda")
+            ops.gemm(a, False, b, False, out, M, N, K, two_cta=two_cta)
+            assert torch.equal(out, want)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("M,N", [(136, 264), (72, 136), (648, 520)])
+def test_grouped_weight_gradient_ragged_rows_is_exact(ops, M, N):
+    """Output matrices with partial last row tiles, slabs of a few k-blocks and experts without rows."""
+    T, E, k = 900, 48, 2
+    topi = torch.randint(0, E // 2, (T, k), device="cuda") * 2
+    sl = ops.expert_slabs(topi, E)
+    dy, x = _ints(T, M), _ints(T, N)
+    dys, xs = ops.gather_rows(dy, sl), ops.gather_rows(x, sl)
+    flat = topi.reshape(-1)
+    for _ in range(4):
+        dw = torch.full((E, M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.grouped_wgrad(dys, xs, (dw[0], M * N), sl)
+        for e in range(E):
+            tok = (flat == e).nonzero().reshape(-1) // k
+            assert torch.equal(dw[e], (dy[tok].float().t() @ x[tok].float()).bfloat16()), e
+    ops.check_status()

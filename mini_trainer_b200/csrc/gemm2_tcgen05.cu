@@ -282,7 +282,29 @@ done:
   }
 }
 
-static int g_pairs[2] = {-1, -1};   // clusters of two that can be co-resident (0: unsupported), plain / gather variant
+// Clusters of two that can be co-resident (0: unsupported), plain / gather variant. All instances of a variant have the same
+// threads and shared memory, so one of them is asked, once.
+template <bool GATHER>
+static int co_resident_pairs() {
+  static int pairs = -1;
+  if (pairs < 0) {
+    auto kern = gemm2_kernel<false, false, false, GATHER>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2, 1, 1);
+    cfg.blockDim = dim3(GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    pairs = n;
+  }
+  return pairs;
+}
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
@@ -294,21 +316,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -4;
     configured = true;
   }
-  int& pairs = g_pairs[GATHER ? 1 : 0];
-  if (pairs < 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = SMEM;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-    pairs = n;
-  }
+  const int pairs = co_resident_pairs<GATHER>();
   if (pairs <= 0) return -6;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   // The arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest.
@@ -345,7 +353,9 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
 extern "C" {
 
 // Same contract as mtb200_gemm_bf16, computed by CTA pairs (256 x 256 tiles). Returns -6 when
-// clusters of two cannot be scheduled on this device; callers then use the one-CTA kernel.
+// clusters of two cannot be scheduled on this device (mtb200_gemm2_pairs() is 0); callers then use the one-CTA kernel.
+int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
+
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
                       float alpha, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {

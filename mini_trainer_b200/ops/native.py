@@ -48,6 +48,7 @@ P, I, L, F = c_void_p, c_int, c_longlong, c_float
 class _Sig:
     mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
     mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
+    mtb200_gemm2_pairs = []
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
     mtb200_norm_bwd_blocks = [I, I]
     mtb200_rmsnorm_bwd = [P, P, P, P, P, P, P, P, I, I, P, P]
@@ -136,6 +137,7 @@ class NativeOps:
         self._scratch = {}
         self._gemm_ws = {}   # stream handle -> split-K workspace
         self._attn_plan_cache = {}
+        self._pairs = None
 
     # -- plumbing ---------------------------------------------------------------------
     def _st(self):
@@ -205,6 +207,12 @@ class NativeOps:
             raise RuntimeError(f"{what} (status code {code})")
 
     # -- GEMM -------------------------------------------------------------------------
+    def cta_pairs(self) -> int:
+        """CTA pairs the device can run at once; 0 where clusters of two cannot be scheduled, and everything runs on single CTAs."""
+        if self._pairs is None:
+            self._pairs = self._fn["mtb200_gemm2_pairs"]()
+        return self._pairs
+
     def _split_workspace(self, stream):
         """Split-K workspace of a stream: arrival counters (zero between launches) and fp32 partials. GEMMs of one stream run
         one after the other, those of different streams may overlap, so each stream has its own (the last eight streams do;
@@ -224,12 +232,15 @@ class NativeOps:
     def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
         """out[M,N] = alpha*A*B (+bias) (+residual). ``a_mn``/``b_mn``: operand stored [K, rows].
         ``stats`` [M, ceil(N / 256), 2] fp32 receives the softmax statistics of the (bf16) output rows per 256 columns.
-        ``two_cta``: force (True) or forbid (False) the cta_group::2 kernel; default by problem size."""
+        ``two_cta``: force (True) or forbid (False) the cta_group::2 kernel; default by problem size. Without CTA pairs on the
+        device the one-CTA kernel runs in any case."""
         out_f32 = out.dtype == torch.float32
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
         assert residual is None or residual.dtype == out.dtype
         if two_cta is None:
             two_cta = (self.use_gemm2 or 2.0 * M * N * K <= self.pair_max_flops) and (-(-M // 256)) * (-(-N // 256)) >= 64
+        if two_cta and self.cta_pairs() <= 0:
+            two_cta = False
         st = self._st()
         ws = self._split_workspace(st)
         self._call("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),

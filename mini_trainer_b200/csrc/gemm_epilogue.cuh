@@ -70,7 +70,7 @@ __device__ __forceinline__ void drain_boxes() { bulk_wait_read<0>(); }
 
 // 32 accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
 // bf16 box; an fp32 box holds 32 columns). Columns past N and rows past M are computed from nothing and clipped by the store.
-template <bool OUT_F32>
+template <bool OUT_F32, bool STATS>
 __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
                                                RowStats& st) {
 #pragma unroll
@@ -109,7 +109,7 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
       o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
       o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
       *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
-      if (p.stats != nullptr && col0 + j < p.N) {   // of the values as stored
+      if (STATS && col0 + j < p.N) {   // of the values as stored
         const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y), r2 = unpack_bf16(o.z), r3 = unpack_bf16(o.w);
         const float mx = fmaxf(fmax3(fmaxf(r0.x, r0.y), r1.x, r1.y), fmax3(fmaxf(r2.x, r2.y), r3.x, r3.y));
         if (mx > st.m) { st.s *= __expf(st.m - mx); st.m = mx; }
@@ -122,8 +122,10 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
 
 // One warp's part of a work item: quarter `q` of the 128-row unit that starts at row `row0`, columns [tn0, tn0 + 256).
 // `taddr`: tensor-memory address of the quarter. `unit`: index of the 128-row unit among all tiles' units. `zero`: the item
-// had nothing to multiply, the accumulator holds an older tile. SPLIT = false leaves the split-K part out.
-template <bool OUT_F32, bool SPLIT>
+// had nothing to multiply, the accumulator holds an older tile. SPLIT = false leaves the split-K part out, STATS = false the
+// statistics: a worker walks this code once per tile, and with the statistics as a run-time branch in every product the
+// instructions to fetch made a launch of one wave 2 us longer (384 x 2048 x 2048: 18.6 and 16.5 us, 4736 x 1024 x 512: 11.3 and 10.4).
+template <bool OUT_F32, bool SPLIT, bool STATS>
 __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane,
                                                  int unit, int split, bool zero) {
   constexpr int PARTS = OUT_F32 ? 1 : 2;      // 32-column pieces per box
@@ -132,7 +134,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
   const bool row_ok = row < p.M;
   RowStats st;
   auto finish = [&]() {
-    if (!OUT_F32 && p.stats != nullptr && row_ok && tn0 < p.N)
+    if (STATS && row_ok && tn0 < p.N)
       p.stats[static_cast<long long>(row) * ((p.N + 255) / 256) + tn0 / 256] = make_float2(st.m, st.s);
   };
   if (!SPLIT || p.splits == 1) {
@@ -150,7 +152,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
         float f[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) f[j] = zero ? 0.f : __uint_as_float(v[k][j]);
-        epilogue_row32<OUT_F32>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
+        epilogue_row32<OUT_F32, STATS>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
       }
       store_box(out, box, col0, row0 + q * 32, lane);
     }
@@ -199,7 +201,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
           }
         }
       }
-      epilogue_row32<OUT_F32>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
+      epilogue_row32<OUT_F32, STATS>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
     }
     store_box(out, box, col0, row0 + q * 32, lane);
   }

@@ -770,3 +770,33 @@ def test_grouped_weight_gradient_ragged_rows_is_exact(ops, M, N):
             tok = (flat == e).nonzero().reshape(-1) // k
             assert torch.equal(dw[e], (dy[tok].float().t() @ x[tok].float()).bfloat16()), e
     ops.check_status()
+
+
+# every operand layout, both kernels, whole tiles and split reductions, a last column tile that is not full
+@pytest.mark.parametrize("M,N,K", [(300, 776, 320), (136, 264, 4096), (1031, 2120, 128)])
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn", "tt"])
+@pytest.mark.parametrize("two_cta", [False, True])
+def test_gemm_row_statistics(ops, M, N, K, layout, two_cta):
+    """Maximum and sum of exponentials per row and 256 columns, against the same of the output as it was stored."""
+    if layout[0] == "t":
+        M = -(-M // 8) * 8
+    torch.manual_seed(M + N)
+    a, b = bf(M, K), bf(N, K, scale=4 * K ** -0.5)
+    at, bt = (a.t().contiguous() if layout[0] == "t" else a), (b if layout[1] == "t" else b.t().contiguous())
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    tiles = -(-N // 256)
+    stats = torch.full((M, tiles, 2), float("nan"), device="cuda")
+    ops.gemm(at, layout[0] == "t", bt, layout[1] == "n", out, M, N, K, two_cta=two_cta, stats=stats)
+    ops.check_status()
+    ref = a.float() @ b.float().t()
+    assert rel_err(out, ref) < 6e-3
+    x = torch.full((M, tiles * 256), float("-inf"), device="cuda")
+    x[:, :N] = out.float()
+    x = x.view(M, tiles, 256)
+    mx = x.max(-1).values
+    assert torch.equal(stats[..., 0], mx)
+    # fp32 sums of up to 256 exponentials, each within a few ulp
+    assert rel_err(stats[..., 1], (x.double() - mx.double()[..., None]).exp().sum(-1)) < 1e-5
+    plain = torch.empty_like(out)
+    ops.gemm(at, layout[0] == "t", bt, layout[1] == "n", plain, M, N, K, two_cta=two_cta)
+    assert torch.equal(plain, out)

@@ -15,8 +15,7 @@
 // threads (two threads per row with their maxima exchanged through shared memory measured 1.92 ms below). P is handed over in
 // two halves of 64 keys, so the first half's products run under the second half's exponentials. 1 x 16384 tokens, 32/8 heads, D = 128: 1.65 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64:
 // 64 us (one tile per CTA, two threads per row: 1.94 ms and 94 us).
-// One long sequence at D = 64, where the products are short and the exponentials bound both forms, is the exception: 1.65 -> 1.81 ms
-// for 16384 tokens.
+// Launches with few pairs, and some long ones at D = 64, are faster in that other form: attention_fwd_one.cu.
 //
 // CTAs are persistent (one per SM): barriers and tensor memory are set up once, K and V of the next item are prefetched
 // under the current one's tail, and the epilogue of an item runs under the next item's first product. Items come most work
@@ -29,7 +28,7 @@
 // Masked scores are -inf. The exponentials that run on the special-function unit turn them into exact zeros;
 // the quarter that runs on the FMA pipe (ex2_fma2) clamps its argument at -126 and returns about 1e-38 instead, so
 // on the diagonal tile one masked key in four adds a term of that size to a row sum that is at least 1 (the row's
-// maximum contributes exp2(0)) and a bf16 zero to P: below fp32 resolution, no effect on out or lse.
+// maximum contributes exp2(0)) and to P: 38 orders of magnitude below either, no effect on out or lse.
 //
 // Outputs: out [T, Hq*D] bf16 and lse [Hq, T] fp32 (natural log, scaled scores), as needed by
 // the backward. Sequence boundaries come from a host-built work table (seq_start, seq_len, q0),
@@ -47,6 +46,7 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
                       uint32_t box_inner, uint32_t box_outer);
 
 constexpr int ATT_B = 128;         // query tile and key tile edge
+constexpr int POLY = 4;            // every POLY-th exponential pair runs on the FMA pipe (2 and 8 measured the same within the spread)
 constexpr int ATT_THREADS = 384;   // three warpgroups: TMA / MMA, softmax of A, softmax of B
 // Registers per thread after the split; over the three warpgroups they add up to at most the 3 x 168 of the launch.
 // A softmax thread holds the 128 scores of its row.
@@ -108,7 +108,7 @@ __device__ __forceinline__ bool att_work(const AttFwdParams& p, int round, AttWo
   return true;
 }
 
-template <int D, int POLY>   // every POLY-th exponential pair runs on the FMA pipe instead of the special-function unit
+template <int D>
 __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, AttFwdParams p) {
   using L = AttFwdSmem<D>;
   constexpr int KB = D / 64;  // 64-element (128 B) column blocks of a D-wide row
@@ -372,11 +372,11 @@ done:
   }
 }
 
-template <int D, int POLY>
+template <int D>
 static int launch_fwd(const CUtensorMap& tm, const AttFwdParams& p, cudaStream_t st) {
   static bool configured = false;
   static int sms = 0;
-  auto kern = attn_fwd_kernel<D, POLY>;
+  auto kern = attn_fwd_kernel<D>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttFwdSmem<D>::TOTAL) != cudaSuccess) return -4;
     int dev = 0;
@@ -403,6 +403,5 @@ extern "C" int mtb200_attn_fwd(const void* qkv, long long ld, void* out, long lo
   const int rc = make_tmap_2d_bf16(&tm, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
   if (rc) return rc;
   AttFwdParams p{reinterpret_cast<__nv_bfloat16*>(out), ldo, lse, plan, n_items, T, Hq, Hkv, row_pairs, scale, status};
-  // one exponential pair in four on the FMA pipe; one in two and one in eight measured the same within the spread
-  return D == 128 ? launch_fwd<128, 4>(tm, p, st) : launch_fwd<64, 4>(tm, p, st);
+  return D == 128 ? launch_fwd<128>(tm, p, st) : launch_fwd<64>(tm, p, st);
 }

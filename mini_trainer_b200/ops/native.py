@@ -17,6 +17,7 @@ import torch
 
 from .. import build as _build
 from ..utils import nvtx
+from . import attention_plan
 
 _LIB = None
 _raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else \
@@ -81,6 +82,7 @@ class _Sig:
     mtb200_moe_glu_bwd = [P, P, P, P, P, I, I, I, I, P, P, P]
     mtb200_moe_combine = [P, P, P, P, P, F, I, I, I, P, P]
     mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
+    mtb200_attn_fwd_one = [P, L, P, L, P, P, I, I, I, I, I, F, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
     mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, P, L, F, P, P]
 
@@ -138,6 +140,7 @@ class NativeOps:
         self._gemm_ws = {}   # stream handle -> split-K workspace
         self._attn_plan_cache = {}
         self._pairs = None
+        self.sms = torch.cuda.get_device_properties(self._index).multi_processor_count
 
     # -- plumbing ---------------------------------------------------------------------
     def _st(self):
@@ -382,15 +385,25 @@ class NativeOps:
         return dqkv
 
     # -- attention --------------------------------------------------------------------
-    def _attn_plan(self, cu_host, block, most_work_last_block: bool):
-        """Work table for the attention kernels: one row (seq_start, seq_len, block_start) per
-        ``block`` rows of every sequence, most work first (forward: late query blocks see the most
-        keys; backward: early key blocks are seen by the most queries). Built once per minibatch
-        and reused by every layer."""
-        key = (id(cu_host), block, most_work_last_block)
+    def _per_batch(self, cu_host, what: tuple, make):
+        """``make()``, computed once per minibatch (its list of sequence starts) and reused by every layer."""
+        key = (id(cu_host),) + what
         hit = self._attn_plan_cache.get(key)
         if hit is not None and hit[0] is cu_host:
             return hit[1]
+        value = make()
+        if len(self._attn_plan_cache) > 16:
+            self._attn_plan_cache.clear()
+        self._attn_plan_cache[key] = (cu_host, value)
+        return value
+
+    def _attn_plan(self, cu_host, block, most_work_last_block: bool):
+        """Work table for the attention kernels: one row (seq_start, seq_len, block_start) per
+        ``block`` rows of every sequence, most work first (forward: late query blocks see the most
+        keys; backward: early key blocks are seen by the most queries)."""
+        return self._per_batch(cu_host, (block, most_work_last_block), lambda: self._attn_table(cu_host, block, most_work_last_block))
+
+    def _attn_table(self, cu_host, block, most_work_last_block: bool):
         items = []
         for a, b in zip(cu_host[:-1], cu_host[1:]):
             n = b - a
@@ -398,11 +411,7 @@ class NativeOps:
                 work = s0 if most_work_last_block else n - s0
                 items.append((work, a, n, s0))
         items.sort(key=lambda it: -it[0])
-        table = torch.tensor([it[1:] for it in items], dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
-        if len(self._attn_plan_cache) > 8:
-            self._attn_plan_cache.clear()
-        self._attn_plan_cache[key] = (cu_host, table)
-        return table
+        return torch.tensor([it[1:] for it in items], dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
 
     def attention(self, qkv, cu_seqlens, cu_host, max_seqlen, hq, hkv, d, scale=None):
         T = qkv.shape[0]
@@ -411,6 +420,12 @@ class NativeOps:
             return self._fa_fwd(qkv, cu_seqlens, max_seqlen, hq, hkv, d, scale)
         out = torch.empty(T, hq * d, dtype=qkv.dtype, device=self.device)
         lse = torch.empty(hq, T, dtype=torch.float32, device=self.device)
+        if not self._per_batch(cu_host, ("pairs", hq, hkv, d), lambda: attention_plan.forward_in_pairs(
+                attention_plan.blocks_per_sequence(cu_host), hq, hkv, d, self.sms)):
+            plan = self._attn_plan(cu_host, 128, True)
+            self._call("mtb200_attn_fwd_one", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), lse.data_ptr(),
+                       plan.data_ptr(), plan.shape[0], T, hq, hkv, d, scale, self.status.data_ptr(), self._st(), tag="mtb200_attn_fwd")
+            return out, lse
         row_pairs = (hq // hkv) % 2   # a work item is two heads of a kv head, or two 128-row blocks of a head where heads do not pair up
         plan = self._attn_plan(cu_host, 256 if row_pairs else 128, True)
         self._call("mtb200_attn_fwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), lse.data_ptr(),

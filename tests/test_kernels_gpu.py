@@ -800,3 +800,25 @@ def test_gemm_row_statistics(ops, M, N, K, layout, two_cta):
     plain = torch.empty_like(out)
     ops.gemm(at, layout[0] == "t", bt, layout[1] == "n", plain, M, N, K, two_cta=two_cta)
     assert torch.equal(plain, out)
+
+
+@pytest.mark.parametrize("pairs", [True, False])
+@pytest.mark.parametrize("D,hq,hkv,lens", ATTN_CASES + [(64, 3, 1, [257, 1, 128, 384]), (64, 14, 2, [2049, 63])])
+def test_attention_forward_both_forms(ops, D, hq, hkv, lens, pairs, monkeypatch):
+    """Every batch through pairs of query tiles and through one tile per CTA, whichever the sizes would choose."""
+    from mini_trainer_b200.ops import attention_plan
+    monkeypatch.setattr(attention_plan, "forward_in_pairs", lambda *a: pairs)
+    torch.manual_seed(sum(lens) + pairs)
+    T = sum(lens)
+    qkv = bf(T, (hq + 2 * hkv) * D)
+    qkv[: T // 2] *= 4    # maxima that move by more than the rescale threshold
+    cu_host, cu = _cu(lens)
+    n0 = ops.launches
+    out, lse = ops.attention(qkv, cu, cu_host, max(lens), hq, hkv, D)
+    assert ops.launches == n0 + 1
+    ro, rl = REF.attention(qkv.float(), cu, cu_host, max(lens), hq, hkv, D)
+    ops.check_status()
+    assert rel_err(lse, rl) < 2e-3 and (lse - rl).abs().max() < 3e-2
+    assert rel_err(out, ro) < 1e-2 and max_err(out, ro) < 0.1
+    out2, lse2 = ops.attention(qkv, cu, cu_host, max(lens), hq, hkv, D)
+    assert torch.equal(out, out2) and torch.equal(lse, lse2)

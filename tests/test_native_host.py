@@ -36,3 +36,48 @@ def test_gemm_runs_on_single_ctas_where_pairs_cannot_be_scheduled(pairs):
     assert gemm(ops, 4096, 2048, 64) == want
     assert gemm(ops, 512, 512, 64, two_cta=True) == want
     assert gemm(ops, 512, 512, 64, two_cta=False) == "mtb200_gemm_bf16"
+
+
+# (lengths, query heads, kv heads, head_dim, pairs): launches with fewer pairs than SMs, and batches of many units; each of these is
+# at least 5 % faster in its form
+@pytest.mark.parametrize("lens,hq,hkv,d,pairs", [([2048], 16, 4, 64, False), ([16384], 2, 1, 128, False), ([8192], 4, 4, 64, False), ([64], 32, 8, 64, False),
+                                                 ([4000, 5200, 3100, 5900], 1, 1, 64, False), ([1024], 14, 2, 128, False),
+                                                 ([300] * 41, 16, 4, 64, True), ([16384], 32, 8, 128, True), ([128] * 100, 32, 8, 128, True),
+                                                 ([100] * 300, 28, 4, 64, True), ([2048], 32, 8, 128, True), ([5000] * 4, 9, 3, 128, True)])
+def test_attention_forward_form(lens, hq, hkv, d, pairs):
+    from mini_trainer_b200.ops import attention_plan as A
+    blocks = [-(-n // 128) for n in lens]
+    assert A.forward_in_pairs(blocks, hq, hkv, d, 148) == pairs
+    # both forms do the same tiles: the choice is asked for every batch, so it has to accept any of them
+    assert A.forward_in_pairs([], hq, hkv, d, 148)
+
+
+def test_attention_finish_time_is_a_lower_bound():
+    from mini_trainer_b200.ops.attention_plan import finish_time
+    import heapq
+    import random
+    rng = random.Random(0)
+    for _ in range(200):
+        units = [(rng.uniform(1, 50), rng.randint(1, 60)) for _ in range(rng.randint(1, 12))]
+        load = [0.0] * 37
+        for c, n in sorted(units, reverse=True):
+            for _ in range(n):
+                heapq.heappush(load, heapq.heappop(load) + c)
+        t = finish_time(units, 37)
+        assert t <= max(load) * (1 + 1e-9) and max(load) <= 2 * t   # a list schedule ends within mean + longest
+
+
+def test_attention_forward_launches_the_chosen_form():
+    ops = make_ops()
+    ops.sms, ops.attention_impl = 148, "native"
+    ops._attn_table = lambda cu, block, last: torch.zeros(block, 3, dtype=torch.int32)
+    for lens, hq, hkv, name, block in (([2048], 16, 4, "mtb200_attn_fwd_one", 128), ([300] * 41, 16, 4, "mtb200_attn_fwd", 128),
+                                       ([300] * 41, 27, 3, "mtb200_attn_fwd", 256)):
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        qkv = torch.empty(cu[-1], (hq + 2 * hkv) * 64, dtype=torch.bfloat16)
+        for _ in range(2):   # the second layer finds the choice and the table
+            out, lse = ops.attention(qkv, None, cu, max(lens), hq, hkv, 64)
+            assert ops.calls[-1][0] == name and ops.calls[-1][1][6] == block
+            assert out.shape == (cu[-1], hq * 64) and lse.shape == (hq, cu[-1])

@@ -540,13 +540,16 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
 
 // plan: key-block work table [n_items, 3] = (seq_start, seq_len, k0), most work first.
 // dq_acc: zero-initialised fp32 [T, Hq*D] scratch; delta: fp32 [Hq, T] scratch.
-// ws: optional workspace of ws_bytes, as the split-K GEMM's (its first SPLIT_COUNTER_BYTES are zero before and after a launch).
+// splits: CTAs that share the query heads of a key block; more than one needs ws, a workspace of ws_bytes as the split-K GEMM's (its first
+// SPLIT_COUNTER_BYTES are zero before and after a launch).
 extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, long long ldo, const void* dout, long long lddo,
                                void* dqkv, long long ldq, const float* lse, float* delta, float* dq_acc, const int* plan,
-                               int n_items, int T, int Hq, int Hkv, int D, float* ws, long long ws_bytes, float scale, int* status, cudaStream_t st) {
+                               int n_items, int T, int Hq, int Hkv, int D, int splits, float* ws, long long ws_bytes, float scale, int* status, cudaStream_t st) {
   using namespace mtb;
   if (n_items <= 0 || T <= 0) return 0;
-  if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8 || lddo % 8 || ldq % 8) return -10;
+  if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8 || lddo % 8 || ldq % 8 || splits < 1 || splits > Hq / Hkv) return -10;
+  const long long units = static_cast<long long>(n_items) * Hkv;
+  if (splits > 1 && (ws == nullptr || units * 8 * 4 > SPLIT_COUNTER_BYTES || splits * units * 2 * AB_B * D * 4 > ws_bytes - SPLIT_COUNTER_BYTES)) return -11;
   CUtensorMap tq, tdo, tdq;
   int rc = make_tmap_2d_bf16(&tq, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
   if (rc) return rc;
@@ -557,16 +560,6 @@ extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, l
   const long long delta_threads = static_cast<long long>(T) * Hq * (D / 8);
   attn_delta_kernel<<<static_cast<int>((delta_threads + 255) / 256), 256, 0, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(out), ldo, reinterpret_cast<const __nv_bfloat16*>(dout), lddo, delta, T, Hq, D);
-  // A key block of a kv head is one CTA's work; with few kv heads and a short batch that leaves SMs idle (2 kv heads, 6000
-  // tokens: 94 CTAs of very different length on 148 SMs), so the query heads of a block are divided until there are about two
-  // CTAs per SM (5987 tokens, 12/2 heads: 437 -> 137 us, 7001 tokens, 24/2 heads: 1141 -> 357 us, both with the reordered loop). More gain nothing: every CTA loads K and V again and adds a partial.
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long units = static_cast<long long>(n_items) * Hkv;
-  int splits = 1;
-  if (ws != nullptr && units * 8 * 4 <= SPLIT_COUNTER_BYTES)
-    while (splits < Hq / Hkv && units * splits < 2 * sms && (splits + 1) * units * 2 * AB_B * D * 4 <= ws_bytes - SPLIT_COUNTER_BYTES) ++splits;
   AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, splits,
                  ws == nullptr ? nullptr : ws + SPLIT_COUNTER_BYTES / 4, reinterpret_cast<unsigned*>(ws), scale, status};
   rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, p, n_items, st);

@@ -14,6 +14,10 @@ BLOCK = 128   # rows of a query block, keys of a key block
 _ONE = {64: (1.87, 4.1, 0.84), 128: (1.88, 5.55, 0.94)}
 _TWO = {64: (3.98, 2.81, 1.65, 3.4, 1.75, 1.89, 1.61), 128: (3.32, 5.27, 1.72, 4.83, 1.66, 3.47, 1.66)}
 
+# Backward, in iterations (one query block of one head, 1.5 us at head_dim 64 and 2.7 at 128): a CTA's start and end (loads of K and V,
+# stores of dK and dV), and what a partial sum of dK and dV adds to it.
+_BWD_CTA, _BWD_PARTIAL = 5.0, 2.0
+
 
 def finish_time(units: list, workers: int) -> float:
     """Lower bound, and in practice about the value, of the finish time of ``units`` [(time, count)] on ``workers``: the longest
@@ -59,3 +63,24 @@ def forward_in_pairs(blocks: list, hq: int, hkv: int, d: int, sms: int) -> bool:
         units = [(ra + rb * n, at[n] * hq) for n in range(2, longest + 1, 2)]
         units += [(la + lb * n, (at[n] - at[n + 1]) * hq) for n in range(1, longest + 1, 2) if at[n] > at[n + 1]]
     return launch + finish_time(units, sms) <= one
+
+
+def backward_splits(blocks: list, hq: int, hkv: int, sms: int, most: int) -> int:
+    """Backward: CTAs (at most ``most``) that share the query heads of a key block. A key block of a kv head is one CTA's work; with few
+    kv heads and a short batch that leaves SMs idle and the longest CTA decides (5987 tokens, 12/2 heads: 437 -> 137 us with
+    the heads divided). But every CTA loads K and V again and adds a partial sum, so short samples are not divided
+    (16 of 128 tokens, 32/8 heads of 128: 47 us whole, 86 when divided until there were two CTAs per SM)."""
+    if not blocks:
+        return 1
+    at = _with_at_least(blocks)
+    longest, group, units = len(at) - 2, hq // hkv, sum(blocks) * hkv
+    best, splits = float("inf"), 1
+    for s in range(1, min(group, most) + 1):
+        if s > 1 and units * (s - 1) >= 2 * sms:   # two CTAs per SM already
+            break
+        cta = _BWD_CTA + (_BWD_PARTIAL if s > 1 else 0.0)
+        t = finish_time([(cta + group / s * n, at[n] * hkv * s) for n in range(1, longest + 1)], sms)
+        t = max(t, cta + -(-group // s) * longest)
+        if t < best:
+            best, splits = t, s
+    return splits

@@ -84,7 +84,7 @@ class _Sig:
     mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
     mtb200_attn_fwd_one = [P, L, P, L, P, P, I, I, I, I, I, F, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
-    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, P, L, F, P, P]
+    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, L, F, P, P]
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
@@ -442,10 +442,16 @@ class NativeOps:
         delta = torch.empty(hq, T, dtype=torch.float32, device=self.device)
         dq_acc = torch.zeros(T, hq * d, dtype=torch.float32, device=self.device)
         st = self._st()
-        ws = self._split_workspace(st)
+        units = plan.shape[0] * hkv   # per unit: 8 counters and, for every CTA that shares it, dK and dV of 128 rows in fp32
+        most = 1 if units * 8 > _SPLIT_COUNTERS else min(hq // hkv, _SPLIT_FLOATS // (units * 2 * 128 * d))
+        splits = 1 if most <= 1 else self._per_batch(cu_host, ("splits", hq, hkv, d), lambda: attention_plan.backward_splits(
+            attention_plan.blocks_per_sequence(cu_host), hq, hkv, self.sms, most))
+        ws = self._split_workspace(st) if splits > 1 else None
+        if ws is None:
+            splits = 1
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
-                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), scale,
+                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits, _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), scale,
                    self.status.data_ptr(), st, n=3)
         return dqkv
 

@@ -81,3 +81,36 @@ def test_attention_forward_launches_the_chosen_form():
             out, lse = ops.attention(qkv, None, cu, max(lens), hq, hkv, 64)
             assert ops.calls[-1][0] == name and ops.calls[-1][1][6] == block
             assert out.shape == (cu[-1], hq * 64) and lse.shape == (hq, cu[-1])
+
+
+# (lengths, query heads, kv heads, range of CTAs per key block): nothing to divide, short samples, short batches, full ones
+@pytest.mark.parametrize("lens,hq,hkv,lo,hi", [([2048], 8, 8, 1, 1), ([128] * 16, 32, 8, 1, 1), ([110] * 100, 4, 1, 1, 1), ([16384], 32, 8, 1, 1),
+                                               ([1024], 12, 2, 6, 6), ([2048], 14, 2, 7, 7), ([8192], 24, 2, 2, 3), ([4096], 16, 4, 2, 2),
+                                               ([900, 1400, 700, 1100, 600, 1300, 1000, 800], 12, 2, 2, 3)])
+def test_attention_backward_splits(lens, hq, hkv, lo, hi):
+    from mini_trainer_b200.ops import attention_plan as A
+    blocks = [-(-n // 128) for n in lens]
+    assert lo <= A.backward_splits(blocks, hq, hkv, 148, 64) <= hi
+    assert A.backward_splits(blocks, hq, hkv, 148, 1) == 1 and A.backward_splits([], hq, hkv, 148, 64) == 1
+    for most in (2, 3):
+        assert A.backward_splits(blocks, hq, hkv, 148, most) <= most
+
+
+def test_attention_backward_divides_only_what_the_workspace_holds():
+    ops = make_ops()
+    ops.sms, ops.attention_impl = 148, "native"
+    ops._attn_table = lambda cu, block, last: torch.zeros(sum(-(-(b - a) // block) for a, b in zip(cu[:-1], cu[1:])), 3, dtype=torch.int32)
+    ws = torch.zeros(8)
+    for lens, have, want in (([1024], True, True), ([1024], False, False), ([110] * 100, True, False), ([2000] * 80, True, False)):
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        ops._split_workspace = lambda st: ws if have else None
+        hq, hkv, d, T = 8, 2, 64, cu[-1]
+        qkv, o = torch.empty(T, 12 * d, dtype=torch.bfloat16), torch.empty(T, hq * d, dtype=torch.bfloat16)
+        ops.attention_bwd(o, qkv, o, torch.empty(hq, T), None, cu, max(lens), hq, hkv, d)
+        args = ops.calls[-1][1]
+        splits, units = args[17], args[12] * hkv
+        assert (splits > 1) == want and (args[18] is not None) == want
+        if want:
+            assert units * 8 <= 4096 and splits * units * 2 * 128 * d <= 32 << 20

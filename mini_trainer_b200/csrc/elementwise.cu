@@ -57,10 +57,12 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // LayerNorm  y = ((x - mean) * rstd) * w + b ; statistics in two passes over the row in registers (the mean first, then the
 //            centred sum of squares), mean and rstd saved
 // A group of LANES threads (one to eight warps) holds a row in registers, VPT 8-wide vectors per thread, and a 256-thread block
-// works on 256 / LANES consecutive rows at a time. Bound by reading x and writing y. Blocks are persistent and rows arrive in
-// shared memory by bulk copies NORM_STAGES row sets ahead: the bytes in flight cost no registers and do not stop for a
-// row's barriers and stores, which is what held the register form back (RMSNorm, 16384 x 4096:
-// 58 -> 53 us; 7001 x 3072: 26 -> 22 us).
+// works on 256 / LANES consecutive rows at a time. Bound by reading x and writing y.
+// BULK: blocks are persistent and rows arrive in shared memory by bulk copies NORM_STAGES row sets ahead: the bytes in flight cost no
+// registers and do not stop for a row's barriers and stores, which is what held the register form back (RMSNorm, 16384 x 4096:
+// 53 -> 47 us; 6000 x 3072: 16 -> 14 us; LayerNorm, 16384 x 3072: 51 -> 43 us). Otherwise (RMSNorm) a block is one row set, loaded straight
+// into registers: with a set or two per block nothing runs ahead, and the stages only cost residency (6000 x 1024: 8.3 us by bulk
+// copies, 6.9 straight; 500 x 12288: 10.4 and 8.3).
 constexpr int NORM_STAGES = 3;
 
 __device__ __forceinline__ float group_sum(float v, float (&red)[EW_THREADS / 32], int lanes, int sub) {
@@ -75,7 +77,7 @@ __device__ __forceinline__ float group_sum(float v, float (&red)[EW_THREADS / 32
   return v;
 }
 
-template <bool LN, int VPT>
+template <bool LN, int VPT, bool BULK>
 __global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                              const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                              float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, int T,
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat1
   __shared__ uint64_t full[NORM_STAGES];
   __shared__ float red[2][2][EW_THREADS / 32];   // [parity of the row set][mean, square]
   __shared__ int abort_word;
+  constexpr bool HOLD = BULK;   // weight and bias: once per persistent block, or behind the row's own loads
   volatile int* abort_flag = &abort_word;
   const int rows_per_block = EW_THREADS / lanes;
   const int sub = threadIdx.x / lanes, l = threadIdx.x % lanes;
@@ -96,28 +99,30 @@ __global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat1
     mbar_arrive_expect_tx(&full[s], bytes);
     bulk_load(norm_smem + s * set_bytes, x + first * H, bytes, &full[s]);
   };
-  if (threadIdx.x == 0) {
+  if (BULK && threadIdx.x == 0) {
     for (int s = 0; s < NORM_STAGES; ++s) mbar_init(&full[s], 1);
     abort_word = 0;
     fence_mbar_init();
     for (int s = 0; s < NORM_STAGES; ++s) request(first0 + s * step, s);
   }
-  bf16x8 wv[VPT], bv[LN ? VPT : 1];
+  bf16x8 wv[HOLD ? VPT : 1], bv[LN && HOLD ? VPT : 1];
+  if constexpr (HOLD) {
 #pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int c = (l + k * lanes) * 8;
-    wv[k].u = make_uint4(0u, 0u, 0u, 0u);
-    if (LN) bv[k].u = wv[k].u;
-    if (c < H) { wv[k].load(w + c); if (LN) bv[k].load(b + c); }
+    for (int k = 0; k < VPT; ++k) {
+      const int c = (l + k * lanes) * 8;
+      wv[k].u = make_uint4(0u, 0u, 0u, 0u);
+      if constexpr (LN) bv[k].u = wv[k].u;
+      if (c < H) { wv[k].load(w + c); if constexpr (LN) bv[k].load(b + c); }
+    }
   }
-  __syncthreads();
+  if (BULK) __syncthreads();
   int it = 0;
   for (long long first = first0; first < T; first += step, ++it) {
     const int s = it % NORM_STAGES, par = it & 1;
     const long long row = first + sub;
     const bool row_ok = row < T;
-    if (!mbar_wait(&full[s], (it / NORM_STAGES) & 1, abort_flag)) { atomicExch(status, 70); break; }
-    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(norm_smem + s * set_bytes) + sub * H;
+    if (BULK && !mbar_wait(&full[s], (it / NORM_STAGES) & 1, abort_flag)) { atomicExch(status, 70); break; }
+    const __nv_bfloat16* src = BULK ? reinterpret_cast<const __nv_bfloat16*>(norm_smem + s * set_bytes) + sub * H : x + row * H;
     float f[VPT][8];
     float acc = 0.f;
 #pragma unroll
@@ -142,9 +147,11 @@ __global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat1
       }
     }
     const float ss = group_sum(acc, red[par][1], lanes, sub);
-    if (lanes <= 32) __syncthreads();
-    // every thread has its part of the rows in registers: the stage may be refilled
-    if (threadIdx.x == 0) request(first + NORM_STAGES * step, s);
+    if (BULK) {
+      if (lanes <= 32) __syncthreads();
+      // every thread has its part of the rows in registers: the stage may be refilled
+      if (threadIdx.x == 0) request(first + NORM_STAGES * step, s);
+    }
     if (!row_ok) continue;
     const float rstd = rsqrtf(ss / H + eps);
     if (l == 0) { rstd_out[row] = rstd; if (LN) mean_out[row] = mean; }
@@ -153,12 +160,60 @@ __global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat1
     for (int k = 0; k < VPT; ++k) {
       const int c = (l + k * lanes) * 8;
       if (c < H) {
-        float g[8], h[8]; wv[k].to_float(g);
-        if (LN) bv[k].to_float(h);
+        float g[8], h[8];
+        if constexpr (!HOLD) { wv[0].load(w + c); bv[0].load(b + c); }
+        wv[HOLD ? k : 0].to_float(g);
+        if constexpr (LN) bv[HOLD ? k : 0].to_float(h);
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[k][i] = LN ? f[k][i] * rstd * g[i] + h[i] : __bfloat162float(__float2bfloat16(f[k][i] * rstd)) * g[i];
         bf16x8 o; o.from_float(f[k]); o.store(yr + c);
       }
+    }
+  }
+}
+
+// LayerNorm forward with one 256-thread block per row, VPT 8-wide vectors per thread, for short batches and for widths at which the
+// form above leaves a quarter of its threads idle with registers for two blocks per SM (norm_fwd): 500 x 4096 5.1 us here and 6.3 there,
+// 2000 x 2048 6.8 and 8.2, 16384 x 5120 69 and 78.
+template <int VPT>
+__global__ void __launch_bounds__(EW_THREADS) layernorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                  const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
+                                                                  float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, int H) {
+  __shared__ float red[32];
+  const long long row = blockIdx.x;
+  const __nv_bfloat16* xr = x + row * H;
+  float f[VPT][8];
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int c = (threadIdx.x + k * EW_THREADS) * 8;
+    if (c < H) {
+      bf16x8 v; v.load(xr + c); v.to_float(f[k]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += f[k][i];
+    }
+  }
+  const float mean = block_sum(s, red) / H;
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int c = (threadIdx.x + k * EW_THREADS) * 8;
+    if (c < H) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { f[k][i] -= mean; ss += f[k][i] * f[k][i]; }
+    }
+  }
+  const float rstd = rsqrtf(block_sum(ss, red) / H + eps);
+  if (threadIdx.x == 0) { mean_out[row] = mean; rstd_out[row] = rstd; }
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int c = (threadIdx.x + k * EW_THREADS) * 8;
+    if (c < H) {
+      bf16x8 wv, bv; wv.load(w + c); bv.load(b + c);
+      float fw[8], fb[8], o[8]; wv.to_float(fw); bv.to_float(fb);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) o[i] = f[k][i] * rstd * fw[i] + fb[i];
+      bf16x8 ov; ov.from_float(o); ov.store(y + row * H + c);
     }
   }
 }
@@ -920,24 +975,28 @@ static int num_sms() {
 using namespace mtb;
 typedef __nv_bfloat16 bf16;
 
-template <bool LN, int VPT>
+template <bool LN, int VPT, bool BULK>
 static int launch_norm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, float eps, int T, int H, int lanes,
                            int* status, cudaStream_t st) {
-  auto kern = norm_fwd_kernel<LN, VPT>;
+  auto kern = norm_fwd_kernel<LN, VPT, BULK>;
   const int rows = EW_THREADS / lanes;
-  const int smem = NORM_STAGES * rows * H * 2;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM_STAGES * 8 * 8 * EW_THREADS * 2) != cudaSuccess) return -4;
-    configured = true;
+  const int smem = BULK ? NORM_STAGES * rows * H * 2 : 0;
+  int grid = cdiv(T, rows);
+  if constexpr (BULK) {
+    static bool configured = false;
+    if (!configured) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM_STAGES * 8 * 8 * EW_THREADS * 2) != cudaSuccess) return -4;
+      configured = true;
+    }
+    static thread_local int for_smem = -1, resident = 0;   // the occupancy of the last shape this thread launched
+    if (for_smem != smem) {
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, EW_THREADS, smem) != cudaSuccess || resident < 1) return -4;
+      for_smem = smem;
+    }
+    const int most = num_sms() * resident;
+    if (grid > most) grid = most;
   }
-  static thread_local int for_smem = -1, resident = 0;   // the occupancy of the last shape this thread launched
-  if (for_smem != smem) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, EW_THREADS, smem) != cudaSuccess || resident < 1) return -4;
-    for_smem = smem;
-  }
-  const int want = cdiv(T, rows), most = num_sms() * resident;
-  kern<<<want < most ? want : most, EW_THREADS, smem, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, T, H, lanes, status);
+  kern<<<grid, EW_THREADS, smem, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, T, H, lanes, status);
   return launch_ok();
 }
 
@@ -951,15 +1010,40 @@ static int norm_fwd(const void* x, const void* w, const void* b, void* y, float*
   int lanes = 32;
   while (lanes < EW_THREADS && lanes * 4 < vecs) lanes *= 2;
   const int vpt = cdiv(vecs, lanes);
-#define NF(V) return launch_norm_fwd<LN, V>(x, w, b, y, mean, rstd, eps, T, H, lanes, status, st)
-  if (vpt <= 1) NF(1);
-  if (vpt <= 2) NF(2);
-  if (vpt <= 3) NF(3);
-  if (vpt <= 4) NF(4);
-  if constexpr (!LN) NF(8);
+  if constexpr (LN) {
+    // Rows of up to 1024 elements: eight and more per block pay at any height (16384 x 1024: 14.5 us, 27 with a block per row). Wider
+    // ones want a batch that lasts: equal at 4000 x 2048 and 6000 x 4096. Three vectors of 256 threads (4104 .. 6144) never win.
+    const long long n = static_cast<long long>(T) * H;
+    const bool bulk = H <= 1024 || (H <= 2048 ? n >= 6000000 : n >= 24000000 && !(lanes == EW_THREADS && vpt == 3));
+    if (!bulk) {
+#define LF(V) layernorm_row_kernel<V><<<T, EW_THREADS, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, H)
+      const int v = cdiv(H, 8 * EW_THREADS);
+      if (v <= 1) LF(1); else if (v == 2) LF(2); else if (v == 3) LF(3); else LF(4);
+#undef LF
+      return launch_ok();
+    }
+#define NF(V) return launch_norm_fwd<true, V, true>(x, w, b, y, mean, rstd, eps, T, H, lanes, status, st)
+    if (vpt <= 1) NF(1);
+    if (vpt <= 2) NF(2);
+    if (vpt <= 3) NF(3);
+    NF(4);
 #undef NF
-  return -10;
+  } else {
+    // By bulk copies when a block gets more than two and a half row sets: blocks that fit on an SM with the stages, eight at most.
+    const int rows = EW_THREADS / lanes, stages = NORM_STAGES * rows * H * 2 + 1280;
+    const int fit = 227 * 1024 / stages < 8 ? 227 * 1024 / stages : 8;
+    const bool bulk = 2 * cdiv(T, rows) > 5 * fit * num_sms();
+#define NF(V) return bulk ? launch_norm_fwd<false, V, true>(x, w, b, y, mean, rstd, eps, T, H, lanes, status, st) \
+                          : launch_norm_fwd<false, V, false>(x, w, b, y, mean, rstd, eps, T, H, lanes, status, st)
+    if (vpt <= 1) NF(1);
+    if (vpt <= 2) NF(2);
+    if (vpt <= 3) NF(3);
+    if (vpt <= 4) NF(4);
+    NF(8);
+#undef NF
+  }
 }
+
 
 // Threads of a norm backward block: the row's vectors over as few vectors per thread as 512 threads allow.
 static int norm_bwd_vpt(int H) { return cdiv(H, 8 * 512); }

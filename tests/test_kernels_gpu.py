@@ -822,3 +822,26 @@ def test_attention_forward_both_forms(ops, D, hq, hkv, lens, pairs, monkeypatch)
     assert rel_err(out, ro) < 1e-2 and max_err(out, ro) < 0.1
     out2, lse2 = ops.attention(qkv, cu, cu_host, max(lens), hq, hkv, D)
     assert torch.equal(out, out2) and torch.equal(lse, lse2)
+
+
+# both sides of every line the forward of the norms is drawn by: few and many row sets per block, one block per row, the widths at
+# which a row takes one to eight warps, partial last row sets
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 256), (2368 * 2 + 1, 512), (20011, 512), (740, 896), (15000, 896), (1481, 12288), (450, 12288), (3, 16384),
+                                 (800, 16384), (2930, 2048), (2929, 2048), (5857, 1024), (9400, 2560), (9375, 2560), (6001, 4096), (5000, 5120), (2930, 8192),
+                                 (100, 8192)])
+def test_norm_forward_forms(ops, T, H):
+    torch.manual_seed(T + H)
+    x, w, b = bf(T, H), bf(H), bf(H)
+    x += 0.5
+    y, rstd = ops.rmsnorm(x, w, 1e-5)
+    xf = x.double()
+    r = (xf.pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt()
+    assert rel_err(rstd, r.reshape(-1)) < 1e-6                    # fp32 sums of up to 16384 squares
+    assert max_err(y, (xf * r).bfloat16().double() * w.double()) < 2e-2   # one bf16 step of the normalised value, one of the product
+    if H <= 8192:
+        y, (mean, rstd) = ops.layernorm(x, w, b, 1e-5)
+        mu = xf.mean(-1, keepdim=True)
+        r = ((xf - mu).pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt()
+        assert (mean - mu.reshape(-1)).abs().max() < 1e-6 and rel_err(rstd, r.reshape(-1)) < 1e-6
+        assert max_err(y, (xf - mu) * r * w.double() + b.double()) < 1e-2
+    ops.check_status()

@@ -832,9 +832,10 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
 
 // ------------------------------------------------------------------------------ column sums (bias grad)
 // part[split, c] = sum over this split's rows of x[r, c]; then reduce_rows_kernel. A lane adds V neighbouring columns of every
-// eighth row: V = 8 (16-byte loads) where rows are 16-byte aligned, V = 2 for any even width. Bound by reading x
-// (7001 rows of 3072 to 12288 columns, four calls: 96 -> 73 us).
-template <int V>
+// eighth row: V = 8 (16-byte loads) where rows are 16-byte aligned, V = 2 for any even width, and for few columns and rows, where more
+// blocks count. Bound by reading x (7001 rows of 3072 to 12288 columns, four calls: 96 -> 73 us). UNROLL rows are in flight per
+// warp: eight where few blocks read many rows (64000 x 1024: 82 -> 64 us, V = 2 70), four otherwise (16384 x 6144: 48 us with eight, 38).
+template <int V, int UNROLL>
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restrict__ part,
                                                             int T, int N) {
   __shared__ float sm[8][32 * V];
@@ -846,7 +847,7 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 #pragma unroll
   for (int i = 0; i < V; ++i) a[i] = 0.f;
   if (c < N) {
-#pragma unroll 4
+#pragma unroll UNROLL
     for (int r = r0 + wy; r < r1; r += 8) {
       const __nv_bfloat16* p = x + static_cast<long long>(r) * ld + c;
       if constexpr (V == 8) {
@@ -1266,9 +1267,12 @@ int mtb200_ce_fwd_bwd(const void* logits, long long ld, int logits_bf16, const f
 
 static void launch_colsum(const void* x, long long ld, void* out, float* scratch, int T, int N, cudaStream_t st) {
   const int splits = T < 32 ? 1 : 32;
-  const bool wide = N % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  if (wide) colsum_partial_kernel<8><<<dim3(cdiv(N, 256), splits), 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
-  else colsum_partial_kernel<2><<<dim3(cdiv(N, 64), splits), 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
+  const bool many = T >= 8192;   // at least four times eight rows per warp
+  const bool wide = N % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (many || N > 1024);
+  const dim3 grid(cdiv(N, wide ? 256 : 64), splits);
+  if (wide && many && N <= 5120) colsum_partial_kernel<8, 8><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
+  else if (wide) colsum_partial_kernel<8, 4><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
+  else colsum_partial_kernel<2, 4><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
   reduce_rows_kernel<<<cdiv(N, 32), 512, 0, st>>>(scratch, (bf16*)out, nullptr, splits, N, N);
 }
 

@@ -845,3 +845,15 @@ def test_norm_forward_forms(ops, T, H):
         assert (mean - mu.reshape(-1)).abs().max() < 1e-6 and rel_err(rstd, r.reshape(-1)) < 1e-6
         assert max_err(y, (xf - mu) * r * w.double() + b.double()) < 1e-2
     ops.check_status()
+
+
+@pytest.mark.parametrize("T,N", [(1, 512), (8, 896), (37, 66), (4000, 1024), (4000, 1032), (8191, 264), (8192, 264), (9001, 5120), (9001, 5128), (700, 6)])
+def test_column_sums_forms(ops, T, N):
+    """Both load widths, both unrollings, one to 32 partial rows."""
+    torch.manual_seed(T + N)
+    x = bf(T, N)
+    out, scratch = torch.empty(N, dtype=torch.bfloat16, device="cuda"), torch.empty(32 * N, device="cuda")
+    ops._call("mtb200_colsum", x.data_ptr(), x.stride(0), out.data_ptr(), scratch.data_ptr(), T, N, ops._st())
+    ref = x.double().sum(0)
+    # one rounding to bf16, and fp32 sums whose terms have the size of the column's norm
+    assert ((out.double() - ref).abs() <= ref.abs() * 2 ** -8 + x.double().pow(2).sum(0).sqrt() * 1e-5).all()

@@ -359,7 +359,8 @@ __global__ void __launch_bounds__(512) norm_bwd_kernel(const __nv_bfloat16* __re
 
 // Sums of R partial rows of C columns; columns [0, D) go to out_a, the rest to out_b (a row may hold the partials of two
 // vectors; D = C when it holds one). 32 columns per block, 16 warps share the rows: a chain of R / 16 loads instead of R
-// (296 rows of 4096: 15 -> 5 us).
+// (296 rows of 4096: 15 -> 5 us). Few rows are one thread's work per column (reduce_few_rows_kernel): with a batch of eight tokens the
+// barrier and the many blocks took longer than the sum (colsum of 8 x 896: 6.3 us, 4.7 like this).
 __global__ void __launch_bounds__(512) reduce_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
                                                          int R, int C, int D) {
   __shared__ float sm[16][32];
@@ -377,6 +378,14 @@ __global__ void __launch_bounds__(512) reduce_rows_kernel(const float* __restric
     for (int k = 1; k < 16; ++k) s += sm[k][lane];
     if (c < D) out_a[c] = __float2bfloat16(s); else out_b[c - D] = __float2bfloat16(s);
   }
+}
+__global__ void __launch_bounds__(256) reduce_few_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
+                                                             int R, int C, int D) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= C) return;
+  float s = 0.f;
+  for (int r = 0; r < R; ++r) s += part[static_cast<long long>(r) * C + c];
+  if (c < D) out_a[c] = __float2bfloat16(s); else out_b[c - D] = __float2bfloat16(s);
 }
 
 // ------------------------------------------------------------------------------ RoPE
@@ -964,6 +973,10 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
 }
 
 static inline int cdiv(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
+static void reduce_rows(const float* part, void* out_a, void* out_b, int R, int C, int D, cudaStream_t st) {
+  if (R <= 16) reduce_few_rows_kernel<<<cdiv(C, 256), 256, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
+  else reduce_rows_kernel<<<cdiv(C, 32), 512, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
+}
 static inline int launch_ok() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }
 static int num_sms() {
   static int n = 0;
@@ -1104,7 +1117,7 @@ int mtb200_rmsnorm_bwd(const void* dy, const void* x, const float* rstd, const v
   if (vpt <= 1) rc = RB(1); else if (vpt == 2) rc = RB(2); else if (vpt == 3) rc = RB(3); else rc = RB(4);
 #undef RB
   if (rc) return rc;
-  reduce_rows_kernel<<<cdiv(H, 32), 512, 0, st>>>(dw_partial, (bf16*)dw_out, nullptr, blocks, H, H);
+  reduce_rows(dw_partial, dw_out, nullptr, blocks, H, H, st);
   return launch_ok();
 }
 
@@ -1120,7 +1133,7 @@ int mtb200_layernorm_bwd(const void* dy, const void* x, const float* mean, const
   if (norm_bwd_vpt(H) <= 1) rc = LB(1); else rc = LB(2);
 #undef LB
   if (rc) return rc;
-  reduce_rows_kernel<<<cdiv(2 * H, 32), 512, 0, st>>>(dw_partial, (bf16*)dw_out, (bf16*)db_out, blocks, 2 * H, H);
+  reduce_rows(dw_partial, dw_out, db_out, blocks, 2 * H, H, st);
   return launch_ok();
 }
 
@@ -1172,7 +1185,7 @@ int mtb200_head_rmsnorm_bwd(void* dqkv, const void* pre, const float* rstd, cons
   else { if (D == 64) HB(2, false); else if (D == 128) HB(4, false); else HB(8, false); }
 #undef HB
   // partial rows are [2, D]: columns 0..D-1 belong to the q weight, D..2D-1 to the k weight
-  reduce_rows_kernel<<<cdiv(2 * D, 32), 512, 0, st>>>(dw_partial, (bf16*)dwq_out, (bf16*)dwk_out, blocks, 2 * D, D);
+  reduce_rows(dw_partial, dwq_out, dwk_out, blocks, 2 * D, D, st);
   return launch_ok();
 }
 
@@ -1273,7 +1286,7 @@ static void launch_colsum(const void* x, long long ld, void* out, float* scratch
   if (wide && many && N <= 5120) colsum_partial_kernel<8, 8><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
   else if (wide) colsum_partial_kernel<8, 4><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
   else colsum_partial_kernel<2, 4><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
-  reduce_rows_kernel<<<cdiv(N, 32), 512, 0, st>>>(scratch, (bf16*)out, nullptr, splits, N, N);
+  reduce_rows(scratch, out, nullptr, splits, N, N, st);
 }
 
 // out[N] (bf16) = column sums of x[T, N]. scratch: fp32 [32, N].

@@ -87,7 +87,7 @@ __device__ __forceinline__ void mbar_arrive_cta0(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & PEER_MASK) : "memory");
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS, 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_d, Params p,
@@ -264,7 +264,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag)) { atomicExch(p.status, 54); goto done; }
       tc_fence_after();
-      epilogue_quarter<OUT_F32, !GATHER, STATS>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
+      epilogue_quarter<OUT_F32, !GATHER, STATS, EXTRA>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
                                 2 * t + static_cast<int>(rank), w / num_tiles, false);
       tc_fence_before();
       __syncwarp();
@@ -306,10 +306,10 @@ static int co_resident_pairs() {
   return pairs;
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
                   long long ws_bytes = 0) {
-  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS>;
+  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA>;
   constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS;
   static bool configured = false;
   if (!configured) {
@@ -382,17 +382,20 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
       default: return launch<true, true, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
     }
   }
+#define GEMM2(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, ws_bytes) \
+                                                              : launch<X, Y, Z, false, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes)
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
-    case 0: return launch<false, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 1: return launch<false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 2: return launch<false, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 3: return launch<false, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 4: return launch<true, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 5: return launch<true, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 6: return launch<true, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    default: return launch<true, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 0: GEMM2(false, false, false);
+    case 1: GEMM2(false, false, true);
+    case 2: GEMM2(false, true, false);
+    case 3: GEMM2(false, true, true);
+    case 4: GEMM2(true, false, false);
+    case 5: GEMM2(true, false, true);
+    case 6: GEMM2(true, true, false);
+    default: GEMM2(true, true, true);
   }
+#undef GEMM2
 }
 
 }  // extern "C"

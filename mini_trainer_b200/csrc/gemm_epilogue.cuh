@@ -70,12 +70,12 @@ __device__ __forceinline__ void drain_boxes() { bulk_wait_read<0>(); }
 
 // 32 accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
 // bf16 box; an fp32 box holds 32 columns). Columns past N and rows past M are computed from nothing and clipped by the store.
-template <bool OUT_F32, bool STATS>
+template <bool OUT_F32, bool STATS, bool EXTRA>
 __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
                                                RowStats& st) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) f[j] *= p.alpha;
-  if (p.bias != nullptr) {
+  if (EXTRA && p.bias != nullptr) {
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
       if (col0 + j < p.N) {
@@ -86,7 +86,7 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
       }
     }
   }
-  const bool res = p.R != nullptr && row_ok;
+  const bool res = EXTRA && p.R != nullptr && row_ok;
   if constexpr (OUT_F32) {
     const float* rptr = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
@@ -123,9 +123,11 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
 // One warp's part of a work item: quarter `q` of the 128-row unit that starts at row `row0`, columns [tn0, tn0 + 256).
 // `taddr`: tensor-memory address of the quarter. `unit`: index of the 128-row unit among all tiles' units. `zero`: the item
 // had nothing to multiply, the accumulator holds an older tile. SPLIT = false leaves the split-K part out, STATS = false the
-// statistics: a worker walks this code once per tile, and with the statistics as a run-time branch in every product the
-// instructions to fetch made a launch of one wave 2 us longer (384 x 2048 x 2048: 18.6 and 16.5 us, 4736 x 1024 x 512: 11.3 and 10.4).
-template <bool OUT_F32, bool SPLIT, bool STATS>
+// statistics, EXTRA = false bias and residual: a worker walks this code once per tile, and what it does not need has to be fetched
+// and branched around all the same. With the statistics as a run-time branch in every product a launch of one wave took 2 us
+// more (384 x 2048 x 2048: 18.6 and 16.5 us, 4736 x 1024 x 512: 11.3 and 10.4), with bias and residual another step for some
+// (824 x 80 x 824: 12.3 and 10.6 us; on pairs 40000 x 768 x 768: 45.2 and 43.2).
+template <bool OUT_F32, bool SPLIT, bool STATS, bool EXTRA>
 __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane,
                                                  int unit, int split, bool zero) {
   constexpr int PARTS = OUT_F32 ? 1 : 2;      // 32-column pieces per box
@@ -152,7 +154,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
         float f[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) f[j] = zero ? 0.f : __uint_as_float(v[k][j]);
-        epilogue_row32<OUT_F32, STATS>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
+        epilogue_row32<OUT_F32, STATS, EXTRA>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
       }
       store_box(out, box, col0, row0 + q * 32, lane);
     }
@@ -201,7 +203,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
           }
         }
       }
-      epilogue_row32<OUT_F32, STATS>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
+      epilogue_row32<OUT_F32, STATS, EXTRA>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
     }
     store_box(out, box, col0, row0 + q * 32, lane);
   }

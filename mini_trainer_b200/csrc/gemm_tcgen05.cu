@@ -57,8 +57,8 @@ struct GemmParams {
 // buffers (reduce_chunks in gather.cuh): the gradient reduce-scatter with ownership by tensor, fused into the GEMM
 // that consumes the reduced gradient (OSFT factor gradients).
 // GROUP: one launch over the expert slabs of a mixture-of-experts layer (gemm_epilogue.cuh).
-// STATS: softmax statistics of the output rows (EpiParams).
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false>
+// STATS: softmax statistics of the output rows (EpiParams). EXTRA: bias or residual.
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true>
 __global__ void __launch_bounds__(GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_d, GemmParams p,
@@ -270,7 +270,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 4); goto done; }
       tc_fence_after();
-      epilogue_quarter<OUT_F32, !GATHER && !GROUP, STATS>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
+      epilogue_quarter<OUT_F32, !GATHER && !GROUP, STATS, EXTRA && !GROUP>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
                                                    w / num_tiles, GROUP == GROUP_REDUCE && gr.counts[e] == 0);
       tc_fence_before();
       __syncwarp();
@@ -380,11 +380,11 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
                   const void* w, int* status, const GatherParams& g, cudaStream_t stream);
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmParams p, cudaStream_t stream,
                   const GatherParams* gp = nullptr, long long ws_bytes = 0, const GroupParams* grp = nullptr) {
   static bool configured = false;
-  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS>;
+  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS, EXTRA>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess) return -4;
     configured = true;
@@ -448,17 +448,20 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
       default: return launch<true, true, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
     }
   }
+#define GEMM(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, ws_bytes) \
+                                                             : launch<X, Y, Z, false, false, GROUP_NONE, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes)
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
-    case 0: return launch<false, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 1: return launch<false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 2: return launch<false, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 3: return launch<false, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 4: return launch<true, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 5: return launch<true, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    case 6: return launch<true, true, false>(ta, tb, td, p, stream, nullptr, ws_bytes);
-    default: return launch<true, true, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+    case 0: GEMM(false, false, false);
+    case 1: GEMM(false, false, true);
+    case 2: GEMM(false, true, false);
+    case 3: GEMM(false, true, true);
+    case 4: GEMM(true, false, false);
+    case 5: GEMM(true, false, true);
+    case 6: GEMM(true, true, false);
+    default: GEMM(true, true, true);
   }
+#undef GEMM
 }
 
 // Grouped GEMM over expert slabs (see gemm_epilogue.cuh); starts [E + 1] and counts [E] are device arrays, `rows` is the

@@ -102,7 +102,7 @@ static int run(int m, int n, int z_count, int first, int step, int q, int splits
     if (z_count > 1) o.z = z;
     for (int s = 0; s < splits; ++s) {
       for (int c = 0; c < 256; ++c) tmem[c] = s == 0 ? value(z, row0 + q * 32, tn0 + c) : 0.f;
-      epilogue_quarter<OUT_F32, SPLIT, false>(p, o, 0, row0, tn0, q, 0, t, s, false);
+      epilogue_quarter<OUT_F32, SPLIT, false, false>(p, o, 0, row0, tn0, q, 0, t, s, false);
     }
   }
   drain_boxes();

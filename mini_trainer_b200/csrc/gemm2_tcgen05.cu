@@ -319,11 +319,10 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int pairs = co_resident_pairs<GATHER>();
   if (pairs <= 0) return -6;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
-  // The arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest.
-  if (!GATHER && p.e.ws != nullptr && tiles * 8 * 4 <= SPLIT_COUNTER_BYTES) {
+  if (p.e.splits > 1) {   // the arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest
+    if (!split_fits(p.e, 2 * tiles, (p.K + BK - 1) / BK, ws_bytes)) return -11;
     p.e.counters = reinterpret_cast<unsigned*>(p.e.ws);
     p.e.ws += SPLIT_COUNTER_BYTES / 4;
-    p.e.splits = choose_splits(tiles, (p.K + BK - 1) / BK, pairs, (ws_bytes - SPLIT_COUNTER_BYTES) / (2 * SPLIT_UNIT * 4));
   }
   // the gathering variant always uses every pair: its extra warps carry the transfer
   const int items = tiles * p.e.splits;
@@ -358,11 +357,11 @@ int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
 
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                      float alpha, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
+                      float alpha, int splits, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   using namespace mtb::g2;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32)) return -10;
+  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32) || splits < 1) return -10;
   CUtensorMap ta, tb, td;
   int rc;
   if (a_mn) rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, 64);
@@ -373,7 +372,7 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
   if (rc) return rc - 10;
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
-  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, stats, nullptr}};
+  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr}};
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
       case 0: return launch<false, false, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);

@@ -253,23 +253,10 @@ __device__ __forceinline__ void fill_group_table(GroupTable& tab, const GroupPar
   if (lane == 0) tab.tile_start[g.E] = base;
 }
 
-// Number of work items per tile: 1 when whole tiles fill the `workers` (SMs or CTA pairs) well, else the smallest cost in
-// units of one k-block of a tile: full waves of items, plus what the extra partials cost (write, one counter, ordered sum).
-// A k-block is about 0.4 us on one SM; an item costs ten more (its share of a partial's write and of the pipeline fill), the
-// ordered sum three per partial: without those terms 2048 x 1536 x 5987 (96 tiles) was split in three and went from 40 to 46 us.
-// `max_items`: what the workspace holds.
-inline int choose_splits(long long tiles, int kblocks, int workers, long long max_items) {
-  if (tiles <= 0 || workers <= 0) return 1;
-  auto waves = [&](long long items) { return (items + workers - 1) / workers; };
-  const double whole = static_cast<double>(waves(tiles)) * kblocks + 8.0;
-  int best = 1;
-  double best_cost = whole * 0.95;   // a split has to win by more than the model's error
-  for (int s = 2; s <= 16; ++s) {
-    if (tiles * s > max_items || kblocks / s < 6) break;
-    const double cost = static_cast<double>(waves(tiles * s)) * ((kblocks + s - 1) / s + 10.0) + 14.0 + 3.0 * s;
-    if (cost < best_cost) { best = s; best_cost = cost; }
-  }
-  return best;
+// Whether a split launch over `units` 128-row units fits its workspace and leaves every item a k-block.
+inline bool split_fits(const EpiParams& e, long long units, int kblocks, long long ws_bytes) {
+  return e.ws != nullptr && e.splits <= kblocks && units * 4 * 4 <= SPLIT_COUNTER_BYTES &&
+         units * e.splits * SPLIT_UNIT * 4 <= ws_bytes - SPLIT_COUNTER_BYTES;
 }
 
 }  // namespace mtb

@@ -396,11 +396,10 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   }
   int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   if (GROUP == GROUP_REDUCE) tiles *= grp->E;
-  // The arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest.
-  if (!GATHER && !GROUP && p.e.ws != nullptr && tiles * 4 * 4 <= SPLIT_COUNTER_BYTES) {
+  if (p.e.splits > 1) {   // the arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest
+    if (!split_fits(p.e, tiles, (p.K + BK - 1) / BK, ws_bytes)) return -11;
     p.e.counters = reinterpret_cast<unsigned*>(p.e.ws);
     p.e.ws += SPLIT_COUNTER_BYTES / 4;
-    p.e.splits = choose_splits(tiles, (p.K + BK - 1) / BK, g_num_sms, (ws_bytes - SPLIT_COUNTER_BYTES) / (SPLIT_UNIT * 4));
   }
   // the gathering variant always uses every SM: its extra warps carry the transfer
   const int items = tiles * p.e.splits;
@@ -418,16 +417,16 @@ extern "C" {
 //   a_mn = 0: A is row-major [M, K] (lda >= K);  a_mn = 1: A is row-major [K, M] (lda >= M)
 //   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
 //   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
-//   ws: optional fp32 workspace of ws_bytes for split-K (null: never split); its first SPLIT_COUNTER_BYTES are zero
-//   before the first call, every launch leaves them zero again, and launches that may overlap have one each
+//   splits: work items per output tile (ops/gemm_plan.py); more than one needs ws, an fp32 workspace of ws_bytes: its first
+//   SPLIT_COUNTER_BYTES are zero before the first call, every launch leaves them zero again, and launches that may overlap have one each
 //   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
 // Returns 0 on success, a negative code on invalid arguments or launch failure.
 int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                     float alpha, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
+                     float alpha, int splits, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32)) return -10;
+  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32) || splits < 1) return -10;
   CUtensorMap ta, tb, td;
   int rc;
   if (a_mn) rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, 64);
@@ -439,7 +438,7 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, 1, ws, stats, nullptr}};
+               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr}};
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
       case 0: return launch<false, false, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);

@@ -17,7 +17,7 @@ import torch
 
 from .. import build as _build
 from ..utils import nvtx
-from . import attention_plan
+from . import attention_plan, gemm_plan
 
 _LIB = None
 _raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else \
@@ -47,8 +47,8 @@ P, I, L, F = c_void_p, c_int, c_longlong, c_float
 
 
 class _Sig:
-    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
-    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, P, L, P, P, P]
+    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, P, P, P]
+    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, P, P, P]
     mtb200_gemm2_pairs = []
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
     mtb200_norm_bwd_blocks = [I, I]
@@ -89,7 +89,8 @@ class _Sig:
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
 _SPLIT_COUNTERS = 4096          # 4-byte words in front of the partials (SPLIT_COUNTER_BYTES in csrc/gemm_epilogue.cuh)
-_SPLIT_FLOATS = 32 << 20        # partials: 128 MB = 1024 work items of 128 x 256
+_SPLIT_FLOATS = 32 << 20        # partials: 128 MB
+_SPLIT_UNITS = 4 * _SPLIT_FLOATS // gemm_plan.UNIT_BYTES   # = 1024 of 128 x 256
 NATIVE_HEAD_DIMS = (64, 128)   # head dimensions of the hand-written attention kernels
 
 
@@ -125,13 +126,11 @@ class NativeOps:
         self.ce_chunk = ce_chunk
         self.attention_impl = attention or os.environ.get("MTB200_ATTENTION", "native")
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-        # GEMM kernel for problems with about a full wave of 256x256 tiles or more. The CTA-pair kernel (cta_group::2) loads half
-        # of what the one-CTA kernel loads per product and is the faster one in itself, but it draws more power: in a step
-        # made of long GEMMs, which runs at the 1000 W cap, it lowers the clock of EVERY kernel by 12-16 % and the step gets
-        # slower (8B model, 64 000-token minibatches: 9.77 s per step with one CTA, 10.36 with pairs). Where GEMMs are short
-        # the cap does not bind (1.5B model, 8000-token minibatches: 729 and 700 ms, clocks 1530 and 1515 MHz; forward +
-        # backward of one of its blocks at 6000 tokens: 1.99 and 1.91 ms). The line is drawn at a GEMM of about 0.8 ms.
-        # MTB200_GEMM2=0 / 1 forces one kernel for all of them (1: also for the fused gathers).
+        # GEMM kernel and splits by size: gemm_plan. The CTA-pair kernel (cta_group::2) draws more power: in a step made of long GEMMs,
+        # which runs at the 1000 W cap, it lowers the clock of EVERY kernel by 12-16 % and the step gets slower (8B model, 64 000-token
+        # minibatches: 9.77 s per step with one CTA, 10.36 with pairs). Where GEMMs are short the cap does not bind (1.5B model,
+        # 8000-token minibatches: 729 and 700 ms, clocks 1530 and 1515 MHz). So a product of more than 1 TFLOP (about 0.8 ms)
+        # stays on single CTAs. MTB200_GEMM2=0 / 1 forces one kernel for all of them (1: also for the fused gathers).
         self.use_gemm2 = os.environ.get("MTB200_GEMM2") == "1"
         self.pair_max_flops = 0.0 if os.environ.get("MTB200_GEMM2") == "0" else 1e12
         self.launches = 0
@@ -240,15 +239,19 @@ class NativeOps:
         out_f32 = out.dtype == torch.float32
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
         assert residual is None or residual.dtype == out.dtype
-        if two_cta is None:
-            two_cta = (self.use_gemm2 or 2.0 * M * N * K <= self.pair_max_flops) and (-(-M // 256)) * (-(-N // 256)) >= 64
-        if two_cta and self.cta_pairs() <= 0:
-            two_cta = False
+        pairs, one = self.cta_pairs(), True
+        if two_cta if two_cta is not None else self.use_gemm2:
+            one = False
+        elif two_cta is not None or 2.0 * M * N * K > self.pair_max_flops:
+            pairs = 0
+        pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
         st = self._st()
-        ws = self._split_workspace(st)
-        self._call("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
+        ws = self._split_workspace(st) if splits > 1 else None
+        if ws is None:
+            splits = 1
+        self._call("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
-                   residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha),
+                   residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha), splits,
                    _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
         return out
 

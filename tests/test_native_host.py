@@ -9,10 +9,11 @@ def make_ops(**fakes):
     ops = object.__new__(native.NativeOps)
     ops.device = torch.device("cpu")
     ops._index, ops.launches, ops.profile = 0, 0, None
-    ops.use_gemm2, ops.pair_max_flops = False, 1e12
+    ops.use_gemm2, ops.pair_max_flops, ops.sms = False, 1e12, 148
     ops.status = torch.zeros(1, dtype=torch.int32)
     ops._scratch, ops._gemm_ws, ops._attn_plan_cache, ops._pairs = {}, {}, {}, None
     ops.calls = []
+    fakes.setdefault("mtb200_gemm2_pairs", lambda: 74)
 
     class Fns(dict):
         def __missing__(self, name):
@@ -33,7 +34,7 @@ def gemm(ops, M, N, K, **kw):
 def test_gemm_runs_on_single_ctas_where_pairs_cannot_be_scheduled(pairs):
     ops = make_ops(mtb200_gemm2_pairs=lambda: pairs)
     want = "mtb200_gemm2_bf16" if pairs else "mtb200_gemm_bf16"
-    assert gemm(ops, 4096, 2048, 64) == want
+    assert gemm(ops, 8192, 2048, 2048) == want
     assert gemm(ops, 512, 512, 64, two_cta=True) == want
     assert gemm(ops, 512, 512, 64, two_cta=False) == "mtb200_gemm_bf16"
 
@@ -114,3 +115,40 @@ def test_attention_backward_divides_only_what_the_workspace_holds():
         assert (splits > 1) == want and (args[18] is not None) == want
         if want:
             assert units * 8 <= 4096 and splits * units * 2 * 128 * d <= 32 << 20
+
+
+# (M, N, K, pair, whole): a round that only single CTAs fill evenly; two rounds where pairs are the faster per k-block; a few tiles with a
+# long reduction; one tile; more than 1 TFLOP. Each is at least 5 % faster than on the other kernel or with the other answer to splitting.
+@pytest.mark.parametrize("M,N,K,pair,whole", [(4736, 1024, 4096, False, True), (3700, 1280, 5120, False, True), (5987, 17920, 1536, True, True), (8192, 2048, 2048, True, True),
+                                              (4096, 2048, 4099, True, True), (128, 256, 4096, None, False), (896, 896, 6000, None, False), (128, 256, 64, None, True),
+                                              (3720, 1536, 151936, False, False), (16384, 4096, 14336, False, True)])
+def test_gemm_choice(M, N, K, pair, whole):
+    ops = make_ops()
+    ws = torch.zeros(1)
+    ops._split_workspace = lambda st: ws
+    a, b, out = (torch.empty(1, dtype=torch.bfloat16).expand(8, 8) for _ in range(3))
+    ops.gemm(a, False, b, False, out, M, N, K)
+    name, args = ops.calls[-1]
+    assert pair is None or (name == "mtb200_gemm2_bf16") == pair
+    assert (args[16] == 1) == whole and (args[17] is None) == whole
+    ops._split_workspace = lambda st: None      # as under capture
+    ops.gemm(a, False, b, False, out, M, N, K)
+    assert ops.calls[-1][0] == name and ops.calls[-1][1][16] == 1
+    for two in (False, True):
+        ops.gemm(a, False, b, False, out, M, N, K, two_cta=two)
+        assert ops.calls[-1][0] == ("mtb200_gemm2_bf16" if two else "mtb200_gemm_bf16")
+
+
+def test_gemm_choice_keeps_within_the_workspace():
+    from mini_trainer_b200.ops import gemm_plan as G
+    import random
+    rng = random.Random(1)
+    for _ in range(500):
+        M, N, K = (int(2 ** rng.uniform(0, 16)) for _ in range(3))
+        units, counted = rng.choice([(1024, 1024), (8, 4), (0, 0)])
+        for pairs, one in ((0, True), (74, True), (74, False), (0, False)):
+            two, s = G.choose(M, N, K, 148, pairs, one, units, counted)
+            u = -(-N // 256) * (2 * -(-M // 256) if two else -(-M // 128))
+            assert two is False or pairs > 0
+            assert two is True or one or pairs == 0
+            assert s == 1 or (u <= counted and u * s <= units and 4 * s <= -(-K // 64))

@@ -321,7 +321,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   if (p.e.splits > 1) {   // the arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest
     if (!split_fits(p.e, 2 * tiles, (p.K + BK - 1) / BK, ws_bytes)) return -11;
-    p.e.counters = reinterpret_cast<unsigned*>(p.e.ws);
+    p.e.counters = reinterpret_cast<unsigned long long*>(p.e.ws);
     p.e.ws += SPLIT_COUNTER_BYTES / 4;
   }
   // the gathering variant always uses every pair: its extra warps carry the transfer
@@ -342,7 +342,7 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
   if (rc) return rc - 10;
   rc = make_tmap_out(&td, D, M, N, ldd, 0);
   if (rc) return rc - 20;
-  Params p{M, N, K, status, 0, EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr}};
+  Params p{M, N, K, status, 0, EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0}};
   return launch<false, false, false, true>(ta, tb, td, p, stream, &g);
 }
 
@@ -357,7 +357,7 @@ int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
 
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                      float alpha, int splits, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
+                      float alpha, int splits, float* ws, long long ws_bytes, unsigned long long epoch, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   using namespace mtb::g2;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -372,7 +372,7 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
   if (rc) return rc - 10;
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
-  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr}};
+  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr, epoch}};
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
       case 0: return launch<false, false, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);

@@ -5,7 +5,8 @@
 // with few tiles and a long reduction, the tail of a two-wave grid). Every item leaves its fp32 partial in a workspace; the
 // warp that arrives last at the counter of a (tile, 32-row quarter) adds the partials in split order and runs the ordinary
 // epilogue. Nobody waits for anybody (the items may run in any order, on any number of SMs), the sum has one fixed order
-// whoever arrives last, and the counters are back at zero when the launch ends. 1536 x 1536 x 5987 (72 tiles on 148 SMs): 40 -> 33 us,
+// whoever arrives last. A counter counts the arrivals of one launch, named by its epoch: whatever an earlier launch that gave up has
+// left there does not count. 1536 x 1536 x 5987 (72 tiles on 148 SMs): 40 -> 33 us,
 // 3720 x 1536 x 151936 (180 tiles): 1791 -> 1231 us.
 #pragma once
 #include "ptx.cuh"
@@ -22,11 +23,21 @@ struct EpiParams {
   float* ws;              // splits > 1: partials, SPLIT_UNIT floats per (128-row unit, split)
   float2* stats;          // optional (bf16 output): per row and column tile, maximum and sum of exp(x - maximum) of the stored
                           // values, [M, ceil(N / 256)]; saves the cross-entropy its first pass over the logits
-  unsigned* counters;     // splits > 1: one arrival counter per (128-row unit, quarter); zero between launches
+  unsigned long long* counters;   // splits > 1: one arrival counter per (128-row unit, quarter)
+  unsigned long long epoch;       // splits > 1: number of this launch, larger than that of any launch before it on these counters
 };
 
-constexpr int SPLIT_COUNTER_BYTES = 16384;
+constexpr int SPLIT_COUNTERS = 4096;
+constexpr int SPLIT_COUNTER_BYTES = SPLIT_COUNTERS * 8;
 constexpr int SPLIT_UNIT = 128 * 256;   // floats of one partial: 128 rows x 256 columns
+
+// Arrival at a counter (one thread); true for the last of the launch's `splits` arrivals. The two operations of a thread on one
+// address are performed in order, so the count starts from this launch's epoch whatever was there. The caller sets the counter
+// to zero once the partials are added, which makes the order of the epochs matter only after a launch that gave up.
+__device__ __forceinline__ bool last_arrival(unsigned long long* counter, unsigned long long epoch, int splits) {
+  atomicMax(counter, epoch << 16);
+  return atomicAdd(counter, 1ull) == (epoch << 16) + static_cast<unsigned long long>(splits - 1);
+}
 
 // Running maximum and sum of exponentials of a row.
 struct RowStats {
@@ -176,10 +187,10 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
   }
   __threadfence();
   __syncwarp();
-  unsigned old = 0;
-  if (lane == 0) old = atomicAdd(p.counters + unit * 4 + q, 1u);
-  old = __shfl_sync(0xffffffffu, old, 0);
-  if (old != static_cast<unsigned>(p.splits) - 1) return;
+  unsigned last = 0;
+  if (lane == 0) last = last_arrival(p.counters + unit * 4 + q, p.epoch, p.splits);
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (!last) return;
   __threadfence();
   const float* base = p.ws + static_cast<long long>(unit) * p.splits * SPLIT_UNIT + q * 8192 + lane * 4;
 #pragma unroll 1
@@ -255,7 +266,7 @@ __device__ __forceinline__ void fill_group_table(GroupTable& tab, const GroupPar
 
 // Whether a split launch over `units` 128-row units fits its workspace and leaves every item a k-block.
 inline bool split_fits(const EpiParams& e, long long units, int kblocks, long long ws_bytes) {
-  return e.ws != nullptr && e.splits <= kblocks && units * 4 * 4 <= SPLIT_COUNTER_BYTES &&
+  return e.ws != nullptr && e.splits <= kblocks && units * 4 <= SPLIT_COUNTERS &&
          units * e.splits * SPLIT_UNIT * 4 <= ws_bytes - SPLIT_COUNTER_BYTES;
 }
 

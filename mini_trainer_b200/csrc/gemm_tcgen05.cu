@@ -398,7 +398,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   if (GROUP == GROUP_REDUCE) tiles *= grp->E;
   if (p.e.splits > 1) {   // the arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest
     if (!split_fits(p.e, tiles, (p.K + BK - 1) / BK, ws_bytes)) return -11;
-    p.e.counters = reinterpret_cast<unsigned*>(p.e.ws);
+    p.e.counters = reinterpret_cast<unsigned long long*>(p.e.ws);
     p.e.ws += SPLIT_COUNTER_BYTES / 4;
   }
   // the gathering variant always uses every SM: its extra warps carry the transfer
@@ -418,12 +418,12 @@ extern "C" {
 //   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
 //   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
 //   splits: work items per output tile (ops/gemm_plan.py); more than one needs ws, an fp32 workspace of ws_bytes: its first
-//   SPLIT_COUNTER_BYTES are zero before the first call, every launch leaves them zero again, and launches that may overlap have one each
+//   SPLIT_COUNTER_BYTES are zero before the first call, and launches that may overlap have one each. epoch (splits > 1): grows with every launch
 //   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
 // Returns 0 on success, a negative code on invalid arguments or launch failure.
 int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                     float alpha, int splits, float* ws, long long ws_bytes, float2* stats, int* status, cudaStream_t stream) {
+                     float alpha, int splits, float* ws, long long ws_bytes, unsigned long long epoch, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32) || splits < 1) return -10;
@@ -438,7 +438,7 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr}};
+               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr, epoch}};
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
       case 0: return launch<false, false, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
@@ -486,7 +486,7 @@ int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long l
   else rc = make_tmap_out(&td, D, rows, N, ldd, 0);
   if (rc) return rc - 20;
   GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr}};
+               EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0}};
   GroupParams g{starts, counts, E};
   if (mode == 0) return launch<false, false, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
   if (mode == 1) return launch<false, true, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
@@ -520,7 +520,7 @@ int mtb200_gemm_bf16_allgather(const void* A, long long lda, void* D, long long 
   rc = make_tmap_out(&td, D, M, N, ldd, 0);
   if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr}};
+               EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0}};
   GatherParams g{};
   for (int i = 0; i < world; ++i) g.peer_base[i] = bases[i];
   g.shard_off = shard_off; g.shard_bytes = shard_bytes; g.dst = reinterpret_cast<unsigned char*>(full);
@@ -562,7 +562,7 @@ int mtb200_gemm_bf16_reduce_a(void* dst, const void* B, long long ldb, float* D,
   rc = make_tmap_out(&td, D, M, N, ldd, 1);
   if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), lim + lim / 2 + 10000000u,
-               EpiParams{M, N, R, ldr, nullptr, 1.0f, 1, nullptr, nullptr, nullptr}};
+               EpiParams{M, N, R, ldr, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0}};
   GatherParams g{};
   for (int i = 0; i < world; ++i) g.peer_base[i] = bases[i];
   g.dst = reinterpret_cast<unsigned char*>(dst);

@@ -9,9 +9,10 @@ there is no silent fallback to PyTorch on a GPU machine.
 from __future__ import annotations
 
 import ctypes
+import itertools
 import os
 from dataclasses import dataclass
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
 import torch
 
@@ -43,12 +44,12 @@ def load_library():
     return lib
 
 
-P, I, L, F = c_void_p, c_int, c_longlong, c_float
+P, I, L, F, U = c_void_p, c_int, c_longlong, c_float, c_ulonglong
 
 
 class _Sig:
-    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, P, P, P]
-    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, P, P, P]
+    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, U, P, P, P]
+    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, U, P, P, P]
     mtb200_gemm2_pairs = []
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
     mtb200_norm_bwd_blocks = [I, I]
@@ -84,11 +85,11 @@ class _Sig:
     mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
     mtb200_attn_fwd_one = [P, L, P, L, P, P, I, I, I, I, I, F, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
-    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, L, F, P, P]
+    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, L, U, F, P, P]
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
-_SPLIT_COUNTERS = 4096          # 4-byte words in front of the partials (SPLIT_COUNTER_BYTES in csrc/gemm_epilogue.cuh)
+_SPLIT_COUNTERS = 4096          # 8-byte words in front of the partials (csrc/gemm_epilogue.cuh)
 _SPLIT_FLOATS = 32 << 20        # partials: 128 MB
 _SPLIT_UNITS = 4 * _SPLIT_FLOATS // gemm_plan.UNIT_BYTES   # = 1024 of 128 x 256
 NATIVE_HEAD_DIMS = (64, 128)   # head dimensions of the hand-written attention kernels
@@ -137,6 +138,7 @@ class NativeOps:
         self.profile = [] if os.environ.get("MTB200_PROFILE") else None
         self._scratch = {}
         self._gemm_ws = {}   # stream handle -> split-K workspace
+        self._epoch = itertools.count(1)   # of the launches that may split
         self._attn_plan_cache = {}
         self._pairs = None
         self.sms = torch.cuda.get_device_properties(self._index).multi_processor_count
@@ -201,8 +203,6 @@ class NativeOps:
         code = int(self.status.item())
         if code:
             self.status.zero_()
-            for ws in self._gemm_ws.values():   # a kernel that gave up may have left arrivals behind
-                ws[: _SPLIT_COUNTERS].zero_()
             what = {60: "a token id outside the embedding table", 61: "an attention work item outside the packed batch",
                     62: "a chosen expert outside the model's experts"}.get(
                 code, "a device-side bounded wait expired")
@@ -216,7 +216,7 @@ class NativeOps:
         return self._pairs
 
     def _split_workspace(self, stream):
-        """Split-K workspace of a stream: arrival counters (zero between launches) and fp32 partials. GEMMs of one stream run
+        """Split-K workspace of a stream: arrival counters and fp32 partials. GEMMs of one stream run
         one after the other, those of different streams may overlap, so each stream has its own (the last eight streams do;
         a dropped one goes back to its stream's pool, behind the launches that use it). ``None`` under capture: a graph may be
         replayed beside anything, so its launches never split."""
@@ -226,8 +226,8 @@ class NativeOps:
         if ws is None:
             if len(self._gemm_ws) >= 8:
                 self._gemm_ws.pop(next(iter(self._gemm_ws), None), None)
-            ws = torch.empty(_SPLIT_COUNTERS + _SPLIT_FLOATS, dtype=torch.float32, device=self.device)
-            ws[: _SPLIT_COUNTERS].zero_()
+            ws = torch.empty(2 * _SPLIT_COUNTERS + _SPLIT_FLOATS, dtype=torch.float32, device=self.device)
+            ws[: 2 * _SPLIT_COUNTERS].zero_()
             self._gemm_ws[stream] = ws
         return ws
 
@@ -252,7 +252,7 @@ class NativeOps:
         self._call("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
                    residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha), splits,
-                   _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
+                   _ptr(ws), 4 * (2 * _SPLIT_COUNTERS + _SPLIT_FLOATS), next(self._epoch), _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
         return out
 
     # -- embedding --------------------------------------------------------------------
@@ -454,7 +454,7 @@ class NativeOps:
             splits = 1
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
-                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits, _ptr(ws), 4 * (_SPLIT_COUNTERS + _SPLIT_FLOATS), scale,
+                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits, _ptr(ws), 4 * (2 * _SPLIT_COUNTERS + _SPLIT_FLOATS), next(self._epoch), scale,
                    self.status.data_ptr(), st, n=3)
         return dqkv
 

@@ -54,7 +54,8 @@ inline float __uint_as_float(unsigned u) { float f; memcpy(&f, &u, 4); return f;
 inline void __threadfence() {}
 inline unsigned __shfl_sync(unsigned, unsigned v, int) { return v; }
 inline int __shfl_up_sync(unsigned, int v, int) { return v; }
-inline unsigned atomicAdd(unsigned* p, unsigned v) { const unsigned o = *p; *p += v; return o; }
+inline unsigned long long atomicAdd(unsigned long long* p, unsigned long long v) { const unsigned long long o = *p; *p += v; return o; }
+inline void atomicMax(unsigned long long* p, unsigned long long v) { if (*p < v) *p = v; }
 inline void __stcg(float4* p, float4 v) { *p = v; }
 inline float4 __ldcg(const float4* p) { return *p; }
 #define __expf expf
@@ -85,7 +86,7 @@ static float value(int z, int row, int col) { return static_cast<float>((z * 7 +
 
 // A worker's share of the tiles of [Z, M, N], every `step`-th, through quarter q of 128-row units.
 template <bool OUT_F32, bool SPLIT>
-static int run(int m, int n, int z_count, int first, int step, int q, int splits) {
+static int run(int m, int n, int z_count, int first, int step, int q, int splits, bool stale = false) {
   f32 = OUT_F32; M = m; N = n;
   out.assign(static_cast<size_t>(z_count) * m * n, -1.f);
   groups.clear();
@@ -93,9 +94,11 @@ static int run(int m, int n, int z_count, int first, int step, int q, int splits
   memset(stage, 0, sizeof stage);
   const int tm = (m + 127) / 128, tn = (n + 255) / 256;
   std::vector<float> ws(static_cast<size_t>(tm) * tn * splits * SPLIT_UNIT);
-  std::vector<unsigned> counters(static_cast<size_t>(tm) * tn * 4);
+  // a launch before this one has given up and left arrivals of its own behind
+  std::vector<unsigned long long> counters(static_cast<size_t>(tm) * tn * 4);
+  for (size_t i = 0; i < counters.size(); ++i) counters[i] = stale ? (41ull << 16) + 1 + i % 3 : 0;
   EpiParams p{};
-  p.M = m; p.N = n; p.alpha = 1.f; p.splits = splits; p.ws = ws.data(); p.counters = counters.data();
+  p.M = m; p.N = n; p.alpha = 1.f; p.splits = splits; p.ws = ws.data(); p.counters = counters.data(); p.epoch = 42;
   EpiOut o{nullptr, stage, z_count > 1 ? 0 : -1, 0};
   for (int w = first; w < tm * tn * z_count; w += step) {
     const int z = w / (tm * tn), t = w % (tm * tn), row0 = t % tm * 128, tn0 = t / tm * 256;
@@ -112,7 +115,7 @@ static int run(int m, int n, int z_count, int first, int step, int q, int splits
     if (row >= m) continue;
     for (int c = tn0; c < n && c < tn0 + 256; ++c) bad += out[(static_cast<size_t>(z) * m + row) * n + c] != value(z, row, c);
   }
-  for (unsigned c : counters) bad += c != 0;
+  if (!stale) for (unsigned long long c : counters) bad += c != 0;
   return bad;
 }
 }
@@ -122,7 +125,8 @@ int main() {
   const int ms[] = {128, 129, 161, 193, 225, 256, 385, 33, 8}, ns[] = {64, 72, 256, 320, 768, 1032};
   for (int m : ms) for (int n : ns) for (int q = 0; q < 4; ++q) for (int step = 1; step <= 3; ++step) {
     const int b = run<false, false>(m, n, 1, 0, step, q, 1) + run<true, false>(m, n, 1, 0, step, q, 1) + run<false, true>(m, n, 1, 0, step, q, 3)
-                  + run<true, true>(m, n, 1, 0, step, q, 2) + run<false, false>(m, n, 3, 0, step, q, 1);
+                  + run<true, true>(m, n, 1, 0, step, q, 2) + run<false, false>(m, n, 3, 0, step, q, 1)
+                  + run<false, true>(m, n, 1, 0, step, q, 4, true) + run<true, true>(m, n, 1, 0, step, q, 2, true);
     if (b) printf("m %d n %d quarter %d step %d: %d wrong elements\n", m, n, q, step, b);
     total += b;
   }
@@ -135,7 +139,7 @@ int main() {
 @pytest.mark.skipif(shutil.which("g++") is None or not (CUDA_INC / "cuda_bf16.h").exists(), reason="no host compiler or CUDA headers")
 def test_staged_boxes_are_not_overwritten_before_they_are_read(tmp_path):
     """Row counts with quarters past the last row, column counts with odd numbers of boxes, several tiles per worker, both
-    output types, split reductions and one matrix per expert."""
+    output types, split reductions (also behind a launch that gave up) and one matrix per expert."""
     shutil.copy(CSRC / "gemm_epilogue.cuh", tmp_path)
     (tmp_path / "ptx.cuh").write_text(PTX)
     (tmp_path / "main.cpp").write_text(MAIN)

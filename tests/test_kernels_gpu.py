@@ -857,3 +857,30 @@ def test_column_sums_forms(ops, T, N):
     ref = x.double().sum(0)
     # one rounding to bf16, and fp32 sums whose terms have the size of the column's norm
     assert ((out.double() - ref).abs() <= ref.abs() * 2 ** -8 + x.double().pow(2).sum(0).sqrt() * 1e-5).all()
+
+
+def test_split_launches_behind_one_that_gave_up(ops):
+    """Arrivals that a launch which gave up has left in the counters do not count in the launches after it."""
+    torch.manual_seed(5)
+    M, N, K = 136, 264, 4096
+    a, b = bf(M, K), bf(N, K, scale=0.1)
+    lens, hq, hkv, D = [300, 200], 8, 2, 64
+    T = sum(lens)
+    qkv, dout = bf(T, (hq + 2 * hkv) * D), bf(T, hq * D)
+    cu_host, cu = _cu(lens)
+    out, lse = ops.attention(qkv, cu, cu_host, max(lens), hq, hkv, D)
+
+    def both():
+        o = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.gemm(a, False, b, False, o, M, N, K)
+        return o, ops.attention_bwd(dout, qkv, out, lse, cu, cu_host, max(lens), hq, hkv, D)[:, hq * D:]
+    first = both()
+    counters = ops._split_workspace(ops._st())[: 8192].view(torch.int64)
+    assert not counters.any()
+    epoch = next(ops._epoch)
+    for stale in (1, 3, 7):
+        counters.fill_((epoch << 16) + stale)
+        for x, y in zip(both(), first):
+            assert torch.equal(x, y)
+    counters.zero_()
+    ops.check_status()

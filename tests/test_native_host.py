@@ -1,4 +1,6 @@
 """Host side of the native backend (choice of kernels, workspaces, plans) with stand-ins for the library's launches: no GPU."""
+import itertools
+
 import pytest
 import torch
 
@@ -12,6 +14,7 @@ def make_ops(**fakes):
     ops.use_gemm2, ops.pair_max_flops, ops.sms = False, 1e12, 148
     ops.status = torch.zeros(1, dtype=torch.int32)
     ops._scratch, ops._gemm_ws, ops._attn_plan_cache, ops._pairs = {}, {}, {}, None
+    ops._epoch = itertools.count(1)
     ops.calls = []
     fakes.setdefault("mtb200_gemm2_pairs", lambda: 74)
 

@@ -93,7 +93,7 @@ static int run(int m, int n, int z_count, int first, int step, int q, int splits
   alignas(1024) static uint8_t stage[2 * STORE_BOX];
   memset(stage, 0, sizeof stage);
   const int tm = (m + 127) / 128, tn = (n + 255) / 256;
-  std::vector<float> ws(static_cast<size_t>(tm) * tn * splits * SPLIT_UNIT);
+  std::vector<float> ws(static_cast<size_t>(tm) * tn * splits * SPLIT_UNIT, NAN);   // read before it is written: not a number
   // a launch before this one has given up and left arrivals of its own behind
   std::vector<unsigned long long> counters(static_cast<size_t>(tm) * tn * 4);
   for (size_t i = 0; i < counters.size(); ++i) counters[i] = stale ? (41ull << 16) + 1 + i % 3 : 0;
@@ -104,7 +104,7 @@ static int run(int m, int n, int z_count, int first, int step, int q, int splits
     const int z = w / (tm * tn), t = w % (tm * tn), row0 = t % tm * 128, tn0 = t / tm * 256;
     if (z_count > 1) o.z = z;
     for (int s = 0; s < splits; ++s) {
-      for (int c = 0; c < 256; ++c) tmem[c] = s == 0 ? value(z, row0 + q * 32, tn0 + c) : 0.f;
+      for (int c = 0; c < 256; ++c) tmem[c] = s == splits - 1 ? value(z, row0 + q * 32, tn0 + c) : 0.f;
       epilogue_quarter<OUT_F32, SPLIT, false, false>(p, o, 0, row0, tn0, q, 0, t, s, false);
     }
   }

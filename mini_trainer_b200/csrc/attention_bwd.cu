@@ -541,16 +541,15 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
 
 // plan: key-block work table [n_items, 3] = (seq_start, seq_len, k0), most work first.
 // dq_acc: zero-initialised fp32 [T, Hq*D] scratch; delta: fp32 [Hq, T] scratch.
-// splits: CTAs that share the query heads of a key block; more than one needs ws, a workspace of ws_bytes as the split-K GEMM's (its first
-// SPLIT_COUNTER_BYTES are zero before the first launch) and an epoch that grows with every launch.
+// splits: CTAs that share the query heads of a key block; more than one needs counters, an epoch and scratch as the split-K GEMM does.
 extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, long long ldo, const void* dout, long long lddo,
                                void* dqkv, long long ldq, const float* lse, float* delta, float* dq_acc, const int* plan,
-                               int n_items, int T, int Hq, int Hkv, int D, int splits, float* ws, long long ws_bytes, unsigned long long epoch, float scale, int* status, cudaStream_t st) {
+                               int n_items, int T, int Hq, int Hkv, int D, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float scale, int* status, cudaStream_t st) {
   using namespace mtb;
   if (n_items <= 0 || T <= 0) return 0;
   if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8 || lddo % 8 || ldq % 8 || splits < 1 || splits > Hq / Hkv) return -10;
   const long long units = static_cast<long long>(n_items) * Hkv;
-  if (splits > 1 && (ws == nullptr || units * 8 > SPLIT_COUNTERS || splits * units * 2 * AB_B * D * 4 > ws_bytes - SPLIT_COUNTER_BYTES)) return -11;
+  if (splits > 1 && (part == nullptr || counters == nullptr || units * 8 > SPLIT_COUNTERS || splits * units * 2 * AB_B * D * 4 > part_bytes)) return -11;
   CUtensorMap tq, tdo, tdq;
   int rc = make_tmap_2d_bf16(&tq, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
   if (rc) return rc;
@@ -562,7 +561,7 @@ extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, l
   attn_delta_kernel<<<static_cast<int>((delta_threads + 255) / 256), 256, 0, st>>>(
       reinterpret_cast<const __nv_bfloat16*>(out), ldo, reinterpret_cast<const __nv_bfloat16*>(dout), lddo, delta, T, Hq, D);
   AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, splits,
-                 ws == nullptr ? nullptr : ws + SPLIT_COUNTER_BYTES / 4, reinterpret_cast<unsigned long long*>(ws), epoch, scale, status};
+                 part, counters, epoch, scale, status};
   rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, p, n_items, st);
   if (rc) return rc;
   attn_dq_store_kernel<<<dim3(static_cast<unsigned>(T), (Hq * D / 8 + 255) / 256), 256, 0, st>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, T, Hq * D);

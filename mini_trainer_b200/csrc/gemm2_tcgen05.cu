@@ -308,7 +308,7 @@ static int co_resident_pairs() {
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
-                  long long ws_bytes = 0) {
+                  long long part_bytes = 0) {
   auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA>;
   constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS;
   static bool configured = false;
@@ -319,11 +319,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int pairs = co_resident_pairs<GATHER>();
   if (pairs <= 0) return -6;
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
-  if (p.e.splits > 1) {   // the arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest
-    if (!split_fits(p.e, 2 * tiles, (p.K + BK - 1) / BK, ws_bytes)) return -11;
-    p.e.counters = reinterpret_cast<unsigned long long*>(p.e.ws);
-    p.e.ws += SPLIT_COUNTER_BYTES / 4;
-  }
+  if (p.e.splits > 1 && !split_fits(p.e, 2 * tiles, (p.K + BK - 1) / BK, part_bytes)) return -11;
   // the gathering variant always uses every pair: its extra warps carry the transfer
   const int items = tiles * p.e.splits;
   p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
@@ -357,7 +353,7 @@ int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
 
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                      float alpha, int splits, float* ws, long long ws_bytes, unsigned long long epoch, float2* stats, int* status, cudaStream_t stream) {
+                      float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   using namespace mtb::g2;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -372,17 +368,17 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
   if (rc) return rc - 10;
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
-  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr, epoch}};
+  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, part, stats, counters, epoch}};
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
-      case 0: return launch<false, false, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-      case 1: return launch<false, true, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-      case 2: return launch<true, false, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-      default: return launch<true, true, false, false, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+      case 0: return launch<false, false, false, false, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+      case 1: return launch<false, true, false, false, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+      case 2: return launch<true, false, false, false, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+      default: return launch<true, true, false, false, true>(ta, tb, td, p, stream, nullptr, part_bytes);
     }
   }
-#define GEMM2(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, ws_bytes) \
-                                                              : launch<X, Y, Z, false, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes)
+#define GEMM2(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, part_bytes) \
+                                                              : launch<X, Y, Z, false, false, false>(ta, tb, td, p, stream, nullptr, part_bytes)
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
     case 0: GEMM2(false, false, false);

@@ -28,7 +28,6 @@ struct EpiParams {
 };
 
 constexpr int SPLIT_COUNTERS = 4096;
-constexpr int SPLIT_COUNTER_BYTES = SPLIT_COUNTERS * 8;
 constexpr int SPLIT_UNIT = 128 * 256;   // floats of one partial: 128 rows x 256 columns
 
 // Arrival at a counter (one thread); true for the last of the launch's `splits` arrivals. The two operations of a thread on one
@@ -264,10 +263,10 @@ __device__ __forceinline__ void fill_group_table(GroupTable& tab, const GroupPar
   if (lane == 0) tab.tile_start[g.E] = base;
 }
 
-// Whether a split launch over `units` 128-row units fits its workspace and leaves every item a k-block.
-inline bool split_fits(const EpiParams& e, long long units, int kblocks, long long ws_bytes) {
-  return e.ws != nullptr && e.splits <= kblocks && units * 4 <= SPLIT_COUNTERS &&
-         units * e.splits * SPLIT_UNIT * 4 <= ws_bytes - SPLIT_COUNTER_BYTES;
+// Whether a split launch over `units` 128-row units fits its scratch and leaves every item a k-block.
+inline bool split_fits(const EpiParams& e, long long units, int kblocks, long long part_bytes) {
+  return e.ws != nullptr && e.counters != nullptr && e.splits <= kblocks && units * 4 <= SPLIT_COUNTERS &&
+         units * e.splits * SPLIT_UNIT * 4 <= part_bytes;
 }
 
 }  // namespace mtb

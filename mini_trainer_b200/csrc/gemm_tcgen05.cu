@@ -382,7 +382,7 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmParams p, cudaStream_t stream,
-                  const GatherParams* gp = nullptr, long long ws_bytes = 0, const GroupParams* grp = nullptr) {
+                  const GatherParams* gp = nullptr, long long part_bytes = 0, const GroupParams* grp = nullptr) {
   static bool configured = false;
   auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS, EXTRA>;
   if (!configured) {
@@ -396,11 +396,7 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   }
   int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   if (GROUP == GROUP_REDUCE) tiles *= grp->E;
-  if (p.e.splits > 1) {   // the arrival counters fill the first SPLIT_COUNTER_BYTES of the workspace, the partials the rest
-    if (!split_fits(p.e, tiles, (p.K + BK - 1) / BK, ws_bytes)) return -11;
-    p.e.counters = reinterpret_cast<unsigned long long*>(p.e.ws);
-    p.e.ws += SPLIT_COUNTER_BYTES / 4;
-  }
+  if (p.e.splits > 1 && !split_fits(p.e, tiles, (p.K + BK - 1) / BK, part_bytes)) return -11;
   // the gathering variant always uses every SM: its extra warps carry the transfer
   const int items = tiles * p.e.splits;
   const int grid = (GATHER || items >= g_num_sms) ? g_num_sms : items;
@@ -417,13 +413,13 @@ extern "C" {
 //   a_mn = 0: A is row-major [M, K] (lda >= K);  a_mn = 1: A is row-major [K, M] (lda >= M)
 //   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
 //   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
-//   splits: work items per output tile (ops/gemm_plan.py); more than one needs ws, an fp32 workspace of ws_bytes: its first
-//   SPLIT_COUNTER_BYTES are zero before the first call, and launches that may overlap have one each. epoch (splits > 1): grows with every launch
+//   splits: work items per output tile (ops/gemm_plan.py); more than one needs counters (SPLIT_COUNTERS words, zero before the first
+//   call; launches that may overlap have their own), an epoch that grows with every launch on them, and part, fp32 scratch of part_bytes
 //   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
 // Returns 0 on success, a negative code on invalid arguments or launch failure.
 int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                     float alpha, int splits, float* ws, long long ws_bytes, unsigned long long epoch, float2* stats, int* status, cudaStream_t stream) {
+                     float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32) || splits < 1) return -10;
@@ -438,17 +434,17 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
   GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, ws, stats, nullptr, epoch}};
+               EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, part, stats, counters, epoch}};
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
-      case 0: return launch<false, false, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-      case 1: return launch<false, true, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-      case 2: return launch<true, false, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
-      default: return launch<true, true, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, ws_bytes);
+      case 0: return launch<false, false, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+      case 1: return launch<false, true, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+      case 2: return launch<true, false, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+      default: return launch<true, true, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
     }
   }
-#define GEMM(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, ws_bytes) \
-                                                             : launch<X, Y, Z, false, false, GROUP_NONE, false, false>(ta, tb, td, p, stream, nullptr, ws_bytes)
+#define GEMM(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, part_bytes) \
+                                                             : launch<X, Y, Z, false, false, GROUP_NONE, false, false>(ta, tb, td, p, stream, nullptr, part_bytes)
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
     case 0: GEMM(false, false, false);

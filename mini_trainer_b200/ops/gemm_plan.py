@@ -19,6 +19,11 @@ _ONE = (1.7, 0.45, 4.8, 7.0, 4.2, 1.32)
 _PAIR = (2.5, 0.33, 5.0, 7.4, 3.9, 1.47)
 
 
+def partial_bytes(M: int, N: int, pair: bool, splits: int) -> int:
+    """Scratch of a split launch."""
+    return -(-N // 256) * (2 * -(-M // 256) if pair else -(-M // 128)) * splits * UNIT_BYTES
+
+
 def _best_split(tiles: int, units: int, kblocks: int, workers: int, max_units: int, t: tuple):
     launch, block, item, least, split, partial = t
     best = launch + -(-tiles // workers) * max(kblocks * block + item, least)
@@ -35,7 +40,7 @@ def _best_split(tiles: int, units: int, kblocks: int, workers: int, max_units: i
 @functools.lru_cache(maxsize=4096)
 def choose(M: int, N: int, K: int, sms: int, pairs: int, one: bool, max_units: int, max_counted: int) -> tuple:
     """``(two_cta, splits)`` for an ``M x N x K`` product. ``pairs``: CTA pairs that may be used (0: none); ``one``: single CTAs may be.
-    ``max_units``: partials the workspace holds, ``max_counted``: 128-row units it has counters for."""
+    ``max_units``: partials the scratch may hold, ``max_counted``: 128-row units it has counters for."""
     kblocks, cols = -(-K // BK), -(-N // 256)
     t1, t2 = -(-M // 128) * cols, -(-M // 256) * cols
     best = None

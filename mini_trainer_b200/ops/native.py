@@ -48,8 +48,8 @@ P, I, L, F, U = c_void_p, c_int, c_longlong, c_float, c_ulonglong
 
 
 class _Sig:
-    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, U, P, P, P]
-    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, L, U, P, P, P]
+    mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, U, P, L, P, P, P]
+    mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, U, P, L, P, P, P]
     mtb200_gemm2_pairs = []
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
     mtb200_norm_bwd_blocks = [I, I]
@@ -85,12 +85,12 @@ class _Sig:
     mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
     mtb200_attn_fwd_one = [P, L, P, L, P, P, I, I, I, I, I, F, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
-    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, L, U, F, P, P]
+    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, U, P, L, F, P, P]
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
-_SPLIT_COUNTERS = 4096          # 8-byte words in front of the partials (csrc/gemm_epilogue.cuh)
-_SPLIT_FLOATS = 32 << 20        # partials: 128 MB
+_SPLIT_COUNTERS = 4096          # csrc/gemm_epilogue.cuh
+_SPLIT_FLOATS = 32 << 20        # most that the partials of a launch take: 128 MB
 _SPLIT_UNITS = 4 * _SPLIT_FLOATS // gemm_plan.UNIT_BYTES   # = 1024 of 128 x 256
 NATIVE_HEAD_DIMS = (64, 128)   # head dimensions of the hand-written attention kernels
 
@@ -137,7 +137,7 @@ class NativeOps:
         self.launches = 0
         self.profile = [] if os.environ.get("MTB200_PROFILE") else None
         self._scratch = {}
-        self._gemm_ws = {}   # stream handle -> split-K workspace
+        self._gemm_ws = {}   # stream handle -> arrival counters of split launches
         self._epoch = itertools.count(1)   # of the launches that may split
         self._attn_plan_cache = {}
         self._pairs = None
@@ -216,20 +216,32 @@ class NativeOps:
         return self._pairs
 
     def _split_workspace(self, stream):
-        """Split-K workspace of a stream: arrival counters and fp32 partials. GEMMs of one stream run
-        one after the other, those of different streams may overlap, so each stream has its own (the last eight streams do;
-        a dropped one goes back to its stream's pool, behind the launches that use it). ``None`` under capture: a graph may be
-        replayed beside anything, so its launches never split."""
+        """Arrival counters of a stream's split launches (32 KB). Launches of one stream run one after the other, those of different
+        streams may overlap, so each stream has its own (the last eight streams do; dropped ones go back to their stream's
+        pool, behind the launches that use them). ``None`` under capture: a graph may be replayed beside anything, so its
+        launches never split."""
         if torch.cuda.is_current_stream_capturing():
             return None
         ws = self._gemm_ws.get(stream)
         if ws is None:
             if len(self._gemm_ws) >= 8:
                 self._gemm_ws.pop(next(iter(self._gemm_ws), None), None)
-            ws = torch.empty(2 * _SPLIT_COUNTERS + _SPLIT_FLOATS, dtype=torch.float32, device=self.device)
-            ws[: 2 * _SPLIT_COUNTERS].zero_()
+            ws = torch.zeros(_SPLIT_COUNTERS, dtype=torch.int64, device=self.device)
             self._gemm_ws[stream] = ws
         return ws
+
+    def _split(self, stream, nbytes):
+        """``(counters, epoch, partials)`` of a split launch, or ``None`` where it has to run whole. The partials are scratch of this call:
+        taken from the allocator (in powers of two, at most 128 MB) and given back behind the launch, so nothing is held
+        between calls, and without memory for them the launch simply does not split."""
+        ws = self._split_workspace(stream)
+        if ws is None:
+            return None
+        try:
+            part = torch.empty(max(1 << 18, 1 << (nbytes // 4 - 1).bit_length()), dtype=torch.float32, device=self.device)
+        except torch.OutOfMemoryError:
+            return None
+        return ws, next(self._epoch), part
 
     def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
         """out[M,N] = alpha*A*B (+bias) (+residual). ``a_mn``/``b_mn``: operand stored [K, rows].
@@ -246,13 +258,12 @@ class NativeOps:
             pairs = 0
         pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
         st = self._st()
-        ws = self._split_workspace(st) if splits > 1 else None
-        if ws is None:
-            splits = 1
+        split = self._split(st, gemm_plan.partial_bytes(M, N, pair, splits)) if splits > 1 else None
+        ws, epoch, part = split or (None, 0, None)
         self._call("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
-                   residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha), splits,
-                   _ptr(ws), 4 * (2 * _SPLIT_COUNTERS + _SPLIT_FLOATS), next(self._epoch), _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
+                   residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha), splits if split else 1,
+                   _ptr(ws), epoch, _ptr(part), 4 * part.numel() if split else 0, _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
         return out
 
     # -- embedding --------------------------------------------------------------------
@@ -449,12 +460,11 @@ class NativeOps:
         most = 1 if units * 8 > _SPLIT_COUNTERS else min(hq // hkv, _SPLIT_FLOATS // (units * 2 * 128 * d))
         splits = 1 if most <= 1 else self._per_batch(cu_host, ("splits", hq, hkv, d), lambda: attention_plan.backward_splits(
             attention_plan.blocks_per_sequence(cu_host), hq, hkv, self.sms, most))
-        ws = self._split_workspace(st) if splits > 1 else None
-        if ws is None:
-            splits = 1
+        split = self._split(st, splits * units * 2 * 128 * d * 4) if splits > 1 else None
+        ws, epoch, part = split or (None, 0, None)
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
-                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits, _ptr(ws), 4 * (2 * _SPLIT_COUNTERS + _SPLIT_FLOATS), next(self._epoch), scale,
+                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits if split else 1, _ptr(ws), epoch, _ptr(part), 4 * part.numel() if split else 0, scale,
                    self.status.data_ptr(), st, n=3)
         return dqkv
 

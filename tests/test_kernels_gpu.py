@@ -875,7 +875,7 @@ def test_split_launches_behind_one_that_gave_up(ops):
         ops.gemm(a, False, b, False, o, M, N, K)
         return o, ops.attention_bwd(dout, qkv, out, lse, cu, cu_host, max(lens), hq, hkv, D)[:, hq * D:]
     first = both()
-    counters = ops._split_workspace(ops._st())[: 8192].view(torch.int64)
+    counters = ops._split_workspace(ops._st())
     assert not counters.any()
     epoch = next(ops._epoch)
     for stale in (1, 3, 7):
@@ -883,4 +883,24 @@ def test_split_launches_behind_one_that_gave_up(ops):
         for x, y in zip(both(), first):
             assert torch.equal(x, y)
     counters.zero_()
+    ops.check_status()
+
+
+def test_split_launches_hold_no_scratch(ops):
+    """What a split product takes beyond its output goes back to the allocator; one that does not split takes nothing."""
+    a, b = bf(256, 8192), bf(256, 8192, scale=0.1)
+    out = torch.empty(256, 256, dtype=torch.bfloat16, device="cuda")
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        ops.gemm(a, False, b, False, out, 256, 256, 8192)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        ops.gemm(a, False, b, False, out, 256, 256, 8192)
+        assert torch.cuda.memory_allocated() == before and 0 < torch.cuda.max_memory_allocated() - before <= 8 << 20
+        torch.cuda.reset_peak_memory_stats()
+        ops.gemm(a, False, b, False, out, 256, 256, 256)
+        assert torch.cuda.max_memory_allocated() == before
+    assert all(w.numel() * w.element_size() <= 32768 for w in ops._gemm_ws.values())
+    torch.cuda.synchronize()
     ops.check_status()

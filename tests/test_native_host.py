@@ -24,6 +24,11 @@ def make_ops(**fakes):
     ops._fn = Fns(fakes)
     ops._st = lambda: 0
     ops._split_workspace = lambda st: None
+
+    def _call(name, *args, n=1, tag=None):
+        assert len(args) == len(getattr(native._Sig, name))
+        ops.calls.append((name, args))
+    ops._call = _call
     return ops
 
 
@@ -115,9 +120,9 @@ def test_attention_backward_divides_only_what_the_workspace_holds():
         ops.attention_bwd(o, qkv, o, torch.empty(hq, T), None, cu, max(lens), hq, hkv, d)
         args = ops.calls[-1][1]
         splits, units = args[17], args[12] * hkv
-        assert (splits > 1) == want and (args[18] is not None) == want
+        assert (splits > 1) == want and (args[18] is not None) == want and (args[20] is not None) == want
         if want:
-            assert units * 8 <= 4096 and splits * units * 2 * 128 * d <= 32 << 20
+            assert units * 8 <= 4096 and splits * units * 2 * 128 * d * 4 <= args[21] <= 128 << 20
 
 
 # (M, N, K, pair, whole): a round that only single CTAs fill evenly; two rounds where pairs are the faster per k-block; a few tiles with a
@@ -133,7 +138,8 @@ def test_gemm_choice(M, N, K, pair, whole):
     ops.gemm(a, False, b, False, out, M, N, K)
     name, args = ops.calls[-1]
     assert pair is None or (name == "mtb200_gemm2_bf16") == pair
-    assert (args[16] == 1) == whole and (args[17] is None) == whole
+    assert (args[16] == 1) == whole and (args[17] is None) == whole and (args[19] is None) == whole
+    assert whole or args[20] >= (1 + (args[16] > 1)) * 128 * 256 * 4
     ops._split_workspace = lambda st: None      # as under capture
     ops.gemm(a, False, b, False, out, M, N, K)
     assert ops.calls[-1][0] == name and ops.calls[-1][1][16] == 1
@@ -155,3 +161,21 @@ def test_gemm_choice_keeps_within_the_workspace():
             assert two is False or pairs > 0
             assert two is True or one or pairs == 0
             assert s == 1 or (u <= counted and u * s <= units and 4 * s <= -(-K // 64))
+
+
+def test_split_launch_runs_whole_without_memory_for_its_partials(monkeypatch):
+    ops = make_ops()
+    ops._split_workspace = lambda st: torch.zeros(1)
+    real, taken = torch.empty, []
+
+    def empty(*shape, **kw):
+        if kw.get("dtype") == torch.float32 and len(shape) == 1:
+            taken.append(shape[0])
+            raise torch.OutOfMemoryError("no memory")
+        return real(*shape, **kw)
+    monkeypatch.setattr(torch, "empty", empty)
+    gemm(ops, 128, 256, 4096)
+    assert taken and ops.calls[-1][1][16] == 1 and ops.calls[-1][1][17] is None
+    taken.clear()
+    gemm(ops, 128, 256, 256)      # nothing to split: nothing asked for
+    assert not taken and ops.calls[-1][1][16] == 1

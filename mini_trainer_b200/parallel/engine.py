@@ -28,6 +28,7 @@ from __future__ import annotations
 import contextlib
 import math
 import os
+import time
 from dataclasses import dataclass, field
 from typing import Iterator, Optional
 
@@ -186,6 +187,7 @@ class ShardedEngine:
         self.activation_budget_bytes = activation_budget_bytes
         self._oom_retries = 0
         self._state_bytes = None   # of the groups, which never change size
+        self._free_reading = None  # (free, when, reserved by the allocator then)
         # Reduce a block's gradients tensor region by tensor region while its backward still runs
         # (MTB200_REGION_OVERLAP=0: one reduction per block, after its backward).
         # A mixture-of-experts block is reduced once: its experts' gradients complete in no fixed layout order.
@@ -513,10 +515,24 @@ class ShardedEngine:
             lvl0 += tokens * ((cfg.q_size + cfg.kv_size) * es + (cfg.num_attention_heads + cfg.num_key_value_heads) * 4)
         return lvl1, lvl0
 
-    # A minibatch whose kept activations and working set stay below this (a hundredth of the device) is planned without asking
-    # the driver and the allocator what is free, which costs the host a few hundred microseconds. Should it not fit after
-    # all, the forward pass is run again with every block at the cheapest level, as after any out-of-memory error.
-    ASSUMED_FREE = 2 << 30
+    # Asking the driver what is free takes the host about 0.1 ms, a tenth of a small model's step. Its answer is therefore used for up to
+    # a second, with what the allocator has taken or returned since, as long as that leaves this much more than the minibatch
+    # wants: another process would have to take it within the second. (An out-of-memory error is only repaired in forward.)
+    FREE_READING_S, FREE_READING_MARGIN = 1.0, 8 << 30
+
+    def _free_bytes(self, needed: int) -> int:
+        """Device memory that can be had: what the driver reports as free plus the allocator's cached blocks."""
+        stats = torch.cuda.memory.memory_stats_as_nested_dict(self.device)   # (the flat form of the same takes ten times as long)
+        reserved, allocated = (stats[k]["all"]["current"] if stats else 0 for k in ("reserved_bytes", "allocated_bytes"))
+        now = time.monotonic()
+        if self._free_reading is not None and not self._oom_retries:
+            free, then, reserved_then = self._free_reading
+            estimate = free + reserved_then - allocated
+            if now - then <= self.FREE_READING_S and estimate >= needed + self.FREE_READING_MARGIN:
+                return estimate
+        free, _ = torch.cuda.mem_get_info(self.device)
+        self._free_reading = (free, now, reserved)
+        return free + reserved - allocated
 
     def _auto_activation_budget(self, tokens: int, wanted: int) -> int:
         """Memory that can hold extra saved activations. Two bounds, the smaller wins:
@@ -544,11 +560,8 @@ class ShardedEngine:
         if self._state_bytes is None:
             self._state_bytes = self.state_bytes()
         static = int(0.93 * total - (self._state_bytes + transient + bufs + (4 << 30)))
-        if wanted + transient <= self.ASSUMED_FREE and wanted <= static and not self._oom_retries and (self.world == 1 or self.symmetric):
-            return static
-        free, _ = torch.cuda.mem_get_info(self.device)
-        cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
-        live = int(0.97 * (free + cached) - transient - (3 << 30))
+        needed = int((wanted + transient + (3 << 30)) / 0.97) + 1
+        live = int(0.97 * self._free_bytes(needed) - transient - (3 << 30))
         if self._oom_retries:   # an earlier microbatch ran out of memory: plan more cautiously from now on
             live -= self._oom_retries * (8 << 30)
         return min(static, live)

@@ -6,7 +6,7 @@ one node"): how many bytes of parameters, master weights, moments and gradient a
 holds, which moment precision ``--optimizer-state-dtype auto`` will pick, how large the gathered
 block buffers are, what a minibatch of the given token budget costs per checkpoint level, and how
 many blocks can keep their activations. It uses the same formulas as the engine
-(``parallel.engine.plan_state_dtype``, ``ShardedEngine.plan_checkpointing``); nothing is allocated.
+(``parallel.engine``: ``plan_state_dtype``, ``kept_bytes``, ``working_set_bytes``); nothing is allocated.
 """
 from __future__ import annotations
 
@@ -22,7 +22,7 @@ def memory_plan(cfg, gpus: int, max_tokens_per_gpu: int, hbm_gb: float = 183.0, 
     import torch
 
     from ..models import layout as L
-    from ..parallel.engine import plan_state_dtype
+    from ..parallel.engine import kept_bytes, plan_state_dtype, working_set_bytes
     hbm = hbm_gb * 2 ** 30
     if state_dtype == "auto":
         moments = plan_state_dtype(cfg, gpus, hbm, max_tokens_per_gpu)
@@ -39,11 +39,9 @@ def memory_plan(cfg, gpus: int, max_tokens_per_gpu: int, hbm_gb: float = 183.0, 
                + 2 * block * 2                    # two block gradient buffers
                + (layouts[0].padded_numel + layouts[-1].padded_numel) * 2 * 2)   # embed / head: gathered and gradient
     t, h, es = max_tokens_per_gpu, cfg.hidden_size, 2
-    f = (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
     inputs = t * h * es * cfg.num_hidden_layers
-    lvl1 = t * (cfg.q_size * es + cfg.num_attention_heads * 4)
-    lvl0 = lvl1 + t * ((h + cfg.qkv_size + 2 * f) * es + 8)
-    work = t * es * (7 * h + cfg.qkv_size + 6 * f)
+    lvl1, lvl0 = kept_bytes(cfg, t, es)
+    work = working_set_bytes(cfg, t, es)
     ce = 8192 * cfg.vocab_size * 2 + cfg.vocab_size * h * 4
     free = 0.93 * hbm - state - buffers - inputs - work - ce - 4 * 2 ** 30
     keep_attn = max(0, min(cfg.num_hidden_layers, int(free // lvl1))) if free > 0 else 0

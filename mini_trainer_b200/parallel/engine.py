@@ -502,18 +502,7 @@ class ShardedEngine:
 
     def _kept_bytes(self, tokens: int) -> tuple:
         """Bytes a block keeps beyond its input at checkpoint levels 1 and 0."""
-        cfg = self.cfg
-        es = 2 if self.param_dtype != torch.float32 else 4
-        h, f = cfg.hidden_size, (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
-        lvl1 = tokens * (cfg.q_size * es + cfg.num_attention_heads * 4)
-        # level 0 keeps qkv, the attention output, h1 and gate/up (the normalised inputs and the SwiGLU
-        # output are rebuilt in backward by elementwise kernels)
-        lvl0 = lvl1 + tokens * ((h + cfg.qkv_size + 2 * f) * es + 8)
-        if cfg.post_norm:   # both branch outputs before their norms and the q|k projections before theirs
-            lvl0 += tokens * (2 * h + cfg.q_size + cfg.kv_size) * es
-        if cfg.qk_norm:   # the q|k heads before their norm and one reciprocal RMS per head
-            lvl0 += tokens * ((cfg.q_size + cfg.kv_size) * es + (cfg.num_attention_heads + cfg.num_key_value_heads) * 4)
-        return lvl1, lvl0
+        return kept_bytes(self.cfg, tokens, 2 if self.param_dtype != torch.float32 else 4)
 
     # Asking the driver what is free takes the host about 0.1 ms, a tenth of a small model's step. Its answer is therefore used for up to
     # a second, with what the allocator has taken or returned since, as long as that leaves this much more than the minibatch
@@ -550,9 +539,8 @@ class ShardedEngine:
         cfg = self.cfg
         total = torch.cuda.get_device_properties(self.device).total_memory
         h, v = cfg.hidden_size, cfg.vocab_size
-        f = (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
         base = tokens * 2 * h * len(self.blocks)
-        work = tokens * 2 * (7 * h + cfg.qkv_size + 6 * f)
+        work = working_set_bytes(cfg, tokens)
         ce = getattr(self.ops, "ce_chunk", 2048) * v * 2 + v * h * 4
         root = 4 * v * h * 2
         bufs = sum(b.numel() * b.element_size() for b in self._pbufs + self._gbufs)
@@ -862,6 +850,38 @@ class ShardedEngine:
 
     def state_bytes(self) -> int:
         return sum(g.state_bytes() for g in self.groups)
+
+
+def routed_rows(cfg: ModelConfig, tokens: int) -> int:
+    """Height of the row buffers of a mixture-of-experts layer: a row per token and chosen expert, each expert's rows padded to a multiple
+    of 128, at the worst split of the tokens."""
+    return -(-(tokens * cfg.num_experts_per_tok + 127 * cfg.num_local_experts) // 128) * 128
+
+
+def kept_bytes(cfg: ModelConfig, tokens: int, es: int = 2) -> tuple:
+    """Bytes a block keeps beyond its input at checkpoint levels 1 (attention output) and 0 (every GEMM output)."""
+    h = cfg.hidden_size
+    lvl1 = tokens * (cfg.q_size * es + cfg.num_attention_heads * 4)
+    # level 0 keeps qkv, the attention output, h1 and gate/up (the normalised inputs and the SwiGLU
+    # output are rebuilt in backward by elementwise kernels)
+    gate_up = 2 * (routed_rows(cfg, tokens) * cfg.expert_intermediate_size if cfg.is_moe else tokens * cfg.intermediate_size)
+    lvl0 = lvl1 + tokens * ((h + cfg.qkv_size) * es + 8) + gate_up * es
+    if cfg.post_norm:   # both branch outputs before their norms and the q|k projections before theirs
+        lvl0 += tokens * (2 * h + cfg.q_size + cfg.kv_size) * es
+    if cfg.qk_norm:   # the q|k heads before their norm and one reciprocal RMS per head
+        lvl0 += tokens * ((cfg.q_size + cfg.kv_size) * es + (cfg.num_attention_heads + cfg.num_key_value_heads) * 4)
+    return lvl1, lvl0
+
+
+def working_set_bytes(cfg: ModelConfig, tokens: int, es: int = 2) -> int:
+    """Working set of one block's backward, with the partial sums of a product that is split."""
+    h = cfg.hidden_size
+    f = (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
+    work = tokens * es * (7 * h + cfg.qkv_size + 6 * f)
+    if cfg.is_moe:   # all experts' rows at once: gathered output gradient, gradient of the activation, of gate/up, then of the inputs
+        fe = cfg.expert_intermediate_size
+        work = max(work, tokens * es * (7 * h + cfg.qkv_size) + routed_rows(cfg, tokens) * es * max(h + 3 * fe, 2 * h + 2 * fe))
+    return work + (128 << 20)
 
 
 def plan_state_dtype(cfg: ModelConfig, world: int, hbm_bytes: float, tokens: int) -> torch.dtype:

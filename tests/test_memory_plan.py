@@ -78,3 +78,31 @@ def test_an_older_reading_changes_no_plan(monkeypatch):
             again = eng.plan_checkpointing(tokens)
             eng._free_reading = None
             assert eng.plan_checkpointing(tokens) == first == again
+
+
+@pytest.mark.parametrize("tokens", [1, 200, 4096, 64000])
+def test_plan_counts_the_rows_that_experts_are_padded_to(tokens):
+    """A mixture-of-experts block keeps, and works on, row buffers with each expert's rows padded to 128."""
+    from dataclasses import replace
+    from mini_trainer_b200.cli.plan import memory_plan
+    cfg = replace(get_preset("mixtral-8x7b"), num_local_experts=128, num_experts_per_tok=8, hidden_size=2048, intermediate_size=768, moe_intermediate_size=768)
+    f, h, es = cfg.expert_intermediate_size, cfg.hidden_size, 2
+    rows = -(-(tokens * 8 + 128 * 127) // 128) * 128      # what the slabs are allocated with
+    lvl1, lvl0 = E.kept_bytes(cfg, tokens)
+    assert lvl0 - lvl1 >= rows * 2 * f * es + tokens * (h + cfg.qkv_size) * es
+    # backward: gathered output gradient, gradient of the activation and of gate/up; then that of gate/up, of the gathered inputs
+    # and the gathered inputs themselves; beside the layer's input, output gradient and input gradient
+    assert E.working_set_bytes(cfg, tokens) >= rows * es * max(h + 3 * f, 2 * h + 2 * f) + 3 * tokens * h * es + (128 << 20)
+    eng = planner("mixtral-8x7b")
+    eng.cfg = cfg
+    assert eng._kept_bytes(tokens) == (lvl1, lvl0)
+    plan = memory_plan(cfg, 8, tokens)
+    assert plan["per_block_gb"]["keep_every_gemm_output"] == round(lvl0 / 2 ** 30, 2)
+
+
+def test_plan_of_a_dense_block_is_what_it_was():
+    cfg, t = get_preset("qwen2.5-1.5b"), 6000
+    lvl1, lvl0 = E.kept_bytes(cfg, t)
+    assert lvl1 == t * (cfg.q_size * 2 + cfg.num_attention_heads * 4)
+    assert lvl0 == lvl1 + t * ((cfg.hidden_size + cfg.qkv_size + 2 * cfg.intermediate_size) * 2 + 8)
+    assert E.working_set_bytes(cfg, t) == t * 2 * (7 * cfg.hidden_size + cfg.qkv_size + 6 * cfg.intermediate_size) + (128 << 20)

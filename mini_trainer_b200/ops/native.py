@@ -638,6 +638,7 @@ class NativeOps:
         stats = self._buf("ce_stats", ck * -(-V // 256) * 2, torch.float32)
         # one chunk: its weight gradient is the whole sum, rounded (or added to what is there) in the GEMM's epilogue
         whole = T <= ck and dw_out.is_contiguous()
+        dw = dw_out.view(V, H) if whole else None
         dw32 = None if whole else self._buf("ce_dw", V * H, torch.float32).view(V, H)
         first = True
         for a in range(0, T, ck):
@@ -647,7 +648,7 @@ class NativeOps:
                        loss[a:a + n].data_ptr(), logits.data_ptr(), V, n, V, float(grad_scale), ignore_index, self._st())
             self.gemm(logits, False, w, True, dx[a:a + n], n, H, V, alpha=logit_scale)
             if whole:
-                self.gemm(logits, True, x, True, dw_out, V, H, n, residual=dw_out if accumulate_dw else None, alpha=logit_scale)
+                self.gemm(logits, True, x, True, dw, V, H, n, residual=dw if accumulate_dw else None, alpha=logit_scale)
             else:
                 self.gemm(logits, True, x[a:a + n], True, dw32, V, H, n, residual=None if first else dw32, alpha=logit_scale)
             first = False

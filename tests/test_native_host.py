@@ -179,3 +179,22 @@ def test_split_launch_runs_whole_without_memory_for_its_partials(monkeypatch):
     taken.clear()
     gemm(ops, 128, 256, 256)      # nothing to split: nothing asked for
     assert not taken and ops.calls[-1][1][16] == 1
+
+
+def test_linear_ce_takes_a_flat_weight_gradient():
+    """``dw_out`` is written as V x H whatever its shape, in one chunk of tokens as in several."""
+    ops = make_ops()
+    T, H, V = 24, 64, 512
+    x, w, t = torch.empty(T, H, dtype=torch.bfloat16), torch.empty(V, H, dtype=torch.bfloat16), torch.zeros(T, dtype=torch.int64)
+    for chunk in (64, 8):
+        ops.ce_chunk = chunk
+        for dw in (torch.empty(V, H, dtype=torch.bfloat16), torch.empty(V * H, dtype=torch.bfloat16)):
+            for acc in (False, True):
+                ops.calls.clear()
+                ops.linear_ce(x, w, t, 1.0, dw, accumulate_dw=acc)
+                name, args = [c for c in ops.calls if c[1][0] == dw.data_ptr() or (len(c[1]) > 6 and c[1][6] == dw.data_ptr())][-1]
+                if chunk >= T:
+                    assert name.startswith("mtb200_gemm") and args[7] == H and args[12:15] == (V, H, T)
+                    assert (args[9] == dw.data_ptr() and args[10] == H) if acc else args[9] is None
+                else:
+                    assert name == "mtb200_f32_to_bf16" and args[2:4] == (V * H, int(acc))

@@ -821,6 +821,13 @@ class ShardedEngine:
         e1.record(cur)
         _Side.stalls.append((e0, e1))
 
+    def check_status(self) -> None:
+        """Raises if a kernel since the last call gave up on a wait or met an input it had to skip: its output, and what was
+        computed from it, is not to be used. Reads a word or two from the device, so call it where the host waits anyway."""
+        for part in (self.ops, self.comm):
+            if hasattr(part, "check_status"):
+                part.check_status()
+
     def zero_grad(self) -> None:
         for g in self.groups:
             g.has_grad = False

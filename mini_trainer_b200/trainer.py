@@ -191,8 +191,9 @@ def train(model: ShardedEngine, optimizer, lr_scheduler: LRSchedule, data_loader
         step += 1
         batches_consumed += 1
         grad_norm = take_gradient_step(model, optimizer, lr_scheduler)
-        # the single device->host read of the step
+        # the single point of the step at which the host waits for the device
         local_loss = float(loss_sum.item())
+        model.check_status()
         batch_totals.accumulate_minibatch_metrics(loss=local_loss,
                                                   loss_backward=local_loss / max(1, batch_num_loss_counted_tokens))
         batch_totals.reduce_batch_metrics(device)

@@ -904,3 +904,55 @@ def test_split_launches_hold_no_scratch(ops):
     assert all(w.numel() * w.element_size() <= 32768 for w in ops._gemm_ws.values())
     torch.cuda.synchronize()
     ops.check_status()
+
+
+# the parts of a routed layer that a Mixtral leaves out: a shared expert behind a sigmoid gate, a branch multiplier, weights that are not
+# renormalised over the chosen experts; alone and together, with idle experts and sizes off the tile edges
+@pytest.mark.parametrize("shared,rm,renorm", [(72, 1.0, True), (0, 0.22, True), (0, 1.0, False), (136, 0.22, False)])
+@pytest.mark.parametrize("T,H,F,E,k,popular", [(300, 264, 136, 8, 2, 5), (65, 128, 72, 40, 4, 40)])
+def test_grouped_experts_shared_scaled_unnormalised(ops, T, H, F, E, k, popular, shared, rm, renorm):
+    from dataclasses import replace
+    from mini_trainer_b200.models import layout as L, moe as M
+    cfg, p0, _, n2, h1, dout = _moe_layer(T, H, F, E, k, popular, seed=3)
+    cfg = replace(cfg, residual_multiplier=rm, norm_topk_prob=renorm, shared_expert_intermediate_size=shared or None,
+                  model_type="qwen2_moe" if shared else "mixtral")
+    entries = [(n, tuple(w.shape)) for n, w in p0.items()]
+    if shared:
+        entries += [("wgus", (2 * shared, H)), ("wds", (H, shared)), ("wsg", (1, H))]
+    lay = L.GroupLayout("x", entries, 1)
+    p = lay.views(bf(lay.padded_numel, scale=0.05))
+    for n, w in p0.items():
+        p[n].copy_(w)
+    res, grads = {}, {}
+    try:
+        for name in ("grouped", "loop"):
+            if name == "loop":
+                ops.expert_stack = lambda *a: None
+            pp = p if name == "grouped" else {n: w.clone() for n, w in p.items()}
+            grads[name] = lay.views(torch.full((lay.padded_numel,), float("nan"), dtype=torch.bfloat16, device="cuda"))
+            out, st = M.moe_forward(ops, cfg, pp, n2, h1, True, False)
+            assert (st.slabs is not None) == (name == "grouped")
+            res[name] = (out, M.moe_backward(ops, cfg, pp, grads[name], st, n2, dout))
+    finally:
+        del ops.expert_stack
+    ops.check_status()
+    # and both against the layer in fp32 on the experts that were chosen
+    ref_ops = TorchOps()
+    pf = {n: w.float() for n, w in p.items()}
+    gf = {n: torch.full_like(w, float("nan")) for n, w in pf.items()}
+    real = M.route
+    try:
+        M.route = lambda c, w, x, topi=None: real(c, w, x, topi=st.topi)
+        fo, fst = M.moe_forward(ref_ops, cfg, pf, n2.float(), h1.float(), True, False)
+        fd = M.moe_backward(ref_ops, cfg, pf, gf, fst, n2.float(), dout.float())
+    finally:
+        M.route = real
+    for a, b, f in zip(res["grouped"], res["loop"], (fo, fd)):
+        assert rel_err(a, b) < 1e-2       # bf16 on both sides; the loop rounds weighted rows and scaled gradients in between
+        assert rel_err(a, f) < 1.5e-2 and rel_err(a, f) < 1.1 * rel_err(b, f) + 1e-4
+    for n in p:
+        a, b, f = grads["grouped"][n], grads["loop"][n], gf[n]
+        if f.norm() == 0:
+            assert a.float().norm() == 0, n
+        else:
+            assert rel_err(a, b) < 2e-2 and rel_err(a, f) < 1.3 * rel_err(b, f) + 1e-3, n

@@ -52,6 +52,12 @@ def forward_in_pairs(blocks: list, hq: int, hkv: int, d: int, sms: int) -> bool:
     tiles exists once per sequence of at least ``n`` blocks."""
     if not blocks:
         return True
+    if sum(blocks) * hq <= sms:   # one tile per CTA is done after the longest tile, and pairs take longer over theirs
+        return False
+    return _forward_in_pairs(blocks, hq, hkv, d, sms)
+
+
+def _forward_in_pairs(blocks: list, hq: int, hkv: int, d: int, sms: int) -> bool:
     at = _with_at_least(blocks)
     longest = len(at) - 2
     launch, a, b = _ONE[d]
@@ -70,8 +76,15 @@ def backward_splits(blocks: list, hq: int, hkv: int, sms: int, most: int) -> int
     kv heads and a short batch that leaves SMs idle and the longest CTA decides (5987 tokens, 12/2 heads: 437 -> 137 us with
     the heads divided). But every CTA loads K and V again and adds a partial sum, so short samples are not divided
     (16 of 128 tokens, 32/8 heads of 128: 47 us whole, 86 when divided until there were two CTAs per SM)."""
-    if not blocks:
+    group = hq // hkv
+    if not blocks or group == 1 or most <= 1:
         return 1
+    if sum(blocks) * hq <= sms and most >= group:   # however divided, everything runs at once: the longest CTA decides
+        return group if _BWD_PARTIAL < (group - 1) * max(blocks) else 1
+    return _backward_splits(blocks, hq, hkv, sms, most)
+
+
+def _backward_splits(blocks: list, hq: int, hkv: int, sms: int, most: int) -> int:
     at = _with_at_least(blocks)
     longest, group, units = len(at) - 2, hq // hkv, sum(blocks) * hkv
     best, splits = float("inf"), 1

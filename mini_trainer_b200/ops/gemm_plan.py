@@ -9,8 +9,6 @@ on average, where pairs for everything of 64 tiles with the earlier split rule c
 """
 from __future__ import annotations
 
-import functools
-
 BK = 64
 MAX_SPLITS = 16
 UNIT_BYTES = 128 * 256 * 4      # partial of 128 rows x 256 columns: one per tile and split of a single CTA, two of a pair
@@ -37,7 +35,6 @@ def _best_split(tiles: int, units: int, kblocks: int, workers: int, max_units: i
     return best, splits
 
 
-@functools.lru_cache(maxsize=4096)
 def choose(M: int, N: int, K: int, sms: int, pairs: int, one: bool, max_units: int, max_counted: int) -> tuple:
     """``(two_cta, splits)`` for an ``M x N x K`` product. ``pairs``: CTA pairs that may be used (0: none); ``one``: single CTAs may be.
     ``max_units``: partials the scratch may hold, ``max_counted``: 128-row units it has counters for."""

@@ -89,6 +89,7 @@ class _Sig:
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
+_GEMM_TAGS = (("gemm_nt", "gemm_nn"), ("gemm_tt", "gemm_tn"))   # [A stored [K, M]][B stored [K, N]]
 _SPLIT_COUNTERS = 4096          # csrc/gemm_epilogue.cuh
 _SPLIT_FLOATS = 32 << 20        # most that the partials of a launch take: 128 MB
 _SPLIT_UNITS = 4 * _SPLIT_FLOATS // gemm_plan.UNIT_BYTES   # = 1024 of 128 x 256
@@ -138,6 +139,7 @@ class NativeOps:
         self.profile = [] if os.environ.get("MTB200_PROFILE") else None
         self._scratch = {}
         self._gemm_ws = {}   # stream handle -> arrival counters of split launches
+        self._gemm_plans = {}   # sizes -> entry point and splits
         self._epoch = itertools.count(1)   # of the launches that may split
         self._attn_plan_cache = {}
         self._pairs = None
@@ -243,6 +245,20 @@ class NativeOps:
             return None
         return ws, next(self._epoch), part
 
+    def _plan_gemm(self, M, N, K, two_cta):
+        """``(entry point, splits, bytes of partials)`` of a product, from its sizes."""
+        pairs, one = self.cta_pairs(), True
+        if two_cta if two_cta is not None else self.use_gemm2:
+            one = False
+        elif two_cta is not None or 2.0 * M * N * K > self.pair_max_flops:
+            pairs = 0
+        pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
+        if len(self._gemm_plans) >= 4096:
+            self._gemm_plans.clear()
+        plan = ("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", splits, gemm_plan.partial_bytes(M, N, pair, splits))
+        self._gemm_plans[(M, N, K, two_cta)] = plan
+        return plan
+
     def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
         """out[M,N] = alpha*A*B (+bias) (+residual). ``a_mn``/``b_mn``: operand stored [K, rows].
         ``stats`` [M, ceil(N / 256), 2] fp32 receives the softmax statistics of the (bf16) output rows per 256 columns.
@@ -251,19 +267,18 @@ class NativeOps:
         out_f32 = out.dtype == torch.float32
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
         assert residual is None or residual.dtype == out.dtype
-        pairs, one = self.cta_pairs(), True
-        if two_cta if two_cta is not None else self.use_gemm2:
-            one = False
-        elif two_cta is not None or 2.0 * M * N * K > self.pair_max_flops:
-            pairs = 0
-        pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
+        plan = self._gemm_plans.get((M, N, K, two_cta))
+        if plan is None:
+            plan = self._plan_gemm(M, N, K, two_cta)
+        name, splits, nbytes = plan
         st = self._st()
-        split = self._split(st, gemm_plan.partial_bytes(M, N, pair, splits)) if splits > 1 else None
+        split = self._split(st, nbytes) if splits > 1 else None
         ws, epoch, part = split or (None, 0, None)
-        self._call("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
+        self._call(name, a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn),
                    out.data_ptr(), out.stride(0), int(out_f32), _ptr(residual),
                    residual.stride(0) if residual is not None else 0, _ptr(bias), M, N, K, float(alpha), splits if split else 1,
-                   _ptr(ws), epoch, _ptr(part), 4 * part.numel() if split else 0, _ptr(stats), self.status.data_ptr(), st, tag=tag or f"gemm_{'t' if a_mn else 'n'}{'n' if b_mn else 't'}")
+                   _ptr(ws), epoch, _ptr(part), 4 * part.numel() if split else 0, _ptr(stats), self.status.data_ptr(), st,
+                   tag=tag or _GEMM_TAGS[bool(a_mn)][bool(b_mn)])
         return out
 
     # -- embedding --------------------------------------------------------------------
@@ -399,23 +414,43 @@ class NativeOps:
         return dqkv
 
     # -- attention --------------------------------------------------------------------
-    def _per_batch(self, cu_host, what: tuple, make):
-        """``make()``, computed once per minibatch (its list of sequence starts) and reused by every layer."""
-        key = (id(cu_host),) + what
-        hit = self._attn_plan_cache.get(key)
-        if hit is not None and hit[0] is cu_host:
-            return hit[1]
-        value = make()
+    def _cached(self, cu_host, what: tuple):
+        """What ``_keep`` has kept for this minibatch (its list of sequence starts), or ``None``."""
+        hit = self._attn_plan_cache.get((id(cu_host),) + what)
+        return hit[1] if hit is not None and hit[0] is cu_host else None
+
+    def _keep(self, cu_host, what: tuple, value):
         if len(self._attn_plan_cache) > 16:
             self._attn_plan_cache.clear()
-        self._attn_plan_cache[key] = (cu_host, value)
+        self._attn_plan_cache[(id(cu_host),) + what] = (cu_host, value)
         return value
 
     def _attn_plan(self, cu_host, block, most_work_last_block: bool):
         """Work table for the attention kernels: one row (seq_start, seq_len, block_start) per
         ``block`` rows of every sequence, most work first (forward: late query blocks see the most
-        keys; backward: early key blocks are seen by the most queries)."""
-        return self._per_batch(cu_host, (block, most_work_last_block), lambda: self._attn_table(cu_host, block, most_work_last_block))
+        keys; backward: early key blocks are seen by the most queries). Built once per minibatch
+        and reused by every layer."""
+        what = (block, most_work_last_block)
+        table = self._cached(cu_host, what)
+        return self._keep(cu_host, what, self._attn_table(cu_host, block, most_work_last_block)) if table is None else table
+
+    def _plan_attention(self, cu_host, hq, hkv, d):
+        """``(entry point, its row_pairs argument, work table)`` of a minibatch's forward. A work item is one 128-row block of a head; or, in
+        pairs, a block of two heads of a kv head, or two blocks of a head where heads do not pair up."""
+        if attention_plan.forward_in_pairs(attention_plan.blocks_per_sequence(cu_host), hq, hkv, d, self.sms):
+            row_pairs = (hq // hkv) % 2
+            plan = ("mtb200_attn_fwd", (row_pairs,), self._attn_plan(cu_host, 256 if row_pairs else 128, True))
+        else:
+            plan = ("mtb200_attn_fwd_one", (), self._attn_plan(cu_host, 128, True))
+        return self._keep(cu_host, ("fwd", hq, hkv, d), plan)
+
+    def _plan_attention_bwd(self, cu_host, hq, hkv, d):
+        """``(work table, CTAs per key block, bytes of their partials)`` of a minibatch's backward."""
+        table = self._attn_plan(cu_host, 128, False)
+        units = table.shape[0] * hkv   # per unit: 8 counters and, for every CTA that shares it, dK and dV of 128 rows in fp32
+        most = 1 if units * 8 > _SPLIT_COUNTERS else min(hq // hkv, _SPLIT_FLOATS // max(1, units * 2 * 128 * d))
+        splits = attention_plan.backward_splits(attention_plan.blocks_per_sequence(cu_host), hq, hkv, self.sms, most)
+        return self._keep(cu_host, ("bwd", hq, hkv, d), (table, splits, splits * units * 2 * 128 * d * 4))
 
     def _attn_table(self, cu_host, block, most_work_last_block: bool):
         items = []
@@ -434,16 +469,9 @@ class NativeOps:
             return self._fa_fwd(qkv, cu_seqlens, max_seqlen, hq, hkv, d, scale)
         out = torch.empty(T, hq * d, dtype=qkv.dtype, device=self.device)
         lse = torch.empty(hq, T, dtype=torch.float32, device=self.device)
-        if not self._per_batch(cu_host, ("pairs", hq, hkv, d), lambda: attention_plan.forward_in_pairs(
-                attention_plan.blocks_per_sequence(cu_host), hq, hkv, d, self.sms)):
-            plan = self._attn_plan(cu_host, 128, True)
-            self._call("mtb200_attn_fwd_one", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), lse.data_ptr(),
-                       plan.data_ptr(), plan.shape[0], T, hq, hkv, d, scale, self.status.data_ptr(), self._st(), tag="mtb200_attn_fwd")
-            return out, lse
-        row_pairs = (hq // hkv) % 2   # a work item is two heads of a kv head, or two 128-row blocks of a head where heads do not pair up
-        plan = self._attn_plan(cu_host, 256 if row_pairs else 128, True)
-        self._call("mtb200_attn_fwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), lse.data_ptr(),
-                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, row_pairs, scale, self.status.data_ptr(), self._st())
+        name, tail, plan = self._cached(cu_host, ("fwd", hq, hkv, d)) or self._plan_attention(cu_host, hq, hkv, d)
+        self._call(name, qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), lse.data_ptr(),
+                   plan.data_ptr(), plan.shape[0], T, hq, hkv, d, *tail, scale, self.status.data_ptr(), self._st(), tag="mtb200_attn_fwd")
         return out, lse
 
     def attention_bwd(self, dout, qkv, out, lse, cu_seqlens, cu_host, max_seqlen, hq, hkv, d, scale=None):
@@ -452,15 +480,11 @@ class NativeOps:
         if self.attention_impl == "flash_attn" or d not in NATIVE_HEAD_DIMS:
             return self._fa_bwd(dout, qkv, out, lse, cu_seqlens, max_seqlen, hq, hkv, d, scale)
         dqkv = torch.empty_like(qkv)
-        plan = self._attn_plan(cu_host, 128, False)
+        plan, splits, nbytes = self._cached(cu_host, ("bwd", hq, hkv, d)) or self._plan_attention_bwd(cu_host, hq, hkv, d)
         delta = torch.empty(hq, T, dtype=torch.float32, device=self.device)
         dq_acc = torch.zeros(T, hq * d, dtype=torch.float32, device=self.device)
         st = self._st()
-        units = plan.shape[0] * hkv   # per unit: 8 counters and, for every CTA that shares it, dK and dV of 128 rows in fp32
-        most = 1 if units * 8 > _SPLIT_COUNTERS else min(hq // hkv, _SPLIT_FLOATS // (units * 2 * 128 * d))
-        splits = 1 if most <= 1 else self._per_batch(cu_host, ("splits", hq, hkv, d), lambda: attention_plan.backward_splits(
-            attention_plan.blocks_per_sequence(cu_host), hq, hkv, self.sms, most))
-        split = self._split(st, splits * units * 2 * 128 * d * 4) if splits > 1 else None
+        split = self._split(st, nbytes) if splits > 1 else None
         ws, epoch, part = split or (None, 0, None)
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),

@@ -13,7 +13,7 @@ def make_ops(**fakes):
     ops._index, ops.launches, ops.profile = 0, 0, None
     ops.use_gemm2, ops.pair_max_flops, ops.sms = False, 1e12, 148
     ops.status = torch.zeros(1, dtype=torch.int32)
-    ops._scratch, ops._gemm_ws, ops._attn_plan_cache, ops._pairs = {}, {}, {}, None
+    ops._scratch, ops._gemm_ws, ops._attn_plan_cache, ops._gemm_plans, ops._pairs = {}, {}, {}, {}, None
     ops._epoch = itertools.count(1)
     ops.calls = []
     fakes.setdefault("mtb200_gemm2_pairs", lambda: 74)
@@ -198,3 +198,18 @@ def test_linear_ce_takes_a_flat_weight_gradient():
                     assert (args[9] == dw.data_ptr() and args[10] == H) if acc else args[9] is None
                 else:
                     assert name == "mtb200_f32_to_bf16" and args[2:4] == (V * H, int(acc))
+
+
+def test_attention_choices_agree_with_the_full_estimate():
+    """What a small batch is answered without the estimate is what the estimate says."""
+    from mini_trainer_b200.ops import attention_plan as A
+    import random
+    rng = random.Random(2)
+    for _ in range(400):
+        blocks = [rng.randint(1, 6) for _ in range(rng.randint(1, 6))]
+        hkv = rng.choice((1, 2, 4))
+        hq = hkv * rng.randint(1, 8)
+        for sms in (148, 40):
+            assert A.backward_splits(blocks, hq, hkv, sms, 64) == A._backward_splits(blocks, hq, hkv, sms, 64)
+            for d in (64, 128):
+                assert A.forward_in_pairs(blocks, hq, hkv, d, sms) == A._forward_in_pairs(blocks, hq, hkv, d, sms)

@@ -803,9 +803,11 @@ def test_gemm_row_statistics(ops, M, N, K, layout, two_cta):
 
 
 @pytest.mark.parametrize("pairs", [True, False])
-@pytest.mark.parametrize("D,hq,hkv,lens", ATTN_CASES + [(64, 3, 1, [257, 1, 128, 384]), (64, 14, 2, [2049, 63])])
+@pytest.mark.parametrize("D,hq,hkv,lens", ATTN_CASES + [(64, 3, 1, [257, 1, 128, 384]), (64, 14, 2, [2049, 63]), (64, 4, 2, [130] * 100),
+                                                        (128, 6, 2, [257, 1, 128, 255, 256, 300] * 12), (128, 2, 2, [129] * 80)])
 def test_attention_forward_both_forms(ops, D, hq, hkv, lens, pairs, monkeypatch):
-    """Every batch through pairs of query tiles and through one tile per CTA, whichever the sizes would choose."""
+    """Every batch through pairs of query tiles and through one tile per CTA, whichever the sizes would choose; among them batches of
+    several rounds of the persistent CTAs."""
     from mini_trainer_b200.ops import attention_plan
     monkeypatch.setattr(attention_plan, "forward_in_pairs", lambda *a: pairs)
     torch.manual_seed(sum(lens) + pairs)
@@ -956,3 +958,44 @@ def test_grouped_experts_shared_scaled_unnormalised(ops, T, H, F, E, k, popular,
             assert a.float().norm() == 0, n
         else:
             assert rel_err(a, b) < 2e-2 and rel_err(a, f) < 1.3 * rel_err(b, f) + 1e-3, n
+
+
+# every number of work items per tile that the choice may take, also where it would not: reductions of 16 to 122 k-blocks divided evenly
+# and unevenly, both kernels
+@pytest.mark.parametrize("splits", [2, 3, 7, 16])
+@pytest.mark.parametrize("two_cta", [False, True])
+@pytest.mark.parametrize("M,N,K", [(136, 264, 1024), (300, 520, 7776)])
+def test_gemm_every_split(ops, M, N, K, two_cta, splits, monkeypatch):
+    from mini_trainer_b200.ops import gemm_plan
+    monkeypatch.setattr(gemm_plan, "choose", lambda *a: (two_cta, splits))
+    monkeypatch.setattr(ops, "_gemm_plans", {})
+    a, b, res = _ints(M, K), _ints(N, K), _ints(M, N)
+    want = a.float() @ b.float().t()       # integers below 2^24: exact in fp32 in any order
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.full((M, N), float("nan"), dtype=dt, device="cuda")
+        ops.gemm(a, False, b, False, out, M, N, K, residual=res.to(dt))
+        assert torch.equal(out, (want + res.float()).to(dt))
+    ops.check_status()
+
+
+@pytest.mark.parametrize("D,hq,hkv,lens", [(128, 7, 1, [300, 129, 1]), (64, 12, 2, [640, 90])])
+def test_attention_backward_every_division(ops, D, hq, hkv, lens, monkeypatch):
+    """A key block's query heads on one to as many CTAs as there are heads, evenly divided or not."""
+    from mini_trainer_b200.ops import attention_plan
+    torch.manual_seed(9)
+    T = sum(lens)
+    qkv, dout = bf(T, (hq + 2 * hkv) * D), bf(T, hq * D)
+    cu_host, cu = _cu(lens)
+    out, lse = ops.attention(qkv, cu, cu_host, max(lens), hq, hkv, D)
+    ro, rl = REF.attention(qkv.float(), cu, cu_host, max(lens), hq, hkv, D)
+    rd = REF.attention_bwd(dout.float(), qkv.float(), ro, rl, cu, cu_host, max(lens), hq, hkv, D)
+    first = None
+    for s in range(1, hq // hkv + 1):
+        monkeypatch.setattr(attention_plan, "backward_splits", lambda *a: s)
+        cu_host = list(cu_host)            # another minibatch: nothing planned for it
+        d = ops.attention_bwd(dout, qkv, out, lse, cu, cu_host, max(lens), hq, hkv, D)
+        assert rel_err(d, rd) < 1.5e-2
+        first = d if first is None else first
+        # the sums of the CTAs' parts are fp32: what differs from the undivided sum is its rounding to bf16
+        assert rel_err(d[:, hq * D:], first[:, hq * D:]) < 3e-3
+    ops.check_status()

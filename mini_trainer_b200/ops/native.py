@@ -650,7 +650,7 @@ class NativeOps:
     def linear_ce(self, x, w, targets, grad_scale, dw_out, accumulate_dw=False, ignore_index=-100, logit_scale=1.0):
         """Per-token CE of ``logit_scale * x @ w.T``. Chunked over tokens (8192 rows): bf16 logits chunk
         by the tcgen05 GEMM (fp32 accumulation, one rounding: what the reference's fused linear-CE holds
-        too), whose epilogue also leaves softmax statistics -> loss and the bf16 gradient written over the logits -> dX
+        too), whose epilogue also leaves softmax statistics where that pays -> loss and the bf16 gradient written over the logits -> dX
         chunk and dW accumulation, again on the tcgen05 GEMM. Only ``[chunk, V]`` logits ever exist.
         dW is accumulated in fp32 over the chunks and rounded to bf16 once."""
         T, H = x.shape
@@ -659,7 +659,10 @@ class NativeOps:
         dx = torch.empty_like(x)
         ck = min(self.ce_chunk, T)
         logits = self._buf("ce_logits", ck * V, torch.bfloat16).view(ck, V)
-        stats = self._buf("ce_stats", ck * -(-V // 256) * 2, torch.float32)
+        # The statistics save the cross-entropy a read of the row, which only costs where a row does not stay on the SM, and take the
+        # epilogue 3 us per tile, which only hides behind longer reductions. Logits and gradient together: 3720 x 151936 x 1536 1646 us
+        # with and 1997 without, 8000 x 32000 x 2048 1039 and 1120, x 1536 771 and 778, but x 1024 682 and 618; 8000 x 512 x 64 86 and 69.
+        stats = self._buf("ce_stats", ck * -(-V // 256) * 2, torch.float32) if V > 16384 and H >= 1536 else None
         # one chunk: its weight gradient is the whole sum, rounded (or added to what is there) in the GEMM's epilogue
         whole = T <= ck and dw_out.is_contiguous()
         dw = dw_out.view(V, H) if whole else None
@@ -668,7 +671,7 @@ class NativeOps:
         for a in range(0, T, ck):
             n = min(ck, T - a)
             self.gemm(x[a:a + n], False, w, False, logits, n, V, H, alpha=logit_scale, stats=stats)
-            self._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, stats.data_ptr(), targets[a:a + n].data_ptr(),
+            self._call("mtb200_ce_fwd_bwd", logits.data_ptr(), V, 1, _ptr(stats), targets[a:a + n].data_ptr(),
                        loss[a:a + n].data_ptr(), logits.data_ptr(), V, n, V, float(grad_scale), ignore_index, self._st())
             self.gemm(logits, False, w, True, dx[a:a + n], n, H, V, alpha=logit_scale)
             if whole:

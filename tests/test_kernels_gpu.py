@@ -999,3 +999,28 @@ def test_attention_backward_every_division(ops, D, hq, hkv, lens, monkeypatch):
         # the sums of the CTAs' parts are fp32: what differs from the undivided sum is its rounding to bf16
         assert rel_err(d[:, hq * D:], first[:, hq * D:]) < 3e-3
     ops.check_status()
+
+
+# logits whose product leaves the statistics and logits whose rows are read for them, in one chunk and in several
+@pytest.mark.parametrize("T,H,V", [(130, 1536, 17008), (130, 1528, 17008), (130, 1536, 16384), (70, 64, 520)])
+def test_linear_ce_with_and_without_statistics(ops, T, H, V, monkeypatch):
+    torch.manual_seed(V + H)
+    x, w = bf(T, H), bf(V, H, scale=3 * H ** -0.5)
+    tg = torch.randint(0, V, (T,), device="cuda")
+    tg[::9] = -100
+    seen = []
+    gemm = ops.gemm
+    monkeypatch.setattr(ops, "gemm", lambda *a, **k: (seen.append(k.get("stats") is not None), gemm(*a, **k))[1])
+    lg = (x.float() @ w.float().t()).bfloat16().double()
+    ref = torch.nn.functional.cross_entropy(lg, tg, reduction="none", ignore_index=-100)
+    p = torch.softmax(lg, -1)
+    p[torch.arange(T, device="cuda"), tg.clamp_min(0)] -= 1
+    p[tg == -100] = 0
+    for chunk in (8192, 64):
+        monkeypatch.setattr(ops, "ce_chunk", chunk)
+        dw = torch.empty_like(w)
+        loss, dx = ops.linear_ce(x, w, tg, 0.5, dw)
+        assert (loss - ref).abs().max() < 2e-3        # a bf16 step of a logit near the row's maximum is what may differ
+        assert rel_err(dx, 0.5 * p @ w.double()) < 1e-2 and rel_err(dw, 0.5 * p.t() @ x.double()) < 1e-2
+    assert any(seen) == (V > 16384 and H >= 1536)
+    ops.check_status()

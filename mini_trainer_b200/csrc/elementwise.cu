@@ -1025,10 +1025,11 @@ static int norm_fwd(const void* x, const void* w, const void* b, void* y, float*
   while (lanes < EW_THREADS && lanes * 4 < vecs) lanes *= 2;
   const int vpt = cdiv(vecs, lanes);
   if constexpr (LN) {
-    // Rows of up to 1024 elements: eight and more per block pay at any height (16384 x 1024: 14.5 us, 27 with a block per row). Wider
-    // ones want a batch that lasts: equal at 4000 x 2048 and 6000 x 4096. Three vectors of 256 threads (4104 .. 6144) never win.
+    // Rows of up to 1024 elements: eight and more per block pay from 1024 rows on (16384 x 1024: 14.5 us, 27 with a block per row; cold,
+    // 8 x 1024: 8.2 and 6.4). Wider ones want a batch that lasts: equal at 4000 x 2048 and 6000 x 4096. Three vectors of 256 threads
+    // (4104 .. 6144) never win.
     const long long n = static_cast<long long>(T) * H;
-    const bool bulk = H <= 1024 || (H <= 2048 ? n >= 6000000 : n >= 24000000 && !(lanes == EW_THREADS && vpt == 3));
+    const bool bulk = H <= 1024 ? T >= 1024 : (H <= 2048 ? n >= 6000000 : n >= 24000000 && !(lanes == EW_THREADS && vpt == 3));
     if (!bulk) {
 #define LF(V) layernorm_row_kernel<V><<<T, EW_THREADS, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, H)
       const int v = cdiv(H, 8 * EW_THREADS);

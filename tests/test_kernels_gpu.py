@@ -829,7 +829,7 @@ def test_attention_forward_both_forms(ops, D, hq, hkv, lens, pairs, monkeypatch)
 # both sides of every line the forward of the norms is drawn by: few and many row sets per block, one block per row, the widths at
 # which a row takes one to eight warps, partial last row sets
 @pytest.mark.parametrize("T,H", [(1, 8), (3, 256), (2368 * 2 + 1, 512), (20011, 512), (740, 896), (15000, 896), (1481, 12288), (450, 12288), (3, 16384),
-                                 (800, 16384), (2930, 2048), (2929, 2048), (5857, 1024), (9400, 2560), (9375, 2560), (6001, 4096), (5000, 5120), (2930, 8192),
+                                 (800, 16384), (2930, 2048), (2929, 2048), (5857, 1024), (1023, 1024), (1024, 1024), (9400, 2560), (9375, 2560), (6001, 4096), (5000, 5120), (2930, 8192),
                                  (100, 8192)])
 def test_norm_forward_forms(ops, T, H):
     torch.manual_seed(T + H)

@@ -439,6 +439,9 @@ __global__ void __launch_bounds__(EW_THREADS) rope_kernel(__nv_bfloat16* __restr
 // further holds; sine and cosine are shared by the warp's heads. `pre` (optional) receives the heads before the norm, which
 // backward reads. Bound by reading and writing the heads once: with the copy, the norm and the rotation as passes of their
 // own they were read three times and written three times (4099 tokens x 24 heads of 128: forward 54 -> 17 us, backward 36 -> 26 us).
+// Forward: HPW heads of a token per warp; four, so that they share the angles and several loads are in flight, or one where that
+// leaves fewer than two blocks per SM (33 tokens x 24 heads of 128, without the rotation, cold: 8.2 and 6.1 us; backward, whose blocks also
+// add up partials, is the faster with four at any height).
 constexpr int HEADS_PER_WARP = 4;
 template <int EPL>
 struct HeadVec {
@@ -485,7 +488,7 @@ __device__ __forceinline__ void head_rotate(float (&f)[EPL], const float (&cs)[E
   for (int i = 0; i < EPL; ++i) f[i] = f[i] * cs[i] + sg * __shfl_xor_sync(0xffffffffu, f[i], 16) * sn[i];
 }
 
-template <int EPL, bool ROPE>
+template <int EPL, bool ROPE, int HPW>
 __global__ void __launch_bounds__(EW_THREADS) head_rmsnorm_fwd_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ wq,
                                                                      const __nv_bfloat16* __restrict__ wk, __nv_bfloat16* __restrict__ pre,
                                                                      float* __restrict__ rstd_out, const int* __restrict__ pos,
@@ -496,15 +499,15 @@ __global__ void __launch_bounds__(EW_THREADS) head_rmsnorm_fwd_kernel(__nv_bfloa
   const int lane = threadIdx.x & 31;
   if (r >= n_items) return;   // whole warps leave together
   const long long t = r / groups;
-  const int h0 = static_cast<int>(r - t * groups) * HEADS_PER_WARP;
+  const int h0 = static_cast<int>(r - t * groups) * HPW;
   __nv_bfloat16* p = qkv + t * ld + static_cast<long long>(h0) * D + lane * EPL;
-  HeadVec<EPL> xv[HEADS_PER_WARP];
+  HeadVec<EPL> xv[HPW];
 #pragma unroll
-  for (int k = 0; k < HEADS_PER_WARP; ++k) if (h0 + k < n_heads) xv[k].load(p + k * D);
+  for (int k = 0; k < HPW; ++k) if (h0 + k < n_heads) xv[k].load(p + k * D);
   float cs[EPL], sn[EPL];
   if (ROPE) head_angles<EPL>(static_cast<float>(pos[t]), inv_freq, lane, cs, sn);
 #pragma unroll
-  for (int k = 0; k < HEADS_PER_WARP; ++k) {
+  for (int k = 0; k < HPW; ++k) {
     const int h = h0 + k;
     if (h >= n_heads) break;
     if (pre != nullptr) xv[k].store(pre + t * (static_cast<long long>(n_heads) * D) + static_cast<long long>(h) * D + lane * EPL);
@@ -1147,19 +1150,25 @@ int mtb200_rope(void* qkv, const int* pos, const float* inv_freq, int T, long lo
   return launch_ok();
 }
 
+static int heads_per_warp(int T, int n_heads) {
+  return static_cast<long long>(T) * cdiv(n_heads, HEADS_PER_WARP) < 2LL * num_sms() * (EW_THREADS / 32) ? 1 : HEADS_PER_WARP;
+}
+
 // Per-head RMSNorm of the q and k heads (n_q then n_heads - n_q) of qkv[T, ld], in place; rstd: [T * n_heads] fp32. With
 // inv_freq [D / 2] (and pos [T]) the heads are also rotated; pre (optional): [T, n_heads * D], the heads as they came.
 int mtb200_head_rmsnorm_fwd(void* qkv, const void* wq, const void* wk, void* pre, float* rstd, const int* pos, const float* inv_freq, float eps,
                             int T, long long ld, int n_q, int n_heads, int D, cudaStream_t st) {
   if (T <= 0 || n_heads <= 0) return 0;
   if ((D != 64 && D != 128 && D != 256) || ld % 8 || n_q < 0 || n_q > n_heads || (inv_freq && !pos)) return -10;
-  const int groups = cdiv(n_heads, HEADS_PER_WARP);
+  const int hpw = heads_per_warp(T, n_heads), groups = cdiv(n_heads, hpw);
   const long long n_items = static_cast<long long>(T) * groups;
   const unsigned blocks = static_cast<unsigned>(cdiv(n_items, EW_THREADS / 32));
-#define HF(E, R) head_rmsnorm_fwd_kernel<E, R><<<blocks, EW_THREADS, 0, st>>>((bf16*)qkv, (const bf16*)wq, (const bf16*)wk, (bf16*)pre, rstd, pos, inv_freq, eps, n_items, groups, ld, n_q, n_heads)
-  if (inv_freq) { if (D == 64) HF(2, true); else if (D == 128) HF(4, true); else HF(8, true); }
-  else { if (D == 64) HF(2, false); else if (D == 128) HF(4, false); else HF(8, false); }
+#define HF(E, R) if (hpw == 1) HFW(E, R, 1); else HFW(E, R, HEADS_PER_WARP)
+#define HFW(E, R, W) head_rmsnorm_fwd_kernel<E, R, W><<<blocks, EW_THREADS, 0, st>>>((bf16*)qkv, (const bf16*)wq, (const bf16*)wk, (bf16*)pre, rstd, pos, inv_freq, eps, n_items, groups, ld, n_q, n_heads)
+  if (inv_freq) { if (D == 64) { HF(2, true); } else if (D == 128) { HF(4, true); } else { HF(8, true); } }
+  else { if (D == 64) { HF(2, false); } else if (D == 128) { HF(4, false); } else { HF(8, false); } }
 #undef HF
+#undef HFW
   return launch_ok();
 }
 

@@ -1024,3 +1024,25 @@ def test_linear_ce_with_and_without_statistics(ops, T, H, V, monkeypatch):
         assert rel_err(dx, 0.5 * p @ w.double()) < 1e-2 and rel_err(dw, 0.5 * p.t() @ x.double()) < 1e-2
     assert any(seen) == (V > 16384 and H >= 1536)
     ops.check_status()
+
+
+# both sides of the line between one head per warp and four: 2 blocks per SM of 8 warps of four heads
+@pytest.mark.parametrize("D,hq,hkv", [(128, 16, 8), (64, 14, 2), (256, 3, 2)])
+def test_head_norm_heads_per_warp(ops, D, hq, hkv):
+    nh = hq + hkv
+    edge = -(-2 * ops.sms * 8 // -(-nh // 4))
+    torch.manual_seed(D)
+    wq, wk = bf(D), bf(D)
+    T = edge
+    qkv = bf(T, (hq + 2 * hkv) * D)
+    pos = torch.arange(T, device="cuda", dtype=torch.int32)
+    inv = 1e4 ** (-torch.arange(0, D, 2, device="cuda").float() / D)
+    for rope in (False, True):
+        a, b = qkv.clone(), qkv.clone()
+        pre, ra = ops.qk_norm_rope_(a, wq, wk, 1e-6, hq, hkv, D, pos if rope else None, inv if rope else None)
+        part, rb = ops.qk_norm_rope_(b[: T - 1], wq, wk, 1e-6, hq, hkv, D, pos if rope else None, inv if rope else None)
+        assert torch.equal(a[: T - 1], b[: T - 1]) and torch.equal(ra[: (T - 1) * nh], rb)     # the same work, dealt differently
+        assert torch.equal(pre[: T - 1], part) and torch.equal(pre, qkv[:, : nh * D]) and torch.equal(a[:, nh * D:], qkv[:, nh * D:])
+    x = qkv[:, : nh * D].float().view(T, nh, D)
+    assert rel_err(ra, (x.pow(2).mean(-1) + 1e-6).rsqrt().reshape(-1)) < 1e-6
+    ops.check_status()

@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(512) norm_bwd_kernel(const __nv_bfloat16* __re
 // Sums of R partial rows of C columns; columns [0, D) go to out_a, the rest to out_b (a row may hold the partials of two
 // vectors; D = C when it holds one). 32 columns per block, 16 warps share the rows: a chain of R / 16 loads instead of R
 // (296 rows of 4096: 15 -> 5 us). Few rows are one thread's work per column (reduce_few_rows_kernel): with a batch of eight tokens the
-// barrier and the many blocks took longer than the sum (colsum of 8 x 896: 6.3 us, 4.7 like this).
+// barrier and the many blocks took longer than the sum (colsum of 8 x 896: 6.3 us, 4.7 like this; below 512 columns there are few blocks).
 __global__ void __launch_bounds__(512) reduce_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
                                                          int R, int C, int D) {
   __shared__ float sm[16][32];
@@ -977,7 +977,7 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
 
 static inline int cdiv(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 static void reduce_rows(const float* part, void* out_a, void* out_b, int R, int C, int D, cudaStream_t st) {
-  if (R <= 16) reduce_few_rows_kernel<<<cdiv(C, 256), 256, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
+  if (R <= 16 && C >= 512) reduce_few_rows_kernel<<<cdiv(C, 256), 256, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
   else reduce_rows_kernel<<<cdiv(C, 32), 512, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
 }
 static inline int launch_ok() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }

@@ -17,8 +17,7 @@
 // P(i+1) is computed while dK(i), dQ(i) run and dQ(i) is drained, dS(i+1) while dV(i+1) and S(i+2) run. The chain that bounds
 // an iteration is dS -> dK dQ -> drain -> dP -> dS, where the form with everything in one chain (S dP | softmax | dK dV dQ |
 // drain) had five products, the whole softmax and the drain. At D = 128 an iteration takes about 4950 clocks for 2560 of MMA,
-// the same for every order of the products tried. A fifth of it is dQ's tensor reduces, 64 KB per iteration (without them, results
-// apart, 16384 tokens take 4.6 instead of 5.7 ms); the rest is the hand-offs and latencies of the chain.
+// the same for every order of the products tried: the chain's hand-offs and latencies, and dQ's tensor reduces of 64 KB.
 // 1 x 16384 tokens, 32/8 heads: 6.5 -> 5.5 ms at D = 128 (main kernel),
 // 5.3 -> 3.2 ms at D = 64 (all passes; 3.6 with dV in front of dP and the shared columns).
 //

@@ -13,9 +13,10 @@
 // queue on the special-function unit. Two independent tiles take turns: while A is in its softmax the tensor core runs
 // P V and the next S of B. K and V are loaded once per pair. A row belongs to one thread, so nothing is exchanged between
 // threads (two threads per row with their maxima exchanged through shared memory measured 1.92 ms below). P is handed over in
-// two halves of 64 keys, so the first half's products run under the second half's exponentials. 1 x 16384 tokens, 32/8 heads, D = 128: 1.65 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64:
-// 64 us (one tile per CTA, two threads per row: 1.94 ms and 94 us).
-// Launches with few pairs, and some long ones at D = 64, are faster in that other form: attention_fwd_one.cu.
+// two halves of 64 keys, so the first half's products run under the second half's exponentials.
+// 1 x 16384 tokens, 32/8 heads, D = 128: 1.65 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64: 64 us (one tile per CTA, two
+// threads per row: 1.94 ms and 94 us). Launches with few pairs are faster in that other form (attention_fwd_one.cu);
+// a long sequence at D = 64 is level (1 x 16384, 32/8 heads: 1.54 ms there, 1.50 here).
 //
 // CTAs are persistent (one per SM): barriers and tensor memory are set up once, K and V of the next item are prefetched
 // under the current one's tail, and the epilogue of an item runs under the next item's first product. Items come most work

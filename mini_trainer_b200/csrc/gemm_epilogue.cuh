@@ -228,7 +228,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
 //   ROWS    D[rows, N] = A[rows, K] * W_e: A and D hold the slabs, the weights are one 3-D tensor [E, ., .]
 //   REDUCE  D_e = A[rows_e, M]^T * B[rows_e, N]: one output matrix per expert, zeros for an expert without rows
 // One launch per product instead of one per expert: forward + backward of 4096 tokens through 8 experts of 4096 x 14336
-// (2 chosen) 12.2 -> 7.6 ms, of 2051 tokens through 64 experts of 2048 x 1024 (8 chosen) 12.3 -> 1.2 ms, where the loop was bound by
+// (2 chosen) 12.4 -> 8.2 ms, of 2051 tokens through 64 experts of 2048 x 1024 (8 chosen) 12.7 -> 1.1 ms, where the loop was bound by
 // its 1200 launches and a grid of a few tiles per expert.
 enum { GROUP_NONE = 0, GROUP_ROWS = 1, GROUP_REDUCE = 2 };
 constexpr int GROUP_ALIGN = 128;

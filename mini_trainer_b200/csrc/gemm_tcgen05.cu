@@ -10,7 +10,8 @@
 //   dgrad    dX[T,K] = dY[T,N] * W[N,K]     A K-major,  B MN-major (W read as [red=N, out=K])
 //   wgrad    dW[N,K] = dY[T,N]^T * X[T,K]   A MN-major, B MN-major (both read as [red=T, .])
 //
-// CTA layout (192 threads, one CTA per SM, grid = min(tiles, SMs)):
+// CTA layout (192 threads, one CTA per SM, grid = min(work items, SMs); an item is a tile, or one
+// split of its reduction):
 //   warp 0     TMA producer: fills a STAGES-deep ring of {A 128x64, B 256x64} tiles
 //   warp 1     allocates 512 TMEM columns (two 128x256 fp32 accumulators) and issues the MMAs
 //   warps 2-5  epilogue: each reads its 32-lane quarter of the accumulator, adds bias / residual,

@@ -415,14 +415,14 @@ class NativeOps:
 
     # -- attention --------------------------------------------------------------------
     def _cached(self, cu_host, what: tuple):
-        """What ``_keep`` has kept for this minibatch (its list of sequence starts), or ``None``."""
+        """What ``_keep`` has kept for this minibatch (its list of sequence starts, as it reads now), or ``None``."""
         hit = self._attn_plan_cache.get((id(cu_host),) + what)
-        return hit[1] if hit is not None and hit[0] is cu_host else None
+        return hit[2] if hit is not None and hit[0] is cu_host and hit[1] == tuple(cu_host) else None
 
     def _keep(self, cu_host, what: tuple, value):
         if len(self._attn_plan_cache) > 16:
             self._attn_plan_cache.clear()
-        self._attn_plan_cache[(id(cu_host),) + what] = (cu_host, value)
+        self._attn_plan_cache[(id(cu_host),) + what] = (cu_host, tuple(cu_host), value)
         return value
 
     def _attn_plan(self, cu_host, block, most_work_last_block: bool):

@@ -92,6 +92,23 @@ def test_attention_forward_launches_the_chosen_form():
             assert out.shape == (cu[-1], hq * 64) and lse.shape == (hq, cu[-1])
 
 
+def test_attention_plan_follows_a_list_that_is_filled_again():
+    ops = make_ops()
+    ops.sms, ops.attention_impl = 148, "native"
+    ops._attn_table = lambda cu, block, last: torch.tensor([[a, b - a, 0] for a, b in zip(cu[:-1], cu[1:])], dtype=torch.int32)
+    cu, hq, hkv, d = [0, 128, 2048], 16, 4, 64
+    qkv, o = torch.empty(2048, 24 * d, dtype=torch.bfloat16), torch.empty(2048, hq * d, dtype=torch.bfloat16)
+    for lens in ([128, 1920], [1000, 1048], [2048], [64] * 32):
+        cu[:] = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        for _ in range(2):
+            ops.attention(qkv, None, cu, max(lens), hq, hkv, d)
+            assert ops._cached(cu, ("fwd", hq, hkv, d))[2][:, 1].tolist() == lens
+            ops.attention_bwd(o, qkv, o, torch.empty(hq, 2048), None, cu, max(lens), hq, hkv, d)
+            assert ops._cached(cu, ("bwd", hq, hkv, d))[0][:, 1].tolist() == lens
+
+
 # (lengths, query heads, kv heads, range of CTAs per key block): nothing to divide, short samples, short batches, full ones
 @pytest.mark.parametrize("lens,hq,hkv,lo,hi", [([2048], 8, 8, 1, 1), ([128] * 16, 32, 8, 1, 1), ([110] * 100, 4, 1, 1, 1), ([16384], 32, 8, 1, 1),
                                                ([1024], 12, 2, 6, 6), ([2048], 14, 2, 7, 7), ([8192], 24, 2, 2, 3), ([4096], 16, 4, 2, 2),

@@ -114,6 +114,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  pdl_wait();   // the work table comes first
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit = blockIdx.x / p.splits, sub = blockIdx.x - unit * p.splits;
   const int item = unit / p.Hkv, hk = unit % p.Hkv;
@@ -177,6 +178,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
             tma_load_2d(smem + L::OFF_DO + kb * 16384, &tm_do, do_full, h * D + kb * 64, seq_start + i * AB_B);
           if (++i == nq) { i = jblk; ++h; }
         }
+        pdl_trigger();   // what is left is the last iteration and the stores of dK and dV
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issuer
@@ -491,6 +493,8 @@ done:
 // reading dO and O once: 16 384 tokens x 32 heads x 128 63 us (one warp per row with 4-byte loads: 97 us).
 __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o, long long ldo, const __nv_bfloat16* __restrict__ dout,
                                                         long long lddo, float* __restrict__ delta, int T, int Hq, int D) {
+  pdl_trigger();
+  pdl_wait();
   const int lanes = D >> 3;   // 8 or 16: a power of two that divides the warp
   const long long x = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long row = x / lanes;
@@ -515,6 +519,8 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
 // dqkv[t, 0:Hq*D] = bf16(dq_acc[t, :])
 __global__ void __launch_bounds__(256) attn_dq_store_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dqkv, long long ldq,
                                                            long long T, int HqD) {
+  pdl_trigger();
+  pdl_wait();
   // grid = (tokens, column blocks): no 64-bit division per thread
   const long long t = blockIdx.x;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
@@ -532,7 +538,7 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem<D>::TOTAL) != cudaSuccess) return -4;
     configured = true;
   }
-  kern<<<n_items * p.Hkv * p.splits, AB_THREADS, AttBwdSmem<D>::TOTAL, st>>>(a, b, c, p);
+  launch_pdl(kern, n_items * p.Hkv * p.splits, AB_THREADS, AttBwdSmem<D>::TOTAL, st, a, b, c, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -557,12 +563,12 @@ extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, l
   rc = make_tmap_2d_f32(&tdq, dq_acc, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(Hq) * D, 32, 128);
   if (rc) return rc - 20;
   const long long delta_threads = static_cast<long long>(T) * Hq * (D / 8);
-  attn_delta_kernel<<<static_cast<int>((delta_threads + 255) / 256), 256, 0, st>>>(
+  launch_pdl(attn_delta_kernel, static_cast<int>((delta_threads + 255) / 256), 256, 0, st, 
       reinterpret_cast<const __nv_bfloat16*>(out), ldo, reinterpret_cast<const __nv_bfloat16*>(dout), lddo, delta, T, Hq, D);
   AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, splits,
                  part, counters, epoch, scale, status};
   rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, p, n_items, st);
   if (rc) return rc;
-  attn_dq_store_kernel<<<dim3(static_cast<unsigned>(T), (Hq * D / 8 + 255) / 256), 256, 0, st>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, T, Hq * D);
+  launch_pdl(attn_dq_store_kernel, dim3(static_cast<unsigned>(T), (Hq * D / 8 + 255) / 256), 256, 0, st, dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, T, Hq * D);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     tma_prefetch_desc(&tmap);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  pdl_wait();   // nothing so far has touched global memory
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
           }
           ++units;
         }
+        pdl_trigger();   // what is left is the last key tiles' softmax and products
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------------ MMA issuer
@@ -387,7 +389,7 @@ static int launch_fwd(const CUtensorMap& tm, const AttFwdParams& p, cudaStream_t
   }
   const long long units = static_cast<long long>(p.n_items) * (p.row_pairs ? p.Hq : p.Hq / 2);
   if (units > (1 << 30)) return -10;
-  kern<<<static_cast<int>(units < sms ? units : sms), ATT_THREADS, AttFwdSmem<D>::TOTAL, st>>>(tm, p);
+  launch_pdl(kern, static_cast<int>(units < sms ? units : sms), ATT_THREADS, AttFwdSmem<D>::TOTAL, st, tm, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_one_kernel(const __gr
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+  pdl_wait();   // the work table comes first
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int item = blockIdx.x / p.Hq, h = blockIdx.x % p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_one_kernel(const __gr
         for (int kb = 0; kb < KB; ++kb)
           tma_load_2d(smem + L::OFF_V + s * L::KV_BYTES + kb * 16384, &tmap, &v_full[s], (p.Hq + p.Hkv + hk) * D + kb * 64, row);
       }
+      pdl_trigger();   // what is left is the last key tiles' softmax and products
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -345,7 +347,7 @@ static int launch(const CUtensorMap& tm, const Params& p, int n_items, cudaStrea
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::TOTAL) != cudaSuccess) return -4;
     configured = true;
   }
-  kern<<<n_items * p.Hq, ATT_THREADS, Smem<D>::TOTAL, st>>>(tm, p);
+  launch_pdl(kern, n_items * p.Hq, ATT_THREADS, Smem<D>::TOTAL, st, tm, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -82,6 +82,8 @@ __global__ void __launch_bounds__(EW_THREADS) norm_fwd_kernel(const __nv_bfloat1
                                                              const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                              float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, int T,
                                                              int H, int lanes, int* status) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t norm_smem[];
   __shared__ uint64_t full[NORM_STAGES];
   __shared__ float red[2][2][EW_THREADS / 32];   // [parity of the row set][mean, square]
@@ -179,6 +181,8 @@ template <int VPT>
 __global__ void __launch_bounds__(EW_THREADS) layernorm_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                                   const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                                   float* __restrict__ mean_out, float* __restrict__ rstd_out, float eps, int H) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const __nv_bfloat16* xr = x + row * H;
@@ -235,6 +239,8 @@ __global__ void __launch_bounds__(512) norm_bwd_kernel(const __nv_bfloat16* __re
                                                       const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ add_to,
                                                       __nv_bfloat16* __restrict__ dx, float* __restrict__ dwp, int T, int H, int stages,
                                                       int* status) {
+  pdl_trigger();
+  pdl_wait();
   constexpr bool KEEP = VPT <= 2;   // wider rows form xhat and g again after the reduction instead of holding them
   extern __shared__ __align__(128) uint8_t norm_smem[];
   __shared__ uint64_t full[8];
@@ -363,6 +369,8 @@ __global__ void __launch_bounds__(512) norm_bwd_kernel(const __nv_bfloat16* __re
 // barrier and the many blocks took longer than the sum (colsum of 8 x 896: 6.3 us, 4.7 like this; below 512 columns there are few blocks).
 __global__ void __launch_bounds__(512) reduce_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
                                                          int R, int C, int D) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[16][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -381,6 +389,8 @@ __global__ void __launch_bounds__(512) reduce_rows_kernel(const float* __restric
 }
 __global__ void __launch_bounds__(256) reduce_few_rows_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out_a, __nv_bfloat16* __restrict__ out_b,
                                                              int R, int C, int D) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= C) return;
   float s = 0.f;
@@ -398,6 +408,8 @@ constexpr int ROPE_HPT = 4;
 __global__ void __launch_bounds__(EW_THREADS) rope_kernel(__nv_bfloat16* __restrict__ qkv, const int* __restrict__ pos,
                                                          const float* __restrict__ inv_freq, int T, long long ld,
                                                          int n_heads, int D, float sign) {
+  pdl_trigger();
+  pdl_wait();
   const int half = D >> 1;
   const int vec_per_tok = half >> 3;  // 8 frequencies per thread
   const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -494,6 +506,8 @@ __global__ void __launch_bounds__(EW_THREADS) head_rmsnorm_fwd_kernel(__nv_bfloa
                                                                      float* __restrict__ rstd_out, const int* __restrict__ pos,
                                                                      const float* __restrict__ inv_freq, float eps, long long n_items, int groups,
                                                                      long long ld, int n_q, int n_heads) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int D = EPL * 32;
   const long long r = static_cast<long long>(blockIdx.x) * (EW_THREADS / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -545,6 +559,8 @@ __global__ void __launch_bounds__(EW_THREADS) head_rmsnorm_bwd_kernel(__nv_bfloa
                                                                      const int* __restrict__ pos, const float* __restrict__ inv_freq,
                                                                      long long n_items, int groups, long long ld, long long ld_pre, int n_q,
                                                                      int n_heads) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int D = EPL * 32;
   constexpr int WARPS = EW_THREADS / 32;
   __shared__ float sm[WARPS][2][D];
@@ -637,6 +653,8 @@ __device__ __forceinline__ float glu_act_grad(float g) {
 template <int ACT>
 __global__ void __launch_bounds__(EW_THREADS) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act,
                                                                long long T, int F) {
+  pdl_trigger();
+  pdl_wait();
   // grid = (tokens, column blocks): no 64-bit division per thread
   const long long t = blockIdx.x;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
@@ -654,6 +672,8 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_fwd_kernel(const __nv_bfloa
 template <bool WITH_ACT, int ACT>
 __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(__nv_bfloat16* dact, const __nv_bfloat16* __restrict__ gu,
                                                                __nv_bfloat16* __restrict__ dgu, long long T, int F) {
+  pdl_trigger();
+  pdl_wait();
   // grid = (tokens, column blocks): no 64-bit division per thread
   const long long t = blockIdx.x;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
@@ -685,6 +705,8 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(__nv_bfloat16* d
 // WITH_ACT: the forward output is also produced, written over dy, for a backward that did not keep it.
 template <int ACT>
 __global__ void __launch_bounds__(EW_THREADS) act_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+  pdl_trigger();
+  pdl_wait();
   const long long i0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i0 >= n) return;
   bf16x8 v; v.load(x + i0);
@@ -695,6 +717,8 @@ __global__ void __launch_bounds__(EW_THREADS) act_fwd_kernel(const __nv_bfloat16
 }
 template <bool WITH_ACT, int ACT>
 __global__ void __launch_bounds__(EW_THREADS) act_bwd_kernel(__nv_bfloat16* dy, const __nv_bfloat16* __restrict__ x, __nv_bfloat16* dx, long long n) {
+  pdl_trigger();
+  pdl_wait();
   const long long i0 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i0 >= n) return;
   bf16x8 v, d; v.load(x + i0); d.load(dy + i0);
@@ -714,6 +738,8 @@ __global__ void __launch_bounds__(EW_THREADS) act_bwd_kernel(__nv_bfloat16* dy, 
 // and code 60 is recorded in the status word, which the host turns into an exception.
 __global__ void __launch_bounds__(128) embedding_fwd_kernel(const __nv_bfloat16* __restrict__ w, const long long* __restrict__ ids,
                                                            __nv_bfloat16* __restrict__ out, int H, int V, int* status) {
+  pdl_trigger();
+  pdl_wait();
   const long long t = blockIdx.x;
   const long long id = ids[t];
   __nv_bfloat16* dst = out + t * H;
@@ -734,6 +760,8 @@ __global__ void __launch_bounds__(128) embedding_fwd_kernel(const __nv_bfloat16*
 __global__ void __launch_bounds__(128) embedding_bwd_kernel(__nv_bfloat16* __restrict__ dw, const long long* __restrict__ sorted_ids,
                                                            const long long* __restrict__ order, const __nv_bfloat16* __restrict__ dx,
                                                            int T, int H, int V, int* status) {
+  pdl_trigger();
+  pdl_wait();
   const int j = blockIdx.x;
   const long long id = sorted_ids[j];
   if (j > 0 && sorted_ids[j - 1] == id) return;
@@ -780,6 +808,8 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
                                                          const long long* __restrict__ targets, float* __restrict__ loss,
                                                          __nv_bfloat16* dlogits, long long ldd, int V, float grad_scale,
                                                          long long ignore_index) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   const long long row = blockIdx.x;
   const LogitT* lr = logits + row * ld;
@@ -850,6 +880,8 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
 template <int V, int UNROLL>
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restrict__ part,
                                                             int T, int N) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[8][32 * V];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + lane) * V;
@@ -889,6 +921,8 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 // acc = (accumulate ? acc : 0) + src   (fp32 accumulator, bf16 or fp32 source)
 template <typename SrcT>
 __global__ void __launch_bounds__(EW_THREADS) accumulate_kernel(float* __restrict__ acc, const SrcT* __restrict__ src, long long n, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i >= n) return;
   float f[8];
@@ -908,6 +942,8 @@ __global__ void __launch_bounds__(EW_THREADS) accumulate_kernel(float* __restric
 
 // dst(bf16) = (accumulate ? dst : 0) + src(fp32)
 __global__ void __launch_bounds__(EW_THREADS) f32_to_bf16_kernel(__nv_bfloat16* __restrict__ dst, const float* __restrict__ src, long long n, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 8;
   if (i >= n) return;
   const float4 a = *reinterpret_cast<const float4*>(src + i), b = *reinterpret_cast<const float4*>(src + i + 4);
@@ -922,6 +958,8 @@ __global__ void __launch_bounds__(EW_THREADS) f32_to_bf16_kernel(__nv_bfloat16* 
 
 // out[0] += sum(x^2): per-block partial sums combined with one atomic per block.
 __global__ void __launch_bounds__(EW_THREADS) sumsq_kernel(const float* __restrict__ x, long long n, float* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   float s = 0.f;
   for (long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4; i < n;
@@ -939,6 +977,8 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
                                                           const float* __restrict__ grad, __nv_bfloat16* __restrict__ param,
                                                           long long n, float lr, float beta1, float beta2, float eps, float wd,
                                                           float inv_bc1, float inv_sqrt_bc2, const float* __restrict__ coef) {
+  pdl_trigger();
+  pdl_wait();
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (i >= n) return;
   const float c = coef[0];
@@ -977,8 +1017,8 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
 
 static inline int cdiv(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 static void reduce_rows(const float* part, void* out_a, void* out_b, int R, int C, int D, cudaStream_t st) {
-  if (R <= 16 && C >= 512) reduce_few_rows_kernel<<<cdiv(C, 256), 256, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
-  else reduce_rows_kernel<<<cdiv(C, 32), 512, 0, st>>>(part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
+  if (R <= 16 && C >= 512) launch_pdl(reduce_few_rows_kernel, cdiv(C, 256), 256, 0, st, part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
+  else launch_pdl(reduce_rows_kernel, cdiv(C, 32), 512, 0, st, part, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, R, C, D);
 }
 static inline int launch_ok() { return cudaGetLastError() == cudaSuccess ? 0 : -5; }
 static int num_sms() {
@@ -1013,7 +1053,7 @@ static int launch_norm_fwd(const void* x, const void* w, const void* b, void* y,
     const int most = num_sms() * resident;
     if (grid > most) grid = most;
   }
-  kern<<<grid, EW_THREADS, smem, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, T, H, lanes, status);
+  launch_pdl(kern, grid, EW_THREADS, smem, st, (const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, T, H, lanes, status);
   return launch_ok();
 }
 
@@ -1034,7 +1074,7 @@ static int norm_fwd(const void* x, const void* w, const void* b, void* y, float*
     const long long n = static_cast<long long>(T) * H;
     const bool bulk = H <= 1024 ? T >= 1024 : (H <= 2048 ? n >= 6000000 : n >= 24000000 && !(lanes == EW_THREADS && vpt == 3));
     if (!bulk) {
-#define LF(V) layernorm_row_kernel<V><<<T, EW_THREADS, 0, st>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, H)
+#define LF(V) launch_pdl(layernorm_row_kernel<V>, T, EW_THREADS, 0, st, (const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, mean, rstd, eps, H)
       const int v = cdiv(H, 8 * EW_THREADS);
       if (v <= 1) LF(1); else if (v == 2) LF(2); else if (v == 3) LF(3); else LF(4);
 #undef LF
@@ -1089,7 +1129,7 @@ static int launch_norm_bwd(const void* dy, const void* x, const float* mean, con
   const int stage = H * 2 * (add_to != nullptr ? 3 : 2), per_sm = cdiv(blocks, num_sms());
   int stages = most / (per_sm * stage);
   stages = stages > 4 ? 4 : (stages < 2 ? 2 : stages);
-  kern<<<blocks, threads, stages * stage, st>>>((const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)w, (const bf16*)add_to, (bf16*)dx, dwp, T, H,
+  launch_pdl(kern, blocks, threads, stages * stage, st, (const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)w, (const bf16*)add_to, (bf16*)dx, dwp, T, H,
                                                 stages, status);
   return launch_ok();
 }
@@ -1145,7 +1185,7 @@ int mtb200_rope(void* qkv, const int* pos, const float* inv_freq, int T, long lo
   if (T <= 0) return 0;
   if (D % 16 || ld % 8) return -10;
   const long long n = static_cast<long long>(T) * (D / 16);
-  rope_kernel<<<dim3(cdiv(n, EW_THREADS), cdiv(n_heads, ROPE_HPT)), EW_THREADS, 0, st>>>((bf16*)qkv, pos, inv_freq, T, ld, n_heads, D,
+  launch_pdl(rope_kernel, dim3(cdiv(n, EW_THREADS), cdiv(n_heads, ROPE_HPT)), EW_THREADS, 0, st, (bf16*)qkv, pos, inv_freq, T, ld, n_heads, D,
                                                                                         inverse ? -1.f : 1.f);
   return launch_ok();
 }
@@ -1164,7 +1204,7 @@ int mtb200_head_rmsnorm_fwd(void* qkv, const void* wq, const void* wk, void* pre
   const long long n_items = static_cast<long long>(T) * groups;
   const unsigned blocks = static_cast<unsigned>(cdiv(n_items, EW_THREADS / 32));
 #define HF(E, R) if (hpw == 1) HFW(E, R, 1); else HFW(E, R, HEADS_PER_WARP)
-#define HFW(E, R, W) head_rmsnorm_fwd_kernel<E, R, W><<<blocks, EW_THREADS, 0, st>>>((bf16*)qkv, (const bf16*)wq, (const bf16*)wk, (bf16*)pre, rstd, pos, inv_freq, eps, n_items, groups, ld, n_q, n_heads)
+#define HFW(E, R, W) launch_pdl(head_rmsnorm_fwd_kernel<E, R, W>, blocks, EW_THREADS, 0, st, (bf16*)qkv, (const bf16*)wq, (const bf16*)wk, (bf16*)pre, rstd, pos, inv_freq, eps, n_items, groups, ld, n_q, n_heads)
   if (inv_freq) { if (D == 64) { HF(2, true); } else if (D == 128) { HF(4, true); } else { HF(8, true); } }
   else { if (D == 64) { HF(2, false); } else if (D == 128) { HF(4, false); } else { HF(8, false); } }
 #undef HF
@@ -1190,7 +1230,7 @@ int mtb200_head_rmsnorm_bwd(void* dqkv, const void* pre, const float* rstd, cons
   const int groups = cdiv(n_heads, HEADS_PER_WARP);
   const long long n_items = static_cast<long long>(T) * groups;
   const int blocks = mtb200_head_rmsnorm_bwd_blocks(T, n_heads);
-#define HB(E, R) head_rmsnorm_bwd_kernel<E, R><<<blocks, EW_THREADS, 0, st>>>((bf16*)dqkv, (const bf16*)pre, rstd, (const bf16*)wq, (const bf16*)wk, dw_partial, pos, inv_freq, n_items, groups, ld, ld_pre, n_q, n_heads)
+#define HB(E, R) launch_pdl(head_rmsnorm_bwd_kernel<E, R>, blocks, EW_THREADS, 0, st, (bf16*)dqkv, (const bf16*)pre, rstd, (const bf16*)wq, (const bf16*)wk, dw_partial, pos, inv_freq, n_items, groups, ld, ld_pre, n_q, n_heads)
   if (inv_freq) { if (D == 64) HB(2, true); else if (D == 128) HB(4, true); else HB(8, true); }
   else { if (D == 64) HB(2, false); else if (D == 128) HB(4, false); else HB(8, false); }
 #undef HB
@@ -1202,14 +1242,14 @@ int mtb200_head_rmsnorm_bwd(void* dqkv, const void* pre, const float* rstd, cons
 int mtb200_swiglu_fwd(const void* gu, void* act, long long T, int F, cudaStream_t st) {
   if (T <= 0) return 0;
   if (F % 8) return -10;
-  swiglu_fwd_kernel<0><<<dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st>>>((const bf16*)gu, (bf16*)act, T, F);
+  launch_pdl(swiglu_fwd_kernel<0>, dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st, (const bf16*)gu, (bf16*)act, T, F);
   return launch_ok();
 }
 
 int mtb200_swiglu_bwd(const void* dact, const void* gu, void* dgu, long long T, int F, cudaStream_t st) {
   if (T <= 0) return 0;
   if (F % 8) return -10;
-  swiglu_bwd_kernel<false, 0><<<dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)const_cast<void*>(dact), (const bf16*)gu, (bf16*)dgu, T, F);
+  launch_pdl(swiglu_bwd_kernel<false, 0>, dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st, (bf16*)const_cast<void*>(dact), (const bf16*)gu, (bf16*)dgu, T, F);
   return launch_ok();
 }
 
@@ -1217,7 +1257,7 @@ int mtb200_swiglu_bwd(const void* dact, const void* gu, void* dgu, long long T, 
 int mtb200_swiglu_bwd_act(void* dact_inout, const void* gu, void* dgu, long long T, int F, cudaStream_t st) {
   if (T <= 0) return 0;
   if (F % 8) return -10;
-  swiglu_bwd_kernel<true, 0><<<dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)dact_inout, (const bf16*)gu, (bf16*)dgu, T, F);
+  launch_pdl(swiglu_bwd_kernel<true, 0>, dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st, (bf16*)dact_inout, (const bf16*)gu, (bf16*)dgu, T, F);
   return launch_ok();
 }
 
@@ -1225,19 +1265,19 @@ int mtb200_swiglu_bwd_act(void* dact_inout, const void* gu, void* dgu, long long
 int mtb200_geglu_fwd(const void* gu, void* act, long long T, int F, cudaStream_t st) {
   if (T <= 0) return 0;
   if (F % 8) return -10;
-  swiglu_fwd_kernel<1><<<dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st>>>((const bf16*)gu, (bf16*)act, T, F);
+  launch_pdl(swiglu_fwd_kernel<1>, dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st, (const bf16*)gu, (bf16*)act, T, F);
   return launch_ok();
 }
 int mtb200_geglu_bwd(const void* dact, const void* gu, void* dgu, long long T, int F, cudaStream_t st) {
   if (T <= 0) return 0;
   if (F % 8) return -10;
-  swiglu_bwd_kernel<false, 1><<<dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)const_cast<void*>(dact), (const bf16*)gu, (bf16*)dgu, T, F);
+  launch_pdl(swiglu_bwd_kernel<false, 1>, dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st, (bf16*)const_cast<void*>(dact), (const bf16*)gu, (bf16*)dgu, T, F);
   return launch_ok();
 }
 int mtb200_geglu_bwd_act(void* dact_inout, const void* gu, void* dgu, long long T, int F, cudaStream_t st) {
   if (T <= 0) return 0;
   if (F % 8) return -10;
-  swiglu_bwd_kernel<true, 1><<<dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)dact_inout, (const bf16*)gu, (bf16*)dgu, T, F);
+  launch_pdl(swiglu_bwd_kernel<true, 1>, dim3(static_cast<unsigned>(T), cdiv(F / 8, EW_THREADS)), EW_THREADS, 0, st, (bf16*)dact_inout, (const bf16*)gu, (bf16*)dgu, T, F);
   return launch_ok();
 }
 
@@ -1245,27 +1285,27 @@ int mtb200_geglu_bwd_act(void* dact_inout, const void* gu, void* dgu, long long 
 int mtb200_gelu_fwd(const void* x, void* y, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -10;
-  act_fwd_kernel<1><<<static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st>>>((const bf16*)x, (bf16*)y, n);
+  launch_pdl(act_fwd_kernel<1>, static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st, (const bf16*)x, (bf16*)y, n);
   return launch_ok();
 }
 int mtb200_gelu_bwd(const void* dy, const void* x, void* dx, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -10;
-  act_bwd_kernel<false, 1><<<static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)const_cast<void*>(dy), (const bf16*)x, (bf16*)dx, n);
+  launch_pdl(act_bwd_kernel<false, 1>, static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st, (bf16*)const_cast<void*>(dy), (const bf16*)x, (bf16*)dx, n);
   return launch_ok();
 }
 // Same, and dy_inout is overwritten with gelu_tanh(x); dx is another buffer.
 int mtb200_gelu_bwd_act(void* dy_inout, const void* x, void* dx, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8 || dx == dy_inout) return -10;
-  act_bwd_kernel<true, 1><<<static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st>>>((bf16*)dy_inout, (const bf16*)x, (bf16*)dx, n);
+  launch_pdl(act_bwd_kernel<true, 1>, static_cast<unsigned>(cdiv(n / 8, EW_THREADS)), EW_THREADS, 0, st, (bf16*)dy_inout, (const bf16*)x, (bf16*)dx, n);
   return launch_ok();
 }
 
 int mtb200_embedding_fwd(const void* w, const long long* ids, void* out, int T, int H, int V, int* status, cudaStream_t st) {
   if (T <= 0) return 0;
   if (H % 8) return -10;
-  embedding_fwd_kernel<<<T, 128, 0, st>>>((const bf16*)w, ids, (bf16*)out, H, V, status);
+  launch_pdl(embedding_fwd_kernel, T, 128, 0, st, (const bf16*)w, ids, (bf16*)out, H, V, status);
   return launch_ok();
 }
 
@@ -1273,7 +1313,7 @@ int mtb200_embedding_bwd(void* dw, const long long* sorted_ids, const long long*
                          int* status, cudaStream_t st) {
   if (T <= 0) return 0;
   if (H % 8) return -10;
-  embedding_bwd_kernel<<<T, 128, 0, st>>>((bf16*)dw, sorted_ids, order, (const bf16*)dx, T, H, V, status);
+  launch_pdl(embedding_bwd_kernel, T, 128, 0, st, (bf16*)dw, sorted_ids, order, (const bf16*)dx, T, H, V, status);
   return launch_ok();
 }
 
@@ -1282,7 +1322,7 @@ int mtb200_ce_fwd_bwd(const void* logits, long long ld, int logits_bf16, const f
                       void* dlogits, long long ldd, int R, int V, float grad_scale, long long ignore_index, cudaStream_t st) {
   if (R <= 0) return 0;
   if (V % 8 || ld % 8 || ldd % 8 || (stats && !logits_bf16)) return -10;
-#define CE(T, S) ce_fwd_bwd_kernel<T, S><<<R, 1024, 0, st>>>((const T*)logits, ld, stats, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index)
+#define CE(T, S) launch_pdl(ce_fwd_bwd_kernel<T, S>, R, 1024, 0, st, (const T*)logits, ld, stats, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index)
   if (stats) CE(bf16, true); else if (logits_bf16) CE(bf16, false); else CE(float, false);
 #undef CE
   return launch_ok();
@@ -1293,9 +1333,9 @@ static void launch_colsum(const void* x, long long ld, void* out, float* scratch
   const bool many = T >= 8192;   // at least four times eight rows per warp
   const bool wide = N % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (many || N > 1024);
   const dim3 grid(cdiv(N, wide ? 256 : 64), splits);
-  if (wide && many && N <= 5120) colsum_partial_kernel<8, 8><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
-  else if (wide) colsum_partial_kernel<8, 4><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
-  else colsum_partial_kernel<2, 4><<<grid, 256, 0, st>>>((const bf16*)x, ld, scratch, T, N);
+  if (wide && many && N <= 5120) launch_pdl(colsum_partial_kernel<8, 8>, grid, 256, 0, st, (const bf16*)x, ld, scratch, T, N);
+  else if (wide) launch_pdl(colsum_partial_kernel<8, 4>, grid, 256, 0, st, (const bf16*)x, ld, scratch, T, N);
+  else launch_pdl(colsum_partial_kernel<2, 4>, grid, 256, 0, st, (const bf16*)x, ld, scratch, T, N);
   reduce_rows(scratch, out, nullptr, splits, N, N, st);
 }
 
@@ -1310,15 +1350,15 @@ int mtb200_colsum(const void* x, long long ld, void* out, float* scratch, int T,
 int mtb200_accumulate(float* acc, const void* src, long long n, int src_is_f32, int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -10;
-  if (src_is_f32) accumulate_kernel<float><<<cdiv(n / 8, EW_THREADS), EW_THREADS, 0, st>>>(acc, (const float*)src, n, accumulate);
-  else accumulate_kernel<bf16><<<cdiv(n / 8, EW_THREADS), EW_THREADS, 0, st>>>(acc, (const bf16*)src, n, accumulate);
+  if (src_is_f32) launch_pdl(accumulate_kernel<float>, cdiv(n / 8, EW_THREADS), EW_THREADS, 0, st, acc, (const float*)src, n, accumulate);
+  else launch_pdl(accumulate_kernel<bf16>, cdiv(n / 8, EW_THREADS), EW_THREADS, 0, st, acc, (const bf16*)src, n, accumulate);
   return launch_ok();
 }
 
 int mtb200_f32_to_bf16(void* dst, const float* src, long long n, int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 8) return -10;
-  f32_to_bf16_kernel<<<cdiv(n / 8, EW_THREADS), EW_THREADS, 0, st>>>((bf16*)dst, src, n, accumulate);
+  launch_pdl(f32_to_bf16_kernel, cdiv(n / 8, EW_THREADS), EW_THREADS, 0, st, (bf16*)dst, src, n, accumulate);
   return launch_ok();
 }
 
@@ -1326,7 +1366,7 @@ int mtb200_sumsq(const float* x, long long n, float* out, cudaStream_t st) {
   if (n <= 0) return 0;
   if (n % 4) return -10;
   const int blocks = static_cast<int>(min(static_cast<long long>(num_sms() * 8), (n / 4 + EW_THREADS - 1) / EW_THREADS));
-  sumsq_kernel<<<blocks, EW_THREADS, 0, st>>>(x, n, out);
+  launch_pdl(sumsq_kernel, blocks, EW_THREADS, 0, st, x, n, out);
   return launch_ok();
 }
 
@@ -1338,9 +1378,9 @@ int mtb200_adamw(float* master, void* m, void* v, int state_is_f32, const float*
   const float inv_sqrt_bc2 = 1.f / sqrtf(1.f - powf(beta2, static_cast<float>(step)));
   const int blocks = cdiv(n / 4, EW_THREADS);
   if (state_is_f32)
-    adamw_kernel<float><<<blocks, EW_THREADS, 0, st>>>(master, (float*)m, (float*)v, grad, (bf16*)param, n, lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2, coef);
+    launch_pdl(adamw_kernel<float>, blocks, EW_THREADS, 0, st, master, (float*)m, (float*)v, grad, (bf16*)param, n, lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2, coef);
   else
-    adamw_kernel<bf16><<<blocks, EW_THREADS, 0, st>>>(master, (bf16*)m, (bf16*)v, grad, (bf16*)param, n, lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2, coef);
+    launch_pdl(adamw_kernel<bf16>, blocks, EW_THREADS, 0, st, master, (bf16*)m, (bf16*)v, grad, (bf16*)param, n, lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2, coef);
   return launch_ok();
 }
 

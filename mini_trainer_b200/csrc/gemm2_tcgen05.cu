@@ -126,6 +126,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  pdl_wait();   // nothing so far has touched global memory
   tc_fence_before();
   __syncthreads();
   cluster_sync();          // the partner's barriers are initialised before anything is sent to them
@@ -192,6 +193,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           }
         }
       }
+      if (!GATHER) pdl_trigger();   // what is left is a few products and the last epilogue
       if (GATHER && g.wait_ns != nullptr) {
         atomicAdd(g.wait_ns, waited_ns);
         atomicAdd(g.wait_ns + 1, 1ull);
@@ -324,7 +326,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int items = tiles * p.e.splits;
   p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
   static const GatherParams none{};
-  kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, p, gp ? *gp : none);
+  if constexpr (GATHER) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, p, *gp);
+  else if (2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, p, none);
+  else launch_pdl(kern, 2 * p.num_pairs, threads, SMEM, stream, ta, tb, td, p, none);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -221,6 +221,12 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
   if (lane == 0) p.counters[unit * 4 + q] = 0;
 }
 
+// Products of at most this many operations start under their predecessor's tail (launch_pdl). It saves about 2 us per launch whatever the
+// size; on the other hand CTAs that are placed as SMs fall free, instead of in order, take neighbouring tiles to distant SMs, and
+// long launches lose what that saves (with every product launched early: 1.5B block 1933 -> 1868 us, q/k-norm block 1786 -> 1723;
+// but 8B block 20.31 -> 20.42 ms, eight-expert layer 8.35 -> 8.56 ms, sixty-four experts 1140 -> 1148 us).
+constexpr double PDL_MAX_FLOPS = 1e12;
+
 // Grouped GEMM: one launch over the slabs of all experts of a mixture-of-experts layer. The rows of expert e are
 // [starts[e], starts[e] + counts[e]) of the gathered row buffers, starts are multiples of GROUP_ALIGN and the rows between the
 // slabs are zero, so a row tile never mixes experts and a reduction over a slab may run into its padding. The row counts are

@@ -93,6 +93,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     tma_prefetch_desc(&tmap_d);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  pdl_wait();   // nothing so far has touched global memory
   if (GROUP && warp == 2) fill_group_table<GROUP>(gtab, gr, BM, tiles_n, num_tiles, lane);
   tc_fence_before();
   __syncthreads();
@@ -187,6 +188,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
         }
       }
+      if (!GATHER && !GROUP) pdl_trigger();   // what is left is a few products and the last epilogue
       if (GATHER && g.wait_ns != nullptr) {   // exposed-communication accounting: how long this producer starved
         atomicAdd(g.wait_ns, waited_ns);
         atomicAdd(g.wait_ns + 1, 1ull);
@@ -402,7 +404,11 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int items = tiles * p.e.splits;
   const int grid = (GATHER || items >= g_num_sms) ? g_num_sms : items;
   static const GatherParams none{};
-  kern<<<grid, GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, p, gp ? *gp : none, grp ? *grp : GroupParams{});
+  // A gathering launch neither overlaps its predecessor nor lets a successor in: its CTAs are counted on to be resident. A long or grouped
+  // launch (PDL_MAX_FLOPS) starts behind its predecessor too.
+  if constexpr (GATHER) kern<<<grid, GEMM_THREADS + GATHER_EXTRA_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, p, *gp, GroupParams{});
+  else if (GROUP || 2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, p, none, grp ? *grp : GroupParams{});
+  else launch_pdl(kern, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, td, p, none, GroupParams{});
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -37,6 +37,8 @@ struct Vec8 {
 __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const long long* __restrict__ topi, int n, int E, int cap,
                                                                int* __restrict__ starts, int* __restrict__ counts,
                                                                int* __restrict__ pair_of, int* __restrict__ row_of, int* status) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int hist[GROUP_MAX];
   __shared__ int wsum[2][PLAN_THREADS / 32];
   __shared__ int start_sh;
@@ -90,6 +92,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const long long*
 // out[row] = scale * src[pair_of[row] / k], zeros in padding. Rows past the last slab are left alone.
 __global__ void __launch_bounds__(128) moe_gather_kernel(const bf16* __restrict__ src, const int* __restrict__ pair_of, const int* __restrict__ starts,
                                                         int E, int k, int H, float scale, bf16* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const long long row = blockIdx.x;
   if (row >= starts[E]) return;
   const int pair = pair_of[row];
@@ -133,6 +137,8 @@ template <int ACT>
 __global__ void __launch_bounds__(MOE_THREADS) moe_glu_bwd_kernel(bf16* __restrict__ du, const bf16* __restrict__ gu, const float* __restrict__ w,
                                                                  const int* __restrict__ pair_of, const int* __restrict__ starts, int E, int F,
                                                                  bf16* __restrict__ dgu, float* __restrict__ dw) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[MOE_THREADS / 32];
   const long long row = blockIdx.x;
   if (row >= starts[E]) return;
@@ -175,6 +181,8 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_glu_bwd_kernel(bf16* __restri
 __global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(const bf16* __restrict__ rows, const int* __restrict__ row_of,
                                                                  const float* __restrict__ w, const float* __restrict__ add,
                                                                  const bf16* __restrict__ base, float scale, int k, int H, bf16* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   const long long t = blockIdx.x;
   const int* ro = row_of + t * k;
   for (int c = threadIdx.x * 8; c < H; c += MOE_THREADS * 8) {
@@ -209,6 +217,8 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_combine_kernel(const bf16* __
 __global__ void __launch_bounds__(MOE_THREADS) moe_route_bwd_kernel(const float* __restrict__ probs, const long long* __restrict__ topi,
                                                                    const float* __restrict__ w, const float* __restrict__ dw, int renorm,
                                                                    int T, int E, int k, bf16* __restrict__ dlogits) {
+  pdl_trigger();
+  pdl_wait();
   const long long t = (static_cast<long long>(blockIdx.x) * MOE_THREADS + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -240,7 +250,7 @@ int mtb200_moe_plan(const long long* topi, int n, int E, int cap, int* starts, i
                     cudaStream_t st) {
   if (n <= 0) return 0;
   if (E <= 0 || E > GROUP_MAX || cap % GROUP_ALIGN || cap < static_cast<long long>(n) + static_cast<long long>(E) * (GROUP_ALIGN - 1)) return -10;
-  moe_plan_kernel<<<E, PLAN_THREADS, 0, st>>>(topi, n, E, cap, starts, counts, pair_of, row_of, status);
+  launch_pdl(moe_plan_kernel, E, PLAN_THREADS, 0, st, topi, n, E, cap, starts, counts, pair_of, row_of, status);
   return ok();
 }
 
@@ -248,7 +258,7 @@ int mtb200_moe_gather(const void* src, const int* pair_of, const int* starts, in
                       cudaStream_t st) {
   if (cap <= 0) return 0;
   if (H % 8 || k <= 0) return -10;
-  moe_gather_kernel<<<cap, 128, 0, st>>>((const bf16*)src, pair_of, starts, E, k, H, scale, (bf16*)out);
+  launch_pdl(moe_gather_kernel, cap, 128, 0, st, (const bf16*)src, pair_of, starts, E, k, H, scale, (bf16*)out);
   return ok();
 }
 
@@ -257,8 +267,8 @@ int mtb200_moe_glu_bwd(void* du, const void* gu, const float* w, const int* pair
                        void* dgu, float* dw, cudaStream_t st) {
   if (cap <= 0) return 0;
   if (F % 8) return -10;
-  if (act == 0) moe_glu_bwd_kernel<0><<<cap, MOE_THREADS, 0, st>>>((bf16*)du, (const bf16*)gu, w, pair_of, starts, E, F, (bf16*)dgu, dw);
-  else moe_glu_bwd_kernel<1><<<cap, MOE_THREADS, 0, st>>>((bf16*)du, (const bf16*)gu, w, pair_of, starts, E, F, (bf16*)dgu, dw);
+  if (act == 0) launch_pdl(moe_glu_bwd_kernel<0>, cap, MOE_THREADS, 0, st, (bf16*)du, (const bf16*)gu, w, pair_of, starts, E, F, (bf16*)dgu, dw);
+  else launch_pdl(moe_glu_bwd_kernel<1>, cap, MOE_THREADS, 0, st, (bf16*)du, (const bf16*)gu, w, pair_of, starts, E, F, (bf16*)dgu, dw);
   return ok();
 }
 
@@ -266,7 +276,7 @@ int mtb200_moe_combine(const void* rows, const int* row_of, const float* w, cons
                        int H, void* out, cudaStream_t st) {
   if (T <= 0) return 0;
   if (H % 8 || k <= 0) return -10;
-  moe_combine_kernel<<<T, MOE_THREADS, 0, st>>>((const bf16*)rows, row_of, w, add, (const bf16*)base, scale, k, H, (bf16*)out);
+  launch_pdl(moe_combine_kernel, T, MOE_THREADS, 0, st, (const bf16*)rows, row_of, w, add, (const bf16*)base, scale, k, H, (bf16*)out);
   return ok();
 }
 
@@ -274,7 +284,7 @@ int mtb200_moe_route_bwd(const float* probs, const long long* topi, const float*
                          void* dlogits, cudaStream_t st) {
   if (T <= 0) return 0;
   if (E <= 0 || k <= 0) return -10;
-  moe_route_bwd_kernel<<<(T + MOE_THREADS / 32 - 1) / (MOE_THREADS / 32), MOE_THREADS, 0, st>>>(probs, topi, w, dw, renorm, T, E, k, (bf16*)dlogits);
+  launch_pdl(moe_route_bwd_kernel, (T + MOE_THREADS / 32 - 1) / (MOE_THREADS / 32), MOE_THREADS, 0, st, probs, topi, w, dw, renorm, T, E, k, (bf16*)dlogits);
   return ok();
 }
 

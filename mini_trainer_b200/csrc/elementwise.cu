@@ -628,28 +628,8 @@ __global__ void __launch_bounds__(EW_THREADS) head_rmsnorm_bwd_kernel(__nv_bfloa
 // ------------------------------------------------------------------------------ gated MLP activations
 // act(gate) * up over gu = [gate | up]. ACT 0: SiLU (SwiGLU: Llama, Qwen, Mistral, Granite, Mixtral, Phi-3);
 // ACT 1: tanh-approximated GELU (GeGLU: Gemma's gelu_pytorch_tanh).
-// gelu_gate is in ptx.cuh: 0.5 * (1 + tanh(u)) = sigmoid(2 u), which costs what SiLU costs (with tanhf the GELU kernels were bound
+// glu_act and gelu_gate are in ptx.cuh: 0.5 * (1 + tanh(u)) = sigmoid(2 u), which costs what SiLU costs (with tanhf the GELU kernels were bound
 // by instructions: 7001 x 12288 forward 92 -> 69 us).
-template <int ACT>
-__device__ __forceinline__ float glu_act(float g) {
-  if constexpr (ACT == 0) {
-    return __fdividef(g, 1.f + __expf(-g));
-  } else {
-    return g * gelu_gate(g);
-  }
-}
-// d act(g) / d g
-template <int ACT>
-__device__ __forceinline__ float glu_act_grad(float g) {
-  if constexpr (ACT == 0) {
-    const float sig = __fdividef(1.f, 1.f + __expf(-g));
-    return sig * (1.f + g * (1.f - sig));
-  } else {
-    const float s = gelu_gate(g);
-    return s + g * s * (1.f - s) * 1.5957691216057308f * (1.f + 0.134145f * g * g);
-  }
-}
-
 template <int ACT>
 __global__ void __launch_bounds__(EW_THREADS) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ act,
                                                                long long T, int F) {

@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "gather.cuh"
+#include "gemm_act.cuh"
 #include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 
@@ -53,7 +54,10 @@ struct Params {
   int* status;
   int num_pairs;
   EpiParams e;
+  ActParams act;   // ACT instances
 };
+
+constexpr int threads_of(int act) { return act == ACT_NONE ? THREADS : 64 + 32 * ACT_WARPS; }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -87,10 +91,10 @@ __device__ __forceinline__ void mbar_arrive_cta0(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & PEER_MASK) : "memory");
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS, 1)
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-             const __grid_constant__ CUtensorMap tmap_d, Params p,
+             const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ ActMaps<ACT> maps, Params p,
              const __grid_constant__ GatherParams g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -114,7 +118,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], ACT ? 2 * ACT_WARPS : 8); }
     *abort_flag = 0;
     *verified = 0;
     fence_mbar_init();
@@ -165,7 +169,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         tile_coords(w % num_tiles, tm, tn);
         k_range(w / num_tiles, kb0, kb1);
         const int row0 = tm * 2 * BM + rank * BM;        // this CTA's rows of A
-        const int col0 = tn * BN + rank * BNH;           // this CTA's half of the B tile
+        // this CTA's half of the B tile; with a gated activation CTA 0 has the gate's weight and CTA 1 up's
+        const int col0 = ACT == ACT_GLU ? tn * BNH + static_cast<int>(rank) * p.act.F : tn * BN + rank * BNH;
         if (GATHER) {
           if (!wait_verified(verified, tl, abort_flag, waited_ns)) { *abort_flag = 1; atomicExch(p.status, 55); goto done; }
           asm volatile("fence.proxy.async;" ::: "memory");   // peer data was written with ordinary stores, TMA reads it
@@ -254,9 +259,9 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // ------------------------------------------------------------------ gather warps (6..13, both CTAs)
     gather_chunks(g, threadIdx.x - THREADS, ticket_slot);
   } else {
-    // ------------------------------------------------------------------ epilogue (both CTAs)
+    // ------------------------------------------------------------------ epilogue (both CTAs; warps 2..5, with an activation 2..9)
     const int q = warp & 3;
-    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + q * 2 * STORE_BOX, -1, 0};
+    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + (ACT ? (warp - 2) * 2 * ACT_BOX : q * 2 * STORE_BOX), -1, 0};
     uint32_t tl = 0;
     for (int w = pair; w < num_items; w += p.num_pairs, ++tl) {
       const int t = w % num_tiles;
@@ -266,7 +271,10 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag)) { atomicExch(p.status, 54); goto done; }
       tc_fence_after();
-      epilogue_quarter<OUT_F32, !GATHER, STATS, EXTRA>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
+      if constexpr (ACT != ACT_NONE)
+        epilogue_act<ACT>(p.e, p.act, maps, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn, q,
+                              (warp - 2) >> 2, lane);
+      else epilogue_quarter<OUT_F32, !GATHER, STATS, EXTRA>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, tm * 2 * BM + rank * BM, tn * BN, q, lane,
                                 2 * t + static_cast<int>(rank), w / num_tiles, false);
       tc_fence_before();
       __syncwarp();
@@ -274,7 +282,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     }
   }
 done:
-  if (warp >= 2 && warp < 6 && lane == 0) drain_boxes();
+  if (warp >= 2 && (ACT || warp < 6) && lane == 0) drain_boxes();
   tc_fence_before();
   __syncthreads();
   cluster_sync();          // nobody tears down while the partner may still signal or read
@@ -308,11 +316,11 @@ static int co_resident_pairs() {
   return pairs;
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
-                  long long part_bytes = 0) {
-  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA>;
-  constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : THREADS;
+                  long long part_bytes = 0, const ActMaps<ACT>& maps = ActMaps<ACT>{}) {
+  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA, ACT>;
+  constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT);
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -4;
@@ -326,9 +334,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int items = tiles * p.e.splits;
   p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
   static const GatherParams none{};
-  if constexpr (GATHER) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, p, *gp);
-  else if (2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, p, none);
-  else launch_pdl(kern, 2 * p.num_pairs, threads, SMEM, stream, ta, tb, td, p, none);
+  if constexpr (GATHER) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, *gp);
+  else if (2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, none);
+  else launch_pdl(kern, 2 * p.num_pairs, threads, SMEM, stream, ta, tb, td, maps, p, none);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -344,6 +352,14 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
   if (rc) return rc - 20;
   Params p{M, N, K, status, 0, EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0}};
   return launch<false, false, false, true>(ta, tb, td, p, stream, &g);
+}
+
+// Products with an activation in the epilogue; called by mtb200_gemm_act.
+int launch_act(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
+               int* status, cudaStream_t stream) {
+  const Params p{e.M, e.N, K, status, 0, e, a};
+  if (mode == ACT_GLU) return launch<false, false, false, false, false, false, ACT_GLU>(ta, tb, m.gate, p, stream, nullptr, 0, m);
+  return launch<false, false, false, false, false, false, ACT_PLAIN>(ta, tb, m.gate, p, stream, nullptr, 0, ActMaps<ACT_PLAIN>{m.gate, m.up, m.act});
 }
 
 }  // namespace g2

@@ -28,6 +28,7 @@
 #include <stdlib.h>
 
 #include "gather.cuh"
+#include "gemm_act.cuh"
 #include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 
@@ -39,6 +40,7 @@ constexpr int A_TILE_BYTES = BM * BK * 2;   // 16 KB
 constexpr int B_TILE_BYTES = BN * BK * 2;   // 32 KB
 constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
 constexpr int GEMM_THREADS = 192;
+constexpr int gemm_threads(int act) { return act == ACT_NONE ? GEMM_THREADS : 64 + 32 * ACT_WARPS; }
 constexpr int GROUP_M = 16;
 constexpr int GATHER_GROUP_N = 4;   // column-tiles per band in the all-gather variant
 constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + EPI_SMEM + 1024 /*alignment slack*/ + 256 /*barriers*/;
@@ -50,6 +52,7 @@ struct GemmParams {
   unsigned wait_hint_ns;  // suspend-time hint of the epilogue's and the MMA thread's long waits (0: plain polling)
   unsigned wait_limit_us; // > 0: every pipeline wait is bounded by this time instead of a poll count (fused reduce + GEMM)
   EpiParams e;            // output, epilogue operands, split-K
+  ActParams act;          // ACT instances
 };
 
 // The fused all-gather variant (GATHER = true) adds the gather warps and the flag checker of gather.cuh;
@@ -58,11 +61,12 @@ struct GemmParams {
 // buffers (reduce_chunks in gather.cuh): the gradient reduce-scatter with ownership by tensor, fused into the GEMM
 // that consumes the reduced gradient (OSFT factor gradients).
 // GROUP: one launch over the expert slabs of a mixture-of-experts layer (gemm_epilogue.cuh).
-// STATS: softmax statistics of the output rows (EpiParams). EXTRA: bias or residual.
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true>
-__global__ void __launch_bounds__(GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : GEMM_THREADS, 1)
+// STATS: softmax statistics of the output rows (EpiParams). EXTRA: bias or residual. ACT: an activation in the epilogue (gemm_act.cuh).
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true,
+          int ACT = ACT_NONE>
+__global__ void __launch_bounds__(GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : gemm_threads(ACT), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-            const __grid_constant__ CUtensorMap tmap_d, GemmParams p,
+            const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ ActMaps<ACT> maps, GemmParams p,
             const __grid_constant__ GatherParams g, GroupParams gr) {
   __shared__ GroupTable gtab;   // unused (and not allocated) outside the grouped forms
   extern __shared__ uint8_t smem_raw[];
@@ -84,7 +88,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 4); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], ACT ? ACT_WARPS : 4); }
     *abort_flag = 0;
     *verified = 0;
     fence_mbar_init();
@@ -183,7 +187,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
               else tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[s], tn * BN + j * 64, k_row + kb * BK);
             }
           } else {
-            if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN, e);
+            if constexpr (ACT == ACT_GLU) {   // 128 rows of the gate's weight and the same of up's
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const int row = (j ? p.act.F : 0) + tn * (BN / 2);
+                if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb + j * (B_TILE_BYTES / 2), &tmap_b, &full_bar[s], kb * BK, row, e);
+                else tma_load_2d(sb + j * (B_TILE_BYTES / 2), &tmap_b, &full_bar[s], kb * BK, row);
+              }
+            } else if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN, e);
             else tma_load_2d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN);
           }
         }
@@ -257,11 +268,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     if constexpr (REDUCE) reduce_chunks<8>(g, threadIdx.x - GEMM_THREADS, ticket_slot);
     else gather_chunks(g, threadIdx.x - GEMM_THREADS, ticket_slot);
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------------ epilogue (warps 2..5; with an activation 2..9)
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t tl = 0;
     int e = 0;
-    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + q * 2 * STORE_BOX, -1, 0};
+    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + (ACT ? (warp - 2) * 2 * ACT_BOX : q * 2 * STORE_BOX), -1, 0};
     for (int w = blockIdx.x; w < num_items; w += gridDim.x, ++tl) {
       const int t = w % num_tiles;
       int tm, tn, row0;
@@ -273,7 +284,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       const uint32_t aph = (tl >> 1) & 1;
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 4); goto done; }
       tc_fence_after();
-      epilogue_quarter<OUT_F32, !GATHER && !GROUP, STATS, EXTRA && !GROUP>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
+      if constexpr (ACT != ACT_NONE)
+        epilogue_act<ACT>(p.e, p.act, maps, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn, q, (warp - 2) >> 2, lane);
+      else epilogue_quarter<OUT_F32, !GATHER && !GROUP, STATS, EXTRA && !GROUP>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
                                                    w / num_tiles, GROUP == GROUP_REDUCE && gr.counts[e] == 0);
       tc_fence_before();
       __syncwarp();
@@ -281,7 +294,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     }
   }
 done:
-  if (warp >= 2 && warp < 6 && lane == 0) drain_boxes();
+  if (warp >= 2 && (ACT || warp < 6) && lane == 0) drain_boxes();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -359,6 +372,21 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
+// bf16 map for the boxes of the activation epilogues: 32 rows x 32 columns, 64B-swizzled.
+int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) return -1;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * 2) % 16) return -2;
+  cuuint64_t dims[2] = {inner, outer};
+  cuuint64_t strides[1] = {ld * 2};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 // Tensor map the epilogue stores D through: boxes of 32 rows x 128 bytes.
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32) {
   return out_f32 ? make_tmap_2d_f32(out, D, N, M, ldd, 32, 32) : make_tmap_2d_bf16(out, D, N, M, ldd, 64, 32);
@@ -379,15 +407,18 @@ static unsigned tune_wait_hint() {
 }
 
 namespace g2 {
+int launch_act(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
+               int* status, cudaStream_t stream);
 int launch_gather(const void* A, long long lda, void* D, long long ldd, const void* bias, int M, int N, int K,
                   const void* w, int* status, const GatherParams& g, cudaStream_t stream);
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true,
+          int ACT = ACT_NONE>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmParams p, cudaStream_t stream,
-                  const GatherParams* gp = nullptr, long long part_bytes = 0, const GroupParams* grp = nullptr) {
+                  const GatherParams* gp = nullptr, long long part_bytes = 0, const GroupParams* grp = nullptr, const ActMaps<ACT>& maps = ActMaps<ACT>{}) {
   static bool configured = false;
-  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS, EXTRA>;
+  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS, EXTRA, ACT>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess) return -4;
     configured = true;
@@ -406,9 +437,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   static const GatherParams none{};
   // A gathering launch neither overlaps its predecessor nor lets a successor in: its CTAs are counted on to be resident. A long or grouped
   // launch (PDL_MAX_FLOPS) starts behind its predecessor too.
-  if constexpr (GATHER) kern<<<grid, GEMM_THREADS + GATHER_EXTRA_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, p, *gp, GroupParams{});
-  else if (GROUP || 2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, p, none, grp ? *grp : GroupParams{});
-  else launch_pdl(kern, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, td, p, none, GroupParams{});
+  if constexpr (GATHER) kern<<<grid, GEMM_THREADS + GATHER_EXTRA_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, maps, p, *gp, GroupParams{});
+  else if (GROUP || 2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<grid, gemm_threads(ACT), GEMM_SMEM, stream>>>(ta, tb, td, maps, p, none, grp ? *grp : GroupParams{});
+  else launch_pdl(kern, grid, gemm_threads(ACT), GEMM_SMEM, stream, ta, tb, td, maps, p, none, GroupParams{});
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -464,6 +495,38 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
     default: GEMM(true, true, true);
   }
 #undef GEMM
+}
+
+// A product with an MLP's activation in its epilogue (gemm_act.cuh), on one CTA or, two_cta, on CTA pairs.
+//   mode 1  out[M, 2F] = A[M, K] * W[2F, K]^T, act[M, F] = f(out[:, :F]) * out[:, F:]
+//   mode 2  out[M, F] = A[M, K] * W[F, K]^T (+ bias), act[M, F] = f(out)
+// All row-major, without padding between rows but in A. f: SiLU, or (gelu) the tanh-approximated GELU.
+int mtb200_gemm_act(const void* A, long long lda, const void* W, void* out, void* act, const void* bias, int mode, int gelu, int M, int F, int K,
+                    int two_cta, int* status, cudaStream_t stream) {
+  using namespace mtb;
+  if (M <= 0 || F <= 0 || K <= 0) return 0;
+  if ((mode != ACT_GLU && mode != ACT_PLAIN) || F % 8 || K % 8 || (bias != nullptr && mode != ACT_PLAIN)) return -10;
+  if (reinterpret_cast<uintptr_t>(bias) & 15) return -11;
+  const int N = mode == ACT_GLU ? 2 * F : F;
+  CUtensorMap ta, tb;
+  ActMaps<ACT_GLU> m;
+  int rc = make_tmap_2d_bf16(&ta, A, K, M, lda, 64, 128);
+  if (rc) return rc;
+  rc = make_tmap_2d_bf16(&tb, W, K, N, K, 64, mode == ACT_GLU || two_cta ? 128 : 256);
+  if (rc) return rc - 10;
+  __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
+  rc = make_tmap_act(&m.gate, o, F, M, N);
+  if (!rc) rc = make_tmap_act(&m.up, mode == ACT_GLU ? o + F : o, F, M, N);
+  if (!rc) rc = make_tmap_act(&m.act, act, F, M, F);
+  if (rc) return rc - 20;
+  const EpiParams e{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0};
+  const ActParams a{F, gelu};
+  if (two_cta) return g2::launch_act(mode, ta, tb, m, e, a, K, status, stream);
+  const GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u, e, a};
+  if (mode == ACT_GLU)
+    return launch<false, false, false, false, false, GROUP_NONE, false, false, ACT_GLU>(ta, tb, m.gate, p, stream, nullptr, 0, nullptr, m);
+  return launch<false, false, false, false, false, GROUP_NONE, false, false, ACT_PLAIN>(ta, tb, m.gate, p, stream, nullptr, 0, nullptr,
+                                                                                     ActMaps<ACT_PLAIN>{m.gate, m.up, m.act});
 }
 
 // Grouped GEMM over expert slabs (see gemm_epilogue.cuh); starts [E + 1] and counts [E] are device arrays, `rows` is the

@@ -370,4 +370,25 @@ __device__ __forceinline__ float gelu_gate(float g) {
   return __fdividef(1.f, 1.f + __expf(-1.5957691216057308f * (g + 0.044715f * g * g * g)));
 }
 
+// Activation of an MLP and its derivative. ACT 0: SiLU, 1: tanh-approximated GELU.
+template <int ACT>
+__device__ __forceinline__ float glu_act(float g) {
+  if constexpr (ACT == 0) {
+    return __fdividef(g, 1.f + __expf(-g));
+  } else {
+    return g * gelu_gate(g);
+  }
+}
+// d act(g) / d g
+template <int ACT>
+__device__ __forceinline__ float glu_act_grad(float g) {
+  if constexpr (ACT == 0) {
+    const float sig = __fdividef(1.f, 1.f + __expf(-g));
+    return sig * (1.f + g * (1.f - sig));
+  } else {
+    const float s = gelu_gate(g);
+    return s + g * s * (1.f - s) * 1.5957691216057308f * (1.f + 0.134145f * g * g);
+  }
+}
+
 }  // namespace mtb

@@ -171,10 +171,13 @@ def block_forward(ops, cfg: ModelConfig, p: dict, x: torch.Tensor, batch: Packed
         elif keep:
             acts = BlockActs(x, n1, rstd1, qkv, attn, lse, h1, n2, rstd2, None, None, qk_pre, rstd_qk, st)
         return out, acts, ((attn, lse) if want_attn else None)
-    gu = ops.linear(n2, p["wgu"], p.get("bgu"), gather=None if plan is None else (plan, 1))
     # a recompute that stops before the down projection does not need the SwiGLU output: backward rebuilds it
-    # inside the SwiGLU-gradient kernel
-    act = (ops.swiglu(gu, cfg.mlp_act) if cfg.mlp_gated else ops.gelu(gu)) if need_out else None
+    # together with the SwiGLU gradient
+    if need_out and plan is None and hasattr(ops, "linear_act") and not (cfg.mlp_gated and "bgu" in p):
+        gu, act = ops.linear_act(n2, p["wgu"], cfg.mlp_act if cfg.mlp_gated else "gelu_tanh", cfg.mlp_gated, p.get("bgu"))
+    else:
+        gu = ops.linear(n2, p["wgu"], p.get("bgu"), gather=None if plan is None else (plan, 1))
+        act = (ops.swiglu(gu, cfg.mlp_act) if cfg.mlp_gated else ops.gelu(gu)) if need_out else None
     out = ops.linear(act, p["wd"], bd, h1, alpha=rm) if need_out else None
     acts = None
     if keep == "compact":   # kept from forward to backward: drop what one elementwise kernel can rebuild

@@ -1093,3 +1093,31 @@ def test_kernels_that_start_under_their_predecessors_tail_wait_for_its_results(o
     for a, b in zip(got, want):
         assert rel_err(a, b) <= tol
     ops.check_status()
+
+
+# widths at and around a tile's 128 gated or 256 plain columns and a box's 32; heights around a quarter, a CTA and a pair
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("fn", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("T,H,F", [(1, 64, 8), (31, 72, 40), (128, 64, 128), (129, 128, 136), (257, 200, 264), (300, 264, 1032), (5000, 512, 1544),
+                                   (2048, 1024, 4096)])
+def test_products_with_an_activation(ops, T, H, F, fn, gated):
+    torch.manual_seed(T + F)
+    f = {"silu": torch.nn.functional.silu, "gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh")}[fn]
+    W = 2 * F if gated else F
+    x, w = bf(T, H), bf(W, H, scale=2.0 / H ** 0.5)
+    bias = None if gated else bf(F)
+
+    def act_of(p):
+        return f(p[:, :F]) * p[:, F:] if gated else f(p)
+
+    for pair_max in (0.0, 1e12):   # on one CTA, and by size
+        ops.pair_max_flops, before = pair_max, ops.pair_max_flops
+        ops._gemm_plans.clear()
+        pre, act = ops.linear_act(x, w, fn, gated, bias)
+        ops.pair_max_flops = before
+        ops._gemm_plans.clear()
+        want = x.float() @ w.float().t() + (0 if bias is None else bias.float())
+        assert rel_err(pre, want) < 6e-3 and max_err(pre, want) < 5e-2
+        # of the pre-activations as they were stored: one rounding of an fp32 value
+        assert rel_err(act, act_of(pre.float())) < 4e-3 and max_err(act, act_of(pre.float()), rtol=1e-2) < 1e-2
+    ops.check_status()

@@ -951,17 +951,13 @@ __global__ void __launch_bounds__(EW_THREADS) sumsq_kernel(const float* __restri
   if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
-// Fused AdamW on a shard: g = grad * coef[0]; moments in fp32 or bf16; master fp32; bf16 working copy refreshed.
+// Fused AdamW on a shard: g = grad * coef; moments in fp32 or bf16; master fp32; bf16 working copy refreshed. Four elements from `i` on.
+struct AdamwParams {
+  float lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2;
+};
 template <typename StateT>
-__global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ master, StateT* __restrict__ m, StateT* __restrict__ v,
-                                                          const float* __restrict__ grad, __nv_bfloat16* __restrict__ param,
-                                                          long long n, float lr, float beta1, float beta2, float eps, float wd,
-                                                          float inv_bc1, float inv_sqrt_bc2, const float* __restrict__ coef) {
-  pdl_trigger();
-  pdl_wait();
-  const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
-  if (i >= n) return;
-  const float c = coef[0];
+__device__ __forceinline__ void adamw4(float* __restrict__ master, StateT* __restrict__ m, StateT* __restrict__ v, const float* __restrict__ grad,
+                                       __nv_bfloat16* __restrict__ param, long long i, float c, const AdamwParams& p) {
   const float4 g4 = *reinterpret_cast<const float4*>(grad + i);
   float4 w4 = *reinterpret_cast<float4*>(master + i);
   float g[4] = {g4.x * c, g4.y * c, g4.z * c, g4.w * c};
@@ -978,11 +974,11 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    w[k] *= (1.f - lr * wd);
-    mm[k] = beta1 * mm[k] + (1.f - beta1) * g[k];
-    vv[k] = beta2 * vv[k] + (1.f - beta2) * g[k] * g[k];
-    const float denom = sqrtf(vv[k]) * inv_sqrt_bc2 + eps;
-    w[k] -= lr * inv_bc1 * mm[k] / denom;
+    w[k] *= (1.f - p.lr * p.wd);
+    mm[k] = p.beta1 * mm[k] + (1.f - p.beta1) * g[k];
+    vv[k] = p.beta2 * vv[k] + (1.f - p.beta2) * g[k] * g[k];
+    const float denom = sqrtf(vv[k]) * p.inv_sqrt_bc2 + p.eps;
+    w[k] -= p.lr * p.inv_bc1 * mm[k] / denom;
   }
   *reinterpret_cast<float4*>(master + i) = make_float4(w[0], w[1], w[2], w[3]);
   if constexpr (sizeof(StateT) == 4) {
@@ -993,6 +989,75 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
     *reinterpret_cast<uint2*>(v + i) = make_uint2(pack_bf16(vv[0], vv[1]), pack_bf16(vv[2], vv[3]));
   }
   *reinterpret_cast<uint2*>(param + i) = make_uint2(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]));
+}
+
+template <typename StateT>
+__global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ master, StateT* __restrict__ m, StateT* __restrict__ v,
+                                                          const float* __restrict__ grad, __nv_bfloat16* __restrict__ param,
+                                                          long long n, AdamwParams p, const float* __restrict__ coef) {
+  pdl_trigger();
+  pdl_wait();
+  const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+  if (i < n) adamw4(master, m, v, grad, param, i, coef[0], p);
+}
+
+// The same over up to OPT_GROUPS groups in one launch, with the clip coefficient min(1, max_norm / (norm + 1e-6)) formed here from the sum
+// of squares; the first block also leaves the norm. A small model's step was five launches for the coefficient and two per group, each
+// taking the host 5 to 10 us: 640 tokens, 2 layers, 4 groups: OPT_TIMES.
+constexpr int OPT_GROUPS = 48;   // 56 bytes each: the parameters of a launch stay below 4 KB
+struct OptGroup {
+  float* master;
+  void *m, *v;
+  const float* grad;
+  __nv_bfloat16* param;
+  long long n;
+  int first_block;   // of this group in the launch
+};
+struct OptTable {
+  OptGroup g[OPT_GROUPS];
+  int groups;
+};
+__device__ __forceinline__ int opt_group(const OptTable& t) {   // of this block (uniform): the last group that starts at or before it
+  int lo = 0, hi = t.groups - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (t.g[mid].first_block <= static_cast<int>(blockIdx.x)) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+template <typename StateT>
+__global__ void __launch_bounds__(EW_THREADS) adamw_groups_kernel(const __grid_constant__ OptTable t, AdamwParams p, const float* __restrict__ sumsq,
+                                                                 float max_norm, float* __restrict__ norm_out) {
+  pdl_trigger();
+  pdl_wait();
+  const float norm = sqrtf(sumsq[0]);
+  float c = 1.f;
+  if (max_norm > 0.f) {
+    c = max_norm / (norm + 1e-6f);
+    c = c > 1.f ? 1.f : c;   // a norm that is not a number stays one
+  }
+  if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) norm_out[0] = norm;
+  const OptGroup& g = t.g[opt_group(t)];
+  const long long i = (static_cast<long long>(blockIdx.x - g.first_block) * blockDim.x + threadIdx.x) * 4;
+  if (i < g.n) adamw4(g.master, static_cast<StateT*>(g.m), static_cast<StateT*>(g.v), g.grad, g.param, i, c, p);
+}
+
+// out[0] += sum of squares over all groups.
+__global__ void __launch_bounds__(EW_THREADS) sumsq_groups_kernel(const __grid_constant__ OptTable t, float* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float red[32];
+  const int k = opt_group(t);
+  const OptGroup& g = t.g[k];
+  const int blocks = (k + 1 < t.groups ? t.g[k + 1].first_block : static_cast<int>(gridDim.x)) - g.first_block;
+  float s = 0.f;
+  for (long long i = (static_cast<long long>(blockIdx.x - g.first_block) * blockDim.x + threadIdx.x) * 4; i < g.n;
+       i += static_cast<long long>(blocks) * blockDim.x * 4) {
+    const float4 v = *reinterpret_cast<const float4*>(g.grad + i);
+    s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+  }
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) atomicAdd(out, s);
 }
 
 static inline int cdiv(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
@@ -1356,11 +1421,63 @@ int mtb200_adamw(float* master, void* m, void* v, int state_is_f32, const float*
   if (n % 4) return -10;
   const float inv_bc1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
   const float inv_sqrt_bc2 = 1.f / sqrtf(1.f - powf(beta2, static_cast<float>(step)));
+  const AdamwParams p{lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2};
   const int blocks = cdiv(n / 4, EW_THREADS);
-  if (state_is_f32)
-    launch_pdl(adamw_kernel<float>, blocks, EW_THREADS, 0, st, master, (float*)m, (float*)v, grad, (bf16*)param, n, lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2, coef);
-  else
-    launch_pdl(adamw_kernel<bf16>, blocks, EW_THREADS, 0, st, master, (bf16*)m, (bf16*)v, grad, (bf16*)param, n, lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2, coef);
+  if (state_is_f32) launch_pdl(adamw_kernel<float>, blocks, EW_THREADS, 0, st, master, (float*)m, (float*)v, grad, (bf16*)param, n, p, coef);
+  else launch_pdl(adamw_kernel<bf16>, blocks, EW_THREADS, 0, st, master, (bf16*)m, (bf16*)v, grad, (bf16*)param, n, p, coef);
+  return launch_ok();
+}
+
+// table: [groups][6] = master, m, v, gradient (fp32), working copy, elements. One launch per OPT_GROUPS groups.
+static int fill_table(OptTable& t, const long long* table, int groups, int per_thread, int most_blocks, long long* blocks) {
+  long long at = 0;
+  t.groups = 0;
+  for (int k = 0; k < groups; ++k) {
+    const long long* r = table + k * 6;
+    if (r[5] <= 0) continue;
+    if (r[5] % 4) return -10;
+    OptGroup& g = t.g[t.groups++];
+    g.master = reinterpret_cast<float*>(r[0]); g.m = reinterpret_cast<void*>(r[1]); g.v = reinterpret_cast<void*>(r[2]);
+    g.grad = reinterpret_cast<const float*>(r[3]); g.param = reinterpret_cast<bf16*>(r[4]); g.n = r[5];
+    g.first_block = static_cast<int>(at);
+    const long long want = (r[5] / 4 + EW_THREADS - 1) / EW_THREADS;
+    at += most_blocks > 0 && want > most_blocks ? most_blocks : want;
+    if (at > 0x7fffffffLL) return -10;
+  }
+  *blocks = at;
+  return 0;
+}
+
+// out[0] += sum of squares of the groups' gradients.
+int mtb200_sumsq_groups(const long long* table, int groups, float* out, cudaStream_t st) {
+  for (int first = 0; first < groups; first += OPT_GROUPS) {
+    OptTable t;
+    long long blocks = 0;
+    const int k = groups - first < OPT_GROUPS ? groups - first : OPT_GROUPS;
+    const int rc = fill_table(t, table + first * 6, k, 4, num_sms() * 8, &blocks);
+    if (rc) return rc;
+    if (blocks > 0) launch_pdl(sumsq_groups_kernel, static_cast<unsigned>(blocks), EW_THREADS, 0, st, t, out);
+  }
+  return launch_ok();
+}
+
+// AdamW on all groups with the gradients scaled by min(1, max_norm / (sqrt(sumsq) + 1e-6)) (max_norm 0: by one); norm_out[0] = sqrt(sumsq).
+int mtb200_adamw_groups(const long long* table, int groups, int state_is_f32, const float* sumsq, float max_norm, float* norm_out, float lr, float beta1,
+                        float beta2, float eps, float wd, int step, cudaStream_t st) {
+  const float inv_bc1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
+  const float inv_sqrt_bc2 = 1.f / sqrtf(1.f - powf(beta2, static_cast<float>(step)));
+  const AdamwParams p{lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2};
+  for (int first = 0; first < groups; first += OPT_GROUPS) {
+    OptTable t;
+    long long blocks = 0;
+    const int k = groups - first < OPT_GROUPS ? groups - first : OPT_GROUPS;
+    const int rc = fill_table(t, table + first * 6, k, 4, 0, &blocks);
+    if (rc) return rc;
+    if (blocks == 0) continue;
+    float* out = first == 0 ? norm_out : nullptr;
+    if (state_is_f32) launch_pdl(adamw_groups_kernel<float>, static_cast<unsigned>(blocks), EW_THREADS, 0, st, t, p, sumsq, max_norm, out);
+    else launch_pdl(adamw_groups_kernel<bf16>, static_cast<unsigned>(blocks), EW_THREADS, 0, st, t, p, sumsq, max_norm, out);
+  }
   return launch_ok();
 }
 

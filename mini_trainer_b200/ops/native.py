@@ -78,6 +78,8 @@ class _Sig:
     mtb200_f32_to_bf16 = [P, P, L, I, P]
     mtb200_sumsq = [P, L, P, P]
     mtb200_adamw = [P, P, P, I, P, P, L, F, F, F, F, F, I, P, P]
+    mtb200_sumsq_groups = [P, I, P, P]
+    mtb200_adamw_groups = [P, I, I, P, F, P, F, F, F, F, F, I, P]
     mtb200_gemm_grouped = [P, L, P, L, P, L, I, I, I, I, I, P, P, I, L, P, P]
     mtb200_moe_plan = [P, I, I, I, P, P, P, P, P, P]
     mtb200_moe_gather = [P, P, P, I, I, I, I, F, P, P]
@@ -711,6 +713,25 @@ class NativeOps:
     def add_sumsq(self, g, out):
         """``out += sum(g ** 2)`` (``out``: one fp32 element on the device)."""
         self._call("mtb200_sumsq", g.data_ptr(), g.numel(), out.data_ptr(), self._st())
+
+    @staticmethod
+    def group_table(groups):
+        """Addresses and sizes of parameter groups ``(master, m, v, gradient, working copy)``, for one call of ``add_sumsq_groups`` or
+        ``adamw_groups``."""
+        rows = [x for g in groups for x in (*(t.data_ptr() for t in g), g[0].numel())]
+        return (c_longlong * len(rows))(*rows), len(groups)
+
+    def add_sumsq_groups(self, table, out):
+        """``add_sumsq`` of the gradients of all groups, in one launch."""
+        self._call("mtb200_sumsq_groups", *table, out.data_ptr(), self._st())
+
+    def adamw_groups(self, table, fp32_moments, sumsq, max_norm, lr, beta1, beta2, eps, weight_decay, step):
+        """``adamw_step`` of all groups in one launch, with the gradients scaled by ``min(1, max_norm / (norm + 1e-6))`` (``max_norm`` 0: as they
+        are). Returns the norm, ``sqrt(sumsq)``, 0-dim."""
+        norm = torch.empty((), dtype=torch.float32, device=self.device)
+        self._call("mtb200_adamw_groups", *table, int(fp32_moments), sumsq.data_ptr(), max_norm, norm.data_ptr(), lr, beta1, beta2, eps, weight_decay,
+                   step, self._st())
+        return norm
 
     def accumulate(self, acc, src, accumulate: bool):
         """acc(fp32) = (acc if accumulate else 0) + src (bf16 or fp32)."""

@@ -766,22 +766,31 @@ class ShardedEngine:
         o = self.optim
         live = [g for g in self.groups if g.has_grad]
         sq = self._sq
-        for g in live:
-            if not g.sq_done:
-                if hasattr(self.ops, "add_sumsq"):
-                    self.ops.add_sumsq(g.gacc, sq)
-                else:
-                    sq += self.ops.sumsq(g.gacc)
-        self.comm.all_reduce_sum(sq)
-        norm = sq.sqrt().squeeze(0)
-        if o.max_grad_norm and o.max_grad_norm > 0:
-            coef = torch.clamp(o.max_grad_norm / (norm + 1e-6), max=1.0)
+        clip = o.max_grad_norm if o.max_grad_norm and o.max_grad_norm > 0 else 0.0
+        if hasattr(self.ops, "adamw_groups") and live:   # all groups in one launch each; the coefficient is formed in the update
+            table = lambda groups: self.ops.group_table([(g.master, g.m, g.v, g.gacc, g.shard) for g in groups])   # noqa: E731
+            new = [g for g in live if not g.sq_done]
+            if new:
+                self.ops.add_sumsq_groups(table(new), sq)
+            self.comm.all_reduce_sum(sq)
+            self.step_count += 1
+            norm = self.ops.adamw_groups(table(live), self.state_dtype == torch.float32, sq, clip, lr, o.beta1, o.beta2, o.eps, o.weight_decay,
+                                         self.step_count)
         else:
-            coef = torch.ones((), dtype=torch.float32, device=self.device)
-        self.step_count += 1
+            for g in live:
+                if not g.sq_done:
+                    if hasattr(self.ops, "add_sumsq"):
+                        self.ops.add_sumsq(g.gacc, sq)
+                    else:
+                        sq += self.ops.sumsq(g.gacc)
+            self.comm.all_reduce_sum(sq)
+            norm = sq.sqrt().squeeze(0)
+            coef = torch.clamp(clip / (norm + 1e-6), max=1.0) if clip else torch.ones((), dtype=torch.float32, device=self.device)
+            self.step_count += 1
+            for g in live:
+                self.ops.adamw_step(g.master, g.m, g.v, g.gacc, g.shard, lr, o.beta1, o.beta2, o.eps, o.weight_decay,
+                                    self.step_count, coef)
         for g in live:
-            self.ops.adamw_step(g.master, g.m, g.v, g.gacc, g.shard, lr, o.beta1, o.beta2, o.eps, o.weight_decay,
-                                self.step_count, coef)
             g.has_grad = False
             g.sq_done = False
         self._sq = torch.zeros(1, dtype=torch.float32, device=self.device)

@@ -1121,3 +1121,33 @@ def test_products_with_an_activation(ops, T, H, F, fn, gated):
         # of the pre-activations as they were stored: one rounding of an fp32 value
         assert rel_err(act, act_of(pre.float())) < 4e-3 and max_err(act, act_of(pre.float()), rtol=1e-2) < 1e-2
     ops.check_status()
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+@pytest.mark.parametrize("sizes,max_norm", [([128], 1.0), ([1 << 16, 4, 1028, 999936], 0.05), ([256 * k + 4 for k in range(1, 101)], 1e9), ([640] * 48, 0.0)])
+def test_optimizer_over_groups_is_the_optimizer_of_each(ops, sizes, max_norm, fp32):
+    """One group, sizes below and above a block, more groups than one launch holds, exactly as many; clipped, not clipped and without a limit."""
+    torch.manual_seed(len(sizes))
+    sd = torch.float32 if fp32 else torch.bfloat16
+    f = lambda n: torch.randn(n, device="cuda")   # noqa: E731
+    groups = [(f(n), f(n).to(sd), f(n).square().to(sd), f(n), torch.zeros(n, dtype=torch.bfloat16, device="cuda")) for n in sizes]
+    alone = [tuple(t.clone() for t in g) for g in groups]
+    table = ops.group_table(groups)
+    sq = torch.zeros(1, device="cuda")
+    ops.add_sumsq_groups(table, sq)
+    want = sum(g[3].double().square().sum() for g in groups)
+    assert abs(sq.item() - want.item()) < 1e-5 * want.item()
+    norm = ops.adamw_groups(table, fp32, sq, max_norm, 1e-3, 0.9, 0.95, 1e-8, 0.01, 3)
+    assert torch.equal(norm, sq.sqrt().squeeze(0))
+    # (a number over a tensor is a product with the reciprocal in torch, up to one rounding off the quotient)
+    coef = torch.div(torch.full((), max_norm, device="cuda"), norm + 1e-6).clamp(max=1.0) if max_norm else torch.ones((), device="cuda")
+    for a, b in zip(alone, groups):
+        ops.adamw_step(*a, 1e-3, 0.9, 0.95, 1e-8, 0.01, 3, coef)
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def test_optimizer_over_groups_with_a_norm_that_is_not_a_number(ops):
+    n = 512
+    g = tuple(torch.ones(n, device="cuda") for _ in range(4)) + (torch.zeros(n, dtype=torch.bfloat16, device="cuda"),)
+    norm = ops.adamw_groups(ops.group_table([g]), True, torch.full((1,), float("nan"), device="cuda"), 1.0, 1e-3, 0.9, 0.95, 1e-8, 0.0, 1)
+    assert norm.isnan() and g[0].isnan().all()   # as the clip coefficient of that norm makes it

@@ -766,6 +766,71 @@ __global__ void __launch_bounds__(128) embedding_bwd_kernel(__nv_bfloat16* __res
   }
 }
 
+// The same without the sort, for up to EMB_SCAN tokens: the block of a token looks through all the others. One that finds its id earlier ends,
+// the first of an id lists the later ones in token order (each thread a stretch of them) and sums as above, bit for bit. The comparisons
+// grow with the square of the tokens; sorting is five launches, which take the host longer still
+// (640 tokens x 512 46 -> 6.5 us, 4096 x 256 50 -> 17, 6000 x 1536 107 -> 33, 8192 x 1024 110 -> 55).
+constexpr int EMB_SCAN = 8192;
+__global__ void __launch_bounds__(EW_THREADS) embedding_bwd_scan_kernel(__nv_bfloat16* __restrict__ dw, const long long* __restrict__ ids,
+                                                                       const __nv_bfloat16* __restrict__ dx, int T, int H, int V, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ unsigned short later[EMB_SCAN];
+  __shared__ int wsum[EW_THREADS / 32];
+  const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long id = ids[t];
+  bool seen = false;
+#pragma unroll 8
+  for (int j = threadIdx.x; j < t; j += EW_THREADS) seen |= ids[j] == id;
+  if (__syncthreads_or(seen)) return;
+  if (id < 0 || id >= V) {   // skipped and reported, never dereferenced
+    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 60);
+    return;
+  }
+  const int per = (T - t - 1 + EW_THREADS - 1) / EW_THREADS;
+  const int j0 = t + 1 + threadIdx.x * per, j1 = min(T, j0 + per);
+  int mine = 0;
+#pragma unroll 4
+  for (int j = j0; j < j1; ++j) mine += ids[j] == id;
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += y; }
+  if (lane == 31) wsum[warp] = incl;
+  __syncthreads();
+  int at = incl - mine, n = 0;
+#pragma unroll
+  for (int k = 0; k < EW_THREADS / 32; ++k) { if (k < warp) at += wsum[k]; n += wsum[k]; }
+  if (mine > 0)
+    for (int j = j0; j < j1; ++j) if (ids[j] == id) later[at++] = static_cast<unsigned short>(j);
+  __syncthreads();
+  __nv_bfloat16* dst = dw + id * H;
+  for (int c = threadIdx.x * 8; c < H; c += EW_THREADS * 8) {
+    float acc[8], f[8];
+    bf16x8 v; v.load(dst + c); v.to_float(acc);
+    for (int k = -1; k < n; ++k) {
+      v.load(dx + static_cast<long long>(k < 0 ? t : later[k]) * H + c); v.to_float(f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += f[i];
+    }
+    v.from_float(acc); v.store(dst + c);
+  }
+}
+
+// out[rows[r]] = src[r] for rows of H columns, and the same for a vector of fp32 (either may be absent).
+__global__ void __launch_bounds__(128) scatter_rows_kernel(const long long* __restrict__ rows, const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ out,
+                                                          const float* __restrict__ vsrc, float* __restrict__ vout, int H, int T, int* status) {
+  pdl_trigger();
+  pdl_wait();
+  const long long r = blockIdx.x, t = rows[r];
+  if (t < 0 || t >= T) {   // skipped and reported, never dereferenced
+    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 60);
+    return;
+  }
+  if (threadIdx.x == 0) vout[t] = vsrc[r];
+  for (int c = threadIdx.x * 8; c < H; c += 128 * 8)
+    *reinterpret_cast<uint4*>(out + t * H + c) = *reinterpret_cast<const uint4*>(src + r * H + c);
+}
+
 // ------------------------------------------------------------------------------ cross-entropy
 // One block per row of a logits chunk ([R, V] fp32 or bf16, leading dimension ld). Pass 1: online
 // max / sum-exp; or, when the GEMM that made the logits left the statistics of every 256 columns (`stats`,
@@ -1359,6 +1424,23 @@ int mtb200_embedding_bwd(void* dw, const long long* sorted_ids, const long long*
   if (T <= 0) return 0;
   if (H % 8) return -10;
   launch_pdl(embedding_bwd_kernel, T, 128, 0, st, (bf16*)dw, sorted_ids, order, (const bf16*)dx, T, H, V, status);
+  return launch_ok();
+}
+
+// The same from the ids as they come, for at most EMB_SCAN tokens.
+int mtb200_embedding_bwd_scan(void* dw, const long long* ids, const void* dx, int T, int H, int V, int* status, cudaStream_t st) {
+  if (T <= 0) return 0;
+  if (H % 8 || T > EMB_SCAN) return -10;
+  launch_pdl(embedding_bwd_scan_kernel, T, EW_THREADS, 0, st, (bf16*)dw, ids, (const bf16*)dx, T, H, V, status);
+  return launch_ok();
+}
+
+// out [T, H] and vout [T] are zero but in `rows` [R], where they are src [R, H] and vsrc [R].
+int mtb200_scatter_rows(const long long* rows, const void* src, void* out, const float* vsrc, float* vout, int R, int H, int T, int* status, cudaStream_t st) {
+  if (T <= 0 || R < 0) return 0;
+  if (H % 8) return -10;
+  if (cudaMemsetAsync(out, 0, static_cast<size_t>(T) * H * 2, st) != cudaSuccess || cudaMemsetAsync(vout, 0, static_cast<size_t>(T) * 4, st) != cudaSuccess) return -5;
+  if (R > 0) launch_pdl(scatter_rows_kernel, R, 128, 0, st, rows, (const bf16*)src, (bf16*)out, vsrc, vout, H, T, status);
   return launch_ok();
 }
 

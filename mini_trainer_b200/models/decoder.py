@@ -285,15 +285,19 @@ def head_forward_backward(ops, cfg: ModelConfig, head_p: dict, head_g: dict, lm_
     # gradient, so the final norm, the three vocabulary-sized GEMMs and the CE kernel only see the
     # rows that count; their input gradient is scattered back into a zero tensor. Exact, not an
     # approximation; the reference's fused linear-CE computes logits for every row.
-    loss = torch.zeros(x.shape[0], dtype=torch.float32, device=x.device)
-    dx = torch.zeros_like(x)
     if rows.numel() == 0:   # nothing to learn from in this minibatch (e.g. only the idle-rank dummy sample);
-        return loss, dx     # the gradient buffers of the head were zeroed by the caller
+        # the gradient buffers of the head were zeroed by the caller
+        return torch.zeros(x.shape[0], dtype=torch.float32, device=x.device), torch.zeros_like(x)
     xs = ops.embedding(x, rows)   # row gather
     n, rstd = _norm(ops, cfg, xs, head_p, "norm", "bnorm")
     loss_s, dn = ops.linear_ce(n, lm_w, batch.loss_targets, grad_scale, lm_g, accumulate_dw=accumulate_lm_grad,
                                logit_scale=ls)
     dxs = _norm_bwd(ops, cfg, dn, xs, rstd, head_p, head_g, "norm", "bnorm")
+    if hasattr(ops, "scatter_rows"):
+        dx, loss = ops.scatter_rows(rows, dxs, loss_s, x.shape[0])
+        return loss, dx
+    loss = torch.zeros(x.shape[0], dtype=torch.float32, device=x.device)
+    dx = torch.zeros_like(x)
     loss.index_copy_(0, rows, loss_s)
     dx.index_copy_(0, rows, dxs)
     return loss, dx

@@ -72,6 +72,8 @@ class _Sig:
     mtb200_gelu_bwd_act = [P, P, P, L, P]
     mtb200_embedding_fwd = [P, P, P, I, I, I, P, P]
     mtb200_embedding_bwd = [P, P, P, P, I, I, I, P, P]
+    mtb200_embedding_bwd_scan = [P, P, P, I, I, I, P, P]
+    mtb200_scatter_rows = [P, P, P, P, P, I, I, I, P, P]
     mtb200_ce_fwd_bwd = [P, L, I, P, P, P, P, L, I, I, F, L, P]
     mtb200_colsum = [P, L, P, P, I, I, P]
     mtb200_accumulate = [P, P, L, I, I, P]
@@ -96,6 +98,7 @@ _GEMM_TAGS = (("gemm_nt", "gemm_nn"), ("gemm_tt", "gemm_tn"))   # [A stored [K, 
 _SPLIT_COUNTERS = 4096          # csrc/gemm_epilogue.cuh
 _SPLIT_FLOATS = 32 << 20        # most that the partials of a launch take: 128 MB
 _SPLIT_UNITS = 4 * _SPLIT_FLOATS // gemm_plan.UNIT_BYTES   # = 1024 of 128 x 256
+_EMB_SCAN = 8192                # tokens up to which the embedding gradient goes without a sort (at most EMB_SCAN of csrc/elementwise.cu)
 NATIVE_HEAD_DIMS = (64, 128)   # head dimensions of the hand-written attention kernels
 
 
@@ -293,10 +296,24 @@ class NativeOps:
         return out
 
     def embedding_bwd(self, dweight, ids, dx):
-        """dweight[ids] += dx, deterministic: a stable sort groups equal ids; one block sums each group in fp32."""
+        """dweight[ids] += dx, deterministic: one block sums the rows of an id in fp32, in token order. Few tokens are searched for equal ids
+        as they are, more are grouped by a stable sort."""
+        if ids.shape[0] <= _EMB_SCAN:
+            self._call("mtb200_embedding_bwd_scan", dweight.data_ptr(), ids.data_ptr(), dx.data_ptr(), ids.shape[0], dweight.shape[1],
+                       dweight.shape[0], self.status.data_ptr(), self._st())
+            return
         sorted_ids, order = torch.sort(ids, stable=True)
         self._call("mtb200_embedding_bwd", dweight.data_ptr(), sorted_ids.data_ptr(), order.data_ptr(), dx.data_ptr(),
                    ids.shape[0], dweight.shape[1], dweight.shape[0], self.status.data_ptr(), self._st())
+
+    def scatter_rows(self, rows, src, vec, T):
+        """``(out [T, H], v [T])``: zero but in ``rows``, where they are ``src`` and ``vec`` (fp32)."""
+        R, H = src.shape
+        out = torch.empty(T, H, dtype=src.dtype, device=self.device)
+        v = torch.empty(T, dtype=torch.float32, device=self.device)
+        self._call("mtb200_scatter_rows", rows.data_ptr(), src.data_ptr(), out.data_ptr(), vec.data_ptr(), v.data_ptr(), R, H, T,
+                   self.status.data_ptr(), self._st())
+        return out, v
 
     # -- rmsnorm ----------------------------------------------------------------------
     def rmsnorm(self, x, w, eps):

@@ -1151,3 +1151,39 @@ def test_optimizer_over_groups_with_a_norm_that_is_not_a_number(ops):
     g = tuple(torch.ones(n, device="cuda") for _ in range(4)) + (torch.zeros(n, dtype=torch.bfloat16, device="cuda"),)
     norm = ops.adamw_groups(ops.group_table([g]), True, torch.full((1,), float("nan"), device="cuda"), 1.0, 1e-3, 0.9, 0.95, 1e-8, 0.0, 1)
     assert norm.isnan() and g[0].isnan().all()   # as the clip coefficient of that norm makes it
+
+
+@pytest.mark.parametrize("T,V,H", [(1, 8, 8), (255, 3, 64), (257, 40, 136), (300, 1, 2056), (4096, 32000, 256), (2049, 500, 4096), (8192, 900, 128), (8193, 64, 128)])
+def test_embedding_gradient_without_a_sort_is_that_with_one(ops, T, V, H, monkeypatch):
+    """Few ids and many, one for all tokens, rows wider than a block, the most tokens that are searched and one more: bit for bit."""
+    from mini_trainer_b200.ops import native
+    torch.manual_seed(T)
+    ids, dx = torch.randint(0, V, (T,), device="cuda"), bf(T, H)
+    got, want = bf(V, H), None
+    want = got.clone()
+    ops.embedding_bwd(got, ids, dx)
+    monkeypatch.setattr(native, "_EMB_SCAN", 0)
+    ops.embedding_bwd(want, ids, dx)
+    assert torch.equal(got, want)
+    ops.check_status()
+
+
+def test_embedding_gradient_reports_an_id_outside_the_table(ops):
+    ids = torch.tensor([2, 9, 2, -1], device="cuda")
+    dw, dx = torch.zeros(4, 64, dtype=torch.bfloat16, device="cuda"), bf(4, 64)
+    ops.embedding_bwd(dw, ids, dx)
+    assert rel_err(dw[2], dx[0].float() + dx[2].float()) < 1e-2 and dw[[0, 1, 3]].abs().sum() == 0
+    with pytest.raises(RuntimeError, match="token id"):
+        ops.check_status()
+
+
+@pytest.mark.parametrize("T,R,H", [(1, 1, 8), (130, 1, 1032), (777, 776, 512), (64, 0, 64)])
+def test_rows_scattered_into_zeros(ops, T, R, H):
+    torch.manual_seed(T)
+    rows = torch.randperm(T, device="cuda")[:R]
+    src, vec = bf(R, H), torch.randn(R, device="cuda")
+    out, v = ops.scatter_rows(rows, src, vec, T)
+    want, wv = torch.zeros(T, H, dtype=torch.bfloat16, device="cuda"), torch.zeros(T, device="cuda")
+    want[rows], wv[rows] = src, vec
+    assert torch.equal(out, want) and torch.equal(v, wv)
+    ops.check_status()

@@ -1068,7 +1068,8 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_kernel(float* __restrict__ m
 
 // The same over up to OPT_GROUPS groups in one launch, with the clip coefficient min(1, max_norm / (norm + 1e-6)) formed here from the sum
 // of squares; the first block also leaves the norm. A small model's step was five launches for the coefficient and two per group, each
-// taking the host 5 to 10 us: 640 tokens, 2 layers, 4 groups: OPT_TIMES.
+// taking the host 5 to 10 us: 13 launches became 2 for 4 groups. With the embedding gradient's change a step of 640 tokens through 2 layers
+// went from 1508 to 1377 us.
 constexpr int OPT_GROUPS = 48;   // 56 bytes each: the parameters of a launch stay below 4 KB
 struct OptGroup {
   float* master;

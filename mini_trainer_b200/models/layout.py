@@ -13,6 +13,7 @@ them back to the HF names (``q_proj``, ``k_proj``, ``v_proj``, ``gate_proj``, ``
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from typing import Iterator
 
@@ -49,12 +50,16 @@ class GroupLayout:
             self.specs[pname] = spec
             off += -(-spec.numel // ALIGN_ELEMS) * ALIGN_ELEMS
         self.numel = off
+        self._cuts = [(s.name, s.shape, tuple(math.prod(s.shape[i + 1:]) for i in range(len(s.shape))), s.offset) for s in self.specs.values()]
         q = world * ALIGN_ELEMS
         self.padded_numel = -(-off // q) * q
         self.shard_numel = self.padded_numel // world
 
     def views(self, flat: torch.Tensor) -> dict:
         """Named tensor views into a full (gathered) flat buffer."""
+        if flat.dim() == 1 and flat.is_contiguous() and flat.numel() >= self.numel:   # one call per view
+            at = flat.storage_offset()
+            return {n: flat.as_strided(shape, strides, at + offset) for n, shape, strides, offset in self._cuts}
         return {n: flat[s.offset: s.offset + s.numel].view(s.shape) for n, s in self.specs.items()}
 
 

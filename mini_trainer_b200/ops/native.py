@@ -18,7 +18,7 @@ import torch
 
 from .. import build as _build
 from ..utils import nvtx
-from . import attention_plan, gemm_plan
+from . import attention_plan, block_exec, gemm_plan
 
 _LIB = None
 _raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else \
@@ -40,6 +40,7 @@ def load_library():
             fn = getattr(lib, name)
             fn.restype = c_int
             fn.argtypes = getattr(_Sig, name)
+    lib.mtb200_block_workspace.restype = c_longlong
     _LIB = lib
     return lib
 
@@ -82,6 +83,9 @@ class _Sig:
     mtb200_adamw = [P, P, P, I, P, P, L, F, F, F, F, F, I, P, P]
     mtb200_sumsq_groups = [P, I, P, P]
     mtb200_adamw_groups = [P, I, I, P, F, P, F, F, F, F, F, I, P]
+    mtb200_block_workspace = [P, P, I]
+    mtb200_block_forward = [P, P, P, P, P]
+    mtb200_block_backward = [P, P, P, P, P, P]
     mtb200_gemm_grouped = [P, L, P, L, P, L, I, I, I, I, I, P, P, I, L, P, P]
     mtb200_moe_plan = [P, I, I, I, P, P, P, P, P, P]
     mtb200_moe_gather = [P, P, P, I, I, I, I, F, P, P]
@@ -148,6 +152,7 @@ class NativeOps:
         self._gemm_plans = {}   # sizes -> entry point and splits
         self._epoch = itertools.count(1)   # of the launches that may split
         self._attn_plan_cache = {}
+        self._block_specs = {}   # sizes of a block -> its products' plans
         self._pairs = None
         self.sms = torch.cuda.get_device_properties(self._index).multi_processor_count
 
@@ -498,7 +503,10 @@ class NativeOps:
                 work = s0 if most_work_last_block else n - s0
                 items.append((work, a, n, s0))
         items.sort(key=lambda it: -it[0])
-        return torch.tensor([it[1:] for it in items], dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
+        table = torch.tensor([it[1:] for it in items], dtype=torch.int32)
+        if table.numel() > 8192 or torch.cuda.is_current_stream_capturing():
+            table = table.pin_memory()   # (the driver stages small copies, which is faster than pinning memory for them)
+        return table.to(self.device, non_blocking=True)
 
     def attention(self, qkv, cu_seqlens, cu_host, max_seqlen, hq, hkv, d, scale=None):
         T = qkv.shape[0]
@@ -559,6 +567,13 @@ class NativeOps:
                                     max_seqlen, max_seqlen, 0.0, scale, True, -1, -1, 0.0, None, False)
         self._ev_end("flash_attn_bwd", ev)
         return dqkv
+
+    # -- a whole decoder block (block_exec.py) ---------------------------------------------
+    def block_forward(self, acts_type, cfg, p, x, batch, inv_freq, keep, saved_attn, want_attn, need_out):
+        return block_exec.forward(self, acts_type, cfg, p, x, batch, inv_freq, keep, saved_attn, want_attn, need_out)
+
+    def block_backward(self, cfg, p, g, acts, dout, batch, inv_freq):
+        return block_exec.backward(self, cfg, p, g, acts, dout, batch, inv_freq)
 
     # -- swiglu -----------------------------------------------------------------------
     def swiglu(self, gate_up, act="silu"):

@@ -405,8 +405,8 @@ class ShardedEngine:
 
     def _region_reducer(self, i: int, gbuf: torch.Tensor, gslot: int, last: bool):
         """Returns ``(notify, finish)`` for block ``i``: ``notify(name)`` reduces the region that ends
-        where the previous one started as soon as backward has written it; ``finish()`` reduces the
-        rest. Backends whose reduction is a collective over the whole buffer (NCCL, gloo) reduce once,
+        where the previous one started as soon as backward has written it (``None`` where nothing is reduced before the end);
+        ``finish()`` reduces the rest. Backends whose reduction is a collective over the whole buffer (NCCL, gloo) reduce once,
         in ``finish``."""
         osft = getattr(self, "osft", None)
         if osft is not None and osft.owner_reduce:
@@ -431,7 +431,7 @@ class ShardedEngine:
                 else:
                     self._reduce(grp, gbuf, gslot, last)
 
-        return notify, finish
+        return notify if per_region else None, finish
 
     def _grad_buffer(self, i: int):
         slot = i % len(self._gbufs)

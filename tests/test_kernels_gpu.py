@@ -1187,3 +1187,71 @@ def test_rows_scattered_into_zeros(ops, T, R, H):
     want[rows], wv[rows] = src, vec
     assert torch.equal(out, want) and torch.equal(v, wv)
     ops.check_status()
+
+
+FAMILIES = {"llama": {}, "qwen2": dict(attention_bias=True), "qwen3": dict(qk_norm=True),
+            "starcoder2": dict(norm_type="layernorm", mlp_gated=False, attention_bias=True, mlp_bias=True, hidden_act="gelu_pytorch_tanh"),
+            "gemma-like": dict(model_type="llama", hidden_act="gelu_pytorch_tanh"), "granite": dict(residual_multiplier=0.22, attention_multiplier=0.02)}
+
+
+@pytest.mark.parametrize("family", list(FAMILIES))
+@pytest.mark.parametrize("T,keep", [(40, "compact"), (700, "compact"), (700, True), (1500, False)])
+def test_block_in_one_call_is_the_block_launch_by_launch(ops, family, T, keep, monkeypatch):
+    """Every form that the native call takes, with kept, partly kept and recomputed activations, against the Python form on the same kernels."""
+    from mini_trainer_b200.data.sampler import mb_collate_fn
+    from mini_trainer_b200.models import decoder as D, layout as L
+    from mini_trainer_b200.models.config import ModelConfig
+    kw = dict(model_type=family, vocab_size=64, hidden_size=256, intermediate_size=392, num_hidden_layers=1, num_attention_heads=6, num_key_value_heads=2,
+              head_dim=128 if family == "qwen3" else 64)
+    cfg = ModelConfig(**{**kw, **FAMILIES[family]})
+    torch.manual_seed(T)
+    lay = L.GroupLayout("block0", L.block_entries(cfg), 1)
+    p = lay.views((torch.randn(lay.padded_numel, device="cuda") * 0.05).bfloat16())
+    ids = [torch.randint(0, 64, (n,)) for n in (T // 3, T - T // 3)]
+    batch = D.make_packed_batch(mb_collate_fn([{"input_ids": i, "labels": i.clone(), "len": len(i), "num_loss_counted_tokens": len(i)} for i in ids], T), "cuda")
+    inv, x, dout = cfg.rope_inv_freq().cuda(), bf(T, 256), bf(T, 256, scale=0.1)
+    cls = type(ops)
+
+    def one(native_call):
+        done = []
+        for name in ("block_forward", "block_backward"):
+            real = getattr(cls, name)
+            monkeypatch.setattr(cls, name, (lambda self, *a, real=real: done.append(real(self, *a)) or done[-1]) if native_call else lambda self, *a: None)
+        g = lay.views(torch.full((lay.padded_numel,), float("nan"), dtype=torch.bfloat16, device="cuda"))
+        out, acts, attn = D.block_forward(ops, cfg, p, x, batch, inv, keep=keep, want_attn=not keep)
+        if not keep:
+            out2, acts, _ = D.block_forward(ops, cfg, p, x, batch, inv, keep=True, saved_attn=attn, need_out=False)
+            assert out2 is None
+        dx = D.block_backward(ops, cfg, p, g, acts, dout, batch, inv)
+        monkeypatch.undo()
+        assert not native_call or (len(done) == (2 if keep else 3) and all(d is not None for d in done))
+        return out, dx, g
+
+    n0 = ops.launches
+    out, dx, g = one(True)
+    n1 = ops.launches
+    out_ref, dx_ref, g_ref = one(False)
+    assert n1 - n0 == ops.launches - n1
+    assert torch.equal(out, out_ref)
+    # behind the attention backward, whose sum of dQ tiles has no fixed order, up to that
+    for a, b in [(dx, dx_ref)] + [(g[n], g_ref[n]) for n in g]:
+        assert rel_err(a, b) < 5e-3, family
+    assert all(torch.equal(g[n], g_ref[n]) for n in ("wd", "wgu", "wo"))
+    ops.check_status()
+
+
+def test_block_in_one_call_leaves_to_the_python_form_what_it_does_not_cover(ops):
+    from mini_trainer_b200.models import decoder as D, layout as L
+    from mini_trainer_b200.models.config import ModelConfig
+    batch = D.PackedBatch(*(torch.zeros(8, dtype=torch.int64, device="cuda"),) * 2, torch.arange(8, dtype=torch.int32, device="cuda"), None, [0, 8], 8)
+    x = bf(8, 64)
+    for change, strided in ((dict(post_norm=True), False), (dict(norm_weight_offset=1.0), False), (dict(mlp_bias=True), False),
+                            (dict(residual_multiplier=0.5, attention_bias=True, attention_out_bias=True), True), (dict(head_dim=32), False)):
+        known = {k: v for k, v in change.items() if k in ModelConfig.__dataclass_fields__}
+        cfg = ModelConfig(**{**dict(vocab_size=64, hidden_size=64, intermediate_size=64, num_hidden_layers=1, num_attention_heads=1, num_key_value_heads=1,
+                                    head_dim=64), **known})
+        p = L.GroupLayout("block0", L.block_entries(cfg), 1)
+        p = p.views(torch.zeros(p.padded_numel, dtype=torch.bfloat16, device="cuda"))
+        if strided:
+            p["wo"] = bf(64, 128)[:, :64]
+        assert ops.block_forward(D.BlockActs, cfg, p, x, batch, None, False, None, False, True) is None

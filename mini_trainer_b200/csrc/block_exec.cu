@@ -183,7 +183,6 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
   // attention
   RUN(gemm(s, io, D_O, dh1, s.H, 0, p.wo, q, 1, dattn, s.T, q, s.H, nullptr, nullptr, s.alpha, st), 1);
   RUN(wgrad(W_O, dh1, s.H, io.attn, q, g.wo, g.bo), 0);
-  if (cudaMemsetAsync(dq, 0, T * q * 4, st) != cudaSuccess) return -5;
   const int splits = io.part != nullptr ? s.bwd_splits : 1;
   RUN(mtb200_attn_bwd(io.qkv, Q, io.attn, q, dattn, q, dqkv, Q, io.lse, delta, dq, io.bwd_plan, s.bwd_items, s.T, s.Hq, s.Hkv, s.D, splits,
                       splits > 1 ? io.counters : nullptr, splits > 1 ? io.epochs[GEMMS] : 0, splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, s.scale,

@@ -528,7 +528,7 @@ class NativeOps:
         dqkv = torch.empty_like(qkv)
         plan, splits, nbytes = self._cached(cu_host, ("bwd", hq, hkv, d)) or self._plan_attention_bwd(cu_host, hq, hkv, d)
         delta = torch.empty(hq, T, dtype=torch.float32, device=self.device)
-        dq_acc = torch.zeros(T, hq * d, dtype=torch.float32, device=self.device)
+        dq_acc = torch.empty(T, hq * d, dtype=torch.float32, device=self.device)
         st = self._st()
         split = self._split(st, nbytes) if splits > 1 else None
         ws, epoch, part = split or (None, 0, None)

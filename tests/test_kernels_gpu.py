@@ -1255,3 +1255,30 @@ def test_block_in_one_call_leaves_to_the_python_form_what_it_does_not_cover(ops)
         if strided:
             p["wo"] = bf(64, 128)[:, :64]
         assert ops.block_forward(D.BlockActs, cfg, p, x, batch, None, False, None, False, True) is None
+
+
+@pytest.mark.parametrize("D,hq,hkv", [(64, 1, 1), (64, 6, 2), (128, 3, 3), (128, 8, 2)])
+@pytest.mark.parametrize("lens", [[1], [17, 3], [129], [700, 45, 260]])
+def test_attention_backward_zeroes_its_accumulator(ops, lens, D, hq, hkv):
+    """Rows that fill no block of the pass that zeroes; the scratch comes from memory that held no numbers."""
+    torch.manual_seed(sum(lens))
+    T, cu = sum(lens), [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    qkv, dout = bf(T, (hq + 2 * hkv) * D), bf(T, hq * D)
+    args = (torch.tensor(cu, dtype=torch.int32, device="cuda"), cu, max(lens), hq, hkv, D)
+    out, lse = ops.attention(qkv, *args)
+    for n in (T * hq * D, T * hq):   # what the call takes its fp32 scratch from
+        poison = [torch.full((n,), float("nan"), device="cuda") for _ in range(4)]
+        del poison
+    got = ops.attention_bwd(dout, qkv, out, lse, *args)
+    q32 = qkv.float().requires_grad_()
+    q, k, v = q32.split([hq * D, hkv * D, hkv * D], -1)
+    ref = []
+    for a, b in zip(cu[:-1], cu[1:]):
+        heads = [t[a:b].view(b - a, -1, D).transpose(0, 1) for t in (q, k, v)]
+        heads[1:] = [t.repeat_interleave(hq // hkv, 0) for t in heads[1:]]
+        ref.append(torch.nn.functional.scaled_dot_product_attention(*heads, is_causal=True).transpose(0, 1).reshape(b - a, hq * D))
+    torch.cat(ref).backward(dout.float())
+    assert rel_err(got, q32.grad) < 1.5e-2
+    ops.check_status()

@@ -5,7 +5,7 @@
 // Eight warps, two per 32-row quarter: with four (one per scheduler) the arithmetic of a tile took longer than short reductions. They work on
 // 32 columns at a time, staged as boxes of 32 rows x 64 bytes (64B-swizzled). Bound by the product. With its activation, on a B200:
 // 5987 x 17920 x 1536 272 -> 231 us (product alone 220), 4099 x 12288 x 2048 167 -> 153, 16384 x 28672 x 4096 3.16 -> 2.8 ms, 7001 x 12288 x 3072 without
-// a gate 448 -> 375 us; whole blocks of those sizes 1836 -> 1793, 1712 -> 1703, 20.05 -> 19.91 ms and 4240 -> 4126 us.
+// a gate 448 -> 375 us; over the slabs of 64 experts (20 500 rows x 2048 x 2048) 150 + 24 -> 153, of 8 (9200 x 28672 x 4096) 1378 + 117 -> 1434; whole blocks of those sizes 1836 -> 1793, 1712 -> 1703, 20.05 -> 19.91 ms and 4240 -> 4126 us.
 //
 // The other direction, the activation's gradient in the epilogue of the product in front of it, was tried with the pre-activations loaded
 // by TMA two boxes ahead and either form of stores. It gained up to a fifth alone (5987 x 8960 x 1536 243 -> 190 us) and nothing in a

@@ -534,16 +534,17 @@ int mtb200_gemm_act(const void* A, long long lda, const void* W, void* out, void
 //   mode 0  D[rows, N] = A[rows, K] * W_e[N, K]^T        W: E matrices [N, K], w_stride elements apart
 //   mode 1  D[rows, N] = A[rows, K] * W_e[K, N]          W: E matrices [K, N], w_stride elements apart
 //   mode 2  W_e[M, N] = A[rows_e, M]^T * B[rows_e, N]    D is W here: E outputs, w_stride elements apart, ldd = N; K is ignored
-int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long ldb, void* D, long long ldd, int mode, int rows,
+//   mode 3  as mode 0, and act[rows, N / 2] = f(gate) * up of D = [gate | up] (gemm_act.cuh); f: SiLU, or (gelu) the tanh-approximated GELU
+int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long ldb, void* D, long long ldd, void* act, int gelu, int mode, int rows,
                         int M, int N, int K, const int* starts, const int* counts, int E, long long w_stride, int* status,
                         cudaStream_t stream) {
   using namespace mtb;
   if (E <= 0 || rows <= 0 || N <= 0 || (mode == 2 ? M : K) <= 0) return 0;
-  if (E > GROUP_MAX || N % 8 || ldd % 8 || rows % GROUP_ALIGN || w_stride % 8 || mode < 0 || mode > 2) return -10;
+  if (E > GROUP_MAX || N % 8 || ldd % 8 || rows % GROUP_ALIGN || w_stride % 8 || mode < 0 || mode > 3 || (mode == 3 && (act == nullptr || N % 16))) return -10;
   CUtensorMap ta, tb, td;
   int rc = mode == 2 ? make_tmap_2d_bf16(&ta, A, M, rows, lda, 64, 64) : make_tmap_2d_bf16(&ta, A, K, rows, lda, BK, BM);
   if (rc) return rc;
-  if (mode == 0) rc = make_tmap_3d_bf16(&tb, B, K, N, E, w_stride, BK, BN);
+  if (mode == 0 || mode == 3) rc = make_tmap_3d_bf16(&tb, B, K, N, E, w_stride, BK, mode == 3 ? BN / 2 : BN);
   else if (mode == 1) rc = make_tmap_3d_bf16(&tb, B, N, K, E, w_stride, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, N, rows, ldb, 64, 64);
   if (rc) return rc - 10;
@@ -552,8 +553,16 @@ int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long l
   else rc = make_tmap_out(&td, D, rows, N, ldd, 0);
   if (rc) return rc - 20;
   GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0}};
+               EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0}, ActParams{N / 2, gelu}};
   GroupParams g{starts, counts, E};
+  if (mode == 3) {
+    ActMaps<ACT_GLU> m;
+    rc = make_tmap_act(&m.gate, D, N / 2, rows, ldd);
+    if (!rc) rc = make_tmap_act(&m.up, reinterpret_cast<__nv_bfloat16*>(D) + N / 2, N / 2, rows, ldd);
+    if (!rc) rc = make_tmap_act(&m.act, act, N / 2, rows, N / 2);
+    if (rc) return rc - 20;
+    return launch<false, false, false, false, false, GROUP_ROWS, false, false, ACT_GLU>(ta, tb, td, p, stream, nullptr, 0, &g, m);
+  }
   if (mode == 0) return launch<false, false, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
   if (mode == 1) return launch<false, true, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
   return launch<true, true, false, false, false, GROUP_REDUCE>(ta, tb, td, p, stream, nullptr, 0, &g);

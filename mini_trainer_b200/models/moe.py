@@ -124,15 +124,21 @@ def moe_forward(ops, cfg, p: dict, n2: torch.Tensor, h1: torch.Tensor, need_out:
 def _grouped_forward(ops, cfg, p: dict, n2, h1, need_out: bool, keep_act: bool, probs, topi, w, wgu, wd):
     """``moe_forward`` on the grouped kernels. The activation is never kept: backward's gradient kernel rebuilds it in the
     pass over gate/up that it makes anyway."""
-    sl = ops.expert_slabs(topi, cfg.num_local_experts)
-    gu = ops.grouped_linear(ops.gather_rows(n2, sl), wgu, sl)
+    sl, fe = ops.expert_slabs(topi, cfg.num_local_experts), cfg.expert_intermediate_size
+    xs, act = ops.gather_rows(n2, sl), None
+    if need_out and fe % 8 == 0:   # the activation with the projection in front of it
+        gu, act = ops.grouped_linear_act(xs, wgu, sl, cfg.mlp_act)
+    else:
+        gu = ops.grouped_linear(xs, wgu, sl)
+    del xs
     st = MoeState(probs, topi, w.contiguous(), None, None, None, gu, None, slabs=sl)
     add = None
     if "wgus" in p:
         st.gu_s = ops.linear(n2, p["wgus"])
     if not need_out:
         return None, st
-    yr = ops.grouped_linear(ops.swiglu(gu, cfg.mlp_act), wd, sl)
+    yr = ops.grouped_linear(ops.swiglu(gu, cfg.mlp_act) if act is None else act, wd, sl)
+    del act
     if "wgus" in p:
         act_s = ops.swiglu(st.gu_s, cfg.mlp_act)
         add = torch.sigmoid((n2 @ p["wsg"].t()).float()) * ops.linear(act_s, p["wds"]).float()

@@ -86,7 +86,7 @@ class _Sig:
     mtb200_block_workspace = [P, P, I]
     mtb200_block_forward = [P, P, P, P, P]
     mtb200_block_backward = [P, P, P, P, P, P]
-    mtb200_gemm_grouped = [P, L, P, L, P, L, I, I, I, I, I, P, P, I, L, P, P]
+    mtb200_gemm_grouped = [P, L, P, L, P, L, P, I, I, I, I, I, I, P, P, I, L, P, P]
     mtb200_moe_plan = [P, I, I, I, P, P, P, P, P, P]
     mtb200_moe_gather = [P, P, P, I, I, I, I, F, P, P]
     mtb200_moe_glu_bwd = [P, P, P, P, P, I, I, I, I, P, P, P]
@@ -631,10 +631,10 @@ class NativeOps:
                    sl.cap, H, float(scale), out.data_ptr(), self._st())
         return out
 
-    def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride):
-        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, mode, sl.cap, M, N, K,
+    def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride, act=None, fn="silu"):
+        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), int(fn != "silu"), mode, sl.cap, M, N, K,
                    sl.starts.data_ptr(), sl.counts.data_ptr(), sl.counts.shape[0], stride, self.status.data_ptr(), self._st(),
-                   tag="gemm_grouped_" + ("nt", "nn", "tn")[mode])
+                   tag="gemm_grouped_" + ("nt", "nn", "tn", "nt_act")[mode])
         return out
 
     def grouped_linear(self, x, stack, sl: ExpertSlabs):
@@ -643,6 +643,14 @@ class NativeOps:
         N, K = w.shape
         out = torch.empty(sl.cap, N, dtype=x.dtype, device=self.device)
         return self._grouped(0, x, w, K, out, N, sl, sl.cap, N, K, stride)
+
+    def grouped_linear_act(self, x, stack, sl: ExpertSlabs, fn="silu"):
+        """``(pre, fn(gate) * up)`` of ``pre = [gate | up] = x_e @ W_e.T`` for every slab, in one launch."""
+        w, stride = stack
+        N, K = w.shape
+        pre = torch.empty(sl.cap, N, dtype=x.dtype, device=self.device)
+        act = torch.empty(sl.cap, N // 2, dtype=x.dtype, device=self.device)
+        return self._grouped(3, x, w, K, pre, N, sl, sl.cap, N, K, stride, act, fn), act
 
     def grouped_dgrad(self, dy, stack, sl: ExpertSlabs):
         """``dy_e @ W_e`` for every slab."""

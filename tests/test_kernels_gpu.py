@@ -1282,3 +1282,57 @@ def test_attention_backward_zeroes_its_accumulator(ops, lens, D, hq, hkv):
     torch.cat(ref).backward(dout.float())
     assert rel_err(got, q32.grad) < 1.5e-2
     ops.check_status()
+
+
+# rows of the experts: none, one, around half and all of a slab's 128 rows, two to five tiles
+EXPERT_ROWS = [0, 1, 63, 64, 65, 127, 128, 129, 0, 192, 255, 256, 257, 320, 500, 513, 0]
+
+
+def _slabs(ops, counts):
+    from mini_trainer_b200.ops.native import ExpertSlabs
+    E = len(counts)
+    starts = [0]
+    for c in counts:
+        starts.append(starts[-1] + -(-c // 128) * 128)
+    cap = -(-(sum(counts) + 127 * E) // 128) * 128
+    t = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+    return ExpertSlabs(t(starts), t(counts), None, None, cap, 1), starts
+
+
+def _rows(counts, starts, cap, width):
+    x = torch.full((cap, width), float("nan"), dtype=torch.bfloat16, device="cuda")   # past the slabs: must not matter
+    x[: starts[-1]] = 0
+    for c, s in zip(counts, starts):
+        x[s:s + c] = bf(c, width)
+    return x
+
+
+@pytest.mark.parametrize("H,F", [(72, 8), (64, 136), (200, 264), (520, 128)])
+def test_grouped_products(ops, H, F):
+    torch.manual_seed(H + F)
+    counts, E = EXPERT_ROWS, len(EXPERT_ROWS)
+    sl, starts = _slabs(ops, counts)
+    wgu, wd = bf(E, 2 * F, H, scale=0.1), bf(E, H, F, scale=0.1)
+    x, y, d = _rows(counts, starts, sl.cap, H), _rows(counts, starts, sl.cap, F), _rows(counts, starts, sl.cap, 2 * F)
+    gu = ops.grouped_linear(x, (wgu[0], 2 * F * H), sl)
+    for fn in ("silu", "gelu_tanh"):
+        pre, act = ops.grouped_linear_act(x, (wgu[0], 2 * F * H), sl, fn)
+        for c, s in zip(counts, starts):
+            assert torch.equal(pre[s:s + c], gu[s:s + c])
+            f = torch.nn.functional.silu(pre[s:s + c, :F].float()) if fn == "silu" else torch.nn.functional.gelu(pre[s:s + c, :F].float(), approximate="tanh")
+            if c:
+                assert rel_err(act[s:s + c], f * pre[s:s + c, F:].float()) < 4e-3
+            assert (act[s + c: s + -(-c // 128) * 128] == 0).all()   # the slab's padding: what a reduction over it reads behind its rows
+    dx = ops.grouped_dgrad(d, (wgu[0], 2 * F * H), sl)
+    for e, (c, s) in enumerate(zip(counts, starts)):
+        if c:
+            assert rel_err(gu[s:s + c], x[s:s + c].float() @ wgu[e].float().t()) < 6e-3
+            assert max_err(gu[s:s + c], x[s:s + c].float() @ wgu[e].float().t()) < 5e-2
+            assert rel_err(dx[s:s + c], d[s:s + c].float() @ wgu[e].float()) < 6e-3
+            assert max_err(dx[s:s + c], d[s:s + c].float() @ wgu[e].float()) < 5e-2
+    g = torch.full((E, H, F), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.grouped_wgrad(x, y, (g[0], H * F), sl)
+    for e, (c, s) in enumerate(zip(counts, starts)):
+        want = x[s:s + c].float().t() @ y[s:s + c].float()
+        assert (g[e] == 0).all() if c == 0 else rel_err(g[e], want) < 6e-3 and max_err(g[e], want) < 5e-2
+    ops.check_status()

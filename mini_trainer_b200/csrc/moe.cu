@@ -31,6 +31,59 @@ struct Vec8 {
   }
 };
 
+// Router of a layer, one warp per token: fp32 softmax of the logits, the k largest (the lower index of equal ones, the largest first) and their
+// weights, renormalised over the chosen ones when `renorm`. A lane holds experts lane, lane + 32, ... As tensor operations these were
+// six launches of 2 to 11 us and the gaps between them (2051 tokens, 64 experts, 8 chosen: 28 us and 10 of
+// gaps, now 6.6).
+__global__ void __launch_bounds__(MOE_THREADS) moe_route_kernel(const bf16* __restrict__ logits, int T, int E, int k, int renorm, float* __restrict__ probs,
+                                                               long long* __restrict__ topi, float* __restrict__ w) {
+  pdl_trigger();
+  pdl_wait();
+  const long long t = (static_cast<long long>(blockIdx.x) * MOE_THREADS + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t >= T) return;
+  constexpr int PER = GROUP_MAX / 32;
+  float x[PER];
+  float m = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane + i * 32;
+    x[i] = e < E ? __bfloat162float(logits[t * E + e]) : -INFINITY;
+    m = fmaxf(m, x[i]);
+  }
+  m = warp_max(m);
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) { x[i] = lane + i * 32 < E ? expf(x[i] - m) : 0.f; s += x[i]; }
+  s = warp_sum(s);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = lane + i * 32;
+    x[i] /= s;
+    if (e < E) probs[t * E + e] = x[i];
+    x[i] = e >= E ? -1.f : (x[i] != x[i] ? INFINITY : x[i]);   // what is not a number counts as the largest, as in a sort
+  }
+  float mine = 0.f, sum = 0.f;   // lane s holds the s-th weight
+  for (int c = 0; c < k; ++c) {
+    float best = -2.f;
+    int at = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) if (x[i] > best) { best = x[i]; at = lane + i * 32; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+      if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) if (at == lane + i * 32) x[i] = -1.f;   // taken
+    const float v = best == INFINITY ? NAN : best;
+    if (lane == c) { mine = v; topi[t * k + c] = at; }
+    sum += v;
+  }
+  if (lane < k) w[t * k + lane] = renorm ? mine / sum : mine;
+}
+
 // One block per expert. Every block counts all experts (the chosen indices are a few hundred KB at most and stay in L2), so
 // the slab starts need no second launch; it then walks the pairs once more and numbers its own, in pair order: the row order
 // inside a slab, and with it every sum over a slab, does not depend on scheduling.
@@ -131,21 +184,24 @@ __device__ __forceinline__ void act_and_grad(float g, float& a, float& da) {
 // Per routed row, with du the gradient of the activation before the expert weight w:
 //   dgu = d(act(g) * u) for the incoming gradient w * du,  du <- w * act(g) * u (the row the down projection's weight
 //   gradient needs),  dw[pair] = du . (act(g) * u)
-// One block per row; one pass over gate/up and du instead of the forward activation, two scalings, a dot product and the
-// activation gradient as passes of their own.
-template <int ACT>
+// One pass over gate/up and du instead of the forward activation, two scalings, a dot product and the activation gradient as passes of their
+// own. TPR threads per row: a warp for narrow rows, whose reduction then needs no barrier (20 500 rows of 1024: 60 us with a block per row,
+// 40 with a warp), up to the whole block for wide ones (14 336: 221 us either way, the copy bandwidth).
+template <int ACT, int TPR>
 __global__ void __launch_bounds__(MOE_THREADS) moe_glu_bwd_kernel(bf16* __restrict__ du, const bf16* __restrict__ gu, const float* __restrict__ w,
-                                                                 const int* __restrict__ pair_of, const int* __restrict__ starts, int E, int F,
+                                                                 const int* __restrict__ pair_of, const int* __restrict__ starts, int E, int cap, int F,
                                                                  bf16* __restrict__ dgu, float* __restrict__ dw) {
   pdl_trigger();
   pdl_wait();
   __shared__ float red[MOE_THREADS / 32];
-  const long long row = blockIdx.x;
-  if (row >= starts[E]) return;
-  const int pair = pair_of[row];
+  const int l = threadIdx.x % TPR;
+  const long long row = static_cast<long long>(blockIdx.x) * (MOE_THREADS / TPR) + threadIdx.x / TPR;
+  const bool here = row < cap && row < starts[E];
+  const int pair = here ? pair_of[row] : -1;
   const float wr = pair < 0 ? 0.f : w[pair];
   float dot = 0.f;
-  for (int c = threadIdx.x * 8; c < F; c += MOE_THREADS * 8) {
+#pragma unroll 2
+  for (int c = l * 8; here && c < F; c += TPR * 8) {
     Vec8 g, u, d;
     g.load(gu + row * 2 * F + c); u.load(gu + row * 2 * F + F + c); d.load(du + row * F + c);
     float fg[8], fu[8], fd[8], oa[8];
@@ -166,14 +222,14 @@ __global__ void __launch_bounds__(MOE_THREADS) moe_glu_bwd_kernel(bf16* __restri
     u.store(dgu + row * 2 * F + F + c);
   }
   dot = warp_sum(dot);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dot;
-  __syncthreads();
-  if (threadIdx.x == 0 && pair >= 0) {
-    float s = 0.f;
+  if constexpr (TPR > 32) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dot;
+    __syncthreads();
+    dot = 0.f;
 #pragma unroll
-    for (int i = 0; i < MOE_THREADS / 32; ++i) s += red[i];
-    dw[pair] = s;
+    for (int i = 0; i < TPR / 32; ++i) dot += red[threadIdx.x / TPR * (TPR / 32) + i];
   }
+  if (l == 0 && pair >= 0) dw[pair] = dot;
 }
 
 // out[t] = base[t] + scale * (sum over slots of w[t, slot] * rows[row_of[t, slot]] + add[t]), summed in fp32 in slot order.
@@ -254,6 +310,14 @@ int mtb200_moe_plan(const long long* topi, int n, int E, int cap, int* starts, i
   return ok();
 }
 
+// probs [T, E], w [T, k]: fp32; topi [T, k]: int64.
+int mtb200_moe_route(const void* logits, int T, int E, int k, int renorm, float* probs, long long* topi, float* w, cudaStream_t st) {
+  if (T <= 0) return 0;
+  if (E <= 0 || E > GROUP_MAX || k <= 0 || k > 32 || k > E) return -10;
+  launch_pdl(moe_route_kernel, (T + MOE_THREADS / 32 - 1) / (MOE_THREADS / 32), MOE_THREADS, 0, st, (const bf16*)logits, T, E, k, renorm, probs, topi, w);
+  return ok();
+}
+
 int mtb200_moe_gather(const void* src, const int* pair_of, const int* starts, int E, int k, int cap, int H, float scale, void* out,
                       cudaStream_t st) {
   if (cap <= 0) return 0;
@@ -267,8 +331,12 @@ int mtb200_moe_glu_bwd(void* du, const void* gu, const float* w, const int* pair
                        void* dgu, float* dw, cudaStream_t st) {
   if (cap <= 0) return 0;
   if (F % 8) return -10;
-  if (act == 0) launch_pdl(moe_glu_bwd_kernel<0>, cap, MOE_THREADS, 0, st, (bf16*)du, (const bf16*)gu, w, pair_of, starts, E, F, (bf16*)dgu, dw);
-  else launch_pdl(moe_glu_bwd_kernel<1>, cap, MOE_THREADS, 0, st, (bf16*)du, (const bf16*)gu, w, pair_of, starts, E, F, (bf16*)dgu, dw);
+  // a thread of a row gets two vectors at least, and a row 256 threads at most
+#define GB(ACT, TPR) launch_pdl(moe_glu_bwd_kernel<ACT, TPR>, (cap + MOE_THREADS / TPR - 1) / (MOE_THREADS / TPR), MOE_THREADS, 0, st, (bf16*)du, (const bf16*)gu, w, pair_of, starts, E, cap, F, (bf16*)dgu, dw)
+#define GBT(ACT) if (F <= 2048) GB(ACT, 32); else if (F <= 4096) GB(ACT, 128); else GB(ACT, 256)
+  if (act == 0) { GBT(0); } else { GBT(1); }
+#undef GBT
+#undef GB
   return ok();
 }
 

@@ -43,7 +43,13 @@ def route(cfg, router_w: torch.Tensor, n2: torch.Tensor, topi: Optional[torch.Te
     are used instead of the top-k while the weights still follow this call's logits (comparisons
     between backends of different precision, where a near-tie may otherwise select differently)."""
     k = cfg.num_experts_per_tok
-    probs = torch.softmax((n2 @ router_w.t()).float(), dim=-1)
+    logits = n2 @ router_w.t()
+    if topi is None and logits.is_cuda:
+        from ..ops.native import route_topk
+        done = route_topk(logits, k, cfg.norm_topk_prob)
+        if done is not None:
+            return done
+    probs = torch.softmax(logits.float(), dim=-1)
     if topi is None:
         topv, topi = torch.topk(probs, k, dim=-1)
     else:
@@ -161,7 +167,7 @@ def _grouped_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor
         add = torch.zeros(n2.shape, dtype=torch.float32, device=n2.device)
         _shared_backward(ops, cfg, p, g, st, n2, dout, add)
     dlogits = ops.route_bwd(st.probs, st.topi, st.w, dw, cfg.norm_topk_prob, n2.dtype)
-    g["router"].copy_(dlogits.t() @ n2)
+    torch.mm(dlogits.t(), n2, out=g["router"])
     return ops.combine_rows(dxs, sl, dlogits @ p["router"], add=add)
 
 

@@ -87,6 +87,7 @@ class _Sig:
     mtb200_block_forward = [P, P, P, P, P]
     mtb200_block_backward = [P, P, P, P, P, P]
     mtb200_gemm_grouped = [P, L, P, L, P, L, P, I, I, I, I, I, I, P, P, I, L, P, P]
+    mtb200_moe_route = [P, I, I, I, I, P, P, P, P]
     mtb200_moe_plan = [P, I, I, I, P, P, P, P, P, P]
     mtb200_moe_gather = [P, P, P, I, I, I, I, F, P, P]
     mtb200_moe_glu_bwd = [P, P, P, P, P, I, I, I, I, P, P, P]
@@ -123,6 +124,22 @@ class ExpertSlabs:
 
 def _ptr(t):
     return None if t is None else t.data_ptr()
+
+
+def route_topk(logits, k: int, renorm: bool):
+    """``(probs, topi, w)`` of a router's logits ``[T, E]``: fp32 softmax, the ``k`` largest of each row and their weights. ``None`` for what the
+    kernel does not take (other types and devices, more than 256 experts or 32 chosen ones), and while no ``NativeOps`` has been made."""
+    T, E = logits.shape
+    if _LIB is None or logits.dtype != torch.bfloat16 or not logits.is_cuda or not logits.is_contiguous() or E > _GROUP_MAX or not 0 < k <= min(E, 32):
+        return None
+    probs = torch.empty(T, E, dtype=torch.float32, device=logits.device)
+    topi = torch.empty(T, k, dtype=torch.int64, device=logits.device)
+    w = torch.empty(T, k, dtype=torch.float32, device=logits.device)
+    rc = _LIB.mtb200_moe_route(logits.data_ptr(), T, E, k, int(renorm), probs.data_ptr(), topi.data_ptr(), w.data_ptr(),
+                                         _raw_stream(logits.device.index))
+    if rc != 0:
+        raise RuntimeError(f"mtb200_moe_route failed with code {rc}")
+    return probs, topi, w
 
 
 class NativeOps:

@@ -1336,3 +1336,73 @@ def test_grouped_products(ops, H, F):
         want = x[s:s + c].float().t() @ y[s:s + c].float()
         assert (g[e] == 0).all() if c == 0 else rel_err(g[e], want) < 6e-3 and max_err(g[e], want) < 5e-2
     ops.check_status()
+
+
+@pytest.mark.parametrize("T,E,k,renorm", [(1, 1, 1, True), (300, 8, 2, True), (77, 33, 5, False), (2051, 64, 8, True), (40, 256, 32, True)])
+def test_router_in_one_launch(ops, T, E, k, renorm):
+    """Against the tensor operations; equal logits (bf16 has few values) go to the lower index."""
+    from mini_trainer_b200.ops.native import route_topk
+    torch.manual_seed(T)
+    logits = torch.randint(-6, 7, (T, E), device="cuda").bfloat16() if T == 77 else bf(T, E, scale=3.0)
+    probs, topi, w = route_topk(logits, k, renorm)
+    want = torch.softmax(logits.float(), -1)
+    assert torch.allclose(probs, want, rtol=1e-5, atol=1e-7)
+    by_rank = torch.sort(probs, dim=-1, descending=True, stable=True).indices[:, :k]
+    assert torch.equal(topi, by_rank)
+    chosen = probs.gather(1, topi)
+    assert torch.allclose(w, chosen / chosen.sum(-1, keepdim=True) if renorm else chosen, rtol=1e-5)
+
+
+def test_router_leaves_other_types_to_the_tensor_operations(ops):
+    from mini_trainer_b200.ops.native import route_topk
+    assert route_topk(torch.zeros(4, 8, device="cuda"), 2, True) is None
+    assert route_topk(bf(4, 257), 2, True) is None and route_topk(bf(4, 64), 33, True) is None and route_topk(bf(8, 8).t(), 2, True) is None
+
+
+@pytest.mark.parametrize("n,E,k", [(1, 1, 1), (31, 3, 1), (4096, 64, 8), (4104, 7, 3), (16408, 256, 8)])
+def test_pairs_are_numbered_in_order_by_expert(ops, n, E, k):
+    torch.manual_seed(n)
+    topi = (torch.rand(n // k, k, device="cuda") ** 3 * E).long()   # uneven, some experts without pairs
+    sl = ops.expert_slabs(topi, E)
+    flat = topi.reshape(-1).cpu()
+    starts, counts, pair_of, row_of = (t.cpu() for t in (sl.starts, sl.counts, sl.pair_of, sl.row_of))
+    at, want = 0, torch.full((sl.cap,), -1, dtype=torch.int32)
+    for e in range(E):
+        mine = (flat == e).nonzero().flatten().int()
+        assert starts[e] == at and counts[e] == len(mine)
+        want[at:at + len(mine)] = mine
+        at += -(-len(mine) // 128) * 128
+    assert starts[E] == at and torch.equal(pair_of, want)
+    assert torch.equal(pair_of[row_of.long()], torch.arange(flat.numel(), dtype=torch.int32))
+    ops.check_status()
+
+
+@pytest.mark.parametrize("T,E,k,W", [(5, 2, 1, 8), (130, 4, 3, 2048), (61, 8, 5, 2056), (40, 3, 2, 4104), (33, 2, 2, 8200)])
+def test_expert_rows_gathered_weighted_and_combined(ops, T, E, k, W):
+    """Widths of a vector, and below and above those at which a row gets more lanes or a second round of them."""
+    torch.manual_seed(W)
+    topi = torch.stack([torch.randperm(max(E, k), device="cuda")[:k] % E for _ in range(T)])
+    sl = ops.expert_slabs(topi, E)
+    src, w = bf(T, W), torch.rand(T, k, device="cuda")
+    rows = ops.gather_rows(src, sl, 0.5)
+    pair = sl.pair_of.long()
+    real = pair >= 0
+    end = int(sl.starts[-1])
+    assert torch.equal(rows[real], (src.float() * 0.5).bfloat16()[pair[real] // k]) and (rows[:end][~real[:end]] == 0).all()
+    base, add = bf(T, W), torch.randn(T, W, device="cuda")
+    out = ops.combine_rows(rows, sl, base, w=w, add=add, scale=0.7)
+    want = base.float() + 0.7 * ((w[..., None] * rows[sl.row_of.long()].view(T, k, W).float()).sum(1) + add)
+    assert rel_err(out, want) < 4e-3
+    gu, du = bf(sl.cap, 2 * W), bf(sl.cap, W)
+    for fn in ("silu", "gelu_tanh"):
+        f = torch.nn.functional.silu if fn == "silu" else lambda x: torch.nn.functional.gelu(x, approximate="tanh")
+        g32 = gu.float().requires_grad_()
+        y = f(g32[:, :W]) * g32[:, W:]
+        wr = torch.zeros(sl.cap, device="cuda")
+        wr[real] = w.reshape(-1)[pair[real]]
+        (y * wr[:, None]).backward(du.float())
+        dgu, wact, dw = ops.expert_glu_bwd(du.clone(), gu, w, sl, fn)
+        assert rel_err(dgu[:end], g32.grad[:end]) < 6e-3 and rel_err(wact[:end], (y * wr[:, None])[:end]) < 6e-3
+        dots = (du.float() * y).sum(-1)
+        assert torch.allclose(dw.reshape(-1)[pair[real]], dots[real].detach(), rtol=1e-3, atol=1e-3 * W ** 0.5)
+    ops.check_status()

@@ -226,6 +226,9 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
 // long launches lose what that saves (with every product launched early: 1.5B block 1933 -> 1868 us, q/k-norm block 1786 -> 1723;
 // but 8B block 20.31 -> 20.42 ms, eight-expert layer 8.35 -> 8.56 ms, sixty-four experts 1140 -> 1148 us).
 constexpr double PDL_MAX_FLOPS = 1e12;
+// Grouped products, counted over the whole row buffers: 477 tokens through 4 experts of 2760 (0.01 TFLOP) 311 -> 301 us, 878 through 32 of 1080 (0.05) 350 -> 342;
+// 2051 through 64 of 1024 (0.2) is the slower early.
+constexpr float PDL_MAX_GROUPED_FLOPS = 1e11f;
 
 // Grouped GEMM: one launch over the slabs of all experts of a mixture-of-experts layer. The rows of expert e are
 // [starts[e], starts[e] + counts[e]) of the gathered row buffers, starts are multiples of GROUP_ALIGN and the rows between the
@@ -244,6 +247,7 @@ struct GroupParams {
   const int* starts;     // [E + 1]
   const int* counts;     // [E]
   int E;
+  float flops;           // of the launch, at most: on all of the row buffers
 };
 
 // Work items of a grouped launch in shared memory: tile_start[e] is the first tile of expert e. (Slab starts and counts are read

@@ -199,7 +199,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
         }
       }
-      if (!GATHER && !GROUP) pdl_trigger();   // what is left is a few products and the last epilogue
+      if (!GATHER && (!GROUP || gr.flops <= PDL_MAX_GROUPED_FLOPS)) pdl_trigger();   // what is left is a few products and the last epilogue
       if (GATHER && g.wait_ns != nullptr) {   // exposed-communication accounting: how long this producer starved
         atomicAdd(g.wait_ns, waited_ns);
         atomicAdd(g.wait_ns + 1, 1ull);
@@ -435,11 +435,11 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int items = tiles * p.e.splits;
   const int grid = (GATHER || items >= g_num_sms) ? g_num_sms : items;
   static const GatherParams none{};
-  // A gathering launch neither overlaps its predecessor nor lets a successor in: its CTAs are counted on to be resident. A long or grouped
+  // A gathering launch neither overlaps its predecessor nor lets a successor in: its CTAs are counted on to be resident. A long
   // launch (PDL_MAX_FLOPS) starts behind its predecessor too.
   if constexpr (GATHER) kern<<<grid, GEMM_THREADS + GATHER_EXTRA_THREADS, GEMM_SMEM, stream>>>(ta, tb, td, maps, p, *gp, GroupParams{});
-  else if (GROUP || 2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<grid, gemm_threads(ACT), GEMM_SMEM, stream>>>(ta, tb, td, maps, p, none, grp ? *grp : GroupParams{});
-  else launch_pdl(kern, grid, gemm_threads(ACT), GEMM_SMEM, stream, ta, tb, td, maps, p, none, GroupParams{});
+  else if (GROUP ? grp->flops > PDL_MAX_GROUPED_FLOPS : 2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<grid, gemm_threads(ACT), GEMM_SMEM, stream>>>(ta, tb, td, maps, p, none, grp ? *grp : GroupParams{});
+  else launch_pdl(kern, grid, gemm_threads(ACT), GEMM_SMEM, stream, ta, tb, td, maps, p, none, grp ? *grp : GroupParams{});
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -554,7 +554,7 @@ int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long l
   if (rc) return rc - 20;
   GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
                EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0}, ActParams{N / 2, gelu}};
-  GroupParams g{starts, counts, E};
+  GroupParams g{starts, counts, E, static_cast<float>(2.0 * rows * N * (mode == 2 ? M : K))};
   if (mode == 3) {
     ActMaps<ACT_GLU> m;
     rc = make_tmap_act(&m.gate, D, N / 2, rows, ldd);

@@ -409,7 +409,9 @@ class NativeOps:
         name, splits, _ = self._gemm_plans.get((T, N, K, None)) or self._plan_gemm(T, N, K, None)
         # A product that splits its reduction is two launches with its activation: 700 x 2048 x 8192 32 us, 43 whole with the activation inside (level at
         # reductions of 4096: 512 x 2048 24.6 and 24.9).
-        if splits > 1 and (gated or fn == "gelu_tanh"):
+        assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+        plain = w.is_contiguous() and K % 8 == 0 and F % 8 == 0   # what one launch can address
+        if (splits > 1 or not plain) and (gated or fn == "gelu_tanh"):
             pre = self.linear(x, w, bias)
             return pre, (self.swiglu(pre, fn) if gated else self.gelu(pre))
         pre = torch.empty(T, N, dtype=x.dtype, device=self.device)

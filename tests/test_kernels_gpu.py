@@ -1406,3 +1406,15 @@ def test_expert_rows_gathered_weighted_and_combined(ops, T, E, k, W):
         dots = (du.float() * y).sum(-1)
         assert torch.allclose(dw.reshape(-1)[pair[real]], dots[real].detach(), rtol=1e-3, atol=1e-3 * W ** 0.5)
     ops.check_status()
+
+
+def test_product_with_an_activation_takes_what_the_two_launches_take(ops):
+    """Weights that are rows of a wider matrix, and a reduction that is no multiple of eight inside padded rows."""
+    torch.manual_seed(0)
+    x, w = bf(50, 64), bf(2 * 40, 96, scale=0.2)
+    for xs, ws in ((x, w[:, :64]), (x[:, :60], w[:, :60])):
+        pre, act = ops.linear_act(xs, ws)
+        assert rel_err(pre, xs.float() @ ws.float().t()) < 6e-3
+        assert torch.equal(act, ops.swiglu(pre))
+    with pytest.raises(AssertionError):
+        ops.linear_act(x.float(), w[:, :64].contiguous())

@@ -142,29 +142,38 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const long long*
   if (me == E - 1) for (int r = end + threadIdx.x; r < cap; r += PLAN_THREADS) pair_of[r] = -1;
 }
 
-// out[row] = scale * src[pair_of[row] / k], zeros in padding. Rows past the last slab are left alone.
-__global__ void __launch_bounds__(128) moe_gather_kernel(const bf16* __restrict__ src, const int* __restrict__ pair_of, const int* __restrict__ starts,
-                                                        int E, int k, int H, float scale, bf16* __restrict__ out) {
+// out[row] = scale * src[pair_of[row] / k], zeros in padding. Rows past the last slab are left alone. A warp per row, eight vectors of it
+// in flight per lane (a block of 128 threads per row had two; layer of 64 experts, three gathers of 20 500 rows of 2048: 1077 -> 1049 us; eight experts level:
+// bound by writing the rows).
+constexpr int GATHER_WARPS = 4;
+__global__ void __launch_bounds__(32 * GATHER_WARPS) moe_gather_kernel(const bf16* __restrict__ src, const int* __restrict__ pair_of, const int* __restrict__ starts,
+                                                                      int E, int k, int cap, int H, float scale, bf16* __restrict__ out) {
   pdl_trigger();
   pdl_wait();
-  const long long row = blockIdx.x;
-  if (row >= starts[E]) return;
+  const long long row = static_cast<long long>(blockIdx.x) * GATHER_WARPS + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= cap || row >= starts[E]) return;
   const int pair = pair_of[row];
   bf16* dst = out + row * H;
-  if (pair < 0) {
-    for (int c = threadIdx.x * 8; c < H; c += 128 * 8) *reinterpret_cast<uint4*>(dst + c) = make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  const bf16* s = src + static_cast<long long>(pair / k) * H;
-  for (int c = threadIdx.x * 8; c < H; c += 128 * 8) {
-    Vec8 v; v.load(s + c);
-    if (scale != 1.f) {
-      float f[8]; v.get(f);
+  const bf16* s = pair < 0 ? nullptr : src + static_cast<long long>(pair / k) * H;
+  for (int c0 = lane * 8; c0 < H; c0 += 8 * 256) {
+    Vec8 v[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] *= scale;
-      v.set(f);
+    for (int j = 0; j < 8; ++j) {
+      v[j].u = make_uint4(0u, 0u, 0u, 0u);
+      if (s != nullptr && c0 + j * 256 < H) v[j].load(s + c0 + j * 256);
     }
-    v.store(dst + c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (c0 + j * 256 >= H) break;
+      if (scale != 1.f) {
+        float f[8]; v[j].get(f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] *= scale;
+        v[j].set(f);
+      }
+      v[j].store(dst + c0 + j * 256);
+    }
   }
 }
 
@@ -322,7 +331,7 @@ int mtb200_moe_gather(const void* src, const int* pair_of, const int* starts, in
                       cudaStream_t st) {
   if (cap <= 0) return 0;
   if (H % 8 || k <= 0) return -10;
-  launch_pdl(moe_gather_kernel, cap, 128, 0, st, (const bf16*)src, pair_of, starts, E, k, H, scale, (bf16*)out);
+  launch_pdl(moe_gather_kernel, (cap + GATHER_WARPS - 1) / GATHER_WARPS, 32 * GATHER_WARPS, 0, st, (const bf16*)src, pair_of, starts, E, k, cap, H, scale, (bf16*)out);
   return ok();
 }
 

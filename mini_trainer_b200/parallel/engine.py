@@ -849,8 +849,8 @@ class ShardedEngine:
     def train_step(self, minibatches: list, lr: float) -> dict:
         """``minibatches``: collated dicts (``data.sampler.mb_collate_fn``). One optimizer step.
 
-        Device work is queued without host synchronisation; the returned tensors
-        (``loss_sum``, ``grad_norm``) are read by the caller when it logs.
+        Device work is queued without host synchronisation; the returned tensors (``loss_sum``, ``grad_norm``) are read by the
+        caller when it logs. (The copies of a minibatch of more than 8192 tokens may wait for the device, see ``make_packed_batch``.)
         """
         loss_sum = torch.zeros((), dtype=torch.float32, device=self.device)
         ntok = h2d = 0

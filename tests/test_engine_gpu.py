@@ -325,3 +325,24 @@ def test_block_inputs_offloaded_to_host_give_identical_gradients(monkeypatch):
     # the attention backward adds dQ tiles in arrival order (fp32), everything else is deterministic
     for a, b in zip(g0, g1):
         assert ((a - b).norm() / (a.norm() + 1e-12)).item() < 1e-5
+
+
+@pytest.mark.parametrize("tokens", [3000, 8000])
+def test_minibatches_are_moved_without_waiting_for_the_device(tokens):
+    """The host runs ahead of the device by several minibatches. (The best of three: the machine's other users hold the host up at times.)"""
+    a = torch.randn(8192, 8192, device="cuda").bfloat16()
+    b = torch.empty_like(a)
+    mb = make_mb([tokens // 3, tokens - tokens // 3], 64)
+    for attempt in range(3):
+        torch.cuda.synchronize()
+        for _ in range(80):   # about 60 ms
+            torch.mm(a, a, out=b)
+        done = torch.cuda.Event()
+        done.record()
+        batches = [D.make_packed_batch(mb, "cuda:0") for _ in range(6)]
+        waited = done.query()
+        torch.cuda.synchronize()
+        if not waited:
+            break
+    assert not waited
+    assert torch.equal(batches[-1].input_ids.cpu(), mb["input_ids"].reshape(-1))

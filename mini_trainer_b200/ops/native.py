@@ -406,14 +406,15 @@ class NativeOps:
         T, K = x.shape
         N = w.shape[0]
         F = N // 2 if gated else N
-        name, splits, _ = self._gemm_plans.get((T, N, K, None)) or self._plan_gemm(T, N, K, None)
-        # A product that splits its reduction is two launches with its activation: 700 x 2048 x 8192 32 us, 43 whole with the activation inside (level at
-        # reductions of 4096: 512 x 2048 24.6 and 24.9).
         assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-        plain = w.is_contiguous() and K % 8 == 0 and F % 8 == 0   # what one launch can address
-        if (splits > 1 or not plain) and (gated or fn == "gelu_tanh"):
+        name, splits, _ = self._gemm_plans.get((T, N, K, None)) or self._plan_gemm(T, N, K, None)
+        # Two launches where one cannot address the weight, and for a product that splits its reduction: 700 x 2048 x 8192 32 us, 43 whole with the
+        # activation inside (level at reductions of 4096: 512 x 2048 24.6 and 24.9). No kernel is SiLU alone.
+        plain = w.is_contiguous() and K % 8 == 0 and F % 8 == 0
+        alone = gated or fn == "gelu_tanh"
+        if not plain or (splits > 1 and alone):
             pre = self.linear(x, w, bias)
-            return pre, (self.swiglu(pre, fn) if gated else self.gelu(pre))
+            return pre, (torch.nn.functional.silu(pre) if not alone else self.swiglu(pre, fn) if gated else self.gelu(pre))
         pre = torch.empty(T, N, dtype=x.dtype, device=self.device)
         act = torch.empty(T, F, dtype=x.dtype, device=self.device)
         self._call("mtb200_gemm_act", x.data_ptr(), x.stride(0), w.data_ptr(), pre.data_ptr(), act.data_ptr(), _ptr(bias), 1 if gated else 2, int(fn != "silu"),

@@ -1418,3 +1418,17 @@ def test_product_with_an_activation_takes_what_the_two_launches_take(ops):
         assert torch.equal(act, ops.swiglu(pre))
     with pytest.raises(AssertionError):
         ops.linear_act(x.float(), w[:, :64].contiguous())
+
+
+@pytest.mark.parametrize("fn", ["silu", "gelu_tanh"])
+@pytest.mark.parametrize("gated", [True, False])
+def test_product_with_an_activation_and_weights_that_are_rows_of_a_wider_matrix(ops, gated, fn):
+    torch.manual_seed(1)
+    f = {"silu": torch.nn.functional.silu, "gelu_tanh": lambda x: torch.nn.functional.gelu(x, approximate="tanh")}[fn]
+    x, w = bf(50, 64), bf(80, 96, scale=0.2)
+    for xs, ws in ((x, w[:, :64]), (x[:, :60], w[:, :60])):
+        pre, act = ops.linear_act(xs, ws, fn, gated)
+        assert rel_err(pre, xs.float() @ ws.float().t()) < 6e-3
+        p = pre.float()
+        assert rel_err(act, f(p[:, :40]) * p[:, 40:] if gated else f(p)) < 4e-3   # one rounding of an fp32 value
+    ops.check_status()

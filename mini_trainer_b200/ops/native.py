@@ -99,6 +99,7 @@ class _Sig:
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
+_ACT = {"silu": 0, "gelu_tanh": 1}   # of csrc/gemm_act.cuh
 _GEMM_TAGS = (("gemm_nt", "gemm_nn"), ("gemm_tt", "gemm_tn"))   # [A stored [K, M]][B stored [K, N]]
 _SPLIT_COUNTERS = 4096          # csrc/gemm_epilogue.cuh
 _SPLIT_FLOATS = 32 << 20        # most that the partials of a launch take: 128 MB
@@ -405,7 +406,7 @@ class NativeOps:
         ``pre`` [T, F] and ``fn(pre)``. A bias only without a gate."""
         T, K = x.shape
         N = w.shape[0]
-        F = N // 2 if gated else N
+        F, code = N // 2 if gated else N, _ACT[fn]
         assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
         name, splits, _ = self._gemm_plans.get((T, N, K, None)) or self._plan_gemm(T, N, K, None)
         # Two launches where one cannot address the weight, and for a product that splits its reduction: 700 x 2048 x 8192 32 us, 43 whole with the
@@ -417,7 +418,7 @@ class NativeOps:
             return pre, (torch.nn.functional.silu(pre) if not alone else self.swiglu(pre, fn) if gated else self.gelu(pre))
         pre = torch.empty(T, N, dtype=x.dtype, device=self.device)
         act = torch.empty(T, F, dtype=x.dtype, device=self.device)
-        self._call("mtb200_gemm_act", x.data_ptr(), x.stride(0), w.data_ptr(), pre.data_ptr(), act.data_ptr(), _ptr(bias), 1 if gated else 2, int(fn != "silu"),
+        self._call("mtb200_gemm_act", x.data_ptr(), x.stride(0), w.data_ptr(), pre.data_ptr(), act.data_ptr(), _ptr(bias), 1 if gated else 2, code,
                    T, F, K, int(name == "mtb200_gemm2_bf16"), self.status.data_ptr(), self._st(), tag="gemm_nt_act")
         return pre, act
 
@@ -652,7 +653,7 @@ class NativeOps:
         return out
 
     def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride, act=None, fn="silu"):
-        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), int(fn != "silu"), mode, sl.cap, M, N, K,
+        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), _ACT[fn], mode, sl.cap, M, N, K,
                    sl.starts.data_ptr(), sl.counts.data_ptr(), sl.counts.shape[0], stride, self.status.data_ptr(), self._st(),
                    tag="gemm_grouped_" + ("nt", "nn", "tn", "nt_act")[mode])
         return out

@@ -1432,3 +1432,12 @@ def test_product_with_an_activation_and_weights_that_are_rows_of_a_wider_matrix(
         p = pre.float()
         assert rel_err(act, f(p[:, :40]) * p[:, 40:] if gated else f(p)) < 4e-3   # one rounding of an fp32 value
     ops.check_status()
+
+
+def test_activations_that_no_kernel_has_are_refused(ops):
+    x, w = bf(8, 64), bf(32, 64)
+    sl, _ = _slabs(ops, [3, 5])
+    for call in (lambda: ops.linear_act(x, w, "relu"), lambda: ops.linear_act(x, w, "relu", False), lambda: ops.linear_act(x, w.t().contiguous().t(), "relu", False),
+                 lambda: ops.grouped_linear_act(bf(sl.cap, 64), (bf(16, 64), 16 * 64), sl, "relu")):
+        with pytest.raises(KeyError):
+            call()

@@ -69,7 +69,7 @@ struct BlockIO {
   const void* dout;       // backward
   void* dx;
   void* ws;               // workspace
-  u64* counters;          // split launches: arrival counters of the stream, one epoch per product (and one for the attention), partial sums
+  u64* counters;          // split launches: arrival counters of the stream, growing epochs (used in launch order: GEMMS + 1 are enough), partial sums
   const u64* epochs;
   float* part;
   long long part_bytes;
@@ -89,11 +89,12 @@ struct Carver {   // 256-byte aligned pieces of the workspace; with a null base 
   }
 };
 
-int gemm(const BlockSpec& s, const BlockIO& io, int which, const void* a, long long lda, int a_mn, const void* b, long long ldb, int b_mn, void* d, int M, int N,
+// `epoch`: the next one. Arrivals on these counters are told apart by epochs that grow from launch to launch.
+int gemm(const BlockSpec& s, const BlockIO& io, const u64*& epoch, int which, const void* a, long long lda, int a_mn, const void* b, long long ldb, int b_mn, void* d, int M, int N,
          int K, const void* r, const void* bias, float alpha, cudaStream_t st) {
   const int splits = io.part != nullptr ? s.splits[which] : 1;
   auto f = s.pair[which] ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
-  return f(a, lda, a_mn, b, ldb, b_mn, d, N, 0, r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? io.epochs[which] : 0,
+  return f(a, lda, a_mn, b, ldb, b_mn, d, N, 0, r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
            splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, nullptr, io.status, st);
 }
 
@@ -111,28 +112,29 @@ long long forward(const BlockSpec& s, const BlockParams& p, const BlockIO& io, b
   void* n2 = io.n2 ? io.n2 : ws.take(T * s.H * 2);
   void* act = io.act ? io.act : ws.take(T * s.F * 2);
   if (measure) return ws.at;
+  const u64* epoch = io.epochs;
   RUN(norm(s, io, io.x, p.ln1, p.bln1, n1, io.mean1, io.rstd1, st), 1);
-  RUN(gemm(s, io, G_QKV, n1, s.H, 0, p.wqkv, s.H, 0, io.qkv, s.T, Q, s.H, nullptr, p.bqkv, 1.f, st), 1);
+  RUN(gemm(s, io, epoch, G_QKV, n1, s.H, 0, p.wqkv, s.H, 0, io.qkv, s.T, Q, s.H, nullptr, p.bqkv, 1.f, st), 1);
   if (s.qk_norm) RUN(mtb200_head_rmsnorm_fwd(io.qkv, p.qn, p.kn, io.qk_pre, io.rstd_qk, io.inv_freq ? io.pos : nullptr, io.inv_freq, s.eps, s.T, Q, s.Hq, nh, s.D, st), 1);
   else if (io.inv_freq) RUN(mtb200_rope(io.qkv, io.pos, io.inv_freq, s.T, Q, nh, s.D, 0, st), 1);
   if (!io.have_attn) {
     if (s.attn_form == 0) RUN(mtb200_attn_fwd_one(io.qkv, Q, io.attn, q, io.lse, io.fwd_plan, s.fwd_items, s.T, s.Hq, s.Hkv, s.D, s.scale, io.status, st), 1);
     else RUN(mtb200_attn_fwd(io.qkv, Q, io.attn, q, io.lse, io.fwd_plan, s.fwd_items, s.T, s.Hq, s.Hkv, s.D, s.attn_form - 1, s.scale, io.status, st), 1);
   }
-  RUN(gemm(s, io, G_O, io.attn, q, 0, p.wo, q, 0, io.h1, s.T, s.H, q, io.x, p.bo, s.alpha, st), 1);
+  RUN(gemm(s, io, epoch, G_O, io.attn, q, 0, p.wo, q, 0, io.h1, s.T, s.H, q, io.x, p.bo, s.alpha, st), 1);
   RUN(norm(s, io, io.h1, p.ln2, p.bln2, n2, io.mean2, io.rstd2, st), 1);
   if (!s.need_out) {
-    RUN(gemm(s, io, G_GU, n2, s.H, 0, p.wgu, s.H, 0, io.gu, s.T, width, s.H, nullptr, p.bgu, 1.f, st), 1);
+    RUN(gemm(s, io, epoch, G_GU, n2, s.H, 0, p.wgu, s.H, 0, io.gu, s.T, width, s.H, nullptr, p.bgu, 1.f, st), 1);
     return 0;
   }
   if (s.splits[G_GU] > 1) {   // a split product has no room for the activation (ops/native.py, linear_act)
-    RUN(gemm(s, io, G_GU, n2, s.H, 0, p.wgu, s.H, 0, io.gu, s.T, width, s.H, nullptr, p.bgu, 1.f, st), 1);
+    RUN(gemm(s, io, epoch, G_GU, n2, s.H, 0, p.wgu, s.H, 0, io.gu, s.T, width, s.H, nullptr, p.bgu, 1.f, st), 1);
     if (!s.gated) RUN(mtb200_gelu_fwd(io.gu, act, T * s.F, st), 1);
     else RUN(s.gelu ? mtb200_geglu_fwd(io.gu, act, T, s.F, st) : mtb200_swiglu_fwd(io.gu, act, T, s.F, st), 1);
   } else {
     RUN(mtb200_gemm_act(n2, s.H, p.wgu, io.gu, act, p.bgu, s.gated ? 1 : 2, s.gelu, s.T, s.F, s.H, s.pair[G_GU], io.status, st), 1);
   }
-  RUN(gemm(s, io, G_DOWN, act, s.F, 0, p.wd, s.F, 0, io.out, s.T, s.H, s.F, io.h1, p.bd, s.alpha, st), 1);
+  RUN(gemm(s, io, epoch, G_DOWN, act, s.F, 0, p.wd, s.F, 0, io.out, s.T, s.H, s.F, io.h1, p.bd, s.alpha, st), 1);
   return 0;
 }
 
@@ -155,8 +157,9 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
   float* again = ws.take<float>(T * 2 * 4);         // statistics of a norm that is formed again
   void* dqkv = dgu;
   if (measure) return ws.at;
+  const u64* epoch = io.epochs;
   auto wgrad = [&](int which, const void* dy, long long N, const void* x, long long K, void* dw, void* db) -> int {
-    int rc = gemm(s, io, which, dy, N, 1, x, K, 1, dw, N, K, s.T, nullptr, nullptr, which == W_DOWN || which == W_O ? s.alpha : 1.f, st);
+    int rc = gemm(s, io, epoch, which, dy, N, 1, x, K, 1, dw, N, K, s.T, nullptr, nullptr, which == W_DOWN || which == W_O ? s.alpha : 1.f, st);
     if (!rc && db) { rc = mtb200_colsum(dy, N, db, cols, s.T, N, st); *launches += 2; }
     ++*launches;
     return rc;
@@ -167,7 +170,7 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
                        : mtb200_rmsnorm_bwd(dn, x, rstd, w, add, dx, rows, dw, s.T, s.H, io.status, st);
   };
   // MLP
-  RUN(gemm(s, io, D_DOWN, io.dout, s.H, 0, p.wd, s.F, 1, dact, s.T, s.F, s.H, nullptr, nullptr, s.alpha, st), 1);
+  RUN(gemm(s, io, epoch, D_DOWN, io.dout, s.H, 0, p.wd, s.F, 1, dact, s.T, s.F, s.H, nullptr, nullptr, s.alpha, st), 1);
   if (io.act) {
     if (!s.gated) RUN(mtb200_gelu_bwd(dact, io.gu, dgu, T * s.F, st), 1);
     else RUN(s.gelu ? mtb200_geglu_bwd(dact, io.gu, dgu, T, s.F, st) : mtb200_swiglu_bwd(dact, io.gu, dgu, T, s.F, st), 1);
@@ -176,21 +179,21 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
     else RUN(s.gelu ? mtb200_geglu_bwd_act(dact, io.gu, dgu, T, s.F, st) : mtb200_swiglu_bwd_act(dact, io.gu, dgu, T, s.F, st), 1);
   }
   RUN(wgrad(W_DOWN, io.dout, s.H, io.act ? io.act : dact, s.F, g.wd, g.bd), 0);
-  RUN(gemm(s, io, D_GU, dgu, width, 0, p.wgu, s.H, 1, dn, s.T, s.H, width, nullptr, nullptr, 1.f, st), 1);
+  RUN(gemm(s, io, epoch, D_GU, dgu, width, 0, p.wgu, s.H, 1, dn, s.T, s.H, width, nullptr, nullptr, 1.f, st), 1);
   if (!io.n2) RUN(norm(s, io, io.h1, p.ln2, p.bln2, n2, again, again + T, st), 1);
   RUN(wgrad(W_GU, dgu, width, n2, s.H, g.wgu, g.bgu), 0);
   RUN(norm_bwd(io.h1, io.mean2, io.rstd2, p.ln2, io.dout, dh1, g.ln2, g.bln2), 0);
   // attention
-  RUN(gemm(s, io, D_O, dh1, s.H, 0, p.wo, q, 1, dattn, s.T, q, s.H, nullptr, nullptr, s.alpha, st), 1);
+  RUN(gemm(s, io, epoch, D_O, dh1, s.H, 0, p.wo, q, 1, dattn, s.T, q, s.H, nullptr, nullptr, s.alpha, st), 1);
   RUN(wgrad(W_O, dh1, s.H, io.attn, q, g.wo, g.bo), 0);
   const int splits = io.part != nullptr ? s.bwd_splits : 1;
   RUN(mtb200_attn_bwd(io.qkv, Q, io.attn, q, dattn, q, dqkv, Q, io.lse, delta, dq, io.bwd_plan, s.bwd_items, s.T, s.Hq, s.Hkv, s.D, splits,
-                      splits > 1 ? io.counters : nullptr, splits > 1 ? io.epochs[GEMMS] : 0, splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, s.scale,
+                      splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0, splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, s.scale,
                       io.status, st), 3);
   if (s.qk_norm) RUN(mtb200_head_rmsnorm_bwd(dqkv, io.qk_pre, io.rstd_qk, p.qn, p.kn, rows, g.qn, g.kn, io.inv_freq ? io.pos : nullptr, io.inv_freq, s.T, Q, nh * s.D,
                                              s.Hq, nh, s.D, st), 2);
   else if (io.inv_freq) RUN(mtb200_rope(dqkv, io.pos, io.inv_freq, s.T, Q, nh, s.D, 1, st), 1);
-  RUN(gemm(s, io, D_QKV, dqkv, Q, 0, p.wqkv, s.H, 1, dn, s.T, s.H, Q, nullptr, nullptr, 1.f, st), 1);
+  RUN(gemm(s, io, epoch, D_QKV, dqkv, Q, 0, p.wqkv, s.H, 1, dn, s.T, s.H, Q, nullptr, nullptr, 1.f, st), 1);
   if (!io.n1) RUN(norm(s, io, io.x, p.ln1, p.bln1, n1, again, again + T, st), 1);
   RUN(wgrad(W_QKV, dqkv, Q, n1, s.H, g.wqkv, g.bqkv), 0);
   RUN(norm_bwd(io.x, io.mean1, io.rstd1, p.ln1, dh1, io.dx, g.ln1, g.bln1), 0);

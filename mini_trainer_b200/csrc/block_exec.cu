@@ -146,7 +146,7 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
   void* dact = ws.take(T * s.F * 2);                // then, unless it was kept, the activation
   void* dn = ws.take(T * s.H * 2);                  // gradient of the normalised rows, of either norm
   void* n2 = io.n2 ? io.n2 : ws.take(T * s.H * 2);
-  void* n1 = io.n1 ? io.n1 : n2 != io.n2 ? n2 : ws.take(T * s.H * 2);
+  void* n1 = io.n1 ? io.n1 : io.n2 ? ws.take(T * s.H * 2) : n2;   // n2 is read for the last time before n1 is formed
   void* dh1 = ws.take(T * s.H * 2);
   void* dattn = ws.take(T * q * 2);
   float* delta = ws.take<float>(T * s.Hq * 4);

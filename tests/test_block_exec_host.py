@@ -99,3 +99,16 @@ def test_split_launches_are_numbered_in_the_order_they_are_queued(lib, bwd, gate
     got = queue(lib, s, io, bwd)
     assert len(got) == (9 if bwd else 4) and all(k == 2 for k, _ in got)
     assert all(a < b for (_, a), (_, b) in zip(got, got[1:])), got
+
+
+@pytest.mark.parametrize("layernorm", [0, 1])
+@pytest.mark.parametrize("keep", [(), ("n1",), ("n2",)])
+def test_workspace_is_what_the_call_lays_out(lib, keep, layernorm):
+    """Statistics of a norm that is formed again come last."""
+    s, io = make(layernorm=layernorm, T=321)
+    for name in keep:
+        setattr(io, name, 1 << 20)
+    size = lib.mtb200_block_workspace(ctypes.byref(s), ctypes.byref(io), 1)
+    queue(lib, s, io, 1)
+    end = ctypes.c_void_p.in_dll(lib, "last_rstd").value - WS + 321 * 4   # the second of two rows
+    assert size == -(-end // 256) * 256

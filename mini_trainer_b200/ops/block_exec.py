@@ -2,8 +2,8 @@
 
 The block is that of ``models/decoder.py`` on the kernels of ``native.py``: the same launches in the same order, without the interpreter
 between them. ``forward`` and ``backward`` return ``None`` for what stays with the Python form: other block forms, parameters that are being
-gathered, tensors that are not laid out as the native call addresses them, and blocks whose temporaries are large (``MOST_WORKSPACE``): there the
-device is the bound, and the Python form gives each temporary back when it is done with.
+gathered, tensors that are not laid out as the native call addresses them, and blocks whose temporaries are large (``MOST_WORKSPACE``; the device
+is the bound there) or find no room: the Python form gives each temporary back when it is done with.
 """
 from __future__ import annotations
 
@@ -81,12 +81,20 @@ def _spec(ops, cfg, T: int):
     return hit
 
 
-def _workspace(ops, spec, io, bwd: int, sizes: dict):
+def _workspace_bytes(ops, spec, io, bwd: int, sizes: dict) -> int:
     what = (bwd, io.n1 is None, io.n2 is None, io.act is None)
     n = sizes.get(what)
     if n is None:
         n = sizes[what] = ops.lib.mtb200_block_workspace(ctypes.byref(spec), ctypes.byref(io), bwd)
-    return None if n > MOST_WORKSPACE else torch.empty(max(n, 1), dtype=torch.uint8, device=ops.device)
+    return n
+
+
+def _workspace(ops, n: int):
+    """The last tensor that a call takes: the Python form needs less than this at a time, and its results as well."""
+    try:
+        return torch.empty(max(n, 1), dtype=torch.uint8, device=ops.device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def _split(ops, io, stream, nbytes: int):
@@ -120,8 +128,8 @@ def forward(ops, acts_type, cfg, p: dict, x, batch, inv_freq, keep, saved_attn, 
     if full:   # (otherwise they live in the workspace)
         n1, n2, act = bf(T, H), bf(T, H), bf(T, F) if need_out else None
         io.n1, io.n2, io.act = n1.data_ptr(), n2.data_ptr(), _ptr(act)
-    ws = _workspace(ops, spec, io, 0, sizes)
-    if ws is None:
+    ws_bytes = _workspace_bytes(ops, spec, io, 0, sizes)
+    if ws_bytes > MOST_WORKSPACE:
         return None
     qkv, h1, gu = bf(T, Q), bf(T, H), bf(T, 2 * F if cfg.mlp_gated else F)
     out = bf(T, H) if need_out else None
@@ -129,6 +137,9 @@ def forward(ops, acts_type, cfg, p: dict, x, batch, inv_freq, keep, saved_attn, 
     r1, r2 = f32(T), f32(T)
     m1, m2 = (f32(T), f32(T)) if ln else (None, None)
     pre, rqk = (bf(T, q + cfg.kv_size) if keep else None, f32(T * (spec.Hq + spec.Hkv))) if spec.qk_norm else (None, None)
+    ws = _workspace(ops, ws_bytes)
+    if ws is None:
+        return None
     io.qkv, io.attn, io.h1, io.gu, io.out, io.qk_pre = qkv.data_ptr(), attn.data_ptr(), h1.data_ptr(), gu.data_ptr(), _ptr(out), _ptr(pre)
     io.mean1, io.rstd1, io.lse, io.mean2, io.rstd2, io.rstd_qk = _ptr(m1), r1.data_ptr(), lse.data_ptr(), _ptr(m2), r2.data_ptr(), _ptr(rqk)
     io.pos, io.inv_freq, io.ws = batch.position_ids.data_ptr(), _ptr(inv_freq), ws.data_ptr()
@@ -160,10 +171,13 @@ def backward(ops, cfg, p: dict, g: dict, a, dout, batch, inv_freq):
     spec = Spec.from_buffer_copy(base)
     io = IO()
     io.n1, io.n2, io.act = _ptr(a.n1), _ptr(a.n2), _ptr(a.act)
-    ws = _workspace(ops, spec, io, 1, sizes)
-    if ws is None:
+    ws_bytes = _workspace_bytes(ops, spec, io, 1, sizes)
+    if ws_bytes > MOST_WORKSPACE:
         return None
     dx = torch.empty_like(x)
+    ws = _workspace(ops, ws_bytes)
+    if ws is None:
+        return None
     io.x, io.qkv, io.attn, io.h1, io.gu, io.qk_pre = x.data_ptr(), a.qkv.data_ptr(), a.attn.data_ptr(), a.h1.data_ptr(), a.gu.data_ptr(), _ptr(a.qk_pre)
     (m1, r1), (m2, r2) = (a.rstd1, a.rstd2) if spec.layernorm else ((None, a.rstd1), (None, a.rstd2))
     io.mean1, io.rstd1, io.lse, io.mean2, io.rstd2, io.rstd_qk = _ptr(m1), r1.data_ptr(), a.lse.data_ptr(), _ptr(m2), r2.data_ptr(), _ptr(a.rstd_qk)

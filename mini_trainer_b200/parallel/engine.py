@@ -890,7 +890,8 @@ def kept_bytes(cfg: ModelConfig, tokens: int, es: int = 2) -> tuple:
 
 
 def working_set_bytes(cfg: ModelConfig, tokens: int, es: int = 2) -> int:
-    """Working set of one block's backward, with the partial sums of a product that is split."""
+    """Working set of one block's backward, with the partial sums of a product that is split. (A dense block that is queued by one call holds all
+    its temporaries until the end: up to 256 MB, which the margins of the plan cover; without room for them it goes launch by launch.)"""
     h = cfg.hidden_size
     f = (cfg.expert_intermediate_size if cfg.is_moe else cfg.intermediate_size) * cfg.mlp_rows_factor
     work = tokens * es * (7 * h + cfg.qkv_size + 6 * f)

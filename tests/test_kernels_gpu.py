@@ -1441,3 +1441,35 @@ def test_activations_that_no_kernel_has_are_refused(ops):
                  lambda: ops.grouped_linear_act(bf(sl.cap, 64), (bf(16, 64), 16 * 64), sl, "relu")):
         with pytest.raises(KeyError):
             call()
+
+
+def test_block_without_memory_for_its_temporaries_goes_launch_by_launch(ops, monkeypatch):
+    from mini_trainer_b200.data.sampler import mb_collate_fn
+    from mini_trainer_b200.models import decoder as D, layout as L
+    from mini_trainer_b200.models.config import ModelConfig
+    from mini_trainer_b200.ops import block_exec
+    cfg = ModelConfig(model_type="llama", vocab_size=64, hidden_size=128, intermediate_size=256, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1,
+                      head_dim=64)
+    torch.manual_seed(0)
+    lay = L.GroupLayout("block0", L.block_entries(cfg), 1)
+    p = lay.views((torch.randn(lay.padded_numel, device="cuda") * 0.05).bfloat16())
+    g = lay.views(torch.zeros(lay.padded_numel, dtype=torch.bfloat16, device="cuda"))
+    ids = torch.randint(0, 64, (90,))
+    batch = D.make_packed_batch(mb_collate_fn([{"input_ids": ids, "labels": ids.clone(), "len": 90, "num_loss_counted_tokens": 90}], 90), "cuda")
+    x, dout, inv = bf(90, 128), bf(90, 128, scale=0.1), cfg.rope_inv_freq().cuda()
+    want, acts, _ = D.block_forward(ops, cfg, p, x, batch, inv, keep="compact")
+
+    class Torch:   # no memory for the workspace, which is the only tensor of bytes
+        def __getattr__(self, name):
+            return getattr(torch, name)
+
+        def empty(self, *a, dtype=None, **kw):
+            if dtype == torch.uint8:
+                raise torch.OutOfMemoryError("no memory")
+            return torch.empty(*a, dtype=dtype, **kw)
+    monkeypatch.setattr(block_exec, "torch", Torch())
+    out, acts, _ = D.block_forward(ops, cfg, p, x, batch, inv, keep="compact")
+    assert torch.equal(out, want)
+    dx = D.block_backward(ops, cfg, p, g, acts, dout, batch, inv)
+    assert dx.isfinite().all() and all(t.isfinite().all() for t in g.values())
+    ops.check_status()

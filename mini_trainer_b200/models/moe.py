@@ -167,7 +167,11 @@ def _grouped_backward(ops, cfg, p: dict, g: dict, st: MoeState, n2: torch.Tensor
         add = torch.zeros(n2.shape, dtype=torch.float32, device=n2.device)
         _shared_backward(ops, cfg, p, g, st, n2, dout, add)
     dlogits = ops.route_bwd(st.probs, st.topi, st.w, dw, cfg.norm_topk_prob, n2.dtype)
-    torch.mm(dlogits.t(), n2, out=g["router"])
+    grouter = g["router"]
+    if (grouter.dtype, grouter.device, grouter.shape) == (n2.dtype, n2.device, p["router"].shape):
+        torch.mm(dlogits.t(), n2, out=grouter)   # in one launch
+    else:
+        grouter.copy_(dlogits.t() @ n2)
     return ops.combine_rows(dxs, sl, dlogits @ p["router"], add=add)
 
 

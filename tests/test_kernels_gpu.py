@@ -1473,3 +1473,22 @@ def test_block_without_memory_for_its_temporaries_goes_launch_by_launch(ops, mon
     dx = D.block_backward(ops, cfg, p, g, acts, dout, batch, inv)
     assert dx.isfinite().all() and all(t.isfinite().all() for t in g.values())
     ops.check_status()
+
+
+def test_router_gradient_of_another_type(ops):
+    """A gradient tensor that is not of the activations' type gets the converted values; one of another shape is refused."""
+    from mini_trainer_b200.models import moe as M
+    cfg, p, g, n2, h1, dout = _moe_layer(70, 64, 40, 4, 2, 4)
+    got = []
+    for dtype in (torch.bfloat16, torch.float32):
+        g["router"] = torch.full_like(p["router"], float("nan"), dtype=dtype)
+        out, st = M.moe_forward(ops, cfg, p, n2, h1, True, False)
+        assert st.slabs is not None
+        M.moe_backward(ops, cfg, p, g, st, n2, dout)
+        got.append(g["router"])
+    assert got[1].dtype == torch.float32 and torch.equal(got[0].float(), got[1])
+    for wrong in (torch.empty(5, 64, dtype=torch.bfloat16, device="cuda"), torch.empty(4, 32, dtype=torch.bfloat16, device="cuda")):
+        g["router"] = wrong
+        with pytest.raises(RuntimeError):
+            M.moe_backward(ops, cfg, p, g, st, n2, dout)
+    ops.check_status()

@@ -322,6 +322,7 @@ class NativeOps:
         """dweight[ids] += dx, deterministic: one block sums the rows of an id in fp32, in token order. Few tokens are searched for equal ids
         as they are, more are grouped by a stable sort."""
         if ids.shape[0] <= _EMB_SCAN:
+            ids = ids.contiguous()
             self._call("mtb200_embedding_bwd_scan", dweight.data_ptr(), ids.data_ptr(), dx.data_ptr(), ids.shape[0], dweight.shape[1],
                        dweight.shape[0], self.status.data_ptr(), self._st())
             return

@@ -1492,3 +1492,14 @@ def test_router_gradient_of_another_type(ops):
         with pytest.raises(RuntimeError):
             M.moe_backward(ops, cfg, p, g, st, n2, dout)
     ops.check_status()
+
+
+@pytest.mark.parametrize("T", [40, 8193])
+def test_embedding_gradient_of_strided_ids(ops, T):
+    torch.manual_seed(T)
+    ids, dx = torch.randint(0, 50, (T, 2), device="cuda"), bf(T, 64)
+    got, want = torch.zeros(50, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(50, 64, dtype=torch.bfloat16, device="cuda")
+    ops.embedding_bwd(got, ids[:, 0], dx)
+    ops.embedding_bwd(want, ids[:, 0].contiguous(), dx)
+    assert torch.equal(got, want)
+    ops.check_status()

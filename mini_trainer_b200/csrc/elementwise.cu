@@ -1103,6 +1103,7 @@ __global__ void __launch_bounds__(EW_THREADS) adamw_groups_kernel(const __grid_c
     c = c > 1.f ? 1.f : c;   // a norm that is not a number stays one
   }
   if (norm_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) norm_out[0] = norm;
+  if (t.groups == 0) return;   // one block, for the norm
   const OptGroup& g = t.g[opt_group(t)];
   const long long i = (static_cast<long long>(blockIdx.x - g.first_block) * blockDim.x + threadIdx.x) * 4;
   if (i < g.n) adamw4(g.master, static_cast<StateT*>(g.m), static_cast<StateT*>(g.v), g.grad, g.param, i, c, p);
@@ -1550,13 +1551,14 @@ int mtb200_adamw_groups(const long long* table, int groups, int state_is_f32, co
   const float inv_bc1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
   const float inv_sqrt_bc2 = 1.f / sqrtf(1.f - powf(beta2, static_cast<float>(step)));
   const AdamwParams p{lr, beta1, beta2, eps, wd, inv_bc1, inv_sqrt_bc2};
-  for (int first = 0; first < groups; first += OPT_GROUPS) {
+  for (int first = 0; first == 0 || first < groups; first += OPT_GROUPS) {
     OptTable t;
     long long blocks = 0;
     const int k = groups - first < OPT_GROUPS ? groups - first : OPT_GROUPS;
     const int rc = fill_table(t, table + first * 6, k, 4, 0, &blocks);
     if (rc) return rc;
-    if (blocks == 0) continue;
+    if (blocks == 0 && first > 0) continue;
+    if (blocks == 0) blocks = 1;   // the first launch leaves the norm, whatever its groups hold
     float* out = first == 0 ? norm_out : nullptr;
     if (state_is_f32) launch_pdl(adamw_groups_kernel<float>, static_cast<unsigned>(blocks), EW_THREADS, 0, st, t, p, sumsq, max_norm, out);
     else launch_pdl(adamw_groups_kernel<bf16>, static_cast<unsigned>(blocks), EW_THREADS, 0, st, t, p, sumsq, max_norm, out);

@@ -1503,3 +1503,18 @@ def test_embedding_gradient_of_strided_ids(ops, T):
     ops.embedding_bwd(want, ids[:, 0].contiguous(), dx)
     assert torch.equal(got, want)
     ops.check_status()
+
+
+@pytest.mark.parametrize("fp32", [True, False])
+def test_optimizer_over_groups_without_elements(ops, fp32):
+    """The norm is written whatever the groups of the first launch hold."""
+    sd = torch.float32 if fp32 else torch.bfloat16
+    kinds = (torch.float32, sd, sd, torch.float32, torch.bfloat16)
+    empty, full = (tuple(torch.ones(n, dtype=d, device="cuda") for d in kinds) for n in (0, 8))
+    for groups in ([empty] * 48 + [full], [empty], [empty] * 49, []):
+        poison = [torch.full((), float("nan"), device="cuda") for _ in range(8)]
+        del poison
+        sq = torch.full((1,), 9.0, device="cuda")
+        table = ops.group_table(groups)
+        ops.add_sumsq_groups(table, sq)
+        assert torch.equal(ops.adamw_groups(table, fp32, sq, 1.0, 1e-3, 0.9, 0.95, 1e-8, 0.0, 1), sq.sqrt().squeeze(0))

@@ -16,6 +16,7 @@ summed in fp32 in slot order, so forward and backward are deterministic (no atom
 """
 from __future__ import annotations
 
+import contextvars
 from dataclasses import dataclass
 from typing import Optional
 
@@ -38,15 +39,29 @@ class MoeState:
     slabs: Optional[object] = None         # grouped path: the expert slabs; order, tok and bounds are None then
 
 
+# Backend of the layer that this thread is routing. Not an argument of ``route``: comparisons put their own function of (cfg, weight, rows) in its place.
+_layer_ops = contextvars.ContextVar("layer_ops", default=None)
+
+
+def _route(ops, cfg, router_w: torch.Tensor, n2: torch.Tensor):
+    """``route`` of a layer on ``ops``."""
+    token = _layer_ops.set(ops)
+    try:
+        return route(cfg, router_w, n2)
+    finally:
+        _layer_ops.reset(token)
+
+
 def route(cfg, router_w: torch.Tensor, n2: torch.Tensor, topi: Optional[torch.Tensor] = None):
     """Router of one block: ``(probs, topi, w)``. With ``topi`` given, those experts
     are used instead of the top-k while the weights still follow this call's logits (comparisons
-    between backends of different precision, where a near-tie may otherwise select differently)."""
+    between backends of different precision, where a near-tie may otherwise select differently).
+    In a layer whose backend has a kernel for it (``route_topk``) that one runs; else differentiable tensor operations."""
     k = cfg.num_experts_per_tok
     logits = n2 @ router_w.t()
-    if topi is None and logits.is_cuda:
-        from ..ops.native import route_topk
-        done = route_topk(logits, k, cfg.norm_topk_prob)
+    ops = _layer_ops.get()
+    if topi is None and hasattr(ops, "route_topk"):
+        done = ops.route_topk(logits, k, cfg.norm_topk_prob)
         if done is not None:
             return done
     probs = torch.softmax(logits.float(), dim=-1)
@@ -91,7 +106,7 @@ def moe_forward(ops, cfg, p: dict, n2: torch.Tensor, h1: torch.Tensor, need_out:
     (a recompute inside backward stops after the gate/up projections)."""
     T, H = n2.shape
     k, fe = cfg.num_experts_per_tok, cfg.expert_intermediate_size
-    probs, topi, w = route(cfg, p["router"], n2)
+    probs, topi, w = _route(ops, cfg, p["router"], n2)
     stacks = _expert_stacks(ops, cfg, p, n2)
     if stacks is not None:
         return _grouped_forward(ops, cfg, p, n2, h1, need_out, keep_act, probs, topi, w, *stacks)

@@ -127,7 +127,13 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def route_topk(logits, k: int, renorm: bool):
+def _launch(name, *args):
+    rc = getattr(_LIB, name)(*args)
+    if rc != 0:
+        raise RuntimeError(f"{name} failed with code {rc}")
+
+
+def route_topk(logits, k: int, renorm: bool, call=_launch):
     """``(probs, topi, w)`` of a router's logits ``[T, E]``: fp32 softmax, the ``k`` largest of each row and their weights. ``None`` for what the
     kernel does not take (other types and devices, more than 256 experts or 32 chosen ones), and while no ``NativeOps`` has been made."""
     T, E = logits.shape
@@ -136,10 +142,7 @@ def route_topk(logits, k: int, renorm: bool):
     probs = torch.empty(T, E, dtype=torch.float32, device=logits.device)
     topi = torch.empty(T, k, dtype=torch.int64, device=logits.device)
     w = torch.empty(T, k, dtype=torch.float32, device=logits.device)
-    rc = _LIB.mtb200_moe_route(logits.data_ptr(), T, E, k, int(renorm), probs.data_ptr(), topi.data_ptr(), w.data_ptr(),
-                                         _raw_stream(logits.device.index))
-    if rc != 0:
-        raise RuntimeError(f"mtb200_moe_route failed with code {rc}")
+    call("mtb200_moe_route", logits.data_ptr(), T, E, k, int(renorm), probs.data_ptr(), topi.data_ptr(), w.data_ptr(), _raw_stream(logits.device.index))
     return probs, topi, w
 
 
@@ -703,6 +706,10 @@ class NativeOps:
         self._call("mtb200_moe_combine", rows.data_ptr(), sl.row_of.data_ptr(), _ptr(w), _ptr(add), base.contiguous().data_ptr(), float(scale), T,
                    sl.k, H, out.data_ptr(), self._st())
         return out
+
+    def route_topk(self, logits, k: int, renorm: bool):
+        """``(probs, topi, w)`` of router logits in one launch, or ``None``: see ``route_topk`` above."""
+        return route_topk(logits, k, renorm, self._call)
 
     def route_bwd(self, probs, topi, w, dw, renorm: bool, dtype):
         """Gradient of the router logits ``[T, E]``."""

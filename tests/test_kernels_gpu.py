@@ -1518,3 +1518,27 @@ def test_optimizer_over_groups_without_elements(ops, fp32):
         table = ops.group_table(groups)
         ops.add_sumsq_groups(table, sq)
         assert torch.equal(ops.adamw_groups(table, fp32, sq, 1.0, 1e-3, 0.9, 0.95, 1e-8, 0.0, 1), sq.sqrt().squeeze(0))
+
+
+def test_router_kernel_belongs_to_the_native_backend(ops, monkeypatch):
+    """It is launched, and counted, for a layer on that backend only; the plain call stays a chain of differentiable tensor operations."""
+    from mini_trainer_b200.models import moe as M
+    from mini_trainer_b200.ops import native
+    cfg, p, _, n2, h1, _ = _moe_layer(70, 64, 40, 4, 2, 4)
+    calls, real = [], ops.lib.mtb200_moe_route
+
+    class Lib:
+        def __getattr__(self, name):
+            return getattr(ops.lib, name) if name != "mtb200_moe_route" else lambda *a: calls.append("not counted") or real(*a)
+    monkeypatch.setattr(native, "_LIB", Lib())
+    monkeypatch.setitem(ops._fn, "mtb200_moe_route", lambda *a: calls.append("counted") or real(*a))
+    w = p["router"].clone().requires_grad_()
+    wt = M.route(cfg, w, n2)[2]
+    assert not calls and wt.requires_grad
+    wt.sum().backward()
+    assert w.grad is not None
+    M.moe_forward(TorchOps(), cfg, p, n2, h1, True, False)
+    assert not calls
+    before = ops.launches
+    M.moe_forward(ops, cfg, p, n2, h1, False, False)   # router, slabs, gather, gate/up
+    assert calls == ["counted"] and ops.launches == before + 4

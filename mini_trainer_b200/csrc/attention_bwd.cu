@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
 #include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 

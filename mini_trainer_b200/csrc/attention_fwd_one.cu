@@ -39,6 +39,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
 #include "ptx.cuh"
 
 namespace mtb {

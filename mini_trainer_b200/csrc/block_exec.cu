@@ -9,39 +9,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
+
 extern "C" {
 
 typedef unsigned long long u64;
-int mtb200_gemm_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
-                     float, int, u64*, u64, float*, long long, float2*, int*, cudaStream_t);
-int mtb200_gemm2_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
-                      float, int, u64*, u64, float*, long long, float2*, int*, cudaStream_t);
-int mtb200_gemm_act(const void*, long long, const void*, void*, void*, const void*, int, int, int, int, int, int, int*, cudaStream_t);
-int mtb200_swiglu_fwd(const void*, void*, long long, int, cudaStream_t);
-int mtb200_geglu_fwd(const void*, void*, long long, int, cudaStream_t);
-int mtb200_gelu_fwd(const void*, void*, long long, cudaStream_t);
-int mtb200_swiglu_bwd(const void*, const void*, void*, long long, int, cudaStream_t);
-int mtb200_swiglu_bwd_act(void*, const void*, void*, long long, int, cudaStream_t);
-int mtb200_geglu_bwd(const void*, const void*, void*, long long, int, cudaStream_t);
-int mtb200_geglu_bwd_act(void*, const void*, void*, long long, int, cudaStream_t);
-int mtb200_gelu_bwd(const void*, const void*, void*, long long, cudaStream_t);
-int mtb200_gelu_bwd_act(void*, const void*, void*, long long, cudaStream_t);
-int mtb200_rmsnorm_fwd(const void*, const void*, void*, float*, float, int, int, int*, cudaStream_t);
-int mtb200_layernorm_fwd(const void*, const void*, const void*, void*, float*, float*, float, int, int, int*, cudaStream_t);
-int mtb200_norm_bwd_blocks(int, int);
-int mtb200_rmsnorm_bwd(const void*, const void*, const float*, const void*, const void*, void*, float*, void*, int, int, int*, cudaStream_t);
-int mtb200_layernorm_bwd(const void*, const void*, const float*, const float*, const void*, const void*, void*, float*, void*, void*, int, int, int*,
-                         cudaStream_t);
-int mtb200_rope(void*, const int*, const float*, int, long long, int, int, int, cudaStream_t);
-int mtb200_head_rmsnorm_fwd(void*, const void*, const void*, void*, float*, const int*, const float*, float, int, long long, int, int, int, cudaStream_t);
-int mtb200_head_rmsnorm_bwd_blocks(int, int);
-int mtb200_head_rmsnorm_bwd(void*, const void*, const float*, const void*, const void*, float*, void*, void*, const int*, const float*, int, long long,
-                            long long, int, int, int, cudaStream_t);
-int mtb200_attn_fwd(const void*, long long, void*, long long, float*, const int*, int, int, int, int, int, int, float, int*, cudaStream_t);
-int mtb200_attn_fwd_one(const void*, long long, void*, long long, float*, const int*, int, int, int, int, int, float, int*, cudaStream_t);
-int mtb200_attn_bwd(const void*, long long, const void*, long long, const void*, long long, void*, long long, const float*, float*, float*, const int*, int,
-                    int, int, int, int, int, u64*, u64, float*, long long, float, int*, cudaStream_t);
-int mtb200_colsum(const void*, long long, void*, float*, int, int, cudaStream_t);
 
 // Products of a block, in the order of the plan: forward qkv, o, gate/up, down; backward the input gradients and the weight gradients.
 enum { G_QKV, G_O, G_GU, G_DOWN, D_DOWN, D_GU, D_O, D_QKV, W_DOWN, W_GU, W_O, W_QKV, GEMMS };
@@ -204,6 +176,10 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
 
 extern "C" {
 
+// Sizes of the structures, for a caller that lays them out itself (ops/block_exec.py).
+void mtb200_block_sizes(int* out) {
+  out[0] = sizeof(BlockSpec); out[1] = sizeof(BlockParams); out[2] = sizeof(BlockIO);
+}
 // Bytes of io->ws for a call with these arguments (backward: with gradients).
 long long mtb200_block_workspace(const BlockSpec* s, const BlockIO* io, int bwd) {
   const BlockParams none{};

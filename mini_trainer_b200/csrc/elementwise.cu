@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
 #include "ptx.cuh"
 
 namespace mtb {

@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "entries.h"
 #include "gather.cuh"
 #include "gemm_act.cuh"
 #include "gemm_epilogue.cuh"

@@ -27,6 +27,7 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "entries.h"
 #include "gather.cuh"
 #include "gemm_act.cuh"
 #include "gemm_epilogue.cuh"

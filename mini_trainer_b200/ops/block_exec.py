@@ -36,6 +36,14 @@ class IO(ctypes.Structure):
         + [("part_bytes", c_longlong), ("status", c_void_p)]
 
 
+def check_layout(lib) -> None:
+    """The structures are laid out here and in ``csrc/block_exec.cu``."""
+    sizes = (c_int * 3)()
+    lib.mtb200_block_sizes(sizes)
+    if list(sizes) != [ctypes.sizeof(t) for t in (Spec, Params, IO)]:
+        raise RuntimeError(f"the library lays its block structures out in {list(sizes)} bytes: it is of another version, build it again")
+
+
 def _ptr(t):
     return None if t is None else t.data_ptr()
 

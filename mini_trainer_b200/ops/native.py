@@ -41,6 +41,7 @@ def load_library():
             fn.restype = c_int
             fn.argtypes = getattr(_Sig, name)
     lib.mtb200_block_workspace.restype = c_longlong
+    block_exec.check_layout(lib)
     _LIB = lib
     return lib
 

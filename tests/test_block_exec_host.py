@@ -112,3 +112,18 @@ def test_workspace_is_what_the_call_lays_out(lib, keep, layernorm):
     queue(lib, s, io, 1)
     end = ctypes.c_void_p.in_dll(lib, "last_rstd").value - WS + 321 * 4   # the second of two rows
     assert size == -(-end // 256) * 256
+
+
+def test_structures_have_the_layout_of_the_library(lib, monkeypatch):
+    B.check_layout(lib)
+    s, io = make(T=321)   # and the sizes it reads give the workspace they should
+    per_token = 2 * (768 + 384 + 4 * 256) + 4 * 4 + 4 * 256 + 8   # dgu, dact, dn, n2, dh1, dattn; delta; dq; statistics
+    rows, cols = 148 * 256 * 4, 32 * 768 * 4
+    size = lib.mtb200_block_workspace(ctypes.byref(s), ctypes.byref(io), 1)
+    assert 0 <= size - (321 * per_token + rows + cols) < 16 * 256
+
+    class Short(ctypes.Structure):
+        _fields_ = B.Spec._fields_[:-1]
+    monkeypatch.setattr(B, "Spec", Short)
+    with pytest.raises(RuntimeError, match="another version"):
+        B.check_layout(lib)

@@ -1,8 +1,8 @@
 // One decoder block, forward or backward, queued by one call: the host side of models/decoder.py's dense pre-norm block for a rank that
 // holds its parameters whole. The kernels, their order and their results are those of the Python form; what goes is the interpreter
 // between the launches (5 to 8 us per launch next to the 2 to 3 us of the launch itself), which is what a step of a small model and
-// a block on a short minibatch are bound by. Training step of 640 tokens through 2 layers 1377 -> 1034 us, of 4096 tokens 1525 -> 1157 (with the
-// batch in one copy and cheaper views).
+// a block on a short minibatch are bound by. Training step of 640 tokens through 2 layers 1207 -> 978 us, of 4096 tokens 1355 -> 1088; a block of
+// 5987 tokens x 1536, which the device bounds, 1798 either way.
 //
 // Memory comes from the caller: what outlives the call as tensors of their own, the rest as one workspace laid out here
 // (mtb200_block_workspace says how large), so nothing is allocated and nothing is kept between calls.

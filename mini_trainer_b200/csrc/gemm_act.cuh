@@ -3,9 +3,11 @@
 //   ACT_GLU    pre = A * [Wg; Wu]^T, act = f(g) * u. A tile's 256 columns are 128 of the gate and the same 128 of up, so that one thread has both.
 //   ACT_PLAIN  pre = A * B (+ bias), act = f(pre): an MLP without a gate
 // Eight warps, two per 32-row quarter: with four (one per scheduler) the arithmetic of a tile took longer than short reductions. They work on
-// 32 columns at a time, staged as boxes of 32 rows x 64 bytes (64B-swizzled). Bound by the product. With its activation, on a B200:
+// 32 columns at a time, staged as boxes of 32 rows x 64 bytes (64B-swizzled). Bound by the product. With its activation, in a loop of its own on a B200:
 // 5987 x 17920 x 1536 272 -> 231 us (product alone 220), 4099 x 12288 x 2048 167 -> 153, 16384 x 28672 x 4096 3.16 -> 2.8 ms, 7001 x 12288 x 3072 without
-// a gate 448 -> 375 us; over the slabs of 64 experts (20 500 rows x 2048 x 2048) 150 + 24 -> 153, of 8 (9200 x 28672 x 4096) 1378 + 117 -> 1434; whole blocks of those sizes 1836 -> 1793, 1712 -> 1703, 20.05 -> 19.91 ms and 4240 -> 4126 us.
+// a gate 448 -> 375 us; over the slabs of 64 experts (20 500 rows x 2048 x 2048) 150 + 24 -> 153, of 8 (9200 x 28672 x 4096) 1378 + 117 -> 1434.
+// Forward and backward of whole layers, without and with it in one process: 1.5B block 1830 -> 1796 us, q/k-norm block 1700 -> 1680, 64 experts 1042 -> 1024,
+// 8 experts 7985 -> 7897; an 8B block (20.0 ms) and a LayerNorm block (4.2 ms) by less than their runs differ.
 //
 // The other direction, the activation's gradient in the epilogue of the product in front of it, was tried with the pre-activations loaded
 // by TMA two boxes ahead and either form of stores. It gained up to a fifth alone (5987 x 8960 x 1536 243 -> 190 us) and nothing in a

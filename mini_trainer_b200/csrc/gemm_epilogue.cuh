@@ -223,8 +223,8 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
 
 // Products of at most this many operations start under their predecessor's tail (launch_pdl). It saves about 2 us per launch whatever the
 // size; on the other hand CTAs that are placed as SMs fall free, instead of in order, take neighbouring tiles to distant SMs, and
-// long launches lose what that saves (with every product launched early: 1.5B block 1933 -> 1868 us, q/k-norm block 1786 -> 1723;
-// but 8B block 20.31 -> 20.42 ms, eight-expert layer 8.35 -> 8.56 ms, sixty-four experts 1140 -> 1148 us).
+// long launches lose what that saves (this rule and every product early, in one process: 1.5B, q/k-norm and LayerNorm blocks within 1 %, which is
+// their spread; 8B block 19.92 and 20.08 ms, LM head 4.66 and 4.73, eight-expert layer 7.88 and 8.13, sixty-four experts 1019 and 1040 us).
 constexpr double PDL_MAX_FLOPS = 1e12;
 // Grouped products, counted over the whole row buffers: 477 tokens through 4 experts of 2760 (0.01 TFLOP) 311 -> 301 us, 878 through 32 of 1080 (0.05) 350 -> 342;
 // 2051 through 64 of 1024 (0.2) is the slower early.

@@ -34,7 +34,7 @@ struct Vec8 {
 // Router of a layer, one warp per token: fp32 softmax of the logits, the k largest (the lower index of equal ones, the largest first) and their
 // weights, renormalised over the chosen ones when `renorm`. A lane holds experts lane, lane + 32, ... As tensor operations these were
 // six launches of 2 to 11 us and the gaps between them (2051 tokens, 64 experts, 8 chosen: 28 us and 10 of
-// gaps, now 6.6).
+// gaps, now 6.6; the layer's forward and backward 1053 -> 1019).
 __global__ void __launch_bounds__(MOE_THREADS) moe_route_kernel(const bf16* __restrict__ logits, int T, int E, int k, int renorm, float* __restrict__ probs,
                                                                long long* __restrict__ topi, float* __restrict__ w) {
   pdl_trigger();
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const long long*
 }
 
 // out[row] = scale * src[pair_of[row] / k], zeros in padding. Rows past the last slab are left alone. A warp per row, eight vectors of it
-// in flight per lane (a block of 128 threads per row had two; layer of 64 experts, three gathers of 20 500 rows of 2048: 1077 -> 1049 us; eight experts level:
+// in flight per lane (a block of 128 threads per row had two; layer of 64 experts, three gathers of 20 500 rows of 2048: 1047 -> 1019 us; eight experts level:
 // bound by writing the rows).
 constexpr int GATHER_WARPS = 4;
 __global__ void __launch_bounds__(32 * GATHER_WARPS) moe_gather_kernel(const bf16* __restrict__ src, const int* __restrict__ pair_of, const int* __restrict__ starts,
@@ -195,7 +195,7 @@ __device__ __forceinline__ void act_and_grad(float g, float& a, float& da) {
 //   gradient needs),  dw[pair] = du . (act(g) * u)
 // One pass over gate/up and du instead of the forward activation, two scalings, a dot product and the activation gradient as passes of their
 // own. TPR threads per row: a warp for narrow rows, whose reduction then needs no barrier (20 500 rows of 1024: 60 us with a block per row,
-// 40 with a warp), up to the whole block for wide ones (14 336: 221 us either way, the copy bandwidth).
+// 40 with a warp; the layer of 64 experts 1042 -> 1019), up to the whole block for wide ones (14 336: 221 us either way, the copy bandwidth).
 template <int ACT, int TPR>
 __global__ void __launch_bounds__(MOE_THREADS) moe_glu_bwd_kernel(bf16* __restrict__ du, const bf16* __restrict__ gu, const float* __restrict__ w,
                                                                  const int* __restrict__ pair_of, const int* __restrict__ starts, int E, int cap, int F,
@@ -340,7 +340,7 @@ int mtb200_moe_glu_bwd(void* du, const void* gu, const float* w, const int* pair
                        void* dgu, float* dw, cudaStream_t st) {
   if (cap <= 0) return 0;
   if (F % 8) return -10;
-  // a thread of a row gets two vectors at least, and a row 256 threads at most
+  // a row of at most 2048 elements (eight vectors a lane) is a warp's, which needs no barrier; a thread of a wider one gets at least two vectors
 #define GB(ACT, TPR) launch_pdl(moe_glu_bwd_kernel<ACT, TPR>, (cap + MOE_THREADS / TPR - 1) / (MOE_THREADS / TPR), MOE_THREADS, 0, st, (bf16*)du, (const bf16*)gu, w, pair_of, starts, E, cap, F, (bf16*)dgu, dw)
 #define GBT(ACT) if (F <= 2048) GB(ACT, 32); else if (F <= 4096) GB(ACT, 128); else GB(ACT, 256)
   if (act == 0) { GBT(0); } else { GBT(1); }

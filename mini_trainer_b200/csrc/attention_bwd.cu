@@ -80,8 +80,6 @@ struct AttBwdParams {
   int* status;
 };
 
-template <int R> __device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
-template <int R> __device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
 template <int D>
 __global__ void __launch_bounds__(AB_THREADS, 1)

@@ -22,7 +22,7 @@ struct BlockSpec {
   int T, H, F, Hq, Hkv, D;
   int gated, gelu, layernorm, qk_norm;
   float eps, scale, alpha;
-  int pair[GEMMS], splits[GEMMS];   // kernel and splits of each product (ops/gemm_plan.py)
+  int pair[GEMMS], splits[GEMMS];   // kernel (0: one CTA, 1: pairs, 2: pairs with wide tiles) and splits of each product (ops/gemm_plan.py)
   int need_out;                     // 0: the forward stops before the activation
   int attn_form;                    // 0: one query tile per CTA, 1: pairs of heads, 2: pairs of row blocks
   int fwd_items, bwd_items, bwd_splits;
@@ -66,7 +66,7 @@ int gemm(const BlockSpec& s, const BlockIO& io, const u64*& epoch, int which, co
          int K, const void* r, const void* bias, float alpha, cudaStream_t st) {
   const int splits = io.part != nullptr ? s.splits[which] : 1;
   auto f = s.pair[which] ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
-  return f(a, lda, a_mn, b, ldb, b_mn, d, N, 0, r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
+  return f(a, lda, a_mn, b, ldb, b_mn, d, N, s.pair[which] == 2 ? GEMM2_WIDE : 0, r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
            splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, nullptr, io.status, st);
 }
 

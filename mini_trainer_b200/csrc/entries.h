@@ -8,6 +8,9 @@ int mtb200_gemm_bf16(const void*, long long, int, const void*, long long, int, v
                      float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
 int mtb200_gemm2_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
                       float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
+enum { GEMM2_WIDE = 2 };   // added to out_f32: wide tiles
+int mtb200_gemm2_wide_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
+                           float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
 int mtb200_gemm_act(const void*, long long, const void*, void*, void*, const void*, int, int, int, int, int, int, int*, cudaStream_t);
 int mtb200_swiglu_fwd(const void*, void*, long long, int, cudaStream_t);
 int mtb200_geglu_fwd(const void*, void*, long long, int, cudaStream_t);

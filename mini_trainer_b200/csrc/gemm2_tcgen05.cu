@@ -13,6 +13,15 @@
 // Only CTA 0's MMA thread issues tcgen05.mma; every wait is bounded as in the one-CTA kernel.
 // The two CTAs synchronise with barrier.cluster once after set-up and once before teardown.
 //
+// WIDE = true computes 256 x 512 tiles: a stage holds a pair's A once and two halves of B, and both 256-column accumulators belong to one tile, so
+// that a product of 256 x 512 x 64 moves 48 KB per SM where two 256 x 256 tiles move 64. What bounds a long product is the 1000 W cap, and operands that
+// travel from L2 (and, where the tiles in flight span more rows than L2 holds, from HBM again) cost as much of it as the multiplications' own smem
+// reads: 28672 x 4096 x 16384 as a weight gradient reads 7.4 GB of HBM in 256 x 256 tiles and 4.2 in wide ones, and in a loop at the cap gives
+// 1261 and 1360 TFLOP/s (single CTAs 1257, the library 1332); 16384 x 4096 x 28672 1239 and 1390 (1280, 1417), 16384 x 28672 x 4096 1376 and 1413 (1325, 1407).
+// With no second pair of accumulators the epilogue would stand between tiles. So the second half runs WIDE_LAG k-blocks behind the first at either end,
+// a warpgroup per half empties its accumulator into registers before it stores anything (epilogue_wide), and the first half's next tile starts
+// while the second's is emptied. What is left of the gap is about 2500 clocks, which short reductions show (5987 x 17920 x 1536: 263 us in 256 x 256 tiles, 281 wide).
+//
 // GATHER = true is the fused all-gather variant (see gather.cuh): both CTAs of a pair carry eight
 // gather warps and a flag checker; each CTA's checker watches the chunks under ITS half of the B
 // tile (128 weight rows, one contiguous byte range) and only that CTA's producer waits for them.
@@ -32,6 +41,7 @@ namespace mtb {
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer);
+int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32);
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32);
 
 namespace g2 {
@@ -44,6 +54,15 @@ constexpr int STAGES = 6;
 constexpr int A_BYTES = BM * BK * 2;     // 16 KB
 constexpr int B_BYTES = BNH * BK * 2;    // 16 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int WIDE_STAGES = 4;                        // wide tiles: a second half of B in every stage
+constexpr int WIDE_STAGE_BYTES = A_BYTES + 2 * B_BYTES;
+constexpr int WIDE_LAG = 2;                           // k-blocks by which the second half of a wide tile runs behind the first at its ends
+constexpr int WIDE_GROUP_M = 14;                      // row-tiles per band, about: the 74 tiles in flight then read 3600 rows of A and 2700 of B
+// Three warpgroups: {TMA, MMA}, and the epilogue of either half, whose threads hold 256 columns as 128 registers and the piece at work on.
+constexpr int WIDE_THREADS = 384;
+constexpr int WIDE_REGS = 168, WIDE_REGS_IO = 40, WIDE_REGS_EPI = 232;   // per thread at launch, and after the split
+static_assert(WIDE_REGS_IO + 2 * WIDE_REGS_EPI == 3 * WIDE_REGS && 3 * 128 * WIDE_REGS <= 65536, "register split");
+static_assert(WIDE_STAGES * WIDE_STAGE_BYTES == STAGES * STAGE_BYTES, "one shared-memory size");
 constexpr int THREADS = 192;
 constexpr int GROUP_M = 8;               // band of 8 pair-tiles = 2048 rows
 constexpr int GATHER_GROUP_N = 4;        // column-tiles per band in the all-gather variant
@@ -54,11 +73,13 @@ struct Params {
   int M, N, K;
   int* status;
   int num_pairs;
+  int group_m;      // wide tiles: row-tiles per band
+  int whole;        // wide tiles: items that are whole tiles, the rest of the tiles go as two halves each
   EpiParams e;
   ActParams act;   // ACT instances
 };
 
-constexpr int threads_of(int act) { return act == ACT_NONE ? THREADS : 64 + 32 * ACT_WARPS; }
+constexpr int threads_of(int act, bool wide) { return wide ? WIDE_THREADS : act == ACT_NONE ? THREADS : 64 + 32 * ACT_WARPS; }
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -92,8 +113,8 @@ __device__ __forceinline__ void mbar_arrive_cta0(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & PEER_MASK) : "memory");
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT), 1)
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE, bool WIDE = false>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT, WIDE), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ ActMaps<ACT> maps, Params p,
              const __grid_constant__ GatherParams g) {
@@ -115,11 +136,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const int num_tiles = tiles_m * tiles_n;
   const int kblocks = (p.K + BK - 1) / BK;
   const int splits = GATHER ? 1 : p.e.splits;
-  const int num_items = num_tiles * splits;   // item = split * num_tiles + tile: neighbours share operand tiles
+  const int wide_n = (p.N + 2 * BN - 1) / (2 * BN);
+  const int num_items = WIDE ? tiles_m * wide_n * splits + (tiles_m * wide_n - p.whole) : num_tiles * splits;   // item = split * num_tiles + tile: neighbours share operand tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], ACT ? 2 * ACT_WARPS : 8); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], ACT && !WIDE ? 2 * ACT_WARPS : 8); }
     *abort_flag = 0;
     *verified = 0;
     fence_mbar_init();
@@ -152,15 +174,155 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       tm = local / cols;
       return;
     }
-    const int band = t / (GROUP_M * tiles_n);
-    const int first_m = band * GROUP_M;
-    const int rows = min(GROUP_M, tiles_m - first_m);
-    const int local = t - band * GROUP_M * tiles_n;
+    const int band = t / (p.group_m * tiles_n);
+    const int first_m = band * p.group_m;
+    const int rows = min(p.group_m, tiles_m - first_m);
+    const int local = t - band * p.group_m * tiles_n;
     tm = first_m + local % rows;
     tn = local / rows;
   };
 
-  if (warp == 0) {
+  // Wide tiles: row-tile, first column and number of 256-column halves (0: a half tile past the last column) of an item.
+  auto wide_coords = [&](int w, int& tm, int& col0, int& halves, int& kb0, int& kb1) {
+    const int all = tiles_m * wide_n;
+    k_range(splits > 1 ? w / all : 0, kb0, kb1);
+    if (splits > 1) w %= all;
+    const int t = w < p.whole ? w : p.whole + (w - p.whole) / 2;
+    const int band = t / (p.group_m * wide_n);
+    const int first_m = band * p.group_m;
+    const int rows = min(p.group_m, tiles_m - first_m);
+    const int local = t - band * p.group_m * wide_n;
+    tm = first_m + local % rows;
+    col0 = local / rows * 2 * BN;
+    if (w < p.whole) {
+      halves = col0 + BN < p.N ? 2 : 1;
+    } else {
+      col0 += ((w - p.whole) & 1) * BN;
+      halves = col0 < p.N ? 1 : 0;
+    }
+  };
+
+  if (WIDE && warp < 4) setmaxnreg_dec<WIDE_REGS_IO>();
+  if (WIDE && warp == 0) {
+    // ------------------------------------------------------------------ wide tiles: TMA producer (both CTAs)
+    if (elect_one()) {
+      uint32_t it = 0;
+      for (int w = pair; w < num_items; w += p.num_pairs) {
+        int tm, col0, halves, kb0, kb1;
+        wide_coords(w, tm, col0, halves, kb0, kb1);
+        if (halves == 0) continue;
+        const int row0 = tm * 2 * BM + rank * BM;
+        // this CTA's part of each half of B: 128 of its columns; with a gated activation CTA 0 has the gate's weight and CTA 1 up's
+        const int b0 = ACT == ACT_GLU ? col0 / 2 + static_cast<int>(rank) * p.act.F : col0 + rank * BNH;
+        constexpr int b_step = ACT == ACT_GLU ? BNH : BN;
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % WIDE_STAGES;
+          const uint32_t ph = (it / WIDE_STAGES) & 1;
+          if (!mbar_wait(&empty_bar[s], ph ^ 1, abort_flag)) { atomicExch(p.status, 51); goto done; }
+          uint8_t* sa = smem + s * WIDE_STAGE_BYTES;
+          const uint32_t fb = smem_u32(&full_bar[s]) & PEER_MASK;   // CTA 0's barrier
+          if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * (A_BYTES + halves * B_BYTES));
+          if (A_MN) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tmap_a, fb, row0 + j * 64, kb * BK);
+          } else {
+            tma_load_2d_pair(sa, &tmap_a, fb, kb * BK, row0);
+          }
+          for (int h = 0; h < halves; ++h) {
+            uint8_t* sb = sa + A_BYTES + h * B_BYTES;
+            if (B_MN) {
+#pragma unroll
+              for (int j = 0; j < BNH / 64; ++j) tma_load_2d_pair(sb + j * 8192, &tmap_b, fb, b0 + h * b_step + j * 64, kb * BK);
+            } else {
+              tma_load_2d_pair(sb, &tmap_b, fb, kb * BK, b0 + h * b_step);
+            }
+          }
+        }
+      }
+      pdl_trigger();
+    }
+  } else if (WIDE && warp == 1) {
+    // ------------------------------------------------------------------ wide tiles: MMA issuer (leader CTA only)
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
+      uint32_t it = 0, used0 = 0, used1 = 0;   // stages so far; tiles that used each accumulator
+      for (int w = pair; w < num_items; w += p.num_pairs) {
+        int tm, col0, halves, kb0, kb1;
+        wide_coords(w, tm, col0, halves, kb0, kb1);
+        if (halves == 0) continue;
+        auto filled = [&](int j) { return mbar_wait(&full_bar[(it + j) % WIDE_STAGES], ((it + j) / WIDE_STAGES) & 1, abort_flag); };
+        auto multiply = [&](int j, int h) {
+          const uint32_t sa = smem_u32(smem + (it + j) % WIDE_STAGES * WIDE_STAGE_BYTES);
+          const uint32_t sb = sa + A_BYTES + h * B_BYTES;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t da = A_MN ? make_smem_desc(sa + k * 2048, 8192, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
+            const uint64_t db = B_MN ? make_smem_desc(sb + k * 2048, 8192, 1024) : make_smem_desc(sb + k * 32, 16, 1024);
+            umma2_bf16(tmem_base + h * BN, da, db, idesc, j != 0 || k != 0);
+          }
+        };
+        auto release = [&](int j) { umma2_commit_pair(&empty_bar[(it + j) % WIDE_STAGES]); };
+        if (!mbar_wait(&tempty_bar[0], (used0 & 1) ^ 1, abort_flag)) { atomicExch(p.status, 52); goto done; }
+        ++used0;
+        tc_fence_after();
+        const int n = kb1 - kb0;
+        const int lag = halves == 2 ? min(WIDE_LAG, n / 2) : 0;
+        for (int j = 0; j < lag; ++j) {
+          if (!filled(j)) { atomicExch(p.status, 53); goto done; }
+          tc_fence_after();
+          multiply(j, 0);
+        }
+        if (halves == 2) {
+          if (!mbar_wait(&tempty_bar[1], (used1 & 1) ^ 1, abort_flag)) { atomicExch(p.status, 52); goto done; }
+          ++used1;
+          tc_fence_after();
+          for (int j = 0; j < lag; ++j) { multiply(j, 1); release(j); }
+        }
+        for (int j = lag; j < n - lag; ++j) {
+          if (!filled(j)) { atomicExch(p.status, 53); goto done; }
+          tc_fence_after();
+          multiply(j, 0);
+          if (halves == 2) multiply(j, 1);
+          release(j);
+        }
+        for (int j = n - lag; j < n; ++j) {
+          if (!filled(j)) { atomicExch(p.status, 53); goto done; }
+          tc_fence_after();
+          multiply(j, 0);
+        }
+        umma2_commit_pair(&tfull_bar[0]);
+        for (int j = n - lag; j < n; ++j) { multiply(j, 1); release(j); }
+        if (halves == 2) umma2_commit_pair(&tfull_bar[1]);
+        it += n;
+      }
+    }
+  } else if (WIDE && warp >= 4) {
+    // ------------------------------------------------------------------ wide tiles: epilogue (both CTAs; warps 4..7 half 0, 8..11 half 1)
+    setmaxnreg_inc<WIDE_REGS_EPI>();
+    const int q = warp & 3, h = (warp - 4) >> 2;
+    EpiOut out{&tmap_d, smem + WIDE_STAGES * WIDE_STAGE_BYTES + (warp - 4) * 2 * ACT_BOX, -1, 0};
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * BN;
+    uint32_t used = 0;
+    for (int w = pair; w < num_items; w += p.num_pairs) {
+      int tm, col0, halves, kb0, kb1;
+      wide_coords(w, tm, col0, halves, kb0, kb1);
+      if (h >= halves) continue;
+      if (!mbar_wait(&tfull_bar[h], used & 1, abort_flag)) { atomicExch(p.status, 54); goto done; }
+      ++used;
+      tc_fence_after();
+      const int row0 = tm * 2 * BM + rank * BM;
+      auto drained = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cta0(&tempty_bar[h]);
+      };
+      if constexpr (ACT != ACT_NONE) epilogue_act_wide<ACT>(p.e, p.act, maps, out, taddr, row0, col0 / BN + h, q, lane, drained);
+      else epilogue_wide<OUT_F32, STATS, EXTRA>(p.e, out, taddr, row0, col0 + h * BN, q, lane, 2 * (tm * tiles_n + col0 / BN + h) + static_cast<int>(rank),
+                                                splits > 1 ? w / (tiles_m * wide_n) : 0, drained);
+    }
+  } else if (WIDE) {
+    // warps 2 and 3 have no part
+  } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (elect_one()) {
       uint32_t it = 0, tl = 0;
@@ -283,7 +445,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     }
   }
 done:
-  if (warp >= 2 && (ACT || warp < 6) && lane == 0) drain_boxes();
+  if (warp >= 2 && (ACT || WIDE || warp < 6) && lane == 0) drain_boxes();
   tc_fence_before();
   __syncthreads();
   cluster_sync();          // nobody tears down while the partner may still signal or read
@@ -317,11 +479,11 @@ static int co_resident_pairs() {
   return pairs;
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE, bool WIDE = false>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
                   long long part_bytes = 0, const ActMaps<ACT>& maps = ActMaps<ACT>{}) {
-  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA, ACT>;
-  constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT);
+  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA, ACT, WIDE>;
+  constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT, WIDE);
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -4;
@@ -332,7 +494,16 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + BN - 1) / BN);
   if (p.e.splits > 1 && !split_fits(p.e, 2 * tiles, (p.K + BK - 1) / BK, part_bytes)) return -11;
   // the gathering variant always uses every pair: its extra warps carry the transfer
-  const int items = tiles * p.e.splits;
+  int items = tiles * p.e.splits;
+  p.group_m = GROUP_M;
+  if constexpr (WIDE) {
+    const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), wide = tiles_m * ((p.N + 2 * BN - 1) / (2 * BN)), rest = wide % pairs;
+    const int bands = max(1, (tiles_m + WIDE_GROUP_M / 2) / WIDE_GROUP_M);
+    p.group_m = (tiles_m + bands - 1) / bands;
+    // a last round that half of the pairs have a tile for is given out as half tiles
+    p.whole = p.e.splits == 1 && 2 * rest <= pairs ? wide - rest : wide;
+    items = wide * p.e.splits + (wide - p.whole);
+  }
   p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
   static const GatherParams none{};
   if constexpr (GATHER) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, *gp);
@@ -351,34 +522,34 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
   if (rc) return rc - 10;
   rc = make_tmap_out(&td, D, M, N, ldd, 0);
   if (rc) return rc - 20;
-  Params p{M, N, K, status, 0, EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0}};
+  Params p{M, N, K, status, 0, 0, 0, EpiParams{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0}};
   return launch<false, false, false, true>(ta, tb, td, p, stream, &g);
 }
 
 // Products with an activation in the epilogue; called by mtb200_gemm_act.
-int launch_act(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
+int launch_act(int mode, bool wide, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
                int* status, cudaStream_t stream) {
-  const Params p{e.M, e.N, K, status, 0, e, a};
+  const Params p{e.M, e.N, K, status, 0, 0, 0, e, a};
+  const ActMaps<ACT_PLAIN> plain{m.gate, m.up, m.act};
+  if (wide) return mode == ACT_GLU ? launch<false, false, false, false, false, false, ACT_GLU, true>(ta, tb, m.gate, p, stream, nullptr, 0, m)
+                                   : launch<false, false, false, false, false, false, ACT_PLAIN, true>(ta, tb, m.gate, p, stream, nullptr, 0, plain);
   if (mode == ACT_GLU) return launch<false, false, false, false, false, false, ACT_GLU>(ta, tb, m.gate, p, stream, nullptr, 0, m);
-  return launch<false, false, false, false, false, false, ACT_PLAIN>(ta, tb, m.gate, p, stream, nullptr, 0, ActMaps<ACT_PLAIN>{m.gate, m.up, m.act});
+  return launch<false, false, false, false, false, false, ACT_PLAIN>(ta, tb, m.gate, p, stream, nullptr, 0, plain);
 }
 
-}  // namespace g2
-}  // namespace mtb
+template <bool A_MN, bool B_MN>
+static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, bool out_f32, long long part_bytes, cudaStream_t stream) {
+  if (out_f32) return launch<A_MN, B_MN, true, false, false, true, ACT_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+  if (p.e.R != nullptr || p.e.bias != nullptr) return launch<A_MN, B_MN, false, false, false, true, ACT_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+  return launch<A_MN, B_MN, false, false, false, false, ACT_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+}
 
-extern "C" {
-
-// Same contract as mtb200_gemm_bf16, computed by CTA pairs (256 x 256 tiles). Returns -6 when
-// clusters of two cannot be scheduled on this device (mtb200_gemm2_pairs() is 0); callers then use the one-CTA kernel.
-int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
-
-int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
-                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                      float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
-  using namespace mtb;
-  using namespace mtb::g2;
+static int gemm2(bool wide, const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D, long long ldd, int out_f32, const void* R,
+                 long long ldr, const void* bias, int M, int N, int K, float alpha, int splits, unsigned long long* counters, unsigned long long epoch,
+                 float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32) || splits < 1) return -10;
+  if (stats != nullptr && (a_mn || b_mn || R || bias)) wide = false;   // of the products with statistics only the plain forward one has wide tiles
   CUtensorMap ta, tb, td;
   int rc;
   if (a_mn) rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, 64);
@@ -387,9 +558,18 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BNH);
   if (rc) return rc - 10;
-  rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
+  rc = wide ? make_tmap_narrow(&td, D, N, M, ldd, out_f32) : make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
-  Params p{M, N, K, status, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, part, stats, counters, epoch}};
+  Params p{M, N, K, status, 0, 0, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, part, stats, counters, epoch}};
+  if (wide) {
+    if (stats != nullptr) return launch<false, false, false, false, true, false, ACT_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
+    switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
+      case 0: return launch_wide<false, false>(ta, tb, td, p, out_f32, part_bytes, stream);
+      case 1: return launch_wide<false, true>(ta, tb, td, p, out_f32, part_bytes, stream);
+      case 2: return launch_wide<true, false>(ta, tb, td, p, out_f32, part_bytes, stream);
+      default: return launch_wide<true, true>(ta, tb, td, p, out_f32, part_bytes, stream);
+    }
+  }
   if (stats != nullptr) {
     switch ((a_mn ? 2 : 0) | (b_mn ? 1 : 0)) {
       case 0: return launch<false, false, false, false, true>(ta, tb, td, p, stream, nullptr, part_bytes);
@@ -412,6 +592,29 @@ int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, lon
     default: GEMM2(true, true, true);
   }
 #undef GEMM2
+}
+
+}  // namespace g2
+}  // namespace mtb
+
+extern "C" {
+
+// Same contract as mtb200_gemm_bf16, computed by CTA pairs (256 x 256 tiles). Returns -6 when
+// clusters of two cannot be scheduled on this device (mtb200_gemm2_pairs() is 0); callers then use the one-CTA kernel.
+int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
+
+int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
+                      long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                      float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
+  return mtb::g2::gemm2((out_f32 & GEMM2_WIDE) != 0, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 & ~GEMM2_WIDE, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part,
+                        part_bytes, stats, status, stream);
+}
+
+// The same with wide tiles (256 x 512).
+int mtb200_gemm2_wide_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
+                           long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                           float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
+  return mtb::g2::gemm2(true, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
 }
 
 }  // extern "C"

@@ -33,12 +33,8 @@ template <> struct ActMaps<ACT_NONE> {};
 
 constexpr int ACT_WARPS = 8;
 constexpr int ACT_BOX = 32 * 64;                     // bytes of a box
-static_assert(ACT_WARPS * 2 * ACT_BOX == EPI_SMEM, "two boxes per warp");
+static_assert(ACT_BOX == NARROW_BOX && ACT_WARPS * 2 * ACT_BOX == EPI_SMEM, "two boxes per warp");
 
-// A thread's row in a box: four 16-byte pieces.
-__device__ __forceinline__ uint4* box_piece(uint8_t* box, int lane, int i) {
-  return reinterpret_cast<uint4*>(box + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
-}
 __device__ __forceinline__ float2 sigmoid2(float2 x) {   // 1 / (1 + exp(-x))
   return make_float2(__fdividef(1.f, 1.f + __expf(-x.x)), __fdividef(1.f, 1.f + __expf(-x.y)));
 }
@@ -115,6 +111,61 @@ __device__ __forceinline__ void epilogue_act(const EpiParams& p, const ActParams
       for (int j = 0; j < 16; ++j) g[j] = act_pair<GLU>(g[j], u[GLU ? j : 0], false);
     }
     send(maps.act, g, col);
+  }
+}
+
+// The same for wide tiles: one warp has all 256 columns of its quarter and reads them before it works on any (epilogue_wide).
+__device__ __forceinline__ void send_piece(EpiOut& out, const CUtensorMap* map, const uint32_t (&d)[16], int col, int y0, int lane) {
+  uint8_t* box = next_narrow_box(out, lane);
+  stage_piece32(box, lane, d);
+  out.map = map;
+  store_box(out, box, col, y0, lane);
+}
+template <int ACT, typename Drained>
+__device__ __forceinline__ void epilogue_act_wide(const EpiParams& p, const ActParams& ap, const ActMaps<ACT>& maps, EpiOut& out, uint32_t taddr,
+                                                  int row0, int tn, int q, int lane, Drained drained) {
+  constexpr bool GLU = ACT == ACT_GLU;
+  const int y0 = row0 + q * 32;
+  if (y0 >= p.M) { drained(); return; }
+  uint32_t d[8][16];   // gated: four pieces of the gate, then four of up
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    uint32_t v[32];
+    tmem_ld_32x32(taddr + c * 32, v);
+    tmem_ld_wait();
+    if (ACT == ACT_PLAIN && p.bias != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int col = tn * 256 + c * 32 + i * 8;
+        if (col < ap.F) {
+          const uint4 b = *reinterpret_cast<const uint4*>(p.bias + col);
+          const float2 b0 = unpack_bf16(b.x), b1 = unpack_bf16(b.y), b2 = unpack_bf16(b.z), b3 = unpack_bf16(b.w);
+          const float add[8] = {b0.x, b0.y, b1.x, b1.y, b2.x, b2.y, b3.x, b3.y};
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[i * 8 + j] = __float_as_uint(__uint_as_float(v[i * 8 + j]) + add[j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) d[c][j] = formed(pack_bf16(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])));
+  }
+  drained();
+#pragma unroll 1
+  for (int c = 0; c < (GLU ? 4 : 8); ++c) {
+    const int col = tn * (GLU ? 128 : 256) + c * 32;
+    if (col >= ap.F) break;
+    send_piece(out, &maps.gate, d[0], col, y0, lane);
+    if constexpr (GLU) send_piece(out, &maps.up, d[4], col, y0, lane);
+    if (ap.gelu) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) d[0][j] = act_pair<GLU>(d[0][j], d[GLU ? 4 : 0][j], true);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) d[0][j] = act_pair<GLU>(d[0][j], d[GLU ? 4 : 0][j], false);
+    }
+    send_piece(out, &maps.act, d[0], col, y0, lane);
+    next_piece<GLU ? 4 : 8>(d);
+    if constexpr (GLU) next_piece<4>(d + 4);
   }
 }
 

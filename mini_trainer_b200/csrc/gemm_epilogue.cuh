@@ -43,6 +43,14 @@ struct RowStats {
   float m = -INFINITY, s = 0.f;
 };
 
+__device__ __forceinline__ void row_stats8(RowStats& st, uint4 o) {   // eight bf16 values
+  const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y), r2 = unpack_bf16(o.z), r3 = unpack_bf16(o.w);
+  const float mx = fmaxf(fmax3(fmaxf(r0.x, r0.y), r1.x, r1.y), fmax3(fmaxf(r2.x, r2.y), r3.x, r3.y));
+  if (mx > st.m) { st.s *= __expf(st.m - mx); st.m = mx; }
+  st.s += __expf(r0.x - st.m) + __expf(r0.y - st.m) + __expf(r1.x - st.m) + __expf(r1.y - st.m) + __expf(r2.x - st.m) +
+          __expf(r2.y - st.m) + __expf(r3.x - st.m) + __expf(r3.y - st.m);
+}
+
 // Output staging. A row of a tile belongs to one thread, so storing it directly sends 32 half-sectors to 32 rows with every
 // instruction: a 128 x 256 tile cost about 4000 clocks of the load/store unit, more than its MMAs when the reduction is short.
 // A warp stages 128 bytes of each of its 32 rows in shared memory (128B-swizzled, conflict-free) and one TMA store writes the
@@ -78,16 +86,17 @@ __device__ __forceinline__ void store_box(EpiOut& o, const uint8_t* box, int x, 
 // Before the CTA's shared memory goes away.
 __device__ __forceinline__ void drain_boxes() { bulk_wait_read<0>(); }
 
-// 32 accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
-// bf16 box; an fp32 box holds 32 columns). Columns past N and rows past M are computed from nothing and clipped by the store.
-template <bool OUT_F32, bool STATS, bool EXTRA>
-__device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
+// COLS accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
+// bf16 box; an fp32 box holds 32 columns). NARROW boxes have rows of 64 bytes: 32 bf16 or 16 fp32 columns. Columns past N and rows past M are
+// computed from nothing and clipped by the store.
+template <bool OUT_F32, bool STATS, bool EXTRA, bool NARROW = false, int COLS = 32>
+__device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[COLS], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
                                                RowStats& st) {
 #pragma unroll
-  for (int j = 0; j < 32; ++j) f[j] *= p.alpha;
+  for (int j = 0; j < COLS; ++j) f[j] *= p.alpha;
   if (EXTRA && p.bias != nullptr) {
 #pragma unroll
-    for (int j = 0; j < 32; j += 8) {
+    for (int j = 0; j < COLS; j += 8) {
       if (col0 + j < p.N) {
         const uint4 b = *reinterpret_cast<const uint4*>(p.bias + col0 + j);
         const float2 b0 = unpack_bf16(b.x), b1 = unpack_bf16(b.y), b2 = unpack_bf16(b.z), b3 = unpack_bf16(b.w);
@@ -100,15 +109,15 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
   if constexpr (OUT_F32) {
     const float* rptr = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
-    for (int j = 0; j < 32; j += 4) {
+    for (int j = 0; j < COLS; j += 4) {
       float4 o = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
       if (res && col0 + j < p.N) { const float4 r = *reinterpret_cast<const float4*>(rptr + j); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
-      *reinterpret_cast<float4*>(srow + (((j >> 2) ^ (lane & 7)) << 4)) = o;
+      *reinterpret_cast<float4*>(srow + (((j >> 2) ^ (NARROW ? (lane >> 1) & 3 : lane & 7)) << 4)) = o;
     }
   } else {
     const __nv_bfloat16* rptr = reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
-    for (int j = 0; j < 32; j += 8) {
+    for (int j = 0; j < COLS; j += 8) {
       if (res && col0 + j < p.N) {
         const uint4 r = *reinterpret_cast<const uint4*>(rptr + j);
         const float2 r0 = unpack_bf16(r.x), r1 = unpack_bf16(r.y), r2 = unpack_bf16(r.z), r3 = unpack_bf16(r.w);
@@ -118,14 +127,51 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
       uint4 o;
       o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
       o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
-      *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
-      if (STATS && col0 + j < p.N) {   // of the values as stored
-        const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y), r2 = unpack_bf16(o.z), r3 = unpack_bf16(o.w);
-        const float mx = fmaxf(fmax3(fmaxf(r0.x, r0.y), r1.x, r1.y), fmax3(fmaxf(r2.x, r2.y), r3.x, r3.y));
-        if (mx > st.m) { st.s *= __expf(st.m - mx); st.m = mx; }
-        st.s += __expf(r0.x - st.m) + __expf(r0.y - st.m) + __expf(r1.x - st.m) + __expf(r1.y - st.m) + __expf(r2.x - st.m) +
-                __expf(r2.y - st.m) + __expf(r3.x - st.m) + __expf(r3.y - st.m);
-      }
+      if constexpr (NARROW) *reinterpret_cast<uint4*>(srow + (((j >> 3) ^ ((lane >> 1) & 3)) << 4)) = o;
+      else *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
+      if (STATS && col0 + j < p.N) row_stats8(st, o);   // of the values as stored
+    }
+  }
+}
+
+// Split-K: this warp's 32 x 256 fp32 partial to the workspace, as lane-interleaved 16-byte pieces, so that every store and load is one contiguous
+// 512 bytes; pieces past N are left out. `drained` is called when the accumulator has been read. True for the warp that arrives last.
+template <typename Drained>
+__device__ __forceinline__ bool leave_partial(const EpiParams& p, uint32_t taddr, int tn0, int q, int lane, int unit, int split, Drained drained) {
+  float* mine = p.ws + (static_cast<long long>(unit) * p.splits + split) * SPLIT_UNIT + q * 8192 + lane * 4;
+#pragma unroll 1
+  for (int c = 0; c < 8; ++c) {
+    if (tn0 + c * 32 >= p.N) break;
+    uint32_t v[32];
+    tmem_ld_32x32(taddr + c * 32, v);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      __stcg(reinterpret_cast<float4*>(mine + c * 1024 + j * 128),
+             make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
+  }
+  drained();
+  __threadfence();
+  __syncwarp();
+  unsigned last = 0;
+  if (lane == 0) last = last_arrival(p.counters + unit * 4 + q, p.epoch, p.splits);
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (last) __threadfence();
+  return last != 0;
+}
+// 32 columns (piece `c` of eight) of the sum of a unit's partials, in split order.
+__device__ __forceinline__ void sum_partials(const EpiParams& p, float (&f)[32], int tn0, int c, int q, int lane, int unit) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) f[j] = 0.f;
+  if (tn0 + c * 32 >= p.N) return;   // never written
+  const float* base = p.ws + static_cast<long long>(unit) * p.splits * SPLIT_UNIT + q * 8192 + lane * 4 + c * 1024;
+#pragma unroll 2
+  for (int s = 0; s < p.splits; ++s) {
+    const float* src = base + static_cast<long long>(s) * SPLIT_UNIT;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(src + j * 128));
+      f[4 * j] += v.x; f[4 * j + 1] += v.y; f[4 * j + 2] += v.z; f[4 * j + 3] += v.w;
     }
   }
 }
@@ -171,27 +217,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
     finish();
     return;
   }
-  // partial to the workspace: lane-interleaved 16-byte pieces, so every store and load is one contiguous 512 bytes
-  float* mine = p.ws + (static_cast<long long>(unit) * p.splits + split) * SPLIT_UNIT + q * 8192 + lane * 4;
-#pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
-    if (tn0 + c * 32 >= p.N) break;
-    uint32_t v[32];
-    tmem_ld_32x32(taddr + c * 32, v);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      __stcg(reinterpret_cast<float4*>(mine + c * 1024 + j * 128),
-             make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
-  }
-  __threadfence();
-  __syncwarp();
-  unsigned last = 0;
-  if (lane == 0) last = last_arrival(p.counters + unit * 4 + q, p.epoch, p.splits);
-  last = __shfl_sync(0xffffffffu, last, 0);
-  if (!last) return;
-  __threadfence();
-  const float* base = p.ws + static_cast<long long>(unit) * p.splits * SPLIT_UNIT + q * 8192 + lane * 4;
+  if (!leave_partial(p, taddr, tn0, q, lane, unit, split, [] {})) return;
 #pragma unroll 1
   for (int c = 0; c < 8; c += PARTS) {
     const int col0 = tn0 + c * 32;
@@ -200,25 +226,132 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
 #pragma unroll 1
     for (int k = 0; k < PARTS; ++k) {
       float f[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) f[j] = 0.f;
-      if (col0 + k * 32 < p.N) {   // pieces past N were never written
-#pragma unroll 2
-        for (int s = 0; s < p.splits; ++s) {
-          const float* src = base + static_cast<long long>(s) * SPLIT_UNIT + (c + k) * 1024;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + j * 128));
-            f[4 * j] += v.x; f[4 * j + 1] += v.y; f[4 * j + 2] += v.z; f[4 * j + 3] += v.w;
-          }
-        }
-      }
+      sum_partials(p, f, tn0, c + k, q, lane, unit);
       epilogue_row32<OUT_F32, STATS, EXTRA>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
     }
     store_box(out, box, col0, row0 + q * 32, lane);
   }
   finish();
   if (lane == 0) p.counters[unit * 4 + q] = 0;
+}
+
+// Wide tiles (gemm2_tcgen05.cu): the same part of an item for the eight epilogue warps of a CTA, two boxes of 32 rows x 64 bytes each. The
+// accumulator is wanted back at once, and reading it is the short part of an epilogue: `drained` is called when the 256 columns are in registers,
+// rounded (bias and residual come before the rounding, so with them the columns are stored as they are read; fp32 columns would not fit).
+// 16384 x 28672 x 4096 in a loop at the power cap: 1320 TFLOP/s storing as it reads, 1413 this way.
+constexpr int NARROW_BOX = 32 * 64;
+__device__ __forceinline__ uint8_t* next_narrow_box(EpiOut& o, int lane) {
+  if (lane == 0) bulk_wait_read<1>();
+  __syncwarp();
+  return o.stage + (o.n & 1) * NARROW_BOX;
+}
+// A thread's row in such a box: four 16-byte pieces, 64B-swizzled.
+__device__ __forceinline__ uint4* box_piece(uint8_t* box, int lane, int i) {
+  return reinterpret_cast<uint4*>(box + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
+}
+// Formed here: the compiler would move the rounding to where the value is stored, past `drained`, and hold the fp32 values until then.
+__device__ __forceinline__ uint32_t formed(uint32_t x) {
+  asm volatile("" : "+r"(x));
+  return x;
+}
+// A loop over pieces that are held in registers works on the first of them and moves the others up: unrolled, the arithmetic of several pieces is
+// started together and the registers spill.
+template <int N>
+__device__ __forceinline__ void next_piece(uint32_t (*d)[16]) {
+#pragma unroll
+  for (int c = 0; c + 1 < N; ++c)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) d[c][j] = d[c + 1][j];
+}
+__device__ __forceinline__ void stage_piece32(uint8_t* box, int lane, const uint32_t (&d)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) *box_piece(box, lane, i) = make_uint4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
+}
+template <bool OUT_F32, bool STATS, bool EXTRA, typename Drained>
+__device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane, int unit, int split,
+                                              Drained drained) {
+  const int y0 = row0 + q * 32, row = y0 + lane;
+  if (y0 >= p.M) { drained(); return; }
+  const bool row_ok = row < p.M;
+  RowStats st;
+  auto finish = [&]() {
+    if (STATS && row_ok && tn0 < p.N) p.stats[static_cast<long long>(row) * ((p.N + 255) / 256) + tn0 / 256] = make_float2(st.m, st.s);
+  };
+  auto send32 = [&](float (&f)[32], int col0) {
+    if constexpr (OUT_F32) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        float h[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) h[j] = f[k * 16 + j];
+        uint8_t* box = next_narrow_box(out, lane);
+        epilogue_row32<true, false, EXTRA, true, 16>(p, h, row, row_ok, col0 + k * 16, box + lane * 64, 0, lane, st);
+        store_box(out, box, col0 + k * 16, y0, lane);
+      }
+    } else {
+      uint8_t* box = next_narrow_box(out, lane);
+      epilogue_row32<false, STATS, EXTRA, true>(p, f, row, row_ok, col0, box + lane * 64, 0, lane, st);
+      store_box(out, box, col0, y0, lane);
+    }
+  };
+  if (p.splits > 1) {
+    if (!leave_partial(p, taddr, tn0, q, lane, unit, split, drained)) return;
+#pragma unroll 1
+    for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
+      float f[32];
+      sum_partials(p, f, tn0, c, q, lane, unit);
+      send32(f, tn0 + c * 32);
+    }
+    finish();
+    if (lane == 0) p.counters[unit * 4 + q] = 0;
+  } else if constexpr (EXTRA || OUT_F32) {
+#pragma unroll 1
+    for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
+      uint32_t v[32];
+      tmem_ld_32x32(taddr + c * 32, v);
+      tmem_ld_wait();
+      float f[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+      send32(f, tn0 + c * 32);
+    }
+    drained();
+    finish();
+  } else {
+    uint32_t d[8][16];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      uint32_t v[2][32];
+      tmem_ld_32x32(taddr + c * 32, v[0]);
+      tmem_ld_32x32(taddr + c * 32 + 32, v[1]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) d[c + k][j] = formed(pack_bf16(__uint_as_float(v[k][2 * j]) * p.alpha, __uint_as_float(v[k][2 * j + 1]) * p.alpha));
+    }
+    drained();
+    auto send = [&](const uint32_t (&x)[16], int col0) {
+      uint8_t* box = next_narrow_box(out, lane);
+      stage_piece32(box, lane, x);
+      store_box(out, box, col0, y0, lane);
+    };
+    if constexpr (STATS) {
+#pragma unroll 1
+      for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (tn0 + c * 32 + i * 8 < p.N) row_stats8(st, make_uint4(d[0][4 * i], d[0][4 * i + 1], d[0][4 * i + 2], d[0][4 * i + 3]));
+        send(d[0], tn0 + c * 32);
+        next_piece<8>(d);
+      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (tn0 + c * 32 < p.N) send(d[c], tn0 + c * 32);
+    }
+    finish();
+  }
 }
 
 // Products of at most this many operations start under their predecessor's tail (launch_pdl). It saves about 2 us per launch whatever the

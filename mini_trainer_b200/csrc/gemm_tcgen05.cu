@@ -373,20 +373,22 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
-// bf16 map for the boxes of the activation epilogues: 32 rows x 32 columns, 64B-swizzled.
-int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld) {
+// Map for boxes of 32 rows x 64 bytes, 64B-swizzled (activation epilogues, wide tiles).
+int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32) {
   EncodeTiledFn enc = get_encode();
   if (enc == nullptr) return -1;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * 2) % 16) return -2;
+  const uint64_t bytes = f32 ? 4 : 2;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * bytes) % 16) return -2;
   cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {ld * 2};
-  cuuint32_t box[2] = {32, 32};
+  cuuint64_t strides[1] = {ld * bytes};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(64 / bytes), 32};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -3;
 }
+int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld) { return make_tmap_narrow(out, base, inner, outer, ld, 0); }
 
 // Tensor map the epilogue stores D through: boxes of 32 rows x 128 bytes.
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32) {
@@ -408,7 +410,7 @@ static unsigned tune_wait_hint() {
 }
 
 namespace g2 {
-int launch_act(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
+int launch_act(int mode, bool wide, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
                int* status, cudaStream_t stream);
 int launch_gather(const void* A, long long lda, void* D, long long ldd, const void* bias, int M, int N, int K,
                   const void* w, int* status, const GatherParams& g, cudaStream_t stream);
@@ -498,7 +500,7 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
 #undef GEMM
 }
 
-// A product with an MLP's activation in its epilogue (gemm_act.cuh), on one CTA or, two_cta, on CTA pairs.
+// A product with an MLP's activation in its epilogue (gemm_act.cuh), on one CTA or, two_cta, on CTA pairs (2: with wide tiles).
 //   mode 1  out[M, 2F] = A[M, K] * W[2F, K]^T, act[M, F] = f(out[:, :F]) * out[:, F:]
 //   mode 2  out[M, F] = A[M, K] * W[F, K]^T (+ bias), act[M, F] = f(out)
 // All row-major, without padding between rows but in A. f: SiLU, or (gelu) the tanh-approximated GELU.
@@ -522,7 +524,7 @@ int mtb200_gemm_act(const void* A, long long lda, const void* W, void* out, void
   if (rc) return rc - 20;
   const EpiParams e{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0};
   const ActParams a{F, gelu};
-  if (two_cta) return g2::launch_act(mode, ta, tb, m, e, a, K, status, stream);
+  if (two_cta) return g2::launch_act(mode, two_cta == 2, ta, tb, m, e, a, K, status, stream);
   const GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u, e, a};
   if (mode == ACT_GLU)
     return launch<false, false, false, false, false, GROUP_NONE, false, false, ACT_GLU>(ta, tb, m.gate, p, stream, nullptr, 0, nullptr, m);

@@ -76,11 +76,13 @@ def _spec(ops, cfg, T: int):
         H, F, q, Q = cfg.hidden_size, cfg.intermediate_size, cfg.q_size, cfg.qkv_size
         gu = 2 * F if cfg.mlp_gated else F
         products = [(T, Q, H), (T, H, q), (T, gu, H), (T, H, F), (T, F, H), (T, H, gu), (T, q, H), (T, H, Q), (H, F, T), (gu, H, T), (H, q, T), (Q, H, T)]
-        plans = [ops._gemm_plans.get((*m, None)) or ops._plan_gemm(*m, None) for m in products]
+        # leading dimensions: forward K and K, input gradients K and N, weight gradients M and N
+        pitches = [k for _, _, k in products[:4]] + [n | k for _, n, k in products[4:8]] + [m | n for m, n, _ in products[8:]]
+        plans = [ops._gemm_plans.get((*m, None, ld & 15 != 0)) or ops._plan_gemm(*m, None, ld & 15 != 0) for m, ld in zip(products, pitches)]
         s = Spec(T, H, F, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, int(cfg.mlp_gated),
                  int((cfg.mlp_act if cfg.mlp_gated else "gelu_tanh") != "silu"), int(cfg.norm_type == "layernorm"), int(cfg.qk_norm), cfg.rms_norm_eps,
                  cfg.attention_scale, cfg.residual_multiplier)
-        s.pair[:] = [int(n == "mtb200_gemm2_bf16") for n, _, _ in plans]
+        s.pair[:] = [ops.FORMS[n] for n, _, _ in plans]
         s.splits[:] = [k for _, k, _ in plans]
         part = [b if k > 1 else 0 for _, k, b in plans]
         if len(ops._block_specs) >= 1024:

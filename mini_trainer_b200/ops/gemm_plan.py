@@ -48,3 +48,42 @@ def choose(M: int, N: int, K: int, sms: int, pairs: int, one: bool, max_units: i
         if best is None or p[0] < best[0]:
             best = p
     return best[2], best[1]
+
+
+# Wide tiles (256 x 512 on a CTA pair) move a quarter less from L2 to the SMs than pairs with 256 x 256. Fitted to 180 products of 0.02 to 1.4 TFLOP,
+# each in a loop of its own of 0.1 s and more, where the clock is already held down by power: a fixed part (launches overlap), a k-block, the rest
+# of an item, a split launch, a partial. Pairs twice: rows that start on 32-byte sectors, and rows that do not (a pitch that is no multiple of 16
+# elements), which cost L2 a request more per 128 bytes; there wide tiles are the faster form by 6 % on average (4285 x 37920 x 3864 1213 -> 1016 us),
+# elsewhere only where the reduction is long enough to hide a wide tile's ends (7001 x 3072 x 12288 458 -> 431 us, but 4099 x 12288 x 2048 179 -> 187).
+_WIDE = (-2.0, 0.85, 4.1, 11.0, 2.9)
+_PAIR_LOOP = ((-4.0, 0.445, 1.6, 5.8, 3.6), (-5.8, 0.51, 2.0, 4.6, 3.4))
+WIDE_RAGGED_FLOPS, WIDE_FLOPS, WIDE_K = 3e10, 1e11, 4096
+LONG_FLOPS = 1e12
+
+
+def _loop_cost(tiles: int, kblocks: int, units: int, max_units: int, workers: int, t: tuple, halves: bool) -> tuple:
+    fixed, block, item, split, partial = t
+    rest = tiles % workers
+    tail = 0.5 if halves and 2 * rest <= workers else 1   # a last round that half the pairs have a wide tile for is given out as half tiles
+    best, splits = tiles // workers * (kblocks * block + item) + (kblocks * block * tail + item if rest else 0), 1
+    for s in range(2, MAX_SPLITS + 1):
+        if units * s > max_units or kblocks < 4 * s or tiles * (s - 1) >= 5 * workers:
+            break
+        c = -(-tiles * s // workers) * (-(-kblocks // s) * block + item) + split + partial * s
+        if c < best:
+            best, splits = c, s
+    return best + fixed, splits
+
+
+def wide(M: int, N: int, K: int, ragged: bool, pairs: int, max_units: int, max_counted: int) -> int:
+    """Splits of the product on wide tiles, or 0 where the other kernels are the faster. ``ragged``: rows of an operand do not start on 32 bytes.
+    Products of more than ``LONG_FLOPS`` run at the power cap, where what is moved costs clock: there wide tiles give 1300 to 1410 TFLOP/s, pairs 1170 to
+    1375 and single CTAs 1180 to 1325 (16384 tokens of an 8B model)."""
+    flops, kblocks, rows, cols = 2.0 * M * N * K, -(-K // BK), -(-M // 256), -(-N // 256)
+    if pairs <= 0 or not (flops > LONG_FLOPS or flops >= WIDE_FLOPS and K >= WIDE_K or ragged and flops >= WIDE_RAGGED_FLOPS):
+        return 0
+    units = 2 * rows * cols
+    most = max_units if units <= max_counted else 0
+    cost, splits = _loop_cost(rows * -(-N // 512), kblocks, units, most, pairs, _WIDE, True)
+    other, _ = _loop_cost(rows * cols, kblocks, units, most, pairs, _PAIR_LOOP[ragged], False)
+    return splits if cost <= other * (1.1 if flops > LONG_FLOPS else 1.0) else 0

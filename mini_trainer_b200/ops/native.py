@@ -52,6 +52,7 @@ P, I, L, F, U = c_void_p, c_int, c_longlong, c_float, c_ulonglong
 class _Sig:
     mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, U, P, L, P, P, P]
     mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, U, P, L, P, P, P]
+    mtb200_gemm2_wide_bf16 = mtb200_gemm2_bf16
     mtb200_gemm2_pairs = []
     mtb200_gemm_act = [P, L, P, P, P, P, I, I, I, I, I, I, P, P]
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
@@ -149,6 +150,7 @@ def route_topk(logits, k: int, renorm: bool, call=_launch):
 
 class NativeOps:
     name = "native"
+    FORMS = {"mtb200_gemm_bf16": 0, "mtb200_gemm2_bf16": 1, "mtb200_gemm2_wide_bf16": 2}   # as csrc/block_exec.cu and mtb200_gemm_act take them
 
     def __init__(self, device, ce_chunk: int = 8192, attention: str | None = None):
         self.device = torch.device(device)
@@ -160,11 +162,10 @@ class NativeOps:
         self.ce_chunk = ce_chunk
         self.attention_impl = attention or os.environ.get("MTB200_ATTENTION", "native")
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-        # GEMM kernel and splits by size: gemm_plan. The CTA-pair kernel (cta_group::2) draws more power: in a step made of long GEMMs,
-        # which runs at the 1000 W cap, it lowers the clock of EVERY kernel by 12-16 % and the step gets slower (8B model, 64 000-token
-        # minibatches: 9.77 s per step with one CTA, 10.36 with pairs). Where GEMMs are short the cap does not bind (1.5B model,
-        # 8000-token minibatches: 729 and 700 ms, clocks 1530 and 1515 MHz). So a product of more than 1 TFLOP (about 0.8 ms)
-        # stays on single CTAs. MTB200_GEMM2=0 / 1 forces one kernel for all of them (1: also for the fused gathers).
+        # GEMM kernel and splits by size: gemm_plan. The CTA-pair kernel (cta_group::2) with 256 x 256 tiles draws more power: in a step made of long
+        # GEMMs, which runs at the 1000 W cap, it lowers the clock of EVERY kernel by 12-16 % and the step gets slower (8B model, 64 000-token
+        # minibatches: 9.77 s per step with one CTA, 10.36 with pairs). So a product of more than 1 TFLOP (about 0.8 ms) takes wide tiles, which move
+        # less (gemm_plan.wide), or single CTAs. MTB200_GEMM2=0 / 1 forces one kernel for all of them (1: also for the fused gathers).
         self.use_gemm2 = os.environ.get("MTB200_GEMM2") == "1"
         self.pair_max_flops = 0.0 if os.environ.get("MTB200_GEMM2") == "0" else 1e12
         self.launches = 0
@@ -278,18 +279,26 @@ class NativeOps:
             return None
         return ws, next(self._epoch), part
 
-    def _plan_gemm(self, M, N, K, two_cta):
-        """``(entry point, splits, bytes of partials)`` of a product, from its sizes."""
+    def _plan_gemm(self, M, N, K, two_cta, ragged=False):
+        """``(entry point, splits, bytes of partials)`` of a product, from its sizes and whether rows of an operand start off 32 bytes."""
         pairs, one = self.cta_pairs(), True
+        wide = 0
         if two_cta if two_cta is not None else self.use_gemm2:
             one = False
-        elif two_cta is not None or 2.0 * M * N * K > self.pair_max_flops:
+        elif two_cta is not None or self.pair_max_flops <= 0:
             pairs = 0
-        pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
+        else:
+            wide = gemm_plan.wide(M, N, K, ragged, pairs, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
+            if 2.0 * M * N * K > self.pair_max_flops:
+                pairs = 0
+        if wide:
+            plan = ("mtb200_gemm2_wide_bf16", wide, gemm_plan.partial_bytes(M, N, True, wide))
+        else:
+            pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
+            plan = ("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", splits, gemm_plan.partial_bytes(M, N, pair, splits))
         if len(self._gemm_plans) >= 4096:
             self._gemm_plans.clear()
-        plan = ("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", splits, gemm_plan.partial_bytes(M, N, pair, splits))
-        self._gemm_plans[(M, N, K, two_cta)] = plan
+        self._gemm_plans[(M, N, K, two_cta, ragged)] = plan
         return plan
 
     def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
@@ -300,10 +309,8 @@ class NativeOps:
         out_f32 = out.dtype == torch.float32
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
         assert residual is None or residual.dtype == out.dtype
-        plan = self._gemm_plans.get((M, N, K, two_cta))
-        if plan is None:
-            plan = self._plan_gemm(M, N, K, two_cta)
-        name, splits, nbytes = plan
+        ragged = bool((a.stride(0) | b.stride(0)) & 15)
+        name, splits, nbytes = self._gemm_plans.get((M, N, K, two_cta, ragged)) or self._plan_gemm(M, N, K, two_cta, ragged)
         st = self._st()
         split = self._split(st, nbytes) if splits > 1 else None
         ws, epoch, part = split or (None, 0, None)
@@ -413,7 +420,8 @@ class NativeOps:
         N = w.shape[0]
         F, code = N // 2 if gated else N, _ACT[fn]
         assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-        name, splits, _ = self._gemm_plans.get((T, N, K, None)) or self._plan_gemm(T, N, K, None)
+        ragged = bool((x.stride(0) | K) & 15)
+        name, splits, _ = self._gemm_plans.get((T, N, K, None, ragged)) or self._plan_gemm(T, N, K, None, ragged)
         # Two launches where one cannot address the weight, and for a product that splits its reduction: 700 x 2048 x 8192 32 us, 43 whole with the
         # activation inside (level at reductions of 4096: 512 x 2048 24.6 and 24.9). No kernel is SiLU alone.
         plain = w.is_contiguous() and K % 8 == 0 and F % 8 == 0
@@ -424,7 +432,7 @@ class NativeOps:
         pre = torch.empty(T, N, dtype=x.dtype, device=self.device)
         act = torch.empty(T, F, dtype=x.dtype, device=self.device)
         self._call("mtb200_gemm_act", x.data_ptr(), x.stride(0), w.data_ptr(), pre.data_ptr(), act.data_ptr(), _ptr(bias), 1 if gated else 2, code,
-                   T, F, K, int(name == "mtb200_gemm2_bf16"), self.status.data_ptr(), self._st(), tag="gemm_nt_act")
+                   T, F, K, self.FORMS[name], self.status.data_ptr(), self._st(), tag="gemm_nt_act")
         return pre, act
 
     def linear_wgrad(self, dy, x, dw_out, dbias_out=None, alpha=1.0):

@@ -1551,3 +1551,50 @@ def test_router_kernel_belongs_to_the_native_backend(ops, monkeypatch):
     before = ops.launches
     M.moe_forward(ops, cfg, p, n2, h1, False, False)   # router, slabs, gather, gate/up
     assert calls == ["counted"] and ops.launches == before + 4
+
+
+# partial last row and column tiles, one or two halves of a wide tile, a last round given out as halves (37 * 256 rows), reductions of one to a few
+# k-blocks, split ones; operands of -1, 0, 1: every sum is exact
+@pytest.mark.parametrize("M,N", [(33, 264), (300, 520), (256 * 37, 2120), (256 * 37 + 65, 2568)])
+@pytest.mark.parametrize("K,splits", [(64, 1), (72, 1), (200, 1), (1032, 2), (1032, 4)])
+def test_gemm_wide_tiles_are_exact(ops, M, N, K, splits, monkeypatch):
+    from mini_trainer_b200.ops import gemm_plan
+    monkeypatch.setattr(gemm_plan, "wide", lambda M, N, K, *a: splits if 2 * -(-M // 256) * -(-N // 256) * splits <= 1024 else 1)
+    monkeypatch.setattr(ops, "_gemm_plans", {})
+    names = []
+    monkeypatch.setattr(ops, "_call", lambda name, *a, call=ops._call, **kw: names.append(name) or call(name, *a, **kw))
+    rows = -(-M // 8) * 8
+    a, b = _ints(rows, K), _ints(N, K)
+    at, bt = a.t().contiguous(), b.t().contiguous()
+    want, res, bias = a.float() @ b.float().t(), _ints(rows, N), _ints(N)
+    for a_mn, b_mn in ((False, False), (False, True), (True, False), (True, True)):
+        m = rows if a_mn else M
+        for dt in (torch.bfloat16, torch.float32):
+            for extra in (False, True):
+                out = torch.full((m, N), float("nan"), dtype=dt, device="cuda")
+                kw = dict(residual=res[:m].to(dt), bias=bias) if extra else {}
+                ops.gemm(at if a_mn else a, a_mn, bt if b_mn else b, b_mn, out, m, N, K, **kw)
+                ref = want[:m] + (res[:m].float() + bias.float() if extra else 0.0)
+                assert torch.equal(out, ref.to(dt)), (a_mn, b_mn, dt, extra)
+    assert set(names) == {"mtb200_gemm2_wide_bf16"}
+    ops.check_status()
+
+
+@pytest.mark.parametrize("T,F,K", [(33, 136, 264), (1000, 1000, 512), (256 * 37, 1096, 72)])
+@pytest.mark.parametrize("fn", ["silu", "gelu_tanh"])
+def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypatch):
+    """Activation and softmax statistics behind wide tiles: the same bits as behind 256 x 256 tiles."""
+    from mini_trainer_b200.ops import gemm_plan
+    torch.manual_seed(T + F)
+    x, w, bias = bf(T, K), bf(2 * F, K, scale=K ** -0.5), bf(2 * F)
+    got = []
+    for splits in (1, 0):
+        monkeypatch.setattr(gemm_plan, "wide", lambda *a: splits)
+        monkeypatch.setattr(gemm_plan, "choose", lambda *a: (True, 1))
+        monkeypatch.setattr(ops, "_gemm_plans", {})
+        out, stats = torch.empty(T, 2 * F, dtype=torch.bfloat16, device="cuda"), torch.full((T, -(-2 * F // 256), 2), float("nan"), device="cuda")
+        ops.gemm(x, False, w, False, out, T, 2 * F, K, alpha=0.5, stats=stats)
+        got.append([*ops.linear_act(x, w, fn), out, stats] + ([*ops.linear_act(x, w, fn, gated=False, bias=bias)] if fn == "gelu_tanh" else []))
+    for g, h in zip(*got):
+        assert torch.equal(g, h)
+    ops.check_status()

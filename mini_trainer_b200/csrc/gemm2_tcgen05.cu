@@ -22,6 +22,9 @@
 // a warpgroup per half empties its accumulator into registers before it stores anything (epilogue_wide), and the first half's next tile starts
 // while the second's is emptied. What is left of the gap is about 2500 clocks, which short reductions show (5987 x 17920 x 1536: 263 us in 256 x 256 tiles, 281 wide).
 //
+// GROUP is the grouped form over expert slabs (gemm_epilogue.cuh) in wide tiles: 4096 tokens through 2 of 8 experts of 4096 x 14336, forward and backward,
+// 8.20 -> 7.78 ms.
+//
 // GATHER = true is the fused all-gather variant (see gather.cuh): both CTAs of a pair carry eight
 // gather warps and a flag checker; each CTA's checker watches the chunks under ITS half of the B
 // tile (128 weight rows, one contiguous byte range) and only that CTA's producer waits for them.
@@ -41,7 +44,7 @@ namespace mtb {
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer);
-int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32);
+int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32, uint64_t n, uint64_t stride);
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32);
 
 namespace g2 {
@@ -68,6 +71,16 @@ constexpr int GROUP_M = 8;               // band of 8 pair-tiles = 2048 rows
 constexpr int GATHER_GROUP_N = 4;        // column-tiles per band in the all-gather variant
 constexpr int SMEM = STAGES * STAGE_BYTES + EPI_SMEM + 1024 + 256;
 constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;   // clears the CTA-rank bit of a shared::cluster address -> CTA 0
+
+// How many of a launch's wide tiles are given out whole: a last round that half of the pairs have a tile for goes as half tiles.
+__host__ __device__ inline int whole_tiles(int tiles, int pairs) {
+  const int rest = tiles % pairs;
+  return 2 * rest <= pairs ? tiles - rest : tiles;
+}
+inline int wide_group_m(int tiles_m) {
+  const int bands = (tiles_m + WIDE_GROUP_M / 2) / WIDE_GROUP_M;
+  return bands > 1 ? (tiles_m + bands - 1) / bands : tiles_m;
+}
 
 struct Params {
   int M, N, K;
@@ -96,6 +109,12 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tma
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_addr_cta0), "r"(c0), "r"(c1)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, uint32_t bar_addr_cta0, int32_t c0, int32_t c1, int32_t c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_addr_cta0), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
 __device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -113,11 +132,14 @@ __device__ __forceinline__ void mbar_arrive_cta0(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(smem_u32(bar) & PEER_MASK) : "memory");
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE, bool WIDE = false>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE, bool WIDE = false,
+          int GROUP = GROUP_NONE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT, WIDE), 1)
 gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
              const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ ActMaps<ACT> maps, Params p,
-             const __grid_constant__ GatherParams g) {
+             const __grid_constant__ GatherParams g, GroupParams gr) {
+  static_assert(GROUP == GROUP_NONE || WIDE, "the grouped forms are wide");
+  __shared__ GroupTable gtab;   // unused (and not allocated) outside the grouped forms
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + EPI_SMEM);
@@ -135,9 +157,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), tiles_n = (p.N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
   const int kblocks = (p.K + BK - 1) / BK;
-  const int splits = GATHER ? 1 : p.e.splits;
+  const int splits = GATHER || GROUP ? 1 : p.e.splits;
   const int wide_n = (p.N + 2 * BN - 1) / (2 * BN);
-  const int num_items = WIDE ? tiles_m * wide_n * splits + (tiles_m * wide_n - p.whole) : num_tiles * splits;   // item = split * num_tiles + tile: neighbours share operand tiles
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -154,12 +175,17 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   pdl_wait();   // nothing so far has touched global memory
+  if (GROUP && warp == 2) fill_group_table<GROUP>(gtab, gr, 2 * BM, wide_n, tiles_m * wide_n, lane);
   tc_fence_before();
   __syncthreads();
   cluster_sync();          // the partner's barriers are initialised before anything is sent to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  // item = split * num_tiles + tile: neighbours share operand tiles. Wide tiles: the first `whole` items are whole tiles, then come half tiles.
+  const int wide_tiles = GROUP ? gtab.tile_start[gr.E] : tiles_m * wide_n;
+  const int whole = GROUP ? whole_tiles(wide_tiles, p.num_pairs) : p.whole;
+  const int num_items = WIDE ? wide_tiles * splits + (wide_tiles - whole) : num_tiles * splits;
   auto k_range = [&](int split, int& kb0, int& kb1) {
     kb0 = static_cast<int>(static_cast<long long>(kblocks) * split / splits);
     kb1 = static_cast<int>(static_cast<long long>(kblocks) * (split + 1) / splits);
@@ -182,22 +208,29 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     tn = local / rows;
   };
 
-  // Wide tiles: row-tile, first column and number of 256-column halves (0: a half tile past the last column) of an item.
-  auto wide_coords = [&](int w, int& tm, int& col0, int& halves, int& kb0, int& kb1) {
-    const int all = tiles_m * wide_n;
-    k_range(splits > 1 ? w / all : 0, kb0, kb1);
-    if (splits > 1) w %= all;
-    const int t = w < p.whole ? w : p.whole + (w - p.whole) / 2;
+  // Wide tiles: row-tile, first column and number of 256-column halves (0: a half tile past the last column) of an item. The grouped forms walk
+  // the experts with the items: `e` only moves forward.
+  auto wide_coords = [&](int w, int& e, int& tm, int& col0, int& halves, int& kb0, int& kb1) {
+    k_range(splits > 1 ? w / wide_tiles : 0, kb0, kb1);
+    if (splits > 1) w %= wide_tiles;
+    int t = w < whole ? w : whole + (w - whole) / 2;
+    int rows_m = tiles_m;
+    if constexpr (GROUP != GROUP_NONE) {
+      while (t >= gtab.tile_start[e + 1]) ++e;
+      t -= gtab.tile_start[e];
+      if (GROUP == GROUP_ROWS) rows_m = (gr.counts[e] + 2 * BM - 1) / (2 * BM);
+      else { kb0 = 0; kb1 = (gr.counts[e] + BK - 1) / BK; }
+    }
     const int band = t / (p.group_m * wide_n);
     const int first_m = band * p.group_m;
-    const int rows = min(p.group_m, tiles_m - first_m);
+    const int rows = min(p.group_m, rows_m - first_m);
     const int local = t - band * p.group_m * wide_n;
     tm = first_m + local % rows;
     col0 = local / rows * 2 * BN;
-    if (w < p.whole) {
+    if (w < whole) {
       halves = col0 + BN < p.N ? 2 : 1;
     } else {
-      col0 += ((w - p.whole) & 1) * BN;
+      col0 += ((w - whole) & 1) * BN;
       halves = col0 < p.N ? 1 : 0;
     }
   };
@@ -207,11 +240,17 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // ------------------------------------------------------------------ wide tiles: TMA producer (both CTAs)
     if (elect_one()) {
       uint32_t it = 0;
+      int e = 0;
       for (int w = pair; w < num_items; w += p.num_pairs) {
         int tm, col0, halves, kb0, kb1;
-        wide_coords(w, tm, col0, halves, kb0, kb1);
+        wide_coords(w, e, tm, col0, halves, kb0, kb1);
         if (halves == 0) continue;
-        const int row0 = tm * 2 * BM + rank * BM;
+        int row0 = tm * 2 * BM + rank * BM;
+        if (GROUP == GROUP_ROWS) {   // a slab may end with CTA 0's rows: CTA 1 multiplies zeros then (from past the matrix), and stores nothing
+          row0 += gr.starts[e];
+          if (row0 >= gr.starts[e + 1]) row0 = p.M;
+        }
+        const int k_row = GROUP == GROUP_REDUCE ? gr.starts[e] : 0;   // first row of the reduction
         // this CTA's part of each half of B: 128 of its columns; with a gated activation CTA 0 has the gate's weight and CTA 1 up's
         const int b0 = ACT == ACT_GLU ? col0 / 2 + static_cast<int>(rank) * p.act.F : col0 + rank * BNH;
         constexpr int b_step = ACT == ACT_GLU ? BNH : BN;
@@ -224,7 +263,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * (A_BYTES + halves * B_BYTES));
           if (A_MN) {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tmap_a, fb, row0 + j * 64, kb * BK);
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * 8192, &tmap_a, fb, row0 + j * 64, k_row + kb * BK);
           } else {
             tma_load_2d_pair(sa, &tmap_a, fb, kb * BK, row0);
           }
@@ -232,23 +271,28 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
             uint8_t* sb = sa + A_BYTES + h * B_BYTES;
             if (B_MN) {
 #pragma unroll
-              for (int j = 0; j < BNH / 64; ++j) tma_load_2d_pair(sb + j * 8192, &tmap_b, fb, b0 + h * b_step + j * 64, kb * BK);
+              for (int j = 0; j < BNH / 64; ++j) {
+                if constexpr (GROUP == GROUP_ROWS) tma_load_3d_pair(sb + j * 8192, &tmap_b, fb, b0 + h * b_step + j * 64, kb * BK, e);
+                else tma_load_2d_pair(sb + j * 8192, &tmap_b, fb, b0 + h * b_step + j * 64, k_row + kb * BK);
+              }
             } else {
-              tma_load_2d_pair(sb, &tmap_b, fb, kb * BK, b0 + h * b_step);
+              if constexpr (GROUP == GROUP_ROWS) tma_load_3d_pair(sb, &tmap_b, fb, kb * BK, b0 + h * b_step, e);
+              else tma_load_2d_pair(sb, &tmap_b, fb, kb * BK, b0 + h * b_step);
             }
           }
         }
       }
-      pdl_trigger();
+      if (!GROUP || gr.flops <= PDL_MAX_GROUPED_FLOPS) pdl_trigger();
     }
   } else if (WIDE && warp == 1) {
     // ------------------------------------------------------------------ wide tiles: MMA issuer (leader CTA only)
     if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       uint32_t it = 0, used0 = 0, used1 = 0;   // stages so far; tiles that used each accumulator
+      int e = 0;
       for (int w = pair; w < num_items; w += p.num_pairs) {
         int tm, col0, halves, kb0, kb1;
-        wide_coords(w, tm, col0, halves, kb0, kb1);
+        wide_coords(w, e, tm, col0, halves, kb0, kb1);
         if (halves == 0) continue;
         auto filled = [&](int j) { return mbar_wait(&full_bar[(it + j) % WIDE_STAGES], ((it + j) / WIDE_STAGES) & 1, abort_flag); };
         auto multiply = [&](int j, int h) {
@@ -303,22 +347,25 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     EpiOut out{&tmap_d, smem + WIDE_STAGES * WIDE_STAGE_BYTES + (warp - 4) * 2 * ACT_BOX, -1, 0};
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * BN;
     uint32_t used = 0;
+    int e = 0;
     for (int w = pair; w < num_items; w += p.num_pairs) {
       int tm, col0, halves, kb0, kb1;
-      wide_coords(w, tm, col0, halves, kb0, kb1);
+      wide_coords(w, e, tm, col0, halves, kb0, kb1);
       if (h >= halves) continue;
       if (!mbar_wait(&tfull_bar[h], used & 1, abort_flag)) { atomicExch(p.status, 54); goto done; }
       ++used;
       tc_fence_after();
-      const int row0 = tm * 2 * BM + rank * BM;
+      int row0 = tm * 2 * BM + rank * BM, row_end = p.M;
+      if constexpr (GROUP == GROUP_ROWS) { row0 += gr.starts[e]; row_end = gr.starts[e + 1]; }   // slabs are padded to 128 rows, all of which may be stored
+      if constexpr (GROUP == GROUP_REDUCE) out.z = e;
       auto drained = [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cta0(&tempty_bar[h]);
       };
-      if constexpr (ACT != ACT_NONE) epilogue_act_wide<ACT>(p.e, p.act, maps, out, taddr, row0, col0 / BN + h, q, lane, drained);
-      else epilogue_wide<OUT_F32, STATS, EXTRA>(p.e, out, taddr, row0, col0 + h * BN, q, lane, 2 * (tm * tiles_n + col0 / BN + h) + static_cast<int>(rank),
-                                                splits > 1 ? w / (tiles_m * wide_n) : 0, drained);
+      if constexpr (ACT != ACT_NONE) epilogue_act_wide<ACT>(p.e, p.act, maps, out, taddr, row0, row_end, col0 / BN + h, q, lane, drained);
+      else epilogue_wide<OUT_F32, !GROUP, STATS, EXTRA>(p.e, out, taddr, row0, row_end, col0 + h * BN, q, lane, 2 * (tm * tiles_n + col0 / BN + h) + static_cast<int>(rank),
+                                                splits > 1 ? w / wide_tiles : 0, GROUP == GROUP_REDUCE && kb1 == 0, drained);
     }
   } else if (WIDE) {
     // warps 2 and 3 have no part
@@ -479,10 +526,11 @@ static int co_resident_pairs() {
   return pairs;
 }
 
-template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE, bool WIDE = false>
+template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool STATS = false, bool EXTRA = true, int ACT = ACT_NONE, bool WIDE = false,
+          int GROUP = GROUP_NONE>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, Params p, cudaStream_t stream, const GatherParams* gp = nullptr,
-                  long long part_bytes = 0, const ActMaps<ACT>& maps = ActMaps<ACT>{}) {
-  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA, ACT, WIDE>;
+                  long long part_bytes = 0, const ActMaps<ACT>& maps = ActMaps<ACT>{}, const GroupParams* grp = nullptr) {
+  auto kern = gemm2_kernel<A_MN, B_MN, OUT_F32, GATHER, STATS, EXTRA, ACT, WIDE, GROUP>;
   constexpr int threads = GATHER ? THREADS + GATHER_EXTRA_THREADS : threads_of(ACT, WIDE);
   static bool configured = false;
   if (!configured) {
@@ -497,18 +545,17 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   int items = tiles * p.e.splits;
   p.group_m = GROUP_M;
   if constexpr (WIDE) {
-    const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), wide = tiles_m * ((p.N + 2 * BN - 1) / (2 * BN)), rest = wide % pairs;
-    const int bands = max(1, (tiles_m + WIDE_GROUP_M / 2) / WIDE_GROUP_M);
-    p.group_m = (tiles_m + bands - 1) / bands;
-    // a last round that half of the pairs have a tile for is given out as half tiles
-    p.whole = p.e.splits == 1 && 2 * rest <= pairs ? wide - rest : wide;
+    const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), wide = tiles_m * ((p.N + 2 * BN - 1) / (2 * BN));
+    p.group_m = wide_group_m(tiles_m);
+    p.whole = p.e.splits == 1 ? whole_tiles(wide, pairs) : wide;
     items = wide * p.e.splits + (wide - p.whole);
+    if (GROUP == GROUP_REDUCE) items *= grp->E;   // at most, both forms
   }
   p.num_pairs = (GATHER || items >= pairs) ? pairs : items;
   static const GatherParams none{};
-  if constexpr (GATHER) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, *gp);
-  else if (2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, none);
-  else launch_pdl(kern, 2 * p.num_pairs, threads, SMEM, stream, ta, tb, td, maps, p, none);
+  if constexpr (GATHER) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, *gp, GroupParams{});
+  else if (GROUP ? grp->flops > PDL_MAX_GROUPED_FLOPS : 2.0 * p.M * p.N * p.K > PDL_MAX_FLOPS) kern<<<2 * p.num_pairs, threads, SMEM, stream>>>(ta, tb, td, maps, p, none, grp ? *grp : GroupParams{});
+  else launch_pdl(kern, 2 * p.num_pairs, threads, SMEM, stream, ta, tb, td, maps, p, none, grp ? *grp : GroupParams{});
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -537,6 +584,16 @@ int launch_act(int mode, bool wide, const CUtensorMap& ta, const CUtensorMap& tb
   return launch<false, false, false, false, false, false, ACT_PLAIN>(ta, tb, m.gate, p, stream, nullptr, 0, plain);
 }
 
+// Grouped products on wide tiles; called by mtb200_gemm_grouped. `td`, `m`: maps of boxes of 32 rows x 64 bytes.
+int launch_grouped(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a,
+                   int K, const GroupParams& g, int* status, cudaStream_t stream) {
+  const Params p{e.M, e.N, K, status, 0, 0, 0, e, a};
+  if (mode == 3) return launch<false, false, false, false, false, false, ACT_GLU, true, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, m, &g);
+  if (mode == 0) return launch<false, false, false, false, false, false, ACT_NONE, true, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, ActMaps<ACT_NONE>{}, &g);
+  if (mode == 1) return launch<false, true, false, false, false, false, ACT_NONE, true, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, ActMaps<ACT_NONE>{}, &g);
+  return launch<true, true, false, false, false, false, ACT_NONE, true, GROUP_REDUCE>(ta, tb, td, p, stream, nullptr, 0, ActMaps<ACT_NONE>{}, &g);
+}
+
 template <bool A_MN, bool B_MN>
 static int launch_wide(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const Params& p, bool out_f32, long long part_bytes, cudaStream_t stream) {
   if (out_f32) return launch<A_MN, B_MN, true, false, false, true, ACT_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
@@ -558,7 +615,7 @@ static int gemm2(bool wide, const void* A, long long lda, int a_mn, const void* 
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BNH);
   if (rc) return rc - 10;
-  rc = wide ? make_tmap_narrow(&td, D, N, M, ldd, out_f32) : make_tmap_out(&td, D, M, N, ldd, out_f32);
+  rc = wide ? make_tmap_narrow(&td, D, N, M, ldd, out_f32, 0, 0) : make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
   Params p{M, N, K, status, 0, 0, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, part, stats, counters, epoch}};
   if (wide) {

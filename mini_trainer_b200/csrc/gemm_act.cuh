@@ -123,10 +123,10 @@ __device__ __forceinline__ void send_piece(EpiOut& out, const CUtensorMap* map, 
 }
 template <int ACT, typename Drained>
 __device__ __forceinline__ void epilogue_act_wide(const EpiParams& p, const ActParams& ap, const ActMaps<ACT>& maps, EpiOut& out, uint32_t taddr,
-                                                  int row0, int tn, int q, int lane, Drained drained) {
+                                                  int row0, int row_end, int tn, int q, int lane, Drained drained) {
   constexpr bool GLU = ACT == ACT_GLU;
   const int y0 = row0 + q * 32;
-  if (y0 >= p.M) { drained(); return; }
+  if (y0 >= row_end) { drained(); return; }
   uint32_t d[8][16];   // gated: four pieces of the gate, then four of up
 #pragma unroll
   for (int c = 0; c < 8; ++c) {

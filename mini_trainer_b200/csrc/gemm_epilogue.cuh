@@ -237,7 +237,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
 
 // Wide tiles (gemm2_tcgen05.cu): the same part of an item for the eight epilogue warps of a CTA, two boxes of 32 rows x 64 bytes each. The
 // accumulator is wanted back at once, and reading it is the short part of an epilogue: `drained` is called when the 256 columns are in registers,
-// rounded (bias and residual come before the rounding, so with them the columns are stored as they are read; fp32 columns would not fit).
+// rounded (`row_end`: the first row that is not the item's; `zero`: it had nothing to multiply; bias and residual come before the rounding, so with them the columns are stored as they are read; fp32 columns would not fit).
 // 16384 x 28672 x 4096 in a loop at the power cap: 1320 TFLOP/s storing as it reads, 1413 this way.
 constexpr int NARROW_BOX = 32 * 64;
 __device__ __forceinline__ uint8_t* next_narrow_box(EpiOut& o, int lane) {
@@ -267,12 +267,12 @@ __device__ __forceinline__ void stage_piece32(uint8_t* box, int lane, const uint
 #pragma unroll
   for (int i = 0; i < 4; ++i) *box_piece(box, lane, i) = make_uint4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
 }
-template <bool OUT_F32, bool STATS, bool EXTRA, typename Drained>
-__device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane, int unit, int split,
-                                              Drained drained) {
+template <bool OUT_F32, bool SPLIT, bool STATS, bool EXTRA, typename Drained>
+__device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int row_end, int tn0, int q, int lane, int unit,
+                                              int split, bool zero, Drained drained) {
   const int y0 = row0 + q * 32, row = y0 + lane;
-  if (y0 >= p.M) { drained(); return; }
-  const bool row_ok = row < p.M;
+  if (y0 >= row_end) { drained(); return; }
+  const bool row_ok = row < row_end;
   RowStats st;
   auto finish = [&]() {
     if (STATS && row_ok && tn0 < p.N) p.stats[static_cast<long long>(row) * ((p.N + 255) / 256) + tn0 / 256] = make_float2(st.m, st.s);
@@ -294,7 +294,7 @@ __device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, u
       store_box(out, box, col0, y0, lane);
     }
   };
-  if (p.splits > 1) {
+  if (SPLIT && p.splits > 1) {
     if (!leave_partial(p, taddr, tn0, q, lane, unit, split, drained)) return;
 #pragma unroll 1
     for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
@@ -328,7 +328,7 @@ __device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, u
 #pragma unroll
       for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) d[c + k][j] = formed(pack_bf16(__uint_as_float(v[k][2 * j]) * p.alpha, __uint_as_float(v[k][2 * j + 1]) * p.alpha));
+        for (int j = 0; j < 16; ++j) d[c + k][j] = zero ? 0u : formed(pack_bf16(__uint_as_float(v[k][2 * j]) * p.alpha, __uint_as_float(v[k][2 * j + 1]) * p.alpha));
     }
     drained();
     auto send = [&](const uint32_t (&x)[16], int col0) {

@@ -373,22 +373,22 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
-// Map for boxes of 32 rows x 64 bytes, 64B-swizzled (activation epilogues, wide tiles).
-int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32) {
+// Map for boxes of 32 rows x 64 bytes, 64B-swizzled (activation epilogues, wide tiles); with n > 0 over n matrices, `stride` elements apart.
+int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32, uint64_t n, uint64_t stride) {
   EncodeTiledFn enc = get_encode();
   if (enc == nullptr) return -1;
   const uint64_t bytes = f32 ? 4 : 2;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * bytes) % 16) return -2;
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {ld * bytes};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(64 / bytes), 32};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * bytes) % 16 || (stride * bytes) % 16) return -2;
+  cuuint64_t dims[3] = {inner, outer, n};
+  cuuint64_t strides[2] = {ld * bytes, stride * bytes};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(64 / bytes), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, n ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -3;
 }
-int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld) { return make_tmap_narrow(out, base, inner, outer, ld, 0); }
+int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld) { return make_tmap_narrow(out, base, inner, outer, ld, 0, 0, 0); }
 
 // Tensor map the epilogue stores D through: boxes of 32 rows x 128 bytes.
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32) {
@@ -412,6 +412,8 @@ static unsigned tune_wait_hint() {
 namespace g2 {
 int launch_act(int mode, bool wide, const CUtensorMap& ta, const CUtensorMap& tb, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a, int K,
                int* status, cudaStream_t stream);
+int launch_grouped(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a,
+                   int K, const GroupParams& g, int* status, cudaStream_t stream);
 int launch_gather(const void* A, long long lda, void* D, long long ldd, const void* bias, int M, int N, int K,
                   const void* w, int* status, const GatherParams& g, cudaStream_t stream);
 }
@@ -532,7 +534,8 @@ int mtb200_gemm_act(const void* A, long long lda, const void* W, void* out, void
                                                                                      ActMaps<ACT_PLAIN>{m.gate, m.up, m.act});
 }
 
-// Grouped GEMM over expert slabs (see gemm_epilogue.cuh); starts [E + 1] and counts [E] are device arrays, `rows` is the
+enum { GROUPED_WIDE = 4 };
+// Grouped GEMM over expert slabs (see gemm_epilogue.cuh); mode + GROUPED_WIDE: on CTA pairs with wide tiles (gemm2_tcgen05.cu). starts [E + 1] and counts [E] are device arrays, `rows` is the
 // height of the row buffers.
 //   mode 0  D[rows, N] = A[rows, K] * W_e[N, K]^T        W: E matrices [N, K], w_stride elements apart
 //   mode 1  D[rows, N] = A[rows, K] * W_e[K, N]          W: E matrices [K, N], w_stride elements apart
@@ -542,30 +545,35 @@ int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long l
                         int M, int N, int K, const int* starts, const int* counts, int E, long long w_stride, int* status,
                         cudaStream_t stream) {
   using namespace mtb;
+  const bool wide = mode >= GROUPED_WIDE;
+  if (wide) mode -= GROUPED_WIDE;
   if (E <= 0 || rows <= 0 || N <= 0 || (mode == 2 ? M : K) <= 0) return 0;
   if (E > GROUP_MAX || N % 8 || ldd % 8 || rows % GROUP_ALIGN || w_stride % 8 || mode < 0 || mode > 3 || (mode == 3 && (act == nullptr || N % 16))) return -10;
   CUtensorMap ta, tb, td;
   int rc = mode == 2 ? make_tmap_2d_bf16(&ta, A, M, rows, lda, 64, 64) : make_tmap_2d_bf16(&ta, A, K, rows, lda, BK, BM);
   if (rc) return rc;
-  if (mode == 0 || mode == 3) rc = make_tmap_3d_bf16(&tb, B, K, N, E, w_stride, BK, mode == 3 ? BN / 2 : BN);
+  if (mode == 0 || mode == 3) rc = make_tmap_3d_bf16(&tb, B, K, N, E, w_stride, BK, mode == 3 || wide ? BN / 2 : BN);
   else if (mode == 1) rc = make_tmap_3d_bf16(&tb, B, N, K, E, w_stride, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, N, rows, ldb, 64, 64);
   if (rc) return rc - 10;
   const int out_rows = mode == 2 ? M : rows;
-  if (mode == 2) rc = ldd == N ? make_tmap_3d_bf16(&td, D, N, M, E, w_stride, 64, 32) : -10;
-  else rc = make_tmap_out(&td, D, rows, N, ldd, 0);
+  if (mode == 2 && ldd != N) rc = -10;
+  else if (wide) rc = make_tmap_narrow(&td, D, N, out_rows, ldd, 0, mode == 2 ? E : 0, mode == 2 ? w_stride : 0);
+  else rc = mode == 2 ? make_tmap_3d_bf16(&td, D, N, M, E, w_stride, 64, 32) : make_tmap_out(&td, D, rows, N, ldd, 0);
   if (rc) return rc - 20;
-  GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u,
-               EpiParams{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0}, ActParams{N / 2, gelu}};
+  const EpiParams ep{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0};
+  const ActParams ap{N / 2, gelu};
   GroupParams g{starts, counts, E, static_cast<float>(2.0 * rows * N * (mode == 2 ? M : K))};
+  ActMaps<ACT_GLU> m{};
   if (mode == 3) {
-    ActMaps<ACT_GLU> m;
     rc = make_tmap_act(&m.gate, D, N / 2, rows, ldd);
     if (!rc) rc = make_tmap_act(&m.up, reinterpret_cast<__nv_bfloat16*>(D) + N / 2, N / 2, rows, ldd);
     if (!rc) rc = make_tmap_act(&m.act, act, N / 2, rows, N / 2);
     if (rc) return rc - 20;
-    return launch<false, false, false, false, false, GROUP_ROWS, false, false, ACT_GLU>(ta, tb, td, p, stream, nullptr, 0, &g, m);
   }
+  if (wide) return g2::launch_grouped(mode, ta, tb, td, m, ep, ap, K, g, status, stream);
+  GemmParams p{out_rows, N, K, status, tune_group_m(), tune_wait_hint(), 0u, ep, ap};
+  if (mode == 3) return launch<false, false, false, false, false, GROUP_ROWS, false, false, ACT_GLU>(ta, tb, td, p, stream, nullptr, 0, &g, m);
   if (mode == 0) return launch<false, false, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
   if (mode == 1) return launch<false, true, false, false, false, GROUP_ROWS>(ta, tb, td, p, stream, nullptr, 0, &g);
   return launch<true, true, false, false, false, GROUP_REDUCE>(ta, tb, td, p, stream, nullptr, 0, &g);

@@ -87,3 +87,17 @@ def wide(M: int, N: int, K: int, ragged: bool, pairs: int, max_units: int, max_c
     cost, splits = _loop_cost(rows * -(-N // 512), kblocks, units, most, pairs, _WIDE, True)
     other, _ = _loop_cost(rows * cols, kblocks, units, most, pairs, _PAIR_LOOP[ragged], False)
     return splits if cost <= other * (1.1 if flops > LONG_FLOPS else 1.0) else 0
+
+
+def grouped_wide(reduce: bool, rows: int, experts: int, flops: float, K: int, ragged: bool) -> bool:
+    """Wide tiles for a grouped product of ``rows`` rows over all experts (``reduce``: a weight gradient), or 128 x 256 tiles on single CTAs. A tile of 256
+    rows may find 128 in a slab's last one, so slabs have to be tall. Of 42 layers, two at a time: rows that start off 32 bytes are 1.1 to 1.7 times as fast
+    wide (749 tokens x 4 of 16 experts of 2376 x 7528: 414 -> 366, 282 -> 178, 228 -> 180, 550 -> 316 us; weight gradients 1.0 to 1.17 from about 330 rows
+    on), others 0.6 to 1.05 unless the launch is long enough for the power cap (8 of 4096 x 14336, 4096 tokens x 2: layer 8200 -> 7780 us)."""
+    tall = rows / experts
+    if flops >= GROUPED_LONG_FLOPS:
+        return tall >= 768
+    return ragged and flops >= 2e10 and (tall >= 330 if reduce else tall >= 160 and K >= 1024)
+
+
+GROUPED_LONG_FLOPS = 8e11

@@ -666,7 +666,11 @@ class NativeOps:
         return out
 
     def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride, act=None, fn="silu"):
-        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), _ACT[fn], mode, sl.cap, M, N, K,
+        E = sl.counts.shape[0]
+        rows = sl.cap - (_GROUP_ALIGN - 1) * E   # of all experts, to within a tile
+        wide = self.pair_max_flops > 0 and self.cta_pairs() > 0 and gemm_plan.grouped_wide(
+            mode == 2, rows, E, 2.0 * rows * N * (M if mode == 2 else K), K, bool((a.stride(0) | ldb) & 15))
+        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), _ACT[fn], mode + 4 * wide, sl.cap, M, N, K,
                    sl.starts.data_ptr(), sl.counts.data_ptr(), sl.counts.shape[0], stride, self.status.data_ptr(), self._st(),
                    tag="gemm_grouped_" + ("nt", "nn", "tn", "nt_act")[mode])
         return out

@@ -1598,3 +1598,27 @@ def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypa
     for g, h in zip(*got):
         assert torch.equal(g, h)
     ops.check_status()
+
+
+# slabs of which the last tile holds 128 rows or 256, experts without rows, partial tiles of every output, a reduction of one k-block
+@pytest.mark.parametrize("T,E,k,popular", [(1, 4, 2, 4), (900, 48, 2, 24), (1500, 5, 2, 4), (260, 3, 1, 2)])
+@pytest.mark.parametrize("H,F", [(64, 72), (648, 520), (1040, 264)])
+def test_grouped_products_in_wide_tiles_match(ops, T, E, k, popular, H, F, monkeypatch):
+    from mini_trainer_b200.ops import gemm_plan
+    torch.manual_seed(T + H)
+    topi = torch.stack([torch.randperm(popular, device="cuda")[:k] for _ in range(T)]) * (E // popular)
+    sl = ops.expert_slabs(topi, E)
+    x, d = ops.gather_rows(bf(T, H), sl), ops.gather_rows(bf(T, 2 * F), sl)
+    w = bf(E, 2 * F, H, scale=H ** -0.5)
+    got = []
+    for wide in (False, True):
+        monkeypatch.setattr(gemm_plan, "grouped_wide", lambda *a: wide)
+        dw = torch.full((E, 2 * F, H), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.grouped_wgrad(d, x, (dw[0], 2 * F * H), sl)
+        stack = (w[0], 2 * F * H)
+        rows = int(sl.starts[-1])
+        got.append([dw, *(t[:rows] for t in (ops.grouped_linear(x, stack, sl), *ops.grouped_linear_act(x, stack, sl), *ops.grouped_linear_act(x, stack, sl, "gelu_tanh"),
+                                             ops.grouped_dgrad(d, stack, sl)))])
+    for a, b in zip(*got):
+        assert not a.isnan().any() and torch.equal(a, b)
+    ops.check_status()

@@ -249,3 +249,11 @@ def test_gemm_wide_tiles_choice(M, N, K, ragged, splits):
     assert ops._plan_gemm(M, N, K, None, ragged)[0] == "mtb200_gemm2_bf16"
     ops.use_gemm2, ops.pair_max_flops = False, 0.0
     assert ops._plan_gemm(M, N, K, None, ragged)[0] == "mtb200_gemm_bf16"
+
+
+@pytest.mark.parametrize("reduce,rows,E,flops,K,ragged,want", [(False, 8192, 8, 1.9e12, 4096, False, True), (True, 8192, 8, 1.9e12, 4096, False, True), (False, 16384, 64, 1.4e11, 2048, False, False),
+                                                               (False, 2996, 16, 2.1e11, 2376, True, True), (True, 2996, 16, 2.1e11, 0, True, False), (True, 7936, 16, 1.4e11, 0, True, True),
+                                                               (False, 2996, 16, 2.1e11, 712, True, False), (False, 1000, 32, 1e11, 2376, True, False), (False, 1310, 4, 1.5e10, 2456, True, False)])
+def test_grouped_products_choice(reduce, rows, E, flops, K, ragged, want):
+    from mini_trainer_b200.ops import gemm_plan as G
+    assert G.grouped_wide(reduce, rows, E, flops, K, ragged) == want

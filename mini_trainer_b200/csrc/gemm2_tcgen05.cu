@@ -44,7 +44,6 @@ namespace mtb {
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld,
                       uint32_t box_inner, uint32_t box_outer);
-int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32, uint64_t n, uint64_t stride);
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32);
 
 namespace g2 {
@@ -65,6 +64,7 @@ constexpr int WIDE_GROUP_M = 14;                      // row-tiles per band, abo
 constexpr int WIDE_THREADS = 384;
 constexpr int WIDE_REGS = 168, WIDE_REGS_IO = 40, WIDE_REGS_EPI = 232;   // per thread at launch, and after the split
 static_assert(WIDE_REGS_IO + 2 * WIDE_REGS_EPI == 3 * WIDE_REGS && 3 * 128 * WIDE_REGS <= 65536, "register split");
+static_assert(2 * 4 * STORE_BOX == EPI_SMEM, "a box per warp");
 static_assert(WIDE_STAGES * WIDE_STAGE_BYTES == STAGES * STAGE_BYTES, "one shared-memory size");
 constexpr int THREADS = 192;
 constexpr int GROUP_M = 8;               // band of 8 pair-tiles = 2048 rows
@@ -344,7 +344,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     // ------------------------------------------------------------------ wide tiles: epilogue (both CTAs; warps 4..7 half 0, 8..11 half 1)
     setmaxnreg_inc<WIDE_REGS_EPI>();
     const int q = warp & 3, h = (warp - 4) >> 2;
-    EpiOut out{&tmap_d, smem + WIDE_STAGES * WIDE_STAGE_BYTES + (warp - 4) * 2 * ACT_BOX, -1, 0};
+    EpiOut out{&tmap_d, smem + WIDE_STAGES * WIDE_STAGE_BYTES + (warp - 4) * STORE_BOX, -1, 0};
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + h * BN;
     uint32_t used = 0;
     int e = 0;
@@ -584,7 +584,7 @@ int launch_act(int mode, bool wide, const CUtensorMap& ta, const CUtensorMap& tb
   return launch<false, false, false, false, false, false, ACT_PLAIN>(ta, tb, m.gate, p, stream, nullptr, 0, plain);
 }
 
-// Grouped products on wide tiles; called by mtb200_gemm_grouped. `td`, `m`: maps of boxes of 32 rows x 64 bytes.
+// Grouped products on wide tiles; called by mtb200_gemm_grouped. `td`, `m`: maps of boxes of 32 rows x 128 bytes.
 int launch_grouped(int mode, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const ActMaps<ACT_GLU>& m, const EpiParams& e, const ActParams& a,
                    int K, const GroupParams& g, int* status, cudaStream_t stream) {
   const Params p{e.M, e.N, K, status, 0, 0, 0, e, a};
@@ -615,7 +615,7 @@ static int gemm2(bool wide, const void* A, long long lda, int a_mn, const void* 
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
   else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BNH);
   if (rc) return rc - 10;
-  rc = wide ? make_tmap_narrow(&td, D, N, M, ldd, out_f32, 0, 0) : make_tmap_out(&td, D, M, N, ldd, out_f32);
+  rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
   Params p{M, N, K, status, 0, 0, 0, EpiParams{M, N, R, ldr, reinterpret_cast<const __nv_bfloat16*>(bias), alpha, splits, part, stats, counters, epoch}};
   if (wide) {

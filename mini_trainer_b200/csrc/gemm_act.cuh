@@ -33,8 +33,12 @@ template <> struct ActMaps<ACT_NONE> {};
 
 constexpr int ACT_WARPS = 8;
 constexpr int ACT_BOX = 32 * 64;                     // bytes of a box
-static_assert(ACT_BOX == NARROW_BOX && ACT_WARPS * 2 * ACT_BOX == EPI_SMEM, "two boxes per warp");
+static_assert(ACT_WARPS * 2 * ACT_BOX == EPI_SMEM, "two boxes per warp");
 
+// A thread's row in a box: four 16-byte pieces.
+__device__ __forceinline__ uint4* box_piece(uint8_t* box, int lane, int i) {
+  return reinterpret_cast<uint4*>(box + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
+}
 __device__ __forceinline__ float2 sigmoid2(float2 x) {   // 1 / (1 + exp(-x))
   return make_float2(__fdividef(1.f, 1.f + __expf(-x.x)), __fdividef(1.f, 1.f + __expf(-x.y)));
 }
@@ -114,13 +118,8 @@ __device__ __forceinline__ void epilogue_act(const EpiParams& p, const ActParams
   }
 }
 
-// The same for wide tiles: one warp has all 256 columns of its quarter and reads them before it works on any (epilogue_wide).
-__device__ __forceinline__ void send_piece(EpiOut& out, const CUtensorMap* map, const uint32_t (&d)[16], int col, int y0, int lane) {
-  uint8_t* box = next_narrow_box(out, lane);
-  stage_piece32(box, lane, d);
-  out.map = map;
-  store_box(out, box, col, y0, lane);
-}
+// The same for wide tiles: one warp has all 256 columns of its quarter and reads them before it works on any; boxes of 32 rows x 128 bytes, one per
+// warp (epilogue_wide). The maps are of such boxes.
 template <int ACT, typename Drained>
 __device__ __forceinline__ void epilogue_act_wide(const EpiParams& p, const ActParams& ap, const ActMaps<ACT>& maps, EpiOut& out, uint32_t taddr,
                                                   int row0, int row_end, int tn, int q, int lane, Drained drained) {
@@ -151,21 +150,29 @@ __device__ __forceinline__ void epilogue_act_wide(const EpiParams& p, const ActP
   }
   drained();
 #pragma unroll 1
-  for (int c = 0; c < (GLU ? 4 : 8); ++c) {
+  for (int c = 0; c < (GLU ? 4 : 8); c += 2) {
     const int col = tn * (GLU ? 128 : 256) + c * 32;
     if (col >= ap.F) break;
-    send_piece(out, &maps.gate, d[0], col, y0, lane);
-    if constexpr (GLU) send_piece(out, &maps.up, d[4], col, y0, lane);
-    if (ap.gelu) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) d[0][j] = act_pair<GLU>(d[0][j], d[GLU ? 4 : 0][j], true);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) d[0][j] = act_pair<GLU>(d[0][j], d[GLU ? 4 : 0][j], false);
+    out.map = &maps.gate;
+    send_columns64(out, d, col, y0, lane);
+    if constexpr (GLU) {
+      out.map = &maps.up;
+      send_columns64(out, d + 4, col, y0, lane);
     }
-    send_piece(out, &maps.act, d[0], col, y0, lane);
-    next_piece<GLU ? 4 : 8>(d);
-    if constexpr (GLU) next_piece<4>(d + 4);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (ap.gelu) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) d[k][j] = act_pair<GLU>(d[k][j], d[GLU ? 4 + k : k][j], true);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) d[k][j] = act_pair<GLU>(d[k][j], d[GLU ? 4 + k : k][j], false);
+      }
+    }
+    out.map = &maps.act;
+    send_columns64(out, d, col, y0, lane);
+    next_pieces<GLU ? 4 : 8, 2>(d);
+    if constexpr (GLU) next_pieces<4, 2>(d + 4);
   }
 }
 

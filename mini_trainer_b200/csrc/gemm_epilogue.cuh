@@ -66,12 +66,13 @@ struct EpiOut {
   uint32_t n;           // boxes so far
 };
 
-// Buffer for the next box: free once at most the last store (the other buffer's) is still reading. Every box that is taken here is
+// Buffer for the next box, of a warp's BOXES: free once at most the other buffer's store is still reading. Every box that is taken here is
 // stored and committed, or the count of pending groups would no longer name the buffer.
+template <int BOXES = 2>
 __device__ __forceinline__ uint8_t* next_box(EpiOut& o, int lane) {
-  if (lane == 0) bulk_wait_read<1>();
+  if (lane == 0) bulk_wait_read<BOXES - 1>();
   __syncwarp();
-  return o.stage + (o.n & 1) * STORE_BOX;
+  return o.stage + (BOXES == 2 ? (o.n & 1) * STORE_BOX : 0);
 }
 __device__ __forceinline__ void store_box(EpiOut& o, const uint8_t* box, int x, int y, int lane) {
   fence_proxy_async_smem();
@@ -86,17 +87,16 @@ __device__ __forceinline__ void store_box(EpiOut& o, const uint8_t* box, int x, 
 // Before the CTA's shared memory goes away.
 __device__ __forceinline__ void drain_boxes() { bulk_wait_read<0>(); }
 
-// COLS accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
-// bf16 box; an fp32 box holds 32 columns). NARROW boxes have rows of 64 bytes: 32 bf16 or 16 fp32 columns. Columns past N and rows past M are
-// computed from nothing and clipped by the store.
-template <bool OUT_F32, bool STATS, bool EXTRA, bool NARROW = false, int COLS = 32>
-__device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[COLS], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
+// 32 accumulator columns of one row through alpha, bias and residual, into the staged row `srow` (`part`: which 64 bytes of a
+// bf16 box; an fp32 box holds 32 columns). Columns past N and rows past M are computed from nothing and clipped by the store.
+template <bool OUT_F32, bool STATS, bool EXTRA>
+__device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32], int row, bool row_ok, int col0, uint8_t* srow, int part, int lane,
                                                RowStats& st) {
 #pragma unroll
-  for (int j = 0; j < COLS; ++j) f[j] *= p.alpha;
+  for (int j = 0; j < 32; ++j) f[j] *= p.alpha;
   if (EXTRA && p.bias != nullptr) {
 #pragma unroll
-    for (int j = 0; j < COLS; j += 8) {
+    for (int j = 0; j < 32; j += 8) {
       if (col0 + j < p.N) {
         const uint4 b = *reinterpret_cast<const uint4*>(p.bias + col0 + j);
         const float2 b0 = unpack_bf16(b.x), b1 = unpack_bf16(b.y), b2 = unpack_bf16(b.z), b3 = unpack_bf16(b.w);
@@ -109,15 +109,15 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[CO
   if constexpr (OUT_F32) {
     const float* rptr = reinterpret_cast<const float*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
-    for (int j = 0; j < COLS; j += 4) {
+    for (int j = 0; j < 32; j += 4) {
       float4 o = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
       if (res && col0 + j < p.N) { const float4 r = *reinterpret_cast<const float4*>(rptr + j); o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w; }
-      *reinterpret_cast<float4*>(srow + (((j >> 2) ^ (NARROW ? (lane >> 1) & 3 : lane & 7)) << 4)) = o;
+      *reinterpret_cast<float4*>(srow + (((j >> 2) ^ (lane & 7)) << 4)) = o;
     }
   } else {
     const __nv_bfloat16* rptr = reinterpret_cast<const __nv_bfloat16*>(p.R) + static_cast<long long>(row) * p.ldr + col0;
 #pragma unroll
-    for (int j = 0; j < COLS; j += 8) {
+    for (int j = 0; j < 32; j += 8) {
       if (res && col0 + j < p.N) {
         const uint4 r = *reinterpret_cast<const uint4*>(rptr + j);
         const float2 r0 = unpack_bf16(r.x), r1 = unpack_bf16(r.y), r2 = unpack_bf16(r.z), r3 = unpack_bf16(r.w);
@@ -127,8 +127,7 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[CO
       uint4 o;
       o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
       o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
-      if constexpr (NARROW) *reinterpret_cast<uint4*>(srow + (((j >> 3) ^ ((lane >> 1) & 3)) << 4)) = o;
-      else *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
+      *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
       if (STATS && col0 + j < p.N) row_stats8(st, o);   // of the values as stored
     }
   }
@@ -235,20 +234,12 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
   if (lane == 0) p.counters[unit * 4 + q] = 0;
 }
 
-// Wide tiles (gemm2_tcgen05.cu): the same part of an item for the eight epilogue warps of a CTA, two boxes of 32 rows x 64 bytes each. The
-// accumulator is wanted back at once, and reading it is the short part of an epilogue: `drained` is called when the 256 columns are in registers,
-// rounded (`row_end`: the first row that is not the item's; `zero`: it had nothing to multiply; bias and residual come before the rounding, so with them the columns are stored as they are read; fp32 columns would not fit).
-// 16384 x 28672 x 4096 in a loop at the power cap: 1320 TFLOP/s storing as it reads, 1413 this way.
-constexpr int NARROW_BOX = 32 * 64;
-__device__ __forceinline__ uint8_t* next_narrow_box(EpiOut& o, int lane) {
-  if (lane == 0) bulk_wait_read<1>();
-  __syncwarp();
-  return o.stage + (o.n & 1) * NARROW_BOX;
-}
-// A thread's row in such a box: four 16-byte pieces, 64B-swizzled.
-__device__ __forceinline__ uint4* box_piece(uint8_t* box, int lane, int i) {
-  return reinterpret_cast<uint4*>(box + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
-}
+// Wide tiles (gemm2_tcgen05.cu): the same part of an item for the eight epilogue warps of a CTA, one box each. The accumulator is wanted back at
+// once, and reading it is the short part of an epilogue: `drained` is called when the 256 columns are in registers, rounded (`row_end`: the first row
+// that is not the item's; `zero`: it had nothing to multiply; bias and residual come before the rounding, so with them the columns are stored as they
+// are read; fp32 columns would not fit). 16384 x 28672 x 4096 in a loop at the power cap: 1320 TFLOP/s storing as it reads, 1413 this way. One box with rows
+// of 128 bytes per warp is better than two with rows of 64, which cost the copy engine as many requests each: 75776 x 4096 x 512 269 -> 249 us, x 64 133 -> 125.
+//
 // Formed here: the compiler would move the rounding to where the value is stored, past `drained`, and hold the fp32 values until then.
 __device__ __forceinline__ uint32_t formed(uint32_t x) {
   asm volatile("" : "+r"(x));
@@ -256,20 +247,27 @@ __device__ __forceinline__ uint32_t formed(uint32_t x) {
 }
 // A loop over pieces that are held in registers works on the first of them and moves the others up: unrolled, the arithmetic of several pieces is
 // started together and the registers spill.
-template <int N>
-__device__ __forceinline__ void next_piece(uint32_t (*d)[16]) {
+template <int N, int BY>
+__device__ __forceinline__ void next_pieces(uint32_t (*d)[16]) {
 #pragma unroll
-  for (int c = 0; c + 1 < N; ++c)
+  for (int c = 0; c + BY < N; ++c)
 #pragma unroll
-    for (int j = 0; j < 16; ++j) d[c][j] = d[c + 1][j];
+    for (int j = 0; j < 16; ++j) d[c][j] = d[c + BY][j];
 }
-__device__ __forceinline__ void stage_piece32(uint8_t* box, int lane, const uint32_t (&d)[16]) {
+// 64 columns of this thread's row, in two pieces.
+__device__ __forceinline__ void send_columns64(EpiOut& out, const uint32_t (*d)[16], int col0, int y0, int lane) {
+  uint8_t* box = next_box<1>(out, lane);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) *box_piece(box, lane, i) = make_uint4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<uint4*>(box + lane * 128 + (((k * 4 + i) ^ (lane & 7)) << 4)) = make_uint4(d[k][4 * i], d[k][4 * i + 1], d[k][4 * i + 2], d[k][4 * i + 3]);
+  store_box(out, box, col0, y0, lane);
 }
 template <bool OUT_F32, bool SPLIT, bool STATS, bool EXTRA, typename Drained>
 __device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int row_end, int tn0, int q, int lane, int unit,
                                               int split, bool zero, Drained drained) {
+  constexpr int PARTS = OUT_F32 ? 1 : 2;
   const int y0 = row0 + q * 32, row = y0 + lane;
   if (y0 >= row_end) { drained(); return; }
   const bool row_ok = row < row_end;
@@ -277,46 +275,30 @@ __device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, u
   auto finish = [&]() {
     if (STATS && row_ok && tn0 < p.N) p.stats[static_cast<long long>(row) * ((p.N + 255) / 256) + tn0 / 256] = make_float2(st.m, st.s);
   };
-  auto send32 = [&](float (&f)[32], int col0) {
-    if constexpr (OUT_F32) {
+  const bool partial = SPLIT && p.splits > 1;
+  if (partial && !leave_partial(p, taddr, tn0, q, lane, unit, split, drained)) return;
+  if (partial || EXTRA || OUT_F32) {
+#pragma unroll 1
+    for (int c = 0; c < 8 && tn0 + c * 32 < p.N; c += PARTS) {
+      uint8_t* box = next_box<1>(out, lane);
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        float h[16];
+      for (int k = 0; k < PARTS; ++k) {
+        float f[32];
+        if (partial) {
+          sum_partials(p, f, tn0, c + k, q, lane, unit);
+        } else {
+          uint32_t v[32];
+          tmem_ld_32x32(taddr + (c + k) * 32, v);
+          tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) h[j] = f[k * 16 + j];
-        uint8_t* box = next_narrow_box(out, lane);
-        epilogue_row32<true, false, EXTRA, true, 16>(p, h, row, row_ok, col0 + k * 16, box + lane * 64, 0, lane, st);
-        store_box(out, box, col0 + k * 16, y0, lane);
+          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+        }
+        epilogue_row32<OUT_F32, STATS, EXTRA>(p, f, row, row_ok, tn0 + (c + k) * 32, box + lane * 128, k, lane, st);
       }
-    } else {
-      uint8_t* box = next_narrow_box(out, lane);
-      epilogue_row32<false, STATS, EXTRA, true>(p, f, row, row_ok, col0, box + lane * 64, 0, lane, st);
-      store_box(out, box, col0, y0, lane);
+      store_box(out, box, tn0 + c * 32, y0, lane);
     }
-  };
-  if (SPLIT && p.splits > 1) {
-    if (!leave_partial(p, taddr, tn0, q, lane, unit, split, drained)) return;
-#pragma unroll 1
-    for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
-      float f[32];
-      sum_partials(p, f, tn0, c, q, lane, unit);
-      send32(f, tn0 + c * 32);
-    }
-    finish();
-    if (lane == 0) p.counters[unit * 4 + q] = 0;
-  } else if constexpr (EXTRA || OUT_F32) {
-#pragma unroll 1
-    for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
-      uint32_t v[32];
-      tmem_ld_32x32(taddr + c * 32, v);
-      tmem_ld_wait();
-      float f[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-      send32(f, tn0 + c * 32);
-    }
-    drained();
-    finish();
+    if (partial) { if (lane == 0) p.counters[unit * 4 + q] = 0; }
+    else drained();
   } else {
     uint32_t d[8][16];
 #pragma unroll
@@ -331,27 +313,22 @@ __device__ __forceinline__ void epilogue_wide(const EpiParams& p, EpiOut& out, u
         for (int j = 0; j < 16; ++j) d[c + k][j] = zero ? 0u : formed(pack_bf16(__uint_as_float(v[k][2 * j]) * p.alpha, __uint_as_float(v[k][2 * j + 1]) * p.alpha));
     }
     drained();
-    auto send = [&](const uint32_t (&x)[16], int col0) {
-      uint8_t* box = next_narrow_box(out, lane);
-      stage_piece32(box, lane, x);
-      store_box(out, box, col0, y0, lane);
-    };
     if constexpr (STATS) {
 #pragma unroll 1
-      for (int c = 0; c < 8 && tn0 + c * 32 < p.N; ++c) {
+      for (int c = 0; c < 8 && tn0 + c * 32 < p.N; c += 2) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (tn0 + c * 32 + i * 8 < p.N) row_stats8(st, make_uint4(d[0][4 * i], d[0][4 * i + 1], d[0][4 * i + 2], d[0][4 * i + 3]));
-        send(d[0], tn0 + c * 32);
-        next_piece<8>(d);
+        for (int i = 0; i < 8; ++i)
+          if (tn0 + c * 32 + i * 8 < p.N) row_stats8(st, make_uint4(d[i / 4][i % 4 * 4], d[i / 4][i % 4 * 4 + 1], d[i / 4][i % 4 * 4 + 2], d[i / 4][i % 4 * 4 + 3]));
+        send_columns64(out, d, tn0 + c * 32, y0, lane);
+        next_pieces<8, 2>(d);
       }
     } else {
 #pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (tn0 + c * 32 < p.N) send(d[c], tn0 + c * 32);
+      for (int c = 0; c < 8; c += 2)
+        if (tn0 + c * 32 < p.N) send_columns64(out, d + c, tn0 + c * 32, y0, lane);
     }
-    finish();
   }
+  finish();
 }
 
 // Products of at most this many operations start under their predecessor's tail (launch_pdl). It saves about 2 us per launch whatever the

@@ -373,22 +373,21 @@ int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t inner, uint64
   return r == CUDA_SUCCESS ? 0 : -3;
 }
 
-// Map for boxes of 32 rows x 64 bytes, 64B-swizzled (activation epilogues, wide tiles); with n > 0 over n matrices, `stride` elements apart.
-int make_tmap_narrow(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, int f32, uint64_t n, uint64_t stride) {
+// bf16 map for the boxes of the activation epilogues: 32 rows x 32 columns, 64B-swizzled; with wide tiles 32 rows x 64 columns, 128B-swizzled.
+int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld, bool wide) {
+  if (wide) return make_tmap_2d_bf16(out, base, inner, outer, ld, 64, 32);
   EncodeTiledFn enc = get_encode();
   if (enc == nullptr) return -1;
-  const uint64_t bytes = f32 ? 4 : 2;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * bytes) % 16 || (stride * bytes) % 16) return -2;
-  cuuint64_t dims[3] = {inner, outer, n};
-  cuuint64_t strides[2] = {ld * bytes, stride * bytes};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(64 / bytes), 32, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, n ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr,
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld * 2) % 16) return -2;
+  cuuint64_t dims[2] = {inner, outer};
+  cuuint64_t strides[1] = {ld * 2};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -3;
 }
-int make_tmap_act(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t ld) { return make_tmap_narrow(out, base, inner, outer, ld, 0, 0, 0); }
 
 // Tensor map the epilogue stores D through: boxes of 32 rows x 128 bytes.
 int make_tmap_out(CUtensorMap* out, const void* D, int M, int N, long long ldd, int out_f32) {
@@ -520,9 +519,9 @@ int mtb200_gemm_act(const void* A, long long lda, const void* W, void* out, void
   rc = make_tmap_2d_bf16(&tb, W, K, N, K, 64, mode == ACT_GLU || two_cta ? 128 : 256);
   if (rc) return rc - 10;
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
-  rc = make_tmap_act(&m.gate, o, F, M, N);
-  if (!rc) rc = make_tmap_act(&m.up, mode == ACT_GLU ? o + F : o, F, M, N);
-  if (!rc) rc = make_tmap_act(&m.act, act, F, M, F);
+  rc = make_tmap_act(&m.gate, o, F, M, N, two_cta == 2);
+  if (!rc) rc = make_tmap_act(&m.up, mode == ACT_GLU ? o + F : o, F, M, N, two_cta == 2);
+  if (!rc) rc = make_tmap_act(&m.act, act, F, M, F, two_cta == 2);
   if (rc) return rc - 20;
   const EpiParams e{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0};
   const ActParams a{F, gelu};
@@ -557,18 +556,17 @@ int mtb200_gemm_grouped(const void* A, long long lda, const void* B, long long l
   else rc = make_tmap_2d_bf16(&tb, B, N, rows, ldb, 64, 64);
   if (rc) return rc - 10;
   const int out_rows = mode == 2 ? M : rows;
-  if (mode == 2 && ldd != N) rc = -10;
-  else if (wide) rc = make_tmap_narrow(&td, D, N, out_rows, ldd, 0, mode == 2 ? E : 0, mode == 2 ? w_stride : 0);
-  else rc = mode == 2 ? make_tmap_3d_bf16(&td, D, N, M, E, w_stride, 64, 32) : make_tmap_out(&td, D, rows, N, ldd, 0);
+  if (mode == 2) rc = ldd == N ? make_tmap_3d_bf16(&td, D, N, M, E, w_stride, 64, 32) : -10;
+  else rc = make_tmap_out(&td, D, rows, N, ldd, 0);
   if (rc) return rc - 20;
   const EpiParams ep{out_rows, N, nullptr, 0, nullptr, 1.0f, 1, nullptr, nullptr, nullptr, 0};
   const ActParams ap{N / 2, gelu};
   GroupParams g{starts, counts, E, static_cast<float>(2.0 * rows * N * (mode == 2 ? M : K))};
   ActMaps<ACT_GLU> m{};
   if (mode == 3) {
-    rc = make_tmap_act(&m.gate, D, N / 2, rows, ldd);
-    if (!rc) rc = make_tmap_act(&m.up, reinterpret_cast<__nv_bfloat16*>(D) + N / 2, N / 2, rows, ldd);
-    if (!rc) rc = make_tmap_act(&m.act, act, N / 2, rows, N / 2);
+    rc = make_tmap_act(&m.gate, D, N / 2, rows, ldd, wide);
+    if (!rc) rc = make_tmap_act(&m.up, reinterpret_cast<__nv_bfloat16*>(D) + N / 2, N / 2, rows, ldd, wide);
+    if (!rc) rc = make_tmap_act(&m.act, act, N / 2, rows, N / 2, wide);
     if (rc) return rc - 20;
   }
   if (wide) return g2::launch_grouped(mode, ta, tb, td, m, ep, ap, K, g, status, stream);

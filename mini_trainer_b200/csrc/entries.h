@@ -37,4 +37,9 @@ int mtb200_attn_fwd_one(const void*, long long, void*, long long, float*, const 
 int mtb200_attn_bwd(const void*, long long, const void*, long long, const void*, long long, void*, long long, const float*, float*, float*, const int*, int,
                     int, int, int, int, int, unsigned long long*, unsigned long long, float*, long long, float, int*, cudaStream_t);
 int mtb200_colsum(const void*, long long, void*, float*, int, int, cudaStream_t);
+int mtb200_embedding_fwd(const void*, const long long*, void*, int, int, int, int*, cudaStream_t);
+int mtb200_embedding_bwd_scan(void*, const long long*, const void*, int, int, int, int*, cudaStream_t);
+int mtb200_scatter_rows(const long long*, const void*, void*, const float*, float*, int, int, int, int*, cudaStream_t);
+int mtb200_ce_fwd_bwd(const void*, long long, int, const float2*, const long long*, float*, void*, long long, int, int, float, long long, cudaStream_t);
+int mtb200_accumulate(float*, const void*, long long, int, int, cudaStream_t);
 }

@@ -78,7 +78,7 @@ def _spec(ops, cfg, T: int):
         products = [(T, Q, H), (T, H, q), (T, gu, H), (T, H, F), (T, F, H), (T, H, gu), (T, q, H), (T, H, Q), (H, F, T), (gu, H, T), (H, q, T), (Q, H, T)]
         # leading dimensions: forward K and K, input gradients K and N, weight gradients M and N
         pitches = [k for _, _, k in products[:4]] + [n | k for _, n, k in products[4:8]] + [m | n for m, n, _ in products[8:]]
-        plans = [ops._gemm_plans.get((*m, None, ld & 15 != 0)) or ops._plan_gemm(*m, None, ld & 15 != 0) for m, ld in zip(products, pitches)]
+        plans = [ops.product_plan(*m, ld) for m, ld in zip(products, pitches)]
         s = Spec(T, H, F, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, int(cfg.mlp_gated),
                  int((cfg.mlp_act if cfg.mlp_gated else "gelu_tanh") != "silu"), int(cfg.norm_type == "layernorm"), int(cfg.qk_norm), cfg.rms_norm_eps,
                  cfg.attention_scale, cfg.residual_multiplier)

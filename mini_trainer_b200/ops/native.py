@@ -18,7 +18,7 @@ import torch
 
 from .. import build as _build
 from ..utils import nvtx
-from . import attention_plan, block_exec, gemm_plan
+from . import attention_plan, block_exec, gemm_plan, step_exec
 
 _LIB = None
 _raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else \
@@ -41,7 +41,9 @@ def load_library():
             fn.restype = c_int
             fn.argtypes = getattr(_Sig, name)
     lib.mtb200_block_workspace.restype = c_longlong
+    lib.mtb200_step_workspace.restype = c_longlong
     block_exec.check_layout(lib)
+    step_exec.check_layout(lib)
     _LIB = lib
     return lib
 
@@ -88,6 +90,8 @@ class _Sig:
     mtb200_block_workspace = [P, P, I]
     mtb200_block_forward = [P, P, P, P, P]
     mtb200_block_backward = [P, P, P, P, P, P]
+    mtb200_step_workspace = [P, P]
+    mtb200_step_forward_backward = [P, P, P, P]
     mtb200_gemm_grouped = [P, L, P, L, P, L, P, I, I, I, I, I, I, P, P, I, L, P, P]
     mtb200_moe_route = [P, I, I, I, I, P, P, P, P]
     mtb200_moe_plan = [P, I, I, I, P, P, P, P, P, P]
@@ -301,6 +305,11 @@ class NativeOps:
         self._gemm_plans[(M, N, K, two_cta, ragged)] = plan
         return plan
 
+    def product_plan(self, M, N, K, pitches):
+        """``_plan_gemm`` of a product whose operands have these leading dimensions (or-ed)."""
+        ragged = pitches & 15 != 0
+        return self._gemm_plans.get((M, N, K, None, ragged)) or self._plan_gemm(M, N, K, None, ragged)
+
     def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
         """out[M,N] = alpha*A*B (+bias) (+residual). ``a_mn``/``b_mn``: operand stored [K, rows].
         ``stats`` [M, ceil(N / 256), 2] fp32 receives the softmax statistics of the (bf16) output rows per 256 columns.
@@ -420,8 +429,7 @@ class NativeOps:
         N = w.shape[0]
         F, code = N // 2 if gated else N, _ACT[fn]
         assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-        ragged = bool((x.stride(0) | K) & 15)
-        name, splits, _ = self._gemm_plans.get((T, N, K, None, ragged)) or self._plan_gemm(T, N, K, None, ragged)
+        name, splits, _ = self.product_plan(T, N, K, x.stride(0) | K)
         # Two launches where one cannot address the weight, and for a product that splits its reduction: 700 x 2048 x 8192 32 us, 43 whole with the
         # activation inside (level at reductions of 4096: 512 x 2048 24.6 and 24.9). No kernel is SiLU alone.
         plain = w.is_contiguous() and K % 8 == 0 and F % 8 == 0
@@ -603,6 +611,11 @@ class NativeOps:
         return dqkv
 
     # -- a whole decoder block (block_exec.py) ---------------------------------------------
+    EMB_SCAN = _EMB_SCAN
+
+    def step_forward_backward(self, eng, batch, grad_scale):
+        return step_exec.forward_backward(eng, batch, grad_scale)
+
     def block_forward(self, acts_type, cfg, p, x, batch, inv_freq, keep, saved_attn, want_attn, need_out):
         return block_exec.forward(self, acts_type, cfg, p, x, batch, inv_freq, keep, saved_attn, want_attn, need_out)
 
@@ -750,6 +763,13 @@ class NativeOps:
         return dx, dy
 
     # -- fused linear + cross-entropy ---------------------------------------------------
+    @staticmethod
+    def ce_wants_stats(V: int, H: int) -> bool:
+        # The statistics save the cross-entropy a read of the row, which only costs where a row does not stay on the SM, and take the
+        # epilogue 3 us per tile, which only hides behind longer reductions. Logits and gradient together: 3720 x 151936 x 1536 1646 us
+        # with and 1997 without, 8000 x 32000 x 2048 1039 and 1120, x 1536 771 and 778, but x 1024 682 and 618; 8000 x 512 x 64 86 and 69.
+        return V > 16384 and H >= 1536
+
     def linear_ce(self, x, w, targets, grad_scale, dw_out, accumulate_dw=False, ignore_index=-100, logit_scale=1.0):
         """Per-token CE of ``logit_scale * x @ w.T``. Chunked over tokens (8192 rows): bf16 logits chunk
         by the tcgen05 GEMM (fp32 accumulation, one rounding: what the reference's fused linear-CE holds
@@ -762,10 +782,7 @@ class NativeOps:
         dx = torch.empty_like(x)
         ck = min(self.ce_chunk, T)
         logits = self._buf("ce_logits", ck * V, torch.bfloat16).view(ck, V)
-        # The statistics save the cross-entropy a read of the row, which only costs where a row does not stay on the SM, and take the
-        # epilogue 3 us per tile, which only hides behind longer reductions. Logits and gradient together: 3720 x 151936 x 1536 1646 us
-        # with and 1997 without, 8000 x 32000 x 2048 1039 and 1120, x 1536 771 and 778, but x 1024 682 and 618; 8000 x 512 x 64 86 and 69.
-        stats = self._buf("ce_stats", ck * -(-V // 256) * 2, torch.float32) if V > 16384 and H >= 1536 else None
+        stats = self._buf("ce_stats", ck * -(-V // 256) * 2, torch.float32) if self.ce_wants_stats(V, H) else None
         # one chunk: its weight gradient is the whole sum, rounded (or added to what is there) in the GEMM's epilogue
         whole = T <= ck and dw_out.is_contiguous()
         dw = dw_out.view(V, H) if whole else None

@@ -37,6 +37,7 @@ import torch
 from ..models import decoder as D
 from ..models import layout as L
 from ..models.config import ModelConfig
+from ..ops import step_exec
 from ..utils import nvtx
 from .comm import LocalComm
 
@@ -187,6 +188,8 @@ class ShardedEngine:
         self.activation_budget_bytes = activation_budget_bytes
         self._oom_retries = 0
         self._state_bytes = None   # of the groups, which never change size
+        self._one_call = None      # whether step_exec covers this model, asked once
+        self._step_specs = {}      # sizes of a minibatch -> its products' plans
         self._free_reading = None  # (free, when, reserved by the allocator then)
         # Reduce a block's gradients tensor region by tensor region while its backward still runs
         # (MTB200_REGION_OVERLAP=0: one reduction per block, after its backward).
@@ -572,6 +575,13 @@ class ShardedEngine:
             raise ValueError(f"a sample of {batch.max_seqlen} tokens exceeds the model's sliding window of {win}: attention "
                              "here is full causal attention, which equals the windowed one only up to that length")
 
+        if self._one_call is None:
+            self._one_call = step_exec.covers(self)
+        if self._one_call:   # one rank and a small model: all of what follows in one native call
+            loss = ops.step_forward_backward(self, batch, grad_scale)
+            if loss is not None:
+                return loss
+
         # ---- forward ----
         levels = self.plan_checkpointing(batch.num_tokens)
         try:
@@ -799,6 +809,14 @@ class ShardedEngine:
         if self.side.cuda:
             self.side.stream.wait_stream(torch.cuda.current_stream())
         return norm
+
+    @staticmethod
+    def stalls_recorded() -> bool:
+        return _Side.stalls is not None
+
+    @staticmethod
+    def wait_event(ev) -> None:
+        _Side.wait(ev)
 
     def measure_exposed_comm(self, on: bool = True) -> None:
         """Starts (or stops) recording how long the compute stream waits for communication: gathers

@@ -346,3 +346,71 @@ def test_minibatches_are_moved_without_waiting_for_the_device(tokens):
             break
     assert not waited
     assert torch.equal(batches[-1].input_ids.cpu(), mb["input_ids"].reshape(-1))
+
+
+STEP_FAMILIES = {"llama": {}, "tied": dict(attention_bias=True, tie_word_embeddings=True), "qwen3": dict(qk_norm=True, head_dim=128),
+                 "starcoder2": dict(norm_type="layernorm", mlp_gated=False, attention_bias=True, mlp_bias=True, hidden_act="gelu_pytorch_tanh", attention_out_bias=True),
+                 "granite": dict(residual_multiplier=0.22, attention_multiplier=0.02, logits_scaling=4.0),
+                 "no-rope": dict(no_rope_layers=[0, 1, 1])}
+
+
+@pytest.mark.parametrize("family", list(STEP_FAMILIES))
+@pytest.mark.parametrize("lens", [[9], [300, 17, 129, 1, 640]])
+def test_minibatch_in_one_call_is_the_engine_launch_by_launch(family, lens, monkeypatch):
+    """Two minibatches and the step, queued by one call each and launch by launch, with and without masked rows."""
+    from mini_trainer_b200.models.config import ModelConfig
+    from mini_trainer_b200.ops.native import NativeOps
+    known = ModelConfig.__dataclass_fields__
+    cfg = ModelConfig(**{**dict(model_type="llama", vocab_size=520, hidden_size=256, intermediate_size=392, num_hidden_layers=3, num_attention_heads=6,
+                                num_key_value_heads=2, head_dim=64), **{k: v for k, v in STEP_FAMILIES[family].items() if k in known}})
+    ops = NativeOps("cuda:0")
+    got = []
+    for one_call in (True, False):
+        eng = ShardedEngine(cfg, "cuda:0", ops, optim=OptimConfig())
+        eng.init_random(seed=5, std=0.05)
+        if not one_call:
+            eng._one_call = False
+        done, n0, res = [], ops.launches, []
+        real = NativeOps.step_forward_backward
+        monkeypatch.setattr(NativeOps, "step_forward_backward", lambda *a: done.append(real(*a)) or done[-1])
+        for seed in (0, 1):
+            mb = make_mb(lens, cfg.vocab_size, seed)
+            batch = D.make_packed_batch(mb, "cuda:0")
+            if seed:   # every row counts
+                batch.targets = torch.where(batch.targets == -100, 3, batch.targets)
+                batch.loss_rows = batch.loss_targets = None
+            res.append(eng.forward_backward(batch, 1.0 / sum(lens)))
+        monkeypatch.undo()
+        assert len(done) == (2 if one_call else 0) and all(d is not None for d in done)
+        accs = [g.gacc.clone() for g in eng.groups]
+        norm = eng.optimizer_step(1e-4)
+        got.append((res, accs, norm, ops.launches - n0, [g.master.clone() for g in eng.groups]))
+        ops.check_status()
+    (l1, a1, n1, c1, m1), (l2, a2, n2, c2, m2) = got
+    assert c1 == c2
+    assert all(torch.equal(a, b) for a, b in zip(l1, l2))
+    # behind an attention backward, whose sum of dQ tiles has no fixed order, up to that
+    assert all((a - b).norm() <= 5e-3 * b.norm() for a, b in zip(a1, a2)) and torch.equal(a1[-1], a2[-1])
+    assert abs(n1 - n2) <= 5e-3 * n2 and all(torch.isfinite(m).all() for m in m1)
+
+
+def test_what_one_call_does_not_cover_goes_launch_by_launch(monkeypatch):
+    """Options that ask for the schedule itself, minibatches that are too large for it, and no room for the workspace."""
+    from mini_trainer_b200.ops import block_exec, step_exec
+    from mini_trainer_b200.ops.native import NativeOps
+    cfg, ops = get_preset("smoke-llama"), NativeOps("cuda:0")
+    eng = ShardedEngine(cfg, "cuda:0", ops, optim=OptimConfig())
+    eng.init_random(seed=5, std=0.05)
+    batch = D.make_packed_batch(make_mb([40, 30], cfg.vocab_size), "cuda:0")
+    run = lambda: step_exec.forward_backward(eng, batch, 0.01)   # noqa: E731
+    assert run() is not None
+    changes = [(eng, "activation_budget_bytes", 0), (ops, "ce_chunk", 16), (ops, "EMB_SCAN", 16), (eng, "poison", True), (step_exec, "MOST_WORKSPACE", 1000),
+               (block_exec, "_workspace", lambda *a: None), (ops, "attention_impl", "flash_attn")]
+    for where, name, value in changes:
+        monkeypatch.setattr(where, name, value)
+        assert run() is None, name
+        assert eng.forward_backward(batch, 0.01) is not None
+        monkeypatch.undo()
+    monkeypatch.setenv("MTB200_OFFLOAD_BLOCKS", "1")
+    assert run() is None
+    ops.check_status()

@@ -18,8 +18,8 @@ namespace {
 int gemm(const BlockSpec& s, const BlockIO& io, const u64*& epoch, int which, const void* a, long long lda, int a_mn, const void* b, long long ldb, int b_mn, void* d, int M, int N,
          int K, const void* r, const void* bias, float alpha, cudaStream_t st) {
   const int splits = io.part != nullptr ? s.splits[which] : 1;
-  auto f = s.pair[which] ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
-  return f(a, lda, a_mn, b, ldb, b_mn, d, N, s.pair[which] == 2 ? GEMM2_WIDE : 0, r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
+  auto f = form_on_pairs(s.form[which]) ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
+  return f(a, lda, a_mn, b, ldb, b_mn, d, N, form_flags(s.form[which]), r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
            splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, nullptr, io.status, st);
 }
 
@@ -57,7 +57,7 @@ long long forward(const BlockSpec& s, const BlockParams& p, const BlockIO& io, b
     if (!s.gated) RUN(mtb200_gelu_fwd(io.gu, act, T * s.F, st), 1);
     else RUN(s.gelu ? mtb200_geglu_fwd(io.gu, act, T, s.F, st) : mtb200_swiglu_fwd(io.gu, act, T, s.F, st), 1);
   } else {
-    RUN(mtb200_gemm_act(n2, s.H, p.wgu, io.gu, act, p.bgu, s.gated ? 1 : 2, s.gelu, s.T, s.F, s.H, s.pair[G_GU], io.status, st), 1);
+    RUN(mtb200_gemm_act(n2, s.H, p.wgu, io.gu, act, p.bgu, s.gated ? 1 : 2, s.gelu, s.T, s.F, s.H, s.act_form, io.status, st), 1);
   }
   RUN(gemm(s, io, epoch, G_DOWN, act, s.F, 0, p.wd, s.F, 0, io.out, s.T, s.H, s.F, io.h1, p.bd, s.alpha, st), 1);
   return 0;

@@ -14,7 +14,8 @@ struct BlockSpec {
   int T, H, F, Hq, Hkv, D;
   int gated, gelu, layernorm, qk_norm;
   float eps, scale, alpha;
-  int pair[GEMMS], splits[GEMMS];   // kernel (0: one CTA, 1: pairs, 2: pairs with wide tiles) and splits of each product (ops/gemm_plan.py)
+  int form[GEMMS], splits[GEMMS];   // kernel (FORM_ of entries.h) and splits of each product (ops/gemm_plan.py)
+  int act_form;                     // kernel of the gate/up product where the activation is in it
   int need_out;                     // 0: the forward stops before the activation
   int attn_form;                    // 0: one query tile per CTA, 1: pairs of heads, 2: pairs of row blocks
   int fwd_items, bwd_items, bwd_splits;

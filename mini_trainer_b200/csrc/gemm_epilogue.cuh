@@ -133,13 +133,13 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
   }
 }
 
-// Split-K: this warp's 32 x 256 fp32 partial to the workspace, as lane-interleaved 16-byte pieces, so that every store and load is one contiguous
+// Split-K: this warp's 32 x COLS fp32 partial to the workspace, as lane-interleaved 16-byte pieces, so that every store and load is one contiguous
 // 512 bytes; pieces past N are left out. `drained` is called when the accumulator has been read. True for the warp that arrives last.
-template <typename Drained>
+template <int COLS = 256, typename Drained>
 __device__ __forceinline__ bool leave_partial(const EpiParams& p, uint32_t taddr, int tn0, int q, int lane, int unit, int split, Drained drained) {
-  float* mine = p.ws + (static_cast<long long>(unit) * p.splits + split) * SPLIT_UNIT + q * 8192 + lane * 4;
+  float* mine = p.ws + (static_cast<long long>(unit) * p.splits + split) * (128 * COLS) + q * 32 * COLS + lane * 4;
 #pragma unroll 1
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < COLS / 32; ++c) {
     if (tn0 + c * 32 >= p.N) break;
     uint32_t v[32];
     tmem_ld_32x32(taddr + c * 32, v);
@@ -158,15 +158,16 @@ __device__ __forceinline__ bool leave_partial(const EpiParams& p, uint32_t taddr
   if (last) __threadfence();
   return last != 0;
 }
-// 32 columns (piece `c` of eight) of the sum of a unit's partials, in split order.
+// 32 columns (piece `c`) of the sum of a unit's partials, in split order.
+template <int COLS = 256>
 __device__ __forceinline__ void sum_partials(const EpiParams& p, float (&f)[32], int tn0, int c, int q, int lane, int unit) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) f[j] = 0.f;
   if (tn0 + c * 32 >= p.N) return;   // never written
-  const float* base = p.ws + static_cast<long long>(unit) * p.splits * SPLIT_UNIT + q * 8192 + lane * 4 + c * 1024;
+  const float* base = p.ws + static_cast<long long>(unit) * p.splits * (128 * COLS) + q * 32 * COLS + lane * 4 + c * 1024;
 #pragma unroll 2
   for (int s = 0; s < p.splits; ++s) {
-    const float* src = base + static_cast<long long>(s) * SPLIT_UNIT;
+    const float* src = base + static_cast<long long>(s) * (128 * COLS);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float4 v = __ldcg(reinterpret_cast<const float4*>(src + j * 128));
@@ -175,14 +176,14 @@ __device__ __forceinline__ void sum_partials(const EpiParams& p, float (&f)[32],
   }
 }
 
-// One warp's part of a work item: quarter `q` of the 128-row unit that starts at row `row0`, columns [tn0, tn0 + 256).
+// One warp's part of a work item: quarter `q` of the 128-row unit that starts at row `row0`, columns [tn0, tn0 + COLS).
 // `taddr`: tensor-memory address of the quarter. `unit`: index of the 128-row unit among all tiles' units. `zero`: the item
 // had nothing to multiply, the accumulator holds an older tile. SPLIT = false leaves the split-K part out, STATS = false the
 // statistics, EXTRA = false bias and residual: a worker walks this code once per tile, and what it does not need has to be fetched
 // and branched around all the same. With the statistics as a run-time branch in every product a launch of one wave took 2 us
 // more (384 x 2048 x 2048: 18.6 and 16.5 us, 4736 x 1024 x 512: 11.3 and 10.4), with bias and residual another step for some
 // (824 x 80 x 824: 12.3 and 10.6 us; on pairs 40000 x 768 x 768: 45.2 and 43.2).
-template <bool OUT_F32, bool SPLIT, bool STATS, bool EXTRA>
+template <bool OUT_F32, bool SPLIT, bool STATS, bool EXTRA, int COLS = 256>
 __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out, uint32_t taddr, int row0, int tn0, int q, int lane,
                                                  int unit, int split, bool zero) {
   constexpr int PARTS = OUT_F32 ? 1 : 2;      // 32-column pieces per box
@@ -196,7 +197,7 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
   };
   if (!SPLIT || p.splits == 1) {
 #pragma unroll 1
-    for (int c = 0; c < 8; c += PARTS) {
+    for (int c = 0; c < COLS / 32; c += PARTS) {
       const int col0 = tn0 + c * 32;
       if (col0 >= p.N) break;  // uniform across the warp
       uint32_t v[PARTS][32];
@@ -216,16 +217,16 @@ __device__ __forceinline__ void epilogue_quarter(const EpiParams& p, EpiOut& out
     finish();
     return;
   }
-  if (!leave_partial(p, taddr, tn0, q, lane, unit, split, [] {})) return;
+  if (!leave_partial<COLS>(p, taddr, tn0, q, lane, unit, split, [] {})) return;
 #pragma unroll 1
-  for (int c = 0; c < 8; c += PARTS) {
+  for (int c = 0; c < COLS / 32; c += PARTS) {
     const int col0 = tn0 + c * 32;
     if (col0 >= p.N) break;
     uint8_t* box = next_box(out, lane);
 #pragma unroll 1
     for (int k = 0; k < PARTS; ++k) {
       float f[32];
-      sum_partials(p, f, tn0, c + k, q, lane, unit);
+      sum_partials<COLS>(p, f, tn0, c + k, q, lane, unit);
       epilogue_row32<OUT_F32, STATS, EXTRA>(p, f, row, row_ok, col0 + k * 32, box + lane * 128, k, lane, st);
     }
     store_box(out, box, col0, row0 + q * 32, lane);
@@ -384,9 +385,9 @@ __device__ __forceinline__ void fill_group_table(GroupTable& tab, const GroupPar
 }
 
 // Whether a split launch over `units` 128-row units fits its scratch and leaves every item a k-block.
-inline bool split_fits(const EpiParams& e, long long units, int kblocks, long long part_bytes) {
+inline bool split_fits(const EpiParams& e, long long units, int kblocks, long long part_bytes, int unit_floats = SPLIT_UNIT) {
   return e.ws != nullptr && e.counters != nullptr && e.splits <= kblocks && units * 4 <= SPLIT_COUNTERS &&
-         units * e.splits * SPLIT_UNIT * 4 <= part_bytes;
+         units * e.splits * unit_floats * 4 <= part_bytes;
 }
 
 }  // namespace mtb

@@ -36,15 +36,17 @@
 namespace mtb {
 
 constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int STAGES = 4;
 constexpr int A_TILE_BYTES = BM * BK * 2;   // 16 KB
-constexpr int B_TILE_BYTES = BN * BK * 2;   // 32 KB
-constexpr int STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES;
+constexpr int RING_BYTES = 4 * (A_TILE_BYTES + BN * BK * 2);   // the ring of operand stages: 4 of 128 x 256 tiles, 8 of 128 x 64
+// Tiles of 128 x 64 and 128 x 128 are for products that have fewer of them than there are SMs. Such a product is a row of latencies (fill, reduction,
+// epilogue, and the partial sums, which the last arrival adds alone), and narrow tiles shorten all of them: the epilogue of a tile is a quarter or
+// half as long, and a long reduction is divided into few splits. 640 x 512 x 3072 20.0 -> 10.9 us (in 256 x 256 tiles adding the partials took
+// 12 of them), 256 x 688 x 4096 20.0 -> 10.6, 640 x 512 x 512 6.7 -> 5.4, 1200 x 1024 x 768 8.9 -> 7.0.
 constexpr int GEMM_THREADS = 192;
 constexpr int gemm_threads(int act) { return act == ACT_NONE ? GEMM_THREADS : 64 + 32 * ACT_WARPS; }
 constexpr int GROUP_M = 16;
 constexpr int GATHER_GROUP_N = 4;   // column-tiles per band in the all-gather variant
-constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + EPI_SMEM + 1024 /*alignment slack*/ + 256 /*barriers*/;
+constexpr int GEMM_SMEM = RING_BYTES + EPI_SMEM + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 struct GemmParams {
   int M, N, K;
@@ -64,15 +66,17 @@ struct GemmParams {
 // GROUP: one launch over the expert slabs of a mixture-of-experts layer (gemm_epilogue.cuh).
 // STATS: softmax statistics of the output rows (EpiParams). EXTRA: bias or residual. ACT: an activation in the epilogue (gemm_act.cuh).
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true,
-          int ACT = ACT_NONE>
+          int ACT = ACT_NONE, int NT = BN>
 __global__ void __launch_bounds__(GATHER ? GEMM_THREADS + GATHER_EXTRA_THREADS : gemm_threads(ACT), 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
             const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ ActMaps<ACT> maps, GemmParams p,
             const __grid_constant__ GatherParams g, GroupParams gr) {
+  constexpr int B_TILE_BYTES = NT * BK * 2, STAGE_BYTES = A_TILE_BYTES + B_TILE_BYTES, STAGES = RING_BYTES / STAGE_BYTES;
+  static_assert(NT == BN || (!GATHER && !GROUP && !STATS && !ACT), "the other forms have tiles of 128 x 256");
   __shared__ GroupTable gtab;   // unused (and not allocated) outside the grouped forms
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + EPI_SMEM);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + RING_BYTES + EPI_SMEM);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tfull_bar = empty_bar + STAGES;   // [2] accumulator ready for the epilogue
   uint64_t* tempty_bar = tfull_bar + 2;       // [2] accumulator drained
@@ -82,7 +86,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   uint32_t* ticket_slot = tmem_slot + 3;   // gather variant: broadcast of the chunk ticket among the gather warps
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
+  const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + NT - 1) / NT;
   const int num_tiles = tiles_m * tiles_n;
   const int kblocks = (p.K + BK - 1) / BK;
   const int splits = (GATHER || GROUP) ? 1 : p.e.splits;
@@ -183,20 +187,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           }
           if (B_MN) {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) {
-              if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb + j * 8192, &tmap_b, &full_bar[s], tn * BN + j * 64, kb * BK, e);
-              else tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[s], tn * BN + j * 64, k_row + kb * BK);
+            for (int j = 0; j < NT / 64; ++j) {
+              if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb + j * 8192, &tmap_b, &full_bar[s], tn * NT + j * 64, kb * BK, e);
+              else tma_load_2d(sb + j * 8192, &tmap_b, &full_bar[s], tn * NT + j * 64, k_row + kb * BK);
             }
           } else {
             if constexpr (ACT == ACT_GLU) {   // 128 rows of the gate's weight and the same of up's
 #pragma unroll
               for (int j = 0; j < 2; ++j) {
-                const int row = (j ? p.act.F : 0) + tn * (BN / 2);
+                const int row = (j ? p.act.F : 0) + tn * (NT / 2);
                 if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb + j * (B_TILE_BYTES / 2), &tmap_b, &full_bar[s], kb * BK, row, e);
                 else tma_load_2d(sb + j * (B_TILE_BYTES / 2), &tmap_b, &full_bar[s], kb * BK, row);
               }
-            } else if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN, e);
-            else tma_load_2d(sb, &tmap_b, &full_bar[s], kb * BK, tn * BN);
+            } else if constexpr (GROUP == GROUP_ROWS) tma_load_3d(sb, &tmap_b, &full_bar[s], kb * BK, tn * NT, e);
+            else tma_load_2d(sb, &tmap_b, &full_bar[s], kb * BK, tn * NT);
           }
         }
       }
@@ -209,7 +213,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc_bf16(BM, NT, A_MN, B_MN);
       uint32_t it = 0, tl = 0;
       int e = 0;
       for (int w = blockIdx.x; w < num_items; w += gridDim.x, ++tl) {
@@ -225,7 +229,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         const uint32_t aph = (tl >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], aph ^ 1, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 2); goto done; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * NT;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -251,10 +255,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tl) {
       int tm, tn;
       tile_coords(t, tm, tn);
-      // rows [tn*BN, tn*BN+BN) of the K-major weight (reduce mode: rows [tm*BM, tm*BM+BM) of the K-major A operand)
+      // rows [tn*NT, tn*NT+NT) of the K-major weight (reduce mode: rows [tm*BM, tm*BM+BM) of the K-major A operand)
       // are one contiguous byte range of the gathered buffer
-      const unsigned long long lo = g.b_byte_off + static_cast<unsigned long long>(REDUCE ? tm * BM : tn * BN) * p.K * 2;
-      const int rows = REDUCE ? min(BM, p.M - tm * BM) : min(BN, p.N - tn * BN);
+      const unsigned long long lo = g.b_byte_off + static_cast<unsigned long long>(REDUCE ? tm * BM : tn * NT) * p.K * 2;
+      const int rows = REDUCE ? min(BM, p.M - tm * BM) : min(NT, p.N - tn * NT);
       const unsigned long long hi = lo + static_cast<unsigned long long>(rows) * p.K * 2 - 1;
       const bool ok = wait_chunks(g, lo, hi, lane, abort_flag, p.wait_limit_us);
       __syncwarp();
@@ -273,7 +277,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     uint32_t tl = 0;
     int e = 0;
-    EpiOut out{&tmap_d, smem + STAGES * STAGE_BYTES + (ACT ? (warp - 2) * 2 * ACT_BOX : q * 2 * STORE_BOX), -1, 0};
+    EpiOut out{&tmap_d, smem + RING_BYTES + (ACT ? (warp - 2) * 2 * ACT_BOX : q * 2 * STORE_BOX), -1, 0};
     for (int w = blockIdx.x; w < num_items; w += gridDim.x, ++tl) {
       const int t = w % num_tiles;
       int tm, tn, row0;
@@ -286,8 +290,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (!mbar_wait(&tfull_bar[acc], aph, abort_flag, p.wait_hint_ns, p.wait_limit_us)) { atomicExch(p.status, 4); goto done; }
       tc_fence_after();
       if constexpr (ACT != ACT_NONE)
-        epilogue_act<ACT>(p.e, p.act, maps, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn, q, (warp - 2) >> 2, lane);
-      else epilogue_quarter<OUT_F32, !GATHER && !GROUP, STATS, EXTRA && !GROUP>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN, row0, tn * BN, q, lane, t,
+        epilogue_act<ACT>(p.e, p.act, maps, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * NT, row0, tn, q, (warp - 2) >> 2, lane);
+      else epilogue_quarter<OUT_F32, !GATHER && !GROUP, STATS, EXTRA && !GROUP, NT>(p.e, out, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * NT, row0, tn * NT, q, lane, t,
                                                    w / num_tiles, GROUP == GROUP_REDUCE && gr.counts[e] == 0);
       tc_fence_before();
       __syncwarp();
@@ -418,11 +422,11 @@ int launch_gather(const void* A, long long lda, void* D, long long ldd, const vo
 }
 
 template <bool A_MN, bool B_MN, bool OUT_F32, bool GATHER = false, bool REDUCE = false, int GROUP = GROUP_NONE, bool STATS = false, bool EXTRA = true,
-          int ACT = ACT_NONE>
+          int ACT = ACT_NONE, int NT = BN>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, GemmParams p, cudaStream_t stream,
                   const GatherParams* gp = nullptr, long long part_bytes = 0, const GroupParams* grp = nullptr, const ActMaps<ACT>& maps = ActMaps<ACT>{}) {
   static bool configured = false;
-  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS, EXTRA, ACT>;
+  auto kern = gemm_kernel<A_MN, B_MN, OUT_F32, GATHER, REDUCE, GROUP, STATS, EXTRA, ACT, NT>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess) return -4;
     configured = true;
@@ -432,9 +436,9 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  int tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  int tiles = ((p.M + BM - 1) / BM) * ((p.N + NT - 1) / NT);
   if (GROUP == GROUP_REDUCE) tiles *= grp->E;
-  if (p.e.splits > 1 && !split_fits(p.e, tiles, (p.K + BK - 1) / BK, part_bytes)) return -11;
+  if (p.e.splits > 1 && !split_fits(p.e, tiles, (p.K + BK - 1) / BK, part_bytes, 128 * NT)) return -11;
   // the gathering variant always uses every SM: its extra warps carry the transfer
   const int items = tiles * p.e.splits;
   const int grid = (GATHER || items >= g_num_sms) ? g_num_sms : items;
@@ -447,6 +451,12 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMa
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
+template <bool A_MN, bool B_MN, bool OUT_F32, int NT>
+static int launch_narrow(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmParams& p, long long part_bytes, cudaStream_t stream) {
+  if (p.e.R != nullptr || p.e.bias != nullptr) return launch<A_MN, B_MN, OUT_F32, false, false, GROUP_NONE, false, true, ACT_NONE, NT>(ta, tb, td, p, stream, nullptr, part_bytes);
+  return launch<A_MN, B_MN, OUT_F32, false, false, GROUP_NONE, false, false, ACT_NONE, NT>(ta, tb, td, p, stream, nullptr, part_bytes);
+}
+
 }  // namespace mtb
 
 extern "C" {
@@ -454,7 +464,7 @@ extern "C" {
 // D[M,N] = alpha * op(A) * op(B) (+bias) (+R).
 //   a_mn = 0: A is row-major [M, K] (lda >= K);  a_mn = 1: A is row-major [K, M] (lda >= M)
 //   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
-//   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
+//   out_f32: D and R are fp32, else bf16; plus GEMM_N64 or GEMM_N128: tiles of 128 x 64 or 128 x 128 (no statistics). R may alias D (accumulate). bias is bf16 [N] or null.
 //   splits: work items per output tile (ops/gemm_plan.py); more than one needs counters (SPLIT_COUNTERS words, zero before the first
 //   call; launches that may overlap have their own), an epoch that grows with every launch on them, and part, fp32 scratch of part_bytes
 //   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
@@ -464,14 +474,16 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
                      float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && out_f32) || splits < 1) return -10;
+  const int nt = out_f32 & GEMM_N64 ? 64 : out_f32 & GEMM_N128 ? 128 : BN;
+  out_f32 &= ~(GEMM_N64 | GEMM_N128);
+  if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && (out_f32 || nt != BN)) || splits < 1) return -10;
   CUtensorMap ta, tb, td;
   int rc;
   if (a_mn) rc = make_tmap_2d_bf16(&ta, A, M, K, lda, 64, 64);
   else rc = make_tmap_2d_bf16(&ta, A, K, M, lda, BK, BM);
   if (rc) return rc;
   if (b_mn) rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, 64);
-  else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);
+  else rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, nt);
   if (rc) return rc - 10;
   rc = make_tmap_out(&td, D, M, N, ldd, out_f32);
   if (rc) return rc - 20;
@@ -485,7 +497,9 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
       default: return launch<true, true, false, false, false, GROUP_NONE, true>(ta, tb, td, p, stream, nullptr, part_bytes);
     }
   }
-#define GEMM(X, Y, Z) return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, part_bytes) \
+#define GEMM(X, Y, Z) if (nt == 64) return launch_narrow<X, Y, Z, 64>(ta, tb, td, p, part_bytes, stream); \
+                      if (nt == 128) return launch_narrow<X, Y, Z, 128>(ta, tb, td, p, part_bytes, stream); \
+                      return R != nullptr || bias != nullptr ? launch<X, Y, Z>(ta, tb, td, p, stream, nullptr, part_bytes) \
                                                              : launch<X, Y, Z, false, false, GROUP_NONE, false, false>(ta, tb, td, p, stream, nullptr, part_bytes)
   const int sel = (a_mn ? 4 : 0) | (b_mn ? 2 : 0) | (out_f32 ? 1 : 0);
   switch (sel) {
@@ -499,6 +513,18 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
     default: GEMM(true, true, true);
   }
 #undef GEMM
+}
+
+// The same in narrow tiles.
+int mtb200_gemm_n64_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
+                         long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                         float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
+  return mtb200_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 | GEMM_N64, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
+}
+int mtb200_gemm_n128_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
+                         long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                         float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
+  return mtb200_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 | GEMM_N128, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
 }
 
 // A product with an MLP's activation in its epilogue (gemm_act.cuh), on one CTA or, two_cta, on CTA pairs (2: with wide tiles).

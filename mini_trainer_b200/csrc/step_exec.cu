@@ -21,7 +21,7 @@ struct StepSpec {
   int layers, V, R;                  // R: rows that the head runs on, T: all of them
   int tied;
   float logit_alpha, grad_scale;
-  int pair[3], splits[3];            // products of the head: logits, input gradient, weight gradient
+  int form[3], splits[3];            // products of the head: logits, input gradient, weight gradient
   long long off[STEP_PARAMS];        // elements from the start of a block's buffers, -1: the model has no such tensor
   long long off_embed, off_norm, off_bnorm, off_lm;   // in the embedding's buffers; in the head's (tied: off_lm in the embedding's)
 };
@@ -146,8 +146,8 @@ long long run(const StepSpec& s, const StepIO& io, bool measure, cudaStream_t st
   auto product = [&](int which, const void* a, long long lda, int a_mn, const void* w_, long long ldw, int w_mn, void* d, long long ldd, int M, int N, int K,
                      const void* r) {
     const int splits = io.part != nullptr ? s.splits[which] : 1;
-    auto f = s.pair[which] ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
-    return f(a, lda, a_mn, w_, ldw, w_mn, d, ldd, s.pair[which] == 2 ? GEMM2_WIDE : 0, r, r ? ldd : 0, nullptr, M, N, K, s.logit_alpha, splits,
+    auto f = form_on_pairs(s.form[which]) ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
+    return f(a, lda, a_mn, w_, ldw, w_mn, d, ldd, form_flags(s.form[which]), r, r ? ldd : 0, nullptr, M, N, K, s.logit_alpha, splits,
              splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0, splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, nullptr, io.status, st);
   };
   const void* W = at(lm.param, s.off_lm);

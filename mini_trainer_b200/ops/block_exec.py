@@ -21,7 +21,7 @@ NAMES = ("ln1", "bln1", "wqkv", "bqkv", "qn", "kn", "wo", "bo", "ln2", "bln2", "
 
 class Spec(ctypes.Structure):
     _fields_ = [(n, c_int) for n in ("T", "H", "F", "Hq", "Hkv", "D", "gated", "gelu", "layernorm", "qk_norm")] \
-        + [(n, c_float) for n in ("eps", "scale", "alpha")] + [("pair", c_int * GEMMS), ("splits", c_int * GEMMS)] \
+        + [(n, c_float) for n in ("eps", "scale", "alpha")] + [("pair", c_int * GEMMS), ("splits", c_int * GEMMS), ("act_form", c_int)] \
         + [(n, c_int) for n in ("need_out", "attn_form", "fwd_items", "bwd_items", "bwd_splits")]
 
 
@@ -83,6 +83,8 @@ def _spec(ops, cfg, T: int):
                  int((cfg.mlp_act if cfg.mlp_gated else "gelu_tanh") != "silu"), int(cfg.norm_type == "layernorm"), int(cfg.qk_norm), cfg.rms_norm_eps,
                  cfg.attention_scale, cfg.residual_multiplier)
         s.pair[:] = [ops.FORMS[n] for n, _, _ in plans]
+        act, _, _ = ops.product_plan(*products[2], pitches[2], act=True)
+        s.act_form = ops.FORMS[act]
         s.splits[:] = [k for _, k, _ in plans]
         part = [b if k > 1 else 0 for _, k, b in plans]
         if len(ops._block_specs) >= 1024:

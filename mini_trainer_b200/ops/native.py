@@ -54,7 +54,7 @@ P, I, L, F, U = c_void_p, c_int, c_longlong, c_float, c_ulonglong
 class _Sig:
     mtb200_gemm_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, U, P, L, P, P, P]
     mtb200_gemm2_bf16 = [P, L, I, P, L, I, P, L, I, P, L, P, I, I, I, F, I, P, U, P, L, P, P, P]
-    mtb200_gemm2_wide_bf16 = mtb200_gemm2_bf16
+    mtb200_gemm2_wide_bf16 = mtb200_gemm_n64_bf16 = mtb200_gemm_n128_bf16 = mtb200_gemm2_bf16
     mtb200_gemm2_pairs = []
     mtb200_gemm_act = [P, L, P, P, P, P, I, I, I, I, I, I, P, P]
     mtb200_rmsnorm_fwd = [P, P, P, P, F, I, I, P, P]
@@ -154,7 +154,8 @@ def route_topk(logits, k: int, renorm: bool, call=_launch):
 
 class NativeOps:
     name = "native"
-    FORMS = {"mtb200_gemm_bf16": 0, "mtb200_gemm2_bf16": 1, "mtb200_gemm2_wide_bf16": 2}   # as csrc/block_exec.cu and mtb200_gemm_act take them
+    # as csrc/entries.h numbers them
+    FORMS = {"mtb200_gemm_bf16": 0, "mtb200_gemm2_bf16": 1, "mtb200_gemm2_wide_bf16": 2, "mtb200_gemm_n64_bf16": 3, "mtb200_gemm_n128_bf16": 4}
 
     def __init__(self, device, ce_chunk: int = 8192, attention: str | None = None):
         self.device = torch.device(device)
@@ -283,32 +284,37 @@ class NativeOps:
             return None
         return ws, next(self._epoch), part
 
-    def _plan_gemm(self, M, N, K, two_cta, ragged=False):
-        """``(entry point, splits, bytes of partials)`` of a product, from its sizes and whether rows of an operand start off 32 bytes."""
+    def _plan_gemm(self, M, N, K, two_cta, ragged=False, act=False):
+        """``(entry point, splits, bytes of partials)`` of a product, from its sizes and whether rows of an operand start off 32 bytes. ``act``: with an
+        epilogue that only tiles of 256 columns have (activation, statistics)."""
         pairs, one = self.cta_pairs(), True
-        wide = 0
+        wide = narrow = None
         if two_cta if two_cta is not None else self.use_gemm2:
             one = False
         elif two_cta is not None or self.pair_max_flops <= 0:
             pairs = 0
         else:
+            narrow = None if act else gemm_plan.narrow(M, N, K, self.sms, pairs, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
             wide = gemm_plan.wide(M, N, K, ragged, pairs, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
             if 2.0 * M * N * K > self.pair_max_flops:
                 pairs = 0
-        if wide:
+        if narrow:
+            tile, splits = narrow
+            plan = (f"mtb200_gemm_n{tile}_bf16", splits, -(-M // 128) * -(-N // tile) * splits * 128 * tile * 4)
+        elif wide:
             plan = ("mtb200_gemm2_wide_bf16", wide, gemm_plan.partial_bytes(M, N, True, wide))
         else:
             pair, splits = gemm_plan.choose(M, N, K, self.sms, pairs, one, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
             plan = ("mtb200_gemm2_bf16" if pair else "mtb200_gemm_bf16", splits, gemm_plan.partial_bytes(M, N, pair, splits))
         if len(self._gemm_plans) >= 4096:
             self._gemm_plans.clear()
-        self._gemm_plans[(M, N, K, two_cta, ragged)] = plan
+        self._gemm_plans[(M, N, K, two_cta, ragged, act)] = plan
         return plan
 
-    def product_plan(self, M, N, K, pitches):
+    def product_plan(self, M, N, K, pitches, act=False):
         """``_plan_gemm`` of a product whose operands have these leading dimensions (or-ed)."""
         ragged = pitches & 15 != 0
-        return self._gemm_plans.get((M, N, K, None, ragged)) or self._plan_gemm(M, N, K, None, ragged)
+        return self._gemm_plans.get((M, N, K, None, ragged, act)) or self._plan_gemm(M, N, K, None, ragged, act)
 
     def gemm(self, a, a_mn, b, b_mn, out, M, N, K, residual=None, bias=None, tag=None, two_cta=None, alpha=1.0, stats=None):
         """out[M,N] = alpha*A*B (+bias) (+residual). ``a_mn``/``b_mn``: operand stored [K, rows].
@@ -318,8 +324,8 @@ class NativeOps:
         out_f32 = out.dtype == torch.float32
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
         assert residual is None or residual.dtype == out.dtype
-        ragged = bool((a.stride(0) | b.stride(0)) & 15)
-        name, splits, nbytes = self._gemm_plans.get((M, N, K, two_cta, ragged)) or self._plan_gemm(M, N, K, two_cta, ragged)
+        ragged, act = (a.stride(0) | b.stride(0)) & 15 != 0, stats is not None
+        name, splits, nbytes = self._gemm_plans.get((M, N, K, two_cta, ragged, act)) or self._plan_gemm(M, N, K, two_cta, ragged, act)
         st = self._st()
         split = self._split(st, nbytes) if splits > 1 else None
         ws, epoch, part = split or (None, 0, None)
@@ -429,7 +435,8 @@ class NativeOps:
         N = w.shape[0]
         F, code = N // 2 if gated else N, _ACT[fn]
         assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-        name, splits, _ = self.product_plan(T, N, K, x.stride(0) | K)
+        name, _, _ = self.product_plan(T, N, K, x.stride(0) | K, act=True)
+        splits = self.product_plan(T, N, K, x.stride(0) | K)[1]
         # Two launches where one cannot address the weight, and for a product that splits its reduction: 700 x 2048 x 8192 32 us, 43 whole with the
         # activation inside (level at reductions of 4096: 512 x 2048 24.6 and 24.9). No kernel is SiLU alone.
         plain = w.is_contiguous() and K % 8 == 0 and F % 8 == 0

@@ -21,7 +21,7 @@ PARAMS = len(block_exec.NAMES)
 
 class Spec(ctypes.Structure):
     _fields_ = [("block", block_exec.Spec)] + [(n, c_int) for n in ("layers", "V", "R", "tied")] \
-        + [(n, c_float) for n in ("logit_alpha", "grad_scale")] + [("pair", c_int * 3), ("splits", c_int * 3), ("off", c_longlong * PARAMS)] \
+        + [(n, c_float) for n in ("logit_alpha", "grad_scale")] + [("form", c_int * 3), ("splits", c_int * 3), ("off", c_longlong * PARAMS)] \
         + [(n, c_longlong) for n in ("off_embed", "off_norm", "off_bnorm", "off_lm")]
 
 
@@ -74,7 +74,7 @@ def _spec(eng, T: int, R: int):
     s.off_embed, s.off_norm, s.off_bnorm = eng.embed.layout.specs["embed"].offset, head["norm"].offset, head["bnorm"].offset if "bnorm" in head else -1
     s.off_lm = s.off_embed if tied else head["lm_head"].offset
     plans = [ops.product_plan(*m) for m in ((R, V, H, H), (R, H, V, V | H), (V, H, R, V | H))]
-    s.pair[:], s.splits[:] = [ops.FORMS[n] for n, _, _ in plans], [k for _, k, _ in plans]
+    s.form[:], s.splits[:] = [ops.FORMS[n] for n, _, _ in plans], [k for _, k, _ in plans]
     return s, max(fwd_part, bwd_part, *(b if k > 1 else 0 for _, k, b in plans))
 
 

@@ -1559,6 +1559,7 @@ def test_router_kernel_belongs_to_the_native_backend(ops, monkeypatch):
 @pytest.mark.parametrize("K,splits", [(64, 1), (72, 1), (200, 1), (1032, 2), (1032, 4)])
 def test_gemm_wide_tiles_are_exact(ops, M, N, K, splits, monkeypatch):
     from mini_trainer_b200.ops import gemm_plan
+    monkeypatch.setattr(gemm_plan, "narrow", lambda *a: None)
     monkeypatch.setattr(gemm_plan, "wide", lambda M, N, K, *a: splits if 2 * -(-M // 256) * -(-N // 256) * splits <= 1024 else 1)
     monkeypatch.setattr(ops, "_gemm_plans", {})
     names = []
@@ -1588,6 +1589,7 @@ def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypa
     torch.manual_seed(T + F)
     x, w, bias = bf(T, K), bf(2 * F, K, scale=K ** -0.5), bf(2 * F)
     got = []
+    monkeypatch.setattr(gemm_plan, "narrow", lambda *a: None)
     for splits in (1, 0):
         monkeypatch.setattr(gemm_plan, "wide", lambda *a: splits)
         monkeypatch.setattr(gemm_plan, "choose", lambda *a: (True, 1))
@@ -1622,3 +1624,39 @@ def test_grouped_products_in_wide_tiles_match(ops, T, E, k, popular, H, F, monke
     for a, b in zip(*got):
         assert not a.isnan().any() and torch.equal(a, b)
     ops.check_status()
+
+
+# partial last row and column tiles, one tile, a ring that is not filled once and one that is filled several times, split reductions; every sum is exact
+@pytest.mark.parametrize("tile", [64, 128])
+@pytest.mark.parametrize("M,N", [(1, 8), (33, 72), (300, 136), (129, 1000), (1160, 520)])
+@pytest.mark.parametrize("K,splits", [(64, 1), (200, 1), (1600, 1), (1032, 2), (3000, 7)])
+def test_gemm_narrow_tiles_are_exact(ops, tile, M, N, K, splits, monkeypatch):
+    from mini_trainer_b200.ops import gemm_plan
+    monkeypatch.setattr(gemm_plan, "narrow", lambda *a: (tile, splits))
+    monkeypatch.setattr(ops, "_gemm_plans", {})
+    names = []
+    monkeypatch.setattr(ops, "_call", lambda name, *a, call=ops._call, **kw: names.append(name) or call(name, *a, **kw))
+    rows = -(-M // 8) * 8
+    a, b = _ints(rows, K), _ints(N, K)
+    at, bt = a.t().contiguous(), b.t().contiguous()
+    want, res, bias = a.float() @ b.float().t(), _ints(rows, N), _ints(N)
+    for a_mn, b_mn in ((False, False), (False, True), (True, False), (True, True)):
+        m = rows if a_mn else M
+        for dt in (torch.bfloat16, torch.float32):
+            for extra in (False, True):
+                out = torch.full((m, N), float("nan"), dtype=dt, device="cuda")
+                kw = dict(residual=res[:m].to(dt), bias=bias) if extra else {}
+                ops.gemm(at if a_mn else a, a_mn, bt if b_mn else b, b_mn, out, m, N, K, **kw)
+                assert torch.equal(out, (want[:m] + (res[:m].float() + bias.float() if extra else 0.0)).to(dt)), (a_mn, b_mn, dt, extra)
+    assert set(names) == {f"mtb200_gemm_n{tile}_bf16"}
+    ops.check_status()
+
+
+@pytest.mark.parametrize("splits", [2, 3, 7, 16])
+@pytest.mark.parametrize("two_cta", [False, True])
+def test_gemm_every_split_in_tiles_of_256_columns(ops, two_cta, splits, monkeypatch):
+    """Products of these sizes take narrow tiles by themselves."""
+    from mini_trainer_b200.ops import gemm_plan
+    monkeypatch.setattr(gemm_plan, "narrow", lambda *a: None)
+    for M, N, K in ((136, 264, 1024), (300, 520, 7776)):
+        test_gemm_every_split(ops, M, N, K, two_cta, splits, monkeypatch)

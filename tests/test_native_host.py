@@ -257,3 +257,22 @@ def test_gemm_wide_tiles_choice(M, N, K, ragged, splits):
 def test_grouped_products_choice(reduce, rows, E, flops, K, ragged, want):
     from mini_trainer_b200.ops import gemm_plan as G
     assert G.grouped_wide(reduce, rows, E, flops, K, ragged) == want
+
+
+# each at least 10 % faster in this form than in tiles of 256 columns, or (None) in those
+@pytest.mark.parametrize("M,N,K,want", [(640, 512, 3072, (64, 3)), (640, 512, 512, (64, 1)), (3072, 512, 640, (128, 1)), (1200, 1024, 768, (128, 1)), (1249, 1296, 616, (128, 1)),
+                                        (1262, 3272, 512, None), (4096, 1376, 256, None), (1200, 4096, 768, None), (16384, 4096, 4096, None)])
+def test_gemm_narrow_tiles_choice(M, N, K, want):
+    from mini_trainer_b200.ops import gemm_plan as G
+    assert G.narrow(M, N, K, 148, 74, 1024, 1024) == want
+    for units, counted in ((1024, 1024), (8, 1024), (1024, 4)):
+        got = G.narrow(M, N, K, 148, 74, units, counted)
+        if got is not None:
+            tile, s = got
+            tiles = -(-M // 128) * -(-N // tile)
+            assert tiles * s <= 148 and (s == 1 or (tiles <= counted and tiles * s * tile <= units * 256 and 3 * s <= -(-K // 64)))
+    ops = make_ops()
+    assert (ops.product_plan(M, N, K, 0)[0] in ("mtb200_gemm_n64_bf16", "mtb200_gemm_n128_bf16")) == (want is not None)
+    assert ops.product_plan(M, N, K, 0, act=True)[0] in ("mtb200_gemm_bf16", "mtb200_gemm2_bf16", "mtb200_gemm2_wide_bf16")
+    ops.use_gemm2 = True
+    assert ops._plan_gemm(M, N, K, None)[0] == "mtb200_gemm2_bf16"

@@ -77,11 +77,12 @@ def narrow(M: int, N: int, K: int, sms: int, pairs: int, max_units: int, max_cou
 
 # Wide tiles (256 x 512 on a CTA pair) move a quarter less from L2 to the SMs than pairs with 256 x 256. Fitted to 180 products of 0.02 to 1.4 TFLOP,
 # each in a loop of its own of 0.1 s and more, where the clock is already held down by power: a fixed part (launches overlap), a k-block, the rest
-# of an item, a split launch, a partial. Pairs twice: rows that start on 32-byte sectors, and rows that do not (a pitch that is no multiple of 16
+# of an item, a split launch, a partial. Pairs and single CTAs twice: rows that start on 32-byte sectors, and rows that do not (a pitch that is no multiple of 16
 # elements), which cost L2 a request more per 128 bytes; there wide tiles are the faster form by 6 % on average (4285 x 37920 x 3864 1213 -> 1016 us),
 # elsewhere only where the reduction is long enough to hide a wide tile's ends (7001 x 3072 x 12288 458 -> 431 us, but 4099 x 12288 x 2048 179 -> 187).
 _WIDE = (-2.0, 0.85, 4.1, 11.0, 2.9)
 _PAIR_LOOP = ((-4.0, 0.445, 1.6, 5.8, 3.6), (-5.8, 0.51, 2.0, 4.6, 3.4))
+_ONE_LOOP = ((-6.7, 0.467, 2.1, 10.5, 1.8), (-7.5, 0.69, 1.7, 0.1, 3.1))
 WIDE_RAGGED_FLOPS, WIDE_FLOPS, WIDE_K = 3e10, 1e11, 4096
 LONG_FLOPS = 1e12
 
@@ -100,7 +101,7 @@ def _loop_cost(tiles: int, kblocks: int, units: int, max_units: int, workers: in
     return best + fixed, splits
 
 
-def wide(M: int, N: int, K: int, ragged: bool, pairs: int, max_units: int, max_counted: int) -> int:
+def wide(M: int, N: int, K: int, ragged: bool, sms: int, pairs: int, max_units: int, max_counted: int) -> int:
     """Splits of the product on wide tiles, or 0 where the other kernels are the faster. ``ragged``: rows of an operand do not start on 32 bytes.
     Products of more than ``LONG_FLOPS`` run at the power cap, where what is moved costs clock: there wide tiles give 1300 to 1410 TFLOP/s, pairs 1170 to
     1375 and single CTAs 1180 to 1325 (16384 tokens of an 8B model)."""
@@ -111,6 +112,8 @@ def wide(M: int, N: int, K: int, ragged: bool, pairs: int, max_units: int, max_c
     most = max_units if units <= max_counted else 0
     cost, splits = _loop_cost(rows * -(-N // 512), kblocks, units, most, pairs, _WIDE, True)
     other, _ = _loop_cost(rows * cols, kblocks, units, most, pairs, _PAIR_LOOP[ragged], False)
+    ones = -(-M // 128) * cols
+    other = min(other, _loop_cost(ones, kblocks, ones, max_units if ones <= max_counted else 0, sms, _ONE_LOOP[ragged], False)[0])
     return splits if cost <= other * (1.1 if flops > LONG_FLOPS else 1.0) else 0
 
 

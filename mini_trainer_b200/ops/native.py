@@ -295,7 +295,7 @@ class NativeOps:
             pairs = 0
         else:
             narrow = None if act else gemm_plan.narrow(M, N, K, self.sms, pairs, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
-            wide = gemm_plan.wide(M, N, K, ragged, pairs, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
+            wide = gemm_plan.wide(M, N, K, ragged, self.sms, pairs, _SPLIT_UNITS, _SPLIT_COUNTERS // 4)
             if 2.0 * M * N * K > self.pair_max_flops:
                 pairs = 0
         if narrow:

@@ -235,13 +235,13 @@ def test_attention_choices_agree_with_the_full_estimate():
 # (M, N, K, rows that start off 32 bytes, splits on wide tiles, 0: another kernel): each at least 3 % faster that way in a loop of its own
 @pytest.mark.parametrize("M,N,K,ragged,splits", [(16384, 4096, 28672, False, 1), (28672, 4096, 16384, False, 1), (7001, 3072, 12288, False, 1), (5987, 1536, 17920, False, 1),
                                                  (4285, 37920, 3864, True, 1), (2534, 2520, 5768, True, 1), (4090, 14832, 1912, True, 1),
-                                                 (5987, 17920, 1536, False, 0), (10324, 1728, 2112, False, 0), (5587, 3328, 7872, False, 0), (2457, 1760, 5264, True, 0)])
+                                                 (5987, 17920, 1536, False, 0), (10324, 1728, 2112, False, 0), (5587, 3328, 7872, False, 0), (2457, 1760, 5264, True, 0), (1384, 3216, 7946, True, 0)])
 def test_gemm_wide_tiles_choice(M, N, K, ragged, splits):
     from mini_trainer_b200.ops import gemm_plan as G
-    assert G.wide(M, N, K, ragged, 74, 1024, 1024) == splits
-    assert G.wide(M, N, K, ragged, 0, 1024, 1024) == 0
+    assert G.wide(M, N, K, ragged, 148, 74, 1024, 1024) == splits
+    assert G.wide(M, N, K, ragged, 148, 0, 1024, 1024) == 0
     for units, counted in ((1024, 1024), (64, 1024), (1024, 4)):
-        s = G.wide(M, N, K, ragged, 74, units, counted)
+        s = G.wide(M, N, K, ragged, 148, 74, units, counted)
         u = 2 * -(-M // 256) * -(-N // 256)
         assert s <= 1 or (u <= counted and u * s <= units and 4 * s <= -(-K // 64))
     ops = make_ops()

@@ -14,7 +14,7 @@
 // P V and the next S of B. K and V are loaded once per pair. A row belongs to one thread, so nothing is exchanged between
 // threads (two threads per row with their maxima exchanged through shared memory measured 1.92 ms below). P is handed over in
 // two halves of 64 keys, so the first half's products run under the second half's exponentials.
-// 1 x 16384 tokens, 32/8 heads, D = 128: 1.65 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64: 64 us (one tile per CTA, two
+// 1 x 16384 tokens, 32/8 heads, D = 128: 1.65 ms; 41 samples, 12 345 tokens, 16/4 heads, D = 64: 53 us (one tile per CTA, two
 // threads per row: 1.94 ms and 94 us). Launches with few pairs are faster in that other form (attention_fwd_one.cu);
 // a long sequence at D = 64 is level (1 x 16384, 32/8 heads: 1.54 ms there, 1.50 here).
 //
@@ -24,11 +24,16 @@
 //
 // A row's reference maximum only moves (and its accumulator is only rescaled) when the running maximum grew by more than
 // 2^8, which is exact: the same reference is used throughout. Only the last key tile of a query tile touches the causal
-// diagonal and is masked.
+// diagonal: its code is its own, a warp leaves out the pieces of 32 keys that none of its rows see, and masks one.
+//
+// What a unit costs beside its key tiles is what short samples are bound by: 3.7 us at D = 64, where a key tile of the pair takes 0.8. Of that, the
+// unit's row of the table and the divisions that find it took 0.7, masking 0.6, storing the output 0.7 (1.4 to 2.9 at D = 128). Without them
+// (before, now): 148 samples of 128 tokens, 16/4 heads, 36.5 -> 30.4 us at D = 64 and 57.6 -> 42.6 at 128, 37 of 1024 163 -> 149 and 232 -> 188,
+// 41 of 12 to 1489 tokens 55.9 -> 53; 1 x 16384 level.
 //
 // Masked scores are -inf. The exponentials that run on the special-function unit turn them into exact zeros;
 // the quarter that runs on the FMA pipe (ex2_fma2) clamps its argument at -126 and returns about 1e-38 instead, so
-// on the diagonal tile one masked key in four adds a term of that size to a row sum that is at least 1 (the row's
+// on the diagonal tile one masked key in four of the masked piece adds a term of that size to a row sum that is at least 1 (the row's
 // maximum contributes exp2(0)) and to P: 38 orders of magnitude below either, no effect on out or lse.
 //
 // Outputs: out [T, Hq*D] bf16 and lse [Hq, T] fp32 (natural log, scaled scores), as needed by
@@ -52,7 +57,7 @@ constexpr int POLY = 4;            // every POLY-th exponential pair runs on the
 constexpr int ATT_THREADS = 384;   // three warpgroups: TMA / MMA, softmax of A, softmax of B
 // Registers per thread after the split; over the three warpgroups they add up to at most the 3 x 168 of the launch.
 // A softmax thread holds the 128 scores of its row.
-constexpr int ATT_REGS_IO = 72, ATT_REGS_SOFTMAX = 216;
+constexpr int ATT_REGS_IO = 88, ATT_REGS_SOFTMAX = 208;
 static_assert(ATT_REGS_IO + 2 * ATT_REGS_SOFTMAX <= 3 * 168, "register split");
 
 template <int D>
@@ -61,7 +66,8 @@ struct AttFwdSmem {
   static constexpr int OFF_Q = 0;                    // A, B
   static constexpr int OFF_K = 2 * TILE;             // 2 stages
   static constexpr int OFF_V = 4 * TILE;             // 2 stages
-  static constexpr int OFF_BAR = 6 * TILE;
+  static constexpr int OFF_OUT = 6 * TILE;           // staged output: a box of 32 rows x 64 columns for each softmax warp
+  static constexpr int OFF_BAR = OFF_OUT + 8 * 4096;
   static constexpr int TOTAL = OFF_BAR + 256 + 1024;
 };
 
@@ -77,41 +83,63 @@ struct AttFwdParams {
   int* status;
 };
 
+struct AttTrue { static constexpr bool value = true; };
+struct AttFalse { static constexpr bool value = false; };
+
 // One unit of work: the two query tiles of a pair. n = key tiles (0: no such tile).
 struct AttWork {
   int seq_start, seq_len, hk, h[2], q0[2], n[2];
   __device__ __forceinline__ int tiles() const { return n[0] > n[1] ? n[0] : n[1]; }
 };
 
-// The `round`-th unit of this CTA; false when there is none left. A row of the table that does not lie inside the packed
-// batch yields a unit without tiles, which every role skips.
-__device__ __forceinline__ bool att_work(const AttFwdParams& p, int round, AttWork& w) {
-  const int per_item = p.row_pairs ? p.Hq : p.Hq / 2;
-  const int total = p.n_items * per_item;
-  const int u = round * static_cast<int>(gridDim.x) + ((round & 1) ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
-  if (round * static_cast<int>(gridDim.x) >= total) return false;
+// Where the next unit of this CTA is in the table. A unit's row is fetched while the unit before it is worked on: read when it is needed, it cost
+// every role 1300 to 3000 clocks, a fifth of a unit of one key tile.
+// x / d for 0 <= x < 2^31 and d > 0, with m = (2^32 - 1) / d: the product is at most one too small.
+struct AttDiv {
+  unsigned m;
+  int d;
+  __device__ __forceinline__ explicit AttDiv(int div) : m(0xffffffffu / static_cast<unsigned>(div)), d(div) {}
+  __device__ __forceinline__ int operator()(int x) const {
+    const int q = static_cast<int>(__umulhi(static_cast<unsigned>(x), m));
+    return x - q * d >= d ? q + 1 : q;
+  }
+};
+struct AttNext {
+  int item, x;                      // item: -1 for none (the last round may be partial in either direction)
+  int seq_start, seq_len, q0;
+  bool more;                        // whether there is such a round at all
+};
+__device__ __forceinline__ void att_fetch(const AttFwdParams& p, const AttDiv& per_item, int round, AttNext& f) {
+  const int total = p.n_items * per_item.d, grid = static_cast<int>(gridDim.x);
+  f.more = round * grid < total;
+  const int u = round * grid + ((round & 1) ? grid - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
+  f.item = -1;
+  if (!f.more || u >= total) return;
+  f.item = per_item(u);
+  f.x = u - f.item * per_item.d;
+  f.seq_start = p.plan[f.item * 3 + 0]; f.seq_len = p.plan[f.item * 3 + 1]; f.q0 = p.plan[f.item * 3 + 2];
+}
+// The unit that was fetched. A row of the table that does not lie inside the packed batch yields a unit without tiles, which every role skips.
+__device__ __forceinline__ void att_unit(const AttFwdParams& p, const AttDiv& group, const AttNext& f, AttWork& w) {
   w.n[0] = w.n[1] = 0;
-  if (u >= total) return true;   // the last round may be partial in either direction
-  const int item = u / per_item, x = u - item * per_item;
-  w.seq_start = p.plan[item * 3 + 0]; w.seq_len = p.plan[item * 3 + 1];
-  const int q0 = p.plan[item * 3 + 2];
+  if (f.item < 0) return;
+  w.seq_start = f.seq_start; w.seq_len = f.seq_len;
+  const int q0 = f.q0;
   if (w.seq_start < 0 || w.seq_len <= 0 || q0 < 0 || q0 >= w.seq_len || static_cast<long long>(w.seq_start) + w.seq_len > p.T) {
     atomicExch(p.status, 61);   // reported, not dereferenced
-    return true;
+    return;
   }
-  const int G = p.Hq / p.Hkv;
-  w.h[0] = p.row_pairs ? x : 2 * x;
-  w.h[1] = p.row_pairs ? x : 2 * x + 1;
-  w.hk = w.h[0] / G;
+  w.h[0] = p.row_pairs ? f.x : 2 * f.x;
+  w.h[1] = p.row_pairs ? f.x : 2 * f.x + 1;
+  w.hk = group(w.h[0]);
   w.q0[0] = q0;
   w.q0[1] = p.row_pairs ? q0 + ATT_B : q0;
   w.n[0] = q0 / ATT_B + 1;
   w.n[1] = w.q0[1] < w.seq_len ? w.q0[1] / ATT_B + 1 : 0;
-  return true;
 }
 
 template <int D>
-__global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, AttFwdParams p) {
+__global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmap_out, AttFwdParams p) {
   using L = AttFwdSmem<D>;
   constexpr int KB = D / 64;  // 64-element (128 B) column blocks of a D-wide row
   extern __shared__ uint8_t smem_raw[];
@@ -139,12 +167,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     *abort_flag = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap);
+    tma_prefetch_desc(&tmap_out);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   pdl_wait();   // nothing so far has touched global memory
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  const AttDiv per_item(p.row_pairs ? p.Hq : p.Hq / 2), group(p.Hq / p.Hkv);
   const uint32_t tmem_base = *tmem_slot;   // S of A and B at columns 0 and 128, O at 256 and 256 + D
 
   if (warp < 4) {
@@ -153,8 +183,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
       // ------------------------------------------------------------------ TMA producer
       if (elect_one()) {
         AttWork w;
+        AttNext f;
         uint32_t units = 0, kt = 0;   // units with tiles so far; key tiles so far
-        for (int round = 0; att_work(p, round, w); ++round) {
+        att_fetch(p, per_item, 0, f);
+        for (int round = 1; f.more; ++round) {
+          att_unit(p, group, f, w);
+          att_fetch(p, per_item, round, f);
           const int n = w.tiles();
           if (n == 0) continue;
           if (units > 0 && !mbar_wait(q_free, (units - 1) & 1, abort_flag)) { atomicExch(p.status, 11); goto done; }
@@ -210,9 +244,13 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
           }
         };
         AttWork w;
+        AttNext f;
         uint32_t units = 0, kt = 0;
         uint32_t cnt[2] = {0, 0};   // tiles of each group so far
-        for (int round = 0; att_work(p, round, w); ++round) {
+        att_fetch(p, per_item, 0, f);
+        for (int round = 1; f.more; ++round) {
+          att_unit(p, group, f, w);
+          att_fetch(p, per_item, round, f);
           const int n = w.tiles();
           if (n == 0) continue;
           if (!mbar_wait(q_full, units & 1, abort_flag)) { atomicExch(p.status, 12); goto done; }
@@ -263,32 +301,39 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t ts = tmem_base + g * ATT_B + lane_addr, to = tmem_base + 2 * ATT_B + g * D + lane_addr;
     const float sl2 = p.scale * 1.4426950408889634f;
+    const int wq = warp & 3;
+    uint8_t* box = smem + L::OFF_OUT + (warp - 4) * 4096;
+    const float2 sl2v = make_float2(sl2, sl2);
     uint32_t cnt = 0;
     AttWork w;
-    for (int round = 0; att_work(p, round, w); ++round) {
+    AttNext f;
+    att_fetch(p, per_item, 0, f);
+    for (int round = 1; f.more; ++round) {
+      att_unit(p, group, f, w);
       const int n = g == 0 ? w.n[0] : w.n[1];
-      if (n == 0) continue;
+      if (n == 0) { att_fetch(p, per_item, round, f); continue; }
       const int qpos = (g == 0 ? w.q0[0] : w.q0[1]) + r;
       float m_ref = -INFINITY, l = 0.f;
-      for (int j = 0; j < n; ++j, ++cnt) {
-        if (!mbar_wait(&s_full[g], cnt & 1, abort_flag)) { atomicExch(p.status, 17); goto done; }
-        tc_fence_after();
+      // One key tile. DIAG: the last one, on the causal diagonal. Of its keys, 32 at a time, the warp's rows see all before piece `wq`, the first
+      // lane + 1 of that piece, and none behind it: nothing is computed for those.
+      auto key_tile = [&](auto diag, int j) -> bool {
+        constexpr bool DIAG = decltype(diag)::value;
         // the row of S is read from tensor memory once and stays in registers for the maximum and the exponentials
         uint32_t sv[4][32];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, sv[c]);
+        for (int c = 0; c < 4; ++c)
+          tmem_ld_32x32(ts + c * 32, sv[c]);
         tmem_ld_wait();
-        if (j == n - 1) {
-          const int kb = j * ATT_B;
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (kb + c * 32 + i > qpos) sv[c][i] = 0xff800000u;   // -inf
-        }
         float mc[4];   // four independent chains
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          mc[c] = -INFINITY;
+          if (DIAG && c > wq) continue;
+          if (DIAG && c == wq) {
+#pragma unroll
+            for (int i = 1; i < 32; ++i)
+              if (i > lane) sv[c][i] = 0xff800000u;   // -inf
+          }
           mc[c] = fmaxf(__uint_as_float(sv[c][0]), __uint_as_float(sv[c][1]));
 #pragma unroll
           for (int i = 2; i < 32; i += 2) mc[c] = fmax3(mc[c], __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
@@ -303,7 +348,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
           l *= factor;
         }
         if (j > 0 && __any_sync(0xffffffffu, rescale)) {   // O must be complete through tile j-1 before it is rescaled
-          if (!mbar_wait(&pv_done[g], (cnt - 1) & 1, abort_flag)) { atomicExch(p.status, 18); goto done; }
+          if (!mbar_wait(&pv_done[g], (cnt - 1) & 1, abort_flag)) return false;
           tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < D / 16; ++c) {
@@ -317,18 +362,23 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
         }
         // probabilities -> bf16 P over the columns of S, row sum; exp2(-inf) = 0 masks
         const float mo = (m_ref == -INFINITY) ? 0.f : m_ref * sl2;
-        const float2 sl2v = make_float2(sl2, sl2), nmo = make_float2(-mo, -mo);
+        const float2 nmo = make_float2(-mo, -mo);
         float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t pk[16];
+          if (!DIAG || c <= wq) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            // scale and shift two scores with one packed FMA; of every POLY pairs one runs its exponentials on the FMA pipe
-            const float2 x = ffma2(make_float2(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])), sl2v, nmo);
-            const float2 e = (i % POLY == POLY - 1) ? ex2_fma2(x) : make_float2(ex2_mufu(x.x), ex2_mufu(x.y));
-            l2[i & 1] = fadd2(l2[i & 1], e);
-            pk[i] = pack_bf16(e.x, e.y);
+            for (int i = 0; i < 16; ++i) {
+              // scale and shift two scores with one packed FMA; of every POLY pairs one runs its exponentials on the FMA pipe
+              const float2 x = ffma2(make_float2(__uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1])), sl2v, nmo);
+              const float2 e = (i % POLY == POLY - 1) ? ex2_fma2(x) : make_float2(ex2_mufu(x.x), ex2_mufu(x.y));
+              l2[i & 1] = fadd2(l2[i & 1], e);
+              pk[i] = pack_bf16(e.x, e.y);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[i] = 0u;
           }
           tmem_st_32x16(ts + c * 16, pk);
           if (c & 1) {   // half of the keys: their products start under the other half's exponentials
@@ -339,11 +389,27 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
           }
         }
         l += (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
+        return true;
+      };
+      for (int j = 0; j < n; ++j, ++cnt) {
+        if (!mbar_wait(&s_full[g], cnt & 1, abort_flag)) { atomicExch(p.status, 17); goto done; }
+        tc_fence_after();
+        bool ok;
+        if (j == n - 1) {
+          att_fetch(p, per_item, round, f);   // here, so that its registers are not held through the other tiles
+          ok = key_tile(AttTrue{}, j);
+        } else {
+          ok = key_tile(AttFalse{}, j);
+        }
+        if (!ok) { atomicExch(p.status, 18); goto done; }
       }
-      // epilogue: O / l -> out, lse. The next unit's first P V overwrites O only after this thread has handed over its P.
+      // epilogue: O / l -> out, lse. The next unit's first P V overwrites O only after this thread has handed over its P. A warp whose rows all exist
+      // stages 64 columns at a time for a tensor store: the rows of a tile are far apart, and 16-byte stores of 32 of them at a time took 1300 clocks
+      // per tile at D = 64 and 2700 to 5400 at 128.
       if (!mbar_wait(&pv_done[g], (cnt - 1) & 1, abort_flag)) { atomicExch(p.status, 19); goto done; }
       tc_fence_after();
       const bool ok = qpos < w.seq_len;
+      const bool whole = qpos - lane + 31 < w.seq_len;   // uniform over the warp
       const float inv = 1.f / l;
       const int h = g == 0 ? w.h[0] : w.h[1];
       const long long tok = static_cast<long long>(w.seq_start) + qpos;
@@ -353,14 +419,28 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
         uint32_t v[2][32];
         tmem_ld_32x32(to + c * 32, v[0]);
         tmem_ld_32x32(to + c * 32 + 32, v[1]);
+        if (whole) {   // the box is free once the last store has read it
+          if (lane == 0) bulk_wait_read<0>();
+          __syncwarp();
+        }
         tmem_ld_wait();
-        if (ok) {
+        if (whole || ok) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
-            float f[8];
+            float o[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(v[k >> 2][(k & 3) * 8 + i]) * inv;
-            *reinterpret_cast<uint4*>(orow + c * 32 + k * 8) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[k >> 2][(k & 3) * 8 + i]) * inv;
+            const uint4 d = make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
+            if (whole) *reinterpret_cast<uint4*>(box + lane * 128 + ((k ^ (lane & 7)) << 4)) = d;
+            else *reinterpret_cast<uint4*>(orow + c * 32 + k * 8) = d;
+          }
+        }
+        if (whole) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tmap_out, box, h * D + c * 32, w.seq_start + qpos);
+            bulk_commit();
           }
         }
       }
@@ -368,6 +448,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_fwd_kernel(const __grid_c
     }
   }
 done:
+  if (warp >= 4 && lane == 0) bulk_wait_read<0>();   // before the shared memory goes away
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -377,7 +458,7 @@ done:
 }
 
 template <int D>
-static int launch_fwd(const CUtensorMap& tm, const AttFwdParams& p, cudaStream_t st) {
+static int launch_fwd(const CUtensorMap& tm, const CUtensorMap& to, const AttFwdParams& p, cudaStream_t st) {
   static bool configured = false;
   static int sms = 0;
   auto kern = attn_fwd_kernel<D>;
@@ -390,7 +471,7 @@ static int launch_fwd(const CUtensorMap& tm, const AttFwdParams& p, cudaStream_t
   }
   const long long units = static_cast<long long>(p.n_items) * (p.row_pairs ? p.Hq : p.Hq / 2);
   if (units > (1 << 30)) return -10;
-  launch_pdl(kern, static_cast<int>(units < sms ? units : sms), ATT_THREADS, AttFwdSmem<D>::TOTAL, st, tm, p);
+  launch_pdl(kern, static_cast<int>(units < sms ? units : sms), ATT_THREADS, AttFwdSmem<D>::TOTAL, st, tm, to, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -404,8 +485,11 @@ extern "C" int mtb200_attn_fwd(const void* qkv, long long ld, void* out, long lo
   if (n_items <= 0 || T <= 0) return 0;
   if ((D != 64 && D != 128) || Hkv <= 0 || Hq % Hkv || ld % 8 || ldo % 8 || (!row_pairs && (Hq / Hkv) % 2)) return -10;
   CUtensorMap tm;
-  const int rc = make_tmap_2d_bf16(&tm, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
+  CUtensorMap to;
+  int rc = make_tmap_2d_bf16(&tm, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
   if (rc) return rc;
+  rc = make_tmap_2d_bf16(&to, out, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(ldo), 64, 32);
+  if (rc) return rc - 10;
   AttFwdParams p{reinterpret_cast<__nv_bfloat16*>(out), ldo, lse, plan, n_items, T, Hq, Hkv, row_pairs, scale, status};
-  return D == 128 ? launch_fwd<128>(tm, p, st) : launch_fwd<64>(tm, p, st);
+  return D == 128 ? launch_fwd<128>(tm, to, p, st) : launch_fwd<64>(tm, to, p, st);
 }

@@ -27,7 +27,11 @@
 // 128B-swizzled so the staging stores are free of bank conflicts); a small kernel rounds the accumulator to bf16 afterwards.
 // Four warps of their own drain, one more issues the reduces, so the softmax warps see nothing of dQ.
 //
-// Rows past the end of the sequence contribute nothing: a query's lse is staged as +infinity, a key's scores are masked.
+// Rows past the end of the sequence contribute nothing: a query's lse is staged as +infinity, a key's dS is zero.
+//
+// With short samples a CTA has few iterations, and its first loads and its stores count: the loads go out before tensor memory is allocated, and dK and dV
+// leave by tensor stores. 148 samples of 128 tokens, 16/4 heads: 106 -> 102 us at D = 64, 193 -> 182 at 128 (all passes); 37 of 1024 492 -> 482, 879 -> 871.
+// The rest of it is dQ's accumulator, which is written, added to and read in fp32: 78 MB of it in 101 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -72,6 +76,8 @@ struct AttBwdParams {
   float* dq_acc;        // [T, Hq*D] fp32, zeroed by attn_delta_kernel
   const int* plan;      // [n_items, 3] = seq_start, seq_len, k0
   int T, Hq, Hkv;
+  int G;                // Hq / Hkv
+  unsigned hkv_inv;     // (2^32 - 1) / Hkv
   int splits;           // CTAs that share a key block's query heads
   float* ws;            // splits > 1: fp32 partials of dK and dV
   unsigned long long* counters;   // splits > 1: one arrival counter per (key block, warp); last_arrival in gemm_epilogue.cuh
@@ -84,7 +90,7 @@ struct AttBwdParams {
 template <int D>
 __global__ void __launch_bounds__(AB_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constant__ CUtensorMap tm_do,
-                const __grid_constant__ CUtensorMap tm_dq, AttBwdParams p) {
+                const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dkv, AttBwdParams p) {
   using L = AttBwdSmem<D>;
   constexpr int KB = D / 64;
   extern __shared__ uint8_t smem_raw[];
@@ -115,10 +121,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
 
   pdl_wait();   // the work table comes first
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int unit = blockIdx.x / p.splits, sub = blockIdx.x - unit * p.splits;
-  const int item = unit / p.Hkv, hk = unit % p.Hkv;
-  const int G = p.Hq / p.Hkv;
-  const int h_first = hk * G + G * sub / p.splits, heads = G * (sub + 1) / p.splits - G * sub / p.splits;
+  const int unit = p.splits == 1 ? blockIdx.x : blockIdx.x / p.splits, sub = blockIdx.x - unit * p.splits;
+  int item = static_cast<int>(__umulhi(static_cast<unsigned>(unit), p.hkv_inv));   // unit / Hkv, or one less
+  if (unit - item * p.Hkv >= p.Hkv) ++item;
+  const int hk = unit - item * p.Hkv;
+  const int G = p.G;
+  const int h_first = hk * G + (p.splits == 1 ? 0 : G * sub / p.splits), heads = p.splits == 1 ? G : G * (sub + 1) / p.splits - G * sub / p.splits;
   const int seq_start = p.plan[item * 3 + 0], seq_len = p.plan[item * 3 + 1], k0 = p.plan[item * 3 + 2];
   const int jblk = k0 / AB_B;
   const int nq = (seq_len + AB_B - 1) / AB_B;      // query blocks of the sequence
@@ -137,9 +145,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     for (int b = 0; b < 2; ++b) { mbar_init(&q_full[b], 1); mbar_init(&q_free[b], 1); mbar_init(&stat_full[b], 1); mbar_init(&stat_free[b], 8); }
     *abort_flag = 0;
     fence_mbar_init();
-    tma_prefetch_desc(&tm_qkv);
-    tma_prefetch_desc(&tm_do);
+    // the first loads go out before anything else is set up
+    mbar_arrive_expect_tx(kv_full, 2 * L::TILE);
+    mbar_arrive_expect_tx(&q_full[0], L::TILE);
+    mbar_arrive_expect_tx(do_full, L::TILE);
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) {
+      tma_load_2d(smem + L::OFF_K + kb * 16384, &tm_qkv, kv_full, (p.Hq + hk) * D + kb * 64, seq_start + k0);
+      tma_load_2d(smem + L::OFF_Q + kb * 16384, &tm_qkv, &q_full[0], h_first * D + kb * 64, seq_start + jblk * AB_B);
+      tma_load_2d(smem + L::OFF_V + kb * 16384, &tm_qkv, kv_full, (p.Hq + p.Hkv + hk) * D + kb * 64, seq_start + k0);
+      tma_load_2d(smem + L::OFF_DO + kb * 16384, &tm_do, do_full, h_first * D + kb * 64, seq_start + jblk * AB_B);
+    }
     tma_prefetch_desc(&tm_dq);
+    tma_prefetch_desc(&tm_dkv);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
@@ -156,14 +174,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       if (elect_one()) {
-        mbar_arrive_expect_tx(kv_full, 2 * L::TILE);
-#pragma unroll
-        for (int kb = 0; kb < KB; ++kb) {
-          tma_load_2d(smem + L::OFF_K + kb * 16384, &tm_qkv, kv_full, (p.Hq + hk) * D + kb * 64, seq_start + k0);
-          tma_load_2d(smem + L::OFF_V + kb * 16384, &tm_qkv, kv_full, (p.Hq + p.Hkv + hk) * D + kb * 64, seq_start + k0);
-        }
         int h = h_first, i = jblk;
-        for (int it = 0; it < n_iters; ++it) {
+        if (++i == nq) { i = jblk; ++h; }
+        for (int it = 1; it < n_iters; ++it) {   // the first iteration's tiles have been asked for above
           const int b = it & 1;
           if (it > 1 && !mbar_wait(&q_free[b], ((it - 2) >> 1) & 1, abort_flag)) { atomicExch(p.status, 21); goto done; }
           mbar_arrive_expect_tx(&q_full[b], L::TILE);
@@ -357,13 +370,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         tmem_ld_32x32(ts, sv[0]);
         tmem_ld_32x32(ts + 32, sv[1]);
         tmem_ld_wait();
-        if (i == jblk || k0 + AB_B > seq_len) {   // diagonal block or last key block: out-of-range entries get P = 0
-          const int q0 = i * AB_B + half * 64;
+        if (i == jblk) {   // diagonal block: of the queries, 32 at a time, a warp's keys are seen by none before piece q, by those from the lane on in it
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc)
+          for (int cc = 0; cc < 2; ++cc) {
+            if (half * 2 + cc <= q) {
 #pragma unroll
-            for (int x = 0; x < 32; ++x)
-              if (kpos > q0 + cc * 32 + x || kpos >= seq_len) sv[cc][x] = 0xff800000u;   // exp2(-inf) = 0
+              for (int x = 0; x < 32; ++x)
+                if (half * 2 + cc < q || lane > x) sv[cc][x] = 0xff800000u;   // exp2(-inf) = 0
+            }
+          }
         }
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
@@ -407,6 +422,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
           dk[x >> 1] = pack_bf16(s0.x, s0.y);
           dk[(x >> 1) + 1] = pack_bf16(s1.x, s1.y);
         }
+        if (k0 + AB_B > seq_len) {   // last key block: keys past the sequence give nothing to dQ (their rows of dK and dV are not stored)
+#pragma unroll
+          for (int x = 0; x < 16; ++x) dk[x] = kpos < seq_len ? dk[x] : 0u;
+        }
         tmem_st_32x16(tp + cc * 16, dk);
 #pragma unroll
         for (int g = 0; g < 4; ++g)
@@ -423,28 +442,43 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     if (!mbar_wait(all_done, 0, abort_flag)) { atomicExch(p.status, 29); goto done; }
     tc_fence_after();
     const bool ok = kpos < seq_len;
+    const bool whole = kpos - lane + 31 < seq_len;   // uniform over the warp
     __nv_bfloat16* rowp = p.dqkv + (static_cast<long long>(seq_start) + kpos) * p.ldq;
-    auto store = [&](int which, int c, const float (&f)[32]) {   // 32 columns of this thread's row of dK (0) or dV (1)
-      if (!ok) return;
-      __nv_bfloat16* o = rowp + (which == 0 ? (p.Hq + hk) * D : (p.Hq + p.Hkv + hk) * D) + c * 32;
+    // A warp has 64 columns of one gradient (D = 64: dK or dV) or of both (D = 128), in pieces of 32; rows that all exist leave by tensor stores, staged
+    // where Q was (stored 16 bytes at a time to rows that are far apart, they took 3500 clocks per CTA at D = 64 and 9000 at 128).
+    constexpr int PIECES = D / 32, BOXES = D / 64;
+    constexpr int PART = PIECES * 1024;   // floats of a warp's partial
+    uint8_t* box = smem + L::OFF_Q + (warp - 4) * BOXES * 4096;
+    auto gradient = [&](int x) { return D == 64 ? half : x >> 1; };                          // 0: dK, 1: dV
+    auto column = [&](int x) { return D == 64 ? x * 32 : half * 64 + (x & 1) * 32; };
+    auto store = [&](int x, const float (&f)[32]) {   // piece x of this thread's row
+      const int col = (gradient(x) == 0 ? p.Hq + hk : p.Hq + p.Hkv + hk) * D + column(x);
 #pragma unroll
-      for (int g = 0; g < 4; ++g)
-        *reinterpret_cast<uint4*>(o + g * 8) = make_uint4(pack_bf16(f[g * 8], f[g * 8 + 1]), pack_bf16(f[g * 8 + 2], f[g * 8 + 3]),
-                                                          pack_bf16(f[g * 8 + 4], f[g * 8 + 5]), pack_bf16(f[g * 8 + 6], f[g * 8 + 7]));
+      for (int g = 0; g < 4; ++g) {
+        const uint4 d = make_uint4(pack_bf16(f[g * 8], f[g * 8 + 1]), pack_bf16(f[g * 8 + 2], f[g * 8 + 3]),
+                                   pack_bf16(f[g * 8 + 4], f[g * 8 + 5]), pack_bf16(f[g * 8 + 6], f[g * 8 + 7]));
+        if (whole) *reinterpret_cast<uint4*>(box + (x >> 1) * 4096 + lane * 128 + ((((x & 1) * 4 + g) ^ (lane & 7)) << 4)) = d;
+        else if (ok) *reinterpret_cast<uint4*>(rowp + col + g * 8) = d;
+      }
+      if (whole && (x & 1)) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tm_dkv, box + (x >> 1) * 4096, col - 32, seq_start + kpos);
+          bulk_commit();
+        }
+      }
     };
-    constexpr int CH = D / 64;            // 32-column pieces per thread and gradient
-    constexpr int PART = 2 * CH * 1024;   // floats of a warp's partial
     float* base = p.ws + (static_cast<long long>(unit) * p.splits * 8 + (warp - 4)) * PART + lane * 4;   // split s: + s * 8 * PART
 #pragma unroll 1
-    for (int x = 0; x < 2 * CH; ++x) {
-      const int which = x / CH, c = half * CH + x % CH;
+    for (int x = 0; x < PIECES; ++x) {
       uint32_t v[32];
-      tmem_ld_32x32((which == 0 ? t_dk : t_dv) + lane_addr + c * 32, v);
+      tmem_ld_32x32((gradient(x) == 0 ? t_dk : t_dv) + lane_addr + column(x), v);
       tmem_ld_wait();
       float f[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-      if (p.splits == 1) store(which, c, f);
+      if (p.splits == 1) store(x, f);
       else {   // lane-interleaved 16-byte pieces: every access is one contiguous 512 bytes
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -461,7 +495,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
       if (last) {
         __threadfence();
 #pragma unroll 1
-        for (int x = 0; x < 2 * CH; ++x) {
+        for (int x = 0; x < PIECES; ++x) {
           float f[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) f[j] = 0.f;
@@ -473,11 +507,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
               f[4 * j] += t.x; f[4 * j + 1] += t.y; f[4 * j + 2] += t.z; f[4 * j + 3] += t.w;
             }
           }
-          store(x / CH, half * CH + x % CH, f);
+          store(x, f);
         }
         if (lane == 0) *counter = 0;
       }
     }
+    if (lane == 0) bulk_wait_read<0>();   // before the shared memory goes away
   }
 done:
   tc_fence_before();
@@ -545,14 +580,14 @@ __global__ void __launch_bounds__(256) attn_dq_store_kernel(const float* __restr
 }
 
 template <int D>
-static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const AttBwdParams& p, int n_items, cudaStream_t st) {
+static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const CUtensorMap& d, const AttBwdParams& p, int n_items, cudaStream_t st) {
   static bool configured = false;
   auto kern = attn_bwd_kernel<D>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem<D>::TOTAL) != cudaSuccess) return -4;
     configured = true;
   }
-  launch_pdl(kern, n_items * p.Hkv * p.splits, AB_THREADS, AttBwdSmem<D>::TOTAL, st, a, b, c, p);
+  launch_pdl(kern, n_items * p.Hkv * p.splits, AB_THREADS, AttBwdSmem<D>::TOTAL, st, a, b, c, d, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -569,19 +604,21 @@ extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, l
   if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8 || lddo % 8 || ldq % 8 || splits < 1 || splits > Hq / Hkv) return -10;
   const long long units = static_cast<long long>(n_items) * Hkv;
   if (splits > 1 && (part == nullptr || counters == nullptr || units * 8 > SPLIT_COUNTERS || splits * units * 2 * AB_B * D * 4 > part_bytes)) return -11;
-  CUtensorMap tq, tdo, tdq;
+  CUtensorMap tq, tdo, tdq, tdkv;
   int rc = make_tmap_2d_bf16(&tq, qkv, static_cast<uint64_t>(ld), static_cast<uint64_t>(T), static_cast<uint64_t>(ld), 64, 128);
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tdo, dout, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(lddo), 64, 128);
   if (rc) return rc - 10;
   rc = make_tmap_2d_f32(&tdq, dq_acc, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(Hq) * D, 32, 128);
   if (rc) return rc - 20;
+  rc = make_tmap_2d_bf16(&tdkv, dqkv, (static_cast<uint64_t>(Hq) + 2 * Hkv) * D, static_cast<uint64_t>(T), static_cast<uint64_t>(ldq), 64, 32);
+  if (rc) return rc - 30;
   const int per_block = 2 * 256 / (D / 8);
   launch_pdl(attn_delta_kernel, static_cast<unsigned>((static_cast<long long>(T) * Hq + per_block - 1) / per_block), 256, 0, st,
       reinterpret_cast<const __nv_bfloat16*>(out), ldo, reinterpret_cast<const __nv_bfloat16*>(dout), lddo, delta, dq_acc, T, Hq, D);
-  AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, splits,
+  AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, Hq / Hkv, 0xffffffffu / static_cast<unsigned>(Hkv), splits,
                  part, counters, epoch, scale, status};
-  rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, p, n_items, st);
+  rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, tdkv, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, tdkv, p, n_items, st);
   if (rc) return rc;
   launch_pdl(attn_dq_store_kernel, dim3(static_cast<unsigned>(T), (Hq * D / 8 + 255) / 256), 256, 0, st, dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, T, Hq * D);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;

@@ -1001,6 +1001,36 @@ def test_attention_backward_every_division(ops, D, hq, hkv, lens, monkeypatch):
     ops.check_status()
 
 
+# rows held in registers (up to 32768 columns, 1024 to a warp) and the first that are not; fewer rows than blocks, and several to a block
+@pytest.mark.parametrize("R,V", [(1, 8), (700, 1024), (300, 1032), (1300, 5000), (400, 16392), (1, 32768), (310, 32768), (5, 32776)])
+@pytest.mark.parametrize("in_place", [True, False])
+def test_cross_entropy_rows(ops, R, V, in_place):
+    torch.manual_seed(R + V)
+    ld = V + 16
+    lg = bf(R, ld, scale=4)
+    if R > 1:
+        lg[0, V // 2:V] = float("-inf")
+    lg[-1, :V // 2] = torch.finfo(torch.bfloat16).min
+    tg = torch.randint(0, V, (R,), device="cuda")
+    tg[0], tg[-1] = 0, V - 1   # not where a row is masked
+    tg[1::7] = -100
+    x = lg[:, :V].double()
+    lse = torch.logsumexp(x, 1)
+    want = lse - x.gather(1, tg.clamp_min(0)[:, None])[:, 0]
+    grad = (x - lse[:, None]).exp()
+    grad.scatter_add_(1, tg.clamp_min(0)[:, None], torch.full((R, 1), -1.0, device="cuda", dtype=torch.double))
+    want[tg == -100], grad[tg == -100] = 0, 0
+    kept = lg[:, V:].clone()
+    out, loss = lg if in_place else torch.full_like(lg, 7.0), torch.full((R,), 7.0, device="cuda")
+    rest = kept if in_place else torch.full_like(kept, 7.0)
+    ops._call("mtb200_ce_fwd_bwd", lg.data_ptr(), ld, 1, 0, tg.data_ptr(), loss.data_ptr(), out.data_ptr(), ld, R, V, 0.5, -100, ops._st())
+    # fp32 sums of V positive terms, each thread's and warp's in turn, and the rounding of a logarithm and a logit of up to 32
+    assert (loss - want).abs().max() < 1e-5
+    assert ((out[:, :V].double() - 0.5 * grad).abs() <= 0.5 * (2 ** -8 * grad.abs() + 2e-6)).all()   # one rounding to bf16
+    assert torch.equal(out[:, V:], rest)
+    ops.check_status()
+
+
 # logits whose product leaves the statistics and logits whose rows are read for them, in one chunk and in several
 @pytest.mark.parametrize("T,H,V", [(130, 1536, 17008), (130, 1528, 17008), (130, 1536, 16384), (70, 64, 520)])
 def test_linear_ce_with_and_without_statistics(ops, T, H, V, monkeypatch):

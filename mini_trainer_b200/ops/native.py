@@ -576,13 +576,13 @@ class NativeOps:
             return self._fa_bwd(dout, qkv, out, lse, cu_seqlens, max_seqlen, hq, hkv, d, scale)
         dqkv = torch.empty_like(qkv)
         plan, splits, nbytes = self._cached(cu_host, ("bwd", hq, hkv, d)) or self._plan_attention_bwd(cu_host, hq, hkv, d)
-        delta = torch.empty(hq, T, dtype=torch.float32, device=self.device)
-        dq_acc = torch.empty(T, hq * d, dtype=torch.float32, device=self.device)
+        scratch = torch.empty(hq * T * (d + 1), dtype=torch.float32, device=self.device)   # dQ's accumulator [T, hq * d] and delta [hq, T]: one allocation
+        dq_acc = scratch.data_ptr()
         st = self._st()
         split = self._split(st, nbytes) if splits > 1 else None
         ws, epoch, part = split or (None, 0, None)
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
-                   dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), delta.data_ptr(), dq_acc.data_ptr(),
+                   dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), dq_acc + 4 * hq * T * d, dq_acc,
                    plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits if split else 1, _ptr(ws), epoch, _ptr(part), 4 * part.numel() if split else 0, scale,
                    self.status.data_ptr(), st, n=3)
         return dqkv

@@ -1001,8 +1001,8 @@ def test_attention_backward_every_division(ops, D, hq, hkv, lens, monkeypatch):
     ops.check_status()
 
 
-# rows held in registers (up to 32768 columns, 1024 to a warp) and the first that are not; fewer rows than blocks, and several to a block
-@pytest.mark.parametrize("R,V", [(1, 8), (700, 1024), (300, 1032), (1300, 5000), (400, 16392), (1, 32768), (310, 32768), (5, 32776)])
+# rows held in registers (up to 32768 columns, 1024 to a warp) and longer ones; fewer rows than blocks, and several to a block
+@pytest.mark.parametrize("R,V", [(1, 8), (700, 1024), (300, 1032), (1300, 5000), (400, 16392), (1, 32768), (310, 32768), (5, 32776), (150, 65544)])
 @pytest.mark.parametrize("in_place", [True, False])
 def test_cross_entropy_rows(ops, R, V, in_place):
     torch.manual_seed(R + V)

@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(EW_THREADS) swiglu_bwd_kernel(__nv_bfloat16* d
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     if constexpr (ACT == 0) {
-      const float sig = __fdividef(1.f, 1.f + __expf(-fg[i]));
+      const float sig = __fdividef(1.f, 1.f + exp_ftz(-fg[i]));
       og[i] = fd[i] * fu[i] * sig * (1.f + fg[i] * (1.f - sig));
       ou[i] = fd[i] * fg[i] * sig;
     } else {
@@ -849,11 +849,6 @@ __device__ __forceinline__ void load8(const LogitT* p, float (&f)[8]) {
   }
 }
 
-// e^x = 2^(x log2 e) in two instructions. Results below 2^-126 are flushed to zero, which nothing here can tell: they are summed beside a one. These kernels are
-// bound by instructions where not by memory; against __expf, rows in registers 3069 x 32000 80 -> 76 us; below 2048 x 40000 87 -> 77, x 65536 129 -> 114,
-// 1500 x 151936 229 -> 215, and with statistics 3720 x 49152 132 -> 127, x 151936 358 -> 355.
-__device__ __forceinline__ float ce_exp(float x) { return ex2_mufu(x * 1.4426950408889634f); }
-
 template <typename LogitT, bool STATS>
 __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, long long ld, const float2* __restrict__ stats,
                                                          const long long* __restrict__ targets, float* __restrict__ loss,
@@ -876,8 +871,8 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
     const int tiles = (V + 255) / 256;
     for (int c = threadIdx.x; c < tiles; c += blockDim.x) {
       const float2 t = stats[row * tiles + c];
-      if (t.x > m) { s *= ce_exp(m - t.x); m = t.x; }
-      s += t.y * ce_exp(t.x - m);
+      if (t.x > m) { s *= exp_ftz(m - t.x); m = t.x; }
+      s += t.y * exp_ftz(t.x - m);
     }
   }
   else for (int c = threadIdx.x * 8; c < V; c += blockDim.x * 8) {
@@ -886,12 +881,12 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
     float mx = v[0];
 #pragma unroll
     for (int i = 1; i < 8; ++i) mx = fmaxf(mx, v[i]);
-    if (mx > m) { s *= ce_exp(m - mx); m = mx; }
+    if (mx > m) { s *= exp_ftz(m - mx); m = mx; }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s += ce_exp(v[i] - m);
+    for (int i = 0; i < 8; ++i) s += exp_ftz(v[i] - m);
   }
   const float gm = block_max(m, red);
-  s *= ce_exp(m - gm);
+  s *= exp_ftz(m - gm);
   const float gs = block_sum(s, red);
   const float lse = gm + logf(gs);
   if (threadIdx.x == 0) {
@@ -913,7 +908,7 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
       if (k == 1 && !two) break;
       const int c = c0 + k * step;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) o[k][i] = ce_exp(o[k][i] - gm) * inv;
+      for (int i = 0; i < 8; ++i) o[k][i] = exp_ftz(o[k][i] - gm) * inv;
       if (tgt >= c && tgt < c + 8) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) if (tgt - c == i) o[k][i] -= grad_scale;   // no dynamic index: the array stays in registers
@@ -967,19 +962,19 @@ __global__ void __launch_bounds__(1024, 1) ce_row_kernel(const __nv_bfloat16* lo
     for (int k = 0; k < CE_ROW_VECS; ++k)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        e[k][i] = ce_exp(e[k][i] - base);
+        e[k][i] = exp_ftz(e[k][i] - base);
         s += e[k][i];
       }
     // maximum and sum of the row from the threads' own; a sum beside a maximum of -infinity is zero, or NaN where a logit is
     float gm = warp_max(m);
-    float gs = warp_sum(m == -INFINITY ? s : s * ce_exp(m - gm));
+    float gs = warp_sum(m == -INFINITY ? s : s * exp_ftz(m - gm));
     if (lane == 0) red[par][warp] = make_float2(gm, gs);
     __syncthreads();   // and the target's logit has been read before any thread overwrites the row
     const float2 w = red[par][lane];
     gm = warp_max(w.x);
-    gs = warp_sum(w.x == -INFINITY ? w.y : w.y * ce_exp(w.x - gm));
+    gs = warp_sum(w.x == -INFINITY ? w.y : w.y * exp_ftz(w.x - gm));
     if (threadIdx.x == 0) loss[row] = ignored ? 0.f : gm + logf(gs) - t;
-    const float scale = ce_exp(base - gm) * (grad_scale / gs);
+    const float scale = exp_ftz(base - gm) * (grad_scale / gs);
     __nv_bfloat16* dr = dlogits + row * ldd;
 #pragma unroll
     for (int k = 0; k < CE_ROW_VECS; ++k) {

@@ -40,7 +40,7 @@ __device__ __forceinline__ uint4* box_piece(uint8_t* box, int lane, int i) {
   return reinterpret_cast<uint4*>(box + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4));
 }
 __device__ __forceinline__ float2 sigmoid2(float2 x) {   // 1 / (1 + exp(-x))
-  return make_float2(__fdividef(1.f, 1.f + __expf(-x.x)), __fdividef(1.f, 1.f + __expf(-x.y)));
+  return make_float2(__fdividef(1.f, 1.f + exp_ftz(-x.x)), __fdividef(1.f, 1.f + exp_ftz(-x.y)));
 }
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
 // The factor s of f(x) = x * s, for two x.

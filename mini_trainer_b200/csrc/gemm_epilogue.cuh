@@ -43,12 +43,15 @@ struct RowStats {
   float m = -INFINITY, s = 0.f;
 };
 
-__device__ __forceinline__ void row_stats8(RowStats& st, uint4 o) {   // eight bf16 values
+// Eight bf16 values. Exponentials in two instructions (exp_ftz): of 3 us per tile that the statistics take where nothing hides them, a third
+// (logits and gradient of 8000 x 32000 x 1536: 848 -> 792 us).
+template <typename Stats>
+__device__ __forceinline__ void row_stats8(Stats& st, uint4 o) {
   const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y), r2 = unpack_bf16(o.z), r3 = unpack_bf16(o.w);
   const float mx = fmaxf(fmax3(fmaxf(r0.x, r0.y), r1.x, r1.y), fmax3(fmaxf(r2.x, r2.y), r3.x, r3.y));
-  if (mx > st.m) { st.s *= __expf(st.m - mx); st.m = mx; }
-  st.s += __expf(r0.x - st.m) + __expf(r0.y - st.m) + __expf(r1.x - st.m) + __expf(r1.y - st.m) + __expf(r2.x - st.m) +
-          __expf(r2.y - st.m) + __expf(r3.x - st.m) + __expf(r3.y - st.m);
+  if (mx > st.m) { st.s *= exp_ftz(st.m - mx); st.m = mx; }
+  st.s += exp_ftz(r0.x - st.m) + exp_ftz(r0.y - st.m) + exp_ftz(r1.x - st.m) + exp_ftz(r1.y - st.m) + exp_ftz(r2.x - st.m) +
+          exp_ftz(r2.y - st.m) + exp_ftz(r3.x - st.m) + exp_ftz(r3.y - st.m);
 }
 
 // Output staging. A row of a tile belongs to one thread, so storing it directly sends 32 half-sectors to 32 rows with every
@@ -128,7 +131,9 @@ __device__ __forceinline__ void epilogue_row32(const EpiParams& p, float (&f)[32
       o.x = pack_bf16(f[j], f[j + 1]); o.y = pack_bf16(f[j + 2], f[j + 3]);
       o.z = pack_bf16(f[j + 4], f[j + 5]); o.w = pack_bf16(f[j + 6], f[j + 7]);
       *reinterpret_cast<uint4*>(srow + (((part * 4 + (j >> 3)) ^ (lane & 7)) << 4)) = o;
-      if (STATS && col0 + j < p.N) row_stats8(st, o);   // of the values as stored
+      if constexpr (STATS) {
+        if (col0 + j < p.N) row_stats8(st, o);   // of the values as stored
+      }
     }
   }
 }

@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(32 * GATHER_WARPS) moe_gather_kernel(const bf1
 template <int ACT>
 __device__ __forceinline__ void act_and_grad(float g, float& a, float& da) {
   if constexpr (ACT == 0) {   // SiLU
-    const float sig = __fdividef(1.f, 1.f + __expf(-g));
+    const float sig = __fdividef(1.f, 1.f + exp_ftz(-g));
     a = g * sig;
     da = sig * (1.f + g * (1.f - sig));
   } else {                    // tanh-approximated GELU

@@ -341,6 +341,11 @@ __device__ __forceinline__ float ex2_mufu(float x) {
   return y;
 }
 
+// e^x = 2^(x log2 e) in two instructions. Results below 2^-126 are flushed to zero: for sums beside a term of at least one, which cannot tell. In the
+// cross-entropy, which is bound by instructions where not by memory, against __expf: rows in registers 3069 x 32000 80 -> 76 us; longer ones 2048 x 40000
+// 87 -> 77, x 65536 129 -> 114, 1500 x 151936 229 -> 215, and with statistics 3720 x 49152 132 -> 127, x 151936 358 -> 355. Gate activations: level.
+__device__ __forceinline__ float exp_ftz(float x) { return ex2_mufu(x * 1.4426950408889634f); }
+
 // 2^x on the FMA pipe (128 per clock per SM): x = n + f with n the nearest integer, 2^f by a cubic
 // fitted on [-0.5, 0.5] (maximum relative error 1.0e-4, a fortieth of a bf16 ulp), 2^n by an integer
 // add into the exponent field. Inputs below -126 (masked scores are -inf) give about 1e-38, not 0.
@@ -371,14 +376,14 @@ __device__ __forceinline__ float2 ex2_fma2(float2 x) {
 
 // The factor of the tanh-approximated GELU, 0.5 * (1 + tanh(sqrt(2 / pi) * (g + 0.044715 g^3))) = sigmoid(2 * that argument).
 __device__ __forceinline__ float gelu_gate(float g) {
-  return __fdividef(1.f, 1.f + __expf(-1.5957691216057308f * (g + 0.044715f * g * g * g)));
+  return __fdividef(1.f, 1.f + exp_ftz(-1.5957691216057308f * (g + 0.044715f * g * g * g)));
 }
 
 // Activation of an MLP and its derivative. ACT 0: SiLU, 1: tanh-approximated GELU.
 template <int ACT>
 __device__ __forceinline__ float glu_act(float g) {
   if constexpr (ACT == 0) {
-    return __fdividef(g, 1.f + __expf(-g));
+    return __fdividef(g, 1.f + exp_ftz(-g));
   } else {
     return g * gelu_gate(g);
   }
@@ -387,7 +392,7 @@ __device__ __forceinline__ float glu_act(float g) {
 template <int ACT>
 __device__ __forceinline__ float glu_act_grad(float g) {
   if constexpr (ACT == 0) {
-    const float sig = __fdividef(1.f, 1.f + __expf(-g));
+    const float sig = __fdividef(1.f, 1.f + exp_ftz(-g));
     return sig * (1.f + g * (1.f - sig));
   } else {
     const float s = gelu_gate(g);

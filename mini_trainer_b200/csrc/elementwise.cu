@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
     for (int c = threadIdx.x; c < tiles; c += blockDim.x) {
       const float2 t = stats[row * tiles + c];
       if (t.x > m) { s *= exp_ftz(m - t.x); m = t.x; }
-      s += t.y * exp_ftz(t.x - m);
+      s += t.y * exp_ftz(t.x - (m == -INFINITY ? 0.f : m));
     }
   }
   else for (int c = threadIdx.x * 8; c < V; c += blockDim.x * 8) {
@@ -882,8 +882,9 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
 #pragma unroll
     for (int i = 1; i < 8; ++i) mx = fmaxf(mx, v[i]);
     if (mx > m) { s *= exp_ftz(m - mx); m = mx; }
+    const float base = m == -INFINITY ? 0.f : m;   // nothing but masked columns so far
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s += exp_ftz(v[i] - m);
+    for (int i = 0; i < 8; ++i) s += exp_ftz(v[i] - base);
   }
   const float gm = block_max(m, red);
   s *= exp_ftz(m - gm);
@@ -1529,7 +1530,11 @@ int mtb200_ce_fwd_bwd(const void* logits, long long ld, int logits_bf16, const f
                       void* dlogits, long long ldd, int R, int V, float grad_scale, long long ignore_index, cudaStream_t st) {
   if (R <= 0) return 0;
   if (V % 8 || ld % 8 || ldd % 8 || (stats && !logits_bf16)) return -10;
-#define CE(T, S) launch_pdl(ce_fwd_bwd_kernel<T, S>, R, 1024, 0, st, (const T*)logits, ld, stats, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index)
+  // Four rows at a time on an SM hide each other's reductions better than two, when there are rows enough to go round: with statistics 8000 x 17008
+  // 151 -> 108 us, x 32000 194 -> 167, 3720 x 49152 127 -> 119, x 151936 level; without 4000 x 40000 152 -> 133, x 57344 200 -> 187, but 2048 x 65536
+  // 114 -> 117 and x 128256 222 -> 262, where the rows at work on no longer stay in L2. 900 x 32000 25 -> 23, 600 level, 200 6.4 -> 9.3.
+  const int per_row = logits_bf16 && V <= 57344 && R >= 6 * num_sms() ? 512 : 1024;
+#define CE(T, S) launch_pdl(ce_fwd_bwd_kernel<T, S>, R, per_row, 0, st, (const T*)logits, ld, stats, targets, loss, (bf16*)dlogits, ldd, V, grad_scale, ignore_index)
   const int threads = cdiv(V, CE_ROW_VECS * 8 * 32) * 32;
   if (logits_bf16 && !stats && threads <= 1024) {
     const int most = num_sms() * (1024 / threads);   // what 64 registers a thread let an SM hold

@@ -773,8 +773,8 @@ class NativeOps:
     @staticmethod
     def ce_wants_stats(V: int, H: int) -> bool:
         # The statistics save the cross-entropy a read of the row, which only costs where a row does not stay on the SM, and take the
-        # epilogue 3 us per tile, which only hides behind longer reductions. Logits and gradient together, with and without: 3720 x 151936 x 1536 1541
-        # and 1790 us, 8000 x 32000 x 2048 975 and 1010, x 1536 792 and 805, but x 1024 700 and 614; 8000 x 512 x 64 90 and 16.
+        # epilogue 3 us per tile, which only hides behind longer reductions. Logits and gradient together, with and without: 3720 x 151936 x 1536 1505
+        # and 1777 us, 8000 x 32000 x 2048 899 and 1002, x 1536 744 and 821, but x 1024 702 and 622; 8000 x 512 x 64 50 and 15.
         return V > 16384 and H >= 1536
 
     def linear_ce(self, x, w, targets, grad_scale, dw_out, accumulate_dw=False, ignore_index=-100, logit_scale=1.0):

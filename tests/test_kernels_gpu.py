@@ -1001,10 +1001,13 @@ def test_attention_backward_every_division(ops, D, hq, hkv, lens, monkeypatch):
     ops.check_status()
 
 
-# rows held in registers (up to 32768 columns, 1024 to a warp) and longer ones; fewer rows than blocks, and several to a block
-@pytest.mark.parametrize("R,V", [(1, 8), (700, 1024), (300, 1032), (1300, 5000), (400, 16392), (1, 32768), (310, 32768), (5, 32776), (150, 65544)])
+# rows held in registers (up to 32768 columns, 1024 to a warp), longer ones and ones with statistics, by blocks of 1024 threads and of 512; fewer rows than
+# blocks, and several to a block
+@pytest.mark.parametrize("R,V,stats", [(1, 8, False), (700, 1024, False), (300, 1032, False), (1300, 5000, False), (400, 16392, False), (1, 32768, False),
+                                       (310, 32768, False), (5, 32776, False), (150, 65544, False), (888, 32776, False), (887, 5000, True), (888, 5000, True),
+                                       (888, 57344, True), (3, 296, True)])
 @pytest.mark.parametrize("in_place", [True, False])
-def test_cross_entropy_rows(ops, R, V, in_place):
+def test_cross_entropy_rows(ops, R, V, stats, in_place):
     torch.manual_seed(R + V)
     ld = V + 16
     lg = bf(R, ld, scale=4)
@@ -1021,9 +1024,14 @@ def test_cross_entropy_rows(ops, R, V, in_place):
     grad.scatter_add_(1, tg.clamp_min(0)[:, None], torch.full((R, 1), -1.0, device="cuda", dtype=torch.double))
     want[tg == -100], grad[tg == -100] = 0, 0
     kept = lg[:, V:].clone()
+    st = None
+    if stats:
+        tiles = torch.nn.functional.pad(x, (0, -V % 256), value=float("-inf")).view(R, -1, 256)
+        top = tiles.amax(-1)
+        st = torch.stack([top, (tiles - top.clamp_min(-1e38)[..., None]).exp().sum(-1)], -1).float().contiguous()
     out, loss = lg if in_place else torch.full_like(lg, 7.0), torch.full((R,), 7.0, device="cuda")
     rest = kept if in_place else torch.full_like(kept, 7.0)
-    ops._call("mtb200_ce_fwd_bwd", lg.data_ptr(), ld, 1, 0, tg.data_ptr(), loss.data_ptr(), out.data_ptr(), ld, R, V, 0.5, -100, ops._st())
+    ops._call("mtb200_ce_fwd_bwd", lg.data_ptr(), ld, 1, st.data_ptr() if stats else 0, tg.data_ptr(), loss.data_ptr(), out.data_ptr(), ld, R, V, 0.5, -100, ops._st())
     # fp32 sums of V positive terms, each thread's and warp's in turn, and the rounding of a logarithm and a logit of up to 32
     assert (loss - want).abs().max() < 1e-5
     assert ((out[:, :V].double() - 0.5 * grad).abs() <= 0.5 * (2 ** -8 * grad.abs() + 2e-6)).all()   # one rounding to bf16

@@ -817,6 +817,16 @@ __global__ void __launch_bounds__(EW_THREADS) embedding_bwd_scan_kernel(__nv_bfl
   }
 }
 
+// Zeros into n 16-byte pieces and m fp32, one launch that starts under its predecessor's tail. Zeros and rows together, two
+// memsets before: 480 rows into 640 x 512 9.1 -> 3.1 us, 3069 into 4096 x 256 9.2 -> 5.5, 3720 into 6000 x 1536 14.4 -> 8.3, 12000 into 16384 x 4096 56 -> 51.
+__global__ void __launch_bounds__(EW_THREADS) zero_rows_kernel(uint4* out, long long n, float* vout, int m) {
+  pdl_trigger();
+  pdl_wait();
+  const long long first = static_cast<long long>(blockIdx.x) * EW_THREADS + threadIdx.x, step = static_cast<long long>(gridDim.x) * EW_THREADS;
+  for (long long i = first; i < n; i += step) out[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (long long i = first; i < m; i += step) vout[i] = 0.f;
+}
+
 // out[rows[r]] = src[r] for rows of H columns, and the same for a vector of fp32.
 __global__ void __launch_bounds__(128) scatter_rows_kernel(const long long* __restrict__ rows, const __nv_bfloat16* __restrict__ src, __nv_bfloat16* __restrict__ out,
                                                           const float* __restrict__ vsrc, float* __restrict__ vout, int H, int T, int* status) {
@@ -1520,7 +1530,10 @@ int mtb200_embedding_bwd_scan(void* dw, const long long* ids, const void* dx, in
 int mtb200_scatter_rows(const long long* rows, const void* src, void* out, const float* vsrc, float* vout, int R, int H, int T, int* status, cudaStream_t st) {
   if (T <= 0 || R < 0) return 0;
   if (H % 8) return -10;
-  if (cudaMemsetAsync(out, 0, static_cast<size_t>(T) * H * 2, st) != cudaSuccess || cudaMemsetAsync(vout, 0, static_cast<size_t>(T) * 4, st) != cudaSuccess) return -5;
+  const long long pieces = static_cast<long long>(T) * H / 8, blocks = (pieces + 4 * EW_THREADS - 1) / (4 * EW_THREADS);
+  if (pieces > (8 << 20)) {   // above 128 MB the memsets are the faster ones: 64000 x 4096 179 us, 187 by the kernel
+    if (cudaMemsetAsync(out, 0, pieces * 16, st) != cudaSuccess || cudaMemsetAsync(vout, 0, static_cast<size_t>(T) * 4, st) != cudaSuccess) return -5;
+  } else launch_pdl(zero_rows_kernel, static_cast<int>(blocks < num_sms() * 8 ? (blocks > 0 ? blocks : 1) : num_sms() * 8), EW_THREADS, 0, st, (uint4*)out, pieces, vout, T);
   if (R > 0) launch_pdl(scatter_rows_kernel, R, 128, 0, st, rows, (const bf16*)src, (bf16*)out, vsrc, vout, H, T, status);
   return launch_ok();
 }

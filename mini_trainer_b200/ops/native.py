@@ -362,7 +362,7 @@ class NativeOps:
         out = torch.empty(T, H, dtype=src.dtype, device=self.device)
         v = torch.empty(T, dtype=torch.float32, device=self.device)
         self._call("mtb200_scatter_rows", rows.data_ptr(), src.data_ptr(), out.data_ptr(), vec.data_ptr(), v.data_ptr(), R, H, T,
-                   self.status.data_ptr(), self._st())
+                   self.status.data_ptr(), self._st(), n=2)
         return out, v
 
     # -- rmsnorm ----------------------------------------------------------------------

@@ -394,6 +394,26 @@ def test_minibatch_in_one_call_is_the_engine_launch_by_launch(family, lens, monk
     assert abs(n1 - n2) <= 5e-3 * n2 and all(torch.isfinite(m).all() for m in m1)
 
 
+# groups without gaps between their tensors, which are written whole, and with gaps, which are zeroed
+@pytest.mark.parametrize("hidden", [256, 264])
+@pytest.mark.parametrize("tied", [False, True])
+def test_minibatch_in_one_call_leaves_nothing_of_the_gradient_buffers(hidden, tied):
+    from mini_trainer_b200.models.config import ModelConfig
+    from mini_trainer_b200.ops.native import NativeOps
+    cfg = ModelConfig(model_type="llama", vocab_size=520, hidden_size=hidden, intermediate_size=392, num_hidden_layers=2, num_attention_heads=4,
+                      num_key_value_heads=2, head_dim=64, tie_word_embeddings=tied)
+    got = []
+    for dirt in (0.0, float("nan")):
+        eng = ShardedEngine(cfg, "cuda:0", NativeOps("cuda:0"), optim=OptimConfig())
+        eng.init_random(seed=5, std=0.05)
+        eng._eg_full.fill_(dirt)
+        eng._hg_full.fill_(dirt)
+        assert eng.ops.step_forward_backward(eng, D.make_packed_batch(make_mb([300, 17], 520), "cuda:0"), 0.01) is not None
+        got.append([g.gacc.clone() for g in eng.groups])
+        eng.ops.check_status()
+    assert all((a - b).norm() <= 5e-3 * a.norm() for a, b in zip(*got))   # up to the order of the attention backward's sums
+
+
 def test_what_one_call_does_not_cover_goes_launch_by_launch(monkeypatch):
     """Options that ask for the schedule itself, minibatches that are too large for it, and no room for the workspace."""
     from mini_trainer_b200.ops import block_exec, step_exec

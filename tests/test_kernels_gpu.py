@@ -1236,6 +1236,17 @@ def test_rows_scattered_into_zeros(ops, T, R, H):
     ops.check_status()
 
 
+# the largest output that the kernel zeroes (8 M pieces of 16 bytes) and the first that memsets do
+@pytest.mark.parametrize("T", [16384, 16385])
+def test_rows_scattered_into_many_zeros(ops, T):
+    rows, src, vec = torch.tensor([T - 1, 3], device="cuda"), bf(2, 4096), torch.randn(2, device="cuda")
+    out, v = ops.scatter_rows(rows, src, vec, T)
+    assert torch.equal(out[rows], src) and torch.equal(v[rows], vec)
+    out[rows], v[rows] = 0, 0
+    assert not out.any() and not v.any()
+    ops.check_status()
+
+
 FAMILIES = {"llama": {}, "qwen2": dict(attention_bias=True), "qwen3": dict(qk_norm=True),
             "starcoder2": dict(norm_type="layernorm", mlp_gated=False, attention_bias=True, mlp_bias=True, hidden_act="gelu_pytorch_tanh"),
             "gemma-like": dict(model_type="llama", hidden_act="gelu_pytorch_tanh"), "granite": dict(residual_multiplier=0.22, attention_multiplier=0.02)}

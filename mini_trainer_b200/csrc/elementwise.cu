@@ -901,8 +901,10 @@ __global__ void __launch_bounds__(1024) ce_fwd_bwd_kernel(const LogitT* logits, 
   const float gs = block_sum(s, red);
   const float lse = gm + logf(gs);
   if (threadIdx.x == 0) {
-    float t;
-    if constexpr (sizeof(LogitT) == 2) t = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(lr)[tgt]); else t = lr[tgt];
+    float t = NAN;   // of a target that is no column
+    if (tgt >= 0 && tgt < V) {
+      if constexpr (sizeof(LogitT) == 2) t = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(lr)[tgt]); else t = lr[tgt];
+    }
     loss[row] = lse - t;
   }
   __syncthreads();   // the target logit has been read before any thread overwrites the row

@@ -1039,6 +1039,42 @@ def test_cross_entropy_rows(ops, R, V, stats, in_place):
     ops.check_status()
 
 
+# rows held in registers, rows that are read twice, rows with statistics, fp32 logits
+CE_FORMS = [(264, "rows"), (32776, "rows"), (264, "statistics"), (520, "fp32")]
+
+
+def _ce_forms(ops, lg, ld, V, form, tg):
+    """``(loss, gradient)`` of ``lg[:, :V]`` (a scale of 1, -100 ignored) from the form of the kernel that is named."""
+    R = lg.shape[0]
+    st = 0
+    if form == "statistics":
+        tiles = torch.nn.functional.pad(lg[:, :V].double(), (0, -V % 256), value=float("-inf")).view(R, -1, 256)
+        top = tiles.amax(-1)
+        st = torch.stack([top, (tiles - top.clamp_min(-1e38)[..., None]).exp().sum(-1)], -1).float().contiguous()
+    src = lg.float() if form == "fp32" else lg
+    out, loss = torch.full_like(lg, 7.0), torch.full((R,), 7.0, device="cuda")
+    ops._call("mtb200_ce_fwd_bwd", src.data_ptr(), ld, int(form != "fp32"), st if isinstance(st, int) else st.data_ptr(), tg.data_ptr(), loss.data_ptr(),
+              out.data_ptr(), ld, R, V, 1.0, -100, ops._st())
+    return loss, out[:, :V]
+
+
+@pytest.mark.parametrize("V,form", CE_FORMS)
+def test_cross_entropy_of_a_target_that_is_no_column(ops, V, form):
+    """Nothing outside the row is read for it: the loss is NaN, the gradient that of no target, and other rows are what they are without it."""
+    torch.manual_seed(V)
+    lg = bf(6, V + 16, scale=4)
+    tg = torch.tensor([3, V, V - 1, -1, 1 << 40, 0], device="cuda")
+    loss, grad = _ce_forms(ops, lg, V + 16, V, form, tg)
+    x = lg[:, :V].double()
+    want = torch.softmax(x, 1)
+    for r in (0, 2, 5):
+        want[r, tg[r]] -= 1
+    none = torch.tensor([False, True, False, True, True, False], device="cuda")
+    assert loss[none].isnan().all() and (loss - torch.nn.functional.cross_entropy(x, tg.clamp(0, V - 1), reduction="none"))[~none].abs().max() < 1e-5
+    assert ((grad.double() - want).abs() <= 2 ** -8 * want.abs() + 2e-6).all()   # one rounding to bf16
+    ops.check_status()
+
+
 # logits whose product leaves the statistics and logits whose rows are read for them, in one chunk and in several
 @pytest.mark.parametrize("T,H,V", [(130, 1536, 17008), (130, 1528, 17008), (130, 1536, 16384), (70, 64, 520)])
 def test_linear_ce_with_and_without_statistics(ops, T, H, V, monkeypatch):

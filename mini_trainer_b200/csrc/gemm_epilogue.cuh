@@ -50,8 +50,9 @@ __device__ __forceinline__ void row_stats8(Stats& st, uint4 o) {
   const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y), r2 = unpack_bf16(o.z), r3 = unpack_bf16(o.w);
   const float mx = fmaxf(fmax3(fmaxf(r0.x, r0.y), r1.x, r1.y), fmax3(fmaxf(r2.x, r2.y), r3.x, r3.y));
   if (mx > st.m) { st.s *= exp_ftz(st.m - mx); st.m = mx; }
-  st.s += exp_ftz(r0.x - st.m) + exp_ftz(r0.y - st.m) + exp_ftz(r1.x - st.m) + exp_ftz(r1.y - st.m) + exp_ftz(r2.x - st.m) +
-          exp_ftz(r2.y - st.m) + exp_ftz(r3.x - st.m) + exp_ftz(r3.y - st.m);
+  const auto base = st.m == -INFINITY ? 0.f : st.m;   // nothing but -infinity so far
+  st.s += exp_ftz(r0.x - base) + exp_ftz(r0.y - base) + exp_ftz(r1.x - base) + exp_ftz(r1.y - base) + exp_ftz(r2.x - base) +
+          exp_ftz(r2.y - base) + exp_ftz(r3.x - base) + exp_ftz(r3.y - base);
 }
 
 // Output staging. A row of a tile belongs to one thread, so storing it directly sends 32 half-sectors to 32 rows with every

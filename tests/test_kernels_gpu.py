@@ -1075,6 +1075,34 @@ def test_cross_entropy_of_a_target_that_is_no_column(ops, V, form):
     ops.check_status()
 
 
+@pytest.mark.parametrize("form", ["one", "pair", "wide"])
+def test_softmax_statistics_of_overflowing_logits(ops, form, monkeypatch):
+    """Columns of -infinity count for nothing, also where they are the first of a tile or all of it."""
+    from mini_trainer_b200.ops import gemm_plan
+    T, K, V = 300, 128, 1032
+    monkeypatch.setattr(gemm_plan, "wide", lambda *a: int(form == "wide"))
+    monkeypatch.setattr(gemm_plan, "choose", lambda *a: (form == "pair", 1))
+    monkeypatch.setattr(ops, "_gemm_plans", {})
+    names = []
+    monkeypatch.setattr(ops, "_call", lambda name, *a, call=ops._call, **kw: names.append(name) or call(name, *a, **kw))
+    torch.manual_seed(6)
+    x = (torch.rand(T, K, device="cuda") + 0.5).bfloat16() * 2.0 ** 100
+    w = (bf(V, K, scale=K ** -0.5).float() * 2.0 ** -100).bfloat16()
+    for a, b in ((0, 8), (40, 48), (256, 512), (768, 808), (1024, 1032)):
+        w[a:b] = -(2.0 ** 100)   # products of -2^200 overflow
+    out, st = torch.empty(T, V, dtype=torch.bfloat16, device="cuda"), torch.full((T, -(-V // 256), 2), float("nan"), device="cuda")
+    ops.gemm(x, False, w, False, out, T, V, K, stats=st)
+    assert names == [{"one": "mtb200_gemm_bf16", "pair": "mtb200_gemm2_bf16", "wide": "mtb200_gemm2_wide_bf16"}[form]]
+    assert (out[:, :8] == float("-inf")).all() and out[:, 8:40].isfinite().all()
+    tiles = torch.nn.functional.pad(out.double(), (0, -V % 256), value=float("-inf")).view(T, -1, 256)
+    top = tiles.amax(-1)
+    assert torch.equal(st[..., 0].double(), top) and (top[:, 1] == float("-inf")).all() and (top[:, 4] == float("-inf")).all()
+    want = (tiles - top.clamp_min(-1e38)[..., None]).exp().sum(-1)
+    # 256 fp32 terms of at most one, added one by one
+    assert ((st[..., 1].double() - want).abs() <= 256 * 2 ** -24 * want).all()
+    ops.check_status()
+
+
 # logits whose product leaves the statistics and logits whose rows are read for them, in one chunk and in several
 @pytest.mark.parametrize("T,H,V", [(130, 1536, 17008), (130, 1528, 17008), (130, 1536, 16384), (70, 64, 520)])
 def test_linear_ce_with_and_without_statistics(ops, T, H, V, monkeypatch):

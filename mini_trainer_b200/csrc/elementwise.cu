@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(1024, 1) ce_row_kernel(const __nv_bfloat16* lo
     gm = warp_max(w.x);
     gs = warp_sum(w.x == -INFINITY ? w.y : w.y * exp_ftz(w.x - gm));
     if (threadIdx.x == 0) loss[row] = ignored ? 0.f : gm + logf(gs) - t;
-    const float scale = exp_ftz(base - gm) * (grad_scale / gs);
+    const float scale = exp_ftz(m - gm) * (grad_scale / gs);   // zero for a thread that has nothing but -infinity, whatever the row's maximum
     __nv_bfloat16* dr = dlogits + row * ldd;
 #pragma unroll
     for (int k = 0; k < CE_ROW_VECS; ++k) {

@@ -1075,6 +1075,24 @@ def test_cross_entropy_of_a_target_that_is_no_column(ops, V, form):
     ops.check_status()
 
 
+@pytest.mark.parametrize("V,form", CE_FORMS + [(5000, "rows")])
+def test_cross_entropy_of_low_logits_beside_masked_ones(ops, V, form):
+    """Every 32nd vector of eight columns is masked, which are all that some threads have, and the others are far below zero."""
+    torch.manual_seed(V)
+    lg = bf(5, V + 16, scale=2) - 300
+    lg[:, (torch.arange(V + 16, device="cuda") // 8) % 32 == 0] = float("-inf")
+    tg = torch.tensor([8, 9, -100, 200, 255], device="cuda")
+    loss, grad = _ce_forms(ops, lg, V + 16, V, form, tg)
+    x = lg[:, :V].double()
+    want = torch.softmax(x, 1)
+    want[torch.arange(5), tg.clamp_min(0)] -= 1
+    want[2] = 0
+    # the maximum and its sum's logarithm are added at 2^-15 a step
+    assert (loss - torch.nn.functional.cross_entropy(x, tg, reduction="none", ignore_index=-100)).abs().max() < 2 ** -15
+    assert ((grad.double() - want).abs() <= 2 ** -8 * want.abs() + 2e-6).all()   # one rounding to bf16
+    ops.check_status()
+
+
 @pytest.mark.parametrize("form", ["one", "pair", "wide"])
 def test_softmax_statistics_of_overflowing_logits(ops, form, monkeypatch):
     """Columns of -infinity count for nothing, also where they are the first of a tile or all of it."""

@@ -128,6 +128,9 @@ class ExpertSlabs:
     cap: int                # height of the row buffers
     k: int                  # experts per token
 
+    def __post_init__(self):
+        self.experts = self.counts.shape[0]
+
 
 def _ptr(t):
     return None if t is None else t.data_ptr()
@@ -177,7 +180,7 @@ class NativeOps:
         self.profile = [] if os.environ.get("MTB200_PROFILE") else None
         self._scratch = {}
         self._gemm_ws = {}   # stream handle -> arrival counters of split launches
-        self._gemm_plans = {}   # sizes -> entry point and splits
+        self._gemm_plans = {}   # sizes of a product, or of a grouped one -> entry point and splits, or mode
         self._epoch = itertools.count(1)   # of the launches that may split
         self._attn_plan_cache = {}
         self._block_specs = {}   # sizes of a block -> its products' plans
@@ -681,17 +684,29 @@ class NativeOps:
         """Rows of ``src`` [T, H] in slab order, zeros between the slabs."""
         H = src.shape[1]
         out = torch.empty(sl.cap, H, dtype=src.dtype, device=self.device)
-        self._call("mtb200_moe_gather", src.contiguous().data_ptr(), sl.pair_of.data_ptr(), sl.starts.data_ptr(), sl.counts.shape[0], sl.k,
+        self._call("mtb200_moe_gather", src.contiguous().data_ptr(), sl.pair_of.data_ptr(), sl.starts.data_ptr(), sl.experts, sl.k,
                    sl.cap, H, float(scale), out.data_ptr(), self._st())
         return out
 
-    def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride, act=None, fn="silu"):
-        E = sl.counts.shape[0]
-        rows = sl.cap - (_GROUP_ALIGN - 1) * E   # of all experts, to within a tile
+    def _plan_grouped(self, key):
+        """``mode`` of a grouped product's entry point, with its kernel, from its sizes and whether rows of an operand start off 32 bytes."""
+        mode, cap, E, M, N, K, off = key
+        rows = cap - (_GROUP_ALIGN - 1) * E   # of all experts, to within a tile
         wide = self.pair_max_flops > 0 and self.cta_pairs() > 0 and gemm_plan.grouped_wide(
-            mode == 2, rows, E, 2.0 * rows * N * (M if mode == 2 else K), K, bool((a.stride(0) | ldb) & 15))
-        self._call("mtb200_gemm_grouped", a.data_ptr(), a.stride(0), b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), _ACT[fn], mode + 4 * wide, sl.cap, M, N, K,
-                   sl.starts.data_ptr(), sl.counts.data_ptr(), sl.counts.shape[0], stride, self.status.data_ptr(), self._st(),
+            mode == 2, rows, E, 2.0 * rows * N * (M if mode == 2 else K), K, off != 0)
+        if len(self._gemm_plans) >= 4096:
+            self._gemm_plans.clear()
+        self._gemm_plans[key] = mode + 4 * wide
+        return mode + 4 * wide
+
+    def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride, act=None, fn="silu"):
+        lda, cap, E = a.stride(0), sl.cap, sl.experts
+        key = (mode, cap, E, M, N, K, (lda | ldb) & 15)   # asked six times a layer, which the host bounds where experts are small
+        form = self._gemm_plans.get(key)
+        if form is None:
+            form = self._plan_grouped(key)
+        self._call("mtb200_gemm_grouped", a.data_ptr(), lda, b.data_ptr(), ldb, out.data_ptr(), ldd, _ptr(act), _ACT[fn], form, cap, M, N, K,
+                   sl.starts.data_ptr(), sl.counts.data_ptr(), E, stride, self.status.data_ptr(), self._st(),
                    tag="gemm_grouped_" + ("nt", "nn", "tn", "nt_act")[mode])
         return out
 
@@ -729,7 +744,7 @@ class NativeOps:
         dgu = torch.empty_like(gu)
         dw = torch.zeros_like(w)
         self._call("mtb200_moe_glu_bwd", du.data_ptr(), gu.data_ptr(), w.data_ptr(), sl.pair_of.data_ptr(), sl.starts.data_ptr(),
-                   sl.counts.shape[0], sl.cap, F, int(act != "silu"), dgu.data_ptr(), dw.data_ptr(), self._st())
+                   sl.experts, sl.cap, F, int(act != "silu"), dgu.data_ptr(), dw.data_ptr(), self._st())
         return dgu, du, dw
 
     def combine_rows(self, rows, sl: ExpertSlabs, base, w=None, add=None, scale=1.0):

@@ -1746,6 +1746,7 @@ def test_grouped_products_in_wide_tiles_match(ops, T, E, k, popular, H, F, monke
     got = []
     for wide in (False, True):
         monkeypatch.setattr(gemm_plan, "grouped_wide", lambda *a: wide)
+        monkeypatch.setattr(ops, "_gemm_plans", {})
         dw = torch.full((E, 2 * F, H), float("nan"), dtype=torch.bfloat16, device="cuda")
         ops.grouped_wgrad(d, x, (dw[0], 2 * F * H), sl)
         stack = (w[0], 2 * F * H)

@@ -259,6 +259,29 @@ def test_grouped_products_choice(reduce, rows, E, flops, K, ragged, want):
     assert G.grouped_wide(reduce, rows, E, flops, K, ragged) == want
 
 
+def test_grouped_product_is_planned_once_per_size(monkeypatch):
+    from mini_trainer_b200.ops import gemm_plan, native
+    asked = []
+    monkeypatch.setattr(gemm_plan, "grouped_wide", lambda reduce, rows, E, flops, K, ragged: asked.append((reduce, rows, E, flops, K, ragged)) or ragged)
+    ops = make_ops()
+    i32 = lambda n: torch.zeros(n, dtype=torch.int32)   # noqa: E731
+    for _ in range(3):
+        sl = native.ExpertSlabs(i32(5), i32(4), None, None, 1024, 2)
+        x, w = torch.empty(1024, 64, dtype=torch.bfloat16), torch.empty(96, 64, dtype=torch.bfloat16)
+        ops.grouped_linear(x, (w, 96 * 64), sl)
+        ops.grouped_linear_act(x, (w, 96 * 64), sl)
+        ops.grouped_dgrad(torch.empty(1024, 104, dtype=torch.bfloat16)[:, :96], (w, 96 * 64), sl)   # rows that start off 32 bytes
+        ops.grouped_wgrad(torch.empty(1024, 96, dtype=torch.bfloat16), x, (w, 96 * 64), sl)
+    assert [a[1][8] for a in ops.calls] == [0, 3, 5, 2] * 3
+    rows = 1024 - 4 * 127
+    assert asked == [(False, rows, 4, 2.0 * rows * 96 * 64, 64, False)] * 2 + [(False, rows, 4, 2.0 * rows * 64 * 96, 96, True),
+                                                                              (True, rows, 4, 2.0 * rows * 64 * 96, 0, False)]
+    ops.pair_max_flops = 0.0        # one kernel for all of them
+    ops._gemm_plans.clear()
+    ops.grouped_dgrad(torch.empty(1024, 104, dtype=torch.bfloat16)[:, :96], (w, 96 * 64), sl)
+    assert ops.calls[-1][1][8] == 1
+
+
 # each at least 10 % faster in this form than in tiles of 256 columns, or (None) in those
 @pytest.mark.parametrize("M,N,K,want", [(640, 512, 3072, (64, 3)), (640, 512, 512, (64, 1)), (3072, 512, 640, (128, 1)), (1200, 1024, 768, (128, 1)), (1249, 1296, 616, (128, 1)),
                                         (1262, 3272, 512, None), (4096, 1376, 256, None), (1200, 4096, 768, None), (16384, 4096, 4096, None)])

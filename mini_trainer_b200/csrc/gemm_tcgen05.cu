@@ -527,31 +527,32 @@ int mtb200_gemm_n128_bf16(const void* A, long long lda, int a_mn, const void* B,
   return mtb200_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 | GEMM_N128, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
 }
 
-// A product with an MLP's activation in its epilogue (gemm_act.cuh), on one CTA or, two_cta, on CTA pairs (2: with wide tiles).
+// A product with an MLP's activation in its epilogue (gemm_act.cuh). `form`: FORM_ONE, FORM_PAIR or FORM_WIDE; narrow tiles have no such epilogue.
 //   mode 1  out[M, 2F] = A[M, K] * W[2F, K]^T, act[M, F] = f(out[:, :F]) * out[:, F:]
 //   mode 2  out[M, F] = A[M, K] * W[F, K]^T (+ bias), act[M, F] = f(out)
 // All row-major, without padding between rows but in A. f: SiLU, or (gelu) the tanh-approximated GELU.
 int mtb200_gemm_act(const void* A, long long lda, const void* W, void* out, void* act, const void* bias, int mode, int gelu, int M, int F, int K,
-                    int two_cta, int* status, cudaStream_t stream) {
+                    int form, int* status, cudaStream_t stream) {
   using namespace mtb;
   if (M <= 0 || F <= 0 || K <= 0) return 0;
-  if ((mode != ACT_GLU && mode != ACT_PLAIN) || F % 8 || K % 8 || (bias != nullptr && mode != ACT_PLAIN)) return -10;
+  if ((mode != ACT_GLU && mode != ACT_PLAIN) || form < FORM_ONE || form > FORM_WIDE || F % 8 || K % 8 || (bias != nullptr && mode != ACT_PLAIN)) return -10;
   if (reinterpret_cast<uintptr_t>(bias) & 15) return -11;
   const int N = mode == ACT_GLU ? 2 * F : F;
+  const bool wide = form == FORM_WIDE;
   CUtensorMap ta, tb;
   ActMaps<ACT_GLU> m;
   int rc = make_tmap_2d_bf16(&ta, A, K, M, lda, 64, 128);
   if (rc) return rc;
-  rc = make_tmap_2d_bf16(&tb, W, K, N, K, 64, mode == ACT_GLU || two_cta ? 128 : 256);
+  rc = make_tmap_2d_bf16(&tb, W, K, N, K, 64, mode == ACT_GLU || form != FORM_ONE ? 128 : 256);
   if (rc) return rc - 10;
   __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out);
-  rc = make_tmap_act(&m.gate, o, F, M, N, two_cta == 2);
-  if (!rc) rc = make_tmap_act(&m.up, mode == ACT_GLU ? o + F : o, F, M, N, two_cta == 2);
-  if (!rc) rc = make_tmap_act(&m.act, act, F, M, F, two_cta == 2);
+  rc = make_tmap_act(&m.gate, o, F, M, N, wide);
+  if (!rc) rc = make_tmap_act(&m.up, mode == ACT_GLU ? o + F : o, F, M, N, wide);
+  if (!rc) rc = make_tmap_act(&m.act, act, F, M, F, wide);
   if (rc) return rc - 20;
   const EpiParams e{M, N, nullptr, 0, reinterpret_cast<const __nv_bfloat16*>(bias), 1.0f, 1, nullptr, nullptr, nullptr, 0};
   const ActParams a{F, gelu};
-  if (two_cta) return g2::launch_act(mode, two_cta == 2, ta, tb, m, e, a, K, status, stream);
+  if (form != FORM_ONE) return g2::launch_act(mode, wide, ta, tb, m, e, a, K, status, stream);
   const GemmParams p{M, N, K, status, tune_group_m(), tune_wait_hint(), 0u, e, a};
   if (mode == ACT_GLU)
     return launch<false, false, false, false, false, GROUP_NONE, false, false, ACT_GLU>(ta, tb, m.gate, p, stream, nullptr, 0, nullptr, m);

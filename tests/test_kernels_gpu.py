@@ -1712,6 +1712,16 @@ def test_gemm_wide_tiles_are_exact(ops, M, N, K, splits, monkeypatch):
     ops.check_status()
 
 
+@pytest.mark.parametrize("form", [-1, 3, 4])
+def test_activation_behind_a_product_refuses_forms_without_that_epilogue(ops, form):
+    """Narrow tiles are numbers 3 and 4 of a plan's kernels."""
+    x, w, pre, act = bf(128, 64), bf(128, 64), bf(128, 128), bf(128, 64)
+    kept = pre.clone()
+    with pytest.raises(RuntimeError, match="code -10"):
+        ops._call("mtb200_gemm_act", x.data_ptr(), 64, w.data_ptr(), pre.data_ptr(), act.data_ptr(), None, 1, 0, 128, 64, 64, form, ops.status.data_ptr(), ops._st())
+    assert torch.equal(pre, kept)
+
+
 @pytest.mark.parametrize("T,F,K", [(33, 136, 264), (1000, 1000, 512), (256 * 37, 1096, 72)])
 @pytest.mark.parametrize("fn", ["silu", "gelu_tanh"])
 def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypatch):

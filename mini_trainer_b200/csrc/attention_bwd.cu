@@ -351,7 +351,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     const int q = warp & 3;
     const int half = (warp >> 2) - 1;      // which 64 queries (softmax) / which half of the D columns (epilogue)
     const int r = q * 32 + lane;
-    const int kpos = k0 + r;               // position of this thread's key inside the sequence
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t ts = t_s + lane_addr + half * 64, tp = t_dp + lane_addr + half * 64;
     const float sl2 = p.scale * 1.4426950408889634f;
@@ -424,7 +423,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
         }
         if (k0 + AB_B > seq_len) {   // last key block: keys past the sequence give nothing to dQ (their rows of dK and dV are not stored)
 #pragma unroll
-          for (int x = 0; x < 16; ++x) dk[x] = kpos < seq_len ? dk[x] : 0u;
+          for (int x = 0; x < 16; ++x) dk[x] = k0 + r < seq_len ? dk[x] : 0u;
         }
         tmem_st_32x16(tp + cc * 16, dk);
 #pragma unroll
@@ -441,6 +440,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkv, const __grid_constan
     // epilogue: dK, dV (rows = keys)
     if (!mbar_wait(all_done, 0, abort_flag)) { atomicExch(p.status, 29); goto done; }
     tc_fence_after();
+    const int kpos = k0 + r;
     const bool ok = kpos < seq_len;
     const bool whole = kpos - lane + 31 < seq_len;   // uniform over the warp
     __nv_bfloat16* rowp = p.dqkv + (static_cast<long long>(seq_start) + kpos) * p.ldq;

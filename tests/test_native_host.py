@@ -299,3 +299,17 @@ def test_gemm_narrow_tiles_choice(M, N, K, want):
     assert ops.product_plan(M, N, K, 0, act=True)[0] in ("mtb200_gemm_bf16", "mtb200_gemm2_bf16", "mtb200_gemm2_wide_bf16")
     ops.use_gemm2 = True
     assert ops._plan_gemm(M, N, K, None)[0] == "mtb200_gemm2_bf16"
+
+
+@pytest.mark.parametrize("source", ["attention_fwd", "attention_fwd_one", "attention_bwd"])
+def test_attention_kernels_hold_their_rows_in_registers(source, tmp_path):
+    """A softmax thread's scores and probabilities: what the compiler spills is stored and read again for every key tile."""
+    import re
+    import subprocess
+    from mini_trainer_b200 import build
+    nvcc = build._nvcc()
+    if nvcc is None:
+        pytest.skip("needs nvcc")
+    r = subprocess.run([nvcc, *build.NVCC_FLAGS, "-Xptxas", "-v", "-c", str(build.CSRC / f"{source}.cu"), "-o", str(tmp_path / "x.o")], capture_output=True, text=True, check=True)
+    spills = [int(n) for n in re.findall(r"(\d+) bytes spill", r.stdout + r.stderr)]
+    assert len(spills) >= 4 and not any(spills)

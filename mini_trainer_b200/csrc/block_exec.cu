@@ -18,8 +18,9 @@ namespace {
 int gemm(const BlockSpec& s, const BlockIO& io, const u64*& epoch, int which, const void* a, long long lda, int a_mn, const void* b, long long ldb, int b_mn, void* d, int M, int N,
          int K, const void* r, const void* bias, float alpha, cudaStream_t st) {
   const int splits = io.part != nullptr ? s.splits[which] : 1;
-  auto f = form_on_pairs(s.form[which]) ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
-  return f(a, lda, a_mn, b, ldb, b_mn, d, N, form_flags(s.form[which]), r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
+  GemmEntry* f = gemm_entry(s.form[which]);
+  if (f == nullptr) return -10;
+  return f(a, lda, a_mn, b, ldb, b_mn, d, N, 0, r, N, bias, M, N, K, alpha, splits, splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0,
            splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, nullptr, io.status, st);
 }
 
@@ -132,6 +133,12 @@ extern "C" {
 // Sizes of the structures, for a caller that lays them out itself (ops/block_exec.py).
 void mtb200_block_sizes(int* out) {
   out[0] = sizeof(BlockSpec); out[1] = sizeof(BlockParams); out[2] = sizeof(BlockIO);
+}
+// Entry point of a product's kernel by its number, null past the last, for a caller that numbers them itself.
+const char* mtb200_gemm_form(int form) {
+#define F(form, entry) case form: return #entry;
+  switch (form) { GEMM_FORMS(F) default: return nullptr; }
+#undef F
 }
 // Bytes of io->ws for a call with these arguments (backward: with gradients).
 long long mtb200_block_workspace(const BlockSpec* s, const BlockIO* io, int bwd) {

@@ -4,22 +4,22 @@
 #include <cuda_runtime.h>
 
 extern "C" {
-int mtb200_gemm_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
-                     float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
-int mtb200_gemm2_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
+// The kernels of a product, as plans number them (ops/gemm_plan.py): single CTAs, CTA pairs, pairs with wide tiles, single CTAs with narrow ones.
+#define GEMM_FORMS(F) \
+  F(FORM_ONE, mtb200_gemm_bf16) F(FORM_PAIR, mtb200_gemm2_bf16) F(FORM_WIDE, mtb200_gemm2_wide_bf16) F(FORM_N64, mtb200_gemm_n64_bf16) F(FORM_N128, mtb200_gemm_n128_bf16)
+typedef int GemmEntry(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
                       float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
-// Added to out_f32: tiles of 256 x 512 (mtb200_gemm2_bf16), of 128 x 64 or 128 x 128 (mtb200_gemm_bf16).
-enum { GEMM2_WIDE = 2, GEMM_N64 = 4, GEMM_N128 = 8 };
-// How a product is computed, as a plan names it (ops/gemm_plan.py): single CTAs, pairs, pairs with wide tiles, single CTAs with narrow ones.
-enum { FORM_ONE = 0, FORM_PAIR = 1, FORM_WIDE = 2, FORM_N64 = 3, FORM_N128 = 4 };
-inline bool form_on_pairs(int form) { return form == FORM_PAIR || form == FORM_WIDE; }
-inline int form_flags(int form) { return form == FORM_WIDE ? GEMM2_WIDE : form == FORM_N64 ? GEMM_N64 : form == FORM_N128 ? GEMM_N128 : 0; }
-int mtb200_gemm_n64_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
-                         float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
-int mtb200_gemm_n128_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
-                          float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
-int mtb200_gemm2_wide_bf16(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int,
-                           float, int, unsigned long long*, unsigned long long, float*, long long, float2*, int*, cudaStream_t);
+#define F(form, entry) form,
+enum { GEMM_FORMS(F) };
+#undef F
+#define F(form, entry) GemmEntry entry;
+GEMM_FORMS(F)
+#undef F
+inline GemmEntry* gemm_entry(int form) {
+#define F(form, entry) case form: return entry;
+  switch (form) { GEMM_FORMS(F) default: return nullptr; }
+#undef F
+}
 int mtb200_gemm_act(const void*, long long, const void*, void*, void*, const void*, int, int, int, int, int, int, int*, cudaStream_t);
 int mtb200_swiglu_fwd(const void*, void*, long long, int, cudaStream_t);
 int mtb200_geglu_fwd(const void*, void*, long long, int, cudaStream_t);

@@ -663,8 +663,7 @@ int mtb200_gemm2_pairs() { return mtb::g2::co_resident_pairs<false>(); }
 int mtb200_gemm2_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                       long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
                       float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
-  return mtb::g2::gemm2((out_f32 & GEMM2_WIDE) != 0, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 & ~GEMM2_WIDE, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part,
-                        part_bytes, stats, status, stream);
+  return mtb::g2::gemm2(false, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
 }
 
 // The same with wide tiles (256 x 512).

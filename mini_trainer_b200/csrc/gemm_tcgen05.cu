@@ -457,25 +457,11 @@ static int launch_narrow(const CUtensorMap& ta, const CUtensorMap& tb, const CUt
   return launch<A_MN, B_MN, OUT_F32, false, false, GROUP_NONE, false, false, ACT_NONE, NT>(ta, tb, td, p, stream, nullptr, part_bytes);
 }
 
-}  // namespace mtb
-
-extern "C" {
-
-// D[M,N] = alpha * op(A) * op(B) (+bias) (+R).
-//   a_mn = 0: A is row-major [M, K] (lda >= K);  a_mn = 1: A is row-major [K, M] (lda >= M)
-//   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
-//   out_f32: D and R are fp32, else bf16; plus GEMM_N64 or GEMM_N128: tiles of 128 x 64 or 128 x 128 (no statistics). R may alias D (accumulate). bias is bf16 [N] or null.
-//   splits: work items per output tile (ops/gemm_plan.py); more than one needs counters (SPLIT_COUNTERS words, zero before the first
-//   call; launches that may overlap have their own), an epoch that grows with every launch on them, and part, fp32 scratch of part_bytes
-//   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
-// Returns 0 on success, a negative code on invalid arguments or launch failure.
-int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
-                     long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                     float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
-  using namespace mtb;
+// `nt`: columns of a tile.
+static int gemm(int nt, const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
+                long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int nt = out_f32 & GEMM_N64 ? 64 : out_f32 & GEMM_N128 ? 128 : BN;
-  out_f32 &= ~(GEMM_N64 | GEMM_N128);
   if (N % 8 || ldd % 8 || (R && ldr % 8) || (stats && (out_f32 || nt != BN)) || splits < 1) return -10;
   CUtensorMap ta, tb, td;
   int rc;
@@ -515,16 +501,34 @@ int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long
 #undef GEMM
 }
 
-// The same in narrow tiles.
+}  // namespace mtb
+
+extern "C" {
+
+// D[M,N] = alpha * op(A) * op(B) (+bias) (+R).
+//   a_mn = 0: A is row-major [M, K] (lda >= K);  a_mn = 1: A is row-major [K, M] (lda >= M)
+//   b_mn = 0: B is row-major [N, K] (ldb >= K);  b_mn = 1: B is row-major [K, N] (ldb >= N)
+//   out_f32: D and R are fp32, else bf16. R may alias D (accumulate). bias is bf16 [N] or null.
+//   splits: work items per output tile (ops/gemm_plan.py); more than one needs counters (SPLIT_COUNTERS words, zero before the first
+//   call; launches that may overlap have their own), an epoch that grows with every launch on them, and part, fp32 scratch of part_bytes
+//   stats: optional softmax statistics of the output rows (EpiParams), bf16 output only
+// Returns 0 on success, a negative code on invalid arguments or launch failure.
+int mtb200_gemm_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
+                     long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                     float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
+  return mtb::gemm(mtb::BN, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
+}
+
+// The same in tiles of 128 x 64 and of 128 x 128, without statistics.
 int mtb200_gemm_n64_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
                          long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
                          float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
-  return mtb200_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 | GEMM_N64, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
+  return mtb::gemm(64, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
 }
 int mtb200_gemm_n128_bf16(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* D,
-                         long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
-                         float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
-  return mtb200_gemm_bf16(A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32 | GEMM_N128, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
+                          long long ldd, int out_f32, const void* R, long long ldr, const void* bias, int M, int N, int K,
+                          float alpha, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float2* stats, int* status, cudaStream_t stream) {
+  return mtb::gemm(128, A, lda, a_mn, B, ldb, b_mn, D, ldd, out_f32, R, ldr, bias, M, N, K, alpha, splits, counters, epoch, part, part_bytes, stats, status, stream);
 }
 
 // A product with an MLP's activation in its epilogue (gemm_act.cuh). `form`: FORM_ONE, FORM_PAIR or FORM_WIDE; narrow tiles have no such epilogue.

@@ -151,8 +151,9 @@ long long run(const StepSpec& s, const StepIO& io, bool measure, cudaStream_t st
   auto product = [&](int which, const void* a, long long lda, int a_mn, const void* w_, long long ldw, int w_mn, void* d, long long ldd, int M, int N, int K,
                      const void* r) {
     const int splits = io.part != nullptr ? s.splits[which] : 1;
-    auto f = form_on_pairs(s.form[which]) ? mtb200_gemm2_bf16 : mtb200_gemm_bf16;
-    return f(a, lda, a_mn, w_, ldw, w_mn, d, ldd, form_flags(s.form[which]), r, r ? ldd : 0, nullptr, M, N, K, s.logit_alpha, splits,
+    GemmEntry* f = gemm_entry(s.form[which]);
+    if (f == nullptr) return -10;
+    return f(a, lda, a_mn, w_, ldw, w_mn, d, ldd, 0, r, r ? ldd : 0, nullptr, M, N, K, s.logit_alpha, splits,
              splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0, splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, nullptr, io.status, st);
   };
   const void* W = at(lm.param, s.off_lm);

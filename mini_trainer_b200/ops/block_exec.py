@@ -8,11 +8,12 @@ is the bound there) or find no room: the Python form gives each temporary back w
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import c_char_p, c_float, c_int, c_longlong, c_void_p
 
 import torch
 
 from ..utils import nvtx
+from . import gemm_plan
 
 MOST_WORKSPACE = 256 << 20
 GEMMS = 12   # G_QKV .. W_QKV of csrc/block_exec.cu
@@ -21,7 +22,7 @@ NAMES = ("ln1", "bln1", "wqkv", "bqkv", "qn", "kn", "wo", "bo", "ln2", "bln2", "
 
 class Spec(ctypes.Structure):
     _fields_ = [(n, c_int) for n in ("T", "H", "F", "Hq", "Hkv", "D", "gated", "gelu", "layernorm", "qk_norm")] \
-        + [(n, c_float) for n in ("eps", "scale", "alpha")] + [("pair", c_int * GEMMS), ("splits", c_int * GEMMS), ("act_form", c_int)] \
+        + [(n, c_float) for n in ("eps", "scale", "alpha")] + [("form", c_int * GEMMS), ("splits", c_int * GEMMS), ("act_form", c_int)] \
         + [(n, c_int) for n in ("need_out", "attn_form", "fwd_items", "bwd_items", "bwd_splits")]
 
 
@@ -37,11 +38,15 @@ class IO(ctypes.Structure):
 
 
 def check_layout(lib) -> None:
-    """The structures are laid out here and in ``csrc/block_exec.cu``."""
+    """The structures are laid out here and in ``csrc/block_exec.h``, the kernels of a product numbered in ``gemm_plan`` and in ``csrc/entries.h``."""
     sizes = (c_int * 3)()
     lib.mtb200_block_sizes(sizes)
     if list(sizes) != [ctypes.sizeof(t) for t in (Spec, Params, IO)]:
         raise RuntimeError(f"the library lays its block structures out in {list(sizes)} bytes: it is of another version, build it again")
+    lib.mtb200_gemm_form.restype = c_char_p
+    names = [lib.mtb200_gemm_form(i) for i in range(len(gemm_plan.FORMS) + 1)]
+    if names != [*(n.encode() for n in gemm_plan.FORMS), None]:
+        raise RuntimeError(f"the library numbers the kernels of a product {names}: it is of another version, build it again")
 
 
 def _ptr(t):
@@ -82,9 +87,9 @@ def _spec(ops, cfg, T: int):
         s = Spec(T, H, F, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, int(cfg.mlp_gated),
                  int((cfg.mlp_act if cfg.mlp_gated else "gelu_tanh") != "silu"), int(cfg.norm_type == "layernorm"), int(cfg.qk_norm), cfg.rms_norm_eps,
                  cfg.attention_scale, cfg.residual_multiplier)
-        s.pair[:] = [ops.FORMS[n] for n, _, _ in plans]
+        s.form[:] = [gemm_plan.FORMS[n] for n, _, _ in plans]
         act, _, _ = ops.product_plan(*products[2], pitches[2], act=True)
-        s.act_form = ops.FORMS[act]
+        s.act_form = gemm_plan.FORMS[act]
         s.splits[:] = [k for _, k, _ in plans]
         part = [b if k > 1 else 0 for _, k, b in plans]
         if len(ops._block_specs) >= 1024:

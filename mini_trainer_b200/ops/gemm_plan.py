@@ -22,6 +22,10 @@ def partial_bytes(M: int, N: int, pair: bool, splits: int) -> int:
     return -(-N // 256) * (2 * -(-M // 256) if pair else -(-M // 128)) * splits * UNIT_BYTES
 
 
+# The kernels of a product, numbered as in csrc/entries.h: single CTAs, CTA pairs, pairs with wide tiles, single CTAs with narrow ones.
+FORMS = {"mtb200_gemm_bf16": 0, "mtb200_gemm2_bf16": 1, "mtb200_gemm2_wide_bf16": 2, "mtb200_gemm_n64_bf16": 3, "mtb200_gemm_n128_bf16": 4}
+
+
 def _best_split(tiles: int, units: int, kblocks: int, workers: int, max_units: int, t: tuple):
     launch, block, item, least, split, partial = t
     best = launch + -(-tiles // workers) * max(kblocks * block + item, least)

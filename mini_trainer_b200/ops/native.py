@@ -157,8 +157,6 @@ def route_topk(logits, k: int, renorm: bool, call=_launch):
 
 class NativeOps:
     name = "native"
-    # as csrc/entries.h numbers them
-    FORMS = {"mtb200_gemm_bf16": 0, "mtb200_gemm2_bf16": 1, "mtb200_gemm2_wide_bf16": 2, "mtb200_gemm_n64_bf16": 3, "mtb200_gemm_n128_bf16": 4}
 
     def __init__(self, device, ce_chunk: int = 8192, attention: str | None = None):
         self.device = torch.device(device)
@@ -450,7 +448,7 @@ class NativeOps:
         pre = torch.empty(T, N, dtype=x.dtype, device=self.device)
         act = torch.empty(T, F, dtype=x.dtype, device=self.device)
         self._call("mtb200_gemm_act", x.data_ptr(), x.stride(0), w.data_ptr(), pre.data_ptr(), act.data_ptr(), _ptr(bias), 1 if gated else 2, code,
-                   T, F, K, self.FORMS[name], self.status.data_ptr(), self._st(), tag="gemm_nt_act")
+                   T, F, K, gemm_plan.FORMS[name], self.status.data_ptr(), self._st(), tag="gemm_nt_act")
         return pre, act
 
     def linear_wgrad(self, dy, x, dw_out, dbias_out=None, alpha=1.0):

@@ -13,7 +13,7 @@ from ctypes import c_float, c_int, c_longlong, c_void_p
 import torch
 
 from ..utils import nvtx
-from . import block_exec
+from . import block_exec, gemm_plan
 
 MOST_WORKSPACE = 1 << 30
 PARAMS = len(block_exec.NAMES)
@@ -74,7 +74,7 @@ def _spec(eng, T: int, R: int):
     s.off_embed, s.off_norm, s.off_bnorm = eng.embed.layout.specs["embed"].offset, head["norm"].offset, head["bnorm"].offset if "bnorm" in head else -1
     s.off_lm = s.off_embed if tied else head["lm_head"].offset
     plans = [ops.product_plan(*m) for m in ((R, V, H, H), (R, H, V, V | H), (V, H, R, V | H))]
-    s.form[:], s.splits[:] = [ops.FORMS[n] for n, _, _ in plans], [k for _, k, _ in plans]
+    s.form[:], s.splits[:] = [gemm_plan.FORMS[n] for n, _, _ in plans], [k for _, k, _ in plans]
     return s, max(fwd_part, bwd_part, *(b if k > 1 else 0 for _, k, b in plans))
 
 

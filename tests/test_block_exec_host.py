@@ -16,12 +16,16 @@ STUBS = r"""
 #include "block_exec.cu"
 extern "C" {
 long long noted[64][2];   // splits and epoch of every product and of the attention backward, in the order of their launches
+const char* entered[64];   // by the products among them
 int n_noted;
 float* last_rstd;
 #define GEMM(name) int name(const void*, long long, int, const void*, long long, int, void*, long long, int, const void*, long long, const void*, int, int, int, \
-  float, int splits, u64*, u64 epoch, float*, long long, float2*, int*, cudaStream_t) { noted[n_noted][0] = splits; noted[n_noted++][1] = epoch; return 0; }
+  float, int splits, u64*, u64 epoch, float*, long long, float2*, int*, cudaStream_t) { entered[n_noted] = #name; noted[n_noted][0] = splits; noted[n_noted++][1] = epoch; return 0; }
 GEMM(mtb200_gemm_bf16)
 GEMM(mtb200_gemm2_bf16)
+GEMM(mtb200_gemm2_wide_bf16)
+GEMM(mtb200_gemm_n64_bf16)
+GEMM(mtb200_gemm_n128_bf16)
 int mtb200_gemm_act(const void*, long long, const void*, void*, void*, const void*, int, int, int, int, int, int, int*, cudaStream_t) { return 0; }
 int mtb200_swiglu_fwd(const void*, void*, long long, int, cudaStream_t) { return 0; }
 int mtb200_geglu_fwd(const void*, void*, long long, int, cudaStream_t) { return 0; }
@@ -69,7 +73,7 @@ def lib(tmp_path_factory):
 
 def make(gated=1, layernorm=0, T=300):
     s = B.Spec(T, 256, 384, 4, 2, 64, gated, 0, layernorm, 0, 1e-5, 0.125, 1.0)
-    s.pair[:], s.splits[:] = [k % 2 for k in range(B.GEMMS)], [2] * B.GEMMS
+    s.form[:], s.splits[:] = [k % 5 for k in range(B.GEMMS)], [2] * B.GEMMS
     s.need_out, s.bwd_splits = 1, 2
     io = B.IO()
     for name, kind in B.IO._fields_:
@@ -125,5 +129,21 @@ def test_structures_have_the_layout_of_the_library(lib, monkeypatch):
     class Short(ctypes.Structure):
         _fields_ = B.Spec._fields_[:-1]
     monkeypatch.setattr(B, "Spec", Short)
+    with pytest.raises(RuntimeError, match="another version"):
+        B.check_layout(lib)
+
+
+def test_kernels_of_a_product_are_those_the_plan_names(lib, monkeypatch):
+    names = list(B.gemm_plan.FORMS)
+    entered = (ctypes.c_char_p * 64).in_dll(lib, "entered")
+    for first in range(len(names)):
+        s, io = make()
+        s.form[:] = [(first + k) % len(names) for k in range(B.GEMMS)]
+        queue(lib, s, io, 0)
+        assert [entered[k].decode() for k in range(4)] == [names[s.form[k]] for k in range(4)]
+    s.form[0] = len(names)   # not a kernel
+    n, p = ctypes.c_int(0), B.Params()
+    assert lib.mtb200_block_forward(ctypes.byref(s), ctypes.byref(p), ctypes.byref(io), ctypes.byref(n), None) == -10
+    monkeypatch.setattr(B.gemm_plan, "FORMS", dict(zip(reversed(names), range(len(names)))))
     with pytest.raises(RuntimeError, match="another version"):
         B.check_layout(lib)

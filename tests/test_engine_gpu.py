@@ -394,6 +394,22 @@ def test_minibatch_in_one_call_is_the_engine_launch_by_launch(family, lens, monk
     assert abs(n1 - n2) <= 5e-3 * n2 and all(torch.isfinite(m).all() for m in m1)
 
 
+@pytest.mark.parametrize("form,splits", [("mtb200_gemm2_wide_bf16", 1), ("mtb200_gemm_n64_bf16", 2), ("mtb200_gemm_n128_bf16", 1)])
+@pytest.mark.parametrize("family", ["llama", "tied"])
+def test_minibatch_in_one_call_on_every_kernel(family, form, splits, monkeypatch):
+    """The same with all products, the head's too, on one of the kernels that long and short ones take."""
+    from mini_trainer_b200.ops import gemm_plan, step_exec
+    tile, specs = {"mtb200_gemm_n64_bf16": 64, "mtb200_gemm_n128_bf16": 128}.get(form), []
+    with pytest.MonkeyPatch.context() as plans:
+        plans.setattr(gemm_plan, "narrow", lambda *a: (tile, splits) if tile else None)
+        plans.setattr(gemm_plan, "wide", lambda *a: 0 if tile else splits)
+        plans.setattr(step_exec, "_spec", lambda *a, real=step_exec._spec: specs.append(real(*a)) or specs[-1])
+        test_minibatch_in_one_call_is_the_engine_launch_by_launch(family, [300, 17, 129, 1, 640], monkeypatch)
+    assert len(specs) == 2
+    for s, _ in specs:
+        assert {*s.form, *s.block.form} == {gemm_plan.FORMS[form]} and {*s.splits, *s.block.splits} == {splits}
+
+
 # groups without gaps between their tensors, which are written whole, and with gaps, which are zeroed
 @pytest.mark.parametrize("hidden", [256, 264])
 @pytest.mark.parametrize("tied", [False, True])

@@ -967,14 +967,19 @@ def test_grouped_experts_shared_scaled_unnormalised(ops, T, H, F, E, k, popular,
 @pytest.mark.parametrize("M,N,K", [(136, 264, 1024), (300, 520, 7776)])
 def test_gemm_every_split(ops, M, N, K, two_cta, splits, monkeypatch):
     from mini_trainer_b200.ops import gemm_plan
+    monkeypatch.setattr(gemm_plan, "narrow", lambda *a: None)   # which products of these sizes take by themselves
+    monkeypatch.setattr(gemm_plan, "wide", lambda *a: 0)
     monkeypatch.setattr(gemm_plan, "choose", lambda *a: (two_cta, splits))
     monkeypatch.setattr(ops, "_gemm_plans", {})
+    ran = []
+    monkeypatch.setattr(ops, "_call", lambda name, *a, call=ops._call, **kw: ran.append((name, a[16])) or call(name, *a, **kw))
     a, b, res = _ints(M, K), _ints(N, K), _ints(M, N)
     want = a.float() @ b.float().t()       # integers below 2^24: exact in fp32 in any order
     for dt in (torch.float32, torch.bfloat16):
         out = torch.full((M, N), float("nan"), dtype=dt, device="cuda")
         ops.gemm(a, False, b, False, out, M, N, K, residual=res.to(dt))
         assert torch.equal(out, (want + res.float()).to(dt))
+    assert ran == [("mtb200_gemm2_bf16" if two_cta else "mtb200_gemm_bf16", splits)] * 2
     ops.check_status()
 
 
@@ -1380,6 +1385,22 @@ def test_block_in_one_call_is_the_block_launch_by_launch(ops, family, T, keep, m
     ops.check_status()
 
 
+@pytest.mark.parametrize("form,splits", [("mtb200_gemm2_wide_bf16", 1), ("mtb200_gemm2_wide_bf16", 2), ("mtb200_gemm_n64_bf16", 1), ("mtb200_gemm_n128_bf16", 2)])
+@pytest.mark.parametrize("family,keep", [("llama", "compact"), ("starcoder2", True), ("qwen3", False)])
+def test_block_in_one_call_on_every_kernel(ops, family, keep, form, splits, monkeypatch):
+    """The same with all products on one of the kernels that long and short ones take."""
+    from mini_trainer_b200.ops import gemm_plan
+    tile = {"mtb200_gemm_n64_bf16": 64, "mtb200_gemm_n128_bf16": 128}.get(form)
+    with pytest.MonkeyPatch.context() as plans:
+        plans.setattr(gemm_plan, "narrow", lambda *a: (tile, splits) if tile else None)
+        plans.setattr(gemm_plan, "wide", lambda *a: 0 if tile else splits)
+        plans.setattr(ops, "_gemm_plans", {})
+        plans.setattr(ops, "_block_specs", {})
+        test_block_in_one_call_is_the_block_launch_by_launch(ops, family, 700, keep, monkeypatch)
+        (spec, *_), = ops._block_specs.values()
+        assert set(spec.form) == {gemm_plan.FORMS[form]} and set(spec.splits) == {splits} and (spec.act_form == 2) == (tile is None)
+
+
 def test_block_in_one_call_leaves_to_the_python_form_what_it_does_not_cover(ops):
     from mini_trainer_b200.models import decoder as D, layout as L
     from mini_trainer_b200.models.config import ModelConfig
@@ -1727,9 +1748,12 @@ def test_activation_behind_a_product_refuses_forms_without_that_epilogue(ops, fo
 def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypatch):
     """Activation and softmax statistics behind wide tiles: the same bits as behind 256 x 256 tiles."""
     from mini_trainer_b200.ops import gemm_plan
+    if ops.cta_pairs() == 0:
+        pytest.skip("no clusters of two CTAs on this device")
     torch.manual_seed(T + F)
     x, w, bias = bf(T, K), bf(2 * F, K, scale=K ** -0.5), bf(2 * F)
-    got = []
+    got, ran = [], []
+    monkeypatch.setattr(ops, "_call", lambda name, *a, call=ops._call, **kw: ran.append((name, a[11] if name == "mtb200_gemm_act" else None)) or call(name, *a, **kw))
     monkeypatch.setattr(gemm_plan, "narrow", lambda *a: None)
     for splits in (1, 0):
         monkeypatch.setattr(gemm_plan, "wide", lambda *a: splits)
@@ -1738,6 +1762,10 @@ def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypa
         out, stats = torch.empty(T, 2 * F, dtype=torch.bfloat16, device="cuda"), torch.full((T, -(-2 * F // 256), 2), float("nan"), device="cuda")
         ops.gemm(x, False, w, False, out, T, 2 * F, K, alpha=0.5, stats=stats)
         got.append([*ops.linear_act(x, w, fn), out, stats] + ([*ops.linear_act(x, w, fn, gated=False, bias=bias)] if fn == "gelu_tanh" else []))
+    for name, form in (("mtb200_gemm2_wide_bf16", 2), ("mtb200_gemm2_bf16", 1)):
+        n = 3 if fn == "gelu_tanh" else 2
+        assert ran[:n] == [(name, None)] + [("mtb200_gemm_act", form)] * (n - 1)
+        del ran[:n]
     for g, h in zip(*got):
         assert torch.equal(g, h)
     ops.check_status()
@@ -1748,6 +1776,10 @@ def test_wide_tiles_epilogues_match_the_other_kernels(ops, T, F, K, fn, monkeypa
 @pytest.mark.parametrize("H,F", [(64, 72), (648, 520), (1040, 264)])
 def test_grouped_products_in_wide_tiles_match(ops, T, E, k, popular, H, F, monkeypatch):
     from mini_trainer_b200.ops import gemm_plan
+    if ops.cta_pairs() == 0:
+        pytest.skip("no clusters of two CTAs on this device")
+    ran = []
+    monkeypatch.setattr(ops, "_call", lambda name, *a, call=ops._call, **kw: (name == "mtb200_gemm_grouped" and ran.append(a[8]), call(name, *a, **kw))[1])
     torch.manual_seed(T + H)
     topi = torch.stack([torch.randperm(popular, device="cuda")[:k] for _ in range(T)]) * (E // popular)
     sl = ops.expert_slabs(topi, E)
@@ -1763,6 +1795,7 @@ def test_grouped_products_in_wide_tiles_match(ops, T, E, k, popular, H, F, monke
         rows = int(sl.starts[-1])
         got.append([dw, *(t[:rows] for t in (ops.grouped_linear(x, stack, sl), *ops.grouped_linear_act(x, stack, sl), *ops.grouped_linear_act(x, stack, sl, "gelu_tanh"),
                                              ops.grouped_dgrad(d, stack, sl)))])
+    assert ran == [2, 0, 3, 3, 1, 6, 4, 7, 7, 5]
     for a, b in zip(*got):
         assert not a.isnan().any() and torch.equal(a, b)
     ops.check_status()
@@ -1792,13 +1825,3 @@ def test_gemm_narrow_tiles_are_exact(ops, tile, M, N, K, splits, monkeypatch):
                 assert torch.equal(out, (want[:m] + (res[:m].float() + bias.float() if extra else 0.0)).to(dt)), (a_mn, b_mn, dt, extra)
     assert set(names) == {f"mtb200_gemm_n{tile}_bf16"}
     ops.check_status()
-
-
-@pytest.mark.parametrize("splits", [2, 3, 7, 16])
-@pytest.mark.parametrize("two_cta", [False, True])
-def test_gemm_every_split_in_tiles_of_256_columns(ops, two_cta, splits, monkeypatch):
-    """Products of these sizes take narrow tiles by themselves."""
-    from mini_trainer_b200.ops import gemm_plan
-    monkeypatch.setattr(gemm_plan, "narrow", lambda *a: None)
-    for M, N, K in ((136, 264, 1024), (300, 520, 7776)):
-        test_gemm_every_split(ops, M, N, K, two_cta, splits, monkeypatch)

@@ -502,8 +502,10 @@ done:
   }
 }
 
-// Clusters of two that can be co-resident (0: unsupported), plain / gather variant. All instances of a variant have the same
-// threads and shared memory, so one of them is asked, once.
+// Clusters of two that can be co-resident (0: unsupported), plain / gather variant. Instances differ in threads and registers (wide tiles: 384 of 168)
+// and in static shared memory (the grouped forms' table), but with tensor memory taken whole and more than half of an SM's shared memory every one
+// of them fits an SM exactly once, so one is asked, once.
+static_assert(SMEM + sizeof(GroupTable) <= 227 * 1024 && 2 * SMEM > 228 * 1024, "one CTA to an SM, in every instance");
 template <bool GATHER>
 static int co_resident_pairs() {
   static int pairs = -1;

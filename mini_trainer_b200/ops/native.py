@@ -688,10 +688,11 @@ class NativeOps:
 
     def _plan_grouped(self, key):
         """``mode`` of a grouped product's entry point, with its kernel, from its sizes and whether rows of an operand start off 32 bytes."""
-        mode, cap, E, M, N, K, off = key
+        mode, cap, E, M, N, K, off_a, off_b = key
         rows = cap - (_GROUP_ALIGN - 1) * E   # of all experts, to within a tile
-        wide = self.pair_max_flops > 0 and self.cta_pairs() > 0 and gemm_plan.grouped_wide(
-            mode == 2, rows, E, 2.0 * rows * N * (M if mode == 2 else K), K, off != 0)
+        wide = rows > 0 and self.pair_max_flops > 0 and self.cta_pairs() > 0 and gemm_plan.grouped_wide(
+            mode == 2, rows, E, 2.0 * rows * N * (M if mode == 2 else K), K, off_a != 0 or off_b != 0,
+            gemm_plan.grouped_ratio(mode == 2, rows, E, M, N, K, off_a != 0, off_b != 0, self.sms, self.cta_pairs()))
         if len(self._gemm_plans) >= 4096:
             self._gemm_plans.clear()
         self._gemm_plans[key] = mode + 4 * wide
@@ -699,7 +700,7 @@ class NativeOps:
 
     def _grouped(self, mode, a, b, ldb, out, ldd, sl, M, N, K, stride, act=None, fn="silu"):
         lda, cap, E = a.stride(0), sl.cap, sl.experts
-        key = (mode, cap, E, M, N, K, (lda | ldb) & 15)   # asked six times a layer, which the host bounds where experts are small
+        key = (mode, cap, E, M, N, K, lda & 15, ldb & 15)   # asked six times a layer, which the host bounds where experts are small
         form = self._gemm_plans.get(key)
         if form is None:
             form = self._plan_grouped(key)

@@ -259,10 +259,29 @@ def test_grouped_products_choice(reduce, rows, E, flops, K, ragged, want):
     assert G.grouped_wide(reduce, rows, E, flops, K, ragged) == want
 
 
+# (reduce, rows, E, M, N, K, rows of A and of B off 32 bytes, wide), each at least 5 % faster that way in a loop of its own: a round of single CTAs and as many of
+# pairs; two rounds and one; a round of pairs and a little; many rounds; tiles of which half is past the last column; long ones
+@pytest.mark.parametrize("reduce,rows,E,M,N,K,off_a,off_b,want", [(False, 1672, 8, 2688, 1944, 12160, False, True, False), (False, 2576, 16, 4608, 1248, 4088, True, True, False),
+                                                                  (False, 1668, 4, 2176, 2552, 7216, False, True, False), (False, 2576, 16, 4608, 4088, 1248, False, True, False),
+                                                                  (False, 3336, 8, 4352, 3704, 5456, False, True, True), (False, 1668, 4, 2176, 3608, 2552, True, True, True),
+                                                                  (False, 32016, 16, 34048, 632, 19744, False, True, True), (False, 5508, 4, 6016, 904, 3600, False, True, True),
+                                                                  (True, 8208, 16, 2832, 600, 0, False, True, False), (True, 10256, 16, 2048, 1144, 0, False, True, False),
+                                                                  (True, 1668, 4, 7216, 2552, 0, False, True, True), (True, 10376, 8, 8448, 536, 0, False, True, True),
+                                                                  (False, 7176, 8, 8192, 28672, 4096, False, False, True), (True, 7176, 8, 28672, 4096, 0, False, False, True)])
+def test_grouped_products_take_wide_tiles_where_their_rounds_come_out_shorter(reduce, rows, E, M, N, K, off_a, off_b, want):
+    ops = make_ops()
+    cap = rows + 127 * E
+    key = (2 if reduce else 1, cap, E, M, N, K, 8 * off_a, 8 * off_b)
+    assert ops._plan_grouped(key) == key[0] + 4 * want
+    ops._gemm_plans.clear()
+    ops._pairs = 0           # no clusters of two CTAs
+    assert ops._plan_grouped(key) == key[0]
+
+
 def test_grouped_product_is_planned_once_per_size(monkeypatch):
     from mini_trainer_b200.ops import gemm_plan, native
     asked = []
-    monkeypatch.setattr(gemm_plan, "grouped_wide", lambda reduce, rows, E, flops, K, ragged: asked.append((reduce, rows, E, flops, K, ragged)) or ragged)
+    monkeypatch.setattr(gemm_plan, "grouped_wide", lambda reduce, rows, E, flops, K, ragged, ratio: asked.append((reduce, rows, E, flops, K, ragged)) or ragged)
     ops = make_ops()
     i32 = lambda n: torch.zeros(n, dtype=torch.int32)   # noqa: E731
     for _ in range(3):

@@ -587,7 +587,15 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem<D>::TOTAL) != cudaSuccess) return -4;
     configured = true;
   }
-  launch_pdl(kern, n_items * p.Hkv * p.splits, AB_THREADS, AttBwdSmem<D>::TOTAL, st, a, b, c, d, p);
+  // Blocks that come under their predecessor's tail stand on whatever SMs are free first; launched behind its end, consecutive ones (the kv heads of a key block)
+  // go round the chip in order. At D = 128 that decides more than the 3 us of an early launch where a CTA has many iterations: the kernel alone takes
+  // 174 and 195 us with 4 samples in 4313 tokens, 32/8 heads, 370 and 406 with one, and forward and backward together 632 and 656, 956 and 990 with one of 9000 and
+  // 12/2 heads; with few iterations 48.6 early and 49.1 (1500 tokens in 8 samples, 12/2). At D = 64 early is the faster or level throughout. 12 iterations of a CTA
+  // on average are where the two meet; a sample leaves half a block empty, which is what their number is told from.
+  const long long empty = static_cast<long long>(n_items) * AB_B - p.T, samples = empty >= AB_B ? empty / (AB_B / 2) : 1;
+  const unsigned grid = n_items * p.Hkv * p.splits;
+  if (D == 128 && (n_items / samples + 1) * p.G >= 24LL * p.splits) kern<<<grid, AB_THREADS, AttBwdSmem<D>::TOTAL, st>>>(a, b, c, d, p);
+  else launch_pdl(kern, grid, AB_THREADS, AttBwdSmem<D>::TOTAL, st, a, b, c, d, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -624,6 +624,28 @@ def test_attention_work_distribution(ops, D, hq, hkv, lens):
     assert torch.equal(again[:, kv:], dqkv[:, kv:])     # dK and dV: one order of summation (dQ is accumulated in any order)
 
 
+# either side of the line between a launch under its predecessor's tail and one behind its end: 12 iterations of a CTA on average
+@pytest.mark.parametrize("lens", [[2800], [3100], [1500, 1600], [3200, 2900]])
+def test_attention_backward_waits_for_what_it_reads(ops, lens):
+    torch.manual_seed(sum(lens))
+    D, hq, hkv, T = 128, 8, 8, sum(lens)
+    qkv, a, b = bf(T, 3 * hq * D), bf(T, 2048, scale=2048 ** -0.5), bf(hq * D, 2048)
+    cu_host, cu = _cu(lens)
+    args = (cu, cu_host, max(lens), hq, hkv, D)
+    out, lse = ops.attention(qkv, *args)
+    want = ops.linear(a, b)
+    torch.cuda.synchronize()
+    ref = ops.attention_bwd(want, qkv, out, lse, *args)
+    rd = REF.attention_bwd(want.float(), qkv.float(), out.float(), lse, *args)
+    assert rel_err(ref, rd) < 1.5e-2
+    for _ in range(3):   # the gradient and the forward's results as they leave their kernels
+        torch.cuda.synchronize()
+        o, l = ops.attention(qkv, *args)
+        got = ops.attention_bwd(ops.linear(a, b), qkv, o, l, *args)
+        assert torch.equal(got[:, hq * D:], ref[:, hq * D:])     # dK and dV: one order of summation
+    ops.check_status()
+
+
 # more rows than resident blocks, row widths of one to eight vectors per thread
 @pytest.mark.parametrize("T,H", [(5000, 512), (3001, 2056), (700, 12296), (1300, 5000)])
 def test_norms_many_rows(ops, T, H):

@@ -60,7 +60,9 @@ constexpr int WIDE_STAGES = 4;                        // wide tiles: a second ha
 constexpr int WIDE_STAGE_BYTES = A_BYTES + 2 * B_BYTES;
 constexpr int WIDE_LAG = 2;                           // k-blocks by which the second half of a wide tile runs behind the first at its ends
 constexpr int WIDE_GROUP_M = 14;                      // row-tiles per band, about: the 74 tiles in flight then read 3600 rows of A and 2700 of B
-// Three warpgroups: {TMA, MMA}, and the epilogue of either half, whose threads hold 256 columns as 128 registers and the piece at work on.
+// Three warpgroups: {TMA, MMA}, and the epilogue of either half, whose threads hold 256 columns as 128 registers and the piece at work on. In the grouped forms and
+// those with an activation 5 to 16 words a thread are spilled all the same, and read back 17 to 42 times per item; the other splits
+// of the registers (24 / 240, 56 / 224, 72 / 216) spill more, also in the plain forms.
 constexpr int WIDE_THREADS = 384;
 constexpr int WIDE_REGS = 168, WIDE_REGS_IO = 40, WIDE_REGS_EPI = 232;   // per thread at launch, and after the split
 static_assert(WIDE_REGS_IO + 2 * WIDE_REGS_EPI == 3 * WIDE_REGS && 3 * 128 * WIDE_REGS <= 65536, "register split");

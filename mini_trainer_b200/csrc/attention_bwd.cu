@@ -580,21 +580,18 @@ __global__ void __launch_bounds__(256) attn_dq_store_kernel(const float* __restr
 }
 
 template <int D>
-static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const CUtensorMap& d, const AttBwdParams& p, int n_items, cudaStream_t st) {
+static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& c, const CUtensorMap& d, const AttBwdParams& p, int n_items, bool in_order, cudaStream_t st) {
   static bool configured = false;
   auto kern = attn_bwd_kernel<D>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttBwdSmem<D>::TOTAL) != cudaSuccess) return -4;
     configured = true;
   }
-  // Blocks that come under their predecessor's tail stand on whatever SMs are free first; launched behind its end, consecutive ones (the kv heads of a key block)
-  // go round the chip in order. At D = 128 that decides more than the 3 us of an early launch where a CTA has many iterations: the kernel alone takes
-  // 174 and 195 us with 4 samples in 4313 tokens, 32/8 heads, 370 and 406 with one, and forward and backward together 632 and 656, 956 and 990 with one of 9000 and
-  // 12/2 heads; with few iterations 48.6 early and 49.1 (1500 tokens in 8 samples, 12/2). At D = 64 early is the faster or level throughout. 12 iterations of a CTA
-  // on average are where the two meet; a sample leaves half a block empty, which is what their number is told from.
-  const long long empty = static_cast<long long>(n_items) * AB_B - p.T, samples = empty >= AB_B ? empty / (AB_B / 2) : 1;
+  // Blocks that come under their predecessor's tail stand on whatever SMs are free first; launched behind its end (in_order), consecutive ones (the kv heads of a
+  // key block) go round the chip in order. Where a block has many iterations that decides more than the 3 us of an early launch: the kernel alone, D = 128, 4313 tokens,
+  // 32/8 heads, 174 us in order and 195 early with 4 samples, 370 and 406 with one. The rule is attention_plan.backward_in_order.
   const unsigned grid = n_items * p.Hkv * p.splits;
-  if (D == 128 && (n_items / samples + 1) * p.G >= 24LL * p.splits) kern<<<grid, AB_THREADS, AttBwdSmem<D>::TOTAL, st>>>(a, b, c, d, p);
+  if (in_order) kern<<<grid, AB_THREADS, AttBwdSmem<D>::TOTAL, st>>>(a, b, c, d, p);
   else launch_pdl(kern, grid, AB_THREADS, AttBwdSmem<D>::TOTAL, st, a, b, c, d, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -604,9 +601,10 @@ static int launch_bwd(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
 // plan: key-block work table [n_items, 3] = (seq_start, seq_len, k0), most work first.
 // dq_acc: fp32 [T, Hq*D] scratch, 16-byte aligned; delta: fp32 [Hq, T] scratch.
 // splits: CTAs that share the query heads of a key block; more than one needs counters, an epoch and scratch as the split-K GEMM does.
+// in_order: the kernel is launched behind its predecessor's end (launch_bwd).
 extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, long long ldo, const void* dout, long long lddo,
                                void* dqkv, long long ldq, const float* lse, float* delta, float* dq_acc, const int* plan,
-                               int n_items, int T, int Hq, int Hkv, int D, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float scale, int* status, cudaStream_t st) {
+                               int n_items, int T, int Hq, int Hkv, int D, int splits, unsigned long long* counters, unsigned long long epoch, float* part, long long part_bytes, float scale, int in_order, int* status, cudaStream_t st) {
   using namespace mtb;
   if (n_items <= 0 || T <= 0) return 0;
   if ((D != 64 && D != 128) || Hq % Hkv || ld % 8 || ldo % 8 || lddo % 8 || ldq % 8 || splits < 1 || splits > Hq / Hkv) return -10;
@@ -626,7 +624,7 @@ extern "C" int mtb200_attn_bwd(const void* qkv, long long ld, const void* out, l
       reinterpret_cast<const __nv_bfloat16*>(out), ldo, reinterpret_cast<const __nv_bfloat16*>(dout), lddo, delta, dq_acc, T, Hq, D);
   AttBwdParams p{reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, lse, delta, dq_acc, plan, T, Hq, Hkv, Hq / Hkv, 0xffffffffu / static_cast<unsigned>(Hkv), splits,
                  part, counters, epoch, scale, status};
-  rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, tdkv, p, n_items, st) : launch_bwd<64>(tq, tdo, tdq, tdkv, p, n_items, st);
+  rc = D == 128 ? launch_bwd<128>(tq, tdo, tdq, tdkv, p, n_items, in_order != 0, st) : launch_bwd<64>(tq, tdo, tdq, tdkv, p, n_items, in_order != 0, st);
   if (rc) return rc;
   launch_pdl(attn_dq_store_kernel, dim3(static_cast<unsigned>(T), (Hq * D / 8 + 255) / 256), 256, 0, st, dq_acc, reinterpret_cast<__nv_bfloat16*>(dqkv), ldq, T, Hq * D);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;

@@ -115,7 +115,7 @@ long long backward(const BlockSpec& s, const BlockParams& p, const BlockParams& 
   const int splits = io.part != nullptr ? s.bwd_splits : 1;
   RUN(mtb200_attn_bwd(io.qkv, Q, io.attn, q, dattn, q, dqkv, Q, io.lse, delta, dq, io.bwd_plan, s.bwd_items, s.T, s.Hq, s.Hkv, s.D, splits,
                       splits > 1 ? io.counters : nullptr, splits > 1 ? *epoch++ : 0, splits > 1 ? io.part : nullptr, splits > 1 ? io.part_bytes : 0, s.scale,
-                      io.status, st), 3);
+                      s.bwd_in_order, io.status, st), 3);
   if (s.qk_norm) RUN(mtb200_head_rmsnorm_bwd(dqkv, io.qk_pre, io.rstd_qk, p.qn, p.kn, rows, g.qn, g.kn, io.inv_freq ? io.pos : nullptr, io.inv_freq, s.T, Q, nh * s.D,
                                              s.Hq, nh, s.D, st), 2);
   else if (io.inv_freq) RUN(mtb200_rope(dqkv, io.pos, io.inv_freq, s.T, Q, nh, s.D, 1, st), 1);

@@ -18,7 +18,7 @@ struct BlockSpec {
   int act_form;                     // kernel of the gate/up product where the activation is in it
   int need_out;                     // 0: the forward stops before the activation
   int attn_form;                    // 0: one query tile per CTA, 1: pairs of heads, 2: pairs of row blocks
-  int fwd_items, bwd_items, bwd_splits;
+  int fwd_items, bwd_items, bwd_splits, bwd_in_order;
 };
 // Parameters, or their gradients; null where the model has none.
 struct BlockParams {

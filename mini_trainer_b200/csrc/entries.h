@@ -44,7 +44,7 @@ int mtb200_head_rmsnorm_bwd(void*, const void*, const float*, const void*, const
 int mtb200_attn_fwd(const void*, long long, void*, long long, float*, const int*, int, int, int, int, int, int, float, int*, cudaStream_t);
 int mtb200_attn_fwd_one(const void*, long long, void*, long long, float*, const int*, int, int, int, int, int, float, int*, cudaStream_t);
 int mtb200_attn_bwd(const void*, long long, const void*, long long, const void*, long long, void*, long long, const float*, float*, float*, const int*, int,
-                    int, int, int, int, int, unsigned long long*, unsigned long long, float*, long long, float, int*, cudaStream_t);
+                    int, int, int, int, int, unsigned long long*, unsigned long long, float*, long long, float, int, int*, cudaStream_t);
 int mtb200_colsum(const void*, long long, void*, float*, int, int, cudaStream_t);
 int mtb200_embedding_fwd(const void*, const long long*, void*, int, int, int, int*, cudaStream_t);
 int mtb200_embedding_bwd_scan(void*, const long long*, const void*, int, int, int, int*, cudaStream_t);

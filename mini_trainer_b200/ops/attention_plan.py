@@ -97,3 +97,15 @@ def _backward_splits(blocks: list, hq: int, hkv: int, sms: int, most: int) -> in
         if t < best:
             best, splits = t, s
     return splits
+
+
+# Iterations of a CTA, on average, from which the backward is launched behind its predecessor's end and not under its tail (csrc/attention_bwd.cu). 85 batches at head_dim 128
+# (16/4, 32/8, 12/2, 16/16 and 8/1 heads, one to 148 sequences), early over in order, with the forward and with a product in front of it: from 20 on 0.99 to 1.15, 1.03 on
+# average (8 of 2048 tokens, 16/4: 675 and 586 us; one of 4096, 32/8: 601 and 569), below 12 0.95 to 1.04, 0.99 (37 of 128, 12/2: 53 and 54), between them
+# 0.97 to 1.05. At head_dim 64 early is the faster or level throughout (0.95 to 1.00 in 13 batches).
+IN_ORDER_ITERATIONS = 20
+
+
+def backward_in_order(blocks: list, hq: int, hkv: int, d: int, splits: int) -> bool:
+    """Backward: whether CTAs go round the chip in order, or come early to whatever SMs are free."""
+    return d == 128 and sum(b * (b + 1) for b in blocks) * (hq // hkv) >= 2 * IN_ORDER_ITERATIONS * splits * sum(blocks) > 0

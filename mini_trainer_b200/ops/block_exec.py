@@ -23,7 +23,7 @@ NAMES = ("ln1", "bln1", "wqkv", "bqkv", "qn", "kn", "wo", "bo", "ln2", "bln2", "
 class Spec(ctypes.Structure):
     _fields_ = [(n, c_int) for n in ("T", "H", "F", "Hq", "Hkv", "D", "gated", "gelu", "layernorm", "qk_norm")] \
         + [(n, c_float) for n in ("eps", "scale", "alpha")] + [("form", c_int * GEMMS), ("splits", c_int * GEMMS), ("act_form", c_int)] \
-        + [(n, c_int) for n in ("need_out", "attn_form", "fwd_items", "bwd_items", "bwd_splits")]
+        + [(n, c_int) for n in ("need_out", "attn_form", "fwd_items", "bwd_items", "bwd_splits", "bwd_in_order")]
 
 
 class Params(ctypes.Structure):
@@ -201,7 +201,7 @@ def backward(ops, cfg, p: dict, g: dict, a, dout, batch, inv_freq):
     io.pos, io.inv_freq, io.ws, io.status = batch.position_ids.data_ptr(), _ptr(inv_freq), ws.data_ptr(), ops.status.data_ptr()
     io.dout, io.dx = dout.data_ptr(), dx.data_ptr()
     cu = batch.cu_seqlens_host
-    plan, spec.bwd_splits, attn_bytes = ops._cached(cu, ("bwd", spec.Hq, spec.Hkv, spec.D)) or ops._plan_attention_bwd(cu, spec.Hq, spec.Hkv, spec.D)
+    plan, spec.bwd_splits, attn_bytes, spec.bwd_in_order = ops._cached(cu, ("bwd", spec.Hq, spec.Hkv, spec.D)) or ops._plan_attention_bwd(cu, spec.Hq, spec.Hkv, spec.D)
     spec.bwd_items, io.bwd_plan = plan.shape[0], plan.data_ptr()
     st = ops._st()
     alive = _split(ops, io, st, max(nbytes, attn_bytes if spec.bwd_splits > 1 else 0))

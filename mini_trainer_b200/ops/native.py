@@ -101,7 +101,7 @@ class _Sig:
     mtb200_moe_route_bwd = [P, P, P, P, I, I, I, I, P, P]
     mtb200_attn_fwd_one = [P, L, P, L, P, P, I, I, I, I, I, F, P, P]
     mtb200_attn_fwd = [P, L, P, L, P, P, I, I, I, I, I, I, F, P, P]
-    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, U, P, L, F, P, P]
+    mtb200_attn_bwd = [P, L, P, L, P, L, P, L, P, P, P, P, I, I, I, I, I, I, P, U, P, L, F, I, P, P]
 
 
 _GLU = {"silu": "mtb200_swiglu", "gelu_tanh": "mtb200_geglu"}
@@ -538,12 +538,13 @@ class NativeOps:
         return self._keep(cu_host, ("fwd", hq, hkv, d), plan)
 
     def _plan_attention_bwd(self, cu_host, hq, hkv, d):
-        """``(work table, CTAs per key block, bytes of their partials)`` of a minibatch's backward."""
+        """``(work table, CTAs per key block, bytes of their partials, launched in order)`` of a minibatch's backward."""
         table = self._attn_plan(cu_host, 128, False)
         units = table.shape[0] * hkv   # per unit: 8 counters and, for every CTA that shares it, dK and dV of 128 rows in fp32
         most = 1 if units * 8 > _SPLIT_COUNTERS else min(hq // hkv, _SPLIT_FLOATS // max(1, units * 2 * 128 * d))
         splits = attention_plan.backward_splits(attention_plan.blocks_per_sequence(cu_host), hq, hkv, self.sms, most)
-        return self._keep(cu_host, ("bwd", hq, hkv, d), (table, splits, splits * units * 2 * 128 * d * 4))
+        in_order = attention_plan.backward_in_order(attention_plan.blocks_per_sequence(cu_host), hq, hkv, d, splits)
+        return self._keep(cu_host, ("bwd", hq, hkv, d), (table, splits, splits * units * 2 * 128 * d * 4, int(in_order)))
 
     def _attn_table(self, cu_host, block, most_work_last_block: bool):
         items = []
@@ -576,7 +577,7 @@ class NativeOps:
         if self.attention_impl == "flash_attn" or d not in NATIVE_HEAD_DIMS:
             return self._fa_bwd(dout, qkv, out, lse, cu_seqlens, max_seqlen, hq, hkv, d, scale)
         dqkv = torch.empty_like(qkv)
-        plan, splits, nbytes = self._cached(cu_host, ("bwd", hq, hkv, d)) or self._plan_attention_bwd(cu_host, hq, hkv, d)
+        plan, splits, nbytes, in_order = self._cached(cu_host, ("bwd", hq, hkv, d)) or self._plan_attention_bwd(cu_host, hq, hkv, d)
         scratch = torch.empty(hq * T * (d + 1), dtype=torch.float32, device=self.device)   # dQ's accumulator [T, hq * d] and delta [hq, T]: one allocation
         dq_acc = scratch.data_ptr()
         st = self._st()
@@ -585,7 +586,7 @@ class NativeOps:
         self._call("mtb200_attn_bwd", qkv.data_ptr(), qkv.stride(0), out.data_ptr(), out.stride(0), dout.data_ptr(),
                    dout.stride(0), dqkv.data_ptr(), dqkv.stride(0), lse.data_ptr(), dq_acc + 4 * hq * T * d, dq_acc,
                    plan.data_ptr(), plan.shape[0], T, hq, hkv, d, splits if split else 1, _ptr(ws), epoch, _ptr(part), 4 * part.numel() if split else 0, scale,
-                   self.status.data_ptr(), st, n=3)
+                   in_order, self.status.data_ptr(), st, n=3)
         return dqkv
 
     # Library attention (flash-attn 2): selectable for A/B comparisons, and the path of head dimensions the

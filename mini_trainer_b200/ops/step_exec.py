@@ -94,7 +94,7 @@ def forward_backward(eng, batch, grad_scale: float):
     b = s.block
     cu = batch.cu_seqlens_host
     name, tail, fwd_plan = ops._cached(cu, ("fwd", b.Hq, b.Hkv, b.D)) or ops._plan_attention(cu, b.Hq, b.Hkv, b.D)
-    bwd_plan, b.bwd_splits, attn_part = ops._cached(cu, ("bwd", b.Hq, b.Hkv, b.D)) or ops._plan_attention_bwd(cu, b.Hq, b.Hkv, b.D)
+    bwd_plan, b.bwd_splits, attn_part, b.bwd_in_order = ops._cached(cu, ("bwd", b.Hq, b.Hkv, b.D)) or ops._plan_attention_bwd(cu, b.Hq, b.Hkv, b.D)
     b.need_out, b.attn_form, b.fwd_items, b.bwd_items = 1, (1 + tail[0] if name == "mtb200_attn_fwd" else 0), fwd_plan.shape[0], bwd_plan.shape[0]
     s.grad_scale = grad_scale
     io = IO()

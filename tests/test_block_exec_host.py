@@ -50,7 +50,7 @@ int mtb200_head_rmsnorm_bwd(void*, const void*, const float*, const void*, const
 int mtb200_attn_fwd(const void*, long long, void*, long long, float*, const int*, int, int, int, int, int, int, float, int*, cudaStream_t) { return 0; }
 int mtb200_attn_fwd_one(const void*, long long, void*, long long, float*, const int*, int, int, int, int, int, float, int*, cudaStream_t) { return 0; }
 int mtb200_attn_bwd(const void*, long long, const void*, long long, const void*, long long, void*, long long, const float*, float*, float*, const int*, int,
-                    int, int, int, int, int splits, u64*, u64 epoch, float*, long long, float, int*, cudaStream_t) {
+                    int, int, int, int, int splits, u64*, u64 epoch, float*, long long, float, int, int*, cudaStream_t) {
   noted[n_noted][0] = splits; noted[n_noted++][1] = epoch; return 0;
 }
 int mtb200_colsum(const void*, long long, void*, float*, int, int, cudaStream_t) { return 0; }

@@ -624,8 +624,8 @@ def test_attention_work_distribution(ops, D, hq, hkv, lens):
     assert torch.equal(again[:, kv:], dqkv[:, kv:])     # dK and dV: one order of summation (dQ is accumulated in any order)
 
 
-# either side of the line between a launch under its predecessor's tail and one behind its end: 12 iterations of a CTA on average
-@pytest.mark.parametrize("lens", [[2800], [3100], [1500, 1600], [3200, 2900]])
+# either side of the line between a launch under its predecessor's tail and one behind its end: 20 iterations of a CTA on average
+@pytest.mark.parametrize("lens", [[4864], [4992], [1500, 1600], [5200, 4900]])
 def test_attention_backward_waits_for_what_it_reads(ops, lens):
     torch.manual_seed(sum(lens))
     D, hq, hkv, T = 128, 8, 8, sum(lens)
@@ -633,6 +633,7 @@ def test_attention_backward_waits_for_what_it_reads(ops, lens):
     cu_host, cu = _cu(lens)
     args = (cu, cu_host, max(lens), hq, hkv, D)
     out, lse = ops.attention(qkv, *args)
+    assert ops._plan_attention_bwd(cu_host, hq, hkv, D)[1::2] == (1, int(min(lens) > 4864))
     want = ops.linear(a, b)
     torch.cuda.synchronize()
     ref = ops.attention_bwd(want, qkv, out, lse, *args)

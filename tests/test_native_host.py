@@ -122,6 +122,29 @@ def test_attention_backward_splits(lens, hq, hkv, lo, hi):
         assert A.backward_splits(blocks, hq, hkv, 148, most) <= most
 
 
+# (lengths, query heads, kv heads, CTAs per key block, in order): lengths that are whole blocks and that are not, many short samples, divided heads
+@pytest.mark.parametrize("lens,hq,hkv,splits,want", [([4096], 32, 8, 1, True), ([4313], 32, 8, 1, True), ([1024] * 37, 16, 4, 1, False), ([1100] * 37, 16, 4, 1, True),
+                                                     ([2048] * 8, 16, 4, 1, True), ([128] * 148, 16, 4, 1, False), ([1500], 12, 2, 6, False), ([4096], 12, 2, 3, True),
+                                                     ([3000], 16, 16, 1, False), ([5000], 16, 16, 1, True), ([], 8, 2, 1, False)])
+def test_attention_backward_in_order(lens, hq, hkv, splits, want):
+    from mini_trainer_b200.ops import attention_plan as A
+    blocks = [-(-n // 128) for n in lens]
+    assert A.backward_in_order(blocks, hq, hkv, 128, splits) == want and not A.backward_in_order(blocks, hq, hkv, 64, splits)
+    mean = sum((b - j) * hq / hkv / splits for b in blocks for j in range(b)) / max(1, sum(blocks))
+    assert (mean >= 20) == want
+    ops = make_ops()
+    ops.attention_impl = "native"
+    ops._attn_table = lambda cu, block, last: torch.zeros(sum(-(-(b - a) // block) for a, b in zip(cu[:-1], cu[1:])), 3, dtype=torch.int32)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    if lens:
+        plan = ops._plan_attention_bwd(cu, hq, hkv, 128)
+        qkv, o = torch.empty(cu[-1], (hq + 2 * hkv) * 128, dtype=torch.bfloat16), torch.empty(cu[-1], hq * 128, dtype=torch.bfloat16)
+        ops.attention_bwd(o, qkv, o, torch.empty(hq, cu[-1]), None, cu, max(lens), hq, hkv, 128)
+        assert ops.calls[-1][1][23] == plan[3] == int(A.backward_in_order(blocks, hq, hkv, 128, plan[1]))
+
+
 def test_attention_backward_divides_only_what_the_workspace_holds():
     ops = make_ops()
     ops.sms, ops.attention_impl = 148, "native"

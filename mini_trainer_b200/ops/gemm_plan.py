@@ -122,37 +122,29 @@ def wide(M: int, N: int, K: int, ragged: bool, sms: int, pairs: int, max_units: 
     return splits if cost <= other * (1.1 if flops > LONG_FLOPS else 1.0) else 0
 
 
-# Grouped products, as above: a k-block on single CTAs, in a weight gradient and else, what rows of A and of B that start off 32 bytes add to it, the rest of an item; a k-block and the rest of
-# an item on wide tiles. Fitted to 900 products of 160 drawn expert layers of 20 GFLOP and more, each in both forms (root mean square 8 to 12 %).
+# Grouped products, as above: a k-block on single CTAs, in a weight gradient and else, what rows of A and of B that start off 32 bytes add to it, the rest of an item;
+# a k-block and the rest of an item on wide tiles. Fitted to 900 products of 160 drawn expert layers of 20 GFLOP and more, each in both forms (root mean square 8 to 12 %).
 _GROUPED_ONE, _GROUPED_WIDE = (0.43, 0.46, 0.08, 0.13, 2.2), (0.84, 4.5)
 
 
 def grouped_ratio(reduce: bool, rows: int, experts: int, M: int, N: int, K: int, off_a: bool, off_b: bool, sms: int, pairs: int) -> float:
     """Estimated time of a grouped product on wide tiles over that on single CTAs. What decides is how many rounds the tiles take, and only the device knows
-    how the rows divide: a slab is taken to end anywhere in its last tile, so that the experts have ``rows`` / tile + half a tile each, and of that number, give
-    or take its spread, the case that is worst for wide tiles counts."""
-    tall, cols, worst = rows / experts, -(-N // 256), 0.0
+    how the rows divide: a slab is taken to end anywhere in its last tile, so that the experts have ``rows`` / tile + half a tile each."""
+    tall, cols = rows / experts, -(-N // 256)
     kblocks = tall / BK + 0.5 if reduce else -(-K // BK)
     gradient, other, add_a, add_b, item = _GROUPED_ONE
     block = (gradient if reduce else other) + add_a * off_a + add_b * off_b
     wide_block, wide_item = _GROUPED_WIDE
-    spread = 0.29 * experts ** 0.5   # of the sum of as many ends, each uniform over a tile
-    for d in ((0.0,) if reduce else (-spread, 0.0, spread)):
-        if reduce:
-            low, high = experts * -(-M // 128), experts * -(-M // 256)
-        else:
-            low, high = (max(experts * (tall / t + 0.5) + d, experts) for t in (128, 256))
-        rounds = low * cols / sms
-        one = (rounds + 0.5 if rounds >= 6 else -(-rounds // 1)) * (kblocks * block + item)   # (many rounds even out)
-        wide = high * -(-N // 512)
-        there = high * cols / (2 * wide)   # of the tiles' columns, those that are there
-        full, rest = divmod(wide, pairs)
-        if wide >= 6 * pairs:
-            full, tail = wide / pairs + 0.25, 0.0
-        else:
-            tail = 0.0 if rest < 0.5 else 0.5 if 2 * rest <= pairs else 1.0   # given out as half tiles
-        worst = max(worst, (full * (kblocks * wide_block * there + wide_item) + (kblocks * wide_block * tail + wide_item if tail else 0.0)) / one)
-    return worst
+    low, high = (experts * -(-M // t) if reduce else max(experts * (tall / t + 0.5), experts) for t in (128, 256))
+    rounds = low * cols / sms
+    one = (rounds + 0.5 if rounds >= 6 else -(-rounds // 1)) * (kblocks * block + item)   # (many rounds even out)
+    wide = high * -(-N // 512)
+    there = high * cols / (2 * wide)   # of the tiles' columns, those that are there
+    full, rest = divmod(wide, pairs)
+    tail = 0.0 if rest < 0.5 else 0.5 if 2 * rest <= pairs else 1.0   # given out as half tiles
+    if wide >= 6 * pairs:
+        full, tail = wide / pairs + 0.25, 0.0
+    return (full * (kblocks * wide_block * there + wide_item) + (kblocks * wide_block * tail + wide_item if tail else 0.0)) / one
 
 
 def grouped_wide(reduce: bool, rows: int, experts: int, flops: float, K: int, ragged: bool, ratio: float = 0.0) -> bool:
@@ -160,12 +152,16 @@ def grouped_wide(reduce: bool, rows: int, experts: int, flops: float, K: int, ra
     rows may find 128 in a slab's last one, so slabs have to be tall. Rows that start off 32 bytes are 1.1 to 1.7 times as fast
     wide (749 tokens x 4 of 16 experts of 2376 x 7528: 414 -> 366, 282 -> 178, 228 -> 180, 550 -> 316 us), others 0.6 to 1.05 unless the launch is long enough
     for the power cap (8 of 4096 x 14336, 4096 tokens x 2: layer 8200 -> 7780 us). But a product that is a round of single CTAs and as many, longer, rounds of
-    pairs, or a little more than a round of them, loses (402 tokens x 4 of 8 experts of 1944 x 6080, a gradient: 107 -> 142 us), so the estimate (``ratio``) has to
-    agree. Of 623 such products, 403 were wide without it, which made them all 1.16 times as fast, but 47 slower, by up to 38 %; with it 298, 1.15, and 2."""
+    pairs loses (402 tokens x 4 of 8 experts of 1944 x 6080: 107 -> 142 us, the layer 696 -> 721), so the estimate (``ratio``) may not be far above 1. The
+    line is drawn by whole layers, 21 of them with some of their products either way, since their loops are at the power cap and a product's own is not: narrow
+    were faster those with a product of 1.17 and more (by 8 to 51 us), wide those whose estimates end at 1.10 (by up to 76 us)."""
     tall = rows / experts
+    if ratio > GROUPED_MOST:
+        return False
     if flops >= GROUPED_LONG_FLOPS:
-        return tall >= 768 and ratio < 1.0
-    return ragged and flops >= 2e10 and (tall >= 330 and ratio < 0.9 if reduce else tall >= 160 and K >= 1024 and ratio < 0.95)
+        return tall >= 768
+    return ragged and flops >= 2e10 and (tall >= 330 if reduce else tall >= 160 and K >= 1024)
 
 
+GROUPED_MOST = 1.13
 GROUPED_LONG_FLOPS = 8e11

@@ -282,14 +282,14 @@ def test_grouped_products_choice(reduce, rows, E, flops, K, ragged, want):
     assert G.grouped_wide(reduce, rows, E, flops, K, ragged) == want
 
 
-# (reduce, rows, E, M, N, K, rows of A and of B off 32 bytes, wide), each at least 5 % faster that way in a loop of its own: a round of single CTAs and as many of
-# pairs; two rounds and one; a round of pairs and a little; many rounds; tiles of which half is past the last column; long ones
+# (reduce, rows, E, M, N, K, rows of A and of B off 32 bytes, wide): a round of single CTAs and as many of pairs; two rounds and one; many rounds; tiles of which half
+# is past the last column; a weight gradient with little more; long ones
 @pytest.mark.parametrize("reduce,rows,E,M,N,K,off_a,off_b,want", [(False, 1672, 8, 2688, 1944, 12160, False, True, False), (False, 2576, 16, 4608, 1248, 4088, True, True, False),
-                                                                  (False, 1668, 4, 2176, 2552, 7216, False, True, False), (False, 2576, 16, 4608, 4088, 1248, False, True, False),
-                                                                  (False, 3336, 8, 4352, 3704, 5456, False, True, True), (False, 1668, 4, 2176, 3608, 2552, True, True, True),
-                                                                  (False, 32016, 16, 34048, 632, 19744, False, True, True), (False, 5508, 4, 6016, 904, 3600, False, True, True),
-                                                                  (True, 8208, 16, 2832, 600, 0, False, True, False), (True, 10256, 16, 2048, 1144, 0, False, True, False),
-                                                                  (True, 1668, 4, 7216, 2552, 0, False, True, True), (True, 10376, 8, 8448, 536, 0, False, True, True),
+                                                                  (False, 4752, 16, 6656, 584, 17760, False, True, False), (False, 1286, 4, 1792, 2888, 18256, False, True, False),
+                                                                  (True, 6532, 4, 2456, 768, 0, True, False, False), (False, 3336, 8, 4352, 3704, 5456, False, True, True),
+                                                                  (False, 1668, 4, 2176, 3608, 2552, True, True, True), (False, 32016, 16, 34048, 632, 19744, False, True, True),
+                                                                  (False, 5508, 4, 6016, 904, 3600, False, True, True), (True, 1668, 4, 7216, 2552, 0, False, True, True),
+                                                                  (True, 10376, 8, 8448, 536, 0, False, True, True), (False, 3460, 4, 4096, 3544, 12144, False, True, True),
                                                                   (False, 7176, 8, 8192, 28672, 4096, False, False, True), (True, 7176, 8, 28672, 4096, 0, False, False, True)])
 def test_grouped_products_take_wide_tiles_where_their_rounds_come_out_shorter(reduce, rows, E, M, N, K, off_a, off_b, want):
     ops = make_ops()
